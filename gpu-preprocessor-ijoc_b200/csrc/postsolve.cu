@@ -5,9 +5,9 @@
 //
 // Reference: postsolve_gpu (cpp/src/presolve/gpu_postsolve.cu:535-670) and the
 // record handlers in cpp/src/presolve/postsolve/*.cuh.  The per-record
-// arithmetic is the reference's; records are replayed in reverse
-// chronological order by one thread per segment walk (the reference's serial
-// interpreter), and the closing projection runs one thread per column.
+// arithmetic is the reference's; records that share a resource are replayed
+// in reverse chronological order by one thread, independent groups of records
+// in parallel, and the closing projection runs one thread per column.
 #include "presolve.hpp"
 #include "sort.hpp"
 
@@ -16,8 +16,6 @@ namespace gpp {
 namespace {
 
 constexpr double kTol = 1e-7;
-// Tapes shorter than this replay on one thread (the grouping costs more).
-constexpr int64_t kParallelMinRecords = 1024;
 enum : int {
   kFixedVariable = 0, kInfiniteBoundDualFix = 1, kSingletonColumnSubstitution = 2, kParallelColumn = 3,
   kParallelRow = 4, kDeletedRow = 5, kRowDualShift = 10, kRowImpliedBoundChange = 12, kDoubletonEquation = 13,
@@ -304,37 +302,35 @@ struct SegView {
   int64_t count;
 };
 
-// The reference's serial interpreter: one thread walks records [lo, hi) of a
-// segment backwards.
-__global__ void replay_serial(SegView t, Sol s, Model M, int primal, int dual, int64_t lo, int64_t hi) {
-  if (blockIdx.x || threadIdx.x) return;
-  for (int64_t k = hi - 1; k >= lo; --k)
-    replay_record(t.types[k], t.idx + t.is[k], t.is[k + 1] - t.is[k], t.val + t.vs[k], t.vs[k + 1] - t.vs[k], s, M,
-                  primal != 0, dual != 0);
+// The reduced solution to original indices: x, z and the retrieval flag of a
+// kept column, y of a kept row, in one launch.
+__global__ void scatter_solution(Sol s, const double* __restrict__ x_red, const double* __restrict__ y_red,
+                                 const double* __restrict__ z_red, const int32_t* __restrict__ rows, int32_t m,
+                                 const int32_t* __restrict__ cols, int32_t n) {
+  const int top = n > m ? n : m;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < top; i += gridDim.x * blockDim.x) {
+    if (i < n) {
+      const int j = cols[i];
+      if (x_red) s.x[j] = x_red[i];
+      if (s.z && z_red) s.z[j] = z_red[i];
+      s.got[j] = 1;
+    }
+    if (i < m && s.y && y_red) s.y[rows[i]] = y_red[i];
+  }
 }
 
-__global__ void scatter(double* __restrict__ dst, const double* __restrict__ src, const int32_t* __restrict__ map,
-                        int32_t n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[map[i]] = src[i];
-}
-__global__ void mark(uint8_t* __restrict__ got, const int32_t* __restrict__ map, int32_t n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) got[map[i]] = 1;
-}
-__global__ void restore_fixed(double* __restrict__ x, const int32_t* __restrict__ idx, const double* __restrict__ val,
-                              int64_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    x[idx[i]] = val[i];
-}
-__global__ void mark_protected(SegView t, uint8_t* __restrict__ prot, int n) {
-  for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < t.count; k += int64_t(gridDim.x) * blockDim.x) {
-    const int type = t.types[k];
-    const int32_t* id = t.idx + t.is[k];
-    int a = -1, b = -1;
-    if (type == kSingletonColumnSubstitution || type == kParallelColumn) a = id[0];
-    if (type == kDoubletonEquation) { a = id[0]; b = id[1]; }
-    if (type == kInfiniteBoundDualFix) a = id[1];
-    if (a >= 0 && a < n) prot[a] = 1;
-    if (b >= 0 && b < n) prot[b] = 1;
+// The fixed-value segments of a record: a column is removed once, so it is in
+// one of them at most and they can be restored together.
+struct FixedView {
+  const int32_t* idx;
+  const double* val;
+  int64_t count;
+};
+__global__ void restore_fixed(double* __restrict__ x, const FixedView* __restrict__ fixed, int segments) {
+  for (int k = 0; k < segments; ++k) {
+    const FixedView f = fixed[k];
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < f.count; i += int64_t(gridDim.x) * blockDim.x)
+      x[f.idx[i]] = f.val[i];
   }
 }
 // project_column_duals_from_original (gpu_postsolve.cu:355-398, postsolve_common.cuh:59-94):
@@ -366,13 +362,14 @@ SegView view(const PostsolveSegment& s) { return {s.types.p, s.is.p, s.vs.p, s.i
 // the columns (x, z and the retrieval flag together) and the rows (y) of the
 // original model; per pass only what that pass reads or writes counts (x is
 // read-only in the dual pass, y and z untouched in the primal pass).  Records
-// that do nothing in a pass (variable bound changes, and the dual-only records
-// in the primal pass) drop out.  Groups come from a lock-free union-find over
-// the records; each group is replayed by one thread, newest record first.
+// that do nothing in a pass (variable bound changes, the dual-only records in
+// the primal pass, records whose own values and x show that they change
+// nothing) drop out.  Groups come from a lock-free union-find over the
+// records.
 
 struct TapeView {
   const SegView* segs;       // device array
-  const int64_t* starts;     // global index of each segment's first record, count+1 entries
+  const int64_t* starts;     // global index of each segment's first record
   int nseg;
   int64_t total;
   __device__ void at(int64_t g, int& type, const int32_t*& id, int64_t& ni, const double*& v, int64_t& nv) const {
@@ -396,6 +393,23 @@ __device__ __forceinline__ bool replays_in(int type, bool dual) {
       type == kParallelColumn || type == kDoubletonEquation || type == kFmeCol)
     return true;
   return dual && (type == kRowDualShift || type == kParallelRow || type == kDeletedRow || type == kRowImpliedBoundChange);
+}
+
+// A record that replay_record leaves without a write whatever z, y and the
+// retrieval flags hold.  A row-implied bound change acts only if exactly one
+// of its bounds moved and x sits at the implied one (x is final before the
+// dual pass).  On most points almost none does, while each would tie all
+// columns of its row into one group: on the QAP N = 30 relaxation the 0.8M
+// records formed one group that a single thread replayed in 1,325 ms; without
+// the records that cannot act the whole call (presolve and postsolve) takes
+// 13.2 ms, 1,350 ms before.
+__device__ __forceinline__ bool acts_in_dual(int type, const int32_t* id, int64_t ni, const double* v,
+                                             const Model& M, const double* x) {
+  if (type != kRowImpliedBoundChange) return true;
+  if (!M.present || ni < 2) return false;
+  const bool lc = v[2] > v[0] + kTol, uc = v[3] < v[1] - kTol;
+  if (lc == uc) return false;
+  return !(fabs(x[id[0]] - (lc ? v[2] : v[3])) > kTol);
 }
 
 // Calls visit(resource, writes) for every resource the record touches in the
@@ -481,43 +495,23 @@ __device__ void record_resources(int type, const int32_t* id, int64_t ni, int64_
   }
 }
 
-__global__ void cp_active(TapeView t, int dual, int64_t lo, int64_t hi, int32_t* __restrict__ flag) {
-  for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < t.total; g += int64_t(gridDim.x) * blockDim.x) {
-    int type;
-    const int32_t* id;
-    int64_t ni, nv;
-    const double* v;
-    t.at(g, type, id, ni, v, nv);
-    flag[g] = g >= lo && g < hi && replays_in(type, dual != 0) ? 1 : 0;
-  }
+// A record that a pass replays.
+__device__ __forceinline__ bool record_acts(int type, const int32_t* id, int64_t ni, const double* v, bool dual,
+                                            const Model& M, const double* x) {
+  return replays_in(type, dual) && (!dual || acts_in_dual(type, id, ni, v, M, x));
 }
 
-__global__ void cp_list(int64_t total, const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
-                        int64_t* __restrict__ act, int32_t* __restrict__ parent) {
-  for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < total; g += int64_t(gridDim.x) * blockDim.x)
-    if (flag[g]) { act[pos[g]] = g; parent[pos[g]] = pos[g]; }
-}
-
-// First writer of each resource owns it.
-__global__ void cp_claim(TapeView t, const int64_t* __restrict__ act, int count, int dual, int m, int n, Model M,
-                         int32_t* __restrict__ owner) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-    int type;
-    const int32_t* id;
-    int64_t ni, nv;
-    const double* v;
-    t.at(act[q], type, id, ni, v, nv);
-    record_resources(type, id, ni, nv, dual != 0, m, n, M, [&](int res, bool w) {
-      if (w) atomicCAS(owner + res, -1, q);
-    });
-  }
-}
-
+// Root of a record's group; the path is halved on the way (a store to a
+// record that is no root, which no link ever targets).
 __device__ __forceinline__ int uf_root(int32_t* parent, int a) {
+  volatile int32_t* p = parent;
   for (;;) {
-    const int b = *(volatile int32_t*)(parent + a);
+    const int b = p[a];
     if (b == a) return a;
-    a = b;
+    const int c = p[b];
+    if (c == b) return b;
+    p[a] = c;
+    a = c;
   }
 }
 // Link the larger root under the smaller; a failed CAS means the root moved,
@@ -533,99 +527,213 @@ __device__ void uf_unite(int32_t* parent, int a, int b) {
   }
 }
 
-// Every record joins the owner of each resource it touches.
-__global__ void cp_connect(TapeView t, const int64_t* __restrict__ act, int count, int dual, int m, int n, Model M,
-                           const int32_t* __restrict__ owner, int32_t* __restrict__ parent) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-    int type;
-    const int32_t* id;
-    int64_t ni, nv;
-    const double* v;
-    t.at(act[q], type, id, ni, v, nv);
-    record_resources(type, id, ni, nv, dual != 0, m, n, M, [&](int res, bool) {
-      const int o = owner[res];
-      if (o >= 0 && o != q) uf_unite(parent, q, o);
+// One record of the tape.
+struct RecordAt {
+  int type;
+  const int32_t* id;
+  int64_t ni, nv;
+  const double* v;
+  __device__ RecordAt(const TapeView& t, int64_t g) { t.at(g, type, id, ni, v, nv); }
+};
+
+// Records lo + q, q < count, of the tape.  First every record that acts
+// claims the resources it writes (owner: record + 1, 0 for none); the others
+// get parent -1.
+__device__ __forceinline__ void claim_record(const TapeView& t, int64_t lo, int q, bool dual, int m, int n,
+                                             const Model& M, const double* x, int32_t* owner, int32_t* parent) {
+  const RecordAt r(t, lo + q);
+  const bool acts = record_acts(r.type, r.id, r.ni, r.v, dual, M, x);
+  parent[q] = acts ? q : -1;
+  if (acts)
+    record_resources(r.type, r.id, r.ni, r.nv, dual, m, n, M, [&](int res, bool w) {
+      if (w && owner[res] == 0) atomicCAS(owner + res, 0, q + 1);
     });
-  }
+}
+// Then every record joins the owner of each resource it touches.
+__device__ __forceinline__ void connect_record(const TapeView& t, int64_t lo, int q, bool dual, int m, int n,
+                                               const Model& M, const int32_t* owner, int32_t* parent) {
+  if (parent[q] < 0) return;
+  const RecordAt r(t, lo + q);
+  record_resources(r.type, r.id, r.ni, r.nv, dual, m, n, M, [&](int res, bool) {
+    const int o = owner[res] - 1;
+    if (o >= 0 && o != q) uf_unite(parent, q, o);
+  });
+}
+__device__ __forceinline__ void replay_at(const TapeView& t, int64_t g, const Sol& s, const Model& M, bool dual) {
+  const RecordAt r(t, g);
+  replay_record(r.type, r.id, r.ni, r.v, r.nv, s, M, !dual, dual);
 }
 
-__global__ void cp_keys(int count, const int32_t* __restrict__ parent, uint64_t* __restrict__ keys,
-                        int32_t* __restrict__ vals) {
+__global__ void rg_claim(TapeView t, int64_t lo, int count, int dual, int m, int n, Model M,
+                         const double* __restrict__ x, int32_t* owner, int32_t* __restrict__ parent) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
+    claim_record(t, lo, q, dual != 0, m, n, M, x, owner, parent);
+}
+__global__ void rg_connect(TapeView t, int64_t lo, int count, int dual, int m, int n, Model M,
+                           const int32_t* __restrict__ owner, int32_t* parent) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
+    connect_record(t, lo, q, dual != 0, m, n, M, owner, parent);
+}
+// Roots are final: a root with another member is marked.
+__global__ void rg_roots(int count, int32_t* parent, uint8_t* __restrict__ shared_root) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-    int r = q;
-    while (parent[r] != r) r = parent[r];
-    keys[q] = (uint64_t(uint32_t(r)) << 32) | uint32_t(q);
-    vals[q] = q;
+    if (parent[q] < 0) continue;
+    const int r = uf_root(parent, q);
+    if (r != q) shared_root[r] = 1;
   }
 }
-
-__global__ void cp_heads(int count, const uint64_t* __restrict__ keys, int32_t* __restrict__ head) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
-    head[q] = q == 0 || (keys[q] >> 32) != (keys[q - 1] >> 32) ? 1 : 0;
+// A record alone in its group is replayed here; the members of larger groups
+// are listed as (root, record) for the sort.  Most records are alone, so the
+// sort sees few, and the whole tape needs one wait per pass (500,000 x
+// 1,250,000 random LP: 862 us before, with every record sorted, four waits
+// and one marking launch per segment; 375 us now).
+__global__ void __launch_bounds__(kThreads) rg_replay_alone(TapeView t, int64_t lo, int count, int dual, Sol s, Model M,
+                                                            int32_t* parent, const uint8_t* __restrict__ shared_root,
+                                                            uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
+                                                            int32_t* counter) {
+  const int stride = gridDim.x * blockDim.x;
+  const int64_t top = (int64_t(count) + stride - 1) / stride * stride;
+  for (int64_t p = blockIdx.x * blockDim.x + threadIdx.x; p < top; p += stride) {
+    const int q = int(p);
+    const int r = p < count && parent[q] >= 0 ? uf_root(parent, q) : -1;
+    const bool listed = r >= 0 && (r != q || shared_root[q]);
+    const int at = block_append(counter, listed);
+    if (listed) {
+      keys[at] = (uint64_t(uint32_t(r)) << 32) | uint32_t(q);
+      vals[at] = q;
+    } else if (r >= 0) {
+      replay_at(t, lo + q, s, M, dual != 0);
+    }
+  }
 }
-__global__ void cp_starts(int count, const int32_t* __restrict__ head, const int32_t* __restrict__ hpos,
-                          int32_t* __restrict__ start) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
-    if (head[q]) start[hpos[q]] = q;
-}
-
-// One thread per group: its records (sorted ascending) replayed newest first.
-__global__ void cp_replay(TapeView t, const int64_t* __restrict__ act, const uint64_t* __restrict__ keys,
-                          const int32_t* __restrict__ start, int groups, int count, Sol s, Model M, int primal,
-                          int dual) {
-  for (int gi = blockIdx.x * blockDim.x + threadIdx.x; gi < groups; gi += gridDim.x * blockDim.x) {
-    const int b = start[gi], e = gi + 1 < groups ? start[gi + 1] : count;
-    for (int q = e - 1; q >= b; --q) {
-      int type;
-      const int32_t* id;
-      int64_t ni, nv;
-      const double* v;
-      t.at(act[uint32_t(keys[q] & 0xffffffffu)], type, id, ni, v, nv);
-      replay_record(type, id, ni, v, nv, s, M, primal != 0, dual != 0);
+// One thread per listed group: the thread at the group's last (newest) record
+// replays it and walks back to the group's first.
+__global__ void rg_replay_groups(TapeView t, int64_t lo, int listed, const uint64_t* __restrict__ keys, int dual, Sol s,
+                                 Model M) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < listed; e += gridDim.x * blockDim.x) {
+    const uint32_t root = uint32_t(keys[e] >> 32);
+    if (e + 1 < listed && uint32_t(keys[e + 1] >> 32) == root) continue;
+    for (int q = e; q >= 0; --q) {
+      const uint64_t k = keys[q];
+      if (uint32_t(k >> 32) != root) break;
+      replay_at(t, lo + int64_t(uint32_t(k)), s, M, dual != 0);
     }
   }
 }
 
-// Replays the records [lo, hi) of the whole tape (global indices).
-void replay_parallel(const std::vector<PostsolveSegment>& segments, int m0, int n0, const Sol& s, const Model& M,
-                     bool dual, cudaStream_t st, int64_t lo, int64_t hi) {
-  std::vector<SegView> hv;
-  std::vector<int64_t> hs{0};
-  for (const auto& seg : segments) {
-    if (!seg.count) continue;
-    hv.push_back(view(seg));
-    hs.push_back(hs.back() + seg.count);
+// Tapes of at most kBlockTape records: the whole replay, both passes, in one
+// block, with the union-find and the sort in shared memory.  A tape this
+// short is bound by launches: the passes above cost about eight launches and
+// a wait each, and one thread alone walks a record in 1-2 us (the 400 x 1,000
+// slack LP's tape took 0.47 ms; with the block its call went from 7.1 to
+// 6.5 ms).
+constexpr int kBlockTape = 2048;
+constexpr int kBlockReplayThreads = 512;
+__global__ void __launch_bounds__(kBlockReplayThreads)
+replay_block(TapeView t, int64_t lo, int count, int primal, int dual, int m, int n, Sol s, Model M, int32_t* owner) {
+  __shared__ int32_t parent[kBlockTape];
+  __shared__ uint32_t key[kBlockTape];
+  __shared__ uint8_t shared_root[kBlockTape];
+  __shared__ int listed;
+  for (int pass = primal ? 0 : 1; pass < (dual ? 2 : 1); ++pass) {
+    const bool d = pass == 1;
+    if (threadIdx.x == 0) listed = 0;
+    for (int q = threadIdx.x; q < count; q += kBlockReplayThreads) {
+      shared_root[q] = 0;
+      claim_record(t, lo, q, d, m, n, M, s.x, owner, parent);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < count; q += kBlockReplayThreads) connect_record(t, lo, q, d, m, n, M, owner, parent);
+    __syncthreads();
+    for (int q = threadIdx.x; q < count; q += kBlockReplayThreads) {
+      if (parent[q] < 0) continue;
+      const int r = uf_root(parent, q);
+      if (r != q) shared_root[r] = 1;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < count; q += kBlockReplayThreads) {
+      if (parent[q] < 0) continue;
+      if (!d && dual) {   // the dual pass claims afresh
+        const RecordAt r(t, lo + q);
+        record_resources(r.type, r.id, r.ni, r.nv, d, m, n, M, [&](int res, bool w) { if (w) owner[res] = 0; });
+      }
+      const int root = uf_root(parent, q);
+      if (root != q || shared_root[q]) key[atomicAdd(&listed, 1)] = (uint32_t(root) << 16) | uint32_t(q);
+      else replay_at(t, lo + q, s, M, d);
+    }
+    __syncthreads();
+    int size = 1;
+    while (size < listed) size <<= 1;
+    for (int i = listed + int(threadIdx.x); i < size; i += kBlockReplayThreads) key[i] = 0xffffffffu;
+    __syncthreads();
+    for (int width = 2; width <= size; width <<= 1)
+      for (int stride = width >> 1; stride > 0; stride >>= 1) {
+        for (int i = threadIdx.x; i < size; i += kBlockReplayThreads) {
+          const int j = i ^ stride;
+          const uint32_t a = key[i], b = j > i ? key[j] : a;
+          if (j > i && (a > b) == ((i & width) == 0)) {
+            key[i] = b;
+            key[j] = a;
+          }
+        }
+        __syncthreads();
+      }
+    for (int e = threadIdx.x; e < listed; e += kBlockReplayThreads) {
+      const uint32_t root = key[e] >> 16;
+      if (e + 1 < listed && key[e + 1] >> 16 == root) continue;
+      for (int q = e; q >= 0 && key[q] >> 16 == root; --q) replay_at(t, lo + int64_t(key[q] & 0xffffu), s, M, d);
+    }
+    __syncthreads();
   }
-  const int64_t total = hs.back();
-  if (!total) return;
-  DBuf<SegView> segs(hv.size(), st);
-  DBuf<int64_t> starts(hs.size(), st);
-  check(cudaMemcpyAsync(segs.p, hv.data(), sizeof(SegView) * hv.size(), cudaMemcpyHostToDevice, st), "tape views");
-  check(cudaMemcpyAsync(starts.p, hs.data(), sizeof(int64_t) * hs.size(), cudaMemcpyHostToDevice, st), "tape starts");
-  const TapeView t{segs.p, starts.p, int(hv.size()), total};
-  DBuf<int32_t> flag(size_t(total) + 1, st), pos(size_t(total) + 1, st);
-  GPP_LAUNCH(cp_active, grid_stride_blocks(total), kThreads, 0, st, t, int(dual), lo, hi, flag.p);
-  exclusive_scan_i32(flag.p, pos.p, total, st);
-  const int count = read_scalar(pos.p + total);
-  if (!count) return;
-  DBuf<int64_t> act(size_t(count), st);
-  DBuf<int32_t> parent(size_t(count), st), owner(size_t(m0) + size_t(n0), st);
-  GPP_LAUNCH(cp_list, grid_stride_blocks(total), kThreads, 0, st, total, flag.p, pos.p, act.p, parent.p);
-  check(cudaMemsetAsync(owner.p, 0xff, sizeof(int32_t) * (size_t(m0) + size_t(n0)), st), "owners");
-  const int g = grid_stride_blocks(count);
-  GPP_LAUNCH(cp_claim, g, kThreads, 0, st, t, act.p, count, int(dual), m0, n0, M, owner.p);
-  GPP_LAUNCH(cp_connect, g, kThreads, 0, st, t, act.p, count, int(dual), m0, n0, M, owner.p, parent.p);
+}
+
+// Replays the records [lo, hi) of the whole tape (global indices): the primal
+// pass, the dual pass or both.
+void replay_range(const TapeView& t, int m0, int n0, const Sol& s, const Model& M, bool primal, bool dual,
+                  cudaStream_t st, int64_t lo, int64_t hi) {
+  if (lo >= hi) return;
+  if (hi - lo > INT32_MAX) throw LengthError("postsolve: more than 2^31 - 1 tape records");
+  const int count = int(hi - lo);
+  const size_t resources = size_t(m0) + size_t(n0);
+  if (count <= kBlockTape) {
+    DBuf<int32_t> owner(std::max<size_t>(resources, 1), st);
+    owner.zero();
+    GPP_LAUNCH(replay_block, 1, kBlockReplayThreads, 0, st, t, lo, count, int(primal), int(dual), m0, n0, s, M,
+               owner.p);
+    return;
+  }
+  // Owners, the marks of shared roots and the list's counter, cleared at once.
+  DBuf<int32_t> scratch(resources + (size_t(count) + 3) / 4 + 1, st);
+  int32_t* owner = scratch.p;
+  auto* shared_root = reinterpret_cast<uint8_t*>(owner + resources);
+  int32_t* counter = scratch.p + scratch.n - 1;
+  DBuf<int32_t> parent(size_t(count), st), vals(size_t(count), st);
   DBuf<uint64_t> keys(size_t(count), st);
-  DBuf<int32_t> vals(size_t(count), st), head(size_t(count) + 1, st), hpos(size_t(count) + 1, st);
-  GPP_LAUNCH(cp_keys, g, kThreads, 0, st, count, parent.p, keys.p, vals.p);
-  radix_sort_pairs(keys.p, vals.p, count, st);
-  GPP_LAUNCH(cp_heads, g, kThreads, 0, st, count, keys.p, head.p);
-  exclusive_scan_i32(head.p, hpos.p, count, st);
-  const int groups = read_scalar(hpos.p + count);
-  DBuf<int32_t> gstart(size_t(groups), st);
-  GPP_LAUNCH(cp_starts, g, kThreads, 0, st, count, head.p, hpos.p, gstart.p);
-  GPP_LAUNCH(cp_replay, grid_stride_blocks(groups, 128), 128, 0, st, t, act.p, keys.p, gstart.p, groups, count, s, M,
-             int(!dual), int(dual));
+  const int g = grid_stride_blocks(count);
+  for (int pass = primal ? 0 : 1; pass < (dual ? 2 : 1); ++pass) {
+    scratch.zero();
+    GPP_LAUNCH(rg_claim, g, kThreads, 0, st, t, lo, count, pass, m0, n0, M, s.x, owner, parent.p);
+    GPP_LAUNCH(rg_connect, g, kThreads, 0, st, t, lo, count, pass, m0, n0, M, owner, parent.p);
+    GPP_LAUNCH(rg_roots, g, kThreads, 0, st, count, parent.p, shared_root);
+    GPP_LAUNCH(rg_replay_alone, g, kThreads, 0, st, t, lo, count, pass, s, M, parent.p, shared_root, keys.p, vals.p,
+               counter);
+    const int listed = read_scalar(counter);
+    if (!listed) continue;
+    radix_sort_pairs(keys.p, vals.p, listed, st);
+    GPP_LAUNCH(rg_replay_groups, grid_stride_blocks(listed), kThreads, 0, st, t, lo, listed, keys.p, pass, s, M);
+  }
+}
+
+__global__ void mark_protected(TapeView t, uint8_t* __restrict__ prot, int n) {
+  for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < t.total; g += int64_t(gridDim.x) * blockDim.x) {
+    const RecordAt r(t, g);
+    int a = -1, b = -1;
+    if (r.type == kSingletonColumnSubstitution || r.type == kParallelColumn) a = r.id[0];
+    if (r.type == kDoubletonEquation) { a = r.id[0]; b = r.id[1]; }
+    if (r.type == kInfiniteBoundDualFix) a = r.id[1];
+    if (a >= 0 && a < n) prot[a] = 1;
+    if (b >= 0 && b < n) prot[b] = 1;
+  }
 }
 
 // ---- piecewise-linear primal recoveries ---------------------------------------
@@ -715,53 +823,71 @@ void run_postsolve(const PresolveOutput& out, const double* x_red, const double*
   if (n0) check(cudaMemsetAsync(x, 0, sizeof(double) * n0, st), "clear x");
   if (m0 && y) check(cudaMemsetAsync(y, 0, sizeof(double) * m0, st), "clear y");
   if (n0 && z) check(cudaMemsetAsync(z, 0, sizeof(double) * n0, st), "clear z");
-  DBuf<uint8_t> got(size_t(std::max(n0, 1)), st);
+  // The retrieval flags, then the marks of columns whose z a record set.
+  const size_t columns = size_t(std::max(n0, 1));
+  DBuf<uint8_t> got(2 * columns, st);
   got.zero();
-  if (x_red && r.n) GPP_LAUNCH(scatter, grid_stride_blocks(r.n), kThreads, 0, st, x, x_red, r.cols.p, r.n);
-  if (y && y_red && r.m) GPP_LAUNCH(scatter, grid_stride_blocks(r.m), kThreads, 0, st, y, y_red, r.rows.p, r.m);
-  if (z && z_red && r.n) GPP_LAUNCH(scatter, grid_stride_blocks(r.n), kThreads, 0, st, z, z_red, r.cols.p, r.n);
-  if (r.n) GPP_LAUNCH(mark, grid_stride_blocks(r.n), kThreads, 0, st, got.p, r.cols.p, r.n);
-  for (const auto& f : r.fixed)
-    GPP_LAUNCH(restore_fixed, grid_stride_blocks(f.count), kThreads, 0, st, x, f.idx.p, f.val.p, f.count);
+  uint8_t* prot = got.p + columns;
+  const Sol s{x, y, z, got.p};
+  if (r.n || r.m)
+    GPP_LAUNCH(scatter_solution, grid_stride_blocks(std::max(r.n, r.m)), kThreads, 0, st, s, x_red, y_red, z_red,
+               r.rows.p, r.m, r.cols.p, r.n);
+  // Views of the record's segments, uploaded together: the tape's segments,
+  // the global index of each one's first record, the fixed-value segments.
+  std::vector<SegView> segs;
+  std::vector<int64_t> starts;
+  std::vector<FixedView> fixed;
+  int64_t total = 0, most_fixed = 0;
+  for (const auto& seg : r.segments) {
+    if (!seg.count) continue;
+    segs.push_back(view(seg));
+    starts.push_back(total);
+    total += seg.count;
+  }
+  for (const auto& f : r.fixed) {
+    if (!f.count) continue;
+    fixed.push_back({f.idx.p, f.val.p, f.count});
+    most_fixed = std::max(most_fixed, f.count);
+  }
+  const size_t seg_bytes = sizeof(SegView) * segs.size(), start_bytes = sizeof(int64_t) * starts.size(),
+               fixed_bytes = sizeof(FixedView) * fixed.size();
+  std::vector<unsigned char> packed(seg_bytes + start_bytes + fixed_bytes);
+  DBuf<unsigned char> views(packed.size(), st);
+  if (!packed.empty()) {
+    if (seg_bytes) std::memcpy(packed.data(), segs.data(), seg_bytes);
+    if (start_bytes) std::memcpy(packed.data() + seg_bytes, starts.data(), start_bytes);
+    if (fixed_bytes) std::memcpy(packed.data() + seg_bytes + start_bytes, fixed.data(), fixed_bytes);
+    check(cudaMemcpyAsync(views.p, packed.data(), packed.size(), cudaMemcpyHostToDevice, st), "record views");
+  }
+  const TapeView t{reinterpret_cast<const SegView*>(views.p), reinterpret_cast<const int64_t*>(views.p + seg_bytes),
+                   int(segs.size()), total};
+  if (!fixed.empty())
+    GPP_LAUNCH(restore_fixed, grid_stride_blocks(most_fixed), kThreads, 0, st, x,
+               reinterpret_cast<const FixedView*>(views.p + seg_bytes + start_bytes), int(fixed.size()));
   Model M{};
   if (original) {
     M = Model{original->A.rowPtr, original->AT.rowPtr, original->A.colVal, original->AT.colVal, original->A.nzVal,
               original->AT.nzVal, original->c, original->l, original->u, true};
   }
-  const Sol s{x, y, z, got.p};
-  // Records [lo, hi) of the tape (global indices), newest first.
-  auto replay = [&](int64_t lo, int64_t hi, bool dual) {
-    if (lo >= hi) return;
-    if (r.records < kParallelMinRecords) {
-      int64_t end = r.records;
-      for (auto it = r.segments.rbegin(); it != r.segments.rend(); ++it) {
-        const int64_t begin = end - it->count;
-        const int64_t a = std::max(lo, begin), b = std::min(hi, end);
-        if (a < b) GPP_LAUNCH(replay_serial, 1, 1, 0, st, view(*it), s, M, !dual, dual, a - begin, b - begin);
-        end = begin;
-      }
-    } else {
-      replay_parallel(r.segments, m0, n0, s, M, dual, st, lo, hi);
-    }
-  };
   // Primal pass split at the piecewise-linear checkpoints, newest first: the
   // records after a checkpoint, then its recovery (postsolve_gpu,
   // gpu_postsolve.cu:637-663); the dual pass over the whole tape.
   int64_t range_end = r.records;
   for (auto it = r.timeline.rbegin(); it != r.timeline.rend(); ++it) {
-    replay(it->tape_position, range_end, false);
+    replay_range(t, m0, n0, s, M, true, false, st, it->tape_position, range_end);
     if (it->kind == 0) restore_absolute_value(x, r.absval[size_t(it->payload)], lower, st);
     else restore_variable_pair(x, r.varpair[size_t(it->payload)], st);
     range_end = it->tape_position;
   }
-  replay(0, range_end, false);
-  replay(0, r.records, true);
+  if (r.timeline.empty()) {
+    replay_range(t, m0, n0, s, M, true, true, st, 0, r.records);
+  } else {
+    replay_range(t, m0, n0, s, M, true, false, st, 0, range_end);
+    replay_range(t, m0, n0, s, M, false, true, st, 0, r.records);
+  }
   if (original && y && z && n0) {
-    DBuf<uint8_t> prot(size_t(n0), st);
-    prot.zero();
-    for (const auto& seg : r.segments)
-      GPP_LAUNCH(mark_protected, grid_stride_blocks(seg.count), kThreads, 0, st, view(seg), prot.p, n0);
-    GPP_LAUNCH(project_duals, grid_stride_blocks(n0), kThreads, 0, st, n0, prot.p, M, x, y, z);
+    if (total) GPP_LAUNCH(mark_protected, grid_stride_blocks(total), kThreads, 0, st, t, prot, n0);
+    GPP_LAUNCH(project_duals, grid_stride_blocks(n0), kThreads, 0, st, n0, prot, M, x, y, z);
   }
   ctx().sync("postsolve");
 }

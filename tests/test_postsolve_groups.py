@@ -28,8 +28,9 @@ def point(kind, l, u, rng):
 
 @pytest.mark.parametrize("kind", ["lower", "upper", "mixed", "odd"])
 @pytest.mark.parametrize("workload,records", [("slack:400x1000", (1, 2048)), ("random:1500x3700", (1, 2048)),
-                                              ("slack:2000x5000", (2049, 1 << 30)), ("qap:4", (1, 2048)),
-                                              ("qap:8", (2049, 1 << 30)), ("random:20000x50000", (2049, 1 << 30))])
+                                              ("slack:2000x5000", (1, 2048)), ("slack:2100x5200", (2049, 1 << 30)),
+                                              ("qap:4", (1, 2048)), ("qap:8", (2049, 1 << 30)),
+                                              ("random:20000x50000", (2049, 1 << 30))])
 def test_groups_replay_as_the_serial_tape(workload, records, kind):
     import torch
     lp = lpgen.workload(workload, seed=3)

@@ -41,23 +41,30 @@ Context::Context() {
         "cudaMallocHost status");
   check(cudaMallocHost(reinterpret_cast<void**>(&host_scalar), 16), "cudaMallocHost scalar");
   check(cudaMallocHost(reinterpret_cast<void**>(&host_later), sizeof(unsigned long long)), "cudaMallocHost later");
+  check(cudaMallocHost(reinterpret_cast<void**>(&host_error), sizeof(int32_t)), "cudaMallocHost error");
+  *host_error = 0;
 }
 
 void Context::sync(const char* label) {
   ++sync_counter();
   if (!profiling()) {
     check(cudaStreamSynchronize(stream), label);
-    return;
+  } else {
+    const auto t0 = std::chrono::steady_clock::now();
+    check(cudaStreamSynchronize(stream), label);
+    profile_sync(label, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
   }
-  const auto t0 = std::chrono::steady_clock::now();
-  check(cudaStreamSynchronize(stream), label);
-  profile_sync(label, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+  if (*static_cast<volatile int32_t*>(host_error)) {
+    *host_error = 0;
+    throw CudaError(std::string(label) + ": a block's bounded wait for its predecessors ran out");
+  }
 }
 
 Context::~Context() {
   if (host_status) cudaFreeHost(host_status);
   if (host_scalar) cudaFreeHost(host_scalar);
   if (host_later) cudaFreeHost(host_later);
+  if (host_error) cudaFreeHost(host_error);
   if (side) cudaStreamDestroy(side);
   if (stream) cudaStreamDestroy(stream);
 }

@@ -223,6 +223,9 @@ struct Context {
   int32_t* host_status = nullptr;   // pinned, kStatusWords ints
   unsigned char* host_scalar = nullptr;   // pinned, 16 bytes for scalar readbacks
   unsigned long long* host_later = nullptr;   // pinned, one word read after a later wait
+  // Page-locked word that a kernel sets when a bounded wait on another block
+  // ran out; sync() turns it into an error.
+  int32_t* host_error = nullptr;
   cudaStream_t side = nullptr;
   // Scratch blocks this context freed on its own stream, by size class,
   // ready to be handed out again without a driver call (pool_alloc/free).

@@ -593,7 +593,7 @@ void transpose_csr_into(const DevCsr& M, const DevCsr& t, cudaStream_t s) {
   } else {
     DBuf<uint64_t> keys(size_t(M.nnz), s);
     GPP_LAUNCH(transpose_keys, g, kThreads, 0, s, M.nnz, M.idx, keys.p, pos.p);
-    radix_sort_pairs(keys.p, pos.p, M.nnz, s);
+    radix_sort_pairs(keys.p, pos.p, M.nnz, s, bits_up_to(int64_t(M.cols) - 1));
   }
   GPP_LAUNCH(row_of_entry, std::max(1, std::min((M.rows + 7) / 8, kNumSMs * 16)), kThreads, 0, s, M.rows, M.ptr,
              row.p);

@@ -136,7 +136,7 @@ struct Side {
   void update(const double* value, double tol, bool write_sig, uint64_t seed, cudaStream_t s) {
     const int g = grid_stride_blocks(n);
     GPP_LAUNCH(fd_pack, g, kThreads, 0, s, n, ids.p, value, keys.p, perm.p);
-    radix_sort_pairs(keys.p, perm.p, n, s);
+    radix_sort_pairs(keys.p, perm.p, n, s, (bits_up_to(n) << 32) | 0xffffffffu);
     GPP_LAUNCH(fd_starts, g, kThreads, 0, s, n, keys.p, tol, start.p);
     exclusive_scan_i32(start.p, excl.p, n, s);
     GPP_LAUNCH(fd_write, g, kThreads, 0, s, n, perm.p, start.p, excl.p, int(write_sig), seed, ids.p, sig.p);
@@ -347,7 +347,7 @@ void members_of(const Side& side, const double* value, const double* lo, const d
   exclusive_scan_i32(mb.counts.p, mb.offsets.p, k, s);
   DBuf<uint64_t> keys(size_t(n), s);
   GPP_LAUNCH(fd_member_keys, g, kThreads, 0, s, n, side.ids.p, keys.p, mb.list.p);
-  radix_sort_pairs(keys.p, mb.list.p, n, s);
+  radix_sort_pairs(keys.p, mb.list.p, n, s, bits_up_to(int64_t(k) - 1) << 32);   // members already ascend
   GPP_LAUNCH(fd_nonconstant, g, kThreads, 0, s, n, mb.list.p, side.ids.p, mb.offsets.p, value, lo, hi, mb.flags.p);
 }
 
@@ -387,7 +387,7 @@ void run_folding(const gpp_lp& lp, double tolerance, FoldingResult& out) {
     GPP_LAUNCH(fd_entries, std::max(1, std::min((lp.A.rows + 7) / 8, kNumSMs * 16)), kThreads, 0, s, lp.A.rows,
                lp.A.rowPtr, lp.A.colVal, lp.A.nzVal, rows.ids.p, cols.ids.p, rm.counts.p, nc, keys.p, order.p,
                weighted.p);
-    radix_sort_pairs(keys.p, order.p, nnz, s);
+    radix_sort_pairs(keys.p, order.p, nnz, s, bits_up_to(int64_t(mr) * nc - 1));
     const int g = grid_stride_blocks(nnz);
     GPP_LAUNCH(fd_heads, g, kThreads, 0, s, nnz, keys.p, head.p);
     exclusive_scan_i32(head.p, hpos.p, nnz, s);

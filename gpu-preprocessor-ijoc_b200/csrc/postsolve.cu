@@ -719,7 +719,7 @@ void replay_range(const TapeView& t, int m0, int n0, const Sol& s, const Model& 
                counter);
     const int listed = read_scalar(counter);
     if (!listed) continue;
-    radix_sort_pairs(keys.p, vals.p, listed, st);
+    radix_sort_pairs(keys.p, vals.p, listed, st, (bits_up_to(count - 1) << 32) | bits_up_to(count - 1));
     GPP_LAUNCH(rg_replay_groups, grid_stride_blocks(listed), kThreads, 0, st, t, lo, listed, keys.p, pass, s, M);
   }
 }

@@ -891,7 +891,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     if (total) {
       GPP_LAUNCH(dt_delta_fill, warp_grid(sel), kThreads, 0, s, sel, rows.p, keep_c.p, elim_c.p, kind.p, alpha.p,
                  AT.ptr, AT.idx, AT.val, plan.keep_row.p, zt, dpos.p, keys.p, order.p, raw.p);
-      radix_sort_pairs(keys.p, order.p, total, s);
+      radix_sort_pairs(keys.p, order.p, total, s, (bits_up_to(m - 1) << 32) | bits_up_to(n - 1));
       GPP_LAUNCH(dt_delta_rows, grid_stride_blocks(total), kThreads, 0, s, int64_t(total), keys.p, order.p, raw.p,
                  dcol.p, dv.p, row_cnt.p);
     }

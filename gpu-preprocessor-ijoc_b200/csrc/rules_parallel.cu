@@ -663,7 +663,7 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
              plan.keep_row.p);
   if (p.record_postsolve_tape) {
     // Records ordered by (merge step, deleted row) (rule_parallel_rows.cu:79-84).
-    radix_sort_pairs(dkeys.p, dids.p, deleted, s);
+    radix_sort_pairs(dkeys.p, dids.p, deleted, s, bits_up_to(deleted) << 32);   // rows already ascend
     PostsolveSegment seg = make_segment(deleted, 2 * int64_t(deleted), 5 * int64_t(deleted));
     GPP_LAUNCH(pack_parallel_records, grid_stride_blocks(deleted + 1), kThreads, 0, s, int64_t(deleted), dids.p,
                merge_to.p, rec.p, 4, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p);

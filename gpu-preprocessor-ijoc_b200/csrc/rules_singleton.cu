@@ -675,7 +675,7 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
     DBuf<uint64_t> keys(size_t(nwin), s);
     DBuf<int32_t> sorted(size_t(nwin), s);
     GPP_LAUNCH(sc_winner_keys, grid_stride_blocks(nwin), kThreads, 0, s, winners.p, nwin, kind.p, keys.p, sorted.p);
-    radix_sort_pairs(keys.p, sorted.p, nwin, s);
+    radix_sort_pairs(keys.p, sorted.p, nwin, s, (uint64_t(1) << 32) | bits_up_to(m - 1));
     const int nshift = nwin - nelim;
     if (nelim) {
       DBuf<int32_t> sel(size_t(nelim) + 1, s), rec(size_t(nelim) + 1, s);

@@ -3,13 +3,16 @@
 // Replaces the reference's thrust::sort of (hash, id) tuples
 // (rule_parallel_rows.cu:742-770, rule_parallel_columns.cu:958-975): with the
 // input in ascending id order, a stable sort by key yields (key, id) order.
-// Each 8-bit pass is three launches: per-tile digit histograms, one scan of
-// the digit-major count table, and a stable scatter in which every warp ranks
-// its keys with __match_any_sync and warps are ordered through shared
-// counters.  Passes whose digit is constant across all keys are skipped
-// (decided from one histogram readback per sort).
+//
+// The caller names the key bits that can differ; every window of eight such
+// bits is one pass.  Inputs of at most kBlockSortMax pairs are sorted by one
+// block in shared memory; larger ones take one histogram launch for all
+// passes and one launch per pass, which reads and writes every pair once: a
+// tile ranks its keys, publishes its digit counts and finds its output
+// offsets by a decoupled look-back over its predecessors.  A digit that turns
+// out constant makes its pass return at once (decided on the device, so the
+// sort waits for nothing).
 #include "sort.hpp"
-#include "sort_kernels.cuh"
 
 #include <mutex>
 #include <vector>
@@ -18,99 +21,427 @@ namespace gpp {
 
 namespace {
 
-// Small inputs (most sorts of a presolve round: the winners of one rule,
-// the hashes of the few changed rows) take one block instead of up to eight
-// three-launch passes and a readback: a bitonic network over (key, original
-// position) in shared memory.  The order on (key, position) is total, so the
-// result is exactly the stable sort's.
-constexpr int kBlockSortMax = 4096;
-constexpr int kBlockSortThreads = 1024;
+constexpr int kDigits = 256;
+constexpr int kMaxPasses = 8;   // windows are disjoint and eight bits wide, of a 64-bit key
 
-__global__ void __launch_bounds__(kBlockSortThreads) block_sort_pairs(uint64_t* keys, int32_t* vals, int n, int size) {
-  extern __shared__ unsigned char block_sort_smem[];
-  auto* k = reinterpret_cast<uint64_t*>(block_sort_smem);
-  auto* pos = reinterpret_cast<int32_t*>(k + size);
-  auto* v = pos + size;
-  for (int i = threadIdx.x; i < size; i += blockDim.x) {
-    const bool in = i < n;
-    k[i] = in ? keys[i] : ~0ull;
-    pos[i] = in ? i : 0x7fffffff;
-    v[i] = in ? vals[i] : 0;
+struct SortPasses {
+  int count = 0;
+  int shift[kMaxPasses] = {};
+};
+SortPasses passes_of(uint64_t varying) {
+  SortPasses p;
+  while (varying) {
+    const int shift = std::min(56, __builtin_ctzll(varying));
+    p.shift[p.count++] = shift;
+    varying &= ~(0xffull << shift);
+  }
+  return p;
+}
+
+__device__ __forceinline__ int digit_of(uint64_t key, int shift) { return int((key >> shift) & 0xff); }
+
+// Exclusive scan over the first 256 threads of a block, one digit each; all
+// threads of the block must call it.  `warp_sums` holds 8 ints.
+__device__ __forceinline__ int scan_digits(int v, int* warp_sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int peer = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += peer;
+  }
+  if (warp < 8 && lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  int before = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) before += w < warp ? warp_sums[w] : 0;
+  __syncthreads();
+  return before + incl - v;
+}
+
+// Rank of a warp's key among the warp's earlier keys of the same digit:
+// `counts` is the warp's own row of 256 running counts, so no other warp is
+// waited for.  `d` is 256 for a position past the end.
+__device__ __forceinline__ int warp_rank(int* counts, int d) {
+  const int lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(0xffffffffu, d);
+  const int leader = __ffs(peers) - 1;
+  int before = 0;
+  if (lane == leader && d < kDigits) {
+    before = counts[d];
+    counts[d] = before + __popc(peers);
+  }
+  __syncwarp();
+  before = __shfl_sync(0xffffffffu, before, leader);
+  return before + __popc(peers & ((1u << lane) - 1u));
+}
+
+// ---- one block --------------------------------------------------------------
+//
+// Most sorts of a presolve round are small (the winners of one rule, the
+// hashes of the rows that may be shared).  One block holds the keys in shared
+// memory and moves 16-bit positions through the passes, so a pass is a rank,
+// two barriers and a scatter in shared memory.  Only the windows that vary are
+// sorted by.  Against the bitonic network over (key, position) this replaced
+// (78 barriered rounds at 4,096 pairs, 34 us on average over a presolve's
+// sorts) it takes 8-12 us for the two to four windows those sorts have.
+constexpr int kBlockSortMax = 8192;
+constexpr int kBlockSortThreads = 1024;
+constexpr int kBlockSortWarps = kBlockSortThreads / 32;
+constexpr int kBlockSortItems = kBlockSortMax / kBlockSortThreads;
+constexpr size_t kBlockSortCounts = sizeof(int) * kBlockSortWarps * kDigits;
+
+size_t block_sort_smem(int n) {
+  const size_t padded = size_t(n + 7) / 8 * 8;
+  return kBlockSortCounts + padded * (sizeof(uint64_t) + 2 * sizeof(uint16_t));
+}
+
+__global__ void __launch_bounds__(kBlockSortThreads)
+block_sort_pairs(uint64_t* keys, int32_t* vals, int n, uint64_t may_vary) {
+  extern __shared__ __align__(16) unsigned char block_sort_mem[];
+  __shared__ int digit_start[kDigits];
+  __shared__ int warp_sums[8];
+  __shared__ unsigned long long varies;
+  const int padded = (n + 7) / 8 * 8;
+  int* counts = reinterpret_cast<int*>(block_sort_mem);
+  auto* k = reinterpret_cast<uint64_t*>(block_sort_mem + kBlockSortCounts);
+  auto* from = reinterpret_cast<uint16_t*>(k + padded);
+  auto* to = from + padded;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int items = (n + kBlockSortThreads - 1) / kBlockSortThreads;
+  if (threadIdx.x == 0) varies = 0;
+  __syncthreads();
+  const uint64_t first = keys[0];
+  uint64_t acc = 0;
+  for (int i = threadIdx.x; i < n; i += kBlockSortThreads) {
+    const uint64_t key = keys[i];
+    k[i] = key;
+    from[i] = uint16_t(i);
+    acc |= key ^ first;
+  }
+  const uint32_t lo = __reduce_or_sync(0xffffffffu, uint32_t(acc));
+  const uint32_t hi = __reduce_or_sync(0xffffffffu, uint32_t(acc >> 32));
+  if (lane == 0 && (lo | hi)) atomicOr(&varies, (uint64_t(hi) << 32) | lo);
+  __syncthreads();
+  uint64_t left = varies & may_vary;
+  int* own = counts + warp * kDigits;
+  const int base = warp * 32 * items + lane;   // a warp owns consecutive positions
+  while (left) {
+    const int shift = min(56, __ffsll((long long)left) - 1);
+    left &= ~(0xffull << shift);
+    for (int d = lane; d < kDigits; d += 32) own[d] = 0;
+    __syncwarp();
+    int rank[kBlockSortItems], at[kBlockSortItems];
+#pragma unroll
+    for (int q = 0; q < kBlockSortItems; ++q) {
+      if (q >= items) break;
+      const int i = base + q * 32;
+      at[q] = i < n ? from[i] : 0;
+      rank[q] = warp_rank(own, i < n ? digit_of(k[at[q]], shift) : kDigits);
+    }
+    __syncthreads();
+    // Digit d's count per warp becomes its start within the digit.
+    int total = 0;
+    if (threadIdx.x < kDigits)
+      for (int w = 0; w < kBlockSortWarps; ++w) {
+        const int c = counts[w * kDigits + threadIdx.x];
+        counts[w * kDigits + threadIdx.x] = total;
+        total += c;
+      }
+    const int start = scan_digits(total, warp_sums);
+    if (threadIdx.x < kDigits) digit_start[threadIdx.x] = start;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kBlockSortItems; ++q) {
+      if (q >= items) break;
+      if (base + q * 32 >= n) continue;
+      const int d = digit_of(k[at[q]], shift);
+      to[digit_start[d] + own[d] + rank[q]] = uint16_t(at[q]);
+    }
+    __syncthreads();
+    auto* t = from;
+    from = to;
+    to = t;
+  }
+  int32_t v[kBlockSortItems];
+#pragma unroll
+  for (int q = 0; q < kBlockSortItems; ++q) {
+    const int i = q * kBlockSortThreads + int(threadIdx.x);
+    v[q] = i < n ? vals[from[i]] : 0;
   }
   __syncthreads();
-  for (int width = 2; width <= size; width <<= 1) {
-    for (int stride = width >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < size; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & width) == 0;
-          const bool greater = k[i] > k[j] || (k[i] == k[j] && pos[i] > pos[j]);
-          if (greater == up) {
-            const uint64_t tk = k[i]; k[i] = k[j]; k[j] = tk;
-            const int32_t tp = pos[i]; pos[i] = pos[j]; pos[j] = tp;
-            const int32_t tv = v[i]; v[i] = v[j]; v[j] = tv;
-          }
-        }
-      }
-      __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kBlockSortItems; ++q) {
+    const int i = q * kBlockSortThreads + int(threadIdx.x);
+    if (i < n) {
+      keys[i] = k[from[i]];
+      vals[i] = v[q];
     }
   }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    keys[i] = k[i];
-    vals[i] = v[i];
+}
+
+// ---- tiles ------------------------------------------------------------------
+
+// What the histogram launch leaves for the passes: per pass the digit counts,
+// then (written by its last block) the digits' first output positions, whether
+// the digit is constant, and which buffer holds the pairs before the pass.
+struct SortPlan {
+  unsigned long long counts[kMaxPasses][kDigits];
+  long long start[kMaxPasses][kDigits];
+  int constant[kMaxPasses];
+  int source[kMaxPasses + 1];   // 0 the caller's arrays, 1 the scratch copy; the last entry after all passes
+  unsigned int tickets[kMaxPasses];
+  unsigned int blocks_done;
+};
+
+__global__ void __launch_bounds__(kThreads)
+sort_histogram(const uint64_t* __restrict__ keys, int64_t n, SortPasses passes, SortPlan* plan) {
+  __shared__ int h[kMaxPasses][kDigits];
+  __shared__ bool last;
+  __shared__ int warp_sums[8];
+  for (int p = 0; p < passes.count; ++p) h[p][threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t stride = int64_t(gridDim.x) * kThreads;
+  const int64_t top = (n + stride - 1) / stride * stride;
+  for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < top; i += stride) {
+    const bool in = i < n;
+    const uint64_t key = in ? keys[i] : 0;
+    for (int p = 0; p < passes.count; ++p) {
+      const int d = in ? digit_of(key, passes.shift[p]) : kDigits;
+      // A digit that all lanes share (high digits of small keys) is added once.
+      int same;
+      __match_all_sync(0xffffffffu, d, &same);
+      if (same) {
+        if ((threadIdx.x & 31) == 0 && d < kDigits) atomicAdd(&h[p][d], 32);
+      } else if (in) {
+        atomicAdd(&h[p][d], 1);
+      }
+    }
   }
+  __syncthreads();
+  for (int p = 0; p < passes.count; ++p) {
+    const int c = h[p][threadIdx.x];
+    if (c) atomicAdd(&plan->counts[p][threadIdx.x], (unsigned long long)c);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&plan->blocks_done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  int source = 0;
+  for (int p = 0; p < passes.count; ++p) {
+    const unsigned long long c = __ldcg(&plan->counts[p][threadIdx.x]);
+    // 64-bit scan of the counts as two 31-bit halves (their sums stay below 2^31 x 256).
+    const int low = scan_digits(int(c & 0x3fffff), warp_sums), high = scan_digits(int(c >> 22), warp_sums);
+    plan->start[p][threadIdx.x] = (long long)low + ((long long)high << 22);
+    const int constant = __syncthreads_or(c == (unsigned long long)n);
+    if (threadIdx.x == 0) {
+      plan->constant[p] = constant;
+      plan->source[p] = source;
+    }
+    if (!constant) source ^= 1;
+  }
+  if (threadIdx.x == 0) plan->source[passes.count] = source;
+}
+
+// A tile's published word per digit: two flag bits (0 nothing yet, 1 the
+// tile's own count, 2 the count of all tiles up to it) over the count.
+template <class Word>
+struct TileWord {
+  static constexpr int kShift = sizeof(Word) * 8 - 2;
+  static constexpr Word kValue = (Word(1) << kShift) - 1;
+  static constexpr Word kOwn = Word(1) << kShift, kAll = Word(2) << kShift;
+};
+__device__ __forceinline__ uint32_t ld_word(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_word(uint32_t* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_word(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// One pass over one tile.  Tiles are taken in ticket order, so every tile that
+// a look-back waits for is running; a wait still gives up after kPolls polls,
+// sets the error word that the host checks at its next wait, and goes on.
+// Bound by the memory traffic (24 bytes a pair) and the ranking; tiles of
+// kItems x 256 pairs: sixteen items keep the look-back short against the
+// tile's work on large inputs, eight spread mid-size inputs over the SMs.
+// 2,000,003 random pairs: 506 us before (four launches a pass: histogram, two
+// of scan, scatter), measured figures beside the dispatch below.
+constexpr int kPolls = 1 << 22;
+
+template <int kItems>
+struct SortTile {
+  static constexpr int kPairs = kThreads * kItems;
+  static constexpr size_t kBytes = size_t(kPairs) * (sizeof(uint64_t) + sizeof(int32_t));
+};
+
+template <int kItems, class Word>
+__global__ void __launch_bounds__(kThreads)
+sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int64_t n, int pass, int shift,
+          SortPlan* plan, Word* words, int32_t* error) {
+  constexpr int kPairs = SortTile<kItems>::kPairs;
+  using W = TileWord<Word>;
+  extern __shared__ __align__(16) unsigned char sort_tile_mem[];
+  __shared__ int counts[8][kDigits];
+  __shared__ int local_start[kDigits];
+  __shared__ long long out_base[kDigits];
+  __shared__ int warp_sums[8];
+  __shared__ unsigned int ticket;
+  if (plan->constant[pass]) return;
+  auto* tile_keys = reinterpret_cast<uint64_t*>(sort_tile_mem);
+  auto* tile_vals = reinterpret_cast<int32_t*>(tile_keys + kPairs);
+  const bool swapped = plan->source[pass] != 0;
+  const uint64_t* in_keys = swapped ? keys1 : keys0;
+  const int32_t* in_vals = swapped ? vals1 : vals0;
+  uint64_t* out_keys = swapped ? keys0 : keys1;
+  int32_t* out_vals = swapped ? vals0 : vals1;
+  if (threadIdx.x == 0) ticket = atomicAdd(&plan->tickets[pass], 1u);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int d = lane; d < kDigits; d += 32) counts[warp][d] = 0;
+  __syncthreads();
+  const int64_t tile = ticket;
+  const int64_t first = tile * kPairs;
+  const int tile_n = int(min(int64_t(kPairs), n - first));
+  uint64_t key[kItems];
+  int32_t val[kItems];
+  int rank[kItems];
+  const int p0 = warp * 32 * kItems + lane;
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    const int i = p0 + q * 32;
+    key[q] = i < tile_n ? in_keys[first + i] : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    const int i = p0 + q * 32;
+    val[q] = i < tile_n ? in_vals[first + i] : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < kItems; ++q)
+    rank[q] = warp_rank(counts[warp], p0 + q * 32 < tile_n ? digit_of(key[q], shift) : kDigits);
+  __syncthreads();
+  {
+    const int d = threadIdx.x;   // one digit per thread
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const int c = counts[w][d];
+      counts[w][d] = total;
+      total += c;
+    }
+    Word* own = words + size_t(tile) * kDigits + d;
+    st_word(own, (tile == 0 ? W::kAll : W::kOwn) | Word(total));
+    const int start = scan_digits(total, warp_sums);
+    local_start[d] = start;
+    Word before = 0;
+    for (int64_t t = tile - 1; t >= 0; --t) {
+      const Word* at = words + size_t(t) * kDigits + d;
+      Word w = ld_word(at);
+      for (int polls = 1; (w >> W::kShift) == 0; ++polls) {
+        if (polls == kPolls) {
+          *reinterpret_cast<volatile int32_t*>(error) = 1;
+          w = W::kAll;
+          break;
+        }
+        w = ld_word(at);
+      }
+      before += w & W::kValue;
+      if ((w >> W::kShift) == 2) break;
+    }
+    if (tile > 0) st_word(own, W::kAll | (before + Word(total)));
+    out_base[d] = plan->start[pass][d] + (long long)before - start;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kItems; ++q) {
+    if (p0 + q * 32 >= tile_n) continue;
+    const int d = digit_of(key[q], shift);
+    const int slot = local_start[d] + counts[warp][d] + rank[q];
+    tile_keys[slot] = key[q];
+    tile_vals[slot] = val[q];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < tile_n; q += kThreads) {
+    const uint64_t k = tile_keys[q];
+    const int64_t dst = out_base[digit_of(k, shift)] + q;
+    out_keys[dst] = k;
+    out_vals[dst] = tile_vals[q];
+  }
+}
+
+// The pairs back into the caller's arrays when the passes left them in the
+// scratch copy.
+__global__ void sort_copy_back(int64_t n, int passes, const SortPlan* __restrict__ plan, uint64_t* __restrict__ keys,
+                               int32_t* __restrict__ vals, const uint64_t* __restrict__ from_keys,
+                               const int32_t* __restrict__ from_vals) {
+  if (plan->source[passes] == 0) return;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    keys[i] = from_keys[i];
+    vals[i] = from_vals[i];
+  }
+}
+
+// The opt-in shared-memory limits are per-device function attributes: set
+// once per device, with that device current.
+void allow_shared_memory() {
+  static std::mutex mu;
+  static std::vector<bool> configured;
+  int dev = 0;
+  check(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  if (size_t(dev) >= configured.size()) configured.resize(size_t(dev) + 1, false);
+  if (configured[size_t(dev)]) return;
+  const auto set = [](auto kernel, size_t bytes) {
+    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)), "sort smem");
+  };
+  set(block_sort_pairs, block_sort_smem(kBlockSortMax));
+  set(sort_pass<8, uint32_t>, SortTile<8>::kBytes);
+  set(sort_pass<16, uint32_t>, SortTile<16>::kBytes);
+  set(sort_pass<16, unsigned long long>, SortTile<16>::kBytes);
+  configured[size_t(dev)] = true;
+}
+
+template <int kItems, class Word>
+void sort_tiles(uint64_t* keys, int32_t* vals, int64_t n, const SortPasses& passes, cudaStream_t s) {
+  const int64_t tiles = (n + SortTile<kItems>::kPairs - 1) / SortTile<kItems>::kPairs;
+  const size_t words = size_t(tiles) * kDigits;
+  DBuf<uint64_t> k2(size_t(n), s);
+  DBuf<int32_t> v2(size_t(n), s);
+  DBuf<unsigned char> scratch(sizeof(SortPlan) + sizeof(Word) * words * size_t(passes.count), s);
+  scratch.zero();
+  auto* plan = reinterpret_cast<SortPlan*>(scratch.p);
+  auto* tile_words = reinterpret_cast<Word*>(scratch.p + sizeof(SortPlan));
+  GPP_LAUNCH_BYTES(sort_histogram, 8.0 * n, grid_stride_blocks(n, kThreads, 4), kThreads, 0, s, keys, n, passes, plan);
+  for (int p = 0; p < passes.count; ++p)
+    GPP_LAUNCH_BYTES((sort_pass<kItems, Word>), 24.0 * n, int(tiles), kThreads, SortTile<kItems>::kBytes, s, keys, vals,
+                     k2.p, v2.p, n, p, passes.shift[p], plan, tile_words + words * size_t(p), ctx().host_error);
+  GPP_LAUNCH(sort_copy_back, grid_stride_blocks(n), kThreads, 0, s, n, passes.count, plan, keys, vals, k2.p, v2.p);
 }
 
 }  // namespace
 
-void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s) {
-  if (n <= 1) return;
+void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, uint64_t may_vary) {
+  if (n <= 1 || may_vary == 0) return;
+  allow_shared_memory();
   if (n <= kBlockSortMax) {
-    int size = 2;
-    while (size < n) size <<= 1;
-    const size_t smem = size_t(size) * (sizeof(uint64_t) + 2 * sizeof(int32_t));
-    // The shared-memory limit is a per-device function attribute: set it once
-    // per device, with that device current.
-    static std::mutex mu;
-    static std::vector<bool> configured;
-    int dev = 0;
-    check(cudaGetDevice(&dev), "cudaGetDevice");
-    {
-      std::lock_guard<std::mutex> lock(mu);
-      if (size_t(dev) >= configured.size()) configured.resize(size_t(dev) + 1, false);
-      if (!configured[size_t(dev)]) {
-        check(cudaFuncSetAttribute(block_sort_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(kBlockSortMax * (sizeof(uint64_t) + 2 * sizeof(int32_t)))),
-              "block_sort_pairs smem");
-        configured[size_t(dev)] = true;
-      }
-    }
-    GPP_LAUNCH(block_sort_pairs, 1, kBlockSortThreads, smem, s, keys, vals, int(n), size);
+    GPP_LAUNCH(block_sort_pairs, 1, kBlockSortThreads, block_sort_smem(int(n)), s, keys, vals, int(n), may_vary);
     return;
   }
-  const int64_t tiles = (n + kTile - 1) / kTile;
-  DBuf<unsigned long long> varies(1, s);
-  varies.zero();
-  GPP_LAUNCH(digit_variation, grid_stride_blocks(n), kThreads, 0, s, keys, n, varies.p);
-  const uint64_t variation = read_scalar(varies.p);
-  DBuf<uint64_t> k2(size_t(n), s);
-  DBuf<int32_t> v2(size_t(n), s), counts(size_t(256 * tiles) + 1, s);
-  uint64_t* ka = keys;
-  int32_t* va = vals;
-  uint64_t* kb = k2.p;
-  int32_t* vb = v2.p;
-  for (int pass = 0; pass < 8; ++pass) {
-    if (((variation >> (8 * pass)) & 0xffu) == 0) continue;  // one digit for every key: the identity
-    GPP_LAUNCH(digit_histogram, int(tiles), kThreads, 0, s, ka, n, 8 * pass, counts.p, tiles);
-    exclusive_scan_i32(counts.p, counts.p, 256 * tiles, s);
-    GPP_LAUNCH(digit_scatter, int(tiles), kThreads, 0, s, ka, va, n, 8 * pass, counts.p, tiles, kb, vb);
-    std::swap(ka, kb);
-    std::swap(va, vb);
-  }
-  if (ka != keys) {
-    check(cudaMemcpyAsync(keys, ka, sizeof(uint64_t) * size_t(n), cudaMemcpyDeviceToDevice, s), "sort copy keys");
-    check(cudaMemcpyAsync(vals, va, sizeof(int32_t) * size_t(n), cudaMemcpyDeviceToDevice, s), "sort copy vals");
-  }
+  const SortPasses passes = passes_of(may_vary);
+  if (n < (int64_t(1) << 20)) sort_tiles<8, uint32_t>(keys, vals, n, passes, s);
+  else if (n < (int64_t(1) << 30)) sort_tiles<16, uint32_t>(keys, vals, n, passes, s);
+  else sort_tiles<16, unsigned long long>(keys, vals, n, passes, s);   // counts past 30 bits
 }
 
 }  // namespace gpp

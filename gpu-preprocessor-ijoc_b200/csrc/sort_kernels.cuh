@@ -1,6 +1,5 @@
-// Kernels of the stable LSD radix sort of (uint64 key, int32 value) pairs,
-// shared by the pooled sort (sort.cu) and the fixed-scratch sort
-// (sort_static.cu).  Each 8-bit pass is a per-tile digit histogram, an
+// Kernels of the fixed-scratch stable LSD radix sort of (uint64 key, int32
+// value) pairs (sort_static.cu).  Each 8-bit pass is a per-tile digit histogram, an
 // exclusive scan of the digit-major count table and a stable scatter in which
 // every warp ranks its keys with __match_any_sync and warps are ordered
 // through shared counters.
@@ -27,20 +26,6 @@ __global__ void digit_histogram(const uint64_t* __restrict__ keys, int64_t n, in
   }
   __syncthreads();
   counts[int64_t(threadIdx.x) * tiles + blockIdx.x] = h[threadIdx.x];
-}
-
-// Which digit positions vary (for pass skipping): the OR over all keys of
-// key ^ keys[0].  A byte of it is zero exactly when every key has the same
-// digit there, and that pass is the identity.  One register OR per thread,
-// a warp reduction, one atomic per warp per half.
-__global__ void digit_variation(const uint64_t* __restrict__ keys, int64_t n, unsigned long long* __restrict__ out) {
-  const uint64_t first = keys[0];
-  uint64_t acc = 0;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    acc |= keys[i] ^ first;
-  const uint32_t lo = __reduce_or_sync(0xffffffffu, uint32_t(acc));
-  const uint32_t hi = __reduce_or_sync(0xffffffffu, uint32_t(acc >> 32));
-  if ((threadIdx.x & 31) == 0 && (lo | hi)) atomicOr(out, (uint64_t(hi) << 32) | lo);
 }
 
 // Stable scatter of one tile: the tile's keys are first ranked into a

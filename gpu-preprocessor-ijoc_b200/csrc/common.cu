@@ -1,5 +1,5 @@
 // Engine context, status block, scans and the canonical deterministic sum.
-#include "common.cuh"
+#include "scan.cuh"
 
 #include <atomic>
 #include <cstdlib>
@@ -201,140 +201,29 @@ const int32_t* Status::read(int words, const char* where) {
   return c.host_status;
 }
 
+LookbackSpace::LookbackSpace(size_t count, cudaStream_t s) {
+  auto& c = ctx();
+  const size_t need = count + 1;   // the counters take the first word
+  unsigned long long* base;
+  if (s == c.stream) {
+    if (c.lookback_words < need) {
+      const size_t grown = std::max({need, 2 * c.lookback_words, size_t(4096)});
+      unsigned long long* p = dalloc<unsigned long long>(grown);
+      dfree(std::exchange(c.lookback, p));
+      c.lookback_words = grown;
+      check(cudaMemsetAsync(p, 0, sizeof(unsigned long long) * grown, s), "look-back words");
+    }
+    base = c.lookback;
+  } else {
+    own.alloc(need, s);
+    own.zero();
+    base = own.p;
+  }
+  counters = reinterpret_cast<unsigned int*>(base);
+  words = base + 1;
+}
+
 namespace {
-constexpr int kScanTile = 2048;  // 256 threads x 8 consecutive items
-constexpr int kScanWarps = kThreads / 32;
-
-// Block-wide sum of one value per thread (integers: any order); every
-// thread gets the result.  Contains __syncthreads.
-template <class T>
-__device__ __forceinline__ T block_total(T v, T* warp_sums) {
-#pragma unroll
-  for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = v;
-  __syncthreads();
-  T t = 0;
-#pragma unroll
-  for (int w = 0; w < kScanWarps; ++w) t += warp_sums[w];
-  __syncthreads();
-  return t;
-}
-
-// Block-wide exclusive scan of one value per thread, in thread order.
-// Contains __syncthreads.
-template <class T>
-__device__ __forceinline__ T block_exclusive(T v, T* warp_sums) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T incl = v;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const T peer = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += peer;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
-  __syncthreads();
-  T before = 0;
-#pragma unroll
-  for (int w = 0; w < kScanWarps; ++w) before += w < warp ? warp_sums[w] : T(0);
-  __syncthreads();
-  return before + incl - v;
-}
-
-template <class T>
-__global__ void __launch_bounds__(kThreads) tile_reduce(const T* __restrict__ in, int64_t n, T* __restrict__ tile_sums) {
-  __shared__ T warp_sums[kScanWarps];
-  const int64_t base = int64_t(blockIdx.x) * kScanTile;
-  T acc = 0;
-#pragma unroll
-  for (int k = 0; k < kScanTile / kThreads; ++k) {
-    const int64_t i = base + int64_t(k) * kThreads + threadIdx.x;
-    if (i < n) acc += in[i];
-  }
-  acc = block_total(acc, warp_sums);
-  if (threadIdx.x == 0) tile_sums[blockIdx.x] = acc;
-}
-
-// Each block scans its tile (thread t owns 8 consecutive items) from the sum
-// of all earlier tiles, which it adds up itself; the last block writes the
-// total to out[n].  `in` and `out` may alias: a thread reads its own items
-// before it writes them, and no thread touches another's.
-template <class T>
-__global__ void __launch_bounds__(kThreads) tile_scan(const T* in, int64_t n, const T* __restrict__ tile_sums,
-                                                     T* out) {
-  __shared__ T warp_sums[kScanWarps];
-  T offset = 0;
-  for (int k = threadIdx.x; k < int(blockIdx.x); k += kThreads) offset += tile_sums[k];
-  offset = block_total(offset, warp_sums);
-  const int64_t base = int64_t(blockIdx.x) * kScanTile + int64_t(threadIdx.x) * 8;
-  T v[8];
-  T local = 0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    v[k] = base + k < n ? in[base + k] : T(0);
-    local += v[k];
-  }
-  T run = offset + block_exclusive(local, warp_sums);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (base + k < n) out[base + k] = run;
-    run += v[k];
-  }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kThreads - 1) out[n] = run;
-}
-
-// Scan of up to kSmallScan items in one block of 1024 threads: thread t owns
-// a run of consecutive items; the runs' sums are scanned across the block by
-// warp shuffles and one shared round of warp totals.  `in` and `out` may
-// alias (each thread reads its items before writing them).
-constexpr int kSmallScanThreads = 1024;
-constexpr int64_t kSmallScan = 32 * kSmallScanThreads;
-
-template <class T>
-__global__ void __launch_bounds__(kSmallScanThreads) small_scan(const T* in, int64_t n, T* out) {
-  __shared__ T warp_sums[kSmallScanThreads / 32];
-  const int64_t per = (n + kSmallScanThreads - 1) / kSmallScanThreads;
-  const int64_t begin = int64_t(threadIdx.x) * per;
-  const int64_t end = min(n, begin + per);
-  T local = 0;
-  for (int64_t i = begin; i < end; ++i) local += in[i];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T incl = local;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const T peer = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += peer;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
-  __syncthreads();
-  T before = 0;
-  for (int w = 0; w < warp; ++w) before += warp_sums[w];
-  T run = before + incl - local;
-  for (int64_t i = begin; i < end; ++i) {
-    const T v = in[i];
-    out[i] = run;
-    run += v;
-  }
-  if (threadIdx.x == kSmallScanThreads - 1) out[n] = before + incl;
-}
-
-// Exclusive scan of n items into out[0..n], out[n] the total: one launch up
-// to kSmallScan items, two above.
-template <class T>
-void exclusive_scan(const T* in, T* out, int64_t n, cudaStream_t s) {
-  if (n <= 0) {
-    check(cudaMemsetAsync(out, 0, sizeof(T), s), "scan empty");
-    return;
-  }
-  if (n <= kSmallScan) {
-    GPP_LAUNCH(small_scan<T>, 1, kSmallScanThreads, 0, s, in, n, out);
-    return;
-  }
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  DBuf<T> sums(size_t(tiles), s);
-  GPP_LAUNCH(tile_reduce<T>, int(tiles), kThreads, 0, s, in, n, sums.p);
-  GPP_LAUNCH(tile_scan<T>, int(tiles), kThreads, 0, s, in, n, sums.p, out);
-}
-
 __global__ void det_sum_chunks(const double* __restrict__ v, int64_t n, double* __restrict__ out) {
   __shared__ double sm[kThreads];
   const int64_t base = int64_t(blockIdx.x) * 2048;
@@ -351,10 +240,28 @@ __global__ void det_sum_chunks(const double* __restrict__ v, int64_t n, double* 
 }  // namespace
 
 void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) {
-  exclusive_scan<int32_t>(in, out, n, s);
+  scan_items<int32_t, 1>(
+      n, [in] __device__(int64_t i, int32_t(&v)[1]) { v[0] = in[i]; },
+      [out] __device__(int64_t i, const int32_t(&before)[1], const int32_t(&)[1]) { out[i] = before[0]; },
+      [out, n] __device__(const int32_t(&sum)[1]) { out[n] = sum[0]; }, s);
 }
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s) {
-  exclusive_scan<int64_t>(in, out, n, s);
+void exclusive_scan_pair_i64(const int64_t* a, int64_t* a_out, const int64_t* b, int64_t* b_out, int64_t n,
+                             cudaStream_t s) {
+  scan_items<int64_t, 2>(
+      n,
+      [=] __device__(int64_t i, int64_t(&v)[2]) {
+        v[0] = a[i];
+        v[1] = b[i];
+      },
+      [=] __device__(int64_t i, const int64_t(&before)[2], const int64_t(&)[2]) {
+        a_out[i] = before[0];
+        b_out[i] = before[1];
+      },
+      [=] __device__(const int64_t(&sum)[2]) {
+        a_out[n] = sum[0];
+        b_out[n] = sum[1];
+      },
+      s);
 }
 
 double det_sum(const double* v, int64_t n, cudaStream_t s) {

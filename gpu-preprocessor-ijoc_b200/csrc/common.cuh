@@ -226,6 +226,10 @@ struct Context {
   // Page-locked word that a kernel sets when a bounded wait on another block
   // ran out; sync() turns it into an error.
   int32_t* host_error = nullptr;
+  // Published words of the single-pass scans on this stream (scan.cuh), zero
+  // between launches.
+  unsigned long long* lookback = nullptr;
+  size_t lookback_words = 0;
   cudaStream_t side = nullptr;
   // Scratch blocks this context freed on its own stream, by size class,
   // ready to be handed out again without a driver call (pool_alloc/free).
@@ -368,11 +372,13 @@ struct Status {
 };
 
 // ---------------------------------------------------------------------------
-// Scans (decoupled into three small kernels; deterministic, any length).
+// Scans (one launch each, scan.cuh; deterministic, any length).
 // exclusive prefix sum of in[0..n) into out[0..n]; out[n] = total.  out may
 // alias in for n+1-sized storage only when in has n+1 slots.
 void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s);
-void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);
+// The same of two arrays of n items in one launch.
+void exclusive_scan_pair_i64(const int64_t* a, int64_t* a_out, const int64_t* b, int64_t* b_out, int64_t n,
+                             cudaStream_t s);
 
 // Canonical deterministic sum (chunks of 2048, 256-thread halving tree, chunk
 // totals added in order on the host).  Returns the value on the host.

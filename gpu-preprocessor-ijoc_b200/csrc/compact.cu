@@ -10,6 +10,7 @@
 // second streaming pass.  The general transpose below is only needed for an
 // input A^T that is not row-sorted and for matrices rebuilt by a rule.
 #include "engine.cuh"
+#include "scan.cuh"
 #include "sort.hpp"
 
 #include <algorithm>
@@ -18,16 +19,6 @@
 namespace gpp {
 
 namespace {
-
-__global__ void mask_to_int(const uint8_t* __restrict__ keep, int32_t n, int32_t* __restrict__ out) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    out[i] = keep[i] != 0;
-}
-__global__ void prefix_to_map(const uint8_t* __restrict__ keep, const int32_t* __restrict__ prefix, int32_t n,
-                              int32_t* __restrict__ old_to_new) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    old_to_new[i] = keep[i] ? prefix[i] : -1;
-}
 
 // ---- entry-tiled compaction -------------------------------------------------
 //
@@ -393,105 +384,29 @@ __global__ void compose_kernel(int32_t* __restrict__ next, const int32_t* __rest
   }
 }
 
-// Old -> new maps of the row and the column masks together, straight from
-// the byte masks: one launch counts the kept items of every tile of
-// kMapTile items (row tiles first, then column tiles), a second gives each
-// kept item its rank (earlier tiles' counts plus a block scan) and writes -1
-// for a dropped one; the last tile of each mask writes its total.
-constexpr int kMapTile = 8 * kThreads;
-
-__device__ __forceinline__ int block_sum_i32(int v, int* sh) {
-  for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int t = 0;
-  for (int w = 0; w < kThreads / 32; ++w) t += sh[w];
-  __syncthreads();
-  return t;
-}
-
-struct MaskPair {
-  const uint8_t* keep[2];
-  int32_t n[2];
-  int32_t tiles0;          // tiles of the first mask; the second's follow
-  int32_t* map[2];
-};
-
-__global__ void __launch_bounds__(kThreads) map_tile_counts(MaskPair mp, int32_t* __restrict__ tile_counts) {
-  __shared__ int sh[kThreads / 32];
-  const int side = int(blockIdx.x) < mp.tiles0 ? 0 : 1;
-  const int tile = side ? int(blockIdx.x) - mp.tiles0 : int(blockIdx.x);
-  const int64_t base = int64_t(tile) * kMapTile + int64_t(threadIdx.x) * 8;
-  int c = 0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) c += base + k < mp.n[side] && mp.keep[side][base + k] != 0;
-  c = block_sum_i32(c, sh);
-  if (threadIdx.x == 0) tile_counts[blockIdx.x] = c;
-}
-
-__global__ void __launch_bounds__(kThreads) map_tile_ranks(MaskPair mp, const int32_t* __restrict__ tile_counts,
-                                                           int32_t* __restrict__ totals) {
-  __shared__ int sh[kThreads / 32];
-  __shared__ int warp_incl[kThreads / 32];
-  const int side = int(blockIdx.x) < mp.tiles0 ? 0 : 1;
-  const int first_tile = side ? mp.tiles0 : 0;
-  const int tile = int(blockIdx.x) - first_tile;
-  int offset = 0;
-  for (int k = first_tile + int(threadIdx.x); k < int(blockIdx.x); k += kThreads) offset += tile_counts[k];
-  offset = block_sum_i32(offset, sh);
-  const int64_t base = int64_t(tile) * kMapTile + int64_t(threadIdx.x) * 8;
-  const uint8_t* keep = mp.keep[side];
-  const int32_t n = mp.n[side];
-  uint8_t kept[8];
-  int local = 0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    kept[k] = base + k < n && keep[base + k] != 0;
-    local += kept[k];
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = local;
-  for (int off = 1; off < 32; off <<= 1) {
-    const int peer = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += peer;
-  }
-  if (lane == 31) warp_incl[warp] = incl;
-  __syncthreads();
-  int before = 0;
-  for (int w = 0; w < warp; ++w) before += warp_incl[w];
-  int run = offset + before + incl - local;
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    if (base + k < n) {
-      mp.map[side][base + k] = kept[k] ? run : -1;
-      run += kept[k];
-    }
-  const int tiles_side = side ? int(gridDim.x) - mp.tiles0 : mp.tiles0;
-  if (tile == tiles_side - 1 && threadIdx.x == kThreads - 1) totals[side] = run;
-}
-
 }  // namespace
+
+// Old -> new map of a mask, straight from its bytes: a kept item's rank, -1
+// for a dropped one; *count receives the number kept.
+void map_kept(const uint8_t* keep, int32_t n, int32_t* map, int32_t* count, cudaStream_t s) {
+  select_items(
+      n, [keep] __device__(int64_t i) { return keep[i] != 0; },
+      [map] __device__(int64_t i, int at, bool kept) { map[i] = kept ? at : -1; }, count, s);
+}
 
 int32_t build_old_to_new(const uint8_t* keep, int32_t n, int32_t* old_to_new, cudaStream_t s) {
   if (n == 0) return 0;
-  DBuf<int32_t> prefix(size_t(n) + 1, s);
-  GPP_LAUNCH(mask_to_int, grid_stride_blocks(n), kThreads, 0, s, keep, n, prefix.p);
-  exclusive_scan_i32(prefix.p, prefix.p, n, s);
-  GPP_LAUNCH(prefix_to_map, grid_stride_blocks(n), kThreads, 0, s, keep, prefix.p, n, old_to_new);
-  return read_scalar(prefix.p + n);
+  DBuf<int32_t> count(1, s);
+  map_kept(keep, n, old_to_new, count.p, s);
+  return read_scalar(count.p);
 }
 
 std::pair<int32_t, int32_t> build_old_to_new_pair(const uint8_t* keep_row, int32_t m, int32_t* row_map,
                                                   const uint8_t* keep_col, int32_t n, int32_t* col_map,
                                                   cudaStream_t s) {
-  const int32_t tr = (m + kMapTile - 1) / kMapTile, tc = (n + kMapTile - 1) / kMapTile;
-  if (tr + tc == 0) return {0, 0};
-  MaskPair mp{{keep_row, keep_col}, {m, n}, tr, {row_map, col_map}};
-  DBuf<int32_t> counts(size_t(tr + tc), s);
   Status st;
-  st.clear(2);   // a mask of no items keeps its total at 0
-  GPP_LAUNCH(map_tile_counts, tr + tc, kThreads, 0, s, mp, counts.p);
-  GPP_LAUNCH(map_tile_ranks, tr + tc, kThreads, 0, s, mp, counts.p, st.d);
+  map_kept(keep_row, m, row_map, st.d, s);
+  map_kept(keep_col, n, col_map, st.d + 1, s);
   const int32_t* t = st.read(2);
   return {t[0], t[1]};
 }

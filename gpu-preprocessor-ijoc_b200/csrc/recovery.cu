@@ -6,6 +6,7 @@
 // rewrites them to original indices with the current maps, so the tape that
 // postsolve replays is expressed in the original model throughout.
 #include "engine.cuh"
+#include "scan.cuh"
 
 namespace gpp {
 
@@ -99,21 +100,6 @@ __global__ void globalize_kernel(int64_t count, const int32_t* __restrict__ type
   }
 }
 
-__global__ void fixed_flags(int32_t n, const uint8_t* __restrict__ keep, const uint8_t* __restrict__ prior,
-                            const double* __restrict__ l, const double* __restrict__ u, int32_t* __restrict__ flag) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    flag[i] = (!prior || prior[i]) && !keep[i] && isfinite(l[i]) && isfinite(u[i]) && fabs(l[i] - u[i]) <= 1e-9;
-}
-__global__ void fixed_pack(int32_t n, const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
-                           const double* __restrict__ l, const double* __restrict__ u, const int32_t* __restrict__ cols,
-                           int32_t* __restrict__ out_idx, double* __restrict__ out_val) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    if (flag[i]) {
-      out_idx[pos[i]] = cols[i];
-      out_val[pos[i]] = 0.5 * (l[i] + u[i]);
-    }
-}
-
 __global__ void globalize_ids(int32_t* __restrict__ ids, int64_t n, const int32_t* __restrict__ cols) {
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     ids[i] = cols[ids[i]];
@@ -195,16 +181,33 @@ void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, cons
   // append_fixed (device_recovery.cu:233-276).
   if (!n) return;
   auto s = ctx().stream;
-  DBuf<int32_t> flag(size_t(n) + 1, s), pos(size_t(n) + 1, s);
-  GPP_LAUNCH(fixed_flags, grid_stride_blocks(n), kThreads, 0, s, n, keep_col, prior, l, u, flag.p);
-  exclusive_scan_i32(flag.p, pos.p, n, s);
-  const int32_t count = read_scalar(pos.p + n);
+  // One selection over the columns finds the fixed ones and packs them (into
+  // arrays for all columns, as their number is not known yet); the segment
+  // keeps the packed part.
+  DBuf<int32_t> idx(size_t(n) + 1, s);
+  DBuf<double> val(size_t(n), s);
+  const int32_t* cols = r.cols.p;
+  int32_t* out_idx = idx.p;
+  double* out_val = val.p;
+  select_items(
+      n,
+      [=] __device__(int64_t i) {
+        return (!prior || prior[i]) && !keep_col[i] && isfinite(l[i]) && isfinite(u[i]) && fabs(l[i] - u[i]) <= 1e-9;
+      },
+      [=] __device__(int64_t i, int at, bool taken) {
+        if (!taken) return;
+        out_idx[at] = cols[i];
+        out_val[at] = 0.5 * (l[i] + u[i]);
+      },
+      idx.p + n, s);
+  const int32_t count = read_scalar(idx.p + n);
   if (!count) return;
   FixedSegment f;
   f.count = count;
   f.idx.alloc(size_t(count), s);
   f.val.alloc(size_t(count), s);
-  GPP_LAUNCH(fixed_pack, grid_stride_blocks(n), kThreads, 0, s, n, flag.p, pos.p, l, u, r.cols.p, f.idx.p, f.val.p);
+  f.idx.copy_from(idx.p, size_t(count));
+  f.val.copy_from(val.p, size_t(count));
   r.fixed.push_back(std::move(f));
 }
 

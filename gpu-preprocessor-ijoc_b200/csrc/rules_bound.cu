@@ -405,8 +405,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     GPP_LAUNCH(support_kernel, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val,
                plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, plan.l.p, plan.u.p, rs, lch.p, uch.p, fl.p,
                fu.p, p.zero_tol, p.bound_tol, support_tol, sl.p, su.p, rc.p, ic.p);
-    exclusive_scan_i64(rc.p, rpos.p, n, s);
-    exclusive_scan_i64(ic.p, ipos.p, n, s);
+    exclusive_scan_pair_i64(rc.p, rpos.p, ic.p, ipos.p, n, s);
     const auto [recs, nidx] = read_scalars(rpos.p + n, ipos.p + n);
     if (recs) {
       PostsolveSegment seg = make_segment(recs, nidx, 4 * recs);
@@ -428,8 +427,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     DBuf<int64_t> rc(size_t(n) + 1, s), nz(size_t(n) + 1, s), rpos(size_t(n) + 1, s), npos(size_t(n) + 1, s);
     GPP_LAUNCH(fixed_record_sizes, grid_stride_blocks(n), kThreads, 0, s, n, fx.p, lp.AT.ptr, lp.AT.idx,
                plan.keep_row.p, rc.p, nz.p);
-    exclusive_scan_i64(rc.p, rpos.p, n, s);
-    exclusive_scan_i64(nz.p, npos.p, n, s);
+    exclusive_scan_pair_i64(rc.p, rpos.p, nz.p, npos.p, n, s);
     const auto [recs, nnz] = read_scalars(rpos.p + n, npos.p + n);
     PostsolveSegment seg = make_segment(recs, recs + nnz, 2 * recs + nnz);
     DBuf<double> oc(size_t(recs), s), ov(size_t(recs), s);

@@ -27,6 +27,7 @@
 #include <climits>
 
 #include "engine.cuh"
+#include "scan.cuh"
 #include "sort.hpp"
 
 namespace gpp {
@@ -162,17 +163,14 @@ __global__ void dt_candidates(int m, const offset_t* __restrict__ ptr, const int
   }
 }
 
-// The smallest flagged index (flag/pos from an exclusive scan).
-__global__ void dt_scatter_first(int count, const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
-                                 int32_t* __restrict__ out) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
-    if (flag[q] && pos[q] == 0) out[0] = q;
-}
-
-__global__ void dt_scatter(int count, const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
-                           const int32_t* __restrict__ ids, int32_t* __restrict__ out) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
-    if (flag[q]) out[pos[q]] = ids ? ids[q] : q;
+// Indices (or `ids`) of the nonzero flags, in order; *total their number.
+void list_flagged(int count, const int32_t* flag, const int32_t* ids, int32_t* out, int32_t* total, cudaStream_t s) {
+  select_items(
+      count, [flag] __device__(int64_t q) { return flag[q] != 0; },
+      [ids, out] __device__(int64_t q, int at, bool taken) {
+        if (taken) out[at] = ids ? ids[q] : int32_t(q);
+      },
+      total, s);
 }
 
 // Matching round (:989-1027): reset the owners of the active rows' columns,
@@ -264,28 +262,25 @@ __global__ void dt_apply(int sel, const int32_t* __restrict__ rows, const int32_
   }
 }
 
-__global__ void dt_subst_flags(int sel, const uint8_t* __restrict__ kind, int32_t* __restrict__ flag) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sel; t += gridDim.x * blockDim.x)
-    flag[t] = kind[t] == kPairSubst ? 1 : 0;
-}
-
-// DoubletonEquation records: indices [elim, keep, row, 0], values [a_e, a_k,
-// rhs, l_e, u_e, l_k, u_k, new l_k, new u_k, c_e, 0, 0] (:641-669).
-__global__ void dt_pack(int sel, const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
-                        const int32_t* __restrict__ rec_idx, const double* __restrict__ rec_val,
-                        int32_t* __restrict__ types, int64_t* __restrict__ is, int64_t* __restrict__ vs,
-                        int32_t* __restrict__ oidx, double* __restrict__ oval) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sel; t += gridDim.x * blockDim.x) {
-    if (!flag[t]) continue;
-    const int64_t r = pos[t];
+// DoubletonEquation record r of pair t: indices [elim, keep, row, 0], values
+// [a_e, a_k, rhs, l_e, u_e, l_k, u_k, new l_k, new u_k, c_e, 0, 0] (:641-669).
+struct PairRecords {
+  const int32_t* rec_idx;
+  const double* rec_val;
+  int32_t* types;
+  int64_t *is, *vs;
+  int32_t* idx;
+  double* val;
+  __device__ void operator()(int64_t t, int64_t r, bool taken) const {
+    if (!taken) return;
     if (r == 0) { is[0] = 0; vs[0] = 0; }
     types[r] = 13;  // DoubletonEquation
     is[r + 1] = 4 * (r + 1);
     vs[r + 1] = 12 * (r + 1);
-    for (int q = 0; q < 4; ++q) oidx[4 * r + q] = rec_idx[4 * int64_t(t) + q];
-    for (int q = 0; q < 12; ++q) oval[12 * r + q] = rec_val[12 * int64_t(t) + q];
+    for (int q = 0; q < 4; ++q) idx[4 * r + q] = rec_idx[4 * t + q];
+    for (int q = 0; q < 12; ++q) val[12 * r + q] = rec_val[12 * t + q];
   }
-}
+};
 
 // Columns whose entries shift row sides: eliminated columns (a * beta) and
 // fixed keep columns (a * value).
@@ -719,7 +714,7 @@ void doubleton_single_row(Plan& plan, const WorkingLp& lp, const gpp_params& p) 
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
   const double zt = p.zero_tol, ratio_tol = std::fmax(1.0e-9, p.bound_tol);
-  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m) + 1, s), pos(size_t(m) + 1, s), keep_c(size_t(m), s),
+  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m), s), acc(size_t(m) + 1, s), keep_c(size_t(m), s),
       elim_c(size_t(m), s);
   DBuf<double> keep_v(size_t(m), s), elim_v(size_t(m), s);
   GPP_LAUNCH(dt_col_nnz, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p,
@@ -728,10 +723,8 @@ void doubleton_single_row(Plan& plan, const WorkingLp& lp, const gpp_params& p) 
              plan.keep_row.p, plan.keep_col.p, col_nnz.p, plan.AL.p, plan.AU.p, zt, p.bound_tol, ratio_tol,
              p.doubleton_equations_max_fill_in_proxy, lp.AT.ptr, lp.AT.idx, lp.AT.val, flag.p, keep_c.p, elim_c.p,
              keep_v.p, elim_v.p);
-  exclusive_scan_i32(flag.p, pos.p, m, s);
-  if (read_scalar(pos.p + m) == 0) return;
-  DBuf<int32_t> acc(size_t(1), s);
-  GPP_LAUNCH(dt_scatter_first, grid_stride_blocks(m), kThreads, 0, s, m, flag.p, pos.p, acc.p);
+  list_flagged(m, flag.p, nullptr, acc.p, acc.p + m, s);   // acc[0] is the smallest
+  if (read_scalar(acc.p + m) == 0) return;
   Status st;
   st.clear(kStWords);
   DBuf<double> meta(3, s), rec_val(12, s);
@@ -796,7 +789,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     ~Release() { if (own) free_csr(M); }
   } release{sorted_at, !at_sorted};
 
-  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m) + 1, s), pos(size_t(m) + 1, s), keep_c(size_t(m), s),
+  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m), s), acc(size_t(m) + 1, s), keep_c(size_t(m), s),
       elim_c(size_t(m), s);
   DBuf<double> keep_v(size_t(m), s), elim_v(size_t(m), s);
   GPP_LAUNCH(dt_col_nnz, grid_stride_blocks(n), kThreads, 0, s, n, AT.ptr, AT.idx, AT.val, plan.keep_row.p,
@@ -805,15 +798,13 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
              plan.keep_row.p, plan.keep_col.p, col_nnz.p, plan.AL.p, plan.AU.p, zt, tol, ratio_tol,
              p.doubleton_equations_max_fill_in_proxy, AT.ptr, AT.idx, AT.val, flag.p, keep_c.p, elim_c.p, keep_v.p,
              elim_v.p);
-  exclusive_scan_i32(flag.p, pos.p, m, s);
-  const int acceptable = read_scalar(pos.p + m);
+  list_flagged(m, flag.p, nullptr, acc.p, acc.p + m, s);
+  const int acceptable = read_scalar(acc.p + m);
   if (acceptable == 0) return;
-  DBuf<int32_t> acc(size_t(acceptable), s);
-  GPP_LAUNCH(dt_scatter, grid_stride_blocks(m), kThreads, 0, s, m, flag.p, pos.p, nullptr, acc.p);
 
   // Matching rounds over the acceptable rows (ascending).
   DBuf<uint8_t> active(size_t(acceptable), s), blocked(size_t(n), s);
-  DBuf<int32_t> owner(size_t(n), s), chosen(size_t(acceptable) + 1, s), cpos(size_t(acceptable) + 1, s);
+  DBuf<int32_t> owner(size_t(n), s), chosen(size_t(acceptable), s), rows(size_t(acceptable) + 1, s);
   check(cudaMemsetAsync(active.p, 1, size_t(acceptable), s), "doubleton active");
   blocked.zero();
   chosen.zero();
@@ -824,13 +815,11 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     GPP_LAUNCH(dt_select, gk, kThreads, 0, s, acceptable, acc.p, active.p, blocked.p, keep_c.p, elim_c.p, owner.p,
                chosen.p);
   }
-  exclusive_scan_i32(chosen.p, cpos.p, acceptable, s);
-  const int sel = read_scalar(cpos.p + acceptable);
+  list_flagged(acceptable, chosen.p, acc.p, rows.p, rows.p + acceptable, s);
+  const int sel = read_scalar(rows.p + acceptable);
   const double ratio = double(sel) / double(acceptable);
   if (sel == 0 || sel < p.doubleton_equations_min_selected_per_batch || ratio < p.doubleton_equations_min_selected_ratio)
     return;
-  DBuf<int32_t> rows(size_t(sel), s);
-  GPP_LAUNCH(dt_scatter, gk, kThreads, 0, s, acceptable, chosen.p, cpos.p, acc.p, rows.p);
 
   // Apply against the values before the batch (columns are distinct).
   Status st;
@@ -847,16 +836,13 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
   if (!f[kStAny]) return;
   const int subst = f[kStSubst];
 
-  DBuf<int32_t> sflag(size_t(sel) + 1, s), spos(size_t(sel) + 1, s);
-  if (subst) {
-    GPP_LAUNCH(dt_subst_flags, gs, kThreads, 0, s, sel, kind.p, sflag.p);
-    exclusive_scan_i32(sflag.p, spos.p, sel, s);
-    if (p.record_postsolve_tape) {
-      PostsolveSegment seg = make_segment(subst, 4 * int64_t(subst), 12 * int64_t(subst));
-      GPP_LAUNCH(dt_pack, gs, kThreads, 0, s, sel, sflag.p, spos.p, rec_idx.p, rec_val.p, seg.types.p, seg.is.p,
-                 seg.vs.p, seg.idx.p, seg.val.p);
-      plan.tape.push_back(std::move(seg));
-    }
+  if (subst && p.record_postsolve_tape) {
+    PostsolveSegment seg = make_segment(subst, 4 * int64_t(subst), 12 * int64_t(subst));
+    DBuf<int32_t> packed(1, s);
+    select_items(
+        sel, [kind = kind.p] __device__(int64_t t) { return kind[t] == kPairSubst; },
+        PairRecords{rec_idx.p, rec_val.p, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p}, packed.p, s);
+    plan.tape.push_back(std::move(seg));
   }
 
   // Row shifts.

@@ -13,6 +13,7 @@
 
 #include "engine.cuh"
 #include "folding.hpp"
+#include "scan.cuh"
 #include "sort.hpp"
 
 namespace gpp {
@@ -171,12 +172,6 @@ row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, con
   for (int q = wid; q < counts[1]; q += nwarps) row_hash_warp(g, longq[q]);
 }
 
-__global__ void gather_live(int n, const int32_t* __restrict__ take, const int32_t* __restrict__ pos,
-                            const uint64_t* __restrict__ hash, uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if (take[i]) { keys[pos[i]] = hash[i]; ids[pos[i]] = i; }
-}
-
 // Repeated-hash filter.  Only a hash that two or more live items share can
 // form a group, so only those items need sorting.  Every live item takes two
 // positions in a bitmap from its mixed hash (the SplitMix64 finaliser, so the
@@ -207,17 +202,10 @@ __global__ void mark_hash_bits(int n, const uint8_t* __restrict__ keep, const ui
     }
   }
 }
-__global__ void flag_repeated(int n, const uint8_t* __restrict__ keep, const uint64_t* __restrict__ hash,
-                              const uint32_t* __restrict__ twice, uint64_t bit_mask, int32_t* __restrict__ flag) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int32_t f = 0;
-    if (keep[i]) {
-      const uint64_t z = mix_hash(hash[i]);
-      const uint64_t b0 = z & bit_mask, b1 = (z >> 32) & bit_mask;
-      f = (twice[b0 >> 5] >> (b0 & 31u) & 1u) && (twice[b1 >> 5] >> (b1 & 31u) & 1u);
-    }
-    flag[i] = f;
-  }
+__device__ __forceinline__ bool hash_may_repeat(uint64_t hash, const uint32_t* twice, uint64_t bit_mask) {
+  const uint64_t z = mix_hash(hash);
+  const uint64_t b0 = z & bit_mask, b1 = (z >> 32) & bit_mask;
+  return (twice[b0 >> 5] >> (b0 & 31u) & 1u) && (twice[b1 >> 5] >> (b1 & 31u) & 1u);
 }
 
 // --- parallel rows ------------------------------------------------------------
@@ -316,16 +304,6 @@ __global__ void row_groups_kernel(int count, const uint64_t* __restrict__ sh, co
   }
 }
 
-__global__ void deleted_keys(int m, const uint8_t* __restrict__ del, const int32_t* __restrict__ step,
-                             const int32_t* __restrict__ pos, uint64_t* __restrict__ keys, int32_t* __restrict__ ids,
-                             uint8_t* __restrict__ keep_row) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-    if (del[i]) {
-      keys[pos[i]] = (uint64_t(uint32_t(step[i])) << 32) | uint32_t(i);
-      ids[pos[i]] = i;
-      keep_row[i] = 0;
-    }
-}
 __global__ void pack_parallel_records(int64_t count, const int32_t* __restrict__ ids, const int32_t* __restrict__ first,
                                       const double* __restrict__ rec_vals, int type, int32_t* __restrict__ types,
                                       int64_t* __restrict__ is, int64_t* __restrict__ vs, int32_t* __restrict__ idx,
@@ -516,9 +494,6 @@ __global__ void col_groups_kernel(int count, const uint64_t* __restrict__ sh, co
   }
 }
 
-__global__ void flag_to_int(int n, const uint8_t* __restrict__ f, int32_t* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = f[i] != 0;
-}
 __global__ void col_apply(int n, int m, const uint8_t* __restrict__ del, const uint8_t* __restrict__ fixed,
                           const double* __restrict__ fval, const double* __restrict__ c, const double* __restrict__ shift,
                           uint8_t* __restrict__ keep_col, double* __restrict__ l, double* __restrict__ u,
@@ -575,7 +550,16 @@ __global__ void fixed_pack(int n, const uint8_t* __restrict__ fx, const offset_t
 constexpr int32_t kRepeatFilterMin = 32768;
 int32_t sorted_live_hashes(const uint64_t* hash, const uint8_t* keep, int32_t n, DBuf<uint64_t>& keys,
                            DBuf<int32_t>& ids, cudaStream_t s) {
-  DBuf<int32_t> flag(size_t(n) + 1, s), pos(size_t(n) + 1, s);
+  // The pairs are packed by one selection into arrays for all items (their
+  // number is known afterwards).
+  keys.alloc(size_t(std::max(n, 1)), s);
+  ids.alloc(size_t(std::max(n, 1)) + 1, s);
+  int32_t* total = ids.p + std::max(n, 1);
+  const auto pack = [hash, out_keys = keys.p, out_ids = ids.p] __device__(int64_t i, int at, bool taken) {
+    if (!taken) return;
+    out_keys[at] = hash[i];
+    out_ids[at] = int32_t(i);
+  };
   if (n > kRepeatFilterMin) {
     // 32 bitmap positions per item, a power of two between 2^20 and 2^29.
     int lg = 20;
@@ -586,16 +570,13 @@ int32_t sorted_live_hashes(const uint64_t* hash, const uint8_t* keep, int32_t n,
     const uint64_t bit_mask = (uint64_t(1) << lg) - 1;
     GPP_LAUNCH(mark_hash_bits, grid_stride_blocks(n), kThreads, 0, s, n, keep, hash, bits.p, bits.p + words,
                bit_mask);
-    GPP_LAUNCH(flag_repeated, grid_stride_blocks(n), kThreads, 0, s, n, keep, hash, bits.p + words, bit_mask,
-               flag.p);
+    const uint32_t* twice = bits.p + words;
+    select_items(
+        n, [=] __device__(int64_t i) { return keep[i] && hash_may_repeat(hash[i], twice, bit_mask); }, pack, total, s);
   } else {
-    GPP_LAUNCH(flag_to_int, grid_stride_blocks(n), kThreads, 0, s, n, keep, flag.p);
+    select_items(n, [keep] __device__(int64_t i) { return keep[i] != 0; }, pack, total, s);
   }
-  exclusive_scan_i32(flag.p, pos.p, n, s);
-  const int32_t count = read_scalar(pos.p + n);
-  keys.alloc(size_t(std::max(count, 1)), s);
-  ids.alloc(size_t(std::max(count, 1)), s);
-  GPP_LAUNCH(gather_live, grid_stride_blocks(n), kThreads, 0, s, n, flag.p, pos.p, hash, keys.p, ids.p);
+  const int32_t count = read_scalar(total);
   radix_sort_pairs(keys.p, ids.p, count, s);
   return count;
 }
@@ -652,15 +633,20 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
              plan.keep_col.p, plan.AL.p, plan.AU.p, lp.A.ptr, lp.A.idx, lp.A.val, p.zero_tol, p.feasibility_tol,
              del.p, merge_to.p, step.p, rec.p, st.d);
   if (st.read(1)[0]) { plan.has_infeasible = true; return; }
-  DBuf<int32_t> flag(size_t(m) + 1, s), pos(size_t(m) + 1, s);
-  GPP_LAUNCH(flag_to_int, grid_stride_blocks(m), kThreads, 0, s, m, del.p, flag.p);
-  exclusive_scan_i32(flag.p, pos.p, m, s);
-  const int32_t deleted = read_scalar(pos.p + m);
+  DBuf<uint64_t> dkeys(size_t(m), s);
+  DBuf<int32_t> dids(size_t(m) + 1, s);
+  select_items(
+      m, [del = del.p] __device__(int64_t i) { return del[i] != 0; },
+      [step = step.p, out_keys = dkeys.p, ids = dids.p, keep_row = plan.keep_row.p] __device__(int64_t i, int at,
+                                                                                               bool taken) {
+        if (!taken) return;
+        out_keys[at] = (uint64_t(uint32_t(step[i])) << 32) | uint32_t(i);
+        ids[at] = int32_t(i);
+        keep_row[i] = 0;
+      },
+      dids.p + m, s);
+  const int32_t deleted = read_scalar(dids.p + m);
   if (!deleted) return;
-  DBuf<uint64_t> dkeys(size_t(deleted), s);
-  DBuf<int32_t> dids(size_t(deleted), s);
-  GPP_LAUNCH(deleted_keys, grid_stride_blocks(m), kThreads, 0, s, m, del.p, step.p, pos.p, dkeys.p, dids.p,
-             plan.keep_row.p);
   if (p.record_postsolve_tape) {
     // Records ordered by (merge step, deleted row) (rule_parallel_rows.cu:79-84).
     radix_sort_pairs(dkeys.p, dids.p, deleted, s, bits_up_to(deleted) << 32);   // rows already ascend
@@ -710,16 +696,14 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
   if (!merged && !any_fixed) return;
   if (merged && p.record_postsolve_tape) {
     // Records ordered by deleted column (rule_parallel_columns.cu:83-87).
-    DBuf<int32_t> flag(size_t(n) + 1, s), pos(size_t(n) + 1, s);
-    GPP_LAUNCH(flag_to_int, grid_stride_blocks(n), kThreads, 0, s, n, del.p, flag.p);
-    exclusive_scan_i32(flag.p, pos.p, n, s);
-    const int32_t merges = read_scalar(pos.p + n);
-    DBuf<uint64_t> dkeys(size_t(merges), s);
-    DBuf<int32_t> dids(size_t(merges), s);
-    DBuf<uint8_t> untouched(size_t(n), s);
-    untouched.copy_from(plan.keep_col.p, size_t(n));
-    GPP_LAUNCH(deleted_keys, grid_stride_blocks(n), kThreads, 0, s, n, del.p, merge_to.p, pos.p, dkeys.p, dids.p,
-               untouched.p);  // ids are already in ascending column order
+    DBuf<int32_t> dids(size_t(n) + 1, s);
+    select_items(
+        n, [del = del.p] __device__(int64_t i) { return del[i] != 0; },
+        [ids = dids.p] __device__(int64_t i, int at, bool taken) {
+          if (taken) ids[at] = int32_t(i);
+        },
+        dids.p + n, s);
+    const int32_t merges = read_scalar(dids.p + n);
     PostsolveSegment seg = make_segment(merges, 2 * int64_t(merges), 5 * int64_t(merges));
     GPP_LAUNCH(pack_parallel_records, grid_stride_blocks(merges + 1), kThreads, 0, s, int64_t(merges), dids.p,
                merge_to.p, rec.p, 3, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p);
@@ -731,8 +715,7 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
       DBuf<int64_t> rc(size_t(n) + 1, s), nz(size_t(n) + 1, s), rpos(size_t(n) + 1, s), npos(size_t(n) + 1, s);
       GPP_LAUNCH(fixed_sizes, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, lp.AT.ptr, lp.AT.idx, plan.keep_row.p,
                  rc.p, nz.p);
-      exclusive_scan_i64(rc.p, rpos.p, n, s);
-      exclusive_scan_i64(nz.p, npos.p, n, s);
+      exclusive_scan_pair_i64(rc.p, rpos.p, nz.p, npos.p, n, s);
       const auto [recs, nnz] = read_scalars(rpos.p + n, npos.p + n);
       PostsolveSegment seg = make_segment(recs, recs + nnz, 2 * recs + nnz);
       GPP_LAUNCH(fixed_pack, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, lp.AT.ptr, lp.AT.idx, lp.AT.val,

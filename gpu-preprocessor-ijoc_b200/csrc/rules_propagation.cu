@@ -237,8 +237,7 @@ void rule_dual_fix(Plan& plan, const WorkingLp& lp, const Stats& stats, const gp
     DBuf<int64_t> rc(size_t(n) + 1, s), sz(size_t(n) + 1, s), rpos(size_t(n) + 1, s), spos(size_t(n) + 1, s);
     GPP_LAUNCH(infinite_sizes, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, plan.keep_row.p,
                plan.rule_entry_keep_col, lp.A.ptr, lp.A.idx, lp.AT.ptr, lp.AT.idx, rc.p, sz.p);
-    exclusive_scan_i64(rc.p, rpos.p, n, s);
-    exclusive_scan_i64(sz.p, spos.p, n, s);
+    exclusive_scan_pair_i64(rc.p, rpos.p, sz.p, spos.p, n, s);
     const auto [recs, size] = read_scalars(rpos.p + n, spos.p + n);
     if (recs) {
       PostsolveSegment seg = make_segment(recs, size + 3 * recs, size + recs);

@@ -22,6 +22,7 @@
 
 #include "engine.cuh"
 #include "live_visit.cuh"
+#include "scan.cuh"
 #include "sort.hpp"
 
 namespace gpp {
@@ -683,8 +684,21 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
       const int blocks = std::max(1, std::min((nelim + 7) / 8, kNumSMs * 16));
       GPP_LAUNCH(sc_sub_sizes, blocks, kThreads, 0, s, sorted.p, nelim, owner.p, lp.A.ptr, lp.A.idx, lp.A.val,
                  plan.keep_col.p, p.zero_tol, sel.p, sup.p);
-      exclusive_scan_i32(sel.p, rec.p, nelim, s);
-      exclusive_scan_i64(sup.p, spos.p, nelim, s);
+      scan_items<int64_t, 2>(
+          nelim,
+          [sel = sel.p, sup = sup.p] __device__(int64_t i, int64_t(&v)[2]) {
+            v[0] = sel[i];
+            v[1] = sup[i];
+          },
+          [rec = rec.p, spos = spos.p] __device__(int64_t i, const int64_t(&before)[2], const int64_t(&)[2]) {
+            rec[i] = int32_t(before[0]);
+            spos[i] = before[1];
+          },
+          [rec = rec.p + nelim, spos = spos.p + nelim] __device__(const int64_t(&sum)[2]) {
+            *rec = int32_t(sum[0]);
+            *spos = sum[1];
+          },
+          s);
       const auto [recs32, support] = read_scalars(rec.p + nelim, spos.p + nelim);
       const int64_t recs = recs32;
       if (recs) {

@@ -496,8 +496,7 @@ void commit_projection(Plan& plan, const WorkingLp& lp, const gpp_params& p, con
     st.clear(1);
     GPP_LAUNCH(projection_sizes<K>, grid_stride_blocks(n), kThreads, 0, s, n, in, selected.p, incident, rc.p, sc.p,
                st.d);
-    exclusive_scan_i64(rc.p, rpos.p, n, s);
-    exclusive_scan_i64(sc.p, spos.p, n, s);
+    exclusive_scan_pair_i64(rc.p, rpos.p, sc.p, spos.p, n, s);
     if (st.read(1)[0]) throw std::runtime_error("projection tape certificate changed before commit");
     const auto [recs, support] = read_scalars(rpos.p + n, spos.p + n);
     if (recs) {

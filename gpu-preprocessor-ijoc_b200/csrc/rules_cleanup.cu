@@ -228,46 +228,71 @@ double domain_objective(const double* contrib, const uint8_t* entry_keep, int32_
   return det_sum(masked.p, n, s);
 }
 
+namespace {
+// What the first checks of the four rules below find on the current plan, in
+// one pass: a thread reads one column and one row and ORs the rules that may
+// act into *found (one atomic per block at most).
+//  - fixed variables: a kept column whose finite bounds lie within bound_tol;
+//  - empty columns: any kept empty column (fixed, infeasible or unbounded);
+//  - empty rows: any kept row without live entries;
+//  - singleton rows: a row that gives a bound, or, when there is none (the
+//    candidate bounds are then the columns' own), a column whose bounds cross
+//    by more than bound_tol or are NaN.
+// Bound by its reads, 18 bytes a column and 6 a row; the four detection kernels
+// of the rules, which also fill the arrays that the rules go on with, took 7
+// launches and copies and about 230 bytes a column.
+__global__ void __launch_bounds__(kThreads)
+cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ keep_row,
+                     const uint8_t* __restrict__ keep_col, const double* __restrict__ l, const double* __restrict__ u,
+                     const uint8_t* __restrict__ empty_col, const int32_t* __restrict__ row_nnz,
+                     const uint8_t* __restrict__ singleton_row, const int32_t* __restrict__ scol,
+                     const double* __restrict__ sval, double bound_tol, double zero_tol, uint32_t* found) {
+  uint32_t f = 0;
+  const int top = n > m ? n : m;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
+    if (k < n) {
+      const double lj = l[k], uj = u[k];
+      if (keep_col[k]) {
+        if (isfinite(lj) && isfinite(uj) && lj <= uj && uj - lj <= bound_tol) f |= kProbeFixed;
+        if (empty_col[k]) f |= kProbeEmptyColumns;
+      }
+      if (lj > uj + bound_tol || lj != lj || uj != uj) f |= kProbeSingletonRows;
+    }
+    if (k < m && keep_row[k]) {
+      if (row_nnz[k] == 0) f |= kProbeEmptyRows;
+      if (singleton_row[k]) {
+        const int col = scol[k];
+        if (col >= 0 && col < n && fabs(sval[k]) > zero_tol) f |= kProbeSingletonRows;
+      }
+    }
+  }
+  f = __reduce_or_sync(0xffffffffu, f & rules);
+  __shared__ uint32_t block_found;
+  if (threadIdx.x == 0) block_found = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0 && f) atomicOr(&block_found, f);
+  __syncthreads();
+  if (threadIdx.x == 0 && block_found) atomicOr(found, block_found);
+}
+}  // namespace
+
 uint32_t cleanup_probe(const Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules) {
   // The first-stage detections of the four rules below, on the current plan,
-  // with one readback.  Each is the kernel its rule launches first and writes
-  // only scratch and status words; a rule whose detection finds nothing
+  // with one launch and one readback; a rule whose detection finds nothing
   // (no candidate, no infeasibility) returns without touching the plan.
   if (plan.has_infeasible || plan.has_unbounded) return rules;
   const int n = lp.n(), m = lp.m();
+  if (n == 0) rules &= ~(kProbeFixed | kProbeEmptyColumns);
+  if (m == 0) rules &= ~(kProbeEmptyRows | kProbeSingletonRows);
+  if (!rules) return 0;
   auto s = ctx().stream;
   Status st;
-  st.clear(16);
-  DBuf<uint8_t> fixed(size_t(std::max(n, 1)), s), remove(size_t(std::max(m, 1)), s);
-  DBuf<double> fval(size_t(std::max(n, 1)), s), contrib(size_t(std::max(n, 1)), s), radius(size_t(std::max(n, 1)), s);
-  DBuf<double> cl, cu;
-  if ((rules & kProbeFixed) && n > 0)
-    GPP_LAUNCH(fixed_candidates, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.l.p, plan.u.p,
-               plan.c.p, p.bound_tol, fixed.p, fval.p, contrib.p, radius.p, st.d + 1);
-  if ((rules & kProbeEmptyColumns) && n > 0)
-    GPP_LAUNCH(empty_columns_classify, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, stats.empty_col.p,
-               plan.c.p, plan.l.p, plan.u.p, p.bound_tol, p.zero_tol, fixed.p, fval.p, contrib.p, st.d + 4);
-  if ((rules & kProbeEmptyRows) && m > 0)
-    GPP_LAUNCH(empty_rows_kernel, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p,
-               plan.AL.p, plan.AU.p, p.feasibility_tol, st.d + 8, 0);
-  if ((rules & kProbeSingletonRows) && m > 0) {
-    cl.alloc(size_t(std::max(n, 1)), s);
-    cu.alloc(size_t(std::max(n, 1)), s);
-    cl.copy_from(plan.l.p, size_t(n));
-    cu.copy_from(plan.u.p, size_t(n));
-    GPP_LAUNCH(singleton_row_bounds, grid_stride_blocks(m), kThreads, 0, s, m, n, plan.keep_row.p,
-               stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, plan.AL.p, plan.AU.p, p.zero_tol, cl.p,
-               cu.p, remove.p);
-    GPP_LAUNCH(singleton_rows_check, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n, cl.p, cu.p, plan.l.p,
-               plan.u.p, remove.p, p.bound_tol, st.d + 12);
-  }
-  const int32_t* f = st.read(16);
-  uint32_t act = 0;
-  if ((rules & kProbeFixed) && n > 0 && f[1] != 0) act |= kProbeFixed;
-  if ((rules & kProbeEmptyColumns) && n > 0 && (f[4] | f[5] | f[6]) != 0) act |= kProbeEmptyColumns;
-  if ((rules & kProbeEmptyRows) && m > 0 && (f[8] | f[9]) != 0) act |= kProbeEmptyRows;
-  if ((rules & kProbeSingletonRows) && m > 0 && (f[12] | f[13] | f[14]) != 0) act |= kProbeSingletonRows;
-  return act;
+  st.clear(1);
+  GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 6.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n,
+                   rules, plan.keep_row.p, plan.keep_col.p, plan.l.p, plan.u.p, stats.empty_col.p, stats.row_nnz.p,
+                   stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol,
+                   reinterpret_cast<uint32_t*>(st.d));
+  return uint32_t(st.read(1)[0]);
 }
 
 void rule_fixed_variables(Plan& plan, const WorkingLp& lp, const gpp_params& p) {

@@ -39,7 +39,6 @@ struct Engine {
   Plan plan;
   Stats stats;
   bool stats_dirty = true;
-  DBuf<uint8_t> entry_cols;
   DBuf<double> ref_bounds;
   uint32_t* inf_hist = nullptr;   // histogram features (scheduled runs only)
   uint64_t deletion_serial = 0;
@@ -67,7 +66,6 @@ struct Engine {
     init_plan(plan);
     plan.inf_hist = inf_hist;
     allocate_stats(stats, cur.m(), cur.n());
-    entry_cols.alloc(size_t(cur.n()), s());
     stats_dirty = true;
     active = true;
   }
@@ -120,8 +118,9 @@ struct Engine {
     const NvtxRange range(name);
     prepare();
     refresh();
-    entry_cols.copy_from(plan.keep_col.p, size_t(cur.n()));
-    plan.rule_entry_keep_col = entry_cols.p;
+    // The statistics are fresh, so the column mask they describe is the
+    // rule's entry mask; it stays as it is until the next refresh.
+    plan.rule_entry_keep_col = stats.seen_col.p;
     plan.has_change = plan.has_row_action = plan.has_col_action = false;
     plan.has_redundant_row_deletion = plan.has_row_deletion = false;
     plan.obj_delta = 0.0;
@@ -136,7 +135,7 @@ struct Engine {
       cur.obj += plan.obj_delta;
       capture_tape(out.record, plan.tape);
       if (plan.has_col_action)
-        append_fixed(out.record, plan.keep_col.p, entry_cols.p, plan.l.p, plan.u.p, cur.n());
+        append_fixed(out.record, plan.keep_col.p, stats.seen_col.p, plan.l.p, plan.u.p, cur.n());
       pending = true;
       if (plan.has_row_action || plan.has_col_action) stats_dirty = true;
     } else {

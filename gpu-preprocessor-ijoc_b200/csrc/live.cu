@@ -600,7 +600,6 @@ void allocate_stats(Stats& st, int32_t m, int32_t n) {
   st.live_nnz.alloc(1, s);
   st.seen_row.alloc(size_t(m), s); st.seen_col.alloc(size_t(n), s);
   st.dirty_row.alloc(size_t(m), s); st.dirty_col.alloc(size_t(n), s);
-  st.dirty_row.zero(); st.dirty_col.zero();
   st.deleted.alloc(size_t(m) + size_t(n), s);
   st.counters.alloc(2, s);
   st.valid = false;
@@ -619,76 +618,163 @@ namespace {
 // the full recount's exactly (integer counts, and the support of a degree-1
 // row is its only live entry).
 
-// Rows (first m) and columns (next n) whose mask went from kept to deleted.
-__global__ void inc_deleted(int m, int n, const uint8_t* __restrict__ seen_row, const uint8_t* __restrict__ keep_row,
-                            const uint8_t* __restrict__ seen_col, const uint8_t* __restrict__ keep_col,
-                            int32_t* __restrict__ list, int32_t* counters) {
-  const int stride = gridDim.x * blockDim.x;
-  const int top = (max(m, n) + stride - 1) / stride * stride;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < top; i += stride) {
-    const bool dr = i < m && seen_row[i] && !keep_row[i];
-    const bool dc = i < n && seen_col[i] && !keep_col[i];
-    const int pr = block_append(counters, dr);
-    if (dr) list[pr] = i;
-    const int pc = block_append(counters + 1, dc);
-    if (dc) list[m + pc] = i;
-  }
-}
-
-// One warp per deleted outer item: its own statistics are reset, and every
-// still-kept inner item it touches loses one degree and is marked dirty.
-// `total` (rows only) drops by the item's old degree; `cross_total` (columns
-// only) drops by one per kept row it leaves.
-__global__ void inc_walk(const int32_t* __restrict__ list, const int32_t* __restrict__ count, const offset_t* __restrict__ ptr,
-                         const int32_t* __restrict__ idx, const uint8_t* __restrict__ keep_inner,
-                         int32_t* __restrict__ degree, uint8_t* __restrict__ empty, uint8_t* __restrict__ singleton,
-                         int32_t* __restrict__ support, double* __restrict__ coefficient,
-                         int32_t* __restrict__ inner_degree, uint8_t* __restrict__ inner_dirty,
-                         unsigned long long* total, unsigned long long* cross_total) {
+// Items of one mask that went from kept to deleted, appended to `list`; the
+// mask last seen is brought up to date.  Sixteen mask bytes per thread: between
+// two refreshes almost no byte differs, so a sweep costs two bytes read and
+// one written per item.
+__device__ __forceinline__ void find_deleted(int n, uint8_t* __restrict__ seen, const uint8_t* __restrict__ keep,
+                                             int32_t* __restrict__ list, int32_t* counter) {
   const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  const int k = *count;
-  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < k; w += warps) {
-    const int r = list[w];
-    unsigned int left = 0;
-    for (offset_t p = ptr[r] + lane; p < ptr[r + 1]; p += 32) {
-      const int c = idx[p];
-      if (keep_inner[c]) {
-        atomicSub(inner_degree + c, 1);
-        inner_dirty[c] = 1;
-        ++left;
+  const int chunks = (n + 15) / 16;
+  const int stride = gridDim.x * blockDim.x;
+  const int top = (chunks + stride - 1) / stride * stride;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < top; c += stride) {
+    unsigned gone = 0;   // bit q: item 16 c + q
+    const int base = c * 16;
+    if (base + 16 <= n) {
+      const uint4 a = reinterpret_cast<const uint4*>(seen)[c], b = reinterpret_cast<const uint4*>(keep)[c];
+      if (a.x != b.x || a.y != b.y || a.z != b.z || a.w != b.w) {
+        for (int q = 0; q < 16; ++q)
+          if (seen[base + q] && !keep[base + q]) gone |= 1u << q;
+        reinterpret_cast<uint4*>(seen)[c] = b;
+      }
+    } else {
+      for (int q = 0; q < 16 && base + q < n; ++q) {
+        if (seen[base + q] && !keep[base + q]) gone |= 1u << q;
+        seen[base + q] = keep[base + q];
       }
     }
-    for (int off = 16; off; off >>= 1) left += __shfl_down_sync(0xffffffffu, left, off);
-    if (lane == 0) {
-      if (total) atomicAdd(total, 0ULL - (unsigned long long)degree[r]);
-      if (cross_total && left) atomicAdd(cross_total, 0ULL - (unsigned long long)left);
-      degree[r] = 0; empty[r] = 0; singleton[r] = 0; support[r] = -1; coefficient[r] = 0.0;
+    if (!__any_sync(0xffffffffu, gone != 0)) continue;
+    const int mine = __popc(gone);
+    int incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int peer = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += peer;
+    }
+    int at = 0;
+    if (lane == 31) at = atomicAdd(counter, incl);
+    at = __shfl_sync(0xffffffffu, at, 31) + incl - mine;
+    for (unsigned g = gone; g; g &= g - 1) list[at++] = base + __ffs(g) - 1;
+  }
+}
+// Deleted rows to list[0 ..], deleted columns to list[m ..]; `counters` holds
+// their numbers (zero at launch).
+__global__ void inc_deleted(int m, int n, uint8_t* __restrict__ seen_row, const uint8_t* __restrict__ keep_row,
+                            uint8_t* __restrict__ seen_col, const uint8_t* __restrict__ keep_col,
+                            int32_t* __restrict__ list, int32_t* counters) {
+  find_deleted(m, seen_row, keep_row, list, counters);
+  find_deleted(n, seen_col, keep_col, list + m, counters + 1);
+}
+
+// One side's arrays of the statistics.
+struct SideStats {
+  const offset_t* ptr;
+  const int32_t* idx;
+  const double* val;
+  const uint8_t* keep;
+  int32_t* degree;
+  uint8_t *empty, *singleton;
+  int32_t* support;
+  double* coefficient;
+  uint8_t* dirty;
+};
+
+// Deleted rows by the first half of the blocks, deleted columns by the rest
+// (the halves touch different items: a deleted item's own statistics, and the
+// degrees of kept items of the other side).  Eight lanes per deleted item: its
+// own statistics are reset, and every still-kept item it touches loses one
+// degree and is marked dirty.  The live total drops by a deleted row's old
+// degree and, for a deleted column, by one per kept row it leaves; added up in
+// registers, one atomic per warp (an atomic per item on the one total took 152
+// us when 0.8M rows went at once, on the QAP N = 30 relaxation).
+__global__ void __launch_bounds__(kThreads) inc_walk(int m, const int32_t* __restrict__ list,
+                                                     const int32_t* __restrict__ counters, SideStats rows,
+                                                     SideStats cols, unsigned long long* live_nnz) {
+  const int half = gridDim.x / 2;
+  const bool row_side = int(blockIdx.x) < half;
+  const SideStats& outer = row_side ? rows : cols;
+  const SideStats& inner = row_side ? cols : rows;
+  const int32_t* deleted = row_side ? list : list + m;
+  const int count = counters[row_side ? 0 : 1];
+  const int gl = threadIdx.x & 7;
+  const int block = row_side ? int(blockIdx.x) : int(blockIdx.x) - half;
+  const int blocks = row_side ? half : int(gridDim.x) - half;
+  unsigned long long dropped = 0;
+  for (int w = block * (kThreads / 8) + (threadIdx.x >> 3); w < count; w += blocks * (kThreads / 8)) {
+    const int r = deleted[w];
+    for (offset_t p = outer.ptr[r] + gl; p < outer.ptr[r + 1]; p += 8) {
+      const int c = outer.idx[p];
+      if (inner.keep[c]) {
+        atomicSub(inner.degree + c, 1);
+        inner.dirty[c] = 1;
+        if (!row_side) ++dropped;
+      }
+    }
+    if (gl == 0) {
+      if (row_side) dropped += (unsigned long long)outer.degree[r];
+      outer.degree[r] = 0; outer.empty[r] = 0; outer.singleton[r] = 0; outer.support[r] = -1;
+      outer.coefficient[r] = 0.0;
     }
   }
+  for (int off = 16; off; off >>= 1) dropped += __shfl_down_sync(0xffffffffu, dropped, off);
+  if ((threadIdx.x & 31) == 0 && dropped) atomicAdd(live_nnz, 0ULL - dropped);
 }
 
 // Flags of the dirty kept items; a degree-1 item finds its only live entry.
-__global__ void inc_fix(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                        const double* __restrict__ val, const uint8_t* __restrict__ keep_outer,
-                        const uint8_t* __restrict__ keep_inner, uint8_t* __restrict__ dirty,
-                        const int32_t* __restrict__ degree, uint8_t* __restrict__ empty,
-                        uint8_t* __restrict__ singleton, int32_t* __restrict__ support,
-                        double* __restrict__ coefficient) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-    if (!dirty[r]) continue;
-    dirty[r] = 0;
-    if (!keep_outer[r]) continue;
-    const int d = degree[r];
-    empty[r] = d == 0;
-    singleton[r] = d == 1;
-    int sup = -1;
-    double coef = 0.0;
-    if (d == 1)
-      for (offset_t p = ptr[r]; p < ptr[r + 1]; ++p)
-        if (keep_inner[idx[p]]) { sup = idx[p]; coef = val[p]; }
-    support[r] = sup;
-    coefficient[r] = coef;
+// Four items per thread (most dirty bytes are clear).
+__device__ __forceinline__ void fix_dirty(int n, const SideStats& outer, const uint8_t* __restrict__ keep_inner) {
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c * 4 < n; c += gridDim.x * blockDim.x) {
+    const int base = c * 4;
+    if (base + 4 <= n && reinterpret_cast<const uint32_t*>(outer.dirty)[c] == 0) continue;
+    for (int r = base; r < base + 4 && r < n; ++r) {
+      if (!outer.dirty[r]) continue;
+      outer.dirty[r] = 0;
+      if (!outer.keep[r]) continue;
+      const int d = outer.degree[r];
+      outer.empty[r] = d == 0;
+      outer.singleton[r] = d == 1;
+      int sup = -1;
+      double coef = 0.0;
+      if (d == 1)
+        for (offset_t p = outer.ptr[r]; p < outer.ptr[r + 1]; ++p)
+          if (keep_inner[outer.idx[p]]) { sup = outer.idx[p]; coef = outer.val[p]; }
+      outer.support[r] = sup;
+      outer.coefficient[r] = coef;
+    }
+  }
+}
+__global__ void inc_fix(int m, int n, SideStats rows, SideStats cols, int32_t* __restrict__ counters) {
+  if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;   // for the next refresh
+  fix_dirty(m, rows, cols.keep);
+  fix_dirty(n, cols, rows.keep);
+}
+
+// Statistics of a model all of whose rows and columns are kept: the degrees
+// are the stored lengths, so nothing but the row pointers (and a one-entry
+// item's entry) is read.
+__device__ __forceinline__ void full_item(int r, const SideStats& s, uint8_t* __restrict__ seen) {
+  const offset_t first = s.ptr[r];
+  const int d = int(s.ptr[r + 1] - first);
+  s.degree[r] = d;
+  s.empty[r] = d == 0;
+  s.singleton[r] = d == 1;
+  s.support[r] = d == 1 ? s.idx[first] : -1;
+  s.coefficient[r] = d == 1 ? s.val[first] : 0.0;
+  s.dirty[r] = 0;
+  seen[r] = 1;
+}
+__global__ void stats_of_full_model(int m, int n, offset_t nnz, SideStats rows, SideStats cols,
+                                    uint8_t* __restrict__ seen_row, uint8_t* __restrict__ seen_col,
+                                    unsigned long long* __restrict__ live_nnz, int32_t* __restrict__ counters) {
+  const int top = n > m ? n : m;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
+    if (k == 0) {
+      *live_nnz = (unsigned long long)nnz;
+      counters[0] = counters[1] = 0;
+    }
+    if (k < m) full_item(k, rows, seen_row);
+    if (k < n) full_item(k, cols, seen_col);
   }
 }
 
@@ -698,38 +784,33 @@ void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan) {
   // refresh_live_stats (gpu_presolve_kernels.cu:493-517).
   auto s = ctx().stream;
   const int m = lp.m(), n = lp.n();
-  if (!st.valid) {
+  const SideStats rows{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, st.row_nnz.p, st.empty_row.p, st.singleton_row.p,
+                       st.srow_col.p, st.srow_val.p, st.dirty_row.p};
+  const SideStats cols{lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_col.p, st.col_nnz.p, st.empty_col.p,
+                       st.singleton_col.p, st.scol_row.p, st.scol_val.p, st.dirty_col.p};
+  if (!st.valid && plan.all_kept && std::max(m, n) > 0) {
     // A full recount normally follows a fresh plan, whose masks keep every
-    // row and column (the host knows: Plan::all_kept): then the counts are
-    // the stored lengths, and the sweeps run without masks (no index or mask
-    // reads), with the same results.
-    const uint8_t* keep_row = plan.all_kept ? nullptr : plan.keep_row.p;
-    const uint8_t* keep_col = plan.all_kept ? nullptr : plan.keep_col.p;
+    // row and column (the host knows: Plan::all_kept).
+    GPP_LAUNCH_BYTES(stats_of_full_model, 22.0 * (double(m) + n), grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m,
+                     n, lp.A.nnz, rows, cols, st.seen_row.p, st.seen_col.p, st.live_nnz.p, st.counters.p);
+  } else if (!st.valid) {
     st.live_nnz.zero();
-    live_stats_side(lp.A, keep_row, keep_col, st.row_nnz.p, st.empty_row.p, st.singleton_row.p, st.srow_col.p,
-                    st.srow_val.p, st.live_nnz.p, s);
-    live_stats_side(lp.AT, keep_col, keep_row, st.col_nnz.p, st.empty_col.p, st.singleton_col.p, st.scol_row.p,
-                    st.scol_val.p, nullptr, s);
-  } else {
+    st.dirty_row.zero();
+    st.dirty_col.zero();
     st.counters.zero();
-    GPP_LAUNCH(inc_deleted, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n, st.seen_row.p, plan.keep_row.p,
-               st.seen_col.p, plan.keep_col.p, st.deleted.p, st.counters.p);
-    const int g = kNumSMs * 8;
-    GPP_LAUNCH(inc_walk, g, kThreads, 0, s, st.deleted.p, st.counters.p, lp.A.ptr, lp.A.idx, plan.keep_col.p,
-               st.row_nnz.p, st.empty_row.p, st.singleton_row.p, st.srow_col.p, st.srow_val.p, st.col_nnz.p,
-               st.dirty_col.p, st.live_nnz.p, nullptr);
-    GPP_LAUNCH(inc_walk, g, kThreads, 0, s, st.deleted.p + m, st.counters.p + 1, lp.AT.ptr, lp.AT.idx,
-               plan.keep_row.p, st.col_nnz.p, st.empty_col.p, st.singleton_col.p, st.scol_row.p, st.scol_val.p,
-               st.row_nnz.p, st.dirty_row.p, nullptr, st.live_nnz.p);
-    GPP_LAUNCH(inc_fix, grid_stride_blocks(m), kThreads, 0, s, m, lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p,
-               plan.keep_col.p, st.dirty_row.p, st.row_nnz.p, st.empty_row.p, st.singleton_row.p, st.srow_col.p,
-               st.srow_val.p);
-    GPP_LAUNCH(inc_fix, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_col.p,
-               plan.keep_row.p, st.dirty_col.p, st.col_nnz.p, st.empty_col.p, st.singleton_col.p, st.scol_row.p,
-               st.scol_val.p);
+    live_stats_side(lp.A, plan.keep_row.p, plan.keep_col.p, st.row_nnz.p, st.empty_row.p, st.singleton_row.p,
+                    st.srow_col.p, st.srow_val.p, st.live_nnz.p, s);
+    live_stats_side(lp.AT, plan.keep_col.p, plan.keep_row.p, st.col_nnz.p, st.empty_col.p, st.singleton_col.p,
+                    st.scol_row.p, st.scol_val.p, nullptr, s);
+    st.seen_row.copy_from(plan.keep_row.p, size_t(m));
+    st.seen_col.copy_from(plan.keep_col.p, size_t(n));
+  } else {
+    GPP_LAUNCH_BYTES(inc_deleted, 2.0 * (double(m) + n), grid_stride_blocks(std::max(m, n) / 16 + 1), kThreads, 0, s, m,
+                     n, st.seen_row.p, plan.keep_row.p, st.seen_col.p, plan.keep_col.p, st.deleted.p, st.counters.p);
+    const int g = 2 * std::max(1, std::min(kNumSMs * 4, (std::max(m, n) + kThreads / 8 - 1) / (kThreads / 8)));
+    GPP_LAUNCH(inc_walk, g, kThreads, 0, s, m, st.deleted.p, st.counters.p, rows, cols, st.live_nnz.p);
+    GPP_LAUNCH(inc_fix, grid_stride_blocks(std::max(m, n) / 4 + 1), kThreads, 0, s, m, n, rows, cols, st.counters.p);
   }
-  st.seen_row.copy_from(plan.keep_row.p, size_t(m));
-  st.seen_col.copy_from(plan.keep_col.p, size_t(n));
   st.valid = true;
 }
 

@@ -369,21 +369,6 @@ __global__ void check_csr_structure(int rows, int cols, offset_t nnz, const offs
   }
 }
 
-__global__ void gather_kernel(double* __restrict__ dst, const double* __restrict__ src,
-                              const int32_t* __restrict__ map, int32_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const int k = map[i];
-    if (k >= 0) dst[k] = src[i];
-  }
-}
-__global__ void compose_kernel(int32_t* __restrict__ next, const int32_t* __restrict__ prev,
-                               const int32_t* __restrict__ map, int32_t n) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const int k = map[i];
-    if (k >= 0) next[k] = prev[i];
-  }
-}
-
 }  // namespace
 
 // Old -> new map of a mask, straight from its bytes: a kept item's rank, -1
@@ -536,14 +521,6 @@ bool rows_strictly_sorted(const DevCsr& M, cudaStream_t s) {
              M.idx, bad.p);
   sch.sorted = read_scalar(bad.p) == 0 ? 1 : 0;
   return sch.sorted != 0;
-}
-
-void gather_by_map(double* dst, const double* src, const int32_t* old_to_new, int32_t n_old, cudaStream_t s) {
-  GPP_LAUNCH(gather_kernel, grid_stride_blocks(n_old), kThreads, 0, s, dst, src, old_to_new, n_old);
-}
-
-void compose_map(int32_t* next, const int32_t* prev, const int32_t* old_to_new, int32_t n_old, cudaStream_t s) {
-  GPP_LAUNCH(compose_kernel, grid_stride_blocks(n_old), kThreads, 0, s, next, prev, old_to_new, n_old);
 }
 
 void free_csr(DevCsr& M) {

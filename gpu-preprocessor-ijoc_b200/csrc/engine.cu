@@ -26,8 +26,55 @@ void WorkingLp::free_owned() {
 
 namespace {
 
-__global__ void fill_u8(uint8_t* p, int n, uint8_t v) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
+// A model's vectors: columns' c, l, u and rows' AL, AU.
+struct Vectors {
+  double *c, *l, *u, *AL, *AU;
+};
+
+// A fresh plan in one launch: all rows and columns kept, the vectors copied.
+__global__ void fresh_plan(int m, int n, Vectors from, Vectors to, uint8_t* __restrict__ keep_row,
+                           uint8_t* __restrict__ keep_col) {
+  const int top = n > m ? n : m;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
+    if (k < n) {
+      keep_col[k] = 1;
+      to.c[k] = from.c[k];
+      to.l[k] = from.l[k];
+      to.u[k] = from.u[k];
+    }
+    if (k < m) {
+      keep_row[k] = 1;
+      to.AL[k] = from.AL[k];
+      to.AU[k] = from.AU[k];
+    }
+  }
+}
+
+// The kept rows' and columns' vectors and original ids to their new places,
+// one launch for all of them.
+__global__ void gather_kept(int m, int n, const int32_t* __restrict__ rmap, const int32_t* __restrict__ cmap,
+                            Vectors from, Vectors to, const int32_t* __restrict__ rows, int32_t* __restrict__ rows_to,
+                            const int32_t* __restrict__ cols, int32_t* __restrict__ cols_to) {
+  const int top = n > m ? n : m;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
+    if (k < n) {
+      const int j = cmap[k];
+      if (j >= 0) {
+        to.c[j] = from.c[k];
+        to.l[j] = from.l[k];
+        to.u[j] = from.u[k];
+        if (cols_to) cols_to[j] = cols[k];
+      }
+    }
+    if (k < m) {
+      const int i = rmap[k];
+      if (i >= 0) {
+        to.AL[i] = from.AL[k];
+        to.AU[i] = from.AU[k];
+        if (rows_to) rows_to[i] = rows[k];
+      }
+    }
+  }
 }
 
 struct Engine {
@@ -46,18 +93,20 @@ struct Engine {
   Engine(const gpp_params& params, PresolveOutput& o) : p(params), out(o) {}
 
   cudaStream_t s() const { return ctx().stream; }
+  static Vectors vectors(const WorkingLp& lp) { return {lp.c, lp.l, lp.u, lp.AL, lp.AU}; }
+  static Vectors vectors(const Plan& pl) { return {pl.c.p, pl.l.p, pl.u.p, pl.AL.p, pl.AU.p}; }
 
   void init_plan(Plan& pl) {
     const int m = cur.m(), n = cur.n();
     pl.keep_row.alloc(size_t(m), s());
     pl.keep_col.alloc(size_t(n), s());
-    GPP_LAUNCH(fill_u8, grid_stride_blocks(m), kThreads, 0, s(), pl.keep_row.p, m, uint8_t(1));
-    GPP_LAUNCH(fill_u8, grid_stride_blocks(n), kThreads, 0, s(), pl.keep_col.p, n, uint8_t(1));
-    pl.c.alloc(size_t(n), s()); pl.c.copy_from(cur.c, size_t(n));
-    pl.l.alloc(size_t(n), s()); pl.l.copy_from(cur.l, size_t(n));
-    pl.u.alloc(size_t(n), s()); pl.u.copy_from(cur.u, size_t(n));
-    pl.AL.alloc(size_t(m), s()); pl.AL.copy_from(cur.AL, size_t(m));
-    pl.AU.alloc(size_t(m), s()); pl.AU.copy_from(cur.AU, size_t(m));
+    pl.c.alloc(size_t(n), s());
+    pl.l.alloc(size_t(n), s());
+    pl.u.alloc(size_t(n), s());
+    pl.AL.alloc(size_t(m), s());
+    pl.AU.alloc(size_t(m), s());
+    GPP_LAUNCH_BYTES(fresh_plan, 49.0 * n + 33.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s(), m, n,
+                     vectors(cur), vectors(pl), pl.keep_row.p, pl.keep_col.p);
     pl.all_kept = true;
   }
   void prepare() {
@@ -168,11 +217,8 @@ struct Engine {
     const auto [m_new, n_new] = build_old_to_new_pair(pl.keep_row.p, m, rmap.p, pl.keep_col.p, n, cmap.p, s());
     if (cur.owns && !pl.has_new_A && m_new == m && n_new == n) {
       capture_tape(r, pl.tape);
-      check(cudaMemcpyAsync(cur.c, pl.c.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s()), "commit c");
-      check(cudaMemcpyAsync(cur.l, pl.l.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s()), "commit l");
-      check(cudaMemcpyAsync(cur.u, pl.u.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s()), "commit u");
-      check(cudaMemcpyAsync(cur.AL, pl.AL.p, sizeof(double) * m, cudaMemcpyDeviceToDevice, s()), "commit AL");
-      check(cudaMemcpyAsync(cur.AU, pl.AU.p, sizeof(double) * m, cudaMemcpyDeviceToDevice, s()), "commit AU");
+      GPP_LAUNCH_BYTES(gather_kept, 52.0 * n + 36.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s(), m, n,
+                       rmap.p, cmap.p, vectors(pl), vectors(cur), nullptr, nullptr, nullptr, nullptr);
       cur.obj += pl.obj_delta;
       return;
     }
@@ -198,11 +244,11 @@ struct Engine {
       next.a_sorted = cur.a_sorted;
     }
     next.at_sorted = 1;
-    next.c = dalloc<double>(size_t(n_new)); gather_by_map(next.c, pl.c.p, cmap.p, n, s());
-    next.l = dalloc<double>(size_t(n_new)); gather_by_map(next.l, pl.l.p, cmap.p, n, s());
-    next.u = dalloc<double>(size_t(n_new)); gather_by_map(next.u, pl.u.p, cmap.p, n, s());
-    next.AL = dalloc<double>(size_t(m_new)); gather_by_map(next.AL, pl.AL.p, rmap.p, m, s());
-    next.AU = dalloc<double>(size_t(m_new)); gather_by_map(next.AU, pl.AU.p, rmap.p, m, s());
+    next.c = dalloc<double>(size_t(n_new));
+    next.l = dalloc<double>(size_t(n_new));
+    next.u = dalloc<double>(size_t(n_new));
+    next.AL = dalloc<double>(size_t(m_new));
+    next.AU = dalloc<double>(size_t(m_new));
     next.obj = cur.obj + pl.obj_delta;
     // update_device_recovery (device_recovery.cu:892-975).
     capture_tape(r, pl.tape);
@@ -215,15 +261,18 @@ struct Engine {
       pl.varpair.reset();
     }
     if (!cleanup_captured && n_new != n) append_fixed(r, pl.keep_col.p, nullptr, pl.l.p, pl.u.p, n);
+    // The vectors and, where the maps change, the original ids.
+    DBuf<int32_t> rows, cols;
+    if (m_new != r.m) rows.alloc(size_t(m_new), s());
+    if (n_new != r.n) cols.alloc(size_t(n_new), s());
+    GPP_LAUNCH_BYTES(gather_kept, 28.0 * n + 20.0 * m + 28.0 * n_new + 20.0 * m_new, grid_stride_blocks(std::max(m, n)),
+                     kThreads, 0, s(), m, n, rmap.p, cmap.p, vectors(pl), vectors(next), r.rows.p, rows.p, r.cols.p,
+                     cols.p);
     if (m_new != r.m) {
-      DBuf<int32_t> rows(size_t(m_new), s());
-      compose_map(rows.p, r.rows.p, rmap.p, m, s());
       r.rows = std::move(rows);
       r.m = m_new;
     }
     if (n_new != r.n) {
-      DBuf<int32_t> cols(size_t(n_new), s());
-      compose_map(cols.p, r.cols.p, cmap.p, n, s());
       r.cols = std::move(cols);
       r.n = n_new;
     }

@@ -218,10 +218,6 @@ void transpose_csr_into(const DevCsr& M, const DevCsr& t, cudaStream_t s);
 // non-decreasing pointers and inner indices in [0, cols).  One readback.
 bool csr_structure_valid(const DevCsr& M, cudaStream_t s);
 bool rows_strictly_sorted(const DevCsr& M, cudaStream_t s);
-void gather_by_map(double* dst, const double* src, const int32_t* old_to_new, int32_t n_old,
-                   cudaStream_t s);
-void compose_map(int32_t* next, const int32_t* prev, const int32_t* old_to_new, int32_t n_old,
-                 cudaStream_t s);
 void free_csr(DevCsr& M);
 
 // recovery.cu

@@ -3,6 +3,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <thread>
 
 #include <algorithm>
 #include <chrono>
@@ -40,9 +41,13 @@ Context::Context() {
   check(cudaMallocHost(reinterpret_cast<void**>(&host_status), sizeof(int32_t) * kStatusWords),
         "cudaMallocHost status");
   check(cudaMallocHost(reinterpret_cast<void**>(&host_scalar), 16), "cudaMallocHost scalar");
-  check(cudaMallocHost(reinterpret_cast<void**>(&host_later), sizeof(unsigned long long)), "cudaMallocHost later");
   check(cudaMallocHost(reinterpret_cast<void**>(&host_error), sizeof(int32_t)), "cudaMallocHost error");
   *host_error = 0;
+  check(cudaMallocHost(reinterpret_cast<void**>(&mail), sizeof(Mailbox) * (1 + kNnzBoxes)), "cudaMallocHost mail");
+  std::memset(static_cast<void*>(mail), 0, sizeof(Mailbox) * (1 + kNnzBoxes));
+  nnz_mail = mail + 1;
+  check(cudaMalloc(reinterpret_cast<void**>(&report_words), sizeof(int32_t) * 16), "cudaMalloc report");
+  check(cudaMemsetAsync(report_words, 0, sizeof(int32_t) * 16, stream), "report words");
 }
 
 void Context::sync(const char* label) {
@@ -54,16 +59,46 @@ void Context::sync(const char* label) {
     check(cudaStreamSynchronize(stream), label);
     profile_sync(label, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
   }
-  if (*static_cast<volatile int32_t*>(host_error)) {
-    *host_error = 0;
-    throw CudaError(std::string(label) + ": a block's bounded wait for its predecessors ran out");
+  raise_device_error(label);
+}
+
+Report Context::open_report(int count) {
+  return Report{report_words, reinterpret_cast<unsigned int*>(report_words + 15), mail, ++mail_seq, count, false};
+}
+Report Context::open_report(int count, int32_t* words) {
+  return Report{words, reinterpret_cast<unsigned int*>(report_words + 15), mail, ++mail_seq, count, true};
+}
+
+const volatile int64_t* Context::await(const Mailbox* box, uint32_t seq, const char* where) {
+  if (box->seq != seq) ++sync_counter();
+  const auto t0 = profiling() ? std::chrono::steady_clock::now() : std::chrono::steady_clock::time_point();
+  for (uint64_t polls = 1; box->seq != seq; ++polls) {
+    if (polls % 4096 == 0) {
+      const cudaError_t e = cudaStreamQuery(stream);
+      if (e == cudaSuccess && box->seq != seq) throw CudaError(std::string(where) + ": the kernel posted no answer");
+      if (e != cudaSuccess && e != cudaErrorNotReady) check(e, where);
+    }
+    if (polls > 4096 && polls % 64 == 0) std::this_thread::yield();
+    __builtin_ia32_pause();
   }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  if (profiling())
+    profile_sync(where, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+  raise_device_error(where);
+  return box->words;
+}
+
+void Context::raise_device_error(const char* where) {
+  if (!*static_cast<volatile int32_t*>(host_error)) return;
+  *host_error = 0;
+  throw CudaError(std::string(where) + ": a block's bounded wait for its predecessors ran out");
 }
 
 Context::~Context() {
+  if (mail) cudaFreeHost(mail);
+  if (report_words) cudaFree(report_words);
   if (host_status) cudaFreeHost(host_status);
   if (host_scalar) cudaFreeHost(host_scalar);
-  if (host_later) cudaFreeHost(host_later);
   if (host_error) cudaFreeHost(host_error);
   if (side) cudaStreamDestroy(side);
   if (stream) cudaStreamDestroy(stream);
@@ -224,18 +259,43 @@ LookbackSpace::LookbackSpace(size_t count, cudaStream_t s) {
 }
 
 namespace {
-__global__ void det_sum_chunks(const double* __restrict__ v, int64_t n, double* __restrict__ out) {
+// Chunk totals, then (the last block to finish) their sum in chunk order,
+// posted to the host.
+__global__ void __launch_bounds__(kThreads)
+det_sum_kernel(const double* __restrict__ v, const uint8_t* __restrict__ mask, int64_t n, double* chunk_totals,
+               unsigned int* done, Mailbox* mail, uint32_t seq) {
   __shared__ double sm[kThreads];
+  __shared__ bool last;
   const int64_t base = int64_t(blockIdx.x) * 2048;
   double acc = 0.0;
-  for (int64_t k = base + threadIdx.x; k < n && k < base + 2048; k += kThreads) acc += v[k];
+  for (int64_t k = base + threadIdx.x; k < n && k < base + 2048; k += kThreads) acc += mask && !mask[k] ? 0.0 : v[k];
   sm[threadIdx.x] = acc;
   __syncthreads();
   for (int h = kThreads / 2; h > 0; h >>= 1) {
     if (threadIdx.x < unsigned(h)) sm[threadIdx.x] = sm[threadIdx.x] + sm[threadIdx.x + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = sm[0];
+  if (threadIdx.x == 0) {
+    chunk_totals[blockIdx.x] = sm[0];
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double total = 0.0;
+  for (int first = 0; first < int(gridDim.x); first += kThreads) {
+    const int c = first + int(threadIdx.x);
+    sm[threadIdx.x] = c < int(gridDim.x) ? __ldcg(chunk_totals + c) : 0.0;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int k = 0; k < kThreads && first + k < int(gridDim.x); ++k) total += sm[k];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    *done = 0;
+    post_values(mail, seq, __double_as_longlong(total));
+  }
 }
 }  // namespace
 
@@ -245,8 +305,25 @@ void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, cudaStream_t
       [out] __device__(int64_t i, const int32_t(&before)[1], const int32_t(&)[1]) { out[i] = before[0]; },
       [out, n] __device__(const int32_t(&sum)[1]) { out[n] = sum[0]; }, s);
 }
-void exclusive_scan_pair_i64(const int64_t* a, int64_t* a_out, const int64_t* b, int64_t* b_out, int64_t n,
-                             cudaStream_t s) {
+int32_t exclusive_scan_total(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s, const char* where) {
+  auto& c = ctx();
+  Mailbox* mail = c.mail;
+  const uint32_t seq = c.open_mail();
+  scan_items<int32_t, 1>(
+      n, [in] __device__(int64_t i, int32_t(&v)[1]) { v[0] = in[i]; },
+      [out] __device__(int64_t i, const int32_t(&before)[1], const int32_t(&)[1]) { out[i] = before[0]; },
+      [=] __device__(const int32_t(&sum)[1]) {
+        out[n] = sum[0];
+        post_values(mail, seq, sum[0]);
+      },
+      s);
+  return int32_t(c.await(mail, seq, where)[0]);
+}
+std::pair<int64_t, int64_t> exclusive_scan_pair_i64(const int64_t* a, int64_t* a_out, const int64_t* b, int64_t* b_out,
+                                                    int64_t n, cudaStream_t s, const char* where) {
+  auto& c = ctx();
+  Mailbox* mail = c.mail;
+  const uint32_t seq = c.open_mail();
   scan_items<int64_t, 2>(
       n,
       [=] __device__(int64_t i, int64_t(&v)[2]) {
@@ -260,38 +337,23 @@ void exclusive_scan_pair_i64(const int64_t* a, int64_t* a_out, const int64_t* b,
       [=] __device__(const int64_t(&sum)[2]) {
         a_out[n] = sum[0];
         b_out[n] = sum[1];
+        post_values(mail, seq, sum[0], sum[1]);
       },
       s);
+  const volatile int64_t* t = c.await(mail, seq, where);
+  return {t[0], t[1]};
 }
 
-double det_sum(const double* v, int64_t n, cudaStream_t s) {
+double det_sum(const double* v, const uint8_t* mask, int64_t n, cudaStream_t s) {
   if (n <= 0) return 0.0;
+  auto& c = ctx();
   const int64_t chunks = (n + 2047) / 2048;
   DBuf<double> part(size_t(chunks), s);
-  GPP_LAUNCH(det_sum_chunks, int(chunks), kThreads, 0, s, v, n, part.p);
-  std::vector<double> h(static_cast<size_t>(chunks));
-  check(cudaMemcpyAsync(h.data(), part.p, sizeof(double) * size_t(chunks), cudaMemcpyDeviceToHost, s), "det_sum d2h");
-  ++sync_counter();
-  check(cudaStreamSynchronize(s), "det_sum sync");
-  double total = 0.0;
-  for (double x : h) total += x;
-  return total;
-}
-
-double det_sum_sparse(std::vector<std::pair<int64_t, double>> entries) {
-  std::sort(entries.begin(), entries.end(),
-            [](const std::pair<int64_t, double>& a, const std::pair<int64_t, double>& b) { return a.first < b.first; });
-  double total = 0.0;
-  size_t k = 0;
-  while (k < entries.size()) {
-    const int64_t chunk = entries[k].first / 2048;
-    double slot[kThreads] = {};
-    for (; k < entries.size() && entries[k].first / 2048 == chunk; ++k)
-      slot[entries[k].first % kThreads] += entries[k].second;
-    for (int h = kThreads / 2; h > 0; h >>= 1)
-      for (int t = 0; t < h; ++t) slot[t] = slot[t] + slot[t + h];
-    total += slot[0];
-  }
+  const Report r = c.open_report(1);
+  GPP_LAUNCH(det_sum_kernel, int(chunks), kThreads, 0, s, v, mask, n, part.p, r.done, r.mail, r.seq);
+  const int64_t bits = c.await(r)[0];
+  double total;
+  std::memcpy(&total, &bits, sizeof(total));
   return total;
 }
 

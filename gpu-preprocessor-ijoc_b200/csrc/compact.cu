@@ -372,28 +372,33 @@ __global__ void check_csr_structure(int rows, int cols, offset_t nnz, const offs
 }  // namespace
 
 // Old -> new map of a mask, straight from its bytes: a kept item's rank, -1
-// for a dropped one; *count receives the number kept.
-void map_kept(const uint8_t* keep, int32_t n, int32_t* map, int32_t* count, cudaStream_t s) {
-  select_items(
-      n, [keep] __device__(int64_t i) { return keep[i] != 0; },
-      [map] __device__(int64_t i, int at, bool kept) { map[i] = kept ? at : -1; }, count, s);
-}
-
+// for a dropped one; returns the number kept.
 int32_t build_old_to_new(const uint8_t* keep, int32_t n, int32_t* old_to_new, cudaStream_t s) {
-  if (n == 0) return 0;
-  DBuf<int32_t> count(1, s);
-  map_kept(keep, n, old_to_new, count.p, s);
-  return read_scalar(count.p);
+  return select_and_count(
+      n, [keep] __device__(int64_t i) { return keep[i] != 0; },
+      [old_to_new] __device__(int64_t i, int at, bool kept) { old_to_new[i] = kept ? at : -1; }, s);
 }
 
 std::pair<int32_t, int32_t> build_old_to_new_pair(const uint8_t* keep_row, int32_t m, int32_t* row_map,
                                                   const uint8_t* keep_col, int32_t n, int32_t* col_map,
                                                   cudaStream_t s) {
-  Status st;
-  map_kept(keep_row, m, row_map, st.d, s);
-  map_kept(keep_col, n, col_map, st.d + 1, s);
-  const int32_t* t = st.read(2);
-  return {t[0], t[1]};
+  // Both masks in one launch, as the prefix sums of m + n items.
+  auto& c = ctx();
+  Mailbox* mail = c.mail;
+  const uint32_t seq = c.open_mail();
+  scan_items<int32_t, 2>(
+      int64_t(m) + n,
+      [=] __device__(int64_t i, int32_t(&v)[2]) {
+        if (i < m) v[0] = keep_row[i] != 0;
+        else v[1] = keep_col[i - m] != 0;
+      },
+      [=] __device__(int64_t i, const int32_t(&before)[2], const int32_t(&v)[2]) {
+        if (i < m) row_map[i] = v[0] ? before[0] : -1;
+        else col_map[i - m] = v[1] ? before[1] : -1;
+      },
+      [=] __device__(const int32_t(&sum)[2]) { post_values(mail, seq, sum[0], sum[1]); }, s);
+  const volatile int64_t* kept = c.await(mail, seq, "kept rows and columns");
+  return {int32_t(kept[0]), int32_t(kept[1])};
 }
 
 DevCsr compact_csr_queued(const DevCsr& M, const int32_t* outer_map, int32_t outer_new, const int32_t* inner_map,

@@ -124,42 +124,22 @@ struct Engine {
       stats_dirty = false;
     }
   }
-  int64_t live_nnz() {
-    if (!active) return cur.A.nnz;
-    refresh();
-    return int64_t(read_scalar(stats.live_nnz.p));
-  }
-  // The live nnz before a phase is used only once the phase is over (its
-  // progress test), after the phase's own waits: it is copied to page-locked
-  // host memory with no wait of its own, and read when needed (waiting only
-  // if no wait has happened since the copy was queued).
+  // The live nnz of the plan as it stands.  A refresh posts it to the host, so
+  // it can be asked for when it is needed: the count before a phase is used
+  // only by the progress test after it, when it has long arrived.
   struct LaterCount {
-    int64_t value = 0;
-    bool pending = false;
-    uint64_t queued_at = 0;
+    int64_t known = -1;
+    uint32_t seq = 0;
   };
   LaterCount live_nnz_later() {
-    LaterCount c;
-    if (!active) {
-      c.value = cur.A.nnz;
-      return c;
-    }
+    if (!active) return {cur.A.nnz, 0};
     refresh();
-    check(cudaMemcpyAsync(ctx().host_later, stats.live_nnz.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          s()),
-          "live nnz (later)");
-    c.pending = true;
-    c.queued_at = sync_counter();
-    return c;
+    return {stats.nnz_known, stats.nnz_seq};
   }
-  int64_t value(LaterCount& c) {
-    if (c.pending) {
-      if (sync_counter() == c.queued_at) ctx().sync("live_nnz");
-      c.value = int64_t(*ctx().host_later);
-      c.pending = false;
-    }
-    return c.value;
+  int64_t value(const LaterCount& c) const {
+    return c.known >= 0 ? c.known : ctx().await(ctx().nnz_box(c.seq), c.seq, "live nnz")[0];
   }
+  int64_t live_nnz() { return value(live_nnz_later()); }
 
   template <class F>
   bool deferred_rule(bool enabled, const char* name, F rule) {
@@ -491,7 +471,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
     // Cleanup does not use the nnz before it (outside traced runs); the other
     // phases read it after their own waits.
     Engine::LaterCount before_count;
-    if (scheduled) before_count.value = e.live_nnz();
+    if (scheduled) before_count.known = e.live_nnz();
     else if (phase != Cleanup) before_count = e.live_nnz_later();
     const auto before_nnz = [&]() { return e.value(before_count); };
     RoundRecord rec;
@@ -500,7 +480,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
       float* f = rec.features;
       f[int(phase)] = 1.0f;
       f[4] = float(round) / 32.0f;
-      f[5] = float(double(before_count.value) / double(initial_nnz_all));
+      f[5] = float(double(before_count.known) / double(initial_nnz_all));
       f[6] = float(double(removed_prev) / double(initial_nnz_all));
       f[7] = float(double(removed_prev2) / double(initial_nnz_all));
       for (int g = 0; g < kGatedRules; ++g) {
@@ -509,7 +489,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
       }
       f[20] = float(bound_only_rounds) / 8.0f;
       f[21] = float(std::log10(double(initial_nnz_all)) / 8.0);
-      f[22] = float(1.0 - double(before_count.value) / double(initial_nnz_all));
+      f[22] = float(1.0 - double(before_count.known) / double(initial_nnz_all));
       f[23] = float(double(cur.m()) / double(initial_rows));
       const std::vector<uint32_t> h = to_host(inf_hist.p, 8);
       for (int side = 0; side < 2; ++side) {
@@ -518,7 +498,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
       }
       rec.phase = int32_t(phase);
       rec.iteration = out.iterations;
-      rec.nnz_before = before_count.value;
+      rec.nnz_before = before_count.known;
       if (policy) {
         bool stop = false;
         skip = policy->decide(f, &stop);
@@ -580,7 +560,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
       rec.ran = ran; rec.changed = changed_rules; rec.nnz_after = after;
       if (trace) trace->push_back(rec);
       removed_prev2 = removed_prev;
-      removed_prev = before_count.value - after;
+      removed_prev = before_count.known - after;
       for (int g = 0; g < kGatedRules; ++g)
         if (ran >> g & 1u) { last_ran[g] = round; last_changed[g] = (changed_rules >> g & 1u) != 0; }
       ++round;

@@ -137,6 +137,10 @@ struct Stats {
   DBuf<uint8_t> empty_row, singleton_row, empty_col, singleton_col;
   DBuf<double> srow_val, scol_val;
   DBuf<unsigned long long> live_nnz;
+  // The live total as the host learns it: known, or in the context's box of
+  // this sequence number once the refresh has run.
+  int64_t nnz_known = -1;
+  uint32_t nnz_seq = 0;
   // Incremental refresh: the masks the statistics describe, the rows and
   // columns deleted since, and which of them need their flags recomputed.
   bool valid = false;

@@ -744,8 +744,10 @@ __device__ __forceinline__ void fix_dirty(int n, const SideStats& outer, const u
     }
   }
 }
-__global__ void inc_fix(int m, int n, SideStats rows, SideStats cols, int32_t* __restrict__ counters) {
+__global__ void inc_fix(int m, int n, SideStats rows, SideStats cols, int32_t* __restrict__ counters,
+                        const unsigned long long* __restrict__ live_nnz, Mailbox* box, uint32_t seq) {
   if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;   // for the next refresh
+  if (blockIdx.x == 0 && threadIdx.x == 0) post_values(box, seq, int64_t(*live_nnz));
   fix_dirty(m, rows, cols.keep);
   fix_dirty(n, cols, rows.keep);
 }
@@ -793,6 +795,7 @@ void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan) {
     // row and column (the host knows: Plan::all_kept).
     GPP_LAUNCH_BYTES(stats_of_full_model, 22.0 * (double(m) + n), grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m,
                      n, lp.A.nnz, rows, cols, st.seen_row.p, st.seen_col.p, st.live_nnz.p, st.counters.p);
+    st.nnz_known = lp.A.nnz;
   } else if (!st.valid) {
     st.live_nnz.zero();
     st.dirty_row.zero();
@@ -804,12 +807,17 @@ void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan) {
                     st.scol_row.p, st.scol_val.p, nullptr, s);
     st.seen_row.copy_from(plan.keep_row.p, size_t(m));
     st.seen_col.copy_from(plan.keep_col.p, size_t(n));
+    st.nnz_known = int64_t(read_scalar(st.live_nnz.p));
   } else {
     GPP_LAUNCH_BYTES(inc_deleted, 2.0 * (double(m) + n), grid_stride_blocks(std::max(m, n) / 16 + 1), kThreads, 0, s, m,
                      n, st.seen_row.p, plan.keep_row.p, st.seen_col.p, plan.keep_col.p, st.deleted.p, st.counters.p);
     const int g = 2 * std::max(1, std::min(kNumSMs * 4, (std::max(m, n) + kThreads / 8 - 1) / (kThreads / 8)));
     GPP_LAUNCH(inc_walk, g, kThreads, 0, s, m, st.deleted.p, st.counters.p, rows, cols, st.live_nnz.p);
-    GPP_LAUNCH(inc_fix, grid_stride_blocks(std::max(m, n) / 4 + 1), kThreads, 0, s, m, n, rows, cols, st.counters.p);
+    const uint32_t seq = ++ctx().nnz_seq;
+    GPP_LAUNCH(inc_fix, grid_stride_blocks(std::max(m, n) / 4 + 1), kThreads, 0, s, m, n, rows, cols, st.counters.p,
+               st.live_nnz.p, ctx().nnz_box(seq), seq);
+    st.nnz_known = -1;
+    st.nnz_seq = seq;
   }
   st.valid = true;
 }

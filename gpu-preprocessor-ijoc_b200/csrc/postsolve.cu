@@ -590,14 +590,14 @@ __global__ void rg_roots(int count, int32_t* parent, uint8_t* __restrict__ share
 __global__ void __launch_bounds__(kThreads) rg_replay_alone(TapeView t, int64_t lo, int count, int dual, Sol s, Model M,
                                                             int32_t* parent, const uint8_t* __restrict__ shared_root,
                                                             uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
-                                                            int32_t* counter) {
+                                                            Report report) {
   const int stride = gridDim.x * blockDim.x;
   const int64_t top = (int64_t(count) + stride - 1) / stride * stride;
   for (int64_t p = blockIdx.x * blockDim.x + threadIdx.x; p < top; p += stride) {
     const int q = int(p);
     const int r = p < count && parent[q] >= 0 ? uf_root(parent, q) : -1;
     const bool listed = r >= 0 && (r != q || shared_root[q]);
-    const int at = block_append(counter, listed);
+    const int at = block_append(report.words, listed);
     if (listed) {
       keys[at] = (uint64_t(uint32_t(r)) << 32) | uint32_t(q);
       vals[at] = q;
@@ -605,6 +605,7 @@ __global__ void __launch_bounds__(kThreads) rg_replay_alone(TapeView t, int64_t 
       replay_at(t, lo + q, s, M, dual != 0);
     }
   }
+  post_report(report);
 }
 // One thread per listed group: the thread at the group's last (newest) record
 // replays it and walks back to the group's first.
@@ -702,11 +703,10 @@ void replay_range(const TapeView& t, int m0, int n0, const Sol& s, const Model& 
                owner.p);
     return;
   }
-  // Owners, the marks of shared roots and the list's counter, cleared at once.
-  DBuf<int32_t> scratch(resources + (size_t(count) + 3) / 4 + 1, st);
+  // Owners and the marks of shared roots, cleared at once.
+  DBuf<int32_t> scratch(resources + (size_t(count) + 3) / 4, st);
   int32_t* owner = scratch.p;
   auto* shared_root = reinterpret_cast<uint8_t*>(owner + resources);
-  int32_t* counter = scratch.p + scratch.n - 1;
   DBuf<int32_t> parent(size_t(count), st), vals(size_t(count), st);
   DBuf<uint64_t> keys(size_t(count), st);
   const int g = grid_stride_blocks(count);
@@ -715,9 +715,10 @@ void replay_range(const TapeView& t, int m0, int n0, const Sol& s, const Model& 
     GPP_LAUNCH(rg_claim, g, kThreads, 0, st, t, lo, count, pass, m0, n0, M, s.x, owner, parent.p);
     GPP_LAUNCH(rg_connect, g, kThreads, 0, st, t, lo, count, pass, m0, n0, M, owner, parent.p);
     GPP_LAUNCH(rg_roots, g, kThreads, 0, st, count, parent.p, shared_root);
+    const Report report = ctx().open_report(1);
     GPP_LAUNCH(rg_replay_alone, g, kThreads, 0, st, t, lo, count, pass, s, M, parent.p, shared_root, keys.p, vals.p,
-               counter);
-    const int listed = read_scalar(counter);
+               report);
+    const int listed = int(ctx().await(report)[0]);
     if (!listed) continue;
     radix_sort_pairs(keys.p, vals.p, listed, st, (bits_up_to(count - 1) << 32) | bits_up_to(count - 1));
     GPP_LAUNCH(rg_replay_groups, grid_stride_blocks(listed), kThreads, 0, st, t, lo, listed, keys.p, pass, s, M);

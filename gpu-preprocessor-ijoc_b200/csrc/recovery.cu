@@ -184,12 +184,12 @@ void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, cons
   // One selection over the columns finds the fixed ones and packs them (into
   // arrays for all columns, as their number is not known yet); the segment
   // keeps the packed part.
-  DBuf<int32_t> idx(size_t(n) + 1, s);
+  DBuf<int32_t> idx(size_t(n), s);
   DBuf<double> val(size_t(n), s);
   const int32_t* cols = r.cols.p;
   int32_t* out_idx = idx.p;
   double* out_val = val.p;
-  select_items(
+  const int32_t count = select_and_count(
       n,
       [=] __device__(int64_t i) {
         return (!prior || prior[i]) && !keep_col[i] && isfinite(l[i]) && isfinite(u[i]) && fabs(l[i] - u[i]) <= 1e-9;
@@ -199,8 +199,7 @@ void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, cons
         out_idx[at] = cols[i];
         out_val[at] = 0.5 * (l[i] + u[i]);
       },
-      idx.p + n, s);
-  const int32_t count = read_scalar(idx.p + n);
+      s);
   if (!count) return;
   FixedSegment f;
   f.count = count;

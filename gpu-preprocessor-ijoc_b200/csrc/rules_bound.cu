@@ -135,7 +135,8 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
                                 const double* __restrict__ vmax_arr, int preserve_free_zero_cost, double zero_tol,
                                 double ft, double upper_relax, double* __restrict__ fl, double* __restrict__ fu,
                                 uint8_t* __restrict__ lch, uint8_t* __restrict__ uch, uint8_t* __restrict__ fx,
-                                double* __restrict__ fixv, int32_t* __restrict__ status) {
+                                double* __restrict__ fixv, Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 a bound moves, 4 a column is fixed
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const double lj = l[j], uj = u[j];
     if (!keep_col[j]) {
@@ -150,14 +151,14 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
     double el = lj, eu = uj;
     if (isfinite(cl)) el = fmax(el, cl);
     if (isfinite(cu)) eu = fmin(eu, cu);
-    if (el > eu + ft) { atomicMax(status + 0, 1); continue; }
+    if (el > eu + ft) { found |= 1u; continue; }
     const bool was_free = !isfinite(ref_l[j]) && !isfinite(ref_u[j]);
     const bool box = isfinite(cl) && isfinite(cu);
     const bool zero_cost = fabs(c[j]) <= zero_tol;
     const bool nearly_fixed = box && (cu <= cl || (cu - cl) * vmax <= ft);
     if (preserve_free_zero_cost && was_free && box && zero_cost && !nearly_fixed) { cl = lj; cu = uj; }
     if (isfinite(cl) && cl > lj && isfinite(uj)) {
-      if (cl >= uj + ft) { atomicMax(status + 0, 1); continue; }
+      if (cl >= uj + ft) { found |= 1u; continue; }
       if (cl >= uj || (uj - cl) * vmax <= ft) { fj = 1; fat = uj; nl = uj; nu = uj; }
     }
     if (!fj && isfinite(cl) && cl > lj) {
@@ -169,7 +170,7 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
       }
     }
     if (!fj && isfinite(cu) && cu < uj && isfinite(nl)) {
-      if (cu <= nl - ft) { atomicMax(status + 0, 1); continue; }
+      if (cu <= nl - ft) { found |= 1u; continue; }
       if (cu <= nl || (cu - nl) * vmax <= ft) { fj = 1; fat = nl; nu = nl; }
     }
     if (!fj && isfinite(cu) && cu < uj) {
@@ -180,10 +181,11 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
         uc = 1;
       }
     }
-    if (fj) { lc = uc = 0; atomicMax(status + 2, 1); }
-    if (lc || uc) atomicMax(status + 1, 1);
+    if (fj) { lc = uc = 0; found |= 4u; }
+    if (lc || uc) found |= 2u;
     fl[j] = nl; fu[j] = nu; lch[j] = lc; uch[j] = uc; fx[j] = fj; fixv[j] = fat;
   }
+  post_flags(report, found);
 }
 
 // Support rows and per-column tape sizes (reference :815-960, :970-1008).
@@ -288,7 +290,8 @@ __global__ void apply_bounds(int n, const double* __restrict__ fl, const double*
 __global__ void shift_and_empty_rows(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                                      const double* __restrict__ shift, const uint8_t* __restrict__ keep_col,
                                      uint8_t* __restrict__ keep_row, double* __restrict__ AL,
-                                     double* __restrict__ AU, double ft, int32_t* __restrict__ status) {
+                                     double* __restrict__ AU, double ft, Report report) {
+  uint32_t infeasible = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     AL[i] -= shift[i];
     AU[i] -= shift[i];
@@ -296,9 +299,10 @@ __global__ void shift_and_empty_rows(int m, const offset_t* __restrict__ ptr, co
     int cnt = 0;
     for (offset_t p = ptr[i]; p < ptr[i + 1] && cnt == 0; ++p) cnt += keep_col[idx[p]] != 0;
     if (cnt) continue;
-    if (AL[i] <= ft && AU[i] >= -ft) { keep_row[i] = 0; atomicMax(status + 4, 1); }
-    else atomicMax(status + 3, 1);
+    if (AL[i] <= ft && AU[i] >= -ft) keep_row[i] = 0;
+    else infeasible = 1;
   }
+  post_flags(report, infeasible);
 }
 
 // FixedVariable records of fixed columns: (col, kept rows...), (value, c, coefficients...).
@@ -365,8 +369,6 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   DBuf<int32_t> ni(size_t(m), s), pi(size_t(m), s);
   cl.copy_from(plan.l.p, size_t(n));
   cu.copy_from(plan.u.p, size_t(n));
-  Status st;
-  st.clear(5);
   // One packed bounds array serves the activity sweep and the candidate sweep.
   DBuf<double2> lu(size_t(n), s);
   pack_bounds(plan.l.p, plan.u.p, plan.keep_col.p, n, lu.p, s);
@@ -390,13 +392,14 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   DBuf<uint8_t> lch(size_t(n), s), uch(size_t(n), s), fx(size_t(n), s);
   const double* ref_l = plan.ref_l ? plan.ref_l : plan.l.p;
   const double* ref_u = plan.ref_u ? plan.ref_u : plan.u.p;
+  Report report = ctx().open_report(1);
   GPP_LAUNCH(finalize_kernel, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.l.p, plan.u.p, cl.p,
              cu.p, ref_l, ref_u, plan.c.p, vmax.p, int(p.bound_strengthening_preserve_free_zero_cost), p.zero_tol,
              p.feasibility_tol, p.bound_strengthening_upper_relaxation_factor, fl.p, fu.p, lch.p, uch.p, fx.p,
-             fixv.p, st.d);
-  const int32_t* f = st.read(3);
-  if (f[0]) { plan.has_infeasible = true; return; }
-  const bool changed = f[1] != 0, fixed = f[2] != 0;
+             fixv.p, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  const bool changed = (found & 2u) != 0, fixed = (found & 4u) != 0;
   if (!changed && !fixed) return;
   if (p.record_postsolve_tape && changed) {
     DBuf<int32_t> sl(size_t(n), s), su(size_t(n), s);
@@ -405,8 +408,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     GPP_LAUNCH(support_kernel, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val,
                plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, plan.l.p, plan.u.p, rs, lch.p, uch.p, fl.p,
                fu.p, p.zero_tol, p.bound_tol, support_tol, sl.p, su.p, rc.p, ic.p);
-    exclusive_scan_pair_i64(rc.p, rpos.p, ic.p, ipos.p, n, s);
-    const auto [recs, nidx] = read_scalars(rpos.p + n, ipos.p + n);
+    const auto [recs, nidx] = exclusive_scan_pair_i64(rc.p, rpos.p, ic.p, ipos.p, n, s);
     if (recs) {
       PostsolveSegment seg = make_segment(recs, nidx, 4 * recs);
       GPP_LAUNCH(pack_bound_records, grid_stride_blocks(n), kThreads, 0, s, n, lch.p, uch.p, sl.p, su.p, plan.l.p,
@@ -420,15 +422,14 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   if (fixed) {
     DBuf<double> shift(size_t(m), s);
     row_gather_shift(lp.A, lp.AT, plan.keep_row.p, fx.p, fixv.p, nullptr, shift.p, s);
+    report = ctx().open_report(1);
     GPP_LAUNCH(shift_and_empty_rows, grid_stride_blocks(m), kThreads, 0, s, m, lp.A.ptr, lp.A.idx, shift.p,
-               plan.keep_col.p, plan.keep_row.p, plan.AL.p, plan.AU.p, p.feasibility_tol, st.d);
-    const int32_t* g = st.read(5);
-    if (g[3]) { plan.has_infeasible = true; return; }
+               plan.keep_col.p, plan.keep_row.p, plan.AL.p, plan.AU.p, p.feasibility_tol, report);
+    if (ctx().await(report)[0]) { plan.has_infeasible = true; return; }
     DBuf<int64_t> rc(size_t(n) + 1, s), nz(size_t(n) + 1, s), rpos(size_t(n) + 1, s), npos(size_t(n) + 1, s);
     GPP_LAUNCH(fixed_record_sizes, grid_stride_blocks(n), kThreads, 0, s, n, fx.p, lp.AT.ptr, lp.AT.idx,
                plan.keep_row.p, rc.p, nz.p);
-    exclusive_scan_pair_i64(rc.p, rpos.p, nz.p, npos.p, n, s);
-    const auto [recs, nnz] = read_scalars(rpos.p + n, npos.p + n);
+    const auto [recs, nnz] = exclusive_scan_pair_i64(rc.p, rpos.p, nz.p, npos.p, n, s);
     PostsolveSegment seg = make_segment(recs, recs + nnz, 2 * recs + nnz);
     DBuf<double> oc(size_t(recs), s), ov(size_t(recs), s);
     GPP_LAUNCH(fixed_record_pack, grid_stride_blocks(n), kThreads, 0, s, n, fx.p, lp.AT.ptr, lp.AT.idx, lp.AT.val,

@@ -76,17 +76,12 @@ __global__ void row_gather_kernel(const int32_t* __restrict__ list, const int32_
   }
 }
 
-__global__ void mask_contrib(int n, const double* __restrict__ contrib, const uint8_t* __restrict__ entry,
-                             double* __restrict__ out) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-    out[j] = entry && !entry[j] ? 0.0 : contrib[j];
-}
-
 // --- infeasible / fixed variables ------------------------------------------
 __global__ void fixed_candidates(int n, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
                                  const double* __restrict__ u, const double* __restrict__ c, double bound_tol,
                                  uint8_t* __restrict__ fixed, double* __restrict__ fval,
-                                 double* __restrict__ contrib, double* __restrict__ radius, int32_t* __restrict__ any) {
+                                 double* __restrict__ contrib, double* __restrict__ radius, Report report) {
+  uint32_t any = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     uint8_t f = 0;
     double v = 0.0, cb = 0.0, rad = 0.0;
@@ -100,13 +95,15 @@ __global__ void fixed_candidates(int n, const uint8_t* __restrict__ keep_col, co
       }
     }
     fixed[j] = f; fval[j] = v; contrib[j] = cb; radius[j] = rad;
-    if (f) *any = 1;
+    any |= f;
   }
+  post_flags(report, any);
 }
 __global__ void fixed_filter(int n, const offset_t* __restrict__ at_ptr, const int32_t* __restrict__ at_idx,
                              const uint8_t* __restrict__ keep_row, const double* __restrict__ l,
                              const double* __restrict__ u, const double* __restrict__ row_error, double budget,
-                             uint8_t* __restrict__ fixed, double* __restrict__ contrib, int32_t* __restrict__ status) {
+                             uint8_t* __restrict__ fixed, double* __restrict__ contrib, Report report) {
+  uint32_t any = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (!fixed[j]) continue;
     bool keep_fix = true;
@@ -116,8 +113,9 @@ __global__ void fixed_filter(int n, const offset_t* __restrict__ at_ptr, const i
         if (keep_row[row] && !(row_error[row] <= budget)) { keep_fix = false; break; }
       }
     if (!keep_fix) { fixed[j] = 0; contrib[j] = 0.0; }
-    else atomicAdd(status, 1);
+    else any = 1;
   }
+  post_flags(report, any);
 }
 __global__ void fixed_apply(int n, int m, const uint8_t* __restrict__ fixed, const double* __restrict__ fval,
                             const double* __restrict__ shift, uint8_t* __restrict__ keep_col, double* __restrict__ l,
@@ -134,21 +132,23 @@ __global__ void empty_columns_classify(int n, const uint8_t* __restrict__ keep_c
                                        const double* __restrict__ c, const double* __restrict__ l,
                                        const double* __restrict__ u, double bound_tol, double zero_tol,
                                        uint8_t* __restrict__ fixed, double* __restrict__ fval,
-                                       double* __restrict__ contrib, int32_t* __restrict__ status) {
+                                       double* __restrict__ contrib, Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 unbounded, 4 fixed
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     fixed[j] = 0; fval[j] = 0.0; contrib[j] = 0.0;
     if (!(keep_col[j] && empty[j])) continue;
     const double cj = c[j], lj = l[j], uj = u[j];
-    if (lj > uj + bound_tol) { atomicMax(status + 0, 1); continue; }
-    if ((cj > zero_tol && !isfinite(lj)) || (cj < -zero_tol && !isfinite(uj))) { atomicMax(status + 1, 1); continue; }
+    if (lj > uj + bound_tol) { found |= 1u; continue; }
+    if ((cj > zero_tol && !isfinite(lj)) || (cj < -zero_tol && !isfinite(uj))) { found |= 2u; continue; }
     double v = 0.0;
     if (cj > zero_tol) v = lj;
     else if (cj < -zero_tol) v = uj;
     else if (isfinite(lj)) v = lj;
     else if (isfinite(uj)) v = uj;
     fixed[j] = 1; fval[j] = v; contrib[j] = cj * v;
-    atomicMax(status + 2, 1);
+    found |= 4u;
   }
+  post_flags(report, found);
 }
 __global__ void fix_columns(int n, const uint8_t* __restrict__ fixed, const double* __restrict__ fval,
                             uint8_t* __restrict__ keep_col, double* __restrict__ l, double* __restrict__ u) {
@@ -157,15 +157,19 @@ __global__ void fix_columns(int n, const uint8_t* __restrict__ fixed, const doub
 }
 
 // --- empty rows ----------------------------------------------------------------
-__global__ void empty_rows_kernel(int m, uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
-                                  const double* __restrict__ AL, const double* __restrict__ AU, double tol,
-                                  int32_t* __restrict__ status, int apply) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    if (!(keep_row[i] && row_nnz[i] == 0)) continue;
-    const bool feasible = AL[i] <= tol && AU[i] >= -tol;
-    if (!apply) atomicMax(status + (feasible ? 1 : 0), 1);
-    else if (feasible) keep_row[i] = 0;
-  }
+__device__ __forceinline__ bool empty_row_feasible(double lo, double hi, double tol) { return lo <= tol && hi >= -tol; }
+__global__ void empty_rows_find(int m, const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
+                                const double* __restrict__ AL, const double* __restrict__ AU, double tol,
+                                Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 removable
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+    if (keep_row[i] && row_nnz[i] == 0) found |= empty_row_feasible(AL[i], AU[i], tol) ? 2u : 1u;
+  post_flags(report, found);
+}
+__global__ void empty_rows_remove(int m, uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
+                                  const double* __restrict__ AL, const double* __restrict__ AU, double tol) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+    if (keep_row[i] && row_nnz[i] == 0 && empty_row_feasible(AL[i], AU[i], tol)) keep_row[i] = 0;
 }
 
 // --- singleton rows -----------------------------------------------------------
@@ -188,15 +192,17 @@ __global__ void singleton_row_bounds(int m, int n, const uint8_t* __restrict__ k
 }
 __global__ void singleton_rows_check(int m, int n, const double* __restrict__ cand_l, const double* __restrict__ cand_u,
                                      const double* __restrict__ l, const double* __restrict__ u,
-                                     const uint8_t* __restrict__ remove, double tol, int32_t* __restrict__ status) {
+                                     const uint8_t* __restrict__ remove, double tol, Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 a row goes, 4 a bound changes
   const int top = n > m ? n : m;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += gridDim.x * blockDim.x) {
     if (j < n) {
-      if (cand_l[j] > cand_u[j] + tol) atomicMax(status + 0, 1);
-      if (cand_l[j] != l[j] || cand_u[j] != u[j]) atomicMax(status + 2, 1);
+      if (cand_l[j] > cand_u[j] + tol) found |= 1u;
+      if (cand_l[j] != l[j] || cand_u[j] != u[j]) found |= 4u;
     }
-    if (j < m && remove[j]) atomicMax(status + 1, 1);
+    if (j < m && remove[j]) found |= 2u;
   }
+  post_flags(report, found);
 }
 __global__ void singleton_rows_commit(int m, int n, const uint8_t* __restrict__ remove, uint8_t* __restrict__ keep_row) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
@@ -223,15 +229,13 @@ double domain_objective(const double* contrib, const uint8_t* entry_keep, int32_
   // sum_cleanup_domain (cleanup_support.cuh:13-31): the sum over the rule's
   // entry domain, with the canonical deterministic reduction.
   if (n <= 0) return 0.0;
-  DBuf<double> masked(size_t(n), s);
-  GPP_LAUNCH(mask_contrib, grid_stride_blocks(n), kThreads, 0, s, n, contrib, entry_keep, masked.p);
-  return det_sum(masked.p, n, s);
+  return det_sum(contrib, entry_keep, n, s);
 }
 
 namespace {
 // What the first checks of the four rules below find on the current plan, in
-// one pass: a thread reads one column and one row and ORs the rules that may
-// act into *found (one atomic per block at most).
+// one pass: a thread reads one column and one row and flags the rules that may
+// act.
 //  - fixed variables: a kept column whose finite bounds lie within bound_tol;
 //  - empty columns: any kept empty column (fixed, infeasible or unbounded);
 //  - empty rows: any kept row without live entries;
@@ -246,7 +250,7 @@ cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ k
                      const uint8_t* __restrict__ keep_col, const double* __restrict__ l, const double* __restrict__ u,
                      const uint8_t* __restrict__ empty_col, const int32_t* __restrict__ row_nnz,
                      const uint8_t* __restrict__ singleton_row, const int32_t* __restrict__ scol,
-                     const double* __restrict__ sval, double bound_tol, double zero_tol, uint32_t* found) {
+                     const double* __restrict__ sval, double bound_tol, double zero_tol, Report report) {
   uint32_t f = 0;
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
@@ -266,13 +270,7 @@ cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ k
       }
     }
   }
-  f = __reduce_or_sync(0xffffffffu, f & rules);
-  __shared__ uint32_t block_found;
-  if (threadIdx.x == 0) block_found = 0;
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0 && f) atomicOr(&block_found, f);
-  __syncthreads();
-  if (threadIdx.x == 0 && block_found) atomicOr(found, block_found);
+  post_flags(report, f & rules);
 }
 }  // namespace
 
@@ -286,13 +284,11 @@ uint32_t cleanup_probe(const Plan& plan, const WorkingLp& lp, const Stats& stats
   if (m == 0) rules &= ~(kProbeEmptyRows | kProbeSingletonRows);
   if (!rules) return 0;
   auto s = ctx().stream;
-  Status st;
-  st.clear(1);
+  const Report report = ctx().open_report(1);
   GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 6.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n,
                    rules, plan.keep_row.p, plan.keep_col.p, plan.l.p, plan.u.p, stats.empty_col.p, stats.row_nnz.p,
-                   stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol,
-                   reinterpret_cast<uint32_t*>(st.d));
-  return uint32_t(st.read(1)[0]);
+                   stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol, report);
+  return uint32_t(ctx().await(report)[0]);
 }
 
 void rule_fixed_variables(Plan& plan, const WorkingLp& lp, const gpp_params& p) {
@@ -303,15 +299,15 @@ void rule_fixed_variables(Plan& plan, const WorkingLp& lp, const gpp_params& p) 
   DBuf<uint8_t> fixed(size_t(n), s);
   DBuf<double> fval(size_t(n), s), contrib(size_t(n), s), radius(size_t(n), s), row_err(size_t(m), s),
       shift(size_t(m), s);
-  Status st;
-  st.clear(4);
+  Report report = ctx().open_report(1);
   GPP_LAUNCH(fixed_candidates, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.l.p, plan.u.p,
-             plan.c.p, p.bound_tol, fixed.p, fval.p, contrib.p, radius.p, st.d + 1);
-  if (st.read(2)[1] == 0) return;
+             plan.c.p, p.bound_tol, fixed.p, fval.p, contrib.p, radius.p, report);
+  if (ctx().await(report)[0] == 0) return;
   row_gather_shift(lp.A, lp.AT, plan.keep_row.p, fixed.p, fval.p, radius.p, row_err.p, s);
+  report = ctx().open_report(1);
   GPP_LAUNCH(fixed_filter, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, plan.keep_row.p,
-             plan.l.p, plan.u.p, row_err.p, 0.1 * p.feasibility_tol, fixed.p, contrib.p, st.d);
-  if (st.read(1)[0] == 0) return;
+             plan.l.p, plan.u.p, row_err.p, 0.1 * p.feasibility_tol, fixed.p, contrib.p, report);
+  if (ctx().await(report)[0] == 0) return;
   row_gather_shift(lp.A, lp.AT, plan.keep_row.p, fixed.p, fval.p, nullptr, shift.p, s);
   GPP_LAUNCH(fixed_apply, grid_stride_blocks(std::max(n, m)), kThreads, 0, s, n, m, fixed.p, fval.p, shift.p,
              plan.keep_col.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p);
@@ -326,14 +322,13 @@ void rule_empty_columns(Plan& plan, const WorkingLp& lp, const Stats& stats, con
   auto s = ctx().stream;
   DBuf<uint8_t> fixed(size_t(n), s);
   DBuf<double> fval(size_t(n), s), contrib(size_t(n), s);
-  Status st;
-  st.clear(3);
+  const Report report = ctx().open_report(1);
   GPP_LAUNCH(empty_columns_classify, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, stats.empty_col.p,
-             plan.c.p, plan.l.p, plan.u.p, p.bound_tol, p.zero_tol, fixed.p, fval.p, contrib.p, st.d);
-  const int32_t* f = st.read(3);
-  if (f[0]) { plan.has_infeasible = true; return; }
-  if (f[1]) { plan.has_unbounded = true; return; }
-  if (!f[2]) return;
+             plan.c.p, plan.l.p, plan.u.p, p.bound_tol, p.zero_tol, fixed.p, fval.p, contrib.p, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  if (found & 2u) { plan.has_unbounded = true; return; }
+  if (!found) return;
   GPP_LAUNCH(fix_columns, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, fval.p, plan.keep_col.p, plan.l.p,
              plan.u.p);
   plan.obj_delta += domain_objective(contrib.p, plan.rule_entry_keep_col, n, s);
@@ -345,15 +340,14 @@ void rule_empty_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, const 
   const int m = lp.m();
   if (m == 0) return;
   auto s = ctx().stream;
-  Status st;
-  st.clear(2);
-  GPP_LAUNCH(empty_rows_kernel, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p,
-             plan.AL.p, plan.AU.p, p.feasibility_tol, st.d, 0);
-  const int32_t* f = st.read(2);
-  if (f[0]) { plan.has_infeasible = true; return; }
-  if (!f[1]) return;
-  GPP_LAUNCH(empty_rows_kernel, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p,
-             plan.AL.p, plan.AU.p, p.feasibility_tol, st.d, 1);
+  const Report report = ctx().open_report(1);
+  GPP_LAUNCH(empty_rows_find, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p, plan.AL.p,
+             plan.AU.p, p.feasibility_tol, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  if (!found) return;
+  GPP_LAUNCH(empty_rows_remove, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p, plan.AL.p,
+             plan.AU.p, p.feasibility_tol);
   plan.has_row_action = plan.has_row_deletion = plan.has_change = true;
 }
 
@@ -366,17 +360,16 @@ void rule_singleton_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, co
   DBuf<uint8_t> remove(size_t(m), s);
   cl.copy_from(plan.l.p, size_t(n));
   cu.copy_from(plan.u.p, size_t(n));
-  Status st;
-  st.clear(3);
+  const Report report = ctx().open_report(1);
   GPP_LAUNCH(singleton_row_bounds, grid_stride_blocks(m), kThreads, 0, s, m, n, plan.keep_row.p,
              stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, plan.AL.p, plan.AU.p, p.zero_tol, cl.p,
              cu.p, remove.p);
   GPP_LAUNCH(singleton_rows_check, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n, cl.p, cu.p, plan.l.p,
-             plan.u.p, remove.p, p.bound_tol, st.d);
-  const int32_t* f = st.read(3);
-  if (f[0]) { plan.has_infeasible = true; return; }
-  if (!f[1] && !f[2]) return;
-  const bool removed = f[1] != 0;
+             plan.u.p, remove.p, p.bound_tol, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  if (!found) return;
+  const bool removed = (found & 2u) != 0;
   GPP_LAUNCH(singleton_rows_commit, grid_stride_blocks(m), kThreads, 0, s, m, n, remove.p, plan.keep_row.p);
   std::swap(plan.l, cl);
   std::swap(plan.u, cu);

@@ -163,14 +163,14 @@ __global__ void dt_candidates(int m, const offset_t* __restrict__ ptr, const int
   }
 }
 
-// Indices (or `ids`) of the nonzero flags, in order; *total their number.
-void list_flagged(int count, const int32_t* flag, const int32_t* ids, int32_t* out, int32_t* total, cudaStream_t s) {
-  select_items(
+// Indices (or `ids`) of the nonzero flags, in order; returns their number.
+int32_t list_flagged(int count, const int32_t* flag, const int32_t* ids, int32_t* out, cudaStream_t s) {
+  return select_and_count(
       count, [flag] __device__(int64_t q) { return flag[q] != 0; },
       [ids, out] __device__(int64_t q, int at, bool taken) {
         if (taken) out[at] = ids ? ids[q] : int32_t(q);
       },
-      total, s);
+      s);
 }
 
 // Matching round (:989-1027): reset the owners of the active rows' columns,
@@ -217,7 +217,9 @@ __global__ void dt_apply(int sel, const int32_t* __restrict__ rows, const int32_
                          uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ kind,
                          double* __restrict__ alpha_out, double* __restrict__ beta_out,
                          double* __restrict__ obj_term, int32_t* __restrict__ rec_idx, double* __restrict__ rec_val,
-                         int32_t* st) {
+                         Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 any pair applied; word 1 counts the substitutions
+  int substituted = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sel; t += gridDim.x * blockDim.x) {
     const int row = rows[t], k = keep_c[row], e = elim_c[row];
     const double kv = keep_v[row], ev = elim_v[row];
@@ -232,7 +234,7 @@ __global__ void dt_apply(int sel, const int32_t* __restrict__ rows, const int32_
     const double nl = isfinite(ml) ? fmax(lk, ml) : lk;
     const double nu = isfinite(mu) ? fmin(uk, mu) : uk;
     kind[t] = kPairNone;
-    if (nl > nu + bound_tol) { atomicOr(st + kStInfeasible, 1); continue; }
+    if (nl > nu + bound_tol) { found |= 1u; continue; }
     alpha_out[t] = alpha;
     beta_out[t] = beta;
     if (isfinite(nl) && isfinite(nu) && nu <= nl + bound_tol) {
@@ -242,7 +244,6 @@ __global__ void dt_apply(int sel, const int32_t* __restrict__ rows, const int32_
       keep_col[k] = 0;
       kind[t] = kPairFixed;
       obj_term[t] = ck * at;
-      atomicAdd(st + kStFixed, 1);
     } else {
       l[k] = nl;
       u[k] = nu;
@@ -251,15 +252,18 @@ __global__ void dt_apply(int sel, const int32_t* __restrict__ rows, const int32_
       keep_col[e] = 0;
       kind[t] = kPairSubst;
       obj_term[t] = ce * beta;
-      atomicAdd(st + kStSubst, 1);
+      ++substituted;
       int32_t* ri = rec_idx + 4 * int64_t(t);
       ri[0] = e; ri[1] = k; ri[2] = row; ri[3] = 0;
       double* rv = rec_val + 12 * int64_t(t);
       rv[0] = ev; rv[1] = kv; rv[2] = rhs; rv[3] = le; rv[4] = ue; rv[5] = lk; rv[6] = uk;
       rv[7] = nl; rv[8] = nu; rv[9] = ce; rv[10] = 0.0; rv[11] = 0.0;
     }
-    atomicOr(st + kStAny, 1);
+    found |= 2u;
   }
+  substituted = __reduce_add_sync(0xffffffffu, substituted);
+  if ((threadIdx.x & 31) == 0 && substituted) atomicAdd(report.words + 1, substituted);
+  post_flags(report, found);
 }
 
 // DoubletonEquation record r of pair t: indices [elim, keep, row, 0], values
@@ -301,7 +305,7 @@ __global__ void dt_roles(int sel, const int32_t* __restrict__ rows, const int32_
 // Rows holding a shifting column, each listed once.
 __global__ void dt_touch(int sel, const int32_t* __restrict__ role_col, const offset_t* __restrict__ tptr,
                          const int32_t* __restrict__ tidx, uint32_t* __restrict__ claimed,
-                         int32_t* __restrict__ touched, int32_t* st) {
+                         int32_t* __restrict__ touched, int32_t* st, Report report) {
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
@@ -320,6 +324,7 @@ __global__ void dt_touch(int sel, const int32_t* __restrict__ role_col, const of
       if (take) touched[at] = r;
     }
   }
+  post_report(report);
 }
 
 // Row shift of a touched kept row: its terms added in stored column order.
@@ -714,7 +719,7 @@ void doubleton_single_row(Plan& plan, const WorkingLp& lp, const gpp_params& p) 
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
   const double zt = p.zero_tol, ratio_tol = std::fmax(1.0e-9, p.bound_tol);
-  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m), s), acc(size_t(m) + 1, s), keep_c(size_t(m), s),
+  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m), s), acc(size_t(m), s), keep_c(size_t(m), s),
       elim_c(size_t(m), s);
   DBuf<double> keep_v(size_t(m), s), elim_v(size_t(m), s);
   GPP_LAUNCH(dt_col_nnz, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p,
@@ -723,8 +728,7 @@ void doubleton_single_row(Plan& plan, const WorkingLp& lp, const gpp_params& p) 
              plan.keep_row.p, plan.keep_col.p, col_nnz.p, plan.AL.p, plan.AU.p, zt, p.bound_tol, ratio_tol,
              p.doubleton_equations_max_fill_in_proxy, lp.AT.ptr, lp.AT.idx, lp.AT.val, flag.p, keep_c.p, elim_c.p,
              keep_v.p, elim_v.p);
-  list_flagged(m, flag.p, nullptr, acc.p, acc.p + m, s);   // acc[0] is the smallest
-  if (read_scalar(acc.p + m) == 0) return;
+  if (list_flagged(m, flag.p, nullptr, acc.p, s) == 0) return;   // acc[0] is the smallest
   Status st;
   st.clear(kStWords);
   DBuf<double> meta(3, s), rec_val(12, s);
@@ -754,8 +758,7 @@ void doubleton_single_row(Plan& plan, const WorkingLp& lp, const gpp_params& p) 
   out.rows = m;
   out.cols = n;
   out.ptr = dalloc<offset_t>(size_t(m) + 1);
-  exclusive_scan_i32(cnt.p, out.ptr, m, s);
-  out.nnz = read_scalar(out.ptr + m);
+  out.nnz = exclusive_scan_total(cnt.p, out.ptr, m, s);
   out.idx = dalloc<int32_t>(size_t(out.nnz));
   out.val = dalloc<double>(size_t(out.nnz));
   GPP_LAUNCH(dt_single_rows<true>, grid_stride_blocks(m), kThreads, 0, s, m, lp.A.ptr, lp.A.idx, lp.A.val, acc.p,
@@ -789,7 +792,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     ~Release() { if (own) free_csr(M); }
   } release{sorted_at, !at_sorted};
 
-  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m), s), acc(size_t(m) + 1, s), keep_c(size_t(m), s),
+  DBuf<int32_t> col_nnz(size_t(n), s), flag(size_t(m), s), acc(size_t(m), s), keep_c(size_t(m), s),
       elim_c(size_t(m), s);
   DBuf<double> keep_v(size_t(m), s), elim_v(size_t(m), s);
   GPP_LAUNCH(dt_col_nnz, grid_stride_blocks(n), kThreads, 0, s, n, AT.ptr, AT.idx, AT.val, plan.keep_row.p,
@@ -798,13 +801,12 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
              plan.keep_row.p, plan.keep_col.p, col_nnz.p, plan.AL.p, plan.AU.p, zt, tol, ratio_tol,
              p.doubleton_equations_max_fill_in_proxy, AT.ptr, AT.idx, AT.val, flag.p, keep_c.p, elim_c.p, keep_v.p,
              elim_v.p);
-  list_flagged(m, flag.p, nullptr, acc.p, acc.p + m, s);
-  const int acceptable = read_scalar(acc.p + m);
+  const int acceptable = list_flagged(m, flag.p, nullptr, acc.p, s);
   if (acceptable == 0) return;
 
   // Matching rounds over the acceptable rows (ascending).
   DBuf<uint8_t> active(size_t(acceptable), s), blocked(size_t(n), s);
-  DBuf<int32_t> owner(size_t(n), s), chosen(size_t(acceptable), s), rows(size_t(acceptable) + 1, s);
+  DBuf<int32_t> owner(size_t(n), s), chosen(size_t(acceptable), s), rows(size_t(acceptable), s);
   check(cudaMemsetAsync(active.p, 1, size_t(acceptable), s), "doubleton active");
   blocked.zero();
   chosen.zero();
@@ -815,26 +817,24 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     GPP_LAUNCH(dt_select, gk, kThreads, 0, s, acceptable, acc.p, active.p, blocked.p, keep_c.p, elim_c.p, owner.p,
                chosen.p);
   }
-  list_flagged(acceptable, chosen.p, acc.p, rows.p, rows.p + acceptable, s);
-  const int sel = read_scalar(rows.p + acceptable);
+  const int sel = list_flagged(acceptable, chosen.p, acc.p, rows.p, s);
   const double ratio = double(sel) / double(acceptable);
   if (sel == 0 || sel < p.doubleton_equations_min_selected_per_batch || ratio < p.doubleton_equations_min_selected_ratio)
     return;
 
   // Apply against the values before the batch (columns are distinct).
-  Status st;
-  st.clear(kStWords);
+  Report report = ctx().open_report(2);
   DBuf<uint8_t> kind(size_t(sel), s);
   DBuf<double> alpha(size_t(sel), s), beta(size_t(sel), s), obj_term(size_t(sel), s), rec_val(size_t(sel) * 12, s);
   DBuf<int32_t> rec_idx(size_t(sel) * 4, s);
   const int gs = grid_stride_blocks(sel);
   GPP_LAUNCH(dt_apply, gs, kThreads, 0, s, sel, rows.p, keep_c.p, elim_c.p, keep_v.p, elim_v.p, p.bound_tol,
              plan.l.p, plan.u.p, plan.c.p, plan.AU.p, plan.keep_row.p, plan.keep_col.p, kind.p, alpha.p, beta.p,
-             obj_term.p, rec_idx.p, rec_val.p, st.d);
-  const int32_t* f = st.read(kStWords);
-  if (f[kStInfeasible]) { plan.has_infeasible = true; return; }
-  if (!f[kStAny]) return;
-  const int subst = f[kStSubst];
+             obj_term.p, rec_idx.p, rec_val.p, report);
+  const volatile int64_t* f = ctx().await(report);
+  if (f[0] & 1) { plan.has_infeasible = true; return; }
+  if (!f[0]) return;
+  const int subst = int(f[1]);
 
   if (subst && p.record_postsolve_tape) {
     PostsolveSegment seg = make_segment(subst, 4 * int64_t(subst), 12 * int64_t(subst));
@@ -853,10 +853,14 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     DBuf<uint32_t> claimed(size_t(m + 31) / 32, s);
     role.zero();
     claimed.zero();
+    Status st;
+    st.clear(kStWords);
+    report = ctx().open_report(kStWords, st.d);
     GPP_LAUNCH(dt_roles, gs, kThreads, 0, s, sel, rows.p, keep_c.p, elim_c.p, kind.p, beta.p, plan.l.p, role.p,
                value.p, role_col.p);
-    GPP_LAUNCH(dt_touch, warp_grid(sel), kThreads, 0, s, sel, role_col.p, AT.ptr, AT.idx, claimed.p, touched.p, st.d);
-    const int ntouched = st.read(kStWords)[kStTouched];
+    GPP_LAUNCH(dt_touch, warp_grid(sel), kThreads, 0, s, sel, role_col.p, AT.ptr, AT.idx, claimed.p, touched.p, st.d,
+               report);
+    const int ntouched = int(ctx().await(report)[kStTouched]);
     if (ntouched)
       GPP_LAUNCH(dt_shift, warp_grid(ntouched), kThreads, 0, s, touched.p, st.d, lp.A.ptr, lp.A.idx, lp.A.val,
                  plan.keep_row.p, role.p, value.p, zt, plan.AL.p, plan.AU.p);
@@ -867,8 +871,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     DBuf<int32_t> dcnt(size_t(sel) + 1, s), dpos(size_t(sel) + 1, s);
     GPP_LAUNCH(dt_delta_count, warp_grid(sel), kThreads, 0, s, sel, rows.p, elim_c.p, kind.p, AT.ptr, AT.idx, AT.val,
                plan.keep_row.p, zt, dcnt.p);
-    exclusive_scan_i32(dcnt.p, dpos.p, sel, s);
-    const int total = read_scalar(dpos.p + sel);
+    const int total = exclusive_scan_total(dcnt.p, dpos.p, sel, s);
     DBuf<uint64_t> keys(size_t(std::max(total, 1)), s);
     DBuf<int32_t> order(size_t(std::max(total, 1)), s), dcol(size_t(std::max(total, 1)), s),
         row_cnt(size_t(m) + 1, s), dptr(size_t(m) + 1, s);
@@ -897,8 +900,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     out.rows = m;
     out.cols = n;
     out.ptr = dalloc<offset_t>(size_t(m) + 1);
-    exclusive_scan_i32(cnt.p, out.ptr, m, s);
-    out.nnz = read_scalar(out.ptr + m);
+    out.nnz = exclusive_scan_total(cnt.p, out.ptr, m, s);
     out.idx = dalloc<int32_t>(size_t(out.nnz));
     out.val = dalloc<double>(size_t(out.nnz));
     GPP_LAUNCH(dt_rebuild<true>, warp_grid(m), kThreads, 0, s, m, lp.A.ptr, lp.A.idx, lp.A.val, dptr.p, dcol.p,

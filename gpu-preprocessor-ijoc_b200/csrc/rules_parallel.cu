@@ -248,9 +248,9 @@ __global__ void row_groups_kernel(int count, const uint64_t* __restrict__ sh, co
                                   double* AL, double* AU, const offset_t* __restrict__ ptr,
                                   const int32_t* __restrict__ idx, const double* __restrict__ val, double coeff_tol,
                                   double interval_tol, uint8_t* __restrict__ del, int32_t* __restrict__ merge_to,
-                                  int32_t* __restrict__ step_out, double* __restrict__ rec_vals,
-                                  int32_t* __restrict__ status) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count; s += gridDim.x * blockDim.x) {
+                                  int32_t* __restrict__ step_out, double* __restrict__ rec_vals, Report report) {
+  uint32_t infeasible = 0;
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count && !infeasible; s += gridDim.x * blockDim.x) {
     const uint64_t hs = sh[s];
     if (s > 0 && sh[s - 1] == hs) continue;
     int e = s;
@@ -287,7 +287,7 @@ __global__ void row_groups_kernel(int count, const uint64_t* __restrict__ sh, co
       found = true;
       double sl, su;
       scaled_interval(AL[row], AU[row], r, &sl, &su);
-      if (fmax(rl, sl) > fmin(ru, su) + interval_tol) { atomicMax(status, 1); return; }
+      if (fmax(rl, sl) > fmin(ru, su) + interval_tol) { infeasible = 1; break; }
       ++step;
       merge_to[row] = rep;
       step_out[row] = step;
@@ -300,8 +300,9 @@ __global__ void row_groups_kernel(int count, const uint64_t* __restrict__ sh, co
       ru = fmin(ru, su);
       del[row] = 1;
     }
-    if (found) { AL[rep] = rl; AU[rep] = ru; }
+    if (found && !infeasible) { AL[rep] = rl; AU[rep] = ru; }
   }
+  post_flags(report, infeasible);
 }
 
 __global__ void pack_parallel_records(int64_t count, const int32_t* __restrict__ ids, const int32_t* __restrict__ first,
@@ -426,15 +427,16 @@ __global__ void col_groups_kernel(int count, const uint64_t* __restrict__ sh, co
                                   double coeff_tol, double obj_tol, double max_abs, const int32_t* __restrict__ guard,
                                   int guard_min, uint8_t* __restrict__ del, uint8_t* __restrict__ fixed,
                                   double* __restrict__ fval, int32_t* __restrict__ merge_to,
-                                  double* __restrict__ rec_vals, int32_t* __restrict__ status) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count; s += gridDim.x * blockDim.x) {
+                                  double* __restrict__ rec_vals, Report report) {
+  uint32_t found_any = 0;   // 1 unbounded, 2 merged, 4 fixed
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count && !(found_any & 1u); s += gridDim.x * blockDim.x) {
     const uint64_t hs = sh[s];
     if (s > 0 && sh[s - 1] == hs) continue;
     int e = s;
     while (e + 1 < count && sh[e + 1] == hs) ++e;
     if (e <= s) continue;
     const double active_max = guard && *guard < guard_min ? INFINITY : max_abs;
-    for (int a = s; a < e; ++a) {
+    for (int a = s; a < e && !(found_any & 1u); ++a) {
       const int j = sc[a];
       if (!keep_col[j] || del[j] || fixed[j]) continue;
       for (int b = a + 1; b <= e; ++b) {
@@ -460,7 +462,7 @@ __global__ void col_groups_kernel(int count, const uint64_t* __restrict__ sh, co
           l[j] = nl;
           u[j] = nu;
           del[k] = 1;
-          atomicMax(status + 1, 1);
+          found_any |= 2u;
           continue;
         }
         bool k_lo = false, k_hi = false, j_lo = false, j_hi = false;
@@ -472,26 +474,27 @@ __global__ void col_groups_kernel(int count, const uint64_t* __restrict__ sh, co
           else { k_hi = !isfinite(tu); j_hi = !isfinite(su); }
         }
         if (k_lo) {
-          if (!isfinite(sl)) { atomicMax(status, 1); return; }
-          fixed[k] = 1; fval[k] = sl; atomicMax(status + 2, 1);
+          if (!isfinite(sl)) { found_any |= 1u; break; }
+          fixed[k] = 1; fval[k] = sl; found_any |= 4u;
           continue;
         } else if (k_hi) {
-          if (!isfinite(su)) { atomicMax(status, 1); return; }
-          fixed[k] = 1; fval[k] = su; atomicMax(status + 2, 1);
+          if (!isfinite(su)) { found_any |= 1u; break; }
+          fixed[k] = 1; fval[k] = su; found_any |= 4u;
           continue;
         }
         if (j_lo) {
-          if (!isfinite(tl)) { atomicMax(status, 1); return; }
-          fixed[j] = 1; fval[j] = tl; atomicMax(status + 2, 1);
+          if (!isfinite(tl)) { found_any |= 1u; break; }
+          fixed[j] = 1; fval[j] = tl; found_any |= 4u;
           break;
         } else if (j_hi) {
-          if (!isfinite(tu)) { atomicMax(status, 1); return; }
-          fixed[j] = 1; fval[j] = tu; atomicMax(status + 2, 1);
+          if (!isfinite(tu)) { found_any |= 1u; break; }
+          fixed[j] = 1; fval[j] = tu; found_any |= 4u;
           break;
         }
       }
     }
   }
+  post_flags(report, found_any);
 }
 
 __global__ void col_apply(int n, int m, const uint8_t* __restrict__ del, const uint8_t* __restrict__ fixed,
@@ -553,13 +556,13 @@ int32_t sorted_live_hashes(const uint64_t* hash, const uint8_t* keep, int32_t n,
   // The pairs are packed by one selection into arrays for all items (their
   // number is known afterwards).
   keys.alloc(size_t(std::max(n, 1)), s);
-  ids.alloc(size_t(std::max(n, 1)) + 1, s);
-  int32_t* total = ids.p + std::max(n, 1);
+  ids.alloc(size_t(std::max(n, 1)), s);
   const auto pack = [hash, out_keys = keys.p, out_ids = ids.p] __device__(int64_t i, int at, bool taken) {
     if (!taken) return;
     out_keys[at] = hash[i];
     out_ids[at] = int32_t(i);
   };
+  int32_t count;
   if (n > kRepeatFilterMin) {
     // 32 bitmap positions per item, a power of two between 2^20 and 2^29.
     int lg = 20;
@@ -571,12 +574,11 @@ int32_t sorted_live_hashes(const uint64_t* hash, const uint8_t* keep, int32_t n,
     GPP_LAUNCH(mark_hash_bits, grid_stride_blocks(n), kThreads, 0, s, n, keep, hash, bits.p, bits.p + words,
                bit_mask);
     const uint32_t* twice = bits.p + words;
-    select_items(
-        n, [=] __device__(int64_t i) { return keep[i] && hash_may_repeat(hash[i], twice, bit_mask); }, pack, total, s);
+    count = select_and_count(
+        n, [=] __device__(int64_t i) { return keep[i] && hash_may_repeat(hash[i], twice, bit_mask); }, pack, s);
   } else {
-    select_items(n, [keep] __device__(int64_t i) { return keep[i] != 0; }, pack, total, s);
+    count = select_and_count(n, [keep] __device__(int64_t i) { return keep[i] != 0; }, pack, s);
   }
-  const int32_t count = read_scalar(total);
   radix_sort_pairs(keys.p, ids.p, count, s);
   return count;
 }
@@ -627,15 +629,14 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
   DBuf<int32_t> merge_to(size_t(m), s), step(size_t(m), s);
   DBuf<double> rec(size_t(5) * size_t(m), s);
   del.zero();
-  Status st;
-  st.clear(2);
+  const Report report = ctx().open_report(1);
   GPP_LAUNCH(row_groups_kernel, grid_stride_blocks(count), kThreads, 0, s, count, keys.p, ids.p, plan.keep_row.p,
              plan.keep_col.p, plan.AL.p, plan.AU.p, lp.A.ptr, lp.A.idx, lp.A.val, p.zero_tol, p.feasibility_tol,
-             del.p, merge_to.p, step.p, rec.p, st.d);
-  if (st.read(1)[0]) { plan.has_infeasible = true; return; }
+             del.p, merge_to.p, step.p, rec.p, report);
+  if (ctx().await(report)[0]) { plan.has_infeasible = true; return; }
   DBuf<uint64_t> dkeys(size_t(m), s);
-  DBuf<int32_t> dids(size_t(m) + 1, s);
-  select_items(
+  DBuf<int32_t> dids(size_t(m), s);
+  const int32_t deleted = select_and_count(
       m, [del = del.p] __device__(int64_t i) { return del[i] != 0; },
       [step = step.p, out_keys = dkeys.p, ids = dids.p, keep_row = plan.keep_row.p] __device__(int64_t i, int at,
                                                                                                bool taken) {
@@ -644,8 +645,7 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
         ids[at] = int32_t(i);
         keep_row[i] = 0;
       },
-      dids.p + m, s);
-  const int32_t deleted = read_scalar(dids.p + m);
+      s);
   if (!deleted) return;
   if (p.record_postsolve_tape) {
     // Records ordered by (merge step, deleted row) (rule_parallel_rows.cu:79-84).
@@ -674,36 +674,38 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
   if (count <= 1) return;
   const double coeff_tol = std::fmax(p.zero_tol, p.bound_tol), obj_tol = coeff_tol;
   const bool guard = std::isfinite(p.parallel_columns_max_abs_ratio) && p.parallel_columns_scale_guard_min_groups > 1;
-  Status st;
-  st.clear(4);
-  if (guard)
+  DBuf<int32_t> guard_groups;
+  if (guard) {
+    guard_groups.alloc(1, s);
+    guard_groups.zero();
     GPP_LAUNCH(count_guard_groups, grid_stride_blocks(count), kThreads, 0, s, count, keys.p, ids.p, plan.keep_col.p,
                plan.keep_row.p, plan.c.p, lp.AT.ptr, lp.AT.idx, lp.AT.val, p.zero_tol, coeff_tol, obj_tol,
                p.parallel_columns_max_abs_ratio, p.parallel_columns_scale_guard_max_group_size,
-               p.parallel_columns_scale_guard_min_groups, st.d + 3);
+               p.parallel_columns_scale_guard_min_groups, guard_groups.p);
+  }
   DBuf<uint8_t> del(size_t(n), s), fixed(size_t(n), s);
   DBuf<double> fval(size_t(n), s), rec(size_t(5) * size_t(n), s), contrib(size_t(n), s);
   DBuf<int32_t> merge_to(size_t(n), s);
   del.zero();
   fixed.zero();
+  const Report report = ctx().open_report(1);
   GPP_LAUNCH(col_groups_kernel, grid_stride_blocks(count), kThreads, 0, s, count, keys.p, ids.p, plan.keep_col.p,
              plan.keep_row.p, plan.c.p, plan.l.p, plan.u.p, lp.AT.ptr, lp.AT.idx, lp.AT.val, p.zero_tol, coeff_tol,
-             obj_tol, p.parallel_columns_max_abs_ratio, guard ? st.d + 3 : nullptr,
-             p.parallel_columns_scale_guard_min_groups, del.p, fixed.p, fval.p, merge_to.p, rec.p, st.d);
-  const int32_t* f = st.read(3);
-  if (f[0]) { plan.has_unbounded = true; return; }
-  const bool merged = f[1] != 0, any_fixed = f[2] != 0;
+             obj_tol, p.parallel_columns_max_abs_ratio, guard_groups.p,
+             p.parallel_columns_scale_guard_min_groups, del.p, fixed.p, fval.p, merge_to.p, rec.p, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 1u) { plan.has_unbounded = true; return; }
+  const bool merged = (found & 2u) != 0, any_fixed = (found & 4u) != 0;
   if (!merged && !any_fixed) return;
   if (merged && p.record_postsolve_tape) {
     // Records ordered by deleted column (rule_parallel_columns.cu:83-87).
-    DBuf<int32_t> dids(size_t(n) + 1, s);
-    select_items(
+    DBuf<int32_t> dids(size_t(n), s);
+    const int32_t merges = select_and_count(
         n, [del = del.p] __device__(int64_t i) { return del[i] != 0; },
         [ids = dids.p] __device__(int64_t i, int at, bool taken) {
           if (taken) ids[at] = int32_t(i);
         },
-        dids.p + n, s);
-    const int32_t merges = read_scalar(dids.p + n);
+        s);
     PostsolveSegment seg = make_segment(merges, 2 * int64_t(merges), 5 * int64_t(merges));
     GPP_LAUNCH(pack_parallel_records, grid_stride_blocks(merges + 1), kThreads, 0, s, int64_t(merges), dids.p,
                merge_to.p, rec.p, 3, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p);
@@ -715,8 +717,7 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
       DBuf<int64_t> rc(size_t(n) + 1, s), nz(size_t(n) + 1, s), rpos(size_t(n) + 1, s), npos(size_t(n) + 1, s);
       GPP_LAUNCH(fixed_sizes, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, lp.AT.ptr, lp.AT.idx, plan.keep_row.p,
                  rc.p, nz.p);
-      exclusive_scan_pair_i64(rc.p, rpos.p, nz.p, npos.p, n, s);
-      const auto [recs, nnz] = read_scalars(rpos.p + n, npos.p + n);
+      const auto [recs, nnz] = exclusive_scan_pair_i64(rc.p, rpos.p, nz.p, npos.p, n, s);
       PostsolveSegment seg = make_segment(recs, recs + nnz, 2 * recs + nnz);
       GPP_LAUNCH(fixed_pack, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, lp.AT.ptr, lp.AT.idx, lp.AT.val,
                  plan.keep_row.p, fval.p, plan.c.p, rpos.p, npos.p, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p,
@@ -729,7 +730,7 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
   }
   GPP_LAUNCH(col_apply, grid_stride_blocks(std::max(n, m)), kThreads, 0, s, n, m, del.p, fixed.p, fval.p, plan.c.p,
              any_fixed ? shift.p : nullptr, plan.keep_col.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, contrib.p);
-  plan.obj_delta += any_fixed ? det_sum(contrib.p, n, s) : 0.0;
+  plan.obj_delta += any_fixed ? det_sum(contrib.p, nullptr, n, s) : 0.0;
   plan.has_col_action = plan.has_change = true;
 }
 

@@ -13,7 +13,8 @@ namespace {
 __global__ void redundant_classify(int m, const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
                                    const double* __restrict__ AL, const double* __restrict__ AU,
                                    const double* __restrict__ mn, const double* __restrict__ mx, double tol,
-                                   uint8_t* __restrict__ action, int32_t* __restrict__ status) {
+                                   uint8_t* __restrict__ action, Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 a row goes, 4 a side goes
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     uint8_t a = 0;
     if (keep_row[i] && row_nnz[i] > 1) {
@@ -22,17 +23,18 @@ __global__ void redundant_classify(int m, const uint8_t* __restrict__ keep_row, 
       if (!(lf && uf && fabs(au - al) <= tol)) {
         const double lo = mn[i], hi = mx[i];
         if ((lf && hi < al - tol) || (uf && lo > au + tol)) {
-          atomicMax(status + 0, 1);
+          found |= 1u;
         } else {
           const bool li = !lf || lo >= al - tol, ui = !uf || hi <= au + tol;
-          if (li && ui) { a = 1; atomicMax(status + 1, 1); }
-          else if (lf && li) { a = 2; atomicMax(status + 2, 1); }
-          else if (uf && ui) { a = 3; atomicMax(status + 3, 1); }
+          if (li && ui) { a = 1; found |= 2u; }
+          else if (lf && li) { a = 2; found |= 4u; }
+          else if (uf && ui) { a = 3; found |= 4u; }
         }
       }
     }
     action[i] = a;
   }
+  post_flags(report, found);
 }
 __global__ void redundant_apply(int m, const uint8_t* __restrict__ action, uint8_t* __restrict__ keep_row,
                                 double* __restrict__ AL, double* __restrict__ AU) {
@@ -52,13 +54,13 @@ __global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col,
                                     const int32_t* __restrict__ at_idx, const double* __restrict__ at_val,
                                     double zt, double bound_tol, int max_degree, const int32_t* __restrict__ col_nnz,
                                     uint8_t* __restrict__ fixed, uint8_t* __restrict__ inf_fix,
-                                    double* __restrict__ fval, double* __restrict__ contrib,
-                                    int32_t* __restrict__ status) {
+                                    double* __restrict__ fval, double* __restrict__ contrib, Report report) {
+  uint32_t found = 0;   // 1 infeasible, 2 unbounded, 4 a column is fixed, 8 at an infinite bound
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     fixed[j] = 0; inf_fix[j] = 0; fval[j] = 0.0; contrib[j] = 0.0;
     if (!keep_col[j]) continue;
     const double lj = l[j], uj = u[j];
-    if (lj > uj + bound_tol) { atomicMax(status + 0, 1); continue; }
+    if (lj > uj + bound_tol) { found |= 1u; continue; }
     const double cj = c[j];
     if (fabs(cj) > zt && col_nnz[j] > max_degree) continue;
     bool down = false, up = false;
@@ -73,19 +75,19 @@ __global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col,
     bool f = false, fi = false;
     double v = 0.0;
     if (cj > zt) {
-      if (!down) { if (isfinite(lj)) { v = lj; f = true; } else { atomicMax(status + 0, 2); continue; } }
+      if (!down) { if (isfinite(lj)) { v = lj; f = true; } else { found |= 2u; continue; } }
     } else if (cj < -zt) {
-      if (!up) { if (isfinite(uj)) { v = uj; f = true; } else { atomicMax(status + 0, 2); continue; } }
+      if (!up) { if (isfinite(uj)) { v = uj; f = true; } else { found |= 2u; continue; } }
     } else if (fabs(cj) <= zt) {
       if (!down) { f = true; if (isfinite(lj)) v = lj; else { v = -INFINITY; fi = true; } }
       else if (!up) { f = true; if (isfinite(uj)) v = uj; else { v = INFINITY; fi = true; } }
     }
     if (f) {
       fixed[j] = 1; inf_fix[j] = fi; fval[j] = v; contrib[j] = fi ? 0.0 : cj * v;
-      atomicMax(status + 1, 1);
-      if (fi) atomicMax(status + 2, 1);
+      found |= fi ? 12u : 4u;
     }
   }
+  post_flags(report, found);
 }
 __global__ void finite_fixed_mask(int n, const uint8_t* __restrict__ fixed, const uint8_t* __restrict__ inf_fix,
                                   uint8_t* __restrict__ out) {
@@ -95,12 +97,14 @@ __global__ void finite_fixed_mask(int n, const uint8_t* __restrict__ fixed, cons
 __global__ void dual_fix_row_remove(int n, const uint8_t* __restrict__ fixed, const uint8_t* __restrict__ inf_fix,
                                     const uint8_t* __restrict__ keep_row, const offset_t* __restrict__ at_ptr,
                                     const int32_t* __restrict__ at_idx, uint8_t* __restrict__ remove,
-                                    int32_t* __restrict__ status) {
+                                    Report report) {
+  uint32_t any = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (!(fixed[j] && inf_fix[j])) continue;
     for (offset_t p = at_ptr[j]; p < at_ptr[j + 1]; ++p)
-      if (keep_row[at_idx[p]]) { remove[at_idx[p]] = 1; atomicMax(status + 3, 1); }
+      if (keep_row[at_idx[p]]) { remove[at_idx[p]] = 1; any = 1; }
   }
+  post_flags(report, any);
 }
 // InfiniteBoundDualFix record sizes: 1 record per column, 3 + rows + entries
 // indices and 1 + rows + entries values (entries restricted to the entry domain).
@@ -176,7 +180,7 @@ __global__ void dual_fix_apply(int n, int m, const uint8_t* __restrict__ fixed, 
     if (k < m) {
       AL[k] -= shift[k];
       AU[k] -= shift[k];
-      if (remove[k]) keep_row[k] = 0;
+      if (remove && remove[k]) keep_row[k] = 0;
     }
   }
 }
@@ -191,14 +195,13 @@ void rule_redundant_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, co
   DBuf<double> mn(size_t(m), s), mx(size_t(m), s);
   DBuf<uint8_t> action(size_t(m), s);
   row_plain_minmax(lp.A, plan.l.p, plan.u.p, plan.keep_row.p, plan.keep_col.p, stats.row_nnz.p, mn.p, mx.p, s);
-  Status st;
-  st.clear(4);
+  const Report report = ctx().open_report(1);
   GPP_LAUNCH(redundant_classify, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p,
-             plan.AL.p, plan.AU.p, mn.p, mx.p, p.bound_tol, action.p, st.d);
-  const int32_t* f = st.read(4);
-  if (f[0]) { plan.has_infeasible = true; return; }
-  if (!f[1] && !f[2] && !f[3]) return;
-  const bool deleted = f[1] != 0;
+             plan.AL.p, plan.AU.p, mn.p, mx.p, p.bound_tol, action.p, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  if (!found) return;
+  const bool deleted = (found & 2u) != 0;
   GPP_LAUNCH(redundant_apply, grid_stride_blocks(m), kThreads, 0, s, m, action.p, plan.keep_row.p, plan.AL.p,
              plan.AU.p);
   plan.has_row_action = true;
@@ -212,33 +215,39 @@ void rule_dual_fix(Plan& plan, const WorkingLp& lp, const Stats& stats, const gp
   const int n = lp.n(), m = lp.m();
   if (n == 0) return;
   auto s = ctx().stream;
-  DBuf<uint8_t> fixed(size_t(n), s), inf_fix(size_t(n), s), finite(size_t(n), s), remove(size_t(std::max(m, 1)), s);
+  DBuf<uint8_t> fixed(size_t(n), s), inf_fix(size_t(n), s), finite, remove;
   DBuf<double> fval(size_t(n), s), contrib(size_t(n), s), shift(size_t(std::max(m, 1)), s);
-  Status st;
-  st.clear(4);
+  Report report = ctx().open_report(1);
   GPP_LAUNCH(dual_fix_candidates, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.keep_row.p,
              plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, lp.AT.ptr, lp.AT.idx, lp.AT.val, p.zero_tol,
              p.bound_tol, p.dual_fix_max_nonzero_cost_col_degree, stats.col_nnz.p, fixed.p, inf_fix.p, fval.p,
-             contrib.p, st.d);
-  const int32_t* f = st.read(3);
-  if (f[0] == 1) { plan.has_infeasible = true; return; }
-  if (f[0] == 2) { plan.has_unbounded = true; return; }
-  if (!f[1]) return;
-  const bool any_inf = f[2] != 0;
-  GPP_LAUNCH(finite_fixed_mask, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, finite.p);
-  if (m) {
-    row_gather_shift(lp.A, lp.AT, plan.keep_row.p, finite.p, fval.p, nullptr, shift.p, s);
-    remove.zero();
+             contrib.p, report);
+  const uint32_t found = uint32_t(ctx().await(report)[0]);
+  if (found & 2u) { plan.has_unbounded = true; return; }
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  if (!found) return;
+  const bool any_inf = (found & 8u) != 0;
+  // Columns fixed at an infinite bound shift no row and take their rows with
+  // them; without any, every fixed column shifts its rows.
+  if (any_inf) {
+    finite.alloc(size_t(n), s);
+    remove.alloc(size_t(std::max(m, 1)), s);
+    GPP_LAUNCH(finite_fixed_mask, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, finite.p);
   }
-  GPP_LAUNCH(dual_fix_row_remove, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, plan.keep_row.p,
-             lp.AT.ptr, lp.AT.idx, remove.p, st.d);
-  const bool row_changed = st.read(4)[3] != 0;
+  if (m) row_gather_shift(lp.A, lp.AT, plan.keep_row.p, any_inf ? finite.p : fixed.p, fval.p, nullptr, shift.p, s);
+  bool row_changed = false;
+  if (any_inf) {
+    remove.zero();
+    report = ctx().open_report(1);
+    GPP_LAUNCH(dual_fix_row_remove, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, plan.keep_row.p,
+               lp.AT.ptr, lp.AT.idx, remove.p, report);
+    row_changed = ctx().await(report)[0] != 0;
+  }
   if (p.record_postsolve_tape && any_inf) {
     DBuf<int64_t> rc(size_t(n) + 1, s), sz(size_t(n) + 1, s), rpos(size_t(n) + 1, s), spos(size_t(n) + 1, s);
     GPP_LAUNCH(infinite_sizes, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, plan.keep_row.p,
                plan.rule_entry_keep_col, lp.A.ptr, lp.A.idx, lp.AT.ptr, lp.AT.idx, rc.p, sz.p);
-    exclusive_scan_pair_i64(rc.p, rpos.p, sz.p, spos.p, n, s);
-    const auto [recs, size] = read_scalars(rpos.p + n, spos.p + n);
+    const auto [recs, size] = exclusive_scan_pair_i64(rc.p, rpos.p, sz.p, spos.p, n, s);
     if (recs) {
       PostsolveSegment seg = make_segment(recs, size + 3 * recs, size + recs);
       GPP_LAUNCH(infinite_pack, grid_stride_blocks(n), kThreads, 0, s, n, fixed.p, inf_fix.p, fval.p, plan.keep_row.p,

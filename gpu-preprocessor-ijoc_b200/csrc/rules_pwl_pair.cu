@@ -954,7 +954,7 @@ bool try_shifted_antipodal(Plan& plan, const WorkingLp& lp, const gpp_params& p)
              minus_cap.p, rho.p, vst.p);
   if (read_scalar(vst.p) != 0) return false;
   // The objective constant sum_i rho_i (l_p + l_m), in pair order.
-  const double delta = det_sum(constant.p, P, s);
+  const double delta = det_sum(constant.p, nullptr, P, s);
   if (!std::isfinite(delta) || !std::isfinite(lp.obj + delta)) return false;
   DBuf<int32_t> counts(size_t(rows) + 1, s), removed(2, s);
   DBuf<uint8_t> keep(size_t(rows), s);

@@ -16,7 +16,7 @@
 // rows that hold them and the columns of eliminated rows, through compacted
 // work lists, instead of sweeping all of A / AT as the reference does.  The
 // objective delta is the reference's canonical sum over the rule's entry
-// domain, evaluated from the sparse contributions (det_sum_sparse).
+// domain.
 #include <algorithm>
 #include <climits>
 
@@ -61,7 +61,7 @@ __global__ void sc_candidates(int n, int m, const uint8_t* __restrict__ keep_col
                               const double* __restrict__ c, const double* __restrict__ l, const double* __restrict__ u,
                               const double* __restrict__ AL, const double* __restrict__ AU, double zero_tol,
                               int32_t* __restrict__ owner, int32_t* __restrict__ cand, int32_t* __restrict__ rows,
-                              int32_t* __restrict__ long_rows, int32_t* st) {
+                              int32_t* __restrict__ long_rows, int32_t* st, Report report) {
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;   // every thread of a block runs the same trips
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += stride) {
@@ -86,6 +86,7 @@ __global__ void sc_candidates(int n, int m, const uint8_t* __restrict__ keep_col
     const int pl = block_append(st + kStLong, is_long);
     if (is_long) long_rows[pl] = srow[j];
   }
+  post_report(report);
 }
 
 struct RowCache {
@@ -365,7 +366,7 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
                          double* __restrict__ AL, double* __restrict__ AU, double tol, int32_t* __restrict__ owner,
                          uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ kind,
                          int32_t* __restrict__ winners, int64_t* __restrict__ contrib_idx,
-                         double* __restrict__ contrib_val) {
+                         double* __restrict__ contrib_val, Report report) {
   const int count = st[kStRows];
   const int stride = gridDim.x * blockDim.x;
   const int top = (count + stride - 1) / stride * stride;
@@ -427,6 +428,7 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
     const int pw = block_append(st + kStWin, k != 0);
     if (k) winners[pw] = row;
   }
+  post_report(report);
 }
 
 // Columns whose cost changes: the live columns of eliminated rows, each
@@ -434,7 +436,8 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
 __global__ void sc_touch(const int32_t* __restrict__ winners, const int32_t* __restrict__ st,
                          const uint8_t* __restrict__ kind, const offset_t* __restrict__ ptr,
                          const int32_t* __restrict__ idx, const uint8_t* __restrict__ keep_col,
-                         uint32_t* __restrict__ claimed, int32_t* __restrict__ touched, int32_t* st_w) {
+                         uint32_t* __restrict__ claimed, int32_t* __restrict__ touched, int32_t* st_w,
+                         Report report) {
   const int count = st[kStWin];
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
@@ -456,6 +459,7 @@ __global__ void sc_touch(const int32_t* __restrict__ winners, const int32_t* __r
       if (take) touched[pos] = col;
     }
   }
+  post_report(report);
 }
 
 // _kernel_apply_singleton_objective_updates_deterministic (:1075-1104): for a
@@ -596,8 +600,16 @@ __global__ void sc_shift_pack(const int32_t* __restrict__ sorted_rows, int count
   }
 }
 
-__global__ void sc_fill_i32(int32_t* p, int n, int32_t v) {
+// Unclaimed owners and zeroed status words.
+__global__ void sc_start(int32_t* p, int n, int32_t v, int32_t* __restrict__ st) {
+  if (blockIdx.x == 0 && threadIdx.x < kStWords) st[threadIdx.x] = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
+}
+
+// The objective contributions as a dense vector for the canonical sum.
+__global__ void sc_scatter_contrib(int count, const int64_t* __restrict__ idx, const double* __restrict__ val,
+                                   double* __restrict__ dense) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) dense[idx[q]] = val[q];
 }
 
 // Sort key: substitution rows first, then dual-shift rows, each ascending.
@@ -618,16 +630,16 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
   Status st;
-  st.clear(kStWords);
   DBuf<int32_t> owner(size_t(m), s), cand(size_t(n), s), rows(size_t(m), s), long_rows(size_t(m), s);
-  GPP_LAUNCH(sc_fill_i32, grid_stride_blocks(m), kThreads, 0, s, owner.p, m, kUnclaimed);
+  GPP_LAUNCH(sc_start, grid_stride_blocks(m), kThreads, 0, s, owner.p, m, kUnclaimed, st.d);
+  Report report = ctx().open_report(4, st.d);
   GPP_LAUNCH_BYTES(sc_candidates, double(n) * 11 + 16.0 * n, grid_stride_blocks(n), kThreads, 0, s, n, m,
                    plan.keep_col.p, plan.keep_row.p, stats.singleton_col.p, stats.scol_row.p, stats.scol_val.p,
                    stats.row_nnz.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.zero_tol, owner.p, cand.p,
-                   rows.p, long_rows.p, st.d);
-  const int32_t* f = st.read(4);
+                   rows.p, long_rows.p, st.d, report);
+  const volatile int64_t* f = ctx().await(report);
   if (f[kStUnbounded]) { plan.has_unbounded = true; return; }
-  const int ncand = f[kStCand], nrows = f[kStRows];
+  const int ncand = int(f[kStCand]), nrows = int(f[kStRows]), nlong = int(f[kStLong]);
   if (ncand == 0) return;
 
   // Activity cache of the claimed rows.
@@ -638,8 +650,8 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   const int warp_blocks = std::max(1, std::min((nrows + 31) / 32, kNumSMs * 16));
   GPP_LAUNCH(sc_cache_rows, warp_blocks, kThreads, 0, s, rows.p, st.d, stats.row_nnz.p, lp.A.ptr, lp.A.idx,
              lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
-  if (f[kStLong])
-    GPP_LAUNCH(sc_cache_long, std::min(f[kStLong], kNumSMs * 8), kThreads, 0, s, long_rows.p, st.d, stats.row_nnz.p,
+  if (nlong)
+    GPP_LAUNCH(sc_cache_long, std::min(nlong, kNumSMs * 8), kThreads, 0, s, long_rows.p, st.d, stats.row_nnz.p,
                lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
 
   // Propose and stage.
@@ -650,11 +662,13 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   GPP_LAUNCH(sc_propose, grid_stride_blocks(ncand), kThreads, 0, s, cand.p, st.d, stats.scol_row.p,
              stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, fmin.p, fmax.p, counts.p,
              invalid.p, p.bound_tol, p.zero_tol, action.p, side.p, owner.p);
+  report = ctx().open_report(kStWords, st.d);
   GPP_LAUNCH(sc_stage, grid_stride_blocks(nrows), kThreads, 0, s, rows.p, st.d, n, action.p, side.p,
              stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.bound_tol, owner.p,
-             plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p);
-  f = st.read(kStWords);
-  const int nwin = f[kStWin], nelim = f[kStElim];
+             plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p,
+             report);
+  f = ctx().await(report);
+  const int nwin = int(f[kStWin]), nelim = int(f[kStElim]);
   const bool any_side = f[kStSide] != 0;
   if (nelim == 0 && !any_side) return;
 
@@ -663,9 +677,10 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
     DBuf<uint32_t> claimed(size_t(n + 31) / 32, s);
     claimed.zero();
     DBuf<int32_t> touched(size_t(n), s);
+    report = ctx().open_report(kStWords, st.d);
     GPP_LAUNCH(sc_touch, std::max(1, std::min((nwin + 7) / 8, kNumSMs * 16)), kThreads, 0, s, winners.p, st.d,
-               kind.p, lp.A.ptr, lp.A.idx, plan.keep_col.p, claimed.p, touched.p, st.d);
-    const int ntouched = st.read(kStWords)[kStTouched];
+               kind.p, lp.A.ptr, lp.A.idx, plan.keep_col.p, claimed.p, touched.p, st.d, report);
+    const int ntouched = int(ctx().await(report)[kStTouched]);
     if (ntouched)
       GPP_LAUNCH(sc_cost, std::max(1, std::min((ntouched + 7) / 8, kNumSMs * 16)), kThreads, 0, s, touched.p, st.d,
                  n, lp.AT.ptr, lp.AT.idx, lp.AT.val, owner.p, stats.scol_val.p, plan.c.p);
@@ -684,6 +699,7 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
       const int blocks = std::max(1, std::min((nelim + 7) / 8, kNumSMs * 16));
       GPP_LAUNCH(sc_sub_sizes, blocks, kThreads, 0, s, sorted.p, nelim, owner.p, lp.A.ptr, lp.A.idx, lp.A.val,
                  plan.keep_col.p, p.zero_tol, sel.p, sup.p);
+      const uint32_t seq = ctx().open_mail();
       scan_items<int64_t, 2>(
           nelim,
           [sel = sel.p, sup = sup.p] __device__(int64_t i, int64_t(&v)[2]) {
@@ -694,13 +710,14 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
             rec[i] = int32_t(before[0]);
             spos[i] = before[1];
           },
-          [rec = rec.p + nelim, spos = spos.p + nelim] __device__(const int64_t(&sum)[2]) {
+          [rec = rec.p + nelim, spos = spos.p + nelim, mail = ctx().mail, seq] __device__(const int64_t(&sum)[2]) {
             *rec = int32_t(sum[0]);
             *spos = sum[1];
+            post_values(mail, seq, sum[0], sum[1]);
           },
           s);
-      const auto [recs32, support] = read_scalars(rec.p + nelim, spos.p + nelim);
-      const int64_t recs = recs32;
+      const volatile int64_t* sums = ctx().await(ctx().mail, seq, "substitution records");
+      const int64_t recs = sums[0], support = sums[1];
       if (recs) {
         PostsolveSegment seg = make_segment(recs, 3 * recs + support, 6 * recs + support);
         GPP_LAUNCH(sc_sub_pack, blocks, kThreads, 0, s, sorted.p, nelim, owner.p, kind.p, sel.p, rec.p, spos.p,
@@ -718,10 +735,11 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   }
 
   if (nelim) {
-    auto [ci, cv] = to_host2(contrib_idx.p, size_t(nelim), contrib_val.p, size_t(nelim));
-    std::vector<std::pair<int64_t, double>> entries(ci.size());
-    for (size_t k = 0; k < ci.size(); ++k) entries[k] = {ci[k], cv[k]};
-    plan.obj_delta += det_sum_sparse(std::move(entries));
+    DBuf<double> contrib(size_t(n), s);
+    contrib.zero();
+    GPP_LAUNCH(sc_scatter_contrib, grid_stride_blocks(nelim), kThreads, 0, s, nelim, contrib_idx.p, contrib_val.p,
+               contrib.p);
+    plan.obj_delta += det_sum(contrib.p, nullptr, n, s);
   }
   plan.has_row_action = true;
   plan.has_col_action = plan.has_col_action || nelim > 0;

@@ -496,9 +496,8 @@ void commit_projection(Plan& plan, const WorkingLp& lp, const gpp_params& p, con
     st.clear(1);
     GPP_LAUNCH(projection_sizes<K>, grid_stride_blocks(n), kThreads, 0, s, n, in, selected.p, incident, rc.p, sc.p,
                st.d);
-    exclusive_scan_pair_i64(rc.p, rpos.p, sc.p, spos.p, n, s);
     if (st.read(1)[0]) throw std::runtime_error("projection tape certificate changed before commit");
-    const auto [recs, support] = read_scalars(rpos.p + n, spos.p + n);
+    const auto [recs, support] = exclusive_scan_pair_i64(rc.p, rpos.p, sc.p, spos.p, n, s);
     if (recs) {
       PostsolveSegment seg = make_segment(recs, int64_t(K + 8) * recs + support, 2 * recs + support);
       GPP_LAUNCH(projection_pack<K>, grid_stride_blocks(n), kThreads, 0, s, n, in, selected.p, incident, rpos.p,

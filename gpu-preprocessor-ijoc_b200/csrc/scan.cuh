@@ -172,12 +172,13 @@ void scan_items(int64_t n, In in, Out out, Total total, cudaStream_t s) {
 
 // Selection in order: pred(i) says whether item i is taken (called once per
 // item), emit(i, rank, taken) gets its rank among the taken ones (for an item
-// not taken: the number taken before it); *count receives the number taken.
+// not taken: the number taken before it); the number taken goes to *count or,
+// in the waiting form, to the host.
 // A warp reads 32 consecutive items at a time, and ranks come from ballots.
 template <class Pred, class Emit>
 __global__ void __launch_bounds__(kThreads)
-select_tiles(int64_t n, int64_t tiles, Pred pred, Emit emit, int32_t* count, unsigned long long* words,
-             unsigned int* counters, int32_t* error) {
+select_tiles(int64_t n, int64_t tiles, Pred pred, Emit emit, int32_t* count, Mailbox* mail, uint32_t seq,
+             unsigned long long* words, unsigned int* counters, int32_t* error) {
   __shared__ int warp_sums[kThreads / 32];
   __shared__ long long tile_before;
   __shared__ unsigned int ticket;
@@ -204,7 +205,10 @@ select_tiles(int64_t n, int64_t tiles, Pred pred, Emit emit, int32_t* count, uns
     const long long before = publish_and_look_back(words, t, tiles, all, error);
     if (lane == 0) {
       tile_before = before;
-      if (t == tiles - 1) *count = int32_t(before + all);
+      if (t == tiles - 1) {
+        if (count) *count = int32_t(before + all);
+        if (mail) post_values(mail, seq, before + all);
+      }
     }
   }
   __syncthreads();
@@ -224,8 +228,21 @@ template <class Pred, class Emit>
 void select_items(int64_t n, Pred pred, Emit emit, int32_t* count, cudaStream_t s) {
   const int64_t tiles = n > 0 ? (n + kScanTile - 1) / kScanTile : 1;   // no items: a count of 0
   LookbackSpace w(size_t(tiles), s);
-  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, count, w.words, w.counters,
-             ctx().host_error);
+  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, count, nullptr, 0u, w.words,
+             w.counters, ctx().host_error);
+}
+
+// The same, waiting for the number taken.
+template <class Pred, class Emit>
+int32_t select_and_count(int64_t n, Pred pred, Emit emit, cudaStream_t s, const char* where = __builtin_FUNCTION()) {
+  if (n <= 0) return 0;
+  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+  LookbackSpace w(size_t(tiles), s);
+  auto& c = ctx();
+  const uint32_t seq = c.open_mail();
+  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, nullptr, c.mail, seq, w.words,
+             w.counters, c.host_error);
+  return int32_t(c.await(c.mail, seq, where)[0]);
 }
 
 }  // namespace gpp

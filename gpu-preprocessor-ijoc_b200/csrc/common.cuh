@@ -294,6 +294,9 @@ struct Context {
   // between launches.
   unsigned long long* lookback = nullptr;
   size_t lookback_words = 0;
+  // Row bits of the compaction (compact.cu), zero between compactions.
+  uint2* row_bits = nullptr;
+  size_t row_bits_words = 0;
   // Mailbox of the kernels' answers and the words they gather them in; one
   // question is open at a time (the host waits for its answer).
   Mailbox* mail = nullptr;

@@ -23,256 +23,175 @@ namespace {
 // ---- entry-tiled compaction -------------------------------------------------
 //
 // The stored entries are cut into tiles of kCompactTile consecutive positions,
-// one block per tile and kCompactPer consecutive positions per thread, so the
-// index and value streams are read with 128-bit loads whatever the row
-// lengths.  A tile learns the row of each of its entries without a search:
-// the rows whose pointer falls inside the tile mark their start positions in
-// shared memory, and a block scan of the marks counts the row starts at or
-// before every position.  The copy is a stream compaction in stored order, so
-// a kept entry's output position is the number of kept entries before it.
-// One pass does it: tiles are handed out in order by a ticket counter, each
-// tile publishes its kept count as soon as it knows it, and looks back over
-// its predecessors' published counts (a decoupled look-back) for its output
-// offset; its block scan then places each kept entry and each kept row's new
-// pointer.
-constexpr int kCompactPer = 8;
-constexpr int kCompactTile = kThreads * kCompactPer;
+// one block per tile; each of its warps takes kCompactWarp of them, 32 at a
+// time, so the index and value streams are read coalesced whatever the row
+// lengths.  Rows come in through two bit arrays over the positions, set by one
+// pass over the row pointers: where a row that holds entries starts, and
+// whether it is kept; an entry's row is the last start at or before it, so a
+// word of 32 positions needs a count of leading zeros per lane.  Ballots rank
+// the kept entries, and as few entries go, a warp's kept entries leave as
+// nearly contiguous stores straight from registers.  The copy is a stream
+// compaction in stored order, so a kept entry's output position is the number
+// of kept entries before it.  One pass does it: tiles are handed out in order
+// by a ticket counter, each tile publishes its kept count as soon as it knows
+// it, and looks back over its predecessors' published counts (a decoupled
+// look-back) for its output offset.  The kept masks and offsets it leaves give
+// every row its new pointer in a last pass over the rows, which also clears the
+// bits again.  A and A^T of a materialisation are two sides of each launch.
+//
+// Bound by the rate of the one random access per entry, to the inner map (the
+// 29.8M-nnz LP's columns and rows, about 250 us a side at 4 bytes of each 32
+// fetched), then by the look-back; DRAM stays at a third of its rate.  Per tile
+// three block barriers (the ticket, the warps' counts, the offset) against the
+// ten of a form that ranked and staged over the block, which took 287 us.  A
+// form whose warps walked the rows of their part stalled on long runs of empty
+// rows (1.5 ms a launch on the QAP N = 30 relaxation, 0.2 ms now).
+constexpr int kCompactRounds = 8;
+constexpr int kCompactWarp = 32 * kCompactRounds;
+constexpr int kCompactWarps = kThreads / 32;
+constexpr int kCompactTile = kCompactWarp * kCompactWarps;
 
-// first_row[t]: the first row whose pointer is at or past t * kCompactTile
-// (rows when there is none).  Row r takes the tiles whose start lies in
-// (ptr[r - 1], ptr[r]]; the virtual row `rows` takes the tiles past the last
-// row's pointer.
-__global__ void compact_tile_rows(int rows, const offset_t* __restrict__ ptr, int tiles,
-                                  int32_t* __restrict__ first_row) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= rows; r += gridDim.x * blockDim.x) {
-    const int64_t lo = r == 0 ? 0 : int64_t(ptr[r - 1]) / kCompactTile + 1;
-    int64_t hi = r == rows ? int64_t(tiles) - 1 : int64_t(ptr[r]) / kCompactTile;
-    if (hi > tiles - 1) hi = tiles - 1;
-    for (int64_t t = lo; t <= hi; ++t) first_row[t] = r;
-  }
-}
+// One matrix to compact: rows by outer_map, entries by inner_map.
+struct CompactSide {
+  offset_t nnz;
+  int rows, cols, tiles;
+  const offset_t* ptr;
+  const int32_t* idx;
+  const double* val;
+  const int32_t *outer_map, *inner_map;
+  uint2* rows_at;       // per 32 positions: bits of the row starts (x) and of the kept ones (y)
+  uint8_t* part_kept;   // per warp part: its first entry's row, where that row starts before it, is kept
+  uint32_t* masks;      // per 32 positions: the kept entries
+  int32_t* before;      // per warp part: the kept entries before it
+  int32_t outer_new;
+  offset_t* out_ptr;
+  int32_t* out_idx;
+  double* out_val;
+};
+struct CompactSides {
+  CompactSide side[2];
+};
 
-// Exclusive scan of one value per thread over the block; the block total goes
-// to *total.  `warp_sums` holds kThreads / 32 ints of shared memory.
-__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
+__global__ void compact_mark_rows(CompactSides sides) {
 #pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += y;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
-  __syncthreads();
-  int before = 0, all = 0;
-#pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) {
-    const int sw = warp_sums[w];
-    before += w < warp ? sw : 0;
-    all += sw;
-  }
-  __syncthreads();
-  *total = all;
-  return before + incl - v;
-}
-
-template <bool kVec>
-__device__ __forceinline__ void load_tile_cols(const int32_t* __restrict__ p, int avail, int (&col)[kCompactPer]) {
-  if (kVec && avail >= kCompactPer) {
-    const int4 a = __ldcs(reinterpret_cast<const int4*>(p));
-    const int4 b = __ldcs(reinterpret_cast<const int4*>(p) + 1);
-    col[0] = a.x; col[1] = a.y; col[2] = a.z; col[3] = a.w;
-    col[4] = b.x; col[5] = b.y; col[6] = b.z; col[7] = b.w;
-  } else {
-#pragma unroll
-    for (int k = 0; k < kCompactPer; ++k) col[k] = k < avail ? __ldcs(p + k) : -1;
-  }
-}
-template <bool kVec>
-__device__ __forceinline__ void load_tile_vals(const double* __restrict__ p, int avail, double (&v)[kCompactPer]) {
-  if (kVec && avail >= kCompactPer) {
-#pragma unroll
-    for (int k = 0; k < kCompactPer / 2; ++k) {
-      const double2 d = __ldcs(reinterpret_cast<const double2*>(p) + k);
-      v[2 * k] = d.x;
-      v[2 * k + 1] = d.y;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < kCompactPer; ++k) v[k] = k < avail ? __ldcs(p + k) : 0.0;
-  }
-}
-
-// Kept-entry mask of this thread's kCompactPer positions: the entry exists,
-// its row is kept and its (remapped) inner index is kept.  `col` holds the
-// inner indices already mapped (-1 for a dropped or missing entry).
-__device__ __forceinline__ unsigned tile_kept_mask(int r0, int64_t base, int len, const offset_t* __restrict__ ptr,
-                                                   int r1, const int32_t* __restrict__ outer_map,
-                                                   const int (&col)[kCompactPer], int* marker, int* warp_sums) {
-  const int p0 = int(threadIdx.x) * kCompactPer;
-  // Row starts inside the tile.
-#pragma unroll
-  for (int k = 0; k < kCompactPer; ++k) marker[p0 + k] = 0;
-  __syncthreads();
-  for (int r = r0 + int(threadIdx.x); r < r1; r += kThreads) {
-    const int64_t pos = int64_t(ptr[r]) - base;
-    if (pos < len) atomicAdd(marker + pos, 1);
-  }
-  __syncthreads();
-  int mk[kCompactPer], local = 0;
-#pragma unroll
-  for (int k = 0; k < kCompactPer; ++k) {
-    mk[k] = marker[p0 + k];
-    local += mk[k];
-  }
-  int total;
-  int row = r0 - 1 + block_exclusive_scan(local, warp_sums, &total);
-  unsigned mask = 0;
-  int cached_row = -1, cached_keep = -1;
-#pragma unroll
-  for (int k = 0; k < kCompactPer; ++k) {
-    row += mk[k];
-    if (p0 + k < len && col[k] >= 0) {
-      if (row != cached_row) {
-        cached_row = row;
-        cached_keep = outer_map[row];
-      }
-      if (cached_keep >= 0) mask |= 1u << k;
+  for (int k = 0; k < 2; ++k) {
+    const CompactSide& s = sides.side[k];
+    if (s.tiles == 0) continue;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < s.rows; r += gridDim.x * blockDim.x) {
+      const int64_t a = s.ptr[r], e = s.ptr[r + 1];
+      if (a == e) continue;
+      const bool kept = s.outer_map[r] >= 0;
+      const uint32_t bit = 1u << (a & 31);
+      atomicOr(&s.rows_at[a >> 5].x, bit);
+      if (kept) atomicOr(&s.rows_at[a >> 5].y, bit);
+      for (int64_t w = a / kCompactWarp + 1; w * kCompactWarp < e; ++w) s.part_kept[w] = kept;
     }
   }
-  return mask;
 }
 
-// Tile status words: the top two bits say what the low 62 hold (an aggregate:
-// the tile's own kept count; an inclusive count: the kept entries of every
-// tile up to and including it).  Zero means nothing published yet.
-constexpr unsigned long long kTileAggregate = 1ull << 62, kTileInclusive = 2ull << 62;
-constexpr unsigned long long kTileValue = (1ull << 62) - 1;
-// Polls of one predecessor before a look-back gives up (well over a second;
-// a predecessor that holds a ticket is running and publishes within
-// microseconds).  Giving up sets the error word, which the host checks.
-constexpr int kLookbackPolls = 1 << 22;
-
-__device__ __forceinline__ unsigned long long ld_tile_status(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_tile_status(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// Kept entries before tile t, by warp 0: 32 predecessors per round, summing
-// aggregates back to the nearest inclusive count (before tile 0: zero).
-__device__ __forceinline__ int64_t tile_lookback(const unsigned long long* status, int t, int32_t* err) {
-  const int lane = threadIdx.x & 31;
-  int64_t before = 0;
-  for (int end = t - 1;; end -= 32) {
-    const int j = end - lane;
-    unsigned long long st = kTileInclusive;
-    if (j >= 0) {
-      st = ld_tile_status(status + j);
-      for (int polls = 1; (st >> 62) == 0; ++polls) {
-        if (polls == kLookbackPolls) {
-          atomicExch(err, 1);
-          st = kTileInclusive;
-          break;
-        }
-        __nanosleep(64);
-        st = ld_tile_status(status + j);
-      }
-    }
-    const unsigned incl = __ballot_sync(0xffffffffu, (st >> 62) == 2);
-    const int first = incl ? __ffs(incl) - 1 : 32;
-    unsigned long long v = lane <= first ? (st & kTileValue) : 0ull;
+// New pointers of the kept rows (an empty row's is the kept entries before its
+// position too), and the row bits cleared for the next compaction.
+__global__ void compact_row_pointers(CompactSides sides) {
 #pragma unroll
-    for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    before += int64_t(v);
-    if (incl) return before;
-  }
-}
-
-// One pass: result[0] receives the kept total, result[1] is set if a
-// look-back gave up.  `status` holds tiles words and then the ticket counter,
-// all zero at launch.
-template <bool kVec>
-__global__ void __launch_bounds__(kThreads)
-compact_tiles(offset_t nnz, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-              const double* __restrict__ val, const int32_t* __restrict__ outer_map,
-              const int32_t* __restrict__ inner_map, const int32_t* __restrict__ first_row, int rows, int tiles,
-              unsigned long long* status, int32_t outer_new, offset_t* __restrict__ out_ptr,
-              int32_t* __restrict__ out_idx, double* __restrict__ out_val, int32_t* result) {
-  // `marker` is free once the rows are known and then stages the kept
-  // indices; `stage_val` the kept values.  The stores go out coalesced.
-  __shared__ __align__(16) int marker[kCompactTile];
-  __shared__ __align__(16) double stage_val[kCompactTile];
-  __shared__ int warp_sums[kThreads / 32];
-  __shared__ int thread_before[kThreads];
-  __shared__ unsigned thread_mask[kThreads];
-  __shared__ int ticket;
-  __shared__ long long tile_before;
-  const int p0 = int(threadIdx.x) * kCompactPer;
-  for (;;) {
-    if (threadIdx.x == 0) ticket = int(atomicAdd(status + tiles, 1ull));
-    __syncthreads();
-    const int t = ticket;
-    if (t >= tiles) return;   // block-uniform
-    const int64_t base = int64_t(t) * kCompactTile;
-    const int len = int(min(int64_t(kCompactTile), int64_t(nnz) - base));
-    int col[kCompactPer];
-    double v[kCompactPer];
-    load_tile_cols<kVec>(idx + base + p0, len - p0, col);
-    load_tile_vals<kVec>(val + base + p0, len - p0, v);
-    const int r0 = first_row[t], r1 = t + 1 < tiles ? first_row[t + 1] : rows;
-#pragma unroll
-    for (int k = 0; k < kCompactPer; ++k) col[k] = col[k] >= 0 ? inner_map[col[k]] : -1;
-    const unsigned mask = tile_kept_mask(r0, base, len, ptr, r1, outer_map, col, marker, warp_sums);
-    int total;
-    const int before = block_exclusive_scan(__popc(mask), warp_sums, &total);
-    if (threadIdx.x < 32) {
-      if (threadIdx.x == 0)
-        st_tile_status(status + t, (t == 0 ? kTileInclusive : kTileAggregate) | (unsigned long long)total);
-      const int64_t ahead = t == 0 ? 0 : tile_lookback(status, t, result + 1);
-      if (threadIdx.x == 0) {
-        if (t > 0) st_tile_status(status + t, kTileInclusive | (unsigned long long)(ahead + total));
-        tile_before = ahead;
-      }
-    }
-    int o = before;
-#pragma unroll
-    for (int k = 0; k < kCompactPer; ++k)
-      if (mask >> k & 1u) {
-        marker[o] = col[k];
-        stage_val[o] = v[k];
-        ++o;
-      }
-    thread_before[threadIdx.x] = before;
-    thread_mask[threadIdx.x] = mask;
-    __syncthreads();
-    const int64_t tile_out = tile_before;
-    for (int q = int(threadIdx.x); q < total; q += kThreads) {
-      out_idx[tile_out + q] = marker[q];
-      out_val[tile_out + q] = stage_val[q];
-    }
-    // New row pointers of the kept rows that start in this tile: the kept
-    // entries before the row's first position.
-    for (int r = r0 + int(threadIdx.x); r < r1; r += kThreads) {
-      const int nr = outer_map[r];
+  for (int k = 0; k < 2; ++k) {
+    const CompactSide& s = sides.side[k];
+    if (s.tiles == 0) continue;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < s.rows; r += gridDim.x * blockDim.x) {
+      const int64_t a = s.ptr[r];
+      if (a < s.nnz) s.rows_at[a >> 5] = make_uint2(0u, 0u);
+      const int nr = s.outer_map[r];
       if (nr < 0) continue;
-      const int64_t pos = int64_t(ptr[r]) - base;
-      int kept_before = total;
-      if (pos < len) {
-        const int q = int(pos) / kCompactPer, j = int(pos) % kCompactPer;
-        kept_before = thread_before[q] + __popc(thread_mask[q] & ((1u << j) - 1u));
+      if (a >= s.nnz) {   // past the last entry
+        s.out_ptr[nr] = s.out_ptr[s.outer_new];
+        continue;
       }
-      out_ptr[nr] = offset_t(tile_out + kept_before);
+      const int64_t part = a / kCompactWarp;
+      int kept = s.before[part];
+      for (int64_t w = part * kCompactRounds; w < a >> 5; ++w) kept += __popc(s.masks[w]);
+      kept += __popc(s.masks[a >> 5] & ((1u << (a & 31)) - 1u));
+      s.out_ptr[nr] = kept;
     }
-    if (t == tiles - 1 && threadIdx.x == 0) {
-      out_ptr[outer_new] = offset_t(tile_out + total);
-      result[0] = int32_t(tile_out + total);
-    }
-    __syncthreads();   // the staging buffers and the ticket are reused by the next tile
   }
+}
+
+// `words` (one per tile of both sides) and `counters` are zero at launch and
+// again after it; the kept counts of both sides are posted to the host.
+__global__ void __launch_bounds__(kThreads)
+compact_tiles(CompactSides sides, unsigned long long* words, unsigned int* counters, int32_t* error, Report report) {
+  __shared__ int warp_counts[kCompactWarps];
+  __shared__ long long tile_before;
+  __shared__ unsigned int ticket;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int total_tiles = sides.side[0].tiles + sides.side[1].tiles;
+  for (;;) {
+    if (threadIdx.x == 0) ticket = atomicAdd(counters, 1u);
+    __syncthreads();
+    if (ticket >= unsigned(total_tiles)) break;   // block-uniform
+    const bool second = int(ticket) >= sides.side[0].tiles;
+    const CompactSide& s = sides.side[second ? 1 : 0];
+    const int t = int(ticket) - (second ? sides.side[0].tiles : 0);
+    const int64_t part = int64_t(t) * kCompactWarps + warp;
+    const int64_t base = part * kCompactWarp;
+    const int len = int(max(int64_t(0), min(int64_t(kCompactWarp), int64_t(s.nnz) - base)));
+    int col[kCompactRounds];
+    double v[kCompactRounds];
+#pragma unroll
+    for (int k = 0; k < kCompactRounds; ++k) col[k] = k * 32 + lane < len ? __ldcs(s.idx + base + k * 32 + lane) : -1;
+#pragma unroll
+    for (int k = 0; k < kCompactRounds; ++k) v[k] = k * 32 + lane < len ? __ldcs(s.val + base + k * 32 + lane) : 0.0;
+    // The part's row bits, one word pair per lane of the first kCompactRounds.
+    const bool has = lane < kCompactRounds && lane * 32 < len;
+    const uint2 mine = has ? s.rows_at[base / 32 + lane] : make_uint2(0u, 0u);
+    bool carry = len > 0 && s.part_kept[part];
+#pragma unroll
+    for (int k = 0; k < kCompactRounds; ++k) col[k] = col[k] >= 0 ? s.inner_map[col[k]] : -1;
+    const unsigned up_to = 0xffffffffu >> (31 - lane);   // this lane and those before it
+    int kept = 0;
+    unsigned mask[kCompactRounds];
+#pragma unroll
+    for (int k = 0; k < kCompactRounds; ++k) {
+      const unsigned starts = __shfl_sync(0xffffffffu, mine.x, k), keeps = __shfl_sync(0xffffffffu, mine.y, k);
+      const unsigned at = starts & up_to;
+      const bool row_kept = at ? (keeps >> (31 - __clz(at)) & 1u) != 0 : carry;
+      if (starts) carry = (keeps >> (31 - __clz(starts)) & 1u) != 0;
+      mask[k] = __ballot_sync(0xffffffffu, row_kept && col[k] >= 0);
+      kept += __popc(mask[k]);
+      if (lane == k) s.masks[base / 32 + k] = mask[k];
+    }
+    if (lane == 0) warp_counts[warp] = kept;
+    __syncthreads();
+    if (warp == 0) {
+      int sum = 0;
+#pragma unroll
+      for (int w = 0; w < kCompactWarps; ++w) sum += warp_counts[w];
+      const long long before =
+          publish_and_look_back(words + (second ? sides.side[0].tiles : 0), t, s.tiles, sum, error);
+      if (lane == 0) {
+        tile_before = before;
+        if (t == s.tiles - 1) {
+          s.out_ptr[s.outer_new] = offset_t(before + sum);
+          report.words[second ? 1 : 0] = int32_t(before + sum);
+        }
+      }
+    }
+    __syncthreads();
+    int64_t out = tile_before;
+#pragma unroll
+    for (int w = 0; w < kCompactWarps; ++w) out += w < warp ? warp_counts[w] : 0;
+    if (lane == 0) s.before[part] = int32_t(out);
+#pragma unroll
+    for (int k = 0; k < kCompactRounds; ++k) {
+      if (mask[k] >> lane & 1u) {
+        const int64_t o = out + __popc(mask[k] & ((1u << lane) - 1u));
+        s.out_idx[o] = col[k];
+        s.out_val[o] = v[k];
+      }
+      out += __popc(mask[k]);
+    }
+    __syncthreads();   // the counts and the ticket are reused by the next tile
+  }
+  leave_zeroed(words, total_tiles, counters);
+  post_report(report);
 }
 
 __global__ void histogram(const int32_t* __restrict__ idx, offset_t nnz, int32_t* __restrict__ counts) {
@@ -401,60 +320,99 @@ std::pair<int32_t, int32_t> build_old_to_new_pair(const uint8_t* keep_row, int32
   return {int32_t(kept[0]), int32_t(kept[1])};
 }
 
-DevCsr compact_csr_queued(const DevCsr& M, const int32_t* outer_map, int32_t outer_new, const int32_t* inner_map,
-                          int32_t inner_new, cudaStream_t s, int32_t* result, int64_t* profile_record) {
+namespace {
+// The output of compacting M, its arrays sized for all stored entries (nothing
+// waits for the kept count before the copy), and the side that fills it; an
+// output without rows, columns or entries is only given its zero pointers.
+DevCsr compact_output(const DevCsr& M, const int32_t* outer_map, int32_t outer_new, const int32_t* inner_map,
+                      int32_t inner_new, CompactSide& side, cudaStream_t s) {
   DevCsr out;
   out.rows = outer_new;
   out.cols = inner_new;
-  out.nnz = -1;
   out.ptr = dalloc<offset_t>(size_t(outer_new) + 1);
-  *profile_record = -1;
   if (outer_new == 0 || inner_new == 0 || M.nnz == 0) {
     check(cudaMemsetAsync(out.ptr, 0, sizeof(offset_t) * (size_t(outer_new) + 1), s), "compact empty ptr");
-    check(cudaMemsetAsync(result, 0, 2 * sizeof(int32_t), s), "compact empty result");
     return out;
   }
-  // The kept entries are at most the stored ones: the outputs are sized for
-  // those, so nothing waits for the kept count before the copy.
   out.idx = dalloc<int32_t>(size_t(M.nnz));
   out.val = dalloc<double>(size_t(M.nnz));
-  const int tiles = int((int64_t(M.nnz) + kCompactTile - 1) / kCompactTile);
-  DBuf<int32_t> first_row(size_t(tiles), s);
-  DBuf<unsigned long long> status(size_t(tiles) + 1, s);   // tile words, then the ticket counter
-  status.zero();
-  check(cudaMemsetAsync(result, 0, 2 * sizeof(int32_t), s), "compact result");
-  GPP_LAUNCH(compact_tile_rows, grid_stride_blocks(int64_t(M.rows) + 1), kThreads, 0, s, M.rows, M.ptr, tiles,
-             first_row.p);
-  // 128-bit loads need 16-byte aligned index and value arrays (always so for
-  // the engine's own matrices; a caller's input may be offset).
-  const bool vec = reinterpret_cast<uintptr_t>(M.idx) % 16 == 0 && reinterpret_cast<uintptr_t>(M.val) % 16 == 0;
-  // Reads; the writes (4 (outer_new + 1) + 12 nnz') are added to the launch's
-  // profile record once the kept count is known.
-  const double read_bytes = 4.0 * (M.rows + 1) + 12.0 * M.nnz + 4.0 * M.rows + 4.0 * M.cols + 4.0 * tiles;
-  const int grid = std::min(tiles, kNumSMs * 5);   // resident blocks at its register budget
-  if (vec)
-    GPP_LAUNCH_BYTES(compact_tiles<true>, read_bytes, grid, kThreads, 0, s, M.nnz, M.ptr, M.idx, M.val, outer_map,
-                     inner_map, first_row.p, M.rows, tiles, status.p, outer_new, out.ptr, out.idx, out.val, result);
-  else
-    GPP_LAUNCH_BYTES(compact_tiles<false>, read_bytes, grid, kThreads, 0, s, M.nnz, M.ptr, M.idx, M.val, outer_map,
-                     inner_map, first_row.p, M.rows, tiles, status.p, outer_new, out.ptr, out.idx, out.val, result);
-  *profile_record = profile_last();
+  side.nnz = M.nnz;
+  side.rows = M.rows;
+  side.cols = M.cols;
+  side.tiles = int((int64_t(M.nnz) + kCompactTile - 1) / kCompactTile);
+  side.ptr = M.ptr;
+  side.idx = M.idx;
+  side.val = M.val;
+  side.outer_map = outer_map;
+  side.inner_map = inner_map;
+  side.outer_new = outer_new;
+  side.out_ptr = out.ptr;
+  side.out_idx = out.idx;
+  side.out_val = out.val;
   return out;
 }
 
-void compact_csr_finish(DevCsr& out, const int32_t* result_host, int64_t profile_record) {
-  if (result_host[1]) throw CudaError("compaction: a tile's look-back timed out waiting for its predecessors");
-  out.nnz = out.rows > 0 && out.cols > 0 ? offset_t(result_host[0]) : 0;
-  profile_add_bytes(profile_record, 4.0 * (out.rows + 1) + 12.0 * out.nnz);
+// Compacts the sides that hold entries; their kept counts go to `out`.
+void compact_sides(CompactSides& sides, DevCsr* const (&out)[2], cudaStream_t s) {
+  const int tiles = sides.side[0].tiles + sides.side[1].tiles;
+  if (tiles == 0) return;
+  const size_t parts = size_t(tiles) * kCompactWarps, words32 = parts * kCompactRounds;
+  auto& c = ctx();
+  if (c.row_bits_words < words32) {   // zero between compactions
+    const size_t grown = std::max(words32, 2 * c.row_bits_words);
+    uint2* p = dalloc<uint2>(grown);
+    dfree(std::exchange(c.row_bits, p));
+    c.row_bits_words = grown;
+    check(cudaMemsetAsync(p, 0, sizeof(uint2) * grown, s), "row bits");
+  }
+  DBuf<uint32_t> masks(words32, s);
+  DBuf<int32_t> before(parts, s);
+  DBuf<uint8_t> part_kept(parts, s);
+  for (int k = 0; k < 2; ++k) {
+    CompactSide& d = sides.side[k];
+    const size_t first = k ? size_t(sides.side[0].tiles) * kCompactWarps : 0;
+    d.rows_at = c.row_bits + first * kCompactRounds;
+    d.masks = masks.p + first * kCompactRounds;
+    d.before = before.p + first;
+    d.part_kept = part_kept.p + first;
+  }
+  const int rows_grid = grid_stride_blocks(std::max(sides.side[0].rows, sides.side[1].rows));
+  GPP_LAUNCH(compact_mark_rows, rows_grid, kThreads, 0, s, sides);
+  // Reads; the writes (12 nnz') are added to the launch's profile record once
+  // the kept count is known.
+  double bytes = 0.0;
+  for (const CompactSide& d : sides.side)
+    if (d.tiles) bytes += 12.0 * d.nnz + 4.0 * d.cols + 0.375 * d.nnz;
+  LookbackSpace w(size_t(tiles), s);
+  const Report report = c.open_report(2);
+  GPP_LAUNCH_BYTES(compact_tiles, bytes, std::min(tiles, kNumSMs * 4), kThreads, 0, s, sides, w.words, w.counters,
+                   c.host_error, report);
+  const int64_t record = profile_last();
+  GPP_LAUNCH(compact_row_pointers, rows_grid, kThreads, 0, s, sides);
+  const volatile int64_t* kept = c.await(report);
+  for (int k = 0; k < 2; ++k)
+    if (sides.side[k].tiles) {
+      out[k]->nnz = offset_t(kept[k]);
+      profile_add_bytes(record, 12.0 * out[k]->nnz);
+    }
 }
+}  // namespace
 
 DevCsr compact_csr(const DevCsr& M, const int32_t* outer_map, int32_t outer_new, const int32_t* inner_map,
                    int32_t inner_new, cudaStream_t s) {
-  Status st;
-  int64_t rec = -1;
-  DevCsr out = compact_csr_queued(M, outer_map, outer_new, inner_map, inner_new, s, st.d, &rec);
-  compact_csr_finish(out, st.read(2), rec);
+  CompactSides sides{};
+  DevCsr out = compact_output(M, outer_map, outer_new, inner_map, inner_new, sides.side[0], s);
+  compact_sides(sides, {&out, nullptr}, s);
   return out;
+}
+
+std::pair<DevCsr, DevCsr> compact_csr_pair(const DevCsr& A, const DevCsr& AT, const int32_t* row_map, int32_t rows_new,
+                                           const int32_t* col_map, int32_t cols_new, cudaStream_t s) {
+  CompactSides sides{};
+  DevCsr a = compact_output(A, row_map, rows_new, col_map, cols_new, sides.side[0], s);
+  DevCsr t = compact_output(AT, col_map, cols_new, row_map, rows_new, sides.side[1], s);
+  compact_sides(sides, {&a, &t}, s);
+  return {a, t};
 }
 
 DevCsr transpose_csr(const DevCsr& M, cudaStream_t s) {

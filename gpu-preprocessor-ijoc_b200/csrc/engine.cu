@@ -9,6 +9,7 @@
 // step for step; every rule reports through one status readback.
 #include <chrono>
 #include <cmath>
+#include <tuple>
 
 #include "engine.cuh"
 #include "presolve.hpp"
@@ -207,15 +208,7 @@ struct Engine {
       next.A = compact_csr(pl.new_A, rmap.p, m_new, cmap.p, n_new, s());
       next.AT = transpose_csr(next.A, s());
     } else if (cur.AT_sorted()) {
-      // A and A^T are compacted back to back; one readback gives both kept
-      // counts (equal) and their look-back error words.
-      Status st;
-      int64_t rec_a = -1, rec_t = -1;
-      next.A = compact_csr_queued(cur.A, rmap.p, m_new, cmap.p, n_new, s(), st.d, &rec_a);
-      next.AT = compact_csr_queued(cur.AT, cmap.p, n_new, rmap.p, m_new, s(), st.d + 2, &rec_t);
-      const int32_t* r = st.read(4);
-      compact_csr_finish(next.A, r, rec_a);
-      compact_csr_finish(next.AT, r + 2, rec_t);
+      std::tie(next.A, next.AT) = compact_csr_pair(cur.A, cur.AT, rmap.p, m_new, cmap.p, n_new, s());
       if (next.A.nnz != next.AT.nnz) throw std::logic_error("compaction: A and A^T kept different entry counts");
       next.a_sorted = cur.a_sorted;
     } else {

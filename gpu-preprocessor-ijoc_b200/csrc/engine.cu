@@ -87,7 +87,6 @@ struct Engine {
   Plan plan;
   Stats stats;
   bool stats_dirty = true;
-  DBuf<double> ref_bounds;
   uint32_t* inf_hist = nullptr;   // histogram features (scheduled runs only)
   uint64_t deletion_serial = 0;
 
@@ -408,12 +407,6 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
     bool bounds_changed = false;
     if (gate(kGateBoundStrengthening, p.enable_bound_strengthening) && !e.terminal && !time_exceeded()) {
       e.prepare();
-      const int n = cur.n();
-      e.ref_bounds.alloc(size_t(2 * std::max(n, 1)), ctx().stream);
-      check(cudaMemcpyAsync(e.ref_bounds.p, e.plan.l.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx().stream), "ref l");
-      check(cudaMemcpyAsync(e.ref_bounds.p + n, e.plan.u.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx().stream), "ref u");
-      e.plan.ref_l = e.ref_bounds.p;
-      e.plan.ref_u = e.ref_bounds.p + n;
       bounds_changed = note(kGateBoundStrengthening,
                             e.deferred_rule(true, "bound_strengthening",
                                             [&] { rule_bound_strengthening(e.plan, cur, e.stats, p); }));

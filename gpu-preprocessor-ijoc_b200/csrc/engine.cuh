@@ -32,6 +32,7 @@ struct RowSchedule {
   int32_t rows = -1;
   offset_t nnz = -1;
   uint64_t epoch = 0;
+  uint64_t degrees_version = 0;   // live-degree schedules: the statistics they were built from
 };
 
 // Builds the schedule of `M` by stored length (live_degrees == nullptr) or by
@@ -123,8 +124,6 @@ struct Plan {
   // rows with 0, 1, 2, >= 3 in the minimum activity, 4-7 the maximum.
   uint32_t* inf_hist = nullptr;
   const uint8_t* rule_entry_keep_col = nullptr;
-  const double* ref_l = nullptr;
-  const double* ref_u = nullptr;
   bool has_new_A = false;
   DevCsr new_A;                  // owned when has_new_A
   std::vector<PostsolveSegment> tape;   // local indices until captured
@@ -144,6 +143,9 @@ struct Stats {
   // Incremental refresh: the masks the statistics describe, the rows and
   // columns deleted since, and which of them need their flags recomputed.
   bool valid = false;
+  // Changes with every refresh: two sweeps over degrees of one version need
+  // the row queues built once.  Never 0.
+  uint64_t version = 0;
   DBuf<uint8_t> seen_row, seen_col, dirty_row, dirty_col;
   DBuf<int32_t> deleted, counters;
 };
@@ -180,18 +182,20 @@ void live_stats_side(const DevCsr& M, const uint8_t* keep_outer, const uint8_t* 
 void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan);
 void allocate_stats(Stats& st, int32_t m, int32_t n);
 // Packs {l_j, u_j} of every column (a removed one as the reserved NaN pair).
+// With cand_l / cand_u, also copies the bounds there (the sweep's candidates
+// start from them).
 void pack_bounds(const double* l, const double* u, const uint8_t* keep_col, int32_t n, double2* lu,
-                 cudaStream_t s);
+                 cudaStream_t s, double* cand_l = nullptr, double* cand_u = nullptr);
 void row_activity_summary_packed(const DevCsr& A, const double2* lu, double zero_tol, const uint8_t* keep_row,
                                  const int32_t* live_deg, double* min_fin, double* max_fin, int32_t* min_inf,
-                                 int32_t* max_inf, cudaStream_t s);
+                                 int32_t* max_inf, cudaStream_t s, uint64_t degrees_version = 0);
 void row_activity_summary(const DevCsr& A, const double* l, const double* u, double zero_tol,
                           const uint8_t* keep_row, const uint8_t* keep_col, const int32_t* live_deg,
                           double* min_fin, double* max_fin, int32_t* min_inf, int32_t* max_inf,
                           cudaStream_t s);
 void row_plain_minmax(const DevCsr& A, const double* l, const double* u, const uint8_t* keep_row,
                       const uint8_t* keep_col, const int32_t* live_deg, double* row_min, double* row_max,
-                      cudaStream_t s);
+                      cudaStream_t s, uint64_t degrees_version = 0);
 void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStream_t s);
 
 // compact.cu

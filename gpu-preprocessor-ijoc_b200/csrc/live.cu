@@ -16,6 +16,7 @@
 #include "live_visit.cuh"
 
 #include <array>
+#include <atomic>
 
 namespace gpp {
 
@@ -310,10 +311,17 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
 }
 
 __global__ void pack_bounds_kernel(int n, const double* __restrict__ l, const double* __restrict__ u,
-                                   const uint8_t* __restrict__ keep, double2* __restrict__ lu) {
+                                   const uint8_t* __restrict__ keep, double2* __restrict__ lu,
+                                   double* __restrict__ cand_l, double* __restrict__ cand_u) {
   const double removed = __longlong_as_double(static_cast<long long>(kRemovedColumnBits));
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-    lu[j] = !keep || keep[j] ? make_double2(l[j], u[j]) : make_double2(removed, removed);
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const double lj = l[j], uj = u[j];
+    lu[j] = !keep || keep[j] ? make_double2(lj, uj) : make_double2(removed, removed);
+    if (cand_l) {
+      cand_l[j] = lj;
+      cand_u[j] = uj;
+    }
+  }
 }
 
 // Live degree / singleton support.  Counts and the max live position are
@@ -819,24 +827,32 @@ void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan) {
     st.nnz_known = -1;
     st.nnz_seq = seq;
   }
+  static std::atomic<uint64_t> versions{0};
+  st.version = ++versions;
   st.valid = true;
 }
 
 void pack_bounds(const double* l, const double* u, const uint8_t* keep_col, int32_t n, double2* lu,
-                 cudaStream_t s) {
+                 cudaStream_t s, double* cand_l, double* cand_u) {
   if (n <= 0) return;
-  GPP_LAUNCH_BYTES(pack_bounds_kernel, 33.0 * n, grid_stride_blocks(n), kThreads, 0, s, n, l, u, keep_col, lu);
+  GPP_LAUNCH_BYTES(pack_bounds_kernel, (cand_l ? 49.0 : 33.0) * n, grid_stride_blocks(n), kThreads, 0, s, n, l, u,
+                   keep_col, lu, cand_l, cand_u);
 }
 
 namespace {
 template <bool Plain>
 void launch_activity(const DevCsr& A, const double2* lu, double zero_tol, const uint8_t* keep_row,
                      const int32_t* live_deg, double* lo, double* hi, int32_t* ni, int32_t* pi, double out_bytes,
-                     cudaStream_t s) {
+                     cudaStream_t s, uint64_t degrees_version) {
   static thread_local RowSchedule* live_schedule = new RowSchedule;  // never destroyed (see schedule_cache)
   const RowSchedule* sch;
   if (live_deg) {
-    build_schedule(*live_schedule, A, live_deg, s);
+    // Statistics versions are unique in the process, so one names its matrix
+    // and degrees; callers with degrees of their own give 0.
+    if (degrees_version == 0 || live_schedule->degrees_version != degrees_version) {
+      build_schedule(*live_schedule, A, live_deg, s);
+      live_schedule->degrees_version = degrees_version;
+    }
     sch = live_schedule;
   } else {
     sch = &stored_schedule(A);
@@ -860,10 +876,11 @@ void launch_activity(const DevCsr& A, const double2* lu, double zero_tol, const 
 
 void row_activity_summary_packed(const DevCsr& A, const double2* lu, double zero_tol, const uint8_t* keep_row,
                                  const int32_t* live_deg, double* min_fin, double* max_fin, int32_t* min_inf,
-                                 int32_t* max_inf, cudaStream_t s) {
+                                 int32_t* max_inf, cudaStream_t s, uint64_t degrees_version) {
   // compute_row_activity_summary (gpu_presolve_kernels.cu:744-787).
   if (!A.rows) return;
-  launch_activity<false>(A, lu, zero_tol, keep_row, live_deg, min_fin, max_fin, min_inf, max_inf, 24.0, s);
+  launch_activity<false>(A, lu, zero_tol, keep_row, live_deg, min_fin, max_fin, min_inf, max_inf, 24.0, s,
+                         degrees_version);
 }
 
 void row_activity_summary(const DevCsr& A, const double* l, const double* u, double zero_tol,
@@ -878,12 +895,13 @@ void row_activity_summary(const DevCsr& A, const double* l, const double* u, dou
 
 void row_plain_minmax(const DevCsr& A, const double* l, const double* u, const uint8_t* keep_row,
                       const uint8_t* keep_col, const int32_t* live_deg, double* row_min, double* row_max,
-                      cudaStream_t s) {
+                      cudaStream_t s, uint64_t degrees_version) {
   // Row sums of the redundant-row rule (rule_infeasible_and_redundant_rows.cu:46-156).
   if (!A.rows) return;
   DBuf<double2> lu(size_t(std::max(A.cols, 1)), s);
   pack_bounds(l, u, keep_col, A.cols, lu.p, s);
-  launch_activity<true>(A, lu.p, 0.0, keep_row, live_deg, row_min, row_max, nullptr, nullptr, 16.0, s);
+  launch_activity<true>(A, lu.p, 0.0, keep_row, live_deg, row_min, row_max, nullptr, nullptr, 16.0, s,
+                        degrees_version);
 }
 
 void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStream_t s) {

@@ -130,8 +130,7 @@ candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, CandArgs g)
 // _kernel_finalize_bound_strengthening (reference :646-796).
 __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
                                 const double* __restrict__ u, const double* __restrict__ cand_l,
-                                const double* __restrict__ cand_u, const double* __restrict__ ref_l,
-                                const double* __restrict__ ref_u, const double* __restrict__ c,
+                                const double* __restrict__ cand_u, const double* __restrict__ c,
                                 const double* __restrict__ vmax_arr, int preserve_free_zero_cost, double zero_tol,
                                 double ft, double upper_relax, double* __restrict__ fl, double* __restrict__ fu,
                                 uint8_t* __restrict__ lch, uint8_t* __restrict__ uch, uint8_t* __restrict__ fx,
@@ -152,7 +151,7 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
     if (isfinite(cl)) el = fmax(el, cl);
     if (isfinite(cu)) eu = fmin(eu, cu);
     if (el > eu + ft) { found |= 1u; continue; }
-    const bool was_free = !isfinite(ref_l[j]) && !isfinite(ref_u[j]);
+    const bool was_free = !isfinite(lj) && !isfinite(uj);   // the bounds at the phase's start
     const bool box = isfinite(cl) && isfinite(cu);
     const bool zero_cost = fabs(c[j]) <= zero_tol;
     const bool nearly_fixed = box && (cu <= cl || (cu - cl) * vmax <= ft);
@@ -367,12 +366,11 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   auto s = ctx().stream;
   DBuf<double> cl(size_t(n), s), cu(size_t(n), s), mn(size_t(m), s), mx(size_t(m), s), vmax(size_t(n), s);
   DBuf<int32_t> ni(size_t(m), s), pi(size_t(m), s);
-  cl.copy_from(plan.l.p, size_t(n));
-  cu.copy_from(plan.u.p, size_t(n));
   // One packed bounds array serves the activity sweep and the candidate sweep.
   DBuf<double2> lu(size_t(n), s);
-  pack_bounds(plan.l.p, plan.u.p, plan.keep_col.p, n, lu.p, s);
-  row_activity_summary_packed(lp.A, lu.p, p.zero_tol, plan.keep_row.p, stats.row_nnz.p, mn.p, mx.p, ni.p, pi.p, s);
+  pack_bounds(plan.l.p, plan.u.p, plan.keep_col.p, n, lu.p, s, cl.p, cu.p);
+  row_activity_summary_packed(lp.A, lu.p, p.zero_tol, plan.keep_row.p, stats.row_nnz.p, mn.p, mx.p, ni.p, pi.p, s,
+                              stats.version);
   const RowSummary rs{mn.p, mx.p, ni.p, pi.p};
   if (plan.inf_hist) {
     check(cudaMemsetAsync(plan.inf_hist, 0, 8 * sizeof(uint32_t), s), "inf_hist");
@@ -390,11 +388,9 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   col_max_abs(lp.AT, plan.keep_row.p, vmax.p, s);
   DBuf<double> fl(size_t(n), s), fu(size_t(n), s), fixv(size_t(n), s);
   DBuf<uint8_t> lch(size_t(n), s), uch(size_t(n), s), fx(size_t(n), s);
-  const double* ref_l = plan.ref_l ? plan.ref_l : plan.l.p;
-  const double* ref_u = plan.ref_u ? plan.ref_u : plan.u.p;
   Report report = ctx().open_report(1);
   GPP_LAUNCH(finalize_kernel, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.l.p, plan.u.p, cl.p,
-             cu.p, ref_l, ref_u, plan.c.p, vmax.p, int(p.bound_strengthening_preserve_free_zero_cost), p.zero_tol,
+             cu.p, plan.c.p, vmax.p, int(p.bound_strengthening_preserve_free_zero_cost), p.zero_tol,
              p.feasibility_tol, p.bound_strengthening_upper_relaxation_factor, fl.p, fu.p, lch.p, uch.p, fx.p,
              fixv.p, report);
   const uint32_t found = uint32_t(ctx().await(report)[0]);

@@ -173,38 +173,57 @@ int32_t list_flagged(int count, const int32_t* flag, const int32_t* ids, int32_t
       s);
 }
 
-// Matching round (:989-1027): reset the owners of the active rows' columns,
-// claim by atomicMin, select rows owning both columns.
-__global__ void dt_reset(int k, const int32_t* __restrict__ rows, const uint8_t* __restrict__ active,
-                         const int32_t* __restrict__ keep_c, const int32_t* __restrict__ elim_c,
-                         int32_t* __restrict__ owner) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x)
-    if (active[q]) { const int i = rows[q]; owner[keep_c[i]] = INT_MAX; owner[elim_c[i]] = INT_MAX; }
-}
-__global__ void dt_claim(int k, const int32_t* __restrict__ rows, const uint8_t* __restrict__ active,
-                         const uint8_t* __restrict__ blocked, const int32_t* __restrict__ keep_c,
-                         const int32_t* __restrict__ elim_c, int32_t* __restrict__ owner) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) {
-    if (!active[q]) continue;
-    const int i = rows[q], kc = keep_c[i], ec = elim_c[i];
-    if (!blocked[kc] && !blocked[ec]) { atomicMin(owner + kc, i); atomicMin(owner + ec, i); }
+// Matching rounds (:989-1027): each active row claims its two columns, and a
+// row that owns both is selected.  A claim is the row below the number of
+// rounds to come, combined by atomicMin, so a round's claims displace those of
+// the rounds before and nothing is reset between rounds.
+struct Matching {
+  int count;
+  const int32_t* rows;
+  uint8_t* active;
+  uint8_t* blocked;
+  const int32_t *keep_c, *elim_c;
+  unsigned long long* owner;   // all ones at the start
+  int32_t* selected;
+  __device__ __forceinline__ unsigned long long claim_of(int round, int i) const {
+    return ((unsigned long long)(kRounds - 1 - round) << 32) | unsigned(i);
   }
-}
-__global__ void dt_select(int k, const int32_t* __restrict__ rows, uint8_t* __restrict__ active,
-                          uint8_t* __restrict__ blocked, const int32_t* __restrict__ keep_c,
-                          const int32_t* __restrict__ elim_c, const int32_t* __restrict__ owner,
-                          int32_t* __restrict__ selected) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) {
-    if (!active[q]) continue;
+  __device__ __forceinline__ void claim(int round, int q) const {
+    if (!active[q]) return;
+    const int i = rows[q], kc = keep_c[i], ec = elim_c[i];
+    if (blocked[kc] || blocked[ec]) return;
+    atomicMin(owner + kc, claim_of(round, i));
+    atomicMin(owner + ec, claim_of(round, i));
+  }
+  __device__ __forceinline__ void select(int round, int q) const {
+    if (!active[q]) return;
     const int i = rows[q], kc = keep_c[i], ec = elim_c[i];
     // A column has one owner, so no row reads a block set in this round by
     // a row it would compete with.
-    if (!blocked[kc] && !blocked[ec] && owner[kc] == i && owner[ec] == i) {
+    const unsigned long long mine = claim_of(round, i);
+    if (!blocked[kc] && !blocked[ec] && __ldcg(owner + kc) == mine && __ldcg(owner + ec) == mine) {
       selected[q] = 1;
       active[q] = 0;
       blocked[kc] = 1;
       blocked[ec] = 1;
     }
+  }
+};
+__global__ void dt_claim(Matching g, int round) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.count; q += gridDim.x * blockDim.x) g.claim(round, q);
+}
+__global__ void dt_select(Matching g, int round) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.count; q += gridDim.x * blockDim.x) g.select(round, q);
+}
+// All rounds in one block: up to kBlockMatch rows the sixteen launches cost
+// more than the rows.
+constexpr int kBlockMatch = 4096;
+__global__ void __launch_bounds__(1024) dt_match_block(Matching g) {
+  for (int round = 0; round < kRounds; ++round) {
+    for (int q = threadIdx.x; q < g.count; q += blockDim.x) g.claim(round, q);
+    __syncthreads();
+    for (int q = threadIdx.x; q < g.count; q += blockDim.x) g.select(round, q);
+    __syncthreads();
   }
 }
 
@@ -806,16 +825,21 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
 
   // Matching rounds over the acceptable rows (ascending).
   DBuf<uint8_t> active(size_t(acceptable), s), blocked(size_t(n), s);
-  DBuf<int32_t> owner(size_t(n), s), chosen(size_t(acceptable), s), rows(size_t(acceptable), s);
+  DBuf<unsigned long long> owner(size_t(n), s);
+  DBuf<int32_t> chosen(size_t(acceptable), s), rows(size_t(acceptable), s);
   check(cudaMemsetAsync(active.p, 1, size_t(acceptable), s), "doubleton active");
+  check(cudaMemsetAsync(owner.p, 0xff, sizeof(unsigned long long) * size_t(n), s), "doubleton owners");
   blocked.zero();
   chosen.zero();
-  const int gk = grid_stride_blocks(acceptable);
-  for (int round = 0; round < kRounds; ++round) {
-    GPP_LAUNCH(dt_reset, gk, kThreads, 0, s, acceptable, acc.p, active.p, keep_c.p, elim_c.p, owner.p);
-    GPP_LAUNCH(dt_claim, gk, kThreads, 0, s, acceptable, acc.p, active.p, blocked.p, keep_c.p, elim_c.p, owner.p);
-    GPP_LAUNCH(dt_select, gk, kThreads, 0, s, acceptable, acc.p, active.p, blocked.p, keep_c.p, elim_c.p, owner.p,
-               chosen.p);
+  const Matching match{acceptable, acc.p, active.p, blocked.p, keep_c.p, elim_c.p, owner.p, chosen.p};
+  if (acceptable <= kBlockMatch) {
+    GPP_LAUNCH(dt_match_block, 1, 1024, 0, s, match);
+  } else {
+    const int gk = grid_stride_blocks(acceptable);
+    for (int round = 0; round < kRounds; ++round) {
+      GPP_LAUNCH(dt_claim, gk, kThreads, 0, s, match, round);
+      GPP_LAUNCH(dt_select, gk, kThreads, 0, s, match, round);
+    }
   }
   const int sel = list_flagged(acceptable, chosen.p, acc.p, rows.p, s);
   const double ratio = double(sel) / double(acceptable);

@@ -194,7 +194,8 @@ void rule_redundant_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, co
   auto s = ctx().stream;
   DBuf<double> mn(size_t(m), s), mx(size_t(m), s);
   DBuf<uint8_t> action(size_t(m), s);
-  row_plain_minmax(lp.A, plan.l.p, plan.u.p, plan.keep_row.p, plan.keep_col.p, stats.row_nnz.p, mn.p, mx.p, s);
+  row_plain_minmax(lp.A, plan.l.p, plan.u.p, plan.keep_row.p, plan.keep_col.p, stats.row_nnz.p, mn.p, mx.p, s,
+                   stats.version);
   const Report report = ctx().open_report(1);
   GPP_LAUNCH(redundant_classify, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p,
              plan.AL.p, plan.AU.p, mn.p, mx.p, p.bound_tol, action.p, report);

@@ -80,13 +80,15 @@ __global__ void fd_starts(int n, const uint64_t* __restrict__ keys, double tol, 
     start[i] = new_id || new_sig ? 1 : 0;
   }
 }
+// Also marks the members that have their colour to themselves.
 __global__ void fd_write(int n, const int32_t* __restrict__ perm, const int32_t* __restrict__ start,
                          const int32_t* __restrict__ excl, int write_sig, uint64_t seed, int32_t* __restrict__ ids,
-                         double* __restrict__ sig_out) {
+                         double* __restrict__ sig_out, uint8_t* __restrict__ alone) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int id = excl[i] + start[i];   // inclusive scan: colours are 1-based
     const int member = perm[i];
     ids[member] = id;
+    alone[member] = start[i] && (i + 1 == n || start[i + 1]);
     if (write_sig) sig_out[member] = color_signature(seed, id);
   }
 }
@@ -95,23 +97,95 @@ __global__ void fd_signatures(int n, const int32_t* __restrict__ ids, uint64_t s
     sig[i] = color_signature(seed, ids[i]);
 }
 
-// y = M x, one warp per row; lane 0 adds the row's products in stored order.
-__global__ void fd_spmv(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                        const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y) {
+// y = M x for the rows that share their colour, each row's products added in
+// stored order (the sums fix the reference's association).  A row alone in its
+// colour cannot be split off again, so its signature decides nothing and is
+// not formed (y = 0): on the random LPs most colours are such, and in the
+// replicated ones so is the coupling row, whose 120,000 products, added one by
+// one, were 1.5 ms of each sweep.  A warp takes 32 consecutive rows: rows of
+// up to kSpmvThread entries one per lane, longer ones by the whole warp, and
+// rows past kSpmvWarp entries are listed for blocks.
+constexpr int kSpmvThread = 16;
+constexpr int kSpmvWarp = 1024;
+__global__ void __launch_bounds__(kThreads)
+fd_spmv(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
+        const double* __restrict__ x, const uint8_t* __restrict__ alone, double* __restrict__ y,
+        int32_t* __restrict__ long_rows, int32_t* long_count) {
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
-    double acc = 0.0;
-    for (offset_t chunk = ptr[r]; chunk < ptr[r + 1]; chunk += 32) {
-      const offset_t p = chunk + lane;
-      const double t = p < ptr[r + 1] ? val[p] * x[idx[p]] : 0.0;
-      const int live = int(min(offset_t(32), ptr[r + 1] - chunk));
-      for (int k = 0; k < live; ++k) {
-        const double v = __shfl_sync(0xffffffffu, t, k);
-        if (lane == 0) acc += v;
+  for (int64_t first = int64_t(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; first < rows;
+       first += int64_t(warps) * 32) {
+    const int64_t r = first + lane;
+    offset_t a = 0, e = 0;
+    bool mine = false;
+    if (r < rows) {
+      mine = !alone[r];
+      if (mine) {
+        a = ptr[r];
+        e = ptr[r + 1];
+      } else {
+        y[r] = 0.0;
       }
     }
-    if (lane == 0) y[r] = acc;
+    if (mine && e - a <= kSpmvThread) {
+      double acc = 0.0;
+      for (offset_t p = a; p < e; ++p) acc += val[p] * x[idx[p]];
+      y[r] = acc;
+    }
+    if (mine && e - a > kSpmvWarp) long_rows[atomicAdd(long_count, 1)] = int32_t(r);
+    unsigned whole = __ballot_sync(0xffffffffu, mine && e - a > kSpmvThread && e - a <= kSpmvWarp);
+    while (whole) {
+      const int src = __ffs(whole) - 1;
+      whole &= whole - 1;
+      const offset_t ra = __shfl_sync(0xffffffffu, a, src), re = __shfl_sync(0xffffffffu, e, src);
+      double acc = 0.0;
+      for (offset_t chunk = ra; chunk < re; chunk += 32) {
+        const offset_t p = chunk + lane;
+        const double t = p < re ? val[p] * x[idx[p]] : 0.0;
+        const int live = int(min(offset_t(32), re - chunk));
+        for (int k = 0; k < live; ++k) {
+          const double v = __shfl_sync(0xffffffffu, t, k);
+          if (lane == 0) acc += v;
+        }
+      }
+      if (lane == 0) y[first + src] = acc;
+    }
+  }
+}
+// The listed long rows, one block each: seven warps form the next products in
+// shared memory while one thread adds the last ones, so a row costs its chain
+// of additions and nothing else.
+constexpr int kSpmvLoaders = kThreads - 32;
+constexpr int kSpmvStage = 8 * kSpmvLoaders;
+__global__ void __launch_bounds__(kThreads)
+fd_spmv_long(const int32_t* __restrict__ long_rows, const int32_t* __restrict__ long_count,
+             const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
+             const double* __restrict__ x, double* __restrict__ y) {
+  __shared__ double stage[2][kSpmvStage];
+  const int count = *long_count;
+  for (int q = blockIdx.x; q < count; q += gridDim.x) {
+    const int r = long_rows[q];
+    const offset_t a = ptr[r], e = ptr[r + 1];
+    const int chunks = int((int64_t(e) - a + kSpmvStage - 1) / kSpmvStage);
+    double acc = 0.0;
+    for (int c = 0; c <= chunks; ++c) {
+      if (threadIdx.x >= 32 && c < chunks) {
+        const int64_t base = int64_t(a) + int64_t(c) * kSpmvStage + (threadIdx.x - 32);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int64_t p = base + k * kSpmvLoaders;
+          if (p < e) stage[c & 1][k * kSpmvLoaders + threadIdx.x - 32] = val[p] * x[idx[p]];
+        }
+      }
+      if (threadIdx.x == 0 && c > 0) {
+        const double* s = stage[(c - 1) & 1];
+        const int n = int(min(int64_t(kSpmvStage), int64_t(e) - a - int64_t(c - 1) * kSpmvStage));
+#pragma unroll 8
+        for (int k = 0; k < n; ++k) acc += s[k];
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) y[r] = acc;
   }
 }
 
@@ -119,6 +193,7 @@ struct Side {
   int n = 0;
   int colors = 1;
   DBuf<int32_t> ids, perm, start, excl;
+  DBuf<uint8_t> alone;
   DBuf<uint64_t> keys;
   DBuf<double> sig;
   void alloc(int count, cudaStream_t s) {
@@ -129,6 +204,7 @@ struct Side {
     excl.alloc(size_t(n) + 1, s);
     keys.alloc(size_t(n), s);
     sig.alloc(size_t(n), s);
+    alone.alloc(size_t(n), s);
     ids.zero();
   }
   // update_color_id (folding_kernels.cu:165-210): split colours by the float
@@ -139,7 +215,24 @@ struct Side {
     radix_sort_pairs(keys.p, perm.p, n, s, (bits_up_to(n) << 32) | 0xffffffffu);
     GPP_LAUNCH(fd_starts, g, kThreads, 0, s, n, keys.p, tol, start.p);
     exclusive_scan_i32(start.p, excl.p, n, s);
-    GPP_LAUNCH(fd_write, g, kThreads, 0, s, n, perm.p, start.p, excl.p, int(write_sig), seed, ids.p, sig.p);
+    GPP_LAUNCH(fd_write, g, kThreads, 0, s, n, perm.p, start.p, excl.p, int(write_sig), seed, ids.p, sig.p,
+               alone.p);
+  }
+  // One refinement step: split the colours by the signatures M x.  With every
+  // member alone nothing can split, and only the colours' own signatures of
+  // the round are needed.
+  void refine(const gpp_csr& M, const double* x, double tol, uint64_t seed, DBuf<double>& value,
+              DBuf<int32_t>& long_rows, cudaStream_t s) {
+    if (colors == n) {
+      GPP_LAUNCH(fd_signatures, grid_stride_blocks(n), kThreads, 0, s, n, ids.p, seed, sig.p);
+      return;
+    }
+    int32_t* long_count = long_rows.p + n;
+    check(cudaMemsetAsync(long_count, 0, sizeof(int32_t), s), "long rows");
+    GPP_LAUNCH(fd_spmv, grid_stride_blocks(n), kThreads, 0, s, n, M.rowPtr, M.colVal, M.nzVal, x, alone.p, value.p,
+               long_rows.p, long_count);
+    GPP_LAUNCH(fd_spmv_long, kNumSMs, kThreads, 0, s, long_rows.p, long_count, M.rowPtr, M.colVal, M.nzVal, x, value.p);
+    update(value.p, tol, true, seed, s);
   }
   int count() { return read_scalar(excl.p + n); }
 };
@@ -162,17 +255,14 @@ bool refine(const gpp_lp& lp, double tol, Side& rows, Side& cols, cudaStream_t s
   GPP_LAUNCH(fd_signatures, grid_stride_blocks(cols.n), kThreads, 0, s, cols.n, cols.ids.p, round_seed(0, 5),
              cols.sig.p);
   if (too_little(rows, cols)) return false;
-  DBuf<double> col_value(size_t(cols.n), s), row_value(size_t(rows.n), s);
+  const size_t most = size_t(std::max(rows.n, cols.n));
+  DBuf<double> value(most, s);
+  DBuf<int32_t> long_rows(most + 1, s);
   const int max_round = std::max(1, rows.n + cols.n);
-  const int gr = std::max(1, std::min((cols.n + 7) / 8, kNumSMs * 16));
-  const int gc = std::max(1, std::min((rows.n + 7) / 8, kNumSMs * 16));
   for (int round = 1; round <= max_round; ++round) {
-    GPP_LAUNCH(fd_spmv, gr, kThreads, 0, s, cols.n, lp.AT.rowPtr, lp.AT.colVal, lp.AT.nzVal, rows.sig.p,
-               col_value.p);
     const int prev_cols = cols.colors, prev_rows = rows.colors;
-    cols.update(col_value.p, tol, true, round_seed(round, 1), s);
-    GPP_LAUNCH(fd_spmv, gc, kThreads, 0, s, rows.n, lp.A.rowPtr, lp.A.colVal, lp.A.nzVal, cols.sig.p, row_value.p);
-    rows.update(row_value.p, tol, true, round_seed(round, 2), s);
+    cols.refine(lp.AT, rows.sig.p, tol, round_seed(round, 1), value, long_rows, s);
+    rows.refine(lp.A, cols.sig.p, tol, round_seed(round, 2), value, long_rows, s);
     rows.colors = rows.count();
     cols.colors = cols.count();
     if (too_little(rows, cols)) return false;
@@ -265,17 +355,24 @@ __global__ void fd_reduce_bounds(int colors, const int32_t* __restrict__ members
 }
 
 // kernel_emit_triplet_warp (folding_reduce.cu:52-74): entry key (R-1)*C +
-// (C-1), value a_ij / |R|.
-__global__ void fd_entries(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+// (C-1), value a_ij / |R|.  Every warp takes kEntryRun consecutive entries, so
+// a long row is spread over as many warps as it needs; an entry finds its row
+// between the rows of the run's first and last entry.
+constexpr int kEntryRun = 128;
+__global__ void fd_entries(int rows, int64_t nnz, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                            const double* __restrict__ val, const int32_t* __restrict__ rid,
                            const int32_t* __restrict__ cid, const int32_t* __restrict__ rcount, int ncc,
                            uint64_t* __restrict__ keys, int32_t* __restrict__ order, double* __restrict__ weighted) {
   const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
-    const int R = rid[r];
-    const double w = 1.0 / double(rcount[R - 1]);
-    for (offset_t p = ptr[r] + lane; p < ptr[r + 1]; p += 32) {
+  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t first = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kEntryRun; first < nnz;
+       first += warps * kEntryRun) {
+    const int64_t last = min(nnz, first + kEntryRun) - 1;
+    const int r0 = row_of(ptr, 0, rows, offset_t(first)), r1 = row_of(ptr, r0, rows, offset_t(last));
+    for (int64_t p = first + lane; p <= last; p += 32) {
+      const int r = row_of(ptr, r0, r1 + 1, offset_t(p));
+      const int R = rid[r];
+      const double w = 1.0 / double(rcount[R - 1]);
       keys[p] = uint64_t(R - 1) * uint64_t(ncc) + uint64_t(cid[idx[p]] - 1);
       order[p] = int32_t(p);
       weighted[p] = val[p] * w;
@@ -384,8 +481,8 @@ void run_folding(const gpp_lp& lp, double tolerance, FoldingResult& out) {
     DBuf<uint64_t> keys(size_t(nnz), s);
     DBuf<int32_t> order(size_t(nnz), s), head(size_t(nnz) + 1, s), hpos(size_t(nnz) + 1, s);
     DBuf<double> weighted(size_t(nnz), s);
-    GPP_LAUNCH(fd_entries, std::max(1, std::min((lp.A.rows + 7) / 8, kNumSMs * 16)), kThreads, 0, s, lp.A.rows,
-               lp.A.rowPtr, lp.A.colVal, lp.A.nzVal, rows.ids.p, cols.ids.p, rm.counts.p, nc, keys.p, order.p,
+    GPP_LAUNCH(fd_entries, grid_stride_blocks(nnz / (kEntryRun / 32) + 1), kThreads, 0, s, lp.A.rows, nnz, lp.A.rowPtr,
+               lp.A.colVal, lp.A.nzVal, rows.ids.p, cols.ids.p, rm.counts.p, nc, keys.p, order.p,
                weighted.p);
     radix_sort_pairs(keys.p, order.p, nnz, s, bits_up_to(int64_t(mr) * nc - 1));
     const int g = grid_stride_blocks(nnz);

@@ -54,48 +54,107 @@ __device__ void row_hash_thread(const RowHashArgs& g, int i) {
   g.out[i] = g.use_xor ? mix(h, agg) : h;
 }
 
-// Warp-cooperative version for longer rows: lanes find the first live entry
-// and the live length, XOR aggregates reduce across lanes, the sequential fold
-// is done by lane 0 in stored order.
-__device__ void row_hash_warp(const RowHashArgs& g, int i) {
-  const int lane = threadIdx.x & 31;
-  if (!g.keep_row[i]) { if (lane == 0) g.out[i] = uint64_t(i); return; }
+// Long rows (past kLongRow stored entries), one block per row.  The FNV fold
+// visits the entries in stored order, two dependent 64-bit multiplications
+// each, so one thread does nothing else: the other seven warps form the live
+// entries' (column, bits of value / pivot) pairs of the next stage in shared
+// memory meanwhile.  A warp that did both, through shuffles, took 0.9 ms for
+// the 5,000-entry hub rows of the 29.8M-nnz LP.
+constexpr int kHashLoaders = kThreads - 32;
+struct HashStage {
+  uint64_t col[kHashLoaders], bits[kHashLoaders];
+  int count;
+};
+__device__ void row_hash_block(const RowHashArgs& g, int i, HashStage* stage) {
+  __shared__ int warp_live[kThreads / 32];
+  __shared__ long long first_live;
+  __shared__ int live_len;
+  __shared__ unsigned long long agg_shared;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (!g.keep_row[i]) {   // block-uniform
+    if (threadIdx.x == 0) g.out[i] = uint64_t(i);
+    return;
+  }
   const offset_t a = g.ptr[i], e = g.ptr[i + 1];
+  if (threadIdx.x == 0) {
+    first_live = LLONG_MAX;
+    live_len = 0;
+    agg_shared = 0;
+  }
+  __syncthreads();
   long long first = LLONG_MAX;
   int len = 0;
-  for (offset_t p = a + lane; p < e; p += 32)
+  for (offset_t p = a + offset_t(threadIdx.x); p < e; p += kThreads)
     if (!g.keep_col || g.keep_col[g.idx[p]]) { first = min(first, (long long)p); ++len; }
   for (int off = 16; off; off >>= 1) {
     len += __shfl_xor_sync(0xffffffffu, len, off);
     first = min(first, __shfl_xor_sync(0xffffffffu, first, off));
   }
-  if (len == 0 || fabs(g.val[first]) <= g.tol) { if (lane == 0) g.out[i] = mix(kFnvOffset, uint64_t(i)); return; }
-  const double pivot = g.val[first];
-  const uint64_t h0 = mix(kFnvOffset, uint64_t(len));
+  if (lane == 0 && len) {
+    atomicAdd(&live_len, len);
+    atomicMin(&first_live, first);
+  }
+  __syncthreads();
+  len = live_len;
+  if (len == 0 || fabs(g.val[first_live]) <= g.tol) {
+    if (threadIdx.x == 0) g.out[i] = mix(kFnvOffset, uint64_t(i));
+    __syncthreads();
+    return;
+  }
+  const offset_t from = offset_t(first_live);
+  const double pivot = g.val[from];
+  uint64_t h = mix(kFnvOffset, uint64_t(len));
   if (g.use_xor) {
     uint64_t agg = 0;
-    for (offset_t p = first + lane; p < e; p += 32) {
-      if (g.keep_col && !g.keep_col[g.idx[p]]) continue;
-      agg ^= mix(mix(kFnvOffset, uint64_t(g.idx[p])), dbits(g.val[p] / pivot));
-    }
+    for (offset_t p = from + offset_t(threadIdx.x); p < e; p += kThreads)
+      if (!g.keep_col || g.keep_col[g.idx[p]]) agg ^= mix(mix(kFnvOffset, uint64_t(g.idx[p])), dbits(g.val[p] / pivot));
     for (int off = 16; off; off >>= 1) agg ^= __shfl_xor_sync(0xffffffffu, agg, off);
-    if (lane == 0) g.out[i] = mix(h0, agg);
-  } else {
-    uint64_t h = h0;
-    for (offset_t chunk = first; chunk < e; chunk += 32) {
-      const offset_t p = chunk + lane;
-      const bool live = p < e && (!g.keep_col || g.keep_col[g.idx[p]]);
-      const uint64_t col = live ? uint64_t(g.idx[p]) : 0;
-      const uint64_t b = live ? dbits(g.val[p] / pivot) : 0;
-      const unsigned mask = __ballot_sync(0xffffffffu, live);
-      for (int t = 0; t < 32; ++t) {
-        const uint64_t ct = __shfl_sync(0xffffffffu, col, t);
-        const uint64_t bt = __shfl_sync(0xffffffffu, b, t);
-        if ((mask >> t) & 1u) h = mix(mix(h, ct), bt);
-      }
-    }
-    if (lane == 0) g.out[i] = h;
+    if (lane == 0) atomicXor(&agg_shared, (unsigned long long)agg);
+    __syncthreads();
+    if (threadIdx.x == 0) g.out[i] = mix(h, agg_shared);
+    __syncthreads();
+    return;
   }
+  const int chunks = int((int64_t(e) - from + kHashLoaders - 1) / kHashLoaders);
+  for (int c = 0; c <= chunks; ++c) {
+    HashStage& next = stage[c & 1];
+    bool live = false;
+    uint64_t col = 0, bits = 0;
+    int rank = 0;
+    if (warp > 0 && c < chunks) {
+      const int64_t p = int64_t(from) + int64_t(c) * kHashLoaders + (threadIdx.x - 32);
+      if (p < e) {
+        const int j = g.idx[p];
+        live = !g.keep_col || g.keep_col[j];
+        col = uint64_t(j);
+        if (live) bits = dbits(g.val[p] / pivot);
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, live);
+      rank = __popc(mask & ((1u << lane) - 1u));
+      if (lane == 0) warp_live[warp] = __popc(mask);
+    }
+    __syncthreads();   // the loaders' counts; the fold of the stage before last is over
+    if (warp > 0 && c < chunks) {
+      int before = 0, all = 0;
+      for (int w = 1; w < kThreads / 32; ++w) {
+        before += w < warp ? warp_live[w] : 0;
+        all += warp_live[w];
+      }
+      if (live) {
+        next.col[before + rank] = col;
+        next.bits[before + rank] = bits;
+      }
+      if (threadIdx.x == 32) next.count = all;
+    }
+    if (threadIdx.x == 0 && c > 0) {
+      const HashStage& last = stage[(c - 1) & 1];
+      const int n = last.count;
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) h = mix(mix(h, last.col[k]), last.bits[k]);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) g.out[i] = h;
 }
 
 // Four rows per warp, eight lanes (a group) per row, eight stored entries per
@@ -160,8 +219,10 @@ row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, con
       if (g.ptr[i + 1] - g.ptr[i] <= kShortRow) row_hash_thread(g, i);
     return;
   }
-  // Medium rows four to a warp; long rows (> kLongRow stored entries) one to
-  // a warp, so that no group waits through a long row's rounds.
+  // Long rows (> kLongRow stored entries) first, one to a block; then medium
+  // rows, four to a warp.
+  __shared__ HashStage stage[2];
+  for (int q = b - short_blocks; q < counts[1]; q += int(gridDim.x) - short_blocks) row_hash_block(g, longq[q], stage);
   const int nwarps = (gridDim.x - short_blocks) * (kThreads / 32);
   const int wid = (b - short_blocks) * (kThreads / 32) + (threadIdx.x >> 5);
   const int nmedium = counts[0];
@@ -169,7 +230,6 @@ row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, con
     const int q = q0 + ((threadIdx.x & 31) >> 3);
     row_hash_grouped(g, q < nmedium ? medium[q] : -1);
   }
-  for (int q = wid; q < counts[1]; q += nwarps) row_hash_warp(g, longq[q]);
 }
 
 // Repeated-hash filter.  Only a hash that two or more live items share can
@@ -419,82 +479,176 @@ __global__ void count_guard_groups(int count, const uint64_t* __restrict__ sh, c
   }
 }
 
-// _kernel_parallel_column_groups (rule_parallel_columns.cu:470-628).
-__global__ void col_groups_kernel(int count, const uint64_t* __restrict__ sh, const int32_t* __restrict__ sc,
-                                  const uint8_t* __restrict__ keep_col, const uint8_t* __restrict__ keep_row,
-                                  const double* __restrict__ c, double* l, double* u, const offset_t* __restrict__ ptr,
-                                  const int32_t* __restrict__ idx, const double* __restrict__ val, double zt,
-                                  double coeff_tol, double obj_tol, double max_abs, const int32_t* __restrict__ guard,
-                                  int guard_min, uint8_t* __restrict__ del, uint8_t* __restrict__ fixed,
-                                  double* __restrict__ fval, int32_t* __restrict__ merge_to,
-                                  double* __restrict__ rec_vals, Report report) {
-  uint32_t found_any = 0;   // 1 unbounded, 2 merged, 4 fixed
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count && !(found_any & 1u); s += gridDim.x * blockDim.x) {
-    const uint64_t hs = sh[s];
-    if (s > 0 && sh[s - 1] == hs) continue;
+// _kernel_parallel_column_groups (rule_parallel_columns.cu:470-628): the pairs
+// (j, k) of a hash group in order; a merge moves j's bounds, which the next
+// pairs of j see.  Whether a pair is proportional, and its cost gap, depends
+// on the matrix alone, so a warp tests 32 partners k of j at once and then
+// takes the pairs that act one after the other; a group of up to kGroupThread
+// columns is one thread's.  (2,400 equal singleton columns of the coupling row
+// in the replicated LPs were 4.1 ms of one thread.)
+struct ColumnGroups {
+  const int32_t* sc;
+  const uint8_t *keep_col, *keep_row;
+  const double* c;
+  double *l, *u;
+  const offset_t* ptr;
+  const int32_t* idx;
+  const double* val;
+  double zt, coeff_tol, obj_tol;
+  uint8_t *del, *fixed;
+  double* fval;
+  int32_t* merge_to;
+  double* rec_vals;
+};
+enum ColumnAction : int { kNoAction = 0, kMerge, kFixK, kFixJ, kUnboundedPair };
+
+// What the pair (j, k) with ratio r does given j's bounds; `at` receives the
+// value a column is fixed at.
+__device__ __forceinline__ ColumnAction column_action(const ColumnGroups& g, double gap, double r, double tl, double tu,
+                                                      double sl, double su, double& at) {
+  if (fabs(gap) <= g.obj_tol) return kMerge;
+  bool k_lo = false, k_hi = false, j_lo = false, j_hi = false;
+  if (gap > g.obj_tol) {
+    if (r > 0.0) { k_lo = !isfinite(tu); j_hi = !isfinite(sl); }
+    else { k_lo = !isfinite(tl); j_lo = !isfinite(sl); }
+  } else {
+    if (r > 0.0) { k_hi = !isfinite(tl); j_lo = !isfinite(su); }
+    else { k_hi = !isfinite(tu); j_hi = !isfinite(su); }
+  }
+  if (k_lo || k_hi) {
+    at = k_lo ? sl : su;
+    return isfinite(at) ? kFixK : kUnboundedPair;
+  }
+  if (j_lo || j_hi) {
+    at = j_lo ? tl : tu;
+    return isfinite(at) ? kFixJ : kUnboundedPair;
+  }
+  return kNoAction;
+}
+// Carries the action out; for a merge j's bounds (tl, tu) move.
+__device__ __forceinline__ void column_apply(const ColumnGroups& g, ColumnAction what, int j, int k, double r,
+                                             double& tl, double& tu, double sl, double su, double at) {
+  if (what == kMerge) {
+    g.merge_to[k] = j;
+    double* rec = g.rec_vals + 5 * int64_t(k);
+    rec[0] = r; rec[1] = sl; rec[2] = su; rec[3] = tl; rec[4] = tu;
+    double nl = -INFINITY, nu = INFINITY;
+    if (r > 0.0) { if (isfinite(tl) && isfinite(sl)) nl = tl + r * sl; }
+    else if (isfinite(tl) && isfinite(su)) nl = tl + r * su;
+    if (r > 0.0) { if (isfinite(tu) && isfinite(su)) nu = tu + r * su; }
+    else if (isfinite(tu) && isfinite(sl)) nu = tu + r * sl;
+    tl = nl;
+    tu = nu;
+    g.l[j] = nl;
+    g.u[j] = nu;
+    g.del[k] = 1;
+  } else if (what == kFixK) {
+    g.fixed[k] = 1;
+    g.fval[k] = at;
+  } else if (what == kFixJ) {
+    g.fixed[j] = 1;
+    g.fval[j] = at;
+  }
+}
+__device__ __forceinline__ uint32_t action_flag(ColumnAction what) {   // 1 unbounded, 2 merged, 4 fixed
+  return what == kUnboundedPair ? 1u : what == kMerge ? 2u : what == kNoAction ? 0u : 4u;
+}
+
+constexpr int kGroupThread = 8;
+__global__ void __launch_bounds__(kThreads)
+col_groups_kernel(int count, const uint64_t* __restrict__ sh, ColumnGroups g, double max_abs,
+                  const int32_t* __restrict__ guard, int guard_min, Report report) {
+  uint32_t found = 0;
+  const int lane = threadIdx.x & 31;
+  const double active_max = guard && *guard < guard_min ? INFINITY : max_abs;
+  const int stride = gridDim.x * blockDim.x;
+  const int64_t top = (int64_t(count) + stride - 1) / stride * stride;
+  for (int64_t s64 = blockIdx.x * blockDim.x + threadIdx.x; s64 < top; s64 += stride) {
+    const int s = int(s64);
+    const bool head = s64 < count && (s == 0 || sh[s - 1] != sh[s]);
     int e = s;
-    while (e + 1 < count && sh[e + 1] == hs) ++e;
-    if (e <= s) continue;
-    const double active_max = guard && *guard < guard_min ? INFINITY : max_abs;
-    for (int a = s; a < e && !(found_any & 1u); ++a) {
-      const int j = sc[a];
-      if (!keep_col[j] || del[j] || fixed[j]) continue;
-      for (int b = a + 1; b <= e; ++b) {
-        const int k = sc[b];
-        if (!keep_col[k] || del[k] || fixed[k]) continue;
-        double r;
-        if (!col_ratio(j, k, ptr, idx, val, keep_row, zt, coeff_tol, &r)) continue;
-        if (ratio_guarded(r, active_max)) continue;
-        const double gap = c[k] - r * c[j];
-        const double tl = l[j], tu = u[j], sl = l[k], su = u[k];
-        if (fabs(gap) <= obj_tol) {
-          merge_to[k] = j;
-          rec_vals[5 * int64_t(k) + 0] = r;
-          rec_vals[5 * int64_t(k) + 1] = sl;
-          rec_vals[5 * int64_t(k) + 2] = su;
-          rec_vals[5 * int64_t(k) + 3] = tl;
-          rec_vals[5 * int64_t(k) + 4] = tu;
-          double nl = -INFINITY, nu = INFINITY;
-          if (r > 0.0) { if (isfinite(tl) && isfinite(sl)) nl = tl + r * sl; }
-          else if (isfinite(tl) && isfinite(su)) nl = tl + r * su;
-          if (r > 0.0) { if (isfinite(tu) && isfinite(su)) nu = tu + r * su; }
-          else if (isfinite(tu) && isfinite(sl)) nu = tu + r * sl;
-          l[j] = nl;
-          u[j] = nu;
-          del[k] = 1;
-          found_any |= 2u;
-          continue;
-        }
-        bool k_lo = false, k_hi = false, j_lo = false, j_hi = false;
-        if (gap > obj_tol) {
-          if (r > 0.0) { k_lo = !isfinite(tu); j_hi = !isfinite(sl); }
-          else { k_lo = !isfinite(tl); j_lo = !isfinite(sl); }
-        } else {
-          if (r > 0.0) { k_hi = !isfinite(tl); j_lo = !isfinite(su); }
-          else { k_hi = !isfinite(tu); j_hi = !isfinite(su); }
-        }
-        if (k_lo) {
-          if (!isfinite(sl)) { found_any |= 1u; break; }
-          fixed[k] = 1; fval[k] = sl; found_any |= 4u;
-          continue;
-        } else if (k_hi) {
-          if (!isfinite(su)) { found_any |= 1u; break; }
-          fixed[k] = 1; fval[k] = su; found_any |= 4u;
-          continue;
-        }
-        if (j_lo) {
-          if (!isfinite(tl)) { found_any |= 1u; break; }
-          fixed[j] = 1; fval[j] = tl; found_any |= 4u;
-          break;
-        } else if (j_hi) {
-          if (!isfinite(tu)) { found_any |= 1u; break; }
-          fixed[j] = 1; fval[j] = tu; found_any |= 4u;
-          break;
+    if (head)
+      while (e + 1 < count && e - s < kGroupThread && sh[e + 1] == sh[s]) ++e;
+    const bool large = head && e - s == kGroupThread;   // more than kGroupThread columns
+    if (head && !large && e > s) {
+      for (int a = s; a < e && !(found & 1u); ++a) {
+        const int j = g.sc[a];
+        if (!g.keep_col[j] || g.del[j] || g.fixed[j]) continue;
+        double tl = g.l[j], tu = g.u[j];
+        for (int b = a + 1; b <= e; ++b) {
+          const int k = g.sc[b];
+          if (!g.keep_col[k] || g.del[k] || g.fixed[k]) continue;
+          double r, at = 0.0;
+          if (!col_ratio(j, k, g.ptr, g.idx, g.val, g.keep_row, g.zt, g.coeff_tol, &r)) continue;
+          if (ratio_guarded(r, active_max)) continue;
+          const double sl = g.l[k], su = g.u[k];
+          const ColumnAction what = column_action(g, g.c[k] - r * g.c[j], r, tl, tu, sl, su, at);
+          found |= action_flag(what);
+          if (what == kUnboundedPair) break;
+          column_apply(g, what, j, k, r, tl, tu, sl, su, at);
+          if (what == kFixJ) break;
         }
       }
     }
+    unsigned rest = __ballot_sync(0xffffffffu, large);
+    while (rest) {
+      const int src = __ffs(rest) - 1;
+      rest &= rest - 1;
+      const int gs = __shfl_sync(0xffffffffu, s, src);
+      const uint64_t hash = sh[gs];
+      int ge = gs;   // last column of the group
+      for (;;) {
+        const int at = ge + 1 + lane;
+        const unsigned same = __ballot_sync(0xffffffffu, at < count && sh[at] == hash);
+        const int run = __ffs(~same) - 1;   // lanes from the first on
+        ge += run < 0 ? 32 : run;
+        if (run >= 0) break;
+      }
+      bool stop = false;
+      for (int a = gs; a < ge && !stop; ++a) {
+        const int j = g.sc[a];
+        __syncwarp();
+        if (!g.keep_col[j] || *(volatile uint8_t*)(g.del + j) || *(volatile uint8_t*)(g.fixed + j)) continue;
+        double tl = g.l[j], tu = g.u[j];
+        const double cj = g.c[j];
+        bool done = false;   // j is fixed
+        for (int first = a + 1; first <= ge && !done && !stop; first += 32) {
+          const int b = first + lane;
+          int k = -1;
+          double r = 0.0, gap = 0.0, sl = 0.0, su = 0.0;
+          bool pending = false;
+          if (b <= ge) {
+            k = g.sc[b];
+            pending = g.keep_col[k] && !*(volatile uint8_t*)(g.del + k) && !*(volatile uint8_t*)(g.fixed + k) &&
+                      col_ratio(j, k, g.ptr, g.idx, g.val, g.keep_row, g.zt, g.coeff_tol, &r) &&
+                      !ratio_guarded(r, active_max);
+            if (pending) {
+              gap = g.c[k] - r * cj;
+              sl = g.l[k];
+              su = g.u[k];
+            }
+          }
+          for (;;) {
+            double at = 0.0;
+            const ColumnAction what = pending ? column_action(g, gap, r, tl, tu, sl, su, at) : kNoAction;
+            const unsigned acting = __ballot_sync(0xffffffffu, what != kNoAction);
+            if (!acting) break;
+            const int who = __ffs(acting) - 1;
+            const ColumnAction act = ColumnAction(__shfl_sync(0xffffffffu, int(what), who));
+            found |= action_flag(act);
+            if (act == kUnboundedPair) { stop = true; break; }
+            if (lane == who) column_apply(g, act, j, k, r, tl, tu, sl, su, at);
+            tl = __shfl_sync(0xffffffffu, tl, who);
+            tu = __shfl_sync(0xffffffffu, tu, who);
+            if (act == kFixJ) { done = true; break; }
+            if (lane <= who) pending = false;   // pairs up to this one are over
+          }
+        }
+        __syncwarp();
+      }
+    }
   }
-  post_flags(report, found_any);
+  post_flags(report, found);
 }
 
 __global__ void col_apply(int n, int m, const uint8_t* __restrict__ del, const uint8_t* __restrict__ fixed,
@@ -689,10 +843,11 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
   del.zero();
   fixed.zero();
   const Report report = ctx().open_report(1);
-  GPP_LAUNCH(col_groups_kernel, grid_stride_blocks(count), kThreads, 0, s, count, keys.p, ids.p, plan.keep_col.p,
-             plan.keep_row.p, plan.c.p, plan.l.p, plan.u.p, lp.AT.ptr, lp.AT.idx, lp.AT.val, p.zero_tol, coeff_tol,
-             obj_tol, p.parallel_columns_max_abs_ratio, guard_groups.p,
-             p.parallel_columns_scale_guard_min_groups, del.p, fixed.p, fval.p, merge_to.p, rec.p, report);
+  const ColumnGroups groups{ids.p,       plan.keep_col.p, plan.keep_row.p, plan.c.p, plan.l.p, plan.u.p, lp.AT.ptr,
+                            lp.AT.idx,   lp.AT.val,       p.zero_tol,      coeff_tol, obj_tol,  del.p,    fixed.p,
+                            fval.p,      merge_to.p,      rec.p};
+  GPP_LAUNCH(col_groups_kernel, grid_stride_blocks(count), kThreads, 0, s, count, keys.p, groups,
+             p.parallel_columns_max_abs_ratio, guard_groups.p, p.parallel_columns_scale_guard_min_groups, report);
   const uint32_t found = uint32_t(ctx().await(report)[0]);
   if (found & 1u) { plan.has_unbounded = true; return; }
   const bool merged = (found & 2u) != 0, any_fixed = (found & 4u) != 0;

@@ -256,9 +256,9 @@ __device__ __forceinline__ void post_report(const Report& r) {
     r.mail->seq = r.seq;
   }
 }
-// The same for a report of flags: `flags` of all threads are ORed into word 0
-// (one atomic per block that has any).
-__device__ __forceinline__ void post_flags(const Report& r, uint32_t flags) {
+// ORs the flags of all threads into word 0, one atomic per block that has any
+// (a later kernel posts it).
+__device__ __forceinline__ void gather_flags(const Report& r, uint32_t flags) {
   __shared__ uint32_t block_flags;
   if (threadIdx.x == 0) block_flags = 0;
   flags = __reduce_or_sync(0xffffffffu, flags);
@@ -266,6 +266,10 @@ __device__ __forceinline__ void post_flags(const Report& r, uint32_t flags) {
   if ((threadIdx.x & 31) == 0 && flags) atomicOr(&block_flags, flags);
   __syncthreads();
   if (threadIdx.x == 0 && block_flags) atomicOr(reinterpret_cast<uint32_t*>(r.words), block_flags);
+}
+// The report of a kernel whose answer is flags.
+__device__ __forceinline__ void post_flags(const Report& r, uint32_t flags) {
+  gather_flags(r, flags);
   post_report(r);
 }
 // One thread's answer of up to two values, for kernels that know which thread

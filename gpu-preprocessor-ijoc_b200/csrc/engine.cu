@@ -32,22 +32,30 @@ struct Vectors {
   double *c, *l, *u, *AL, *AU;
 };
 
+__device__ __forceinline__ void copy_at(int k, int m, int n, const Vectors& from, const Vectors& to) {
+  if (k < n) {
+    to.c[k] = from.c[k];
+    to.l[k] = from.l[k];
+    to.u[k] = from.u[k];
+  }
+  if (k < m) {
+    to.AL[k] = from.AL[k];
+    to.AU[k] = from.AU[k];
+  }
+}
+__global__ void copy_vectors(int m, int n, Vectors from, Vectors to) {
+  const int top = n > m ? n : m;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) copy_at(k, m, n, from, to);
+}
+
 // A fresh plan in one launch: all rows and columns kept, the vectors copied.
 __global__ void fresh_plan(int m, int n, Vectors from, Vectors to, uint8_t* __restrict__ keep_row,
                            uint8_t* __restrict__ keep_col) {
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
-    if (k < n) {
-      keep_col[k] = 1;
-      to.c[k] = from.c[k];
-      to.l[k] = from.l[k];
-      to.u[k] = from.u[k];
-    }
-    if (k < m) {
-      keep_row[k] = 1;
-      to.AL[k] = from.AL[k];
-      to.AU[k] = from.AU[k];
-    }
+    if (k < n) keep_col[k] = 1;
+    if (k < m) keep_row[k] = 1;
+    copy_at(k, m, n, from, to);
   }
 }
 
@@ -84,6 +92,7 @@ struct Engine {
   WorkingLp cur;
   bool terminal = false;
   bool active = false, pending = false;
+  bool reshaped = false;   // a rule since the plan's start acted on rows or columns
   Plan plan;
   Stats stats;
   bool stats_dirty = true;
@@ -117,6 +126,7 @@ struct Engine {
     allocate_stats(stats, cur.m(), cur.n());
     stats_dirty = true;
     active = true;
+    reshaped = false;
   }
   void refresh() {
     if (stats_dirty) {
@@ -166,7 +176,7 @@ struct Engine {
       if (plan.has_col_action)
         append_fixed(out.record, plan.keep_col.p, stats.seen_col.p, plan.l.p, plan.u.p, cur.n());
       pending = true;
-      if (plan.has_row_action || plan.has_col_action) stats_dirty = true;
+      if (plan.has_row_action || plan.has_col_action) stats_dirty = reshaped = true;
     } else {
       plan.tape.clear();
     }
@@ -255,11 +265,25 @@ struct Engine {
   }
 
   void materialize(const char* boundary) {
+    // Most propagation rounds move a few bounds and nothing else: then the
+    // vectors are committed and the plan, whose masks still keep everything,
+    // its statistics and its row queues serve the next phase as they are.  A
+    // plan without a change stays open too.
+    if (active && !reshaped && (!pending || cur.owns)) {
+      if (pending) {
+        const int m = cur.m(), n = cur.n();
+        GPP_LAUNCH_BYTES(copy_vectors, 48.0 * n + 32.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s(), m, n,
+                         vectors(plan), vectors(cur));
+        out.trace.push_back(std::string("apply=") + boundary);
+      }
+      pending = false;
+      return;
+    }
     if (active && pending) {
       apply(plan, true);
       out.trace.push_back(std::string("apply=") + boundary);
     }
-    active = pending = false;
+    active = pending = reshaped = false;
     plan = Plan{};
     stats = Stats{};
   }
@@ -281,7 +305,7 @@ struct Engine {
       // so the next deferred rule starts a fresh plan on the new model.
       if (active) {
         if (pending) throw std::logic_error("materialized rule over a plan with unapplied changes");
-        active = false;
+        active = reshaped = false;
         plan = Plan{};
         stats = Stats{};
       }

@@ -8,6 +8,7 @@
 #include <climits>
 
 #include "engine.cuh"
+#include "scan.cuh"
 
 namespace gpp {
 
@@ -134,7 +135,7 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
                                 const double* __restrict__ vmax_arr, int preserve_free_zero_cost, double zero_tol,
                                 double ft, double upper_relax, double* __restrict__ fl, double* __restrict__ fu,
                                 uint8_t* __restrict__ lch, uint8_t* __restrict__ uch, uint8_t* __restrict__ fx,
-                                double* __restrict__ fixv, Report report) {
+                                double* __restrict__ fixv, Report report, bool post) {
   uint32_t found = 0;   // 1 infeasible, 2 a bound moves, 4 a column is fixed
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const double lj = l[j], uj = u[j];
@@ -150,14 +151,14 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
     double el = lj, eu = uj;
     if (isfinite(cl)) el = fmax(el, cl);
     if (isfinite(cu)) eu = fmin(eu, cu);
-    if (el > eu + ft) { found |= 1u; continue; }
+    if (el > eu + ft) { found |= 1u; lch[j] = uch[j] = 0; continue; }
     const bool was_free = !isfinite(lj) && !isfinite(uj);   // the bounds at the phase's start
     const bool box = isfinite(cl) && isfinite(cu);
     const bool zero_cost = fabs(c[j]) <= zero_tol;
     const bool nearly_fixed = box && (cu <= cl || (cu - cl) * vmax <= ft);
     if (preserve_free_zero_cost && was_free && box && zero_cost && !nearly_fixed) { cl = lj; cu = uj; }
     if (isfinite(cl) && cl > lj && isfinite(uj)) {
-      if (cl >= uj + ft) { found |= 1u; continue; }
+      if (cl >= uj + ft) { found |= 1u; lch[j] = uch[j] = 0; continue; }
       if (cl >= uj || (uj - cl) * vmax <= ft) { fj = 1; fat = uj; nl = uj; nu = uj; }
     }
     if (!fj && isfinite(cl) && cl > lj) {
@@ -169,7 +170,7 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
       }
     }
     if (!fj && isfinite(cu) && cu < uj && isfinite(nl)) {
-      if (cu <= nl - ft) { found |= 1u; continue; }
+      if (cu <= nl - ft) { found |= 1u; lch[j] = uch[j] = 0; continue; }
       if (cu <= nl || (cu - nl) * vmax <= ft) { fj = 1; fat = nl; nu = nl; }
     }
     if (!fj && isfinite(cu) && cu < uj) {
@@ -184,10 +185,12 @@ __global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, con
     if (lc || uc) found |= 2u;
     fl[j] = nl; fu[j] = nu; lch[j] = lc; uch[j] = uc; fx[j] = fj; fixv[j] = fat;
   }
-  post_flags(report, found);
+  if (post) post_flags(report, found);
+  else gather_flags(report, found);
 }
 
-// Support rows and per-column tape sizes (reference :815-960, :970-1008).
+// Support rows (reference :815-960); the per-column tape sizes (:970-1008)
+// follow from them in the scan.
 __global__ void support_kernel(int n, const offset_t* __restrict__ at_ptr, const int32_t* __restrict__ at_idx,
                                const double* __restrict__ at_val, const uint8_t* __restrict__ keep_row,
                                const int32_t* __restrict__ row_nnz, const double* __restrict__ AL,
@@ -195,8 +198,7 @@ __global__ void support_kernel(int n, const offset_t* __restrict__ at_ptr, const
                                const double* __restrict__ u, RowSummary rs, const uint8_t* __restrict__ lch,
                                const uint8_t* __restrict__ uch, const double* __restrict__ fl,
                                const double* __restrict__ fu, double zero_tol, double tol, double support_tol,
-                               int32_t* __restrict__ sup_l, int32_t* __restrict__ sup_u,
-                               int64_t* __restrict__ rec_count, int64_t* __restrict__ idx_count) {
+                               int32_t* __restrict__ sup_l, int32_t* __restrict__ sup_u) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     int sl = INT_MAX, su = INT_MAX;
     const bool nl = lch[j], nu = uch[j];
@@ -237,49 +239,50 @@ __global__ void support_kernel(int n, const offset_t* __restrict__ at_ptr, const
     }
     sup_l[j] = sl;
     sup_u[j] = su;
-    rec_count[j] = int64_t(nl) + int64_t(nu);
-    idx_count[j] = (nl ? (sl == INT_MAX ? 1 : 2) : 0) + (nu ? (su == INT_MAX ? 1 : 2) : 0);
   }
 }
 
 constexpr int kVariableBoundChange = 11, kRowImpliedBoundChange = 12, kFixedVariable = 0;
 
-__global__ void pack_bound_records(int n, const uint8_t* __restrict__ lch, const uint8_t* __restrict__ uch,
-                                   const int32_t* __restrict__ sup_l, const int32_t* __restrict__ sup_u,
-                                   const double* __restrict__ l, const double* __restrict__ u,
-                                   const double* __restrict__ fl, const double* __restrict__ fu,
-                                   const int64_t* __restrict__ rec_pos, const int64_t* __restrict__ idx_pos,
-                                   int32_t* __restrict__ types, int64_t* __restrict__ is, int64_t* __restrict__ vs,
-                                   int32_t* __restrict__ idx, double* __restrict__ val) {
+// The bound records of a column (`records` set), then its new bounds and mask.
+struct BoundRecords {
+  const int32_t *sup_l, *sup_u, *rec_pos, *idx_pos;
+  int32_t* types;
+  int64_t *is, *vs;
+  int32_t* idx;
+  double* val;
+};
+__global__ void commit_bounds(int n, const uint8_t* __restrict__ lch, const uint8_t* __restrict__ uch,
+                              const double* __restrict__ fl, const double* __restrict__ fu,
+                              const uint8_t* __restrict__ fx, bool records, BoundRecords rec, double* __restrict__ l,
+                              double* __restrict__ u, uint8_t* __restrict__ keep_col) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    if (j == 0) { is[0] = 0; vs[0] = 0; }
-    if (!lch[j] && !uch[j]) continue;
-    int64_t k = rec_pos[j], ip = idx_pos[j];
-    double cur_l = l[j];
-    const double cur_u = u[j];
-    auto emit = [&](int sup, double a, double b, double c2, double d) {
-      types[k] = sup == INT_MAX ? kVariableBoundChange : kRowImpliedBoundChange;
-      idx[ip++] = j;
-      if (sup != INT_MAX) idx[ip++] = sup;
-      val[4 * k] = a; val[4 * k + 1] = b; val[4 * k + 2] = c2; val[4 * k + 3] = d;
-      is[k + 1] = ip;
-      vs[k + 1] = 4 * (k + 1);
-      ++k;
-    };
-    if (lch[j]) {
-      emit(sup_l[j], cur_l, cur_u, fl[j], cur_u);
-      cur_l = fl[j];
+    const double nl = fl[j], nu = fu[j];
+    if (records) {
+      if (j == 0) { rec.is[0] = 0; rec.vs[0] = 0; }
+      const bool lc = lch[j], uc = uch[j];
+      if (lc || uc) {
+        int64_t k = rec.rec_pos[j], ip = rec.idx_pos[j];
+        double cur_l = l[j];
+        const double cur_u = u[j];
+        auto emit = [&](int sup, double a, double b, double c2, double d) {
+          rec.types[k] = sup == INT_MAX ? kVariableBoundChange : kRowImpliedBoundChange;
+          rec.idx[ip++] = j;
+          if (sup != INT_MAX) rec.idx[ip++] = sup;
+          rec.val[4 * k] = a; rec.val[4 * k + 1] = b; rec.val[4 * k + 2] = c2; rec.val[4 * k + 3] = d;
+          rec.is[k + 1] = ip;
+          rec.vs[k + 1] = 4 * (k + 1);
+          ++k;
+        };
+        if (lc) {
+          emit(rec.sup_l[j], cur_l, cur_u, nl, cur_u);
+          cur_l = nl;
+        }
+        if (uc) emit(rec.sup_u[j], cur_l, cur_u, cur_l, nu);
+      }
     }
-    if (uch[j]) emit(sup_u[j], cur_l, cur_u, cur_l, fu[j]);
-  }
-}
-
-__global__ void apply_bounds(int n, const double* __restrict__ fl, const double* __restrict__ fu,
-                             const uint8_t* __restrict__ fx, double* __restrict__ l, double* __restrict__ u,
-                             uint8_t* __restrict__ keep_col) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    l[j] = fl[j];
-    u[j] = fu[j];
+    l[j] = nl;
+    u[j] = nu;
     if (fx[j]) keep_col[j] = 0;
   }
 }
@@ -388,32 +391,61 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   col_max_abs(lp.AT, plan.keep_row.p, vmax.p, s);
   DBuf<double> fl(size_t(n), s), fu(size_t(n), s), fixv(size_t(n), s);
   DBuf<uint8_t> lch(size_t(n), s), uch(size_t(n), s), fx(size_t(n), s);
+  // Finalisation, support rows and the records' positions run in a row, with
+  // one answer: what was found and the tape sizes.
+  const bool records = p.record_postsolve_tape != 0;
   Report report = ctx().open_report(1);
   GPP_LAUNCH(finalize_kernel, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.l.p, plan.u.p, cl.p,
              cu.p, plan.c.p, vmax.p, int(p.bound_strengthening_preserve_free_zero_cost), p.zero_tol,
              p.feasibility_tol, p.bound_strengthening_upper_relaxation_factor, fl.p, fu.p, lch.p, uch.p, fx.p,
-             fixv.p, report);
-  const uint32_t found = uint32_t(ctx().await(report)[0]);
-  if (found & 1u) { plan.has_infeasible = true; return; }
-  const bool changed = (found & 2u) != 0, fixed = (found & 4u) != 0;
-  if (!changed && !fixed) return;
-  if (p.record_postsolve_tape && changed) {
-    DBuf<int32_t> sl(size_t(n), s), su(size_t(n), s);
-    DBuf<int64_t> rc(size_t(n) + 1, s), ic(size_t(n) + 1, s), rpos(size_t(n) + 1, s), ipos(size_t(n) + 1, s);
+             fixv.p, report, !records);
+  DBuf<int32_t> sl, su, rpos, ipos;
+  if (records) {
+    sl.alloc(size_t(n), s);
+    su.alloc(size_t(n), s);
+    rpos.alloc(size_t(n), s);
+    ipos.alloc(size_t(n), s);
     const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
     GPP_LAUNCH(support_kernel, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val,
                plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, plan.l.p, plan.u.p, rs, lch.p, uch.p, fl.p,
-               fu.p, p.zero_tol, p.bound_tol, support_tol, sl.p, su.p, rc.p, ic.p);
-    const auto [recs, nidx] = exclusive_scan_pair_i64(rc.p, rpos.p, ic.p, ipos.p, n, s);
-    if (recs) {
-      PostsolveSegment seg = make_segment(recs, nidx, 4 * recs);
-      GPP_LAUNCH(pack_bound_records, grid_stride_blocks(n), kThreads, 0, s, n, lch.p, uch.p, sl.p, su.p, plan.l.p,
-                 plan.u.p, fl.p, fu.p, rpos.p, ipos.p, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p);
-      plan.tape.push_back(std::move(seg));
-    }
+               fu.p, p.zero_tol, p.bound_tol, support_tol, sl.p, su.p);
+    scan_items<int32_t, 2>(
+        n,
+        [lch = lch.p, uch = uch.p, sl = sl.p, su = su.p] __device__(int64_t j, int32_t(&v)[2]) {
+          const bool nl = lch[j], nu = uch[j];
+          v[0] = int(nl) + int(nu);
+          if (v[0]) v[1] = (nl ? (sl[j] == INT_MAX ? 1 : 2) : 0) + (nu ? (su[j] == INT_MAX ? 1 : 2) : 0);
+        },
+        [rpos = rpos.p, ipos = ipos.p] __device__(int64_t j, const int32_t(&before)[2], const int32_t(&v)[2]) {
+          if (!v[0]) return;
+          rpos[j] = before[0];
+          ipos[j] = before[1];
+        },
+        [report] __device__(const int32_t(&sum)[2]) {
+          report.mail->words[1] = sum[0];
+          report.mail->words[2] = sum[1];
+          report.mail->words[0] = __ldcg(report.words);
+          report.words[0] = 0;
+          __threadfence_system();
+          report.mail->seq = report.seq;
+        },
+        s);
   }
-  GPP_LAUNCH(apply_bounds, grid_stride_blocks(n), kThreads, 0, s, n, fl.p, fu.p, fx.p, plan.l.p, plan.u.p,
-             plan.keep_col.p);
+  const volatile int64_t* answer = ctx().await(report);
+  const uint32_t found = uint32_t(answer[0]);
+  if (found & 1u) { plan.has_infeasible = true; return; }
+  const bool changed = (found & 2u) != 0, fixed = (found & 4u) != 0;
+  if (!changed && !fixed) return;
+  BoundRecords rec{};
+  PostsolveSegment seg;
+  const int64_t recs = records ? answer[1] : 0, nidx = records ? answer[2] : 0;
+  if (recs) {
+    seg = make_segment(recs, nidx, 4 * recs);
+    rec = BoundRecords{sl.p, su.p, rpos.p, ipos.p, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p};
+  }
+  GPP_LAUNCH(commit_bounds, grid_stride_blocks(n), kThreads, 0, s, n, lch.p, uch.p, fl.p, fu.p, fx.p, recs > 0, rec,
+             plan.l.p, plan.u.p, plan.keep_col.p);
+  if (recs) plan.tape.push_back(std::move(seg));
   double obj_delta = 0.0;
   if (fixed) {
     DBuf<double> shift(size_t(m), s);

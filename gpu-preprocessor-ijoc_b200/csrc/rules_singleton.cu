@@ -61,7 +61,7 @@ __global__ void sc_candidates(int n, int m, const uint8_t* __restrict__ keep_col
                               const double* __restrict__ c, const double* __restrict__ l, const double* __restrict__ u,
                               const double* __restrict__ AL, const double* __restrict__ AU, double zero_tol,
                               int32_t* __restrict__ owner, int32_t* __restrict__ cand, int32_t* __restrict__ rows,
-                              int32_t* __restrict__ long_rows, int32_t* st, Report report) {
+                              int32_t* __restrict__ long_rows, int32_t* st) {
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;   // every thread of a block runs the same trips
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += stride) {
@@ -86,7 +86,6 @@ __global__ void sc_candidates(int n, int m, const uint8_t* __restrict__ keep_col
     const int pl = block_append(st + kStLong, is_long);
     if (is_long) long_rows[pl] = srow[j];
   }
-  post_report(report);
 }
 
 struct RowCache {
@@ -125,14 +124,14 @@ struct CacheOut {
 // other x.  Rows of at most 32 stored entries (nearly all) take eight lanes
 // each, four rows per warp, with all of a row's loads issued before its
 // chain; longer rows take a whole warp, 32 entries at a time.
-__global__ void sc_cache_rows(const int32_t* __restrict__ rows, const int32_t* __restrict__ st,
+__device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, const int32_t* __restrict__ st,
                               const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
                               const int32_t* __restrict__ idx, const double* __restrict__ val,
                               const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
                               const double* __restrict__ u, CacheOut out) {
   const int count = st[kStRows];
   const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
-  const int warps = gridDim.x * (blockDim.x >> 5);
+  const int warps = blocks * (blockDim.x >> 5);
   const auto group_bits = [&](bool v) { return (__ballot_sync(0xffffffffu, v) >> (grp * 8)) & 0xffu; };
   const auto whole_row = [&](int row) {
     RowCache r{0.0, 0.0, 0, 0, 0, 0, 0};
@@ -236,22 +235,18 @@ __global__ void sc_cache_rows(const int32_t* __restrict__ rows, const int32_t* _
 
 // _kernel_singleton_long_row_activity_cache (:642-754): block per row; live
 // rank k goes to thread k mod 256, then a shared-memory halving tree.
-__global__ void __launch_bounds__(kThreads) sc_cache_long(const int32_t* __restrict__ long_rows,
-                                                          const int32_t* __restrict__ st,
-                                                          const int32_t* __restrict__ row_nnz,
-                                                          const offset_t* __restrict__ ptr,
-                                                          const int32_t* __restrict__ idx,
-                                                          const double* __restrict__ val,
-                                                          const uint8_t* __restrict__ keep_col,
-                                                          const double* __restrict__ l, const double* __restrict__ u,
-                                                          CacheOut out) {
+__device__ void sc_cache_long(int block, int blocks, const int32_t* __restrict__ long_rows,
+                              const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz,
+                              const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                              const double* __restrict__ val, const uint8_t* __restrict__ keep_col,
+                              const double* __restrict__ l, const double* __restrict__ u, CacheOut out) {
   __shared__ int slots[kThreads];
   __shared__ int warp_counts[8];
   __shared__ double s_min[kThreads], s_max[kThreads];
   __shared__ int s_cnt[5][kThreads];
   const int count = st[kStLong];
   const int t = threadIdx.x;
-  for (int q = blockIdx.x; q < count; q += gridDim.x) {
+  for (int q = block; q < count; q += blocks) {
     const int row = long_rows[q];
     const offset_t first = ptr[row], last = ptr[row + 1];
     const uint8_t* mask = row_nnz[row] != int(last - first) ? keep_col : nullptr;
@@ -278,6 +273,22 @@ __global__ void __launch_bounds__(kThreads) sc_cache_long(const int32_t* __restr
       out.store(row, RowCache{s_min[0], s_max[0], s_cnt[0][0], s_cnt[1][0], s_cnt[2][0], s_cnt[3][0], s_cnt[4][0]});
     __syncthreads();
   }
+}
+
+// Both roles in one launch: the first `row_blocks` blocks take the claimed
+// rows of up to kLongRow live entries, the rest the long ones.  The grid does
+// not know their numbers (the rule asks the host once, at its end); blocks
+// without rows return at once.
+__global__ void __launch_bounds__(kThreads)
+sc_cache(int row_blocks, const int32_t* __restrict__ rows, const int32_t* __restrict__ long_rows,
+         const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
+         const int32_t* __restrict__ idx, const double* __restrict__ val, const uint8_t* __restrict__ keep_col,
+         const double* __restrict__ l, const double* __restrict__ u, CacheOut out) {
+  if (int(blockIdx.x) < row_blocks)
+    sc_cache_rows(row_blocks, rows, st, row_nnz, ptr, idx, val, keep_col, l, u, out);
+  else
+    sc_cache_long(int(blockIdx.x) - row_blocks, int(gridDim.x) - row_blocks, long_rows, st, row_nnz, ptr, idx, val,
+                  keep_col, l, u, out);
 }
 
 // Propose (:905-1018) over the candidate list.
@@ -367,7 +378,8 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
                          uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ kind,
                          int32_t* __restrict__ winners, int64_t* __restrict__ contrib_idx,
                          double* __restrict__ contrib_val, Report report) {
-  const int count = st[kStRows];
+  // An unbounded candidate ends the rule with the plan as it was.
+  const int count = st[kStUnbounded] ? 0 : st[kStRows];
   const int stride = gridDim.x * blockDim.x;
   const int top = (count + stride - 1) / stride * stride;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < top; q += stride) {
@@ -436,8 +448,7 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
 __global__ void sc_touch(const int32_t* __restrict__ winners, const int32_t* __restrict__ st,
                          const uint8_t* __restrict__ kind, const offset_t* __restrict__ ptr,
                          const int32_t* __restrict__ idx, const uint8_t* __restrict__ keep_col,
-                         uint32_t* __restrict__ claimed, int32_t* __restrict__ touched, int32_t* st_w,
-                         Report report) {
+                         uint32_t* __restrict__ claimed, int32_t* __restrict__ touched, int32_t* st_w) {
   const int count = st[kStWin];
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
@@ -459,7 +470,6 @@ __global__ void sc_touch(const int32_t* __restrict__ winners, const int32_t* __r
       if (take) touched[pos] = col;
     }
   }
-  post_report(report);
 }
 
 // _kernel_apply_singleton_objective_updates_deterministic (:1075-1104): for a
@@ -632,42 +642,36 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   Status st;
   DBuf<int32_t> owner(size_t(m), s), cand(size_t(n), s), rows(size_t(m), s), long_rows(size_t(m), s);
   GPP_LAUNCH(sc_start, grid_stride_blocks(m), kThreads, 0, s, owner.p, m, kUnclaimed, st.d);
-  Report report = ctx().open_report(4, st.d);
   GPP_LAUNCH_BYTES(sc_candidates, double(n) * 11 + 16.0 * n, grid_stride_blocks(n), kThreads, 0, s, n, m,
                    plan.keep_col.p, plan.keep_row.p, stats.singleton_col.p, stats.scol_row.p, stats.scol_val.p,
                    stats.row_nnz.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.zero_tol, owner.p, cand.p,
-                   rows.p, long_rows.p, st.d, report);
-  const volatile int64_t* f = ctx().await(report);
-  if (f[kStUnbounded]) { plan.has_unbounded = true; return; }
-  const int ncand = int(f[kStCand]), nrows = int(f[kStRows]), nlong = int(f[kStLong]);
-  if (ncand == 0) return;
+                   rows.p, long_rows.p, st.d);
 
-  // Activity cache of the claimed rows.
+  // Activity cache of the claimed rows, proposals and their staging follow with
+  // no wait between: the kernels read the candidate and row counts on the
+  // device, and the one answer, after the staging, tells what the rule did.
+  const int claims = std::min(m, n);   // at most: one per row and per candidate
   DBuf<double> fmin(size_t(m), s), fmax(size_t(m), s);
   DBuf<int4> counts(size_t(m), s);
   DBuf<uint8_t> invalid(size_t(m), s);
   const CacheOut cache{fmin.p, fmax.p, counts.p, invalid.p};
-  const int warp_blocks = std::max(1, std::min((nrows + 31) / 32, kNumSMs * 16));
-  GPP_LAUNCH(sc_cache_rows, warp_blocks, kThreads, 0, s, rows.p, st.d, stats.row_nnz.p, lp.A.ptr, lp.A.idx,
-             lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
-  if (nlong)
-    GPP_LAUNCH(sc_cache_long, std::min(nlong, kNumSMs * 8), kThreads, 0, s, long_rows.p, st.d, stats.row_nnz.p,
-               lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
-
-  // Propose and stage.
+  const int row_blocks = std::max(1, std::min((claims + 31) / 32, kNumSMs * 16));
+  const int long_blocks = std::max(1, std::min(kNumSMs * 4, int(lp.A.nnz / kLongRow)));
+  GPP_LAUNCH(sc_cache, row_blocks + long_blocks, kThreads, 0, s, row_blocks, rows.p, long_rows.p, st.d,
+             stats.row_nnz.p, lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
   DBuf<uint8_t> action(size_t(n), s), kind(size_t(m), s);
-  DBuf<double> side(size_t(n), s), contrib_val(size_t(nrows), s);
-  DBuf<int64_t> contrib_idx(size_t(nrows), s);
-  DBuf<int32_t> winners(size_t(nrows), s);
-  GPP_LAUNCH(sc_propose, grid_stride_blocks(ncand), kThreads, 0, s, cand.p, st.d, stats.scol_row.p,
-             stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, fmin.p, fmax.p, counts.p,
-             invalid.p, p.bound_tol, p.zero_tol, action.p, side.p, owner.p);
-  report = ctx().open_report(kStWords, st.d);
-  GPP_LAUNCH(sc_stage, grid_stride_blocks(nrows), kThreads, 0, s, rows.p, st.d, n, action.p, side.p,
+  DBuf<double> side(size_t(n), s), contrib_val(size_t(claims), s);
+  DBuf<int64_t> contrib_idx(size_t(claims), s);
+  DBuf<int32_t> winners(size_t(claims), s);
+  GPP_LAUNCH(sc_propose, grid_stride_blocks(n), kThreads, 0, s, cand.p, st.d, stats.scol_row.p, stats.scol_val.p,
+             plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, fmin.p, fmax.p, counts.p, invalid.p, p.bound_tol,
+             p.zero_tol, action.p, side.p, owner.p);
+  const Report report = ctx().open_report(kStWords, st.d);
+  GPP_LAUNCH(sc_stage, grid_stride_blocks(claims), kThreads, 0, s, rows.p, st.d, n, action.p, side.p,
              stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.bound_tol, owner.p,
-             plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p,
-             report);
-  f = ctx().await(report);
+             plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p, report);
+  const volatile int64_t* f = ctx().await(report);
+  if (f[kStUnbounded]) { plan.has_unbounded = true; return; }
   const int nwin = int(f[kStWin]), nelim = int(f[kStElim]);
   const bool any_side = f[kStSide] != 0;
   if (nelim == 0 && !any_side) return;
@@ -677,13 +681,10 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
     DBuf<uint32_t> claimed(size_t(n + 31) / 32, s);
     claimed.zero();
     DBuf<int32_t> touched(size_t(n), s);
-    report = ctx().open_report(kStWords, st.d);
     GPP_LAUNCH(sc_touch, std::max(1, std::min((nwin + 7) / 8, kNumSMs * 16)), kThreads, 0, s, winners.p, st.d,
-               kind.p, lp.A.ptr, lp.A.idx, plan.keep_col.p, claimed.p, touched.p, st.d, report);
-    const int ntouched = int(ctx().await(report)[kStTouched]);
-    if (ntouched)
-      GPP_LAUNCH(sc_cost, std::max(1, std::min((ntouched + 7) / 8, kNumSMs * 16)), kThreads, 0, s, touched.p, st.d,
-                 n, lp.AT.ptr, lp.AT.idx, lp.AT.val, owner.p, stats.scol_val.p, plan.c.p);
+               kind.p, lp.A.ptr, lp.A.idx, plan.keep_col.p, claimed.p, touched.p, st.d);
+    GPP_LAUNCH(sc_cost, std::max(1, std::min((n + 7) / 8, kNumSMs * 16)), kThreads, 0, s, touched.p, st.d, n, lp.AT.ptr,
+               lp.AT.idx, lp.AT.val, owner.p, stats.scol_val.p, plan.c.p);
   }
 
   // Records, in ascending row order: substitutions, then dual shifts.

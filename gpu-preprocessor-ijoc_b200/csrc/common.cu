@@ -139,16 +139,14 @@ void inject_alloc_failure(int64_t after) { g_alloc_countdown.store(after < 0 ? -
 // order, so a kernel that gets the block runs after every kernel that used it.
 // A block freed by another thread or on another stream goes back to the pool.
 // At most kCachedCap bytes are held this way across all contexts; past that a
-// freed block goes back to the pool.  GPP_ALLOC_CACHE=0 turns the reuse off.
+// freed block goes back to the pool.  The lists and the record of blocks in use
+// belong to the context, so the batched form's threads share nothing here but
+// the cap, drawn on in steps of kCreditStep.  GPP_ALLOC_CACHE=0 turns the reuse
+// off.
 namespace {
-struct HandedOut {
-  size_t bytes;
-  const Context* owner;
-};
-std::mutex g_blocks_mu;
-std::unordered_map<void*, HandedOut>* g_blocks = new std::unordered_map<void*, HandedOut>();   // never destroyed
-std::atomic<int64_t> g_cached_bytes{0};
+std::atomic<int64_t> g_cache_credit{0};
 constexpr int64_t kCachedCap = int64_t(8) << 30;
+constexpr int64_t kCreditStep = int64_t(64) << 20;
 
 bool alloc_cache_on() {
   static const bool on = [] {
@@ -162,6 +160,23 @@ size_t size_class(size_t bytes) {
   const int high = 63 - __builtin_clzll(uint64_t(bytes));
   const size_t grain = size_t(1) << std::max(8, high - 2);
   return (bytes + grain - 1) / grain * grain;
+}
+// Index of a size class: its power of two and its quarter.
+int class_index(size_t cls) {
+  const int high = 63 - __builtin_clzll(uint64_t(cls));
+  return high * 4 + int((cls >> (high - 2)) & 3);
+}
+// Whether the context may hold `bytes` more.
+bool may_cache(Context& c, int64_t bytes) {
+  const int64_t over = c.cached_bytes + bytes - c.cache_credit;
+  if (over <= 0) return true;
+  const int64_t draw = (over + kCreditStep - 1) / kCreditStep * kCreditStep;
+  if (g_cache_credit.fetch_add(draw, std::memory_order_relaxed) + draw > kCachedCap) {
+    g_cache_credit.fetch_sub(draw, std::memory_order_relaxed);
+    return false;
+  }
+  c.cache_credit += draw;
+  return true;
 }
 }  // namespace
 
@@ -179,43 +194,36 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   if (!alloc_cache_on()) return cudaMallocFromPoolAsync(p, bytes, c.pool, s);
   const size_t cls = size_class(bytes);
   if (s == c.stream) {
-    auto it = c.free_blocks.find(cls);
-    if (it != c.free_blocks.end() && !it->second.empty()) {
-      *p = it->second.back();
-      it->second.pop_back();
-      g_cached_bytes.fetch_sub(int64_t(cls), std::memory_order_relaxed);
-      std::lock_guard<std::mutex> lock(g_blocks_mu);
-      (*g_blocks)[*p] = HandedOut{cls, &c};
+    auto& list = c.free_blocks[class_index(cls)];
+    if (!list.empty()) {
+      *p = list.back();
+      list.pop_back();
+      c.cached_bytes -= int64_t(cls);
+      c.handed_out[*p] = cls;
       return cudaSuccess;
     }
   }
   const cudaError_t e = cudaMallocFromPoolAsync(p, cls, c.pool, s);
-  if (e == cudaSuccess) {
-    std::lock_guard<std::mutex> lock(g_blocks_mu);
-    (*g_blocks)[*p] = HandedOut{cls, &c};
-  }
+  if (e == cudaSuccess) c.handed_out[*p] = cls;
   return e;
 }
 
 void pool_free(void* p, cudaStream_t s) {
   if (!p) return;
   if (alloc_cache_on()) {
-    HandedOut b{0, nullptr};
-    {
-      std::lock_guard<std::mutex> lock(g_blocks_mu);
-      auto it = g_blocks->find(p);
-      if (it != g_blocks->end()) {
-        b = it->second;
-        g_blocks->erase(it);
+    // A block of another context is in that context's record only; its entry
+    // there is overwritten when its pool hands the address out again.
+    Context& c = ctx();
+    const auto it = c.handed_out.find(p);
+    if (it != c.handed_out.end()) {
+      const size_t cls = it->second;
+      c.handed_out.erase(it);
+      if (s == c.stream && may_cache(c, int64_t(cls))) {
+        c.cached_bytes += int64_t(cls);
+        c.free_blocks[class_index(cls)].push_back(p);
+        return;
       }
     }
-    Context& c = ctx();
-    if (b.owner == &c && s == c.stream &&
-        g_cached_bytes.fetch_add(int64_t(b.bytes), std::memory_order_relaxed) + int64_t(b.bytes) <= kCachedCap) {
-      c.free_blocks[b.bytes].push_back(p);
-      return;
-    }
-    if (b.owner == &c && s == c.stream) g_cached_bytes.fetch_sub(int64_t(b.bytes), std::memory_order_relaxed);
   }
   cudaFreeAsync(p, s);
 }

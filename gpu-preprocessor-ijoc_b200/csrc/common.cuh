@@ -322,8 +322,13 @@ struct Context {
   }
   cudaStream_t side = nullptr;
   // Scratch blocks this context freed on its own stream, by size class,
-  // ready to be handed out again without a driver call (pool_alloc/free).
-  std::unordered_map<size_t, std::vector<void*>> free_blocks;
+  // ready to be handed out again without a driver call (pool_alloc/free), and
+  // the classes of the blocks it handed out.  Only this context's thread
+  // touches them.
+  static constexpr int kBlockClasses = 256;
+  std::vector<void*> free_blocks[kBlockClasses];
+  std::unordered_map<void*, size_t> handed_out;
+  int64_t cached_bytes = 0, cache_credit = 0;
   static constexpr int kStatusWords = 64;
   // A second stream for host-to-device copies that overlap the engine
   // stream's kernels (created on first use; ordered by events).

@@ -93,6 +93,7 @@ struct Engine {
   bool terminal = false;
   bool active = false, pending = false;
   bool reshaped = false;   // a rule since the plan's start acted on rows or columns
+  bool unsaved = false;    // the plan's vectors are ahead of the working LP's
   Plan plan;
   Stats stats;
   bool stats_dirty = true;
@@ -123,6 +124,9 @@ struct Engine {
     plan = Plan{};
     init_plan(plan);
     plan.inf_hist = inf_hist;
+    plan.save_committed = [this] {
+      if (!pending) save_vectors();
+    };
     allocate_stats(stats, cur.m(), cur.n());
     stats_dirty = true;
     active = true;
@@ -177,6 +181,7 @@ struct Engine {
         append_fixed(out.record, plan.keep_col.p, stats.seen_col.p, plan.l.p, plan.u.p, cur.n());
       pending = true;
       if (plan.has_row_action || plan.has_col_action) stats_dirty = reshaped = true;
+      if (plan.has_col_action) plan.bounds_mirrored = false;
     } else {
       plan.tape.clear();
     }
@@ -264,25 +269,34 @@ struct Engine {
     invalidate_schedules();
   }
 
+  // The open plan's vectors to the working LP (nothing else differs).
+  void save_vectors() {
+    if (!unsaved) return;
+    const int m = cur.m(), n = cur.n();
+    GPP_LAUNCH_BYTES(copy_vectors, 48.0 * n + 32.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s(), m, n,
+                     vectors(plan), vectors(cur));
+    unsaved = false;
+  }
+
   void materialize(const char* boundary) {
     // Most propagation rounds move a few bounds and nothing else: then the
-    // vectors are committed and the plan, whose masks still keep everything,
-    // its statistics and its row queues serve the next phase as they are.  A
-    // plan without a change stays open too.
+    // plan, whose masks still keep everything, its statistics and its row
+    // queues serve the next phase as they are; the vectors reach the working
+    // LP when something reads them there.  A plan without a change stays open
+    // too.
     if (active && !reshaped && (!pending || cur.owns)) {
-      if (pending) {
-        const int m = cur.m(), n = cur.n();
-        GPP_LAUNCH_BYTES(copy_vectors, 48.0 * n + 32.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s(), m, n,
-                         vectors(plan), vectors(cur));
-        out.trace.push_back(std::string("apply=") + boundary);
-      }
+      if (pending) out.trace.push_back(std::string("apply=") + boundary);
+      unsaved = unsaved || pending;
       pending = false;
       return;
     }
     if (active && pending) {
       apply(plan, true);
       out.trace.push_back(std::string("apply=") + boundary);
+    } else if (active) {
+      save_vectors();
     }
+    unsaved = false;
     active = pending = reshaped = false;
     plan = Plan{};
     stats = Stats{};
@@ -292,6 +306,7 @@ struct Engine {
   bool materialized_rule(bool enabled, const char* name, F rule) {
     if (!enabled || terminal) return false;
     const NvtxRange range(name);
+    save_vectors();
     Plan pl;
     init_plan(pl);
     rule(pl);
@@ -577,6 +592,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
     }
   }
   e.materialize("finalize");
+  e.save_vectors();
   ctx().sync("presolve finalize");
   out.reduced_rows = cur.m();
   out.reduced_cols = cur.n();

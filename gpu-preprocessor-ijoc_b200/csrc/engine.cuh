@@ -3,6 +3,7 @@
 // explicit ownership flags; everything runs on ctx().stream.
 #pragma once
 
+#include <functional>
 #include <memory>
 #include <vector>
 
@@ -124,6 +125,23 @@ struct Plan {
   // rows with 0, 1, 2, >= 3 in the minimum activity, 4-7 the maximum.
   uint32_t* inf_hist = nullptr;
   const uint8_t* rule_entry_keep_col = nullptr;
+  // The bounds once more as the sweeps use them: packed records and the
+  // candidates' starting values.  While no rule but bound strengthening moves
+  // a bound or removes a column (bounds_mirrored), they stay current.
+  DBuf<double2> lu;
+  DBuf<double> cand_l, cand_u;
+  bool bounds_mirrored = false;
+  // Column max |a| over the kept rows, as of the statistics' version.
+  DBuf<double> col_max;
+  uint64_t col_max_version = 0;
+  // Singleton columns' row owners and status words, cleared by the Cleanup
+  // probe on its way (sc_ready) or by the rule.
+  DBuf<int32_t> sc_owner, sc_words;
+  bool sc_ready = false;
+  // Saves the vectors that are committed but still only here (the engine's
+  // open plan); a rule calls it before writes that an infeasible or unbounded
+  // end would leave half done.
+  std::function<void()> save_committed;
   bool has_new_A = false;
   DevCsr new_A;                  // owned when has_new_A
   std::vector<PostsolveSegment> tape;   // local indices until captured
@@ -193,9 +211,20 @@ void row_activity_summary(const DevCsr& A, const double* l, const double* u, dou
                           const uint8_t* keep_row, const uint8_t* keep_col, const int32_t* live_deg,
                           double* min_fin, double* max_fin, int32_t* min_inf, int32_t* max_inf,
                           cudaStream_t s);
-void row_plain_minmax(const DevCsr& A, const double* l, const double* u, const uint8_t* keep_row,
-                      const uint8_t* keep_col, const int32_t* live_deg, double* row_min, double* row_max,
-                      cudaStream_t s, uint64_t degrees_version = 0);
+// Brings plan.lu, cand_l and cand_u up to date with the plan's bounds.
+void mirror_bounds(Plan& plan, int32_t n, cudaStream_t s);
+// The redundant-row test (rule_infeasible_and_redundant_rows.cu:46-331) on the
+// plain activity sums of every row: action[i] 0 none, 1 the row goes, 2 its
+// lower side, 3 its upper side; the report's flags are 1 infeasible, 2 a row
+// goes, 4 a side goes.
+struct RedundantTest {
+  const double *AL, *AU;
+  double tol;
+  uint8_t* action;
+  Report report;
+};
+void redundant_rows_test(const DevCsr& A, const double2* lu, const uint8_t* keep_row, const int32_t* live_deg,
+                         const RedundantTest& test, cudaStream_t s, uint64_t degrees_version);
 void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStream_t s);
 
 // compact.cu
@@ -243,8 +272,10 @@ void capture_variable_pair(Record& r, VarPairRecovery&& step);
 // one readback: returns the kProbe* bits of `rules` whose rule may change the
 // plan.  A rule whose bit comes back clear would return at its first check
 // without changing anything, as long as the plan is the probed one.
+constexpr int32_t kUnclaimedRow = INT32_MAX;   // Plan::sc_owner of a row without a candidate
+constexpr int kSingletonWords = 8;             // Plan::sc_words
 constexpr uint32_t kProbeFixed = 1, kProbeEmptyColumns = 2, kProbeEmptyRows = 4, kProbeSingletonRows = 8;
-uint32_t cleanup_probe(const Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules);
+uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules);
 void rule_fixed_variables(Plan& plan, const WorkingLp& lp, const gpp_params& p);
 void rule_empty_columns(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 void rule_empty_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);

@@ -124,6 +124,31 @@ struct ActivityTerm {
 // sums.
 constexpr int kGroupRowMax = 32;
 
+// The test of one row from its plain sums (rule_infeasible_and_redundant_rows.cu:158-240).
+__device__ __forceinline__ uint32_t redundant_test(const RedundantTest& t, int row, bool tested, double lo, double hi) {
+  uint32_t found = 0;
+  uint8_t a = 0;
+  if (tested) {
+    const double al = t.AL[row], au = t.AU[row];
+    const bool lf = isfinite(al), uf = isfinite(au);
+    if (!(lf && uf && fabs(au - al) <= t.tol)) {
+      if ((lf && hi < al - t.tol) || (uf && lo > au + t.tol)) {
+        found = 1u;
+      } else {
+        const bool li = !lf || lo >= al - t.tol, ui = !uf || hi <= au + t.tol;
+        if (li && ui) { a = 1; found = 2u; }
+        else if (lf && li) { a = 2; found = 4u; }
+        else if (uf && ui) { a = 3; found = 4u; }
+      }
+    }
+  }
+  t.action[row] = a;
+  return found;
+}
+
+// With Plain the kernel forms the redundant-row rule's sums, in which
+// infinities propagate, and tests each row as soon as its sums stand; the sums
+// themselves are not stored.
 template <bool Plain>
 __global__ void __launch_bounds__(kThreads)
 activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
@@ -132,7 +157,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
                 const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
                 const int32_t* __restrict__ counts, int short_blocks, int medium_blocks,
                 double* __restrict__ min_fin, double* __restrict__ max_fin, int32_t* __restrict__ min_inf,
-                int32_t* __restrict__ max_inf) {
+                int32_t* __restrict__ max_inf, RedundantTest test) {
   __shared__ int slots[256];
   __shared__ int warp_counts[8];
   __shared__ double dagg[8];
@@ -141,6 +166,15 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
   __shared__ double group_hi[(kThreads / 32) * 4 * kGroupRowMax];
   const ActivityTerm<Plain> term{idx, val, lu, zero_tol, l2_hints()};
   const auto live_at = [&](offset_t p) { return !removed_column(term.bounds(p)); };
+  uint32_t found = 0;
+  const auto finish = [&](int row, double lo, double hi, int ni, int pi) {
+    if constexpr (Plain) {
+      found |= redundant_test(test, row, keep_row[row] && live_deg[row] > 1, lo, hi);
+    } else {
+      min_fin[row] = lo; max_fin[row] = hi;
+      if (min_inf) { min_inf[row] = ni; max_inf[row] = pi; }
+    }
+  };
   const int b = blockIdx.x;
   if (b < short_blocks) {
     // The next row's pointers and live length are loaded one iteration ahead.
@@ -181,12 +215,9 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
           if (!removed_column(bnd)) term(p, bnd, lo, hi, ni, pi);
         }
       }
-      min_fin[i] = lo; max_fin[i] = hi;
-      if (min_inf) { min_inf[i] = ni; max_inf[i] = pi; }
+      finish(i, lo, hi, ni, pi);
     }
-    return;
-  }
-  if (b < short_blocks + medium_blocks) {
+  } else if (b < short_blocks + medium_blocks) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = lane >> 3, gl = lane & 7;
     const int nwarps = medium_blocks * (kThreads / 32);
@@ -202,10 +233,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
         live_visit_by<32>(first, last, all_live, live_at, slots + warp * 32, nullptr,
                           [&](offset_t p) { term(p, term.bounds(p), lo, hi, ni, pi); });
       lo = warp_sum_down(lo); hi = warp_sum_down(hi); ni = warp_sum_down(ni); pi = warp_sum_down(pi);
-      if (lane == 0) {
-        min_fin[row] = lo; max_fin[row] = hi;
-        if (min_inf) { min_inf[row] = ni; max_inf[row] = pi; }
-      }
+      if (lane == 0) finish(row, lo, hi, ni, pi);
     };
     // The row ids and row pointers of later iterations are loaded ahead (the
     // queue entry two iterations ahead, the pointers one ahead), so each
@@ -272,10 +300,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
         ni = ni + __shfl_down_sync(0xffffffffu, ni, off, 8);
         pi = pi + __shfl_down_sync(0xffffffffu, pi, off, 8);
       }
-      if (grouped && gl == 0) {
-        min_fin[row] = lo; max_fin[row] = hi;
-        if (min_inf) { min_inf[row] = ni; max_inf[row] = pi; }
-      }
+      if (grouped && gl == 0) finish(row, lo, hi, ni, pi);
       // Longer medium rows: one warp each, as before.
       unsigned rest = __ballot_sync(0xffffffffu, have && !grouped && gl == 0);
       while (rest) {
@@ -284,30 +309,28 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
         full_row(__shfl_sync(0xffffffffu, row, src));
       }
     }
-    return;
-  }
-  const int lb = b - short_blocks - medium_blocks;
-  const int nlong = gridDim.x - short_blocks - medium_blocks;
-  const int count = counts[1];
-  for (int q = lb; q < count; q += nlong) {
-    const int row = longq[q];
-    double lo = 0.0, hi = 0.0;
-    int ni = 0, pi = 0;
-    const offset_t first = ptr[row], last = ptr[row + 1];
-    const bool all_live = live_deg && live_deg[row] == int(last - first);
-    if (!keep_row || keep_row[row])
-      live_visit_by<256>(first, last, all_live, live_at, slots, warp_counts,
-                         [&](offset_t p) { term(p, term.bounds(p), lo, hi, ni, pi); });
-    lo = block_sum_cub_order(lo, dagg);
-    hi = block_sum_cub_order(hi, dagg);
-    ni = block_sum_cub_order(ni, iagg);
-    pi = block_sum_cub_order(pi, iagg);
-    if (threadIdx.x == 0) {
-      min_fin[row] = lo; max_fin[row] = hi;
-      if (min_inf) { min_inf[row] = ni; max_inf[row] = pi; }
+  } else {
+    const int lb = b - short_blocks - medium_blocks;
+    const int nlong = gridDim.x - short_blocks - medium_blocks;
+    const int count = counts[1];
+    for (int q = lb; q < count; q += nlong) {
+      const int row = longq[q];
+      double lo = 0.0, hi = 0.0;
+      int ni = 0, pi = 0;
+      const offset_t first = ptr[row], last = ptr[row + 1];
+      const bool all_live = live_deg && live_deg[row] == int(last - first);
+      if (!keep_row || keep_row[row])
+        live_visit_by<256>(first, last, all_live, live_at, slots, warp_counts,
+                           [&](offset_t p) { term(p, term.bounds(p), lo, hi, ni, pi); });
+      lo = block_sum_cub_order(lo, dagg);
+      hi = block_sum_cub_order(hi, dagg);
+      ni = block_sum_cub_order(ni, iagg);
+      pi = block_sum_cub_order(pi, iagg);
+      if (threadIdx.x == 0) finish(row, lo, hi, ni, pi);
+      __syncthreads();
     }
-    __syncthreads();
   }
+  if constexpr (Plain) post_flags(test.report, found);
 }
 
 __global__ void pack_bounds_kernel(int n, const double* __restrict__ l, const double* __restrict__ u,
@@ -843,7 +866,7 @@ namespace {
 template <bool Plain>
 void launch_activity(const DevCsr& A, const double2* lu, double zero_tol, const uint8_t* keep_row,
                      const int32_t* live_deg, double* lo, double* hi, int32_t* ni, int32_t* pi, double out_bytes,
-                     cudaStream_t s, uint64_t degrees_version) {
+                     cudaStream_t s, uint64_t degrees_version, const RedundantTest& test = {}) {
   static thread_local RowSchedule* live_schedule = new RowSchedule;  // never destroyed (see schedule_cache)
   const RowSchedule* sch;
   if (live_deg) {
@@ -866,11 +889,11 @@ void launch_activity(const DevCsr& A, const double2* lu, double zero_tol, const 
   if constexpr (Plain)
     GPP_LAUNCH_BYTES(activity_kernel<true>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu, zero_tol,
                      keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
-                     r.medium_blocks, lo, hi, ni, pi);
+                     r.medium_blocks, lo, hi, ni, pi, test);
   else
     GPP_LAUNCH_BYTES(activity_kernel<false>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu, zero_tol,
                      keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
-                     r.medium_blocks, lo, hi, ni, pi);
+                     r.medium_blocks, lo, hi, ni, pi, test);
 }
 }  // namespace
 
@@ -893,15 +916,21 @@ void row_activity_summary(const DevCsr& A, const double* l, const double* u, dou
   row_activity_summary_packed(A, lu.p, zero_tol, keep_row, live_deg, min_fin, max_fin, min_inf, max_inf, s);
 }
 
-void row_plain_minmax(const DevCsr& A, const double* l, const double* u, const uint8_t* keep_row,
-                      const uint8_t* keep_col, const int32_t* live_deg, double* row_min, double* row_max,
-                      cudaStream_t s, uint64_t degrees_version) {
-  // Row sums of the redundant-row rule (rule_infeasible_and_redundant_rows.cu:46-156).
-  if (!A.rows) return;
-  DBuf<double2> lu(size_t(std::max(A.cols, 1)), s);
-  pack_bounds(l, u, keep_col, A.cols, lu.p, s);
-  launch_activity<true>(A, lu.p, 0.0, keep_row, live_deg, row_min, row_max, nullptr, nullptr, 16.0, s,
-                        degrees_version);
+void redundant_rows_test(const DevCsr& A, const double2* lu, const uint8_t* keep_row, const int32_t* live_deg,
+                         const RedundantTest& test, cudaStream_t s, uint64_t degrees_version) {
+  launch_activity<true>(A, lu, 0.0, keep_row, live_deg, nullptr, nullptr, nullptr, nullptr, 17.0, s, degrees_version,
+                        test);
+}
+
+void mirror_bounds(Plan& plan, int32_t n, cudaStream_t s) {
+  if (plan.bounds_mirrored) return;
+  if (plan.lu.n < size_t(n)) {
+    plan.lu.alloc(size_t(n), s);
+    plan.cand_l.alloc(size_t(n), s);
+    plan.cand_u.alloc(size_t(n), s);
+  }
+  pack_bounds(plan.l.p, plan.u.p, plan.keep_col.p, n, plan.lu.p, s, plan.cand_l.p, plan.cand_u.p);
+  plan.bounds_mirrored = true;
 }
 
 void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStream_t s) {

@@ -128,162 +128,269 @@ candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, CandArgs g)
   }
 }
 
-// _kernel_finalize_bound_strengthening (reference :646-796).
-__global__ void finalize_kernel(int n, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
-                                const double* __restrict__ u, const double* __restrict__ cand_l,
-                                const double* __restrict__ cand_u, const double* __restrict__ c,
-                                const double* __restrict__ vmax_arr, int preserve_free_zero_cost, double zero_tol,
-                                double ft, double upper_relax, double* __restrict__ fl, double* __restrict__ fu,
-                                uint8_t* __restrict__ lch, uint8_t* __restrict__ uch, uint8_t* __restrict__ fx,
-                                double* __restrict__ fixv, Report report, bool post) {
-  uint32_t found = 0;   // 1 infeasible, 2 a bound moves, 4 a column is fixed
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const double lj = l[j], uj = u[j];
-    if (!keep_col[j]) {
-      fl[j] = lj; fu[j] = uj; lch[j] = uch[j] = fx[j] = 0; fixv[j] = 0.0;
-      continue;
-    }
-    double cl = cand_l[j], cu = cand_u[j];
-    const double vmax = vmax_arr[j];
-    double nl = lj, nu = uj;
-    uint8_t lc = 0, uc = 0, fj = 0;
-    double fat = 0.0;
-    double el = lj, eu = uj;
-    if (isfinite(cl)) el = fmax(el, cl);
-    if (isfinite(cu)) eu = fmin(eu, cu);
-    if (el > eu + ft) { found |= 1u; lch[j] = uch[j] = 0; continue; }
-    const bool was_free = !isfinite(lj) && !isfinite(uj);   // the bounds at the phase's start
-    const bool box = isfinite(cl) && isfinite(cu);
-    const bool zero_cost = fabs(c[j]) <= zero_tol;
-    const bool nearly_fixed = box && (cu <= cl || (cu - cl) * vmax <= ft);
-    if (preserve_free_zero_cost && was_free && box && zero_cost && !nearly_fixed) { cl = lj; cu = uj; }
-    if (isfinite(cl) && cl > lj && isfinite(uj)) {
-      if (cl >= uj + ft) { found |= 1u; lch[j] = uch[j] = 0; continue; }
-      if (cl >= uj || (uj - cl) * vmax <= ft) { fj = 1; fat = uj; nl = uj; nu = uj; }
-    }
-    if (!fj && isfinite(cl) && cl > lj) {
-      const bool tighten = !isfinite(lj) || ((cl - lj > ft * 1.0e4) && (cl - lj > 1.0e-2 * fabs(lj)));
-      if (tighten) {
-        if (cl != nearbyint(cl)) cl -= 0.5 * ft * fabs(cl);
-        nl = cl;
-        lc = 1;
-      }
-    }
-    if (!fj && isfinite(cu) && cu < uj && isfinite(nl)) {
-      if (cu <= nl - ft) { found |= 1u; lch[j] = uch[j] = 0; continue; }
-      if (cu <= nl || (cu - nl) * vmax <= ft) { fj = 1; fat = nl; nu = nl; }
-    }
-    if (!fj && isfinite(cu) && cu < uj) {
-      const bool tighten = !isfinite(uj) || ((uj - cu > ft * 1.0e4) && (uj - cu > 1.0e-2 * fabs(uj)));
-      if (tighten) {
-        if (cu != nearbyint(cu)) cu += upper_relax * ft * fabs(cu);
-        nu = cu;
-        uc = 1;
-      }
-    }
-    if (fj) { lc = uc = 0; found |= 4u; }
-    if (lc || uc) found |= 2u;
-    fl[j] = nl; fu[j] = nu; lch[j] = lc; uch[j] = uc; fx[j] = fj; fixv[j] = fat;
+// One column's outcome.
+struct ColumnBounds {
+  double l, u, fixed_at;
+  bool l_changed, u_changed, fixed, infeasible;
+};
+
+// _kernel_finalize_bound_strengthening (reference :646-796) for a kept column
+// with bounds lj, uj and candidates cl, cu.
+__device__ __forceinline__ ColumnBounds finalize_column(double lj, double uj, double cl, double cu, double cj, double vmax,
+                                                        bool preserve_free_zero_cost, double zero_tol, double ft,
+                                                        double upper_relax) {
+  ColumnBounds r{lj, uj, 0.0, false, false, false, false};
+  double el = lj, eu = uj;
+  if (isfinite(cl)) el = fmax(el, cl);
+  if (isfinite(cu)) eu = fmin(eu, cu);
+  if (el > eu + ft) { r.infeasible = true; return r; }
+  const bool was_free = !isfinite(lj) && !isfinite(uj);   // the bounds at the phase's start
+  const bool box = isfinite(cl) && isfinite(cu);
+  const bool zero_cost = fabs(cj) <= zero_tol;
+  const bool nearly_fixed = box && (cu <= cl || (cu - cl) * vmax <= ft);
+  if (preserve_free_zero_cost && was_free && box && zero_cost && !nearly_fixed) { cl = lj; cu = uj; }
+  if (isfinite(cl) && cl > lj && isfinite(uj)) {
+    if (cl >= uj + ft) { r.infeasible = true; return r; }
+    if (cl >= uj || (uj - cl) * vmax <= ft) { r.fixed = true; r.fixed_at = uj; r.l = uj; r.u = uj; }
   }
-  if (post) post_flags(report, found);
-  else gather_flags(report, found);
+  if (!r.fixed && isfinite(cl) && cl > lj) {
+    const bool tighten = !isfinite(lj) || ((cl - lj > ft * 1.0e4) && (cl - lj > 1.0e-2 * fabs(lj)));
+    if (tighten) {
+      if (cl != nearbyint(cl)) cl -= 0.5 * ft * fabs(cl);
+      r.l = cl;
+      r.l_changed = true;
+    }
+  }
+  if (!r.fixed && isfinite(cu) && cu < uj && isfinite(r.l)) {
+    if (cu <= r.l - ft) { r.infeasible = true; return r; }
+    if (cu <= r.l || (cu - r.l) * vmax <= ft) { r.fixed = true; r.fixed_at = r.l; r.u = r.l; }
+  }
+  if (!r.fixed && isfinite(cu) && cu < uj) {
+    const bool tighten = !isfinite(uj) || ((uj - cu > ft * 1.0e4) && (uj - cu > 1.0e-2 * fabs(uj)));
+    if (tighten) {
+      if (cu != nearbyint(cu)) cu += upper_relax * ft * fabs(cu);
+      r.u = cu;
+      r.u_changed = true;
+    }
+  }
+  if (r.fixed) r.l_changed = r.u_changed = false;
+  return r;
 }
 
-// Support rows (reference :815-960); the per-column tape sizes (:970-1008)
-// follow from them in the scan.
-__global__ void support_kernel(int n, const offset_t* __restrict__ at_ptr, const int32_t* __restrict__ at_idx,
-                               const double* __restrict__ at_val, const uint8_t* __restrict__ keep_row,
-                               const int32_t* __restrict__ row_nnz, const double* __restrict__ AL,
-                               const double* __restrict__ AU, const double* __restrict__ l,
-                               const double* __restrict__ u, RowSummary rs, const uint8_t* __restrict__ lch,
-                               const uint8_t* __restrict__ uch, const double* __restrict__ fl,
-                               const double* __restrict__ fu, double zero_tol, double tol, double support_tol,
-                               int32_t* __restrict__ sup_l, int32_t* __restrict__ sup_u) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    int sl = INT_MAX, su = INT_MAX;
-    const bool nl = lch[j], nu = uch[j];
-    if (nl || nu) {
-      const double lj = l[j], uj = u[j], flj = fl[j], fuj = fu[j];
-      const bool want_l = nl && flj > lj + tol, want_u = nu && fuj < uj - tol;
-      // Four entries per round with every load issued before the first use
-      // (one memory round trip per four entries); the support row is the
-      // smallest qualifying row, which does not depend on the visiting order.
-      constexpr int kBatch = 4;
-      const offset_t end = at_ptr[j + 1];
-      for (offset_t p0 = at_ptr[j]; p0 < end && (want_l || want_u); p0 += kBatch) {
-        int row[kBatch];
-        double a[kBatch];
+struct SupportArgs {
+  const offset_t* at_ptr;
+  const int32_t* at_idx;
+  const double* at_val;
+  const uint8_t* keep_row;
+  const int32_t* row_nnz;
+  const double *AL, *AU;
+  RowSummary rs;
+  double zero_tol, tol, support_tol;
+};
+// Support rows of a changed column (reference :815-960): the smallest row that
+// implies each new bound, INT_MAX when none does.
+__device__ __forceinline__ void support_rows(const SupportArgs& g, int j, double lj, double uj, const ColumnBounds& b,
+                                             int& sl, int& su) {
+  sl = su = INT_MAX;
+  const bool want_l = b.l_changed && b.l > lj + g.tol, want_u = b.u_changed && b.u < uj - g.tol;
+  // Four entries per round with every load issued before the first use
+  // (one memory round trip per four entries); the support row is the
+  // smallest qualifying row, which does not depend on the visiting order.
+  constexpr int kBatch = 4;
+  const offset_t end = g.at_ptr[j + 1];
+  for (offset_t p0 = g.at_ptr[j]; p0 < end && (want_l || want_u); p0 += kBatch) {
+    int row[kBatch];
+    double a[kBatch];
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-          row[k] = p0 + k < end ? at_idx[p0 + k] : -1;
-          a[k] = p0 + k < end ? at_val[p0 + k] : 0.0;
-        }
-        bool live[kBatch];
-        double al[kBatch], au[kBatch], mn[kBatch], mx[kBatch];
-        int ni[kBatch], pi[kBatch];
+    for (int k = 0; k < kBatch; ++k) {
+      row[k] = p0 + k < end ? g.at_idx[p0 + k] : -1;
+      a[k] = p0 + k < end ? g.at_val[p0 + k] : 0.0;
+    }
+    bool live[kBatch];
+    double al[kBatch], au[kBatch], mn[kBatch], mx[kBatch];
+    int ni[kBatch], pi[kBatch];
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-          const int i = row[k] >= 0 ? row[k] : 0;
-          live[k] = row[k] >= 0 && (keep_row[i] != 0) & (row_nnz[i] > 1);
-          al[k] = AL[i]; au[k] = AU[i]; mn[k] = rs.mn[i]; mx[k] = rs.mx[i]; ni[k] = rs.ni[i]; pi[k] = rs.pi[i];
-        }
+    for (int k = 0; k < kBatch; ++k) {
+      const int i = row[k] >= 0 ? row[k] : 0;
+      live[k] = row[k] >= 0 && (g.keep_row[i] != 0) & (g.row_nnz[i] > 1);
+      al[k] = g.AL[i]; au[k] = g.AU[i]; mn[k] = g.rs.mn[i]; mx[k] = g.rs.mx[i]; ni[k] = g.rs.ni[i]; pi[k] = g.rs.pi[i];
+    }
 #pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-          if (!live[k] || fabs(a[k]) <= zero_tol) continue;
-          double il, iu;
-          implied_bounds(a[k], lj, uj, al[k], au[k], mn[k], mx[k], ni[k], pi[k], il, iu);
-          if (want_l && isfinite(il) && fabs(il - flj) <= support_tol) sl = min(sl, row[k]);
-          if (want_u && isfinite(iu) && fabs(iu - fuj) <= support_tol) su = min(su, row[k]);
+    for (int k = 0; k < kBatch; ++k) {
+      if (!live[k] || fabs(a[k]) <= g.zero_tol) continue;
+      double il, iu;
+      implied_bounds(a[k], lj, uj, al[k], au[k], mn[k], mx[k], ni[k], pi[k], il, iu);
+      if (want_l && isfinite(il) && fabs(il - b.l) <= g.support_tol) sl = min(sl, row[k]);
+      if (want_u && isfinite(iu) && fabs(iu - b.u) <= g.support_tol) su = min(su, row[k]);
+    }
+  }
+}
+
+// What the finalisation leaves per column.  `change` bits: 1 lower, 2 upper
+// bound moved, 4 fixed (at its new lower bound); the support rows and the
+// records' positions stand for the moved ones only.
+struct FinalBounds {
+  double *l, *u;
+  uint8_t* change;
+  int32_t *sup_l, *sup_u, *rec_pos, *idx_pos;
+};
+
+// Finalisation, support rows and the records' positions (:970-1008) in one
+// pass over the columns, 32 consecutive ones per warp and round: the records
+// of a column, at most two with at most four indices, are ranked by ballots
+// within the warp and by a look-back over the tiles.  The packed bounds and the
+// candidates are left as the next sweep needs them.  Report: word 0 flags (1
+// infeasible, 2 a bound moves, 4 a column is fixed), 1 records, 2 indices.
+__global__ void __launch_bounds__(kThreads)
+finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
+                const double* __restrict__ u, double* __restrict__ cand_l, double* __restrict__ cand_u,
+                double2* __restrict__ lu, const double* __restrict__ c, const double* __restrict__ vmax,
+                int preserve_free_zero_cost, double ft, double upper_relax, bool records, SupportArgs g, FinalBounds out,
+                unsigned long long* words, unsigned int* counters, int32_t* error, Report report) {
+  __shared__ int warp_sums[2][kThreads / 32];
+  __shared__ long long tile_before[2];
+  __shared__ unsigned int ticket;
+  if (threadIdx.x == 0) ticket = tiles > 1 ? atomicAdd(counters, 1u) : 0u;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t t = ticket;
+  const int64_t base = t * kScanTile + warp * 32 * kScanItems + lane;
+  uint32_t found = 0;
+  unsigned packed = 0;   // per round: 2 bits records, 2 bits indices beyond one per record
+  int sum0 = 0, sum1 = 0;
+#pragma unroll 1
+  for (int k = 0; k < kScanItems; ++k) {
+    const int64_t j64 = base + k * 32;
+    unsigned recs = 0, extra = 0;
+    if (j64 < n) {
+      const int j = int(j64);
+      const double lj = l[j], uj = u[j];
+      ColumnBounds b{lj, uj, 0.0, false, false, false, false};
+      const bool kept = keep_col[j];
+      if (kept)
+        b = finalize_column(lj, uj, cand_l[j], cand_u[j], c[j], vmax[j], preserve_free_zero_cost != 0, g.zero_tol, ft,
+                            upper_relax);
+      if (b.infeasible) {
+        found |= 1u;
+        b = ColumnBounds{lj, uj, 0.0, false, false, false, false};
+      }
+      if (b.fixed) found |= 4u;
+      if (b.l_changed || b.u_changed) {
+        found |= 2u;
+        if (records) {
+          int sl, su;
+          support_rows(g, j, lj, uj, b, sl, su);
+          recs = unsigned(b.l_changed) + unsigned(b.u_changed);
+          extra = unsigned(b.l_changed && sl != INT_MAX) + unsigned(b.u_changed && su != INT_MAX);
+          out.sup_l[j] = sl;
+          out.sup_u[j] = su;
         }
       }
+      out.l[j] = b.l;
+      out.u[j] = b.u;
+      out.change[j] = uint8_t((b.l_changed ? 1 : 0) | (b.u_changed ? 2 : 0) | (b.fixed ? 4 : 0));
+      cand_l[j] = b.l;
+      cand_u[j] = b.u;
+      if (kept && !b.fixed) lu[j] = make_double2(b.l, b.u);
+      else {
+        const double removed = __longlong_as_double(static_cast<long long>(kRemovedColumnBits));
+        lu[j] = make_double2(removed, removed);
+      }
     }
-    sup_l[j] = sl;
-    sup_u[j] = su;
+    packed |= (recs | extra << 2) << (4 * k);
+    const int r = __popc(__ballot_sync(0xffffffffu, recs & 1)) + 2 * __popc(__ballot_sync(0xffffffffu, recs >> 1));
+    sum0 += r;
+    sum1 += r + __popc(__ballot_sync(0xffffffffu, extra & 1)) + 2 * __popc(__ballot_sync(0xffffffffu, extra >> 1));
   }
+  if (lane == 0) {
+    warp_sums[0][warp] = sum0;
+    warp_sums[1][warp] = sum1;
+  }
+  __syncthreads();
+  if (warp < 2) {
+    int all = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) all += warp_sums[warp][w];
+    const long long before = publish_and_look_back(words + int64_t(warp) * tiles, t, tiles, all, error);
+    if (lane == 0) {
+      tile_before[warp] = before;
+      if (t == tiles - 1) report.words[1 + warp] = int32_t(before + all);
+    }
+  }
+  __syncthreads();
+  if (records) {
+    int at0 = int(tile_before[0]), at1 = int(tile_before[1]);
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+      at0 += w < warp ? warp_sums[0][w] : 0;
+      at1 += w < warp ? warp_sums[1][w] : 0;
+    }
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
+    for (int k = 0; k < kScanItems; ++k) {
+      const unsigned recs = packed >> (4 * k) & 3u, extra = packed >> (4 * k + 2) & 3u;
+      const unsigned r0 = __ballot_sync(0xffffffffu, recs & 1), r1 = __ballot_sync(0xffffffffu, recs >> 1);
+      const unsigned e0 = __ballot_sync(0xffffffffu, extra & 1), e1 = __ballot_sync(0xffffffffu, extra >> 1);
+      if (recs) {
+        const int64_t j = base + k * 32;
+        const int rb = __popc(r0 & below) + 2 * __popc(r1 & below);
+        out.rec_pos[j] = at0 + rb;
+        out.idx_pos[j] = at1 + rb + __popc(e0 & below) + 2 * __popc(e1 & below);
+      }
+      const int r = __popc(r0) + 2 * __popc(r1);
+      at0 += r;
+      at1 += r + __popc(e0) + 2 * __popc(e1);
+    }
+  }
+  if (tiles > 1) leave_zeroed(words, int64_t(tiles) * 2, counters);
+  gather_flags(report, found);
+  post_report(report);
 }
 
 constexpr int kVariableBoundChange = 11, kRowImpliedBoundChange = 12, kFixedVariable = 0;
 
 // The bound records of a column (`records` set), then its new bounds and mask.
 struct BoundRecords {
-  const int32_t *sup_l, *sup_u, *rec_pos, *idx_pos;
   int32_t* types;
   int64_t *is, *vs;
   int32_t* idx;
   double* val;
 };
-__global__ void commit_bounds(int n, const uint8_t* __restrict__ lch, const uint8_t* __restrict__ uch,
-                              const double* __restrict__ fl, const double* __restrict__ fu,
-                              const uint8_t* __restrict__ fx, bool records, BoundRecords rec, double* __restrict__ l,
-                              double* __restrict__ u, uint8_t* __restrict__ keep_col) {
+__global__ void commit_bounds(int n, FinalBounds f, bool records, BoundRecords rec, double* __restrict__ l,
+                              double* __restrict__ u, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ fixed,
+                              double* __restrict__ fixed_at) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const double nl = fl[j], nu = fu[j];
-    if (records) {
-      if (j == 0) { rec.is[0] = 0; rec.vs[0] = 0; }
-      const bool lc = lch[j], uc = uch[j];
-      if (lc || uc) {
-        int64_t k = rec.rec_pos[j], ip = rec.idx_pos[j];
-        double cur_l = l[j];
-        const double cur_u = u[j];
-        auto emit = [&](int sup, double a, double b, double c2, double d) {
-          rec.types[k] = sup == INT_MAX ? kVariableBoundChange : kRowImpliedBoundChange;
-          rec.idx[ip++] = j;
-          if (sup != INT_MAX) rec.idx[ip++] = sup;
-          rec.val[4 * k] = a; rec.val[4 * k + 1] = b; rec.val[4 * k + 2] = c2; rec.val[4 * k + 3] = d;
-          rec.is[k + 1] = ip;
-          rec.vs[k + 1] = 4 * (k + 1);
-          ++k;
-        };
-        if (lc) {
-          emit(rec.sup_l[j], cur_l, cur_u, nl, cur_u);
-          cur_l = nl;
-        }
-        if (uc) emit(rec.sup_u[j], cur_l, cur_u, cur_l, nu);
+    if (records && j == 0) { rec.is[0] = 0; rec.vs[0] = 0; }
+    const uint8_t change = f.change[j];
+    if (fixed) {
+      fixed[j] = (change & 4) != 0;
+      fixed_at[j] = (change & 4) ? f.l[j] : 0.0;
+    }
+    if (!change) continue;
+    const double nl = f.l[j], nu = f.u[j];
+    const bool lc = change & 1, uc = change & 2;
+    if (records && (lc || uc)) {
+      int64_t k = f.rec_pos[j], ip = f.idx_pos[j];
+      double cur_l = l[j];
+      const double cur_u = u[j];
+      auto emit = [&](int sup, double a, double b, double c2, double d) {
+        rec.types[k] = sup == INT_MAX ? kVariableBoundChange : kRowImpliedBoundChange;
+        rec.idx[ip++] = j;
+        if (sup != INT_MAX) rec.idx[ip++] = sup;
+        rec.val[4 * k] = a; rec.val[4 * k + 1] = b; rec.val[4 * k + 2] = c2; rec.val[4 * k + 3] = d;
+        rec.is[k + 1] = ip;
+        rec.vs[k + 1] = 4 * (k + 1);
+        ++k;
+      };
+      if (lc) {
+        emit(f.sup_l[j], cur_l, cur_u, nl, cur_u);
+        cur_l = nl;
       }
+      if (uc) emit(f.sup_u[j], cur_l, cur_u, cur_l, nu);
     }
     l[j] = nl;
     u[j] = nu;
-    if (fx[j]) keep_col[j] = 0;
+    if (change & 4) keep_col[j] = 0;
   }
 }
 
@@ -367,12 +474,12 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   const int m = lp.m(), n = lp.n();
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
-  DBuf<double> cl(size_t(n), s), cu(size_t(n), s), mn(size_t(m), s), mx(size_t(m), s), vmax(size_t(n), s);
+  DBuf<double> mn(size_t(m), s), mx(size_t(m), s);
   DBuf<int32_t> ni(size_t(m), s), pi(size_t(m), s);
-  // One packed bounds array serves the activity sweep and the candidate sweep.
-  DBuf<double2> lu(size_t(n), s);
-  pack_bounds(plan.l.p, plan.u.p, plan.keep_col.p, n, lu.p, s, cl.p, cu.p);
-  row_activity_summary_packed(lp.A, lu.p, p.zero_tol, plan.keep_row.p, stats.row_nnz.p, mn.p, mx.p, ni.p, pi.p, s,
+  // One packed bounds array serves the activity sweep, the candidate sweep
+  // and the redundant-row test after them.
+  mirror_bounds(plan, n, s);
+  row_activity_summary_packed(lp.A, plan.lu.p, p.zero_tol, plan.keep_row.p, stats.row_nnz.p, mn.p, mx.p, ni.p, pi.p, s,
                               stats.version);
   const RowSummary rs{mn.p, mx.p, ni.p, pi.p};
   if (plan.inf_hist) {
@@ -380,57 +487,38 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     GPP_LAUNCH(inf_histogram, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, ni.p, pi.p, plan.inf_hist);
   }
   {
-    CandArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, lu.p, rs,
-               p.zero_tol, cl.p, cu.p};
+    CandArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, plan.lu.p, rs,
+               p.zero_tol, plan.cand_l.p, plan.cand_u.p};
     const double bytes = 4.0 * (m + 1) + 12.0 * lp.A.nnz + double(m) + 4.0 * m + 16.0 * m + 24.0 * m + 16.0 * n +
                          16.0 * n;
     const RowSchedule& sch = stored_schedule(lp.A);
     GPP_LAUNCH_BYTES(candidates_entries, bytes, int(std::max<int64_t>(1, std::min<int64_t>(sch.tiles, kNumSMs * 8))),
                      kThreads, 0, s, lp.A.nnz, sch.tile_rows.p, g);
   }
-  col_max_abs(lp.AT, plan.keep_row.p, vmax.p, s);
-  DBuf<double> fl(size_t(n), s), fu(size_t(n), s), fixv(size_t(n), s);
-  DBuf<uint8_t> lch(size_t(n), s), uch(size_t(n), s), fx(size_t(n), s);
-  // Finalisation, support rows and the records' positions run in a row, with
-  // one answer: what was found and the tape sizes.
-  const bool records = p.record_postsolve_tape != 0;
-  Report report = ctx().open_report(1);
-  GPP_LAUNCH(finalize_kernel, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.l.p, plan.u.p, cl.p,
-             cu.p, plan.c.p, vmax.p, int(p.bound_strengthening_preserve_free_zero_cost), p.zero_tol,
-             p.feasibility_tol, p.bound_strengthening_upper_relaxation_factor, fl.p, fu.p, lch.p, uch.p, fx.p,
-             fixv.p, report, !records);
-  DBuf<int32_t> sl, su, rpos, ipos;
-  if (records) {
-    sl.alloc(size_t(n), s);
-    su.alloc(size_t(n), s);
-    rpos.alloc(size_t(n), s);
-    ipos.alloc(size_t(n), s);
-    const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
-    GPP_LAUNCH(support_kernel, grid_stride_blocks(n), kThreads, 0, s, n, lp.AT.ptr, lp.AT.idx, lp.AT.val,
-               plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, plan.l.p, plan.u.p, rs, lch.p, uch.p, fl.p,
-               fu.p, p.zero_tol, p.bound_tol, support_tol, sl.p, su.p);
-    scan_items<int32_t, 2>(
-        n,
-        [lch = lch.p, uch = uch.p, sl = sl.p, su = su.p] __device__(int64_t j, int32_t(&v)[2]) {
-          const bool nl = lch[j], nu = uch[j];
-          v[0] = int(nl) + int(nu);
-          if (v[0]) v[1] = (nl ? (sl[j] == INT_MAX ? 1 : 2) : 0) + (nu ? (su[j] == INT_MAX ? 1 : 2) : 0);
-        },
-        [rpos = rpos.p, ipos = ipos.p] __device__(int64_t j, const int32_t(&before)[2], const int32_t(&v)[2]) {
-          if (!v[0]) return;
-          rpos[j] = before[0];
-          ipos[j] = before[1];
-        },
-        [report] __device__(const int32_t(&sum)[2]) {
-          report.mail->words[1] = sum[0];
-          report.mail->words[2] = sum[1];
-          report.mail->words[0] = __ldcg(report.words);
-          report.words[0] = 0;
-          __threadfence_system();
-          report.mail->seq = report.seq;
-        },
-        s);
+  // Column maxima depend on the kept rows alone: rounds that only move bounds
+  // share one sweep.
+  if (stats.version == 0 || plan.col_max_version != stats.version) {
+    if (plan.col_max.n < size_t(n)) plan.col_max.alloc(size_t(n), s);
+    col_max_abs(lp.AT, plan.keep_row.p, plan.col_max.p, s);
+    plan.col_max_version = stats.version;
   }
+  const bool records = p.record_postsolve_tape != 0;
+  DBuf<double> fl(size_t(n), s), fu(size_t(n), s);
+  DBuf<uint8_t> change(size_t(n), s);
+  DBuf<int32_t> sl, su, rpos, ipos;
+  if (records)
+    for (DBuf<int32_t>* b : {&sl, &su, &rpos, &ipos}) b->alloc(size_t(n), s);
+  const FinalBounds fin{fl.p, fu.p, change.p, sl.p, su.p, rpos.p, ipos.p};
+  const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
+  const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p, stats.row_nnz.p, plan.AL.p,
+                            plan.AU.p, rs,        p.zero_tol, p.bound_tol,    support_tol};
+  const int tiles = int((int64_t(n) + kScanTile - 1) / kScanTile);
+  LookbackSpace w(size_t(tiles) * 2, s);
+  Report report = ctx().open_report(3);
+  GPP_LAUNCH(finalize_kernel, tiles, kThreads, 0, s, n, tiles, plan.keep_col.p, plan.l.p, plan.u.p, plan.cand_l.p,
+             plan.cand_u.p, plan.lu.p, plan.c.p, plan.col_max.p, int(p.bound_strengthening_preserve_free_zero_cost),
+             p.feasibility_tol, p.bound_strengthening_upper_relaxation_factor, records, support, fin, w.words, w.counters,
+             ctx().host_error, report);
   const volatile int64_t* answer = ctx().await(report);
   const uint32_t found = uint32_t(answer[0]);
   if (found & 1u) { plan.has_infeasible = true; return; }
@@ -438,13 +526,20 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   if (!changed && !fixed) return;
   BoundRecords rec{};
   PostsolveSegment seg;
-  const int64_t recs = records ? answer[1] : 0, nidx = records ? answer[2] : 0;
+  const int64_t recs = answer[1], nidx = answer[2];
   if (recs) {
     seg = make_segment(recs, nidx, 4 * recs);
-    rec = BoundRecords{sl.p, su.p, rpos.p, ipos.p, seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p};
+    rec = BoundRecords{seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p};
   }
-  GPP_LAUNCH(commit_bounds, grid_stride_blocks(n), kThreads, 0, s, n, lch.p, uch.p, fl.p, fu.p, fx.p, recs > 0, rec,
-             plan.l.p, plan.u.p, plan.keep_col.p);
+  DBuf<uint8_t> fx;
+  DBuf<double> fixv;
+  if (fixed) {
+    if (plan.save_committed) plan.save_committed();
+    fx.alloc(size_t(n), s);
+    fixv.alloc(size_t(n), s);
+  }
+  GPP_LAUNCH(commit_bounds, grid_stride_blocks(n), kThreads, 0, s, n, fin, recs > 0, rec, plan.l.p, plan.u.p,
+             plan.keep_col.p, fx.p, fixv.p);
   if (recs) plan.tape.push_back(std::move(seg));
   double obj_delta = 0.0;
   if (fixed) {

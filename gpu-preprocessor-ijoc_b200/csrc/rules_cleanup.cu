@@ -250,8 +250,11 @@ cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ k
                      const uint8_t* __restrict__ keep_col, const double* __restrict__ l, const double* __restrict__ u,
                      const uint8_t* __restrict__ empty_col, const int32_t* __restrict__ row_nnz,
                      const uint8_t* __restrict__ singleton_row, const int32_t* __restrict__ scol,
-                     const double* __restrict__ sval, double bound_tol, double zero_tol, Report report) {
+                     const double* __restrict__ sval, double bound_tol, double zero_tol, int32_t* __restrict__ sc_owner,
+                     int32_t* __restrict__ sc_words, Report report) {
   uint32_t f = 0;
+  // The singleton-column rule's scratch, which it needs cleared.
+  if (blockIdx.x == 0 && threadIdx.x < kSingletonWords) sc_words[threadIdx.x] = 0;
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
     if (k < n) {
@@ -262,6 +265,7 @@ cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ k
       }
       if (lj > uj + bound_tol || lj != lj || uj != uj) f |= kProbeSingletonRows;
     }
+    if (k < m) sc_owner[k] = kUnclaimedRow;
     if (k < m && keep_row[k]) {
       if (row_nnz[k] == 0) f |= kProbeEmptyRows;
       if (singleton_row[k]) {
@@ -274,7 +278,7 @@ cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ k
 }
 }  // namespace
 
-uint32_t cleanup_probe(const Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules) {
+uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules) {
   // The first-stage detections of the four rules below, on the current plan,
   // with one launch and one readback; a rule whose detection finds nothing
   // (no candidate, no infeasibility) returns without touching the plan.
@@ -284,10 +288,14 @@ uint32_t cleanup_probe(const Plan& plan, const WorkingLp& lp, const Stats& stats
   if (m == 0) rules &= ~(kProbeEmptyRows | kProbeSingletonRows);
   if (!rules) return 0;
   auto s = ctx().stream;
+  if (plan.sc_owner.n < size_t(m)) plan.sc_owner.alloc(size_t(m), s);
+  if (!plan.sc_words.p) plan.sc_words.alloc(kSingletonWords, s);
+  plan.sc_ready = true;
   const Report report = ctx().open_report(1);
-  GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 6.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n,
+  GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 10.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n,
                    rules, plan.keep_row.p, plan.keep_col.p, plan.l.p, plan.u.p, stats.empty_col.p, stats.row_nnz.p,
-                   stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol, report);
+                   stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol, plan.sc_owner.p,
+                   plan.sc_words.p, report);
   return uint32_t(ctx().await(report)[0]);
 }
 
@@ -373,6 +381,7 @@ void rule_singleton_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, co
   GPP_LAUNCH(singleton_rows_commit, grid_stride_blocks(m), kThreads, 0, s, m, n, remove.p, plan.keep_row.p);
   std::swap(plan.l, cl);
   std::swap(plan.u, cu);
+  plan.bounds_mirrored = false;
   plan.has_row_action = plan.has_change = true;
   plan.has_row_deletion = plan.has_row_deletion || removed;
 }

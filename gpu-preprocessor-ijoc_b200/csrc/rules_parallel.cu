@@ -783,6 +783,7 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
   DBuf<int32_t> merge_to(size_t(m), s), step(size_t(m), s);
   DBuf<double> rec(size_t(5) * size_t(m), s);
   del.zero();
+  if (plan.save_committed) plan.save_committed();
   const Report report = ctx().open_report(1);
   GPP_LAUNCH(row_groups_kernel, grid_stride_blocks(count), kThreads, 0, s, count, keys.p, ids.p, plan.keep_row.p,
              plan.keep_col.p, plan.AL.p, plan.AU.p, lp.A.ptr, lp.A.idx, lp.A.val, p.zero_tol, p.feasibility_tol,
@@ -842,6 +843,7 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
   DBuf<int32_t> merge_to(size_t(n), s);
   del.zero();
   fixed.zero();
+  if (plan.save_committed) plan.save_committed();
   const Report report = ctx().open_report(1);
   const ColumnGroups groups{ids.p,       plan.keep_col.p, plan.keep_row.p, plan.c.p, plan.l.p, plan.u.p, lp.AT.ptr,
                             lp.AT.idx,   lp.AT.val,       p.zero_tol,      coeff_tol, obj_tol,  del.p,    fixed.p,

@@ -10,32 +10,6 @@ namespace gpp {
 
 namespace {
 
-__global__ void redundant_classify(int m, const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
-                                   const double* __restrict__ AL, const double* __restrict__ AU,
-                                   const double* __restrict__ mn, const double* __restrict__ mx, double tol,
-                                   uint8_t* __restrict__ action, Report report) {
-  uint32_t found = 0;   // 1 infeasible, 2 a row goes, 4 a side goes
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    uint8_t a = 0;
-    if (keep_row[i] && row_nnz[i] > 1) {
-      const double al = AL[i], au = AU[i];
-      const bool lf = isfinite(al), uf = isfinite(au);
-      if (!(lf && uf && fabs(au - al) <= tol)) {
-        const double lo = mn[i], hi = mx[i];
-        if ((lf && hi < al - tol) || (uf && lo > au + tol)) {
-          found |= 1u;
-        } else {
-          const bool li = !lf || lo >= al - tol, ui = !uf || hi <= au + tol;
-          if (li && ui) { a = 1; found |= 2u; }
-          else if (lf && li) { a = 2; found |= 4u; }
-          else if (uf && ui) { a = 3; found |= 4u; }
-        }
-      }
-    }
-    action[i] = a;
-  }
-  post_flags(report, found);
-}
 __global__ void redundant_apply(int m, const uint8_t* __restrict__ action, uint8_t* __restrict__ keep_row,
                                 double* __restrict__ AL, double* __restrict__ AU) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
@@ -192,13 +166,11 @@ void rule_redundant_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, co
   const int m = lp.m();
   if (m == 0) return;
   auto s = ctx().stream;
-  DBuf<double> mn(size_t(m), s), mx(size_t(m), s);
   DBuf<uint8_t> action(size_t(m), s);
-  row_plain_minmax(lp.A, plan.l.p, plan.u.p, plan.keep_row.p, plan.keep_col.p, stats.row_nnz.p, mn.p, mx.p, s,
-                   stats.version);
+  mirror_bounds(plan, lp.n(), s);
   const Report report = ctx().open_report(1);
-  GPP_LAUNCH(redundant_classify, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, stats.row_nnz.p,
-             plan.AL.p, plan.AU.p, mn.p, mx.p, p.bound_tol, action.p, report);
+  redundant_rows_test(lp.A, plan.lu.p, plan.keep_row.p, stats.row_nnz.p,
+                      RedundantTest{plan.AL.p, plan.AU.p, p.bound_tol, action.p, report}, s, stats.version);
   const uint32_t found = uint32_t(ctx().await(report)[0]);
   if (found & 1u) { plan.has_infeasible = true; return; }
   if (!found) return;

@@ -36,12 +36,12 @@ enum : uint8_t {
 // Row kinds after staging (only rows in the winner list carry one).
 enum : uint8_t { kRowElimKept = 1, kRowElimDeleted = 2, kRowDualShift = 3 };
 
-constexpr int kUnclaimed = INT_MAX;
+constexpr int kUnclaimed = kUnclaimedRow;
 constexpr int kClaimed = INT_MAX - 1;   // row holds a candidate, no owner yet
 
 // Status words.
 enum { kStUnbounded = 0, kStCand = 1, kStRows = 2, kStLong = 3, kStWin = 4, kStElim = 5, kStSide = 6,
-       kStTouched = 7, kStWords = 8 };
+       kStTouched = 7, kStWords = kSingletonWords };
 
 __device__ __forceinline__ bool direct_unbounded(double cj, double a, double lhs, double rhs, double lb, double ub,
                                                  double zt) {
@@ -639,13 +639,19 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   const int m = lp.m(), n = lp.n();
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
-  Status st;
-  DBuf<int32_t> owner(size_t(m), s), cand(size_t(n), s), rows(size_t(m), s), long_rows(size_t(m), s);
-  GPP_LAUNCH(sc_start, grid_stride_blocks(m), kThreads, 0, s, owner.p, m, kUnclaimed, st.d);
+  DBuf<int32_t> cand(size_t(n), s), rows(size_t(m), s), long_rows(size_t(m), s);
+  if (!plan.sc_ready) {
+    if (plan.sc_owner.n < size_t(m)) plan.sc_owner.alloc(size_t(m), s);
+    if (!plan.sc_words.p) plan.sc_words.alloc(kSingletonWords, s);
+    GPP_LAUNCH(sc_start, grid_stride_blocks(m), kThreads, 0, s, plan.sc_owner.p, m, kUnclaimed, plan.sc_words.p);
+  }
+  plan.sc_ready = false;
+  DBuf<int32_t>& owner = plan.sc_owner;
+  int32_t* const st = plan.sc_words.p;
   GPP_LAUNCH_BYTES(sc_candidates, double(n) * 11 + 16.0 * n, grid_stride_blocks(n), kThreads, 0, s, n, m,
                    plan.keep_col.p, plan.keep_row.p, stats.singleton_col.p, stats.scol_row.p, stats.scol_val.p,
                    stats.row_nnz.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.zero_tol, owner.p, cand.p,
-                   rows.p, long_rows.p, st.d);
+                   rows.p, long_rows.p, st);
 
   // Activity cache of the claimed rows, proposals and their staging follow with
   // no wait between: the kernels read the candidate and row counts on the
@@ -657,17 +663,17 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   const CacheOut cache{fmin.p, fmax.p, counts.p, invalid.p};
   const int row_blocks = std::max(1, std::min((claims + 31) / 32, kNumSMs * 16));
   const int long_blocks = std::max(1, std::min(kNumSMs * 4, int(lp.A.nnz / kLongRow)));
-  GPP_LAUNCH(sc_cache, row_blocks + long_blocks, kThreads, 0, s, row_blocks, rows.p, long_rows.p, st.d,
+  GPP_LAUNCH(sc_cache, row_blocks + long_blocks, kThreads, 0, s, row_blocks, rows.p, long_rows.p, st,
              stats.row_nnz.p, lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
   DBuf<uint8_t> action(size_t(n), s), kind(size_t(m), s);
   DBuf<double> side(size_t(n), s), contrib_val(size_t(claims), s);
   DBuf<int64_t> contrib_idx(size_t(claims), s);
   DBuf<int32_t> winners(size_t(claims), s);
-  GPP_LAUNCH(sc_propose, grid_stride_blocks(n), kThreads, 0, s, cand.p, st.d, stats.scol_row.p, stats.scol_val.p,
+  GPP_LAUNCH(sc_propose, grid_stride_blocks(n), kThreads, 0, s, cand.p, st, stats.scol_row.p, stats.scol_val.p,
              plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, fmin.p, fmax.p, counts.p, invalid.p, p.bound_tol,
              p.zero_tol, action.p, side.p, owner.p);
-  const Report report = ctx().open_report(kStWords, st.d);
-  GPP_LAUNCH(sc_stage, grid_stride_blocks(claims), kThreads, 0, s, rows.p, st.d, n, action.p, side.p,
+  const Report report = ctx().open_report(kStWords, st);
+  GPP_LAUNCH(sc_stage, grid_stride_blocks(claims), kThreads, 0, s, rows.p, st, n, action.p, side.p,
              stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.bound_tol, owner.p,
              plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p, report);
   const volatile int64_t* f = ctx().await(report);
@@ -681,9 +687,9 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
     DBuf<uint32_t> claimed(size_t(n + 31) / 32, s);
     claimed.zero();
     DBuf<int32_t> touched(size_t(n), s);
-    GPP_LAUNCH(sc_touch, std::max(1, std::min((nwin + 7) / 8, kNumSMs * 16)), kThreads, 0, s, winners.p, st.d,
-               kind.p, lp.A.ptr, lp.A.idx, plan.keep_col.p, claimed.p, touched.p, st.d);
-    GPP_LAUNCH(sc_cost, std::max(1, std::min((n + 7) / 8, kNumSMs * 16)), kThreads, 0, s, touched.p, st.d, n, lp.AT.ptr,
+    GPP_LAUNCH(sc_touch, std::max(1, std::min((nwin + 7) / 8, kNumSMs * 16)), kThreads, 0, s, winners.p, st,
+               kind.p, lp.A.ptr, lp.A.idx, plan.keep_col.p, claimed.p, touched.p, st);
+    GPP_LAUNCH(sc_cost, std::max(1, std::min((n + 7) / 8, kNumSMs * 16)), kThreads, 0, s, touched.p, st, n, lp.AT.ptr,
                lp.AT.idx, lp.AT.val, owner.p, stats.scol_val.p, plan.c.p);
   }
 

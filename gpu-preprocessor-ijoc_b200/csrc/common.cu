@@ -272,6 +272,7 @@ namespace {
 __global__ void __launch_bounds__(kThreads)
 det_sum_kernel(const double* __restrict__ v, const uint8_t* __restrict__ mask, int64_t n, double* chunk_totals,
                unsigned int* done, Mailbox* mail, uint32_t seq) {
+  after_previous_kernel();
   __shared__ double sm[kThreads];
   __shared__ bool last;
   const int64_t base = int64_t(blockIdx.x) * 2048;

@@ -63,6 +63,31 @@ cudaEvent_t profile_event();
 int64_t profile_last();
 void profile_add_bytes(int64_t record, double bytes);
 
+// Kernels of a stream follow one another with programmatic dependent launch:
+// a kernel's blocks are placed while its predecessor still runs and wait at
+// their first statement, after_previous_kernel(), until the predecessor has
+// completed and its writes are visible.  Every kernel launched here must begin
+// with it; it also lets the kernel's own successor be placed.
+__device__ __forceinline__ void after_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_after_previous(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t s,
+                                         Args&&... args) {
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(unsigned(grid));
+  config.blockDim = dim3(unsigned(block));
+  config.dynamicSmemBytes = smem;
+  config.stream = s;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+
 #define GPP_LAUNCH_BYTES(kernel, bytes, grid, block, smem, stream, ...)             \
   do {                                                                              \
     if ((grid) > 0) {                                                               \
@@ -72,8 +97,7 @@ void profile_add_bytes(int64_t record, double bytes);
         gpp_ev1 = ::gpp::profile_event();                                           \
         cudaEventRecord(gpp_ev0, (stream));                                         \
       }                                                                             \
-      kernel<<<(grid), (block), (smem), (stream)>>>(__VA_ARGS__);                   \
-      ::gpp::check(cudaGetLastError(), #kernel);                                    \
+      ::gpp::check(::gpp::launch_after_previous(kernel, (grid), (block), (smem), (stream), __VA_ARGS__), #kernel); \
       ++::gpp::launch_counter();                                                    \
       if (gpp_ev1) {                                                                \
         cudaEventRecord(gpp_ev1, (stream));                                         \

@@ -73,6 +73,7 @@ struct CompactSides {
 };
 
 __global__ void compact_mark_rows(CompactSides sides) {
+  after_previous_kernel();
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const CompactSide& s = sides.side[k];
@@ -92,6 +93,7 @@ __global__ void compact_mark_rows(CompactSides sides) {
 // New pointers of the kept rows (an empty row's is the kept entries before its
 // position too), and the row bits cleared for the next compaction.
 __global__ void compact_row_pointers(CompactSides sides) {
+  after_previous_kernel();
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const CompactSide& s = sides.side[k];
@@ -118,6 +120,7 @@ __global__ void compact_row_pointers(CompactSides sides) {
 // again after it; the kept counts of both sides are posted to the host.
 __global__ void __launch_bounds__(kThreads)
 compact_tiles(CompactSides sides, unsigned long long* words, unsigned int* counters, int32_t* error, Report report) {
+  after_previous_kernel();
   __shared__ int warp_counts[kCompactWarps];
   __shared__ long long tile_before;
   __shared__ unsigned int ticket;
@@ -195,11 +198,13 @@ compact_tiles(CompactSides sides, unsigned long long* words, unsigned int* count
 }
 
 __global__ void histogram(const int32_t* __restrict__ idx, offset_t nnz, int32_t* __restrict__ counts) {
+  after_previous_kernel();
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < nnz; p += int64_t(gridDim.x) * blockDim.x)
     atomicAdd(counts + idx[p], 1);
 }
 // Longest column (the histogram's largest count), one atomic per warp.
 __global__ void longest_count(const int32_t* __restrict__ counts, int n, int32_t* __restrict__ out) {
+  after_previous_kernel();
   int32_t best = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) best = max(best, counts[j]);
   best = __reduce_max_sync(0xffffffffu, best);
@@ -212,10 +217,12 @@ __global__ void longest_count(const int32_t* __restrict__ counts, int n, int32_t
 constexpr int kShortColumn = 64;
 __global__ void place_positions(offset_t nnz, const int32_t* __restrict__ idx, int32_t* __restrict__ cursor,
                                 int32_t* __restrict__ pos) {
+  after_previous_kernel();
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < nnz; p += int64_t(gridDim.x) * blockDim.x)
     pos[atomicAdd(cursor + idx[p], 1)] = int32_t(p);
 }
 __global__ void order_columns(int n, const offset_t* __restrict__ ptr, int32_t* __restrict__ pos) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const offset_t first = ptr[j];
     const int len = int(ptr[j + 1] - first);
@@ -234,6 +241,7 @@ __global__ void order_columns(int n, const offset_t* __restrict__ ptr, int32_t* 
 // Column keys and entry positions of M, in stored (row-major) order.
 __global__ void transpose_keys(offset_t nnz, const int32_t* __restrict__ idx, uint64_t* __restrict__ keys,
                                int32_t* __restrict__ pos) {
+  after_previous_kernel();
   for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < nnz; p += int64_t(gridDim.x) * blockDim.x) {
     keys[p] = uint64_t(uint32_t(idx[p]));
     pos[p] = int32_t(p);
@@ -241,6 +249,7 @@ __global__ void transpose_keys(offset_t nnz, const int32_t* __restrict__ idx, ui
 }
 // Row of every stored entry: one warp per row writes its run.
 __global__ void row_of_entry(int rows, const offset_t* __restrict__ ptr, int32_t* __restrict__ row) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps)
@@ -250,6 +259,7 @@ __global__ void row_of_entry(int rows, const offset_t* __restrict__ ptr, int32_t
 __global__ void transpose_gather(offset_t nnz, const int32_t* __restrict__ pos, const int32_t* __restrict__ row,
                                  const double* __restrict__ val, int32_t* __restrict__ out_idx,
                                  double* __restrict__ out_val) {
+  after_previous_kernel();
   for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nnz; q += int64_t(gridDim.x) * blockDim.x) {
     const int32_t p = pos[q];
     out_idx[q] = row[p];
@@ -261,6 +271,7 @@ __global__ void transpose_gather(offset_t nnz, const int32_t* __restrict__ pos, 
 // (p - 1, p) of its stride.
 __global__ void check_sorted(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                              int32_t* bad) {
+  after_previous_kernel();
   const int g = threadIdx.x & 7;
   const int groups = gridDim.x * (blockDim.x >> 3);
   for (int r = blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3); r < rows; r += groups)
@@ -272,6 +283,7 @@ __global__ void check_sorted(int rows, const offset_t* __restrict__ ptr, const i
 // decrease; every inner index lies in [0, cols).  Any violation sets *bad.
 __global__ void check_csr_structure(int rows, int cols, offset_t nnz, const offset_t* __restrict__ ptr,
                                     const int32_t* __restrict__ idx, int32_t* bad) {
+  after_previous_kernel();
   const int64_t top = int64_t(rows) + 1 > int64_t(nnz) ? int64_t(rows) + 1 : int64_t(nnz);
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < top; i += int64_t(gridDim.x) * blockDim.x) {
     bool fail = false;

@@ -44,6 +44,7 @@ __device__ __forceinline__ void copy_at(int k, int m, int n, const Vectors& from
   }
 }
 __global__ void copy_vectors(int m, int n, Vectors from, Vectors to) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) copy_at(k, m, n, from, to);
 }
@@ -51,6 +52,7 @@ __global__ void copy_vectors(int m, int n, Vectors from, Vectors to) {
 // A fresh plan in one launch: all rows and columns kept, the vectors copied.
 __global__ void fresh_plan(int m, int n, Vectors from, Vectors to, uint8_t* __restrict__ keep_row,
                            uint8_t* __restrict__ keep_col) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
     if (k < n) keep_col[k] = 1;
@@ -64,6 +66,7 @@ __global__ void fresh_plan(int m, int n, Vectors from, Vectors to, uint8_t* __re
 __global__ void gather_kept(int m, int n, const int32_t* __restrict__ rmap, const int32_t* __restrict__ cmap,
                             Vectors from, Vectors to, const int32_t* __restrict__ rows, int32_t* __restrict__ rows_to,
                             const int32_t* __restrict__ cols, int32_t* __restrict__ cols_to) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
     if (k < n) {

@@ -65,6 +65,7 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 
 __global__ void fd_pack(int n, const int32_t* __restrict__ ids, const double* __restrict__ sig,
                         uint64_t* __restrict__ keys, int32_t* __restrict__ perm) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     keys[i] = (uint64_t(uint32_t(ids[i])) << 32) | float_key(float(sig[i]));
     perm[i] = i;
@@ -72,6 +73,7 @@ __global__ void fd_pack(int n, const int32_t* __restrict__ ids, const double* __
 }
 // kernel_mark_color_start (folding_kernels.cu:75-90).
 __global__ void fd_starts(int n, const uint64_t* __restrict__ keys, double tol, int32_t* __restrict__ start) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (i == 0) { start[i] = 1; continue; }
     const uint64_t a = keys[i - 1], b = keys[i];
@@ -84,6 +86,7 @@ __global__ void fd_starts(int n, const uint64_t* __restrict__ keys, double tol, 
 __global__ void fd_write(int n, const int32_t* __restrict__ perm, const int32_t* __restrict__ start,
                          const int32_t* __restrict__ excl, int write_sig, uint64_t seed, int32_t* __restrict__ ids,
                          double* __restrict__ sig_out, uint8_t* __restrict__ alone) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int id = excl[i] + start[i];   // inclusive scan: colours are 1-based
     const int member = perm[i];
@@ -93,6 +96,7 @@ __global__ void fd_write(int n, const int32_t* __restrict__ perm, const int32_t*
   }
 }
 __global__ void fd_signatures(int n, const int32_t* __restrict__ ids, uint64_t seed, double* __restrict__ sig) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     sig[i] = color_signature(seed, ids[i]);
 }
@@ -111,6 +115,7 @@ __global__ void __launch_bounds__(kThreads)
 fd_spmv(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
         const double* __restrict__ x, const uint8_t* __restrict__ alone, double* __restrict__ y,
         int32_t* __restrict__ long_rows, int32_t* long_count) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int64_t first = int64_t(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; first < rows;
@@ -161,6 +166,7 @@ __global__ void __launch_bounds__(kThreads)
 fd_spmv_long(const int32_t* __restrict__ long_rows, const int32_t* __restrict__ long_count,
              const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
              const double* __restrict__ x, double* __restrict__ y) {
+  after_previous_kernel();
   __shared__ double stage[2][kSpmvStage];
   const int count = *long_count;
   for (int q = blockIdx.x; q < count; q += gridDim.x) {
@@ -274,10 +280,12 @@ bool refine(const gpp_lp& lp, double tol, Side& rows, Side& cols, cudaStream_t s
 // ---- quotient LP ----------------------------------------------------------
 
 __global__ void fd_count(int n, const int32_t* __restrict__ ids, int32_t* __restrict__ counts) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) atomicAdd(counts + ids[i] - 1, 1);
 }
 __global__ void fd_member_keys(int n, const int32_t* __restrict__ ids, uint64_t* __restrict__ keys,
                                int32_t* __restrict__ vals) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     keys[i] = (uint64_t(uint32_t(ids[i] - 1)) << 32) | uint32_t(i);
     vals[i] = i;
@@ -289,6 +297,7 @@ __global__ void fd_nonconstant(int n, const int32_t* __restrict__ members, const
                                const int32_t* __restrict__ offsets, const double* __restrict__ value,
                                const double* __restrict__ lo, const double* __restrict__ hi,
                                uint32_t* __restrict__ flags) {
+  after_previous_kernel();
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const int member = members[p];
     const int color = ids[member] - 1;
@@ -323,6 +332,7 @@ __device__ bool exact_repeat_sum(double value, int count, double& sum) {
 __global__ void fd_reduce_values(int colors, const int32_t* __restrict__ members, const int32_t* __restrict__ offsets,
                                  const int32_t* __restrict__ counts, const uint32_t* __restrict__ flags,
                                  const double* __restrict__ value, double* __restrict__ out) {
+  after_previous_kernel();
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < colors; col += gridDim.x * blockDim.x) {
     const int b = offsets[col], k = counts[col];
     double sum = 0.0;
@@ -336,6 +346,7 @@ __global__ void fd_reduce_bounds(int colors, const int32_t* __restrict__ members
                                  const int32_t* __restrict__ counts, const uint32_t* __restrict__ flags,
                                  const double* __restrict__ lo, const double* __restrict__ hi,
                                  double* __restrict__ lo_out, double* __restrict__ hi_out) {
+  after_previous_kernel();
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < colors; col += gridDim.x * blockDim.x) {
     const int b = offsets[col], k = counts[col];
     double ls = 0.0, us = 0.0;
@@ -363,6 +374,7 @@ __global__ void fd_entries(int rows, int64_t nnz, const offset_t* __restrict__ p
                            const double* __restrict__ val, const int32_t* __restrict__ rid,
                            const int32_t* __restrict__ cid, const int32_t* __restrict__ rcount, int ncc,
                            uint64_t* __restrict__ keys, int32_t* __restrict__ order, double* __restrict__ weighted) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
   for (int64_t first = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kEntryRun; first < nnz;
@@ -380,6 +392,7 @@ __global__ void fd_entries(int rows, int64_t nnz, const offset_t* __restrict__ p
   }
 }
 __global__ void fd_heads(int64_t n, const uint64_t* __restrict__ keys, int32_t* __restrict__ head) {
+  after_previous_kernel();
   for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < n; q += int64_t(gridDim.x) * blockDim.x)
     head[q] = q == 0 || keys[q] != keys[q - 1] ? 1 : 0;
 }
@@ -388,6 +401,7 @@ __global__ void fd_heads(int64_t n, const uint64_t* __restrict__ keys, int32_t* 
 __global__ void fd_sum_unique(int64_t n, const int32_t* __restrict__ head, const int32_t* __restrict__ hpos,
                               const int32_t* __restrict__ order, const double* __restrict__ weighted,
                               double tol, double* __restrict__ usum, int32_t* __restrict__ keep) {
+  after_previous_kernel();
   for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < n; q += int64_t(gridDim.x) * blockDim.x) {
     if (!head[q]) continue;
     double sum = 0.0;
@@ -401,6 +415,7 @@ __global__ void fd_write_entries(int64_t n, const int32_t* __restrict__ head, co
                                  const uint64_t* __restrict__ keys, const double* __restrict__ usum,
                                  const int32_t* __restrict__ keep, const int32_t* __restrict__ kpos, int ncc,
                                  int32_t* __restrict__ row_cnt, int32_t* __restrict__ oidx, double* __restrict__ oval) {
+  after_previous_kernel();
   for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < n; q += int64_t(gridDim.x) * blockDim.x) {
     if (!head[q]) continue;
     const int u = hpos[q];
@@ -414,6 +429,7 @@ __global__ void fd_write_entries(int64_t n, const int32_t* __restrict__ head, co
 
 __global__ void fd_scale(int n, const int32_t* __restrict__ ids, const int32_t* __restrict__ counts,
                          double* __restrict__ scale) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     scale[i] = 1.0 / double(counts[ids[i] - 1]);
 }
@@ -421,6 +437,7 @@ __global__ void fd_scale(int n, const int32_t* __restrict__ ids, const int32_t* 
 // kernel_unfold_cols / kernel_unfold_rows (folding_map.cu:72-110).
 __global__ void fd_unfold(int n, const int32_t* __restrict__ ids, const double* __restrict__ scale,
                           const double* __restrict__ value, double* __restrict__ out, int scaled) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     out[i] = scaled ? value[ids[i] - 1] * scale[i] : value[ids[i] - 1];
 }

@@ -29,6 +29,7 @@ __device__ __forceinline__ int row_len(const offset_t* ptr, const int32_t* live_
 __global__ void classify_rows(const offset_t* __restrict__ ptr, int m, const int32_t* __restrict__ live_deg,
                               int32_t* __restrict__ medium, int32_t* __restrict__ longq,
                               int32_t* __restrict__ counts) {
+  after_previous_kernel();
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   const int len = row < m ? row_len(ptr, live_deg, row) : 0;
   for (int g = 0; g < 2; ++g) {
@@ -158,6 +159,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
                 const int32_t* __restrict__ counts, int short_blocks, int medium_blocks,
                 double* __restrict__ min_fin, double* __restrict__ max_fin, int32_t* __restrict__ min_inf,
                 int32_t* __restrict__ max_inf, RedundantTest test) {
+  after_previous_kernel();
   __shared__ int slots[256];
   __shared__ int warp_counts[8];
   __shared__ double dagg[8];
@@ -336,6 +338,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
 __global__ void pack_bounds_kernel(int n, const double* __restrict__ l, const double* __restrict__ u,
                                    const uint8_t* __restrict__ keep, double2* __restrict__ lu,
                                    double* __restrict__ cand_l, double* __restrict__ cand_u) {
+  after_previous_kernel();
   const double removed = __longlong_as_double(static_cast<long long>(kRemovedColumnBits));
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const double lj = l[j], uj = u[j];
@@ -368,6 +371,7 @@ live_stats_kernel(int rows, const offset_t* __restrict__ ptr, const int32_t* __r
                   const int32_t* __restrict__ longq, const int32_t* __restrict__ counts, int short_blocks,
                   int medium_blocks, int32_t* degree, uint8_t* empty, uint8_t* singleton,
                   int32_t* support, double* coefficient, unsigned long long* total) {
+  after_previous_kernel();
   __shared__ int scount[8];
   __shared__ long long spos[8];
   __shared__ unsigned long long stotal[8];
@@ -459,6 +463,7 @@ col_max_kernel(int rows, const offset_t* __restrict__ ptr, const int32_t* __rest
                const double* __restrict__ val, const uint8_t* __restrict__ keep_row,
                const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
                const int32_t* __restrict__ counts, int short_blocks, int medium_blocks, double* out) {
+  after_previous_kernel();
   __shared__ double smax[8];
   const int b = blockIdx.x;
   if (b < short_blocks) {
@@ -558,6 +563,7 @@ namespace {
 // tile ends at nnz - 1), falls in [ptr[r], ptr[r+1]): every tile gets both
 // rows with no search, in one pass over the row pointers.
 __global__ void tile_rows_kernel(int rows, offset_t nnz, const offset_t* __restrict__ ptr, int2* __restrict__ tile_rows) {
+  after_previous_kernel();
   constexpr int64_t T = kEntryTile;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
     const int64_t a = ptr[r], b = ptr[r + 1];
@@ -694,6 +700,7 @@ __device__ __forceinline__ void find_deleted(int n, uint8_t* __restrict__ seen, 
 __global__ void inc_deleted(int m, int n, uint8_t* __restrict__ seen_row, const uint8_t* __restrict__ keep_row,
                             uint8_t* __restrict__ seen_col, const uint8_t* __restrict__ keep_col,
                             int32_t* __restrict__ list, int32_t* counters) {
+  after_previous_kernel();
   find_deleted(m, seen_row, keep_row, list, counters);
   find_deleted(n, seen_col, keep_col, list + m, counters + 1);
 }
@@ -722,6 +729,7 @@ struct SideStats {
 __global__ void __launch_bounds__(kThreads) inc_walk(int m, const int32_t* __restrict__ list,
                                                      const int32_t* __restrict__ counters, SideStats rows,
                                                      SideStats cols, unsigned long long* live_nnz) {
+  after_previous_kernel();
   const int half = gridDim.x / 2;
   const bool row_side = int(blockIdx.x) < half;
   const SideStats& outer = row_side ? rows : cols;
@@ -777,6 +785,7 @@ __device__ __forceinline__ void fix_dirty(int n, const SideStats& outer, const u
 }
 __global__ void inc_fix(int m, int n, SideStats rows, SideStats cols, int32_t* __restrict__ counters,
                         const unsigned long long* __restrict__ live_nnz, Mailbox* box, uint32_t seq) {
+  after_previous_kernel();
   if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;   // for the next refresh
   if (blockIdx.x == 0 && threadIdx.x == 0) post_values(box, seq, int64_t(*live_nnz));
   fix_dirty(m, rows, cols.keep);
@@ -800,6 +809,7 @@ __device__ __forceinline__ void full_item(int r, const SideStats& s, uint8_t* __
 __global__ void stats_of_full_model(int m, int n, offset_t nnz, SideStats rows, SideStats cols,
                                     uint8_t* __restrict__ seen_row, uint8_t* __restrict__ seen_col,
                                     unsigned long long* __restrict__ live_nnz, int32_t* __restrict__ counters) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
     if (k == 0) {

@@ -307,6 +307,7 @@ struct SegView {
 __global__ void scatter_solution(Sol s, const double* __restrict__ x_red, const double* __restrict__ y_red,
                                  const double* __restrict__ z_red, const int32_t* __restrict__ rows, int32_t m,
                                  const int32_t* __restrict__ cols, int32_t n) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < top; i += gridDim.x * blockDim.x) {
     if (i < n) {
@@ -327,6 +328,7 @@ struct FixedView {
   int64_t count;
 };
 __global__ void restore_fixed(double* __restrict__ x, const FixedView* __restrict__ fixed, int segments) {
+  after_previous_kernel();
   for (int k = 0; k < segments; ++k) {
     const FixedView f = fixed[k];
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < f.count; i += int64_t(gridDim.x) * blockDim.x)
@@ -337,6 +339,7 @@ __global__ void restore_fixed(double* __restrict__ x, const FixedView* __restric
 // warp per column, A^T y summed sequentially by lane 0 in stored order.
 __global__ void project_duals(int n, const uint8_t* __restrict__ prot, Model M, const double* __restrict__ x,
                               const double* __restrict__ y, double* __restrict__ z) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (prot[j]) continue;
     double aty = 0.0;
@@ -566,16 +569,19 @@ __device__ __forceinline__ void replay_at(const TapeView& t, int64_t g, const So
 
 __global__ void rg_claim(TapeView t, int64_t lo, int count, int dual, int m, int n, Model M,
                          const double* __restrict__ x, int32_t* owner, int32_t* __restrict__ parent) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
     claim_record(t, lo, q, dual != 0, m, n, M, x, owner, parent);
 }
 __global__ void rg_connect(TapeView t, int64_t lo, int count, int dual, int m, int n, Model M,
                            const int32_t* __restrict__ owner, int32_t* parent) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x)
     connect_record(t, lo, q, dual != 0, m, n, M, owner, parent);
 }
 // Roots are final: a root with another member is marked.
 __global__ void rg_roots(int count, int32_t* parent, uint8_t* __restrict__ shared_root) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
     if (parent[q] < 0) continue;
     const int r = uf_root(parent, q);
@@ -591,6 +597,7 @@ __global__ void __launch_bounds__(kThreads) rg_replay_alone(TapeView t, int64_t 
                                                             int32_t* parent, const uint8_t* __restrict__ shared_root,
                                                             uint64_t* __restrict__ keys, int32_t* __restrict__ vals,
                                                             Report report) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int64_t top = (int64_t(count) + stride - 1) / stride * stride;
   for (int64_t p = blockIdx.x * blockDim.x + threadIdx.x; p < top; p += stride) {
@@ -611,6 +618,7 @@ __global__ void __launch_bounds__(kThreads) rg_replay_alone(TapeView t, int64_t 
 // replays it and walks back to the group's first.
 __global__ void rg_replay_groups(TapeView t, int64_t lo, int listed, const uint64_t* __restrict__ keys, int dual, Sol s,
                                  Model M) {
+  after_previous_kernel();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < listed; e += gridDim.x * blockDim.x) {
     const uint32_t root = uint32_t(keys[e] >> 32);
     if (e + 1 < listed && uint32_t(keys[e + 1] >> 32) == root) continue;
@@ -632,6 +640,7 @@ constexpr int kBlockTape = 2048;
 constexpr int kBlockReplayThreads = 512;
 __global__ void __launch_bounds__(kBlockReplayThreads)
 replay_block(TapeView t, int64_t lo, int count, int primal, int dual, int m, int n, Sol s, Model M, int32_t* owner) {
+  after_previous_kernel();
   __shared__ int32_t parent[kBlockTape];
   __shared__ uint32_t key[kBlockTape];
   __shared__ uint8_t shared_root[kBlockTape];
@@ -726,6 +735,7 @@ void replay_range(const TapeView& t, int m0, int n0, const Sol& s, const Model& 
 }
 
 __global__ void mark_protected(TapeView t, uint8_t* __restrict__ prot, int n) {
+  after_previous_kernel();
   for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < t.total; g += int64_t(gridDim.x) * blockDim.x) {
     const RecordAt r(t, g);
     int a = -1, b = -1;
@@ -742,6 +752,7 @@ __global__ void mark_protected(TapeView t, uint8_t* __restrict__ prot, int n) {
 
 __global__ void restore_splits(double* __restrict__ x, const int32_t* __restrict__ t, const int32_t* __restrict__ e,
                                const double* __restrict__ rho, int k) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
     const double tv = x[t[i]], ev = x[e[i]];
     x[t[i]] = tv + ev;
@@ -750,10 +761,12 @@ __global__ void restore_splits(double* __restrict__ x, const int32_t* __restrict
 }
 __global__ void restore_pairs(double* __restrict__ x, const int32_t* __restrict__ bound,
                               const int32_t* __restrict__ free_col, int k) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) x[free_col[i]] = x[bound[i]];
 }
 __global__ void restore_links(double* __restrict__ x, const int32_t* __restrict__ slack, const int32_t* __restrict__ t,
                               const double* __restrict__ f, int k) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) x[slack[i]] = f[i] * x[t[i]];
 }
 // One warp per group: slack = max(l_slack (0 when absent or not finite),
@@ -762,6 +775,7 @@ __global__ void restore_links(double* __restrict__ x, const int32_t* __restrict_
 __global__ void restore_max_slacks(double* __restrict__ x, const int32_t* __restrict__ slack,
                                    const int32_t* __restrict__ start, const int32_t* __restrict__ t,
                                    const double* __restrict__ f, int groups, const double* __restrict__ lower) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < groups; g += (gridDim.x * blockDim.x) >> 5) {
     const int32_t sc = slack[g];
@@ -778,6 +792,7 @@ __global__ void restore_max_slacks(double* __restrict__ x, const int32_t* __rest
 // postsolve_piecewise_linear_reformulation_variable_pair.cu:9-95).
 __global__ void cache_pair_roots(double* __restrict__ pc, double* __restrict__ mc, const double* __restrict__ x,
                                  const int32_t* __restrict__ rp, const int32_t* __restrict__ rm, int k) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
     pc[i] = x[rp[i]];
     mc[i] = x[rm[i]];
@@ -787,6 +802,7 @@ __global__ void restore_pair_members(double* __restrict__ x, const int32_t* __re
                                      const int32_t* __restrict__ minus, const double* __restrict__ ps,
                                      const double* __restrict__ ms, const double* __restrict__ pc,
                                      const double* __restrict__ mc, int k) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
     x[plus[i]] = ps[i] + pc[i];
     x[minus[i]] = ms[i] + mc[i];

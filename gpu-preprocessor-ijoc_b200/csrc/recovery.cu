@@ -13,6 +13,7 @@ namespace gpp {
 namespace {
 
 __global__ void iota(int32_t* a, int32_t n) {
+  after_previous_kernel();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     a[i] = int32_t(i);
 }
@@ -31,6 +32,7 @@ enum : int {
 __global__ void globalize_kernel(int64_t count, const int32_t* __restrict__ types, const int64_t* __restrict__ is,
                                  int32_t* __restrict__ idx, const int32_t* __restrict__ rows, int m,
                                  const int32_t* __restrict__ cols, int n) {
+  after_previous_kernel();
   for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < count; k += int64_t(gridDim.x) * blockDim.x) {
     int32_t* id = idx + is[k];
     const int64_t sz = is[k + 1] - is[k];
@@ -101,6 +103,7 @@ __global__ void globalize_kernel(int64_t count, const int32_t* __restrict__ type
 }
 
 __global__ void globalize_ids(int32_t* __restrict__ ids, int64_t n, const int32_t* __restrict__ cols) {
+  after_previous_kernel();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     ids[i] = cols[ids[i]];
 }

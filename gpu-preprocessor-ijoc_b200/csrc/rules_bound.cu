@@ -91,6 +91,7 @@ constexpr int kTileRows = 2048;
 
 __global__ void __launch_bounds__(kThreads)
 candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, CandArgs g) {
+  after_previous_kernel();
   __shared__ offset_t sptr[kTileRows + 1];
   const L2Hints hint = l2_hints();
   for (offset_t base = offset_t(blockIdx.x) * kEntryTile; base < nnz; base += offset_t(gridDim.x) * kEntryTile) {
@@ -247,6 +248,7 @@ finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const do
                 double2* __restrict__ lu, const double* __restrict__ c, const double* __restrict__ vmax,
                 int preserve_free_zero_cost, double ft, double upper_relax, bool records, SupportArgs g, FinalBounds out,
                 unsigned long long* words, unsigned int* counters, int32_t* error, Report report) {
+  after_previous_kernel();
   __shared__ int warp_sums[2][kThreads / 32];
   __shared__ long long tile_before[2];
   __shared__ unsigned int ticket;
@@ -359,6 +361,7 @@ struct BoundRecords {
 __global__ void commit_bounds(int n, FinalBounds f, bool records, BoundRecords rec, double* __restrict__ l,
                               double* __restrict__ u, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ fixed,
                               double* __restrict__ fixed_at) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (records && j == 0) { rec.is[0] = 0; rec.vs[0] = 0; }
     const uint8_t change = f.change[j];
@@ -400,6 +403,7 @@ __global__ void shift_and_empty_rows(int m, const offset_t* __restrict__ ptr, co
                                      const double* __restrict__ shift, const uint8_t* __restrict__ keep_col,
                                      uint8_t* __restrict__ keep_row, double* __restrict__ AL,
                                      double* __restrict__ AU, double ft, Report report) {
+  after_previous_kernel();
   uint32_t infeasible = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     AL[i] -= shift[i];
@@ -418,6 +422,7 @@ __global__ void shift_and_empty_rows(int m, const offset_t* __restrict__ ptr, co
 __global__ void fixed_record_sizes(int n, const uint8_t* __restrict__ fx, const offset_t* __restrict__ at_ptr,
                                    const int32_t* __restrict__ at_idx, const uint8_t* __restrict__ keep_row,
                                    int64_t* __restrict__ recs, int64_t* __restrict__ nz) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     int64_t c = 0;
     if (fx[j])
@@ -433,6 +438,7 @@ __global__ void fixed_record_pack(int n, const uint8_t* __restrict__ fx, const o
                                   const int64_t* __restrict__ nz_pos, int32_t* __restrict__ types,
                                   int64_t* __restrict__ is, int64_t* __restrict__ vs, int32_t* __restrict__ idx,
                                   double* __restrict__ val, double* __restrict__ obj_c, double* __restrict__ obj_v) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (j == 0) { is[0] = 0; vs[0] = 0; }
     if (!fx[j]) continue;
@@ -455,6 +461,7 @@ __global__ void fixed_record_pack(int n, const uint8_t* __restrict__ fx, const o
 // activity (0, 1, 2, >= 3): the learned schedule's histogram features.
 __global__ void inf_histogram(int m, const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ ni,
                               const int32_t* __restrict__ pi, uint32_t* __restrict__ hist) {
+  after_previous_kernel();
   __shared__ uint32_t bins[8];
   if (threadIdx.x < 8) bins[threadIdx.x] = 0;
   __syncthreads();

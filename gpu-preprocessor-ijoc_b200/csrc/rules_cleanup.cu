@@ -17,6 +17,7 @@ namespace {
 __global__ void mark_touched_rows(int n, const offset_t* __restrict__ at_ptr, const int32_t* __restrict__ at_idx,
                                   const uint8_t* __restrict__ selected, const double* __restrict__ radius,
                                   uint8_t* __restrict__ touched) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (!selected[j] || (radius && !(radius[j] > 0.0))) continue;
     for (offset_t p = at_ptr[j]; p < at_ptr[j + 1]; ++p) touched[at_idx[p]] = 1;
@@ -26,6 +27,7 @@ __global__ void mark_touched_rows(int n, const offset_t* __restrict__ at_ptr, co
 // Kept touched rows are listed; every other row's sum is 0.
 __global__ void list_touched_rows(int m, const uint8_t* __restrict__ keep_row, const uint8_t* __restrict__ touched,
                                   int32_t* __restrict__ list, int32_t* counter, double* __restrict__ out) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (m + stride - 1) / stride * stride;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < top; i += stride) {
@@ -44,6 +46,7 @@ __global__ void row_gather_kernel(const int32_t* __restrict__ list, const int32_
                                   const double* __restrict__ val, const uint8_t* __restrict__ selected,
                                   const double* __restrict__ value, const double* __restrict__ radius,
                                   double* __restrict__ out) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   const int k = *count;
@@ -81,6 +84,7 @@ __global__ void fixed_candidates(int n, const uint8_t* __restrict__ keep_col, co
                                  const double* __restrict__ u, const double* __restrict__ c, double bound_tol,
                                  uint8_t* __restrict__ fixed, double* __restrict__ fval,
                                  double* __restrict__ contrib, double* __restrict__ radius, Report report) {
+  after_previous_kernel();
   uint32_t any = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     uint8_t f = 0;
@@ -103,6 +107,7 @@ __global__ void fixed_filter(int n, const offset_t* __restrict__ at_ptr, const i
                              const uint8_t* __restrict__ keep_row, const double* __restrict__ l,
                              const double* __restrict__ u, const double* __restrict__ row_error, double budget,
                              uint8_t* __restrict__ fixed, double* __restrict__ contrib, Report report) {
+  after_previous_kernel();
   uint32_t any = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (!fixed[j]) continue;
@@ -120,6 +125,7 @@ __global__ void fixed_filter(int n, const offset_t* __restrict__ at_ptr, const i
 __global__ void fixed_apply(int n, int m, const uint8_t* __restrict__ fixed, const double* __restrict__ fval,
                             const double* __restrict__ shift, uint8_t* __restrict__ keep_col, double* __restrict__ l,
                             double* __restrict__ u, double* __restrict__ AL, double* __restrict__ AU) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += gridDim.x * blockDim.x) {
     if (j < n && fixed[j]) { l[j] = fval[j]; u[j] = fval[j]; keep_col[j] = 0; }
@@ -133,6 +139,7 @@ __global__ void empty_columns_classify(int n, const uint8_t* __restrict__ keep_c
                                        const double* __restrict__ u, double bound_tol, double zero_tol,
                                        uint8_t* __restrict__ fixed, double* __restrict__ fval,
                                        double* __restrict__ contrib, Report report) {
+  after_previous_kernel();
   uint32_t found = 0;   // 1 infeasible, 2 unbounded, 4 fixed
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     fixed[j] = 0; fval[j] = 0.0; contrib[j] = 0.0;
@@ -152,6 +159,7 @@ __global__ void empty_columns_classify(int n, const uint8_t* __restrict__ keep_c
 }
 __global__ void fix_columns(int n, const uint8_t* __restrict__ fixed, const double* __restrict__ fval,
                             uint8_t* __restrict__ keep_col, double* __restrict__ l, double* __restrict__ u) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
     if (fixed[j]) { l[j] = fval[j]; u[j] = fval[j]; keep_col[j] = 0; }
 }
@@ -161,6 +169,7 @@ __device__ __forceinline__ bool empty_row_feasible(double lo, double hi, double 
 __global__ void empty_rows_find(int m, const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
                                 const double* __restrict__ AL, const double* __restrict__ AU, double tol,
                                 Report report) {
+  after_previous_kernel();
   uint32_t found = 0;   // 1 infeasible, 2 removable
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     if (keep_row[i] && row_nnz[i] == 0) found |= empty_row_feasible(AL[i], AU[i], tol) ? 2u : 1u;
@@ -168,6 +177,7 @@ __global__ void empty_rows_find(int m, const uint8_t* __restrict__ keep_row, con
 }
 __global__ void empty_rows_remove(int m, uint8_t* __restrict__ keep_row, const int32_t* __restrict__ row_nnz,
                                   const double* __restrict__ AL, const double* __restrict__ AU, double tol) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     if (keep_row[i] && row_nnz[i] == 0 && empty_row_feasible(AL[i], AU[i], tol)) keep_row[i] = 0;
 }
@@ -178,6 +188,7 @@ __global__ void singleton_row_bounds(int m, int n, const uint8_t* __restrict__ k
                                      const double* __restrict__ sval, const double* __restrict__ AL,
                                      const double* __restrict__ AU, double zero_tol, double* cand_l, double* cand_u,
                                      uint8_t* __restrict__ remove) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     remove[i] = 0;
     if (!(keep_row[i] && singleton[i])) continue;
@@ -193,6 +204,7 @@ __global__ void singleton_row_bounds(int m, int n, const uint8_t* __restrict__ k
 __global__ void singleton_rows_check(int m, int n, const double* __restrict__ cand_l, const double* __restrict__ cand_u,
                                      const double* __restrict__ l, const double* __restrict__ u,
                                      const uint8_t* __restrict__ remove, double tol, Report report) {
+  after_previous_kernel();
   uint32_t found = 0;   // 1 infeasible, 2 a row goes, 4 a bound changes
   const int top = n > m ? n : m;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += gridDim.x * blockDim.x) {
@@ -205,6 +217,7 @@ __global__ void singleton_rows_check(int m, int n, const double* __restrict__ ca
   post_flags(report, found);
 }
 __global__ void singleton_rows_commit(int m, int n, const uint8_t* __restrict__ remove, uint8_t* __restrict__ keep_row) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     if (remove[i]) keep_row[i] = 0;
 }
@@ -252,6 +265,7 @@ cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ k
                      const uint8_t* __restrict__ singleton_row, const int32_t* __restrict__ scol,
                      const double* __restrict__ sval, double bound_tol, double zero_tol, int32_t* __restrict__ sc_owner,
                      int32_t* __restrict__ sc_words, Report report) {
+  after_previous_kernel();
   uint32_t f = 0;
   // The singleton-column rule's scratch, which it needs cleared.
   if (blockIdx.x == 0 && threadIdx.x < kSingletonWords) sc_words[threadIdx.x] = 0;

@@ -47,6 +47,7 @@ enum : uint8_t { kPairNone = 0, kPairSubst = 1, kPairFixed = 2 };
 __global__ void dt_col_nnz(int n, const offset_t* __restrict__ tptr, const int32_t* __restrict__ tidx,
                            const double* __restrict__ tval, const uint8_t* __restrict__ keep_row,
                            const uint8_t* __restrict__ keep_col, double zt, int32_t* __restrict__ col_nnz) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     int cnt = 0;
     if (keep_col[j])
@@ -125,6 +126,7 @@ __global__ void dt_candidates(int m, const offset_t* __restrict__ ptr, const int
                               const int32_t* __restrict__ tidx, const double* __restrict__ tval,
                               int32_t* __restrict__ flag, int32_t* __restrict__ keep_c, int32_t* __restrict__ elim_c,
                               double* __restrict__ keep_v, double* __restrict__ elim_v) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     flag[i] = 0;
     if (!keep_row[i]) continue;
@@ -210,15 +212,18 @@ struct Matching {
   }
 };
 __global__ void dt_claim(Matching g, int round) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.count; q += gridDim.x * blockDim.x) g.claim(round, q);
 }
 __global__ void dt_select(Matching g, int round) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.count; q += gridDim.x * blockDim.x) g.select(round, q);
 }
 // All rounds in one block: up to kBlockMatch rows the sixteen launches cost
 // more than the rows.
 constexpr int kBlockMatch = 4096;
 __global__ void __launch_bounds__(1024) dt_match_block(Matching g) {
+  after_previous_kernel();
   for (int round = 0; round < kRounds; ++round) {
     for (int q = threadIdx.x; q < g.count; q += blockDim.x) g.claim(round, q);
     __syncthreads();
@@ -237,6 +242,7 @@ __global__ void dt_apply(int sel, const int32_t* __restrict__ rows, const int32_
                          double* __restrict__ alpha_out, double* __restrict__ beta_out,
                          double* __restrict__ obj_term, int32_t* __restrict__ rec_idx, double* __restrict__ rec_val,
                          Report report) {
+  after_previous_kernel();
   uint32_t found = 0;   // 1 infeasible, 2 any pair applied; word 1 counts the substitutions
   int substituted = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sel; t += gridDim.x * blockDim.x) {
@@ -311,6 +317,7 @@ __global__ void dt_roles(int sel, const int32_t* __restrict__ rows, const int32_
                          const int32_t* __restrict__ elim_c, const uint8_t* __restrict__ kind,
                          const double* __restrict__ beta, const double* __restrict__ l, uint8_t* __restrict__ role,
                          double* __restrict__ value, int32_t* __restrict__ role_col) {
+  after_previous_kernel();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sel; t += gridDim.x * blockDim.x) {
     const int row = rows[t];
     int col = -1;
@@ -325,6 +332,7 @@ __global__ void dt_roles(int sel, const int32_t* __restrict__ rows, const int32_
 __global__ void dt_touch(int sel, const int32_t* __restrict__ role_col, const offset_t* __restrict__ tptr,
                          const int32_t* __restrict__ tidx, uint32_t* __restrict__ claimed,
                          int32_t* __restrict__ touched, int32_t* st, Report report) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
@@ -352,6 +360,7 @@ __global__ void dt_shift(const int32_t* __restrict__ touched, const int32_t* __r
                          const double* __restrict__ val, const uint8_t* __restrict__ keep_row,
                          const uint8_t* __restrict__ role, const double* __restrict__ value, double zt,
                          double* __restrict__ AL, double* __restrict__ AU) {
+  after_previous_kernel();
   const int count = st[kStTouched];
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
@@ -384,6 +393,7 @@ __global__ void dt_delta_count(int sel, const int32_t* __restrict__ rows, const 
                                const uint8_t* __restrict__ kind, const offset_t* __restrict__ tptr,
                                const int32_t* __restrict__ tidx, const double* __restrict__ tval,
                                const uint8_t* __restrict__ keep_row, double zt, int32_t* __restrict__ cnt) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
@@ -405,6 +415,7 @@ __global__ void dt_delta_fill(int sel, const int32_t* __restrict__ rows, const i
                               const int32_t* __restrict__ tidx, const double* __restrict__ tval,
                               const uint8_t* __restrict__ keep_row, double zt, const int32_t* __restrict__ pos,
                               uint64_t* __restrict__ keys, int32_t* __restrict__ order, double* __restrict__ dval) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
@@ -436,6 +447,7 @@ __global__ void dt_delta_fill(int sel, const int32_t* __restrict__ rows, const i
 __global__ void dt_delta_rows(int64_t total, const uint64_t* __restrict__ keys, const int32_t* __restrict__ order,
                               const double* __restrict__ raw, int32_t* __restrict__ dcol, double* __restrict__ dv,
                               int32_t* __restrict__ row_cnt) {
+  after_previous_kernel();
   for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < total; q += int64_t(gridDim.x) * blockDim.x) {
     const uint64_t key = keys[q];
     dcol[q] = int32_t(key & 0xffffffffu);
@@ -474,6 +486,7 @@ __global__ void dt_rebuild(int m, const offset_t* __restrict__ ptr, const int32_
                            const int32_t* __restrict__ dcol, const double* __restrict__ dv, double zt, bool sorted,
                            int32_t* __restrict__ cnt, const offset_t* __restrict__ optr, int32_t* __restrict__ oidx,
                            double* __restrict__ oval) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += warps) {
@@ -506,6 +519,7 @@ __global__ void dt_rebuild(int m, const offset_t* __restrict__ ptr, const int32_
 // kernel leaves out, listed once.
 __global__ void dt_long_delta_rows(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ dptr,
                                    int32_t* __restrict__ list, int32_t* counter) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (m + stride - 1) / stride * stride;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < top; r += stride) {
@@ -542,6 +556,7 @@ dt_rebuild_block(const int32_t* __restrict__ list, const int32_t* __restrict__ c
                  const int32_t* __restrict__ idx, const double* __restrict__ val, const int32_t* __restrict__ dptr,
                  const int32_t* __restrict__ dcol, const double* __restrict__ dv, double zt, int32_t* __restrict__ cnt,
                  const offset_t* __restrict__ optr, int32_t* __restrict__ oidx, double* __restrict__ oval) {
+  after_previous_kernel();
   __shared__ int scan[kThreads];
   __shared__ int kcol[kBlockMergeDeltas];
   __shared__ int kins[kBlockMergeDeltas];
@@ -626,6 +641,7 @@ __global__ void dt_single_apply(const int32_t* __restrict__ acc, const int32_t* 
                                 uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col,
                                 double* __restrict__ meta, int32_t* __restrict__ rec_idx, double* __restrict__ rec_val,
                                 int32_t* st) {
+  after_previous_kernel();
   const int row = acc[0], k = keep_c[row], e = elim_c[row];
   const double kv = keep_v[row], ev = elim_v[row], rhs = AU[row];
   const double le = l[e], ue = u[e], lk = l[k], uk = u[k], ce = c[e];
@@ -657,6 +673,7 @@ __global__ void dt_single_shift(const int32_t* __restrict__ acc, const int32_t* 
                                 const offset_t* __restrict__ tptr, const int32_t* __restrict__ tidx,
                                 const double* __restrict__ tval, const double* __restrict__ meta,
                                 const int32_t* __restrict__ st, double* __restrict__ AL, double* __restrict__ AU) {
+  after_previous_kernel();
   if (!st[kStAny]) return;
   const int e = elim_c[acc[0]];
   const offset_t b = tptr[e], end = tptr[e + 1];
@@ -681,6 +698,7 @@ __global__ void dt_single_rows(int m, const offset_t* __restrict__ ptr, const in
                                const double* __restrict__ meta, double zt, int32_t* __restrict__ cnt,
                                const offset_t* __restrict__ optr, int32_t* __restrict__ oidx,
                                double* __restrict__ oval) {
+  after_previous_kernel();
   const int target = acc[0], e = elim_c[target], k = keep_c[target];
   const double alpha = meta[0];
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {

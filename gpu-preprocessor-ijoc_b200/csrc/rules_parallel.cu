@@ -213,6 +213,7 @@ __device__ void row_hash_grouped(const RowHashArgs& g, int i) {
 __global__ void __launch_bounds__(kThreads)
 row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
                 const int32_t* __restrict__ counts, int short_blocks) {
+  after_previous_kernel();
   const int b = blockIdx.x;
   if (b < short_blocks) {
     for (int i = b * blockDim.x + threadIdx.x; i < rows; i += short_blocks * blockDim.x)
@@ -251,6 +252,7 @@ __device__ __forceinline__ uint64_t mix_hash(uint64_t z) {
 }
 __global__ void mark_hash_bits(int n, const uint8_t* __restrict__ keep, const uint64_t* __restrict__ hash,
                                uint32_t* __restrict__ seen, uint32_t* __restrict__ twice, uint64_t bit_mask) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (!keep[i]) continue;
     const uint64_t z = mix_hash(hash[i]);
@@ -309,6 +311,7 @@ __global__ void row_groups_kernel(int count, const uint64_t* __restrict__ sh, co
                                   const int32_t* __restrict__ idx, const double* __restrict__ val, double coeff_tol,
                                   double interval_tol, uint8_t* __restrict__ del, int32_t* __restrict__ merge_to,
                                   int32_t* __restrict__ step_out, double* __restrict__ rec_vals, Report report) {
+  after_previous_kernel();
   uint32_t infeasible = 0;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count && !infeasible; s += gridDim.x * blockDim.x) {
     const uint64_t hs = sh[s];
@@ -369,6 +372,7 @@ __global__ void pack_parallel_records(int64_t count, const int32_t* __restrict__
                                       const double* __restrict__ rec_vals, int type, int32_t* __restrict__ types,
                                       int64_t* __restrict__ is, int64_t* __restrict__ vs, int32_t* __restrict__ idx,
                                       double* __restrict__ val) {
+  after_previous_kernel();
   for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k <= count; k += int64_t(gridDim.x) * blockDim.x) {
     is[k] = 2 * k;
     vs[k] = 5 * k;
@@ -386,6 +390,7 @@ __global__ void pack_parallel_records(int64_t count, const int32_t* __restrict__
 __global__ void col_hash_kernel(int n, const uint8_t* __restrict__ keep_col, const uint8_t* __restrict__ keep_row,
                                 const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                                 const double* __restrict__ val, double tol, uint64_t* __restrict__ out) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (!keep_col[j]) { out[j] = uint64_t(j); continue; }
     int len = 0;
@@ -452,6 +457,7 @@ __global__ void count_guard_groups(int count, const uint64_t* __restrict__ sh, c
                                    const int32_t* __restrict__ idx, const double* __restrict__ val, double zt,
                                    double coeff_tol, double obj_tol, double max_abs, int max_size, int stop_after,
                                    int32_t* __restrict__ out) {
+  after_previous_kernel();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < count; s += gridDim.x * blockDim.x) {
     // Early exit once enough groups are counted: a plain (volatile) read, as
     // an atomic read of one address from every thread serialises them.
@@ -558,6 +564,7 @@ constexpr int kGroupThread = 8;
 __global__ void __launch_bounds__(kThreads)
 col_groups_kernel(int count, const uint64_t* __restrict__ sh, ColumnGroups g, double max_abs,
                   const int32_t* __restrict__ guard, int guard_min, Report report) {
+  after_previous_kernel();
   uint32_t found = 0;
   const int lane = threadIdx.x & 31;
   const double active_max = guard && *guard < guard_min ? INFINITY : max_abs;
@@ -655,6 +662,7 @@ __global__ void col_apply(int n, int m, const uint8_t* __restrict__ del, const u
                           const double* __restrict__ fval, const double* __restrict__ c, const double* __restrict__ shift,
                           uint8_t* __restrict__ keep_col, double* __restrict__ l, double* __restrict__ u,
                           double* __restrict__ AL, double* __restrict__ AU, double* __restrict__ contrib) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < top; q += gridDim.x * blockDim.x) {
     if (q < n) {
@@ -671,6 +679,7 @@ __global__ void col_apply(int n, int m, const uint8_t* __restrict__ del, const u
 __global__ void fixed_sizes(int n, const uint8_t* __restrict__ fx, const offset_t* __restrict__ at_ptr,
                             const int32_t* __restrict__ at_idx, const uint8_t* __restrict__ keep_row,
                             int64_t* __restrict__ recs, int64_t* __restrict__ nz) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     int64_t c = 0;
     if (fx[j])
@@ -685,6 +694,7 @@ __global__ void fixed_pack(int n, const uint8_t* __restrict__ fx, const offset_t
                            const double* __restrict__ c, const int64_t* __restrict__ rpos,
                            const int64_t* __restrict__ npos, int32_t* __restrict__ types, int64_t* __restrict__ is,
                            int64_t* __restrict__ vs, int32_t* __restrict__ idx, double* __restrict__ val) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (j == 0) { is[0] = 0; vs[0] = 0; }
     if (!fx[j]) continue;

@@ -12,6 +12,7 @@ namespace {
 
 __global__ void redundant_apply(int m, const uint8_t* __restrict__ action, uint8_t* __restrict__ keep_row,
                                 double* __restrict__ AL, double* __restrict__ AU) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     const uint8_t a = action[i];
     if (a == 1) keep_row[i] = 0;
@@ -29,6 +30,7 @@ __global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col,
                                     double zt, double bound_tol, int max_degree, const int32_t* __restrict__ col_nnz,
                                     uint8_t* __restrict__ fixed, uint8_t* __restrict__ inf_fix,
                                     double* __restrict__ fval, double* __restrict__ contrib, Report report) {
+  after_previous_kernel();
   uint32_t found = 0;   // 1 infeasible, 2 unbounded, 4 a column is fixed, 8 at an infinite bound
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     fixed[j] = 0; inf_fix[j] = 0; fval[j] = 0.0; contrib[j] = 0.0;
@@ -65,6 +67,7 @@ __global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col,
 }
 __global__ void finite_fixed_mask(int n, const uint8_t* __restrict__ fixed, const uint8_t* __restrict__ inf_fix,
                                   uint8_t* __restrict__ out) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
     out[j] = fixed[j] && !inf_fix[j];
 }
@@ -72,6 +75,7 @@ __global__ void dual_fix_row_remove(int n, const uint8_t* __restrict__ fixed, co
                                     const uint8_t* __restrict__ keep_row, const offset_t* __restrict__ at_ptr,
                                     const int32_t* __restrict__ at_idx, uint8_t* __restrict__ remove,
                                     Report report) {
+  after_previous_kernel();
   uint32_t any = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (!(fixed[j] && inf_fix[j])) continue;
@@ -87,6 +91,7 @@ __global__ void infinite_sizes(int n, const uint8_t* __restrict__ fixed, const u
                                const offset_t* __restrict__ a_ptr, const int32_t* __restrict__ a_idx,
                                const offset_t* __restrict__ at_ptr, const int32_t* __restrict__ at_idx,
                                int64_t* __restrict__ recs, int64_t* __restrict__ sizes) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const bool sel = fixed[j] && inf_fix[j];
     int64_t size = 0;
@@ -111,6 +116,7 @@ __global__ void infinite_pack(int n, const uint8_t* __restrict__ fixed, const ui
                               const int64_t* __restrict__ rpos, const int64_t* __restrict__ spos,
                               int32_t* __restrict__ types, int64_t* __restrict__ is, int64_t* __restrict__ vs,
                               int32_t* __restrict__ idx, double* __restrict__ val) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     if (j == 0) { is[0] = 0; vs[0] = 0; }
     if (!(fixed[j] && inf_fix[j])) continue;
@@ -148,6 +154,7 @@ __global__ void dual_fix_apply(int n, int m, const uint8_t* __restrict__ fixed, 
                                uint8_t* __restrict__ keep_col, uint8_t* __restrict__ keep_row,
                                double* __restrict__ l, double* __restrict__ u, double* __restrict__ AL,
                                double* __restrict__ AU) {
+  after_previous_kernel();
   const int top = n > m ? n : m;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
     if (k < n && fixed[k]) { l[k] = fval[k]; u[k] = fval[k]; keep_col[k] = 0; }

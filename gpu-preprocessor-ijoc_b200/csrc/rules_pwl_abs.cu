@@ -86,6 +86,7 @@ __device__ PairRow pair_row(int row, const offset_t* __restrict__ ptr, const int
 __global__ void row_metadata(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                              const double* __restrict__ val, const double* __restrict__ AL,
                              const double* __restrict__ AU, PairRow* __restrict__ rows) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     rows[i] = pair_row(i, ptr, idx, val, AL, AU);
 }
@@ -136,6 +137,7 @@ __device__ __forceinline__ void fail(int32_t* status) { atomicMax(status, 1); }
 __global__ void prefix_screen(int m, int n, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                               const double* __restrict__ val, const double* __restrict__ AL,
                               const double* __restrict__ AU, int32_t* __restrict__ out) {
+  after_previous_kernel();
   if (blockIdx.x || threadIdx.x) return;
   PairRow r[4];
   for (int i = 0; i < 4; ++i) r[i] = i < m ? pair_row(i, ptr, idx, val, AL, AU) : PairRow{-1, -1, 0, 0, 0, 0, 0u};
@@ -213,12 +215,14 @@ __device__ void split_row(int lane, offset_t lo, offset_t hi, const int32_t* __r
 // Are the rows strictly ascending?  (_kernel_structural_check_csr_sorted)
 __global__ void rows_ascending(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                                int32_t* __restrict__ bad) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     for (offset_t p = ptr[i] + 1; p < ptr[i + 1]; ++p)
       if (idx[p - 1] >= idx[p]) { atomicMax(bad, 1); break; }
 }
 __global__ void row_sort_keys(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                               uint64_t* __restrict__ keys, int32_t* __restrict__ pos) {
+  after_previous_kernel();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   for (int i = warp; i < m; i += (gridDim.x * blockDim.x) >> 5)
     for (offset_t p = ptr[i] + lane; p < ptr[i + 1]; p += 32) {
@@ -229,6 +233,7 @@ __global__ void row_sort_keys(int m, const offset_t* __restrict__ ptr, const int
 __global__ void row_sort_gather(offset_t nnz, const uint64_t* __restrict__ keys, const int32_t* __restrict__ pos,
                                 const double* __restrict__ val, int32_t* __restrict__ oidx,
                                 double* __restrict__ oval) {
+  after_previous_kernel();
   for (offset_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += gridDim.x * blockDim.x) {
     oidx[q] = int32_t(uint32_t(keys[q] & 0xffffffffu));
     oval[q] = val[pos[q]];
@@ -257,10 +262,12 @@ bool sort_rows_unique(DevCsr& M, Status& st, cudaStream_t s) {
 }
 
 __global__ void fill_i32(int32_t* p, int64_t n, int32_t v) {
+  after_previous_kernel();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     p[i] = v;
 }
 __global__ void fill_f64(double* p, int64_t n, double v) {
+  after_previous_kernel();
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     p[i] = v;
 }
@@ -270,6 +277,7 @@ __global__ void fill_f64(double* p, int64_t n, double v) {
 // Every t and e column has one owner (_kernel_..._split_claim_roles, :442-468).
 __global__ void claim_roles(int blocks, int n, const int32_t* __restrict__ t_cols, const int32_t* __restrict__ e_cols,
                             int32_t* __restrict__ owner, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const int32_t t = t_cols[b], e = e_cols[b];
@@ -283,6 +291,7 @@ __global__ void claim_roles(int blocks, int n, const int32_t* __restrict__ t_col
 
 __global__ void split_extract(int blocks, const PairRow* __restrict__ rows, int32_t* __restrict__ t_cols,
                               int32_t* __restrict__ e_cols, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const PairRow& eq = rows[3 * b];
     const PairRow r1 = rows[3 * b + 1], r2 = rows[3 * b + 2];
@@ -312,6 +321,7 @@ struct SplitArgs {
 
 // _kernel_..._split_validate_blocks (:470-617).
 __global__ void split_validate(int blocks, SplitArgs g, uint8_t* __restrict__ preserve, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     preserve[b] = 0;
@@ -367,6 +377,7 @@ __global__ void split_validate(int blocks, SplitArgs g, uint8_t* __restrict__ pr
 
 __global__ void split_counts(int m, const offset_t* __restrict__ ptr, const uint8_t* __restrict__ preserve,
                              int32_t* __restrict__ counts) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     const int k = i % 3;
     counts[i] = k == 0 ? ptr[i + 1] - ptr[i] + 1 : (k == 1 && preserve[i / 3] ? 2 : 0);
@@ -378,6 +389,7 @@ __global__ void split_fill(int m, const offset_t* __restrict__ ptr, const int32_
                            const int32_t* __restrict__ e_cols, const uint8_t* __restrict__ preserve,
                            const offset_t* __restrict__ optr, int32_t* __restrict__ oidx,
                            double* __restrict__ oval) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += (gridDim.x * blockDim.x) >> 5) {
     const int b = i / 3, k = i % 3;
@@ -400,6 +412,7 @@ __global__ void split_fill(int m, const offset_t* __restrict__ ptr, const int32_
 __global__ void split_apply(int blocks, const int32_t* __restrict__ t_cols, const int32_t* __restrict__ e_cols,
                             const uint8_t* __restrict__ preserve, uint8_t* __restrict__ keep_row, double* c,
                             double* l, double* u, double* AL, double* AU) {
+  after_previous_kernel();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const int32_t t = t_cols[b], e = e_cols[b];
     const int r1 = 3 * b + 1, r2 = r1 + 1;
@@ -437,6 +450,7 @@ struct GraphArgs {
 // _kernel_structural_graph_extract_blocks (:756-889).
 __global__ void graph_extract(int blocks, GraphArgs g, int32_t* __restrict__ t_cols, int32_t* __restrict__ e_cols,
                               double* __restrict__ rhos, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const int eq = 4 * b;
     const PairRow r1 = g.rows[eq + 1], r2 = g.rows[eq + 2], r3 = g.rows[eq + 3];
@@ -492,6 +506,7 @@ __global__ void graph_mark_rows(int blocks, GraphArgs g, const int32_t* __restri
                                 int32_t* __restrict__ row_block, int32_t* __restrict__ row_slack,
                                 double* __restrict__ row_factor, int32_t* __restrict__ owner,
                                 int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const int32_t t = t_cols[b];
@@ -531,6 +546,7 @@ __global__ void graph_mark_rows(int blocks, GraphArgs g, const int32_t* __restri
 __global__ void graph_aux_rows(GraphArgs g, const int32_t* __restrict__ owner, const int32_t* __restrict__ row_block,
                                const int32_t* __restrict__ row_slack, uint8_t* __restrict__ removable,
                                int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < g.n; j += gridDim.x * blockDim.x) {
     if (owner[j] != kAuxRole) continue;
@@ -549,6 +565,7 @@ __global__ void graph_aux_rows(GraphArgs g, const int32_t* __restrict__ owner, c
 __global__ void graph_required_rows(int blocks, int n, const int32_t* __restrict__ row_block,
                                     const int32_t* __restrict__ row_slack, const double* __restrict__ row_factor,
                                     const uint8_t* __restrict__ removable, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const int r = 4 * b + 3;
@@ -559,6 +576,7 @@ __global__ void graph_required_rows(int blocks, int n, const int32_t* __restrict
 }
 
 __global__ void graph_counts(int m, const offset_t* __restrict__ ptr, int32_t* __restrict__ counts) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     counts[i] = i % 4 == 0 ? ptr[i + 1] - ptr[i] + 1 : 0;
 }
@@ -566,6 +584,7 @@ __global__ void graph_fill(int m, const offset_t* __restrict__ ptr, const int32_
                            const double* __restrict__ val, const int32_t* __restrict__ t_cols,
                            const int32_t* __restrict__ e_cols, const double* __restrict__ rhos,
                            const offset_t* __restrict__ optr, int32_t* __restrict__ oidx, double* __restrict__ oval) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += (gridDim.x * blockDim.x) >> 5) {
     if (i % 4) continue;
@@ -579,6 +598,7 @@ __global__ void graph_apply(int blocks, GraphArgs g, const int32_t* __restrict__
                             const int32_t* __restrict__ e_cols, const double* __restrict__ rhos,
                             const uint8_t* __restrict__ removable, uint8_t* __restrict__ keep_row, double* c, double* l,
                             double* u, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += gridDim.x * blockDim.x) {
     const int r1 = 4 * b + 1, r2 = r1 + 1;
     const int32_t t = t_cols[b], e = e_cols[b];
@@ -603,6 +623,7 @@ __global__ void graph_apply(int blocks, GraphArgs g, const int32_t* __restrict__
   }
 }
 __global__ void drop_aux(int n, const int32_t* __restrict__ owner, uint8_t* __restrict__ keep_col) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
     if (owner[j] == kAuxRole) keep_col[j] = 0;
 }
@@ -612,17 +633,20 @@ __global__ void drop_aux(int n, const int32_t* __restrict__ owner, uint8_t* __re
 // device_recovery.cu:698-748).
 __global__ void slack_first_row(int m, const int32_t* __restrict__ row_block, const int32_t* __restrict__ row_slack,
                                 const uint8_t* __restrict__ removable, int32_t* __restrict__ first) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x)
     if (removable[r] && row_block[r] >= 0 && row_slack[r] >= 0) atomicMin(first + row_slack[r], r);
 }
 __global__ void slack_flags(int m, const int32_t* __restrict__ row_block, const int32_t* __restrict__ row_slack,
                             const uint8_t* __restrict__ removable, int32_t* __restrict__ flag) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x)
     flag[r] = removable[r] && row_block[r] >= 0 && row_slack[r] >= 0 ? 1 : 0;
 }
 __global__ void slack_keys(int m, const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
                            const int32_t* __restrict__ row_slack, const int32_t* __restrict__ first,
                            uint64_t* __restrict__ keys, int32_t* __restrict__ rows) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x)
     if (flag[r]) {
       keys[pos[r]] = (uint64_t(uint32_t(first[row_slack[r]])) << 32) | uint32_t(r);
@@ -630,6 +654,7 @@ __global__ void slack_keys(int m, const int32_t* __restrict__ flag, const int32_
     }
 }
 __global__ void slack_heads(int k, const uint64_t* __restrict__ keys, int32_t* __restrict__ head) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x)
     head[q] = q == 0 || (keys[q] >> 32) != (keys[q - 1] >> 32) ? 1 : 0;
 }
@@ -639,6 +664,7 @@ __global__ void slack_pack(int k, const uint64_t* __restrict__ keys, const int32
                            const int32_t* __restrict__ row_slack, const double* __restrict__ row_factor,
                            int32_t* __restrict__ slack, int32_t* __restrict__ start, int32_t* __restrict__ t_out,
                            double* __restrict__ f_out) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < k; q += gridDim.x * blockDim.x) {
     const int r = rows[q];
     if (head[q]) {
@@ -656,6 +682,7 @@ __global__ void slack_pack(int k, const uint64_t* __restrict__ keys, const int32
 // Leading run of valid 3-row pair groups (_kernel_structural_outer_count_pairs):
 // the first invalid group index, by atomicMin.
 __global__ void outer_first_bad(int groups, const PairRow* __restrict__ rows, int32_t* __restrict__ first_bad) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < groups; q += gridDim.x * blockDim.x) {
     const PairRow a = rows[3 * q], b = rows[3 * q + 1], c = rows[3 * q + 2];
     if (!(zero_sided(a) && zero_sided(b) && zero_sided(c) && outer_signature(a, b, c))) atomicMin(first_bad, q);
@@ -674,6 +701,7 @@ struct OuterArgs {
 // (_kernel_structural_outer_validate_pairs_and_build_free_to_bound, first loop).
 __global__ void outer_pairs_check(OuterArgs g, int32_t* __restrict__ free_to_bound, uint64_t* __restrict__ keys,
                                   int32_t* __restrict__ vals, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.pairs; i += gridDim.x * blockDim.x) {
     const PairRow& r = g.rows[3 * i];
     const int32_t b = r.c1, f = r.c2;
@@ -694,6 +722,7 @@ __global__ void outer_pairs_check(OuterArgs g, int32_t* __restrict__ free_to_bou
 // sum finite.
 __global__ void outer_pair_costs(OuterArgs g, const uint64_t* __restrict__ keys, const int32_t* __restrict__ vals,
                                  double* __restrict__ bound_cost, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < g.pairs; q += gridDim.x * blockDim.x) {
     const uint32_t b = uint32_t(keys[q] >> 32);
@@ -712,11 +741,13 @@ __global__ void outer_pair_costs(OuterArgs g, const uint64_t* __restrict__ keys,
 // No bounded column is also a free one; then mark the bounded role
 // (second loop of the same kernel).
 __global__ void outer_bound_check(OuterArgs g, const int32_t* __restrict__ free_to_bound, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.pairs; i += gridDim.x * blockDim.x)
     if (free_to_bound[g.rows[3 * i].c1] >= 0) fail(status);
 }
 __global__ void outer_bound_mark(OuterArgs g, int32_t* __restrict__ free_to_bound, const int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile const int32_t*)status) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.pairs; i += gridDim.x * blockDim.x)
     free_to_bound[g.rows[3 * i].c1] = kBoundRole;
@@ -731,6 +762,7 @@ __device__ __forceinline__ int32_t outer_map(const int32_t* free_to_bound, int32
 __global__ void outer_extract(OuterArgs g, const int32_t* __restrict__ free_to_bound, int32_t* __restrict__ q_cols,
                               int32_t* __restrict__ e_cols, int32_t* __restrict__ s_cols, double* __restrict__ alphas,
                               int32_t* __restrict__ x_cols, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < g.blocks; b += gridDim.x * blockDim.x) {
     const int dense = g.start_row + 8 * b;
@@ -793,6 +825,7 @@ __global__ void outer_extract(OuterArgs g, const int32_t* __restrict__ free_to_b
 __global__ void outer_roles(OuterArgs g, const int32_t* __restrict__ q_cols, const int32_t* __restrict__ e_cols,
                             const int32_t* __restrict__ s_cols, int32_t* __restrict__ free_to_bound,
                             int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * g.blocks; k += gridDim.x * blockDim.x) {
     const int b = k / 3, which = k % 3;
@@ -804,6 +837,7 @@ __global__ void outer_roles(OuterArgs g, const int32_t* __restrict__ q_cols, con
 // No x column is another block's q, e or s (_kernel_structural_outer_validate_local_x_roles).
 __global__ void outer_x_roles(OuterArgs g, const int32_t* __restrict__ free_to_bound,
                               const int32_t* __restrict__ x_cols, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 4 * g.blocks; k += gridDim.x * blockDim.x) {
     const int32_t x = x_cols[k];
@@ -815,6 +849,7 @@ __global__ void outer_block_check(OuterArgs g, const int32_t* __restrict__ free_
                                   const int32_t* __restrict__ q_cols, const int32_t* __restrict__ e_cols,
                                   const int32_t* __restrict__ s_cols, const double* __restrict__ alphas,
                                   const int32_t* __restrict__ x_cols, int32_t* __restrict__ status) {
+  after_previous_kernel();
   if (*(volatile int32_t*)status) return;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < g.blocks; b += gridDim.x * blockDim.x) {
     const int32_t q = q_cols[b], e = e_cols[b], s = s_cols[b];
@@ -853,6 +888,7 @@ __global__ void outer_block_check(OuterArgs g, const int32_t* __restrict__ free_
 }
 
 __global__ void outer_counts(int m, int start_row, const offset_t* __restrict__ ptr, int32_t* __restrict__ counts) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     const int k = (i - start_row) % 8;
     counts[i] = i >= start_row && (k == 0 || k >= 4) ? ptr[i + 1] - ptr[i] + 1 : 0;
@@ -866,6 +902,7 @@ __global__ void outer_fill(int m, int start_row, const offset_t* __restrict__ pt
                            const int32_t* __restrict__ q_cols, const int32_t* __restrict__ e_cols,
                            const int32_t* __restrict__ s_cols, const double* __restrict__ alphas,
                            const offset_t* __restrict__ optr, int32_t* __restrict__ oidx, double* __restrict__ oval) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += (gridDim.x * blockDim.x) >> 5) {
     if (i < start_row) continue;
@@ -904,6 +941,7 @@ __global__ void outer_fill(int m, int start_row, const offset_t* __restrict__ pt
 // _kernel_structural_outer_pair_apply and _block_apply (:1437-1585).
 __global__ void outer_pair_apply(OuterArgs g, const double* __restrict__ bound_cost, uint8_t* __restrict__ keep_row,
                                  uint8_t* __restrict__ keep_col, double* __restrict__ c) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.pairs; i += gridDim.x * blockDim.x) {
     const PairRow& r = g.rows[3 * i];
     keep_row[3 * i] = 0;
@@ -917,6 +955,7 @@ __global__ void outer_block_apply(OuterArgs g, const int32_t* __restrict__ q_col
                                   const int32_t* __restrict__ s_cols, const double* __restrict__ alphas,
                                   uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col, double* c, double* l,
                                   double* u) {
+  after_previous_kernel();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < g.blocks; b += gridDim.x * blockDim.x) {
     const int dense = g.start_row + 8 * b;
     const int32_t q = q_cols[b], e = e_cols[b], s = s_cols[b];
@@ -936,6 +975,7 @@ __global__ void outer_block_apply(OuterArgs g, const int32_t* __restrict__ q_col
 }
 __global__ void outer_pair_ids(int pairs, const PairRow* __restrict__ rows, int32_t* __restrict__ bound,
                                int32_t* __restrict__ free_col) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
     bound[i] = rows[3 * i].c1;
     free_col[i] = rows[3 * i].c2;

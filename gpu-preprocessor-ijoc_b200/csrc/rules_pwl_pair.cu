@@ -76,6 +76,7 @@ __global__ void merge_row_probe(int rows, int P, int probes, const offset_t* __r
                                 const int32_t* __restrict__ idx, const double* __restrict__ val,
                                 const double* __restrict__ AL, const double* __restrict__ AU,
                                 int32_t* __restrict__ count) {
+  after_previous_kernel();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < probes; s += gridDim.x * blockDim.x) {
     const int row = int(int64_t(s) * rows / probes);
     const offset_t lo = ptr[row];
@@ -91,6 +92,7 @@ __global__ void epi_pair_probe(int P, int cols, int probes, const offset_t* __re
                                const double* __restrict__ val, const double* __restrict__ AL,
                                const double* __restrict__ AU, const double* __restrict__ c,
                                const double* __restrict__ l, const double* __restrict__ u, int32_t* __restrict__ failed) {
+  after_previous_kernel();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < probes; s += gridDim.x * blockDim.x) {
     const int pair = int(int64_t(s) * P / probes), mate = pair + P;
     const offset_t b = at_ptr[pair], mb = at_ptr[mate];
@@ -125,6 +127,7 @@ __global__ void anti_pair_probe(int P, int probes, const offset_t* __restrict__ 
                                 const int32_t* __restrict__ at_idx, const double* __restrict__ at_val,
                                 const double* __restrict__ c, const double* __restrict__ l,
                                 const double* __restrict__ u, int32_t* __restrict__ failed) {
+  after_previous_kernel();
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < probes; s += gridDim.x * blockDim.x) {
     const int col = int(int64_t(s) * P / probes), mate = col + P;
     const offset_t b = at_ptr[col], e = at_ptr[col + 1], mb = at_ptr[mate];
@@ -142,6 +145,7 @@ __global__ void anti_pair_probe(int P, int probes, const offset_t* __restrict__ 
 // ---- union-find over the merge edges (roots are the smallest pair) -----------------------
 
 __global__ void uf_init(int P, int32_t* __restrict__ parent) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) parent[i] = i;
 }
 __device__ int32_t uf_find(int32_t* parent, int32_t v) {
@@ -160,6 +164,7 @@ __device__ int32_t uf_find(int32_t* parent, int32_t v) {
 // Links point from a larger root to a smaller one, so the forest stays
 // acyclic and every retry makes progress.
 __global__ void uf_union(int rows, const unsigned long long* __restrict__ edge, int32_t* parent) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
     const unsigned long long e = edge[r];
     if (e == kNoEdge) continue;
@@ -175,6 +180,7 @@ __global__ void uf_union(int rows, const unsigned long long* __restrict__ edge, 
 // Every pair points at its root; roots[0] counts the roots (one atomic per
 // warp).
 __global__ void uf_flatten(int P, int32_t* parent, int32_t* __restrict__ roots) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   for (int base = blockIdx.x * blockDim.x; base < P; base += stride) {
     const int i = base + threadIdx.x;
@@ -189,6 +195,7 @@ __global__ void uf_flatten(int P, int32_t* parent, int32_t* __restrict__ roots) 
   }
 }
 __global__ void fill_minus_one(int32_t* p, int n) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = -1;
 }
 
@@ -196,6 +203,7 @@ __global__ void fill_minus_one(int32_t* p, int n) {
 // size, the min of two per-pair values, and the sum of a third.
 __global__ void component_keys(int P, const int32_t* __restrict__ parent, uint64_t* __restrict__ keys,
                                int32_t* __restrict__ vals) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
     keys[i] = (uint64_t(uint32_t(parent[i])) << 32) | uint32_t(i);
     vals[i] = i;
@@ -287,6 +295,7 @@ struct EpiArgs {
 // bounds, positive-cost tail columns.
 __global__ void epi_columns(EpiArgs g, double* __restrict__ shift, double* __restrict__ lower_sum,
                             int32_t* __restrict__ status) {
+  after_previous_kernel();
   const int top = max(g.P, g.cols - 2 * g.P);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < top; i += gridDim.x * blockDim.x) {
     if (i < g.P) {
@@ -315,6 +324,7 @@ __global__ void epi_classify(EpiArgs g, const double* __restrict__ shift, unsign
                              int32_t* __restrict__ g_pair_by_row, int32_t* __restrict__ pair_g_row,
                              int32_t* __restrict__ pair_tail, double* __restrict__ pair_gcoef,
                              int32_t* __restrict__ counts, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < g.rows; row += gridDim.x * blockDim.x) {
     const offset_t lo = g.ptr[row], len = g.ptr[row + 1] - lo;
     const double al = g.AL[row], au = g.AU[row];
@@ -360,6 +370,7 @@ __global__ void epi_classify(EpiArgs g, const double* __restrict__ shift, unsign
 __global__ void epi_aggregate(int P, const uint64_t* __restrict__ keys, const int32_t* __restrict__ vals,
                               const double* __restrict__ u, int32_t* __restrict__ size, double* __restrict__ plus_up,
                               double* __restrict__ minus_up) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P; q += gridDim.x * blockDim.x) {
     const uint32_t r = uint32_t(keys[q] >> 32);
     if (q > 0 && uint32_t(keys[q - 1] >> 32) == r) continue;
@@ -384,6 +395,7 @@ __global__ void epi_validate(EpiArgs g, const int32_t* __restrict__ parent, cons
                              const double* __restrict__ shift, const double* __restrict__ lower_sum,
                              const double* __restrict__ plus_up, const double* __restrict__ minus_up,
                              int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int pair = blockIdx.x * blockDim.x + threadIdx.x; pair < g.P; pair += gridDim.x * blockDim.x) {
     const int32_t root = parent[pair];
     const int32_t row = pair_g_row[pair];
@@ -411,6 +423,7 @@ __global__ void epi_rows(EpiArgs g, const int32_t* __restrict__ parent, const in
                          const double* __restrict__ shift, const unsigned long long* __restrict__ edge,
                          const int32_t* __restrict__ g_pair_by_row, double feas_tol, RowOut out,
                          int32_t* __restrict__ removed, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < g.rows; row += gridDim.x * blockDim.x) {
     const int32_t pair = g_pair_by_row[row];
     const double al = g.AL[row], au = g.AU[row];
@@ -494,6 +507,7 @@ __global__ void epi_fill(EpiArgs g, const int32_t* __restrict__ parent, const in
                          const double* __restrict__ shift, const int32_t* __restrict__ pair_tail,
                          const unsigned long long* __restrict__ edge, const int32_t* __restrict__ g_pair_by_row,
                          const offset_t* __restrict__ optr, int32_t* __restrict__ oidx, double* __restrict__ oval) {
+  after_previous_kernel();
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < g.rows; row += gridDim.x * blockDim.x) {
     const offset_t w0 = optr[row];
     if (w0 == optr[row + 1]) continue;
@@ -529,6 +543,7 @@ __global__ void epi_fill(EpiArgs g, const int32_t* __restrict__ parent, const in
 __global__ void epi_columns_apply(int P, const int32_t* __restrict__ parent, const double* __restrict__ plus_up,
                                   const double* __restrict__ minus_up, uint8_t* __restrict__ keep_col,
                                   double* __restrict__ c, double* __restrict__ l, double* __restrict__ u) {
+  after_previous_kernel();
   for (int pair = blockIdx.x * blockDim.x + threadIdx.x; pair < P; pair += gridDim.x * blockDim.x) {
     const bool root = parent[pair] == pair;
     keep_col[pair] = root && plus_up[pair] > l[pair] ? 1 : 0;
@@ -549,6 +564,7 @@ __global__ void epi_columns_apply(int P, const int32_t* __restrict__ parent, con
 __global__ void anti_columns(int P, const double* __restrict__ c, const double* __restrict__ l,
                              const double* __restrict__ u, double* __restrict__ shift, double* __restrict__ constant,
                              int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
     const int mate = i + P;
     const double rho = c[i], lp = l[i], ln = l[mate];
@@ -568,6 +584,7 @@ __global__ void anti_classify(const offset_t* __restrict__ ptr, const int32_t* _
                               const double* __restrict__ AU, const double* __restrict__ shift, int rows, int P,
                               int max_terms, unsigned long long* __restrict__ edge, int32_t* __restrict__ counts,
                               int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
     const offset_t lo = ptr[row], len = ptr[row + 1] - lo;
     const double al = AL[row], au = AU[row];
@@ -596,6 +613,7 @@ __global__ void anti_aggregate(int P, const uint64_t* __restrict__ keys, const i
                                const double* __restrict__ c, const double* __restrict__ l,
                                const double* __restrict__ u, double* __restrict__ plus_cap,
                                double* __restrict__ minus_cap, double* __restrict__ rho, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P; q += gridDim.x * blockDim.x) {
     const uint32_t r = uint32_t(keys[q] >> 32);
     if (q > 0 && uint32_t(keys[q - 1] >> 32) == r) continue;
@@ -616,6 +634,7 @@ __global__ void anti_aggregate(int P, const uint64_t* __restrict__ keys, const i
 // Every merge edge ended inside one component (_kernel_verify_...).
 __global__ void anti_verify(int rows, const unsigned long long* __restrict__ edge, const int32_t* __restrict__ parent,
                             const double* __restrict__ shift, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
     const unsigned long long e = edge[r];
     if (e == kNoEdge) continue;
@@ -631,6 +650,7 @@ __global__ void anti_rows(const offset_t* __restrict__ ptr, const int32_t* __res
                           int rows, const int32_t* __restrict__ parent, const double* __restrict__ shift,
                           const unsigned long long* __restrict__ edge, double feas_tol, RowOut out,
                           int32_t* __restrict__ removed, int32_t* __restrict__ status) {
+  after_previous_kernel();
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
     const double al = AL[row], au = AU[row];
     out.AL[row] = al;
@@ -677,6 +697,7 @@ __global__ void anti_fill(const offset_t* __restrict__ ptr, const int32_t* __res
                           const double* __restrict__ val, int rows, int P, const int32_t* __restrict__ parent,
                           const double* __restrict__ shift, const offset_t* __restrict__ optr,
                           int32_t* __restrict__ oidx, double* __restrict__ oval) {
+  after_previous_kernel();
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
     const offset_t w0 = optr[row];
     if (w0 == optr[row + 1]) continue;
@@ -698,6 +719,7 @@ __global__ void anti_columns_apply(int P, const int32_t* __restrict__ parent, co
                                    const double* __restrict__ minus_cap, const double* __restrict__ rho,
                                    uint8_t* __restrict__ keep_col, double* __restrict__ c, double* __restrict__ l,
                                    double* __restrict__ u) {
+  after_previous_kernel();
   for (int pair = blockIdx.x * blockDim.x + threadIdx.x; pair < P; pair += gridDim.x * blockDim.x) {
     const bool root = parent[pair] == pair;
     keep_col[pair] = root ? 1 : 0;
@@ -718,6 +740,7 @@ __global__ void anti_columns_apply(int P, const int32_t* __restrict__ parent, co
 __global__ void commit_rows(int rows, const uint8_t* __restrict__ keep, const double* __restrict__ al,
                             const double* __restrict__ au, uint8_t* __restrict__ keep_row, double* __restrict__ AL,
                             double* __restrict__ AU) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
     keep_row[r] = keep[r];
     AL[r] = al[r];
@@ -730,6 +753,7 @@ __global__ void pair_recovery(int P, const int32_t* __restrict__ parent, const d
                               int32_t* __restrict__ plus, int32_t* __restrict__ minus, int32_t* __restrict__ root_plus,
                               int32_t* __restrict__ root_minus, double* __restrict__ plus_shift,
                               double* __restrict__ minus_shift) {
+  after_previous_kernel();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
     plus[i] = i;
     minus[i] = i + P;

@@ -62,6 +62,7 @@ __global__ void sc_candidates(int n, int m, const uint8_t* __restrict__ keep_col
                               const double* __restrict__ AL, const double* __restrict__ AU, double zero_tol,
                               int32_t* __restrict__ owner, int32_t* __restrict__ cand, int32_t* __restrict__ rows,
                               int32_t* __restrict__ long_rows, int32_t* st) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;   // every thread of a block runs the same trips
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += stride) {
@@ -284,6 +285,7 @@ sc_cache(int row_blocks, const int32_t* __restrict__ rows, const int32_t* __rest
          const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
          const int32_t* __restrict__ idx, const double* __restrict__ val, const uint8_t* __restrict__ keep_col,
          const double* __restrict__ l, const double* __restrict__ u, CacheOut out) {
+  after_previous_kernel();
   if (int(blockIdx.x) < row_blocks)
     sc_cache_rows(row_blocks, rows, st, row_nnz, ptr, idx, val, keep_col, l, u, out);
   else
@@ -300,6 +302,7 @@ __global__ void sc_propose(const int32_t* __restrict__ cand, const int32_t* __re
                            const int4* __restrict__ counts, const uint8_t* __restrict__ invalid, double tol,
                            double zero_tol, uint8_t* __restrict__ action, double* __restrict__ side,
                            int32_t* __restrict__ owner) {
+  after_previous_kernel();
   const int count = st[kStCand];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
     const int j = cand[q];
@@ -378,6 +381,7 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
                          uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ kind,
                          int32_t* __restrict__ winners, int64_t* __restrict__ contrib_idx,
                          double* __restrict__ contrib_val, Report report) {
+  after_previous_kernel();
   // An unbounded candidate ends the rule with the plan as it was.
   const int count = st[kStUnbounded] ? 0 : st[kStRows];
   const int stride = gridDim.x * blockDim.x;
@@ -449,6 +453,7 @@ __global__ void sc_touch(const int32_t* __restrict__ winners, const int32_t* __r
                          const uint8_t* __restrict__ kind, const offset_t* __restrict__ ptr,
                          const int32_t* __restrict__ idx, const uint8_t* __restrict__ keep_col,
                          uint32_t* __restrict__ claimed, int32_t* __restrict__ touched, int32_t* st_w) {
+  after_previous_kernel();
   const int count = st[kStWin];
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
@@ -480,6 +485,7 @@ __global__ void sc_cost(const int32_t* __restrict__ touched, const int32_t* __re
                         const offset_t* __restrict__ tptr, const int32_t* __restrict__ tidx,
                         const double* __restrict__ tval, const int32_t* __restrict__ owner,
                         const double* __restrict__ sval, double* __restrict__ c) {
+  after_previous_kernel();
   const int count = st[kStTouched];
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
@@ -513,6 +519,7 @@ __global__ void sc_sub_sizes(const int32_t* __restrict__ sorted_rows, int count,
                              const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                              const double* __restrict__ val, const uint8_t* __restrict__ keep_col, double zero_tol,
                              int32_t* __restrict__ sel, int64_t* __restrict__ support) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < count; w += warps) {
@@ -550,6 +557,7 @@ __global__ void sc_sub_pack(const int32_t* __restrict__ sorted_rows, int count, 
                             const double* __restrict__ l, const double* __restrict__ u, int32_t* __restrict__ types,
                             int64_t* __restrict__ is, int64_t* __restrict__ vs, int32_t* __restrict__ oidx,
                             double* __restrict__ oval) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < count; w += warps) {
@@ -600,6 +608,7 @@ __global__ void sc_sub_pack(const int32_t* __restrict__ sorted_rows, int count, 
 __global__ void sc_shift_pack(const int32_t* __restrict__ sorted_rows, int count, int32_t* __restrict__ types,
                               int64_t* __restrict__ is, int64_t* __restrict__ vs, int32_t* __restrict__ oidx,
                               double* __restrict__ oval) {
+  after_previous_kernel();
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < count; r += gridDim.x * blockDim.x) {
     if (r == 0) { is[0] = 0; vs[0] = 0; }
     types[r] = 10;  // RowDualShift
@@ -612,6 +621,7 @@ __global__ void sc_shift_pack(const int32_t* __restrict__ sorted_rows, int count
 
 // Unclaimed owners and zeroed status words.
 __global__ void sc_start(int32_t* p, int n, int32_t v, int32_t* __restrict__ st) {
+  after_previous_kernel();
   if (blockIdx.x == 0 && threadIdx.x < kStWords) st[threadIdx.x] = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
 }
@@ -619,12 +629,14 @@ __global__ void sc_start(int32_t* p, int n, int32_t v, int32_t* __restrict__ st)
 // The objective contributions as a dense vector for the canonical sum.
 __global__ void sc_scatter_contrib(int count, const int64_t* __restrict__ idx, const double* __restrict__ val,
                                    double* __restrict__ dense) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) dense[idx[q]] = val[q];
 }
 
 // Sort key: substitution rows first, then dual-shift rows, each ascending.
 __global__ void sc_winner_keys(const int32_t* __restrict__ winners, int count, const uint8_t* __restrict__ kind,
                                uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+  after_previous_kernel();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
     const int row = winners[q];
     keys[q] = (uint64_t(kind[row] == kRowDualShift ? 1 : 0) << 32) | uint32_t(row);

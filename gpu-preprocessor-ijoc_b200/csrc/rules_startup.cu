@@ -41,6 +41,7 @@ enum : int32_t { kBadRow = 1, kBadColumn = 2, kBadValue = 4, kNoWitness = 8 };
 __global__ void cd_validate_sides(int m, int n, const double* __restrict__ c, const double* __restrict__ AL,
                                   const double* __restrict__ AU, const double* __restrict__ l,
                                   const double* __restrict__ u, int32_t* __restrict__ failure) {
+  after_previous_kernel();
   int32_t bad = 0;
   const int stride = gridDim.x * blockDim.x;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
@@ -57,6 +58,7 @@ __global__ void cd_validate_entries(int m, offset_t nnz, const offset_t* __restr
                                     const int32_t* __restrict__ idx, const double* __restrict__ a,
                                     const double* __restrict__ at, const double* __restrict__ c,
                                     int32_t* __restrict__ failure) {
+  after_previous_kernel();
   int32_t bad = 0;
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < nnz; t += stride)
@@ -73,6 +75,7 @@ __global__ void cd_validate_entries(int m, offset_t nnz, const offset_t* __restr
 // Cost above degree: dominated.  Counted per block, one atomic per block.
 __global__ void cd_mark(int n, const offset_t* __restrict__ at_ptr, const double* __restrict__ c,
                         uint8_t* __restrict__ dominated, int32_t* __restrict__ count) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += stride) {
@@ -87,6 +90,7 @@ __global__ void cd_mark(int n, const offset_t* __restrict__ at_ptr, const double
 
 __global__ void cd_apply(int n, const uint8_t* __restrict__ dominated, uint8_t* __restrict__ keep_col,
                          double* __restrict__ l, double* __restrict__ u) {
+  after_previous_kernel();
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
     if (dominated[j]) {
       keep_col[j] = 0;
@@ -230,6 +234,7 @@ struct ProjectionInput {
 __global__ void tr_detect(int n, ProjectionInput in, int max_row_nnz, double zero_tol, double safety_tol,
                           uint8_t* __restrict__ candidate, int32_t* __restrict__ incident,
                           int32_t* __restrict__ live_count) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < top; col += stride) {
@@ -307,6 +312,7 @@ __device__ McCormickRow mccormick_row(const ProjectionInput& in, int row, int z)
 __global__ void zc_detect(int n, ProjectionInput in, uint8_t* __restrict__ candidate, int32_t* __restrict__ end0,
                           int32_t* __restrict__ end1, int32_t* __restrict__ incident,
                           int32_t* __restrict__ live_count) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;
   for (int z = blockIdx.x * blockDim.x + threadIdx.x; z < top; z += stride) {
@@ -347,6 +353,7 @@ __global__ void zc_detect(int n, ProjectionInput in, uint8_t* __restrict__ candi
 template <int K>
 __global__ void count_candidate_rows(int n, const uint8_t* __restrict__ candidate, const int32_t* __restrict__ incident,
                                      int32_t* __restrict__ row_count) {
+  after_previous_kernel();
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n; col += gridDim.x * blockDim.x)
     if (candidate[col])
       for (int k = 0; k < K; ++k) atomicAdd(row_count + incident[size_t(col) * K + k], 1);
@@ -359,6 +366,7 @@ __global__ void select_candidates(int n, const uint8_t* __restrict__ candidate, 
                                   const int32_t* __restrict__ end1, const int32_t* __restrict__ incident,
                                   const int32_t* __restrict__ row_count, uint8_t* __restrict__ selected,
                                   int32_t* __restrict__ selected_count) {
+  after_previous_kernel();
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < top; col += stride) {
@@ -401,6 +409,7 @@ template <int K>
 __global__ void projection_sizes(int n, ProjectionInput in, const uint8_t* __restrict__ selected,
                                  const int32_t* __restrict__ incident, int64_t* __restrict__ records,
                                  int64_t* __restrict__ support, int32_t* __restrict__ failure) {
+  after_previous_kernel();
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n; col += gridDim.x * blockDim.x) {
     records[col] = selected[col] ? 1 : 0;
     int64_t len = 0;
@@ -427,6 +436,7 @@ __global__ void projection_pack(int n, ProjectionInput in, const uint8_t* __rest
                                 const int64_t* __restrict__ spos, int32_t* __restrict__ types,
                                 int64_t* __restrict__ is, int64_t* __restrict__ vs, int32_t* __restrict__ idx,
                                 double* __restrict__ val) {
+  after_previous_kernel();
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n; col += gridDim.x * blockDim.x) {
     if (!selected[col]) continue;
     const int64_t k = rpos[col], s0 = spos[col], len = spos[col + 1] - s0;
@@ -461,6 +471,7 @@ __global__ void projection_pack(int n, ProjectionInput in, const uint8_t* __rest
 template <int K>
 __global__ void projection_apply(int n, const uint8_t* __restrict__ selected, const int32_t* __restrict__ incident,
                                  uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col) {
+  after_previous_kernel();
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n; col += gridDim.x * blockDim.x)
     if (selected[col]) {
       keep_col[col] = 0;

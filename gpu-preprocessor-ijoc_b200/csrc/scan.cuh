@@ -105,6 +105,7 @@ template <class T, int K, class In, class Out, class Total>
 __global__ void __launch_bounds__(kThreads)
 scan_tiles(int64_t n, int64_t tiles, In in, Out out, Total total, unsigned long long* words, unsigned int* counters,
            int32_t* error) {
+  after_previous_kernel();
   __shared__ T warp_sums[K][kThreads / 32];
   __shared__ long long tile_before[K];
   __shared__ unsigned int ticket;
@@ -179,6 +180,7 @@ template <class Pred, class Emit>
 __global__ void __launch_bounds__(kThreads)
 select_tiles(int64_t n, int64_t tiles, Pred pred, Emit emit, int32_t* count, Mailbox* mail, uint32_t seq,
              unsigned long long* words, unsigned int* counters, int32_t* error) {
+  after_previous_kernel();
   __shared__ int warp_sums[kThreads / 32];
   __shared__ long long tile_before;
   __shared__ unsigned int ticket;

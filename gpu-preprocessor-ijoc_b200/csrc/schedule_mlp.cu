@@ -30,6 +30,7 @@ static_assert(kB3 + O == kScheduleParams, "parameter layout");
 // Y[r][j] = act(b[j] + sum_k X[r][k] W[k][j]); one thread per (r, j).
 __global__ void dense_forward(const float* __restrict__ X, int64_t rows, int K, const float* __restrict__ W,
                               const float* __restrict__ b, int N, int relu, float* __restrict__ Y) {
+  after_previous_kernel();
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= rows * N) return;
   const int64_t r = t / N;
@@ -43,6 +44,7 @@ __global__ void dense_forward(const float* __restrict__ X, int64_t rows, int K, 
 // the summed loss (numerically stable form).
 __global__ void bce_grad(const float* __restrict__ Z, const float* __restrict__ Y, const float* __restrict__ M,
                          int64_t count, float scale, float* __restrict__ dZ, float* __restrict__ loss) {
+  after_previous_kernel();
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   float l = 0.0f;
   if (t < count) {
@@ -59,6 +61,7 @@ __global__ void bce_grad(const float* __restrict__ Z, const float* __restrict__ 
 // output; one thread per (r, k).
 __global__ void dense_backward_input(const float* __restrict__ dY, int64_t rows, int N, const float* __restrict__ W,
                                      int K, const float* __restrict__ Xrelu, float* __restrict__ dX) {
+  after_previous_kernel();
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= rows * K) return;
   const int64_t r = t / K;
@@ -72,6 +75,7 @@ __global__ void dense_backward_input(const float* __restrict__ dY, int64_t rows,
 // rows in order (deterministic); one thread per parameter.
 __global__ void dense_backward_params(const float* __restrict__ X, const float* __restrict__ dY, int64_t rows, int K,
                                       int N, float* __restrict__ dW, float* __restrict__ db) {
+  after_previous_kernel();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < K * N) {
     const int k = t / N, j = t % N;
@@ -90,6 +94,7 @@ __global__ void dense_backward_params(const float* __restrict__ X, const float* 
 __global__ void adam_step(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
                           const float* __restrict__ g, int64_t count, float lr, float beta1, float beta2, float eps,
                           float c1, float c2) {
+  after_previous_kernel();
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const float gt = g[t];
@@ -102,12 +107,14 @@ __global__ void adam_step(float* __restrict__ w, float* __restrict__ m, float* _
 
 __global__ void gather_rows(const float* __restrict__ src, const int32_t* __restrict__ rows, int64_t count, int width,
                             float* __restrict__ dst) {
+  after_previous_kernel();
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= count * width) return;
   dst[t] = src[int64_t(rows[t / width]) * width + t % width];
 }
 
 __global__ void sigmoid_kernel(float* z, int64_t count) {
+  after_previous_kernel();
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t < count) z[t] = 1.0f / (1.0f + expf(-z[t]));
 }
@@ -116,6 +123,7 @@ __global__ void sigmoid_kernel(float* z, int64_t count) {
 // shared memory; out[o] = sigmoid(logit o).
 __global__ void __launch_bounds__(kScheduleHidden) forward_one(const float* __restrict__ params,
                                                                const float* __restrict__ x, float* __restrict__ out) {
+  after_previous_kernel();
   __shared__ float in[kScheduleFeatures], h1[kScheduleHidden], h2[kScheduleHidden];
   const int j = threadIdx.x;
   if (j < F) in[j] = x[j];

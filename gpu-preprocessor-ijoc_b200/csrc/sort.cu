@@ -106,6 +106,7 @@ size_t block_sort_smem(int n) {
 
 __global__ void __launch_bounds__(kBlockSortThreads)
 block_sort_pairs(uint64_t* keys, int32_t* vals, int n, uint64_t may_vary) {
+  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char block_sort_mem[];
   __shared__ int digit_start[kDigits];
   __shared__ int warp_sums[8];
@@ -204,6 +205,7 @@ struct SortPlan {
 
 __global__ void __launch_bounds__(kThreads)
 sort_histogram(const uint64_t* __restrict__ keys, int64_t n, SortPasses passes, SortPlan* plan) {
+  after_previous_kernel();
   __shared__ int h[kMaxPasses][kDigits];
   __shared__ bool last;
   __shared__ int warp_sums[8];
@@ -300,6 +302,7 @@ template <int kItems, class Word>
 __global__ void __launch_bounds__(kThreads)
 sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int64_t n, int pass, int shift,
           SortPlan* plan, Word* words, int32_t* error) {
+  after_previous_kernel();
   constexpr int kPairs = SortTile<kItems>::kPairs;
   using W = TileWord<Word>;
   extern __shared__ __align__(16) unsigned char sort_tile_mem[];
@@ -395,6 +398,7 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
 __global__ void sort_copy_back(int64_t n, int passes, const SortPlan* __restrict__ plan, uint64_t* __restrict__ keys,
                                int32_t* __restrict__ vals, const uint64_t* __restrict__ from_keys,
                                const int32_t* __restrict__ from_vals) {
+  after_previous_kernel();
   if (plan->source[passes] == 0) return;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     keys[i] = from_keys[i];

@@ -69,13 +69,18 @@ Report Context::open_report(int count, int32_t* words) {
   return Report{words, reinterpret_cast<unsigned int*>(report_words + 15), mail, ++mail_seq, count, true};
 }
 
-const volatile int64_t* Context::await(const Mailbox* box, uint32_t seq, const char* where) {
-  if (box->seq != seq) ++sync_counter();
+void Context::poll(const Mailbox* box, uint32_t seq, int words, const char* where) {
+  int k = 0;   // words seen
+  auto posted = [&] {
+    while (k < words && uint32_t(box->words[k] >> 32) == seq) ++k;
+    return k == words;
+  };
+  if (!posted()) ++sync_counter();
   const auto t0 = profiling() ? std::chrono::steady_clock::now() : std::chrono::steady_clock::time_point();
-  for (uint64_t polls = 1; box->seq != seq; ++polls) {
+  for (uint64_t polls = 1; !posted(); ++polls) {
     if (polls % 4096 == 0) {
       const cudaError_t e = cudaStreamQuery(stream);
-      if (e == cudaSuccess && box->seq != seq) throw CudaError(std::string(where) + ": the kernel posted no answer");
+      if (e == cudaSuccess && !posted()) throw CudaError(std::string(where) + ": the kernel posted no answer");
       if (e != cudaSuccess && e != cudaErrorNotReady) check(e, where);
     }
     if (polls > 4096 && polls % 64 == 0) std::this_thread::yield();
@@ -85,7 +90,6 @@ const volatile int64_t* Context::await(const Mailbox* box, uint32_t seq, const c
   if (profiling())
     profile_sync(where, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
   raise_device_error(where);
-  return box->words;
 }
 
 void Context::raise_device_error(const char* where) {
@@ -297,8 +301,10 @@ det_sum_kernel(const double* __restrict__ v, const uint8_t* __restrict__ mask, i
     const int c = first + int(threadIdx.x);
     sm[threadIdx.x] = c < int(gridDim.x) ? __ldcg(chunk_totals + c) : 0.0;
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (int k = 0; k < kThreads && first + k < int(gridDim.x); ++k) total += sm[k];
+    if (threadIdx.x == 0) {   // zeros past the last chunk change nothing
+#pragma unroll 16
+      for (int k = 0; k < kThreads; ++k) total += sm[k];
+    }
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -349,7 +355,7 @@ std::pair<int64_t, int64_t> exclusive_scan_pair_i64(const int64_t* a, int64_t* a
         post_values(mail, seq, sum[0], sum[1]);
       },
       s);
-  const volatile int64_t* t = c.await(mail, seq, where);
+  const int64_t* t = c.await(mail, seq, where);
   return {t[0], t[1]};
 }
 
@@ -360,7 +366,7 @@ double det_sum(const double* v, const uint8_t* mask, int64_t n, cudaStream_t s) 
   DBuf<double> part(size_t(chunks), s);
   const Report r = c.open_report(1);
   GPP_LAUNCH(det_sum_kernel, int(chunks), kThreads, 0, s, v, mask, n, part.p, r.done, r.mail, r.seq);
-  const int64_t bits = c.await(r)[0];
+  const int64_t bits = c.await(r.mail, r.seq, __func__)[0];
   double total;
   std::memcpy(&total, &bits, sizeof(total));
   return total;

@@ -240,15 +240,17 @@ __device__ __forceinline__ int block_append(int32_t* counter, bool take) {
 // Answers to the host.  Between two rules the host asks the device a question
 // (does the rule act, how many items were selected) and waits for the answer.
 // A kernel posts it itself: its last block to finish writes the words to a
-// page-locked mailbox, then the sequence number that the host polls for, and
-// leaves the device words zeroed for the next kernel.  That takes the place of
+// page-locked mailbox, each 32 bits beside the question's number that the host
+// polls for (so no fence stands between the answer and its number), and leaves
+// the device words zeroed for the next kernel.  That takes the place of
 // a memset before the kernel, a copy after it and a stream synchronisation
 // (about 25 us from the kernel's launch to the host's next, against 12).
 struct Mailbox {
-  volatile uint32_t seq;
-  uint32_t unused;
-  volatile int64_t words[15];
+  volatile uint64_t words[16];   // 32 bits of the answer below the question's number
 };
+__device__ __forceinline__ void post_word(Mailbox* mail, int k, uint32_t seq, uint32_t value) {
+  mail->words[k] = uint64_t(seq) << 32 | value;
+}
 struct Report {
   int32_t* words;        // device words that blocks OR or add into, zero at launch
   unsigned int* done;    // blocks finished, zero at launch
@@ -257,28 +259,29 @@ struct Report {
   int count;             // words to post
   bool keep;             // leave the words as they are (later kernels read them)
 };
-// Called once by every thread of every block, at the end of the kernel.
-__device__ __forceinline__ void post_report(const Report& r) {
-  __shared__ bool last_to_report;
+// Called once by every thread of every block, at the end of the kernel: true
+// in the last block to get here, which sees what the others wrote.
+__device__ __forceinline__ bool last_to_report(const Report& r) {
+  __shared__ bool last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    last_to_report = atomicAdd(r.done, 1u) == gridDim.x - 1;
+    last = atomicAdd(r.done, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!last_to_report) return;
+  if (!last) return false;
   __threadfence();
+  return true;
+}
+__device__ __forceinline__ void post_words(const Report& r) {
   if (int(threadIdx.x) < r.count) {
-    r.mail->words[threadIdx.x] = __ldcg(r.words + threadIdx.x);
+    post_word(r.mail, threadIdx.x, r.seq, uint32_t(__ldcg(r.words + threadIdx.x)));
     if (!r.keep) r.words[threadIdx.x] = 0;
-    __threadfence_system();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *r.done = 0;
-    __threadfence_system();
-    r.mail->seq = r.seq;
-  }
+  if (threadIdx.x == 0) *r.done = 0;
+}
+__device__ __forceinline__ void post_report(const Report& r) {
+  if (last_to_report(r)) post_words(r);
 }
 // ORs the flags of all threads into word 0, one atomic per block that has any
 // (a later kernel posts it).
@@ -299,10 +302,10 @@ __device__ __forceinline__ void post_flags(const Report& r, uint32_t flags) {
 // One thread's answer of up to two values, for kernels that know which thread
 // has it.
 __device__ __forceinline__ void post_values(Mailbox* mail, uint32_t seq, int64_t a, int64_t b = 0) {
-  mail->words[0] = a;
-  mail->words[1] = b;
-  __threadfence_system();
-  mail->seq = seq;
+  post_word(mail, 0, seq, uint32_t(a));
+  post_word(mail, 1, seq, uint32_t(uint64_t(a) >> 32));
+  post_word(mail, 2, seq, uint32_t(b));
+  post_word(mail, 3, seq, uint32_t(uint64_t(b) >> 32));
 }
 
 // ---------------------------------------------------------------------------
@@ -338,12 +341,21 @@ struct Context {
   Report open_report(int count);                       // words of this context
   Report open_report(int count, int32_t* words);       // the caller's words (zero at launch), kept
   uint32_t open_mail() { return ++mail_seq; }
-  // Polls until `box` holds `seq`; a stream that has finished or failed
-  // without it is an error.
-  const volatile int64_t* await(const Mailbox* box, uint32_t seq, const char* where);
-  const volatile int64_t* await(const Report& r, const char* where = __builtin_FUNCTION()) {
-    return await(r.mail, r.seq, where);
+  // Polls until `box` holds the answer to `seq`; a stream that has finished or
+  // failed without it is an error.  The answer stays until the next question's.
+  const int64_t* await(const Mailbox* box, uint32_t seq, const char* where) {   // of post_values
+    poll(box, seq, 4, where);
+    for (int k = 0; k < 2; ++k)
+      answer[k] = int64_t(box->words[2 * k + 1] << 32 | (box->words[2 * k] & 0xffffffffu));
+    return answer;
   }
+  const int64_t* await(const Report& r, const char* where = __builtin_FUNCTION()) {   // of post_report
+    poll(r.mail, r.seq, r.count, where);
+    for (int k = 0; k < r.count; ++k) answer[k] = int32_t(uint32_t(r.mail->words[k]));
+    return answer;
+  }
+  int64_t answer[16] = {};
+  void poll(const Mailbox* box, uint32_t seq, int words, const char* where);
   cudaStream_t side = nullptr;
   // Scratch blocks this context freed on its own stream, by size class,
   // ready to be handed out again without a driver call (pool_alloc/free), and

@@ -328,7 +328,7 @@ std::pair<int32_t, int32_t> build_old_to_new_pair(const uint8_t* keep_row, int32
         else col_map[i - m] = v[1] ? before[1] : -1;
       },
       [=] __device__(const int32_t(&sum)[2]) { post_values(mail, seq, sum[0], sum[1]); }, s);
-  const volatile int64_t* kept = c.await(mail, seq, "kept rows and columns");
+  const int64_t* kept = c.await(mail, seq, "kept rows and columns");
   return {int32_t(kept[0]), int32_t(kept[1])};
 }
 
@@ -401,7 +401,7 @@ void compact_sides(CompactSides& sides, DevCsr* const (&out)[2], cudaStream_t s)
                    c.host_error, report);
   const int64_t record = profile_last();
   GPP_LAUNCH(compact_row_pointers, rows_grid, kThreads, 0, s, sides);
-  const volatile int64_t* kept = c.await(report);
+  const int64_t* kept = c.await(report);
   for (int k = 0; k < 2; ++k)
     if (sides.side[k].tiles) {
       out[k]->nnz = offset_t(kept[k]);

@@ -873,7 +873,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
   GPP_LAUNCH(dt_apply, gs, kThreads, 0, s, sel, rows.p, keep_c.p, elim_c.p, keep_v.p, elim_v.p, p.bound_tol,
              plan.l.p, plan.u.p, plan.c.p, plan.AU.p, plan.keep_row.p, plan.keep_col.p, kind.p, alpha.p, beta.p,
              obj_term.p, rec_idx.p, rec_val.p, report);
-  const volatile int64_t* f = ctx().await(report);
+  const int64_t* f = ctx().await(report);
   if (f[0] & 1) { plan.has_infeasible = true; return; }
   if (!f[0]) return;
   const int subst = int(f[1]);

@@ -54,6 +54,7 @@ __device__ __forceinline__ long long scan_lookback(const unsigned long long* wor
       for (int polls = 1; (w >> 62) == 0; ++polls) {
         if (polls == kScanPolls) {
           *reinterpret_cast<volatile int32_t*>(error) = 1;
+          __threadfence_system();   // before any answer
           w = kScanAll;
           break;
         }

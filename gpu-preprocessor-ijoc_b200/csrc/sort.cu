@@ -364,6 +364,7 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
       for (int polls = 1; (w >> W::kShift) == 0; ++polls) {
         if (polls == kPolls) {
           *reinterpret_cast<volatile int32_t*>(error) = 1;
+          __threadfence_system();   // before any answer
           w = W::kAll;
           break;
         }

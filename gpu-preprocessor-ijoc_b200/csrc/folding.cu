@@ -25,6 +25,7 @@
 #include <cmath>
 
 #include "folding.hpp"
+#include "scan.cuh"
 #include "sort.hpp"
 
 namespace gpp {
@@ -71,29 +72,14 @@ __global__ void fd_pack(int n, const int32_t* __restrict__ ids, const double* __
     perm[i] = i;
   }
 }
-// kernel_mark_color_start (folding_kernels.cu:75-90).
-__global__ void fd_starts(int n, const uint64_t* __restrict__ keys, double tol, int32_t* __restrict__ start) {
-  after_previous_kernel();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (i == 0) { start[i] = 1; continue; }
-    const uint64_t a = keys[i - 1], b = keys[i];
-    const bool new_id = (a >> 32) != (b >> 32);
-    const bool new_sig = double(key_float(uint32_t(b))) > double(key_float(uint32_t(a))) + tol;
-    start[i] = new_id || new_sig ? 1 : 0;
-  }
-}
-// Also marks the members that have their colour to themselves.
-__global__ void fd_write(int n, const int32_t* __restrict__ perm, const int32_t* __restrict__ start,
-                         const int32_t* __restrict__ excl, int write_sig, uint64_t seed, int32_t* __restrict__ ids,
-                         double* __restrict__ sig_out, uint8_t* __restrict__ alone) {
-  after_previous_kernel();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int id = excl[i] + start[i];   // inclusive scan: colours are 1-based
-    const int member = perm[i];
-    ids[member] = id;
-    alone[member] = start[i] && (i + 1 == n || start[i + 1]);
-    if (write_sig) sig_out[member] = color_signature(seed, id);
-  }
+// Whether position i of the sorted (colour, signature) keys starts a colour
+// (kernel_mark_color_start, folding_kernels.cu:75-90).
+__device__ __forceinline__ int starts_color(const uint64_t* __restrict__ keys, int64_t i, double tol) {
+  if (i == 0) return 1;
+  const uint64_t a = keys[i - 1], b = keys[i];
+  const bool new_id = (a >> 32) != (b >> 32);
+  const bool new_sig = double(key_float(uint32_t(b))) > double(key_float(uint32_t(a))) + tol;
+  return new_id || new_sig ? 1 : 0;
 }
 __global__ void fd_signatures(int n, const int32_t* __restrict__ ids, uint64_t seed, double* __restrict__ sig) {
   after_previous_kernel();
@@ -198,16 +184,15 @@ fd_spmv_long(const int32_t* __restrict__ long_rows, const int32_t* __restrict__ 
 struct Side {
   int n = 0;
   int colors = 1;
-  DBuf<int32_t> ids, perm, start, excl;
+  DBuf<int32_t> ids, perm, count;
   DBuf<uint8_t> alone;
   DBuf<uint64_t> keys;
   DBuf<double> sig;
-  void alloc(int count, cudaStream_t s) {
-    n = count;
+  void alloc(int members, cudaStream_t s) {
+    n = members;
     ids.alloc(size_t(n), s);
     perm.alloc(size_t(n), s);
-    start.alloc(size_t(n) + 1, s);
-    excl.alloc(size_t(n) + 1, s);
+    count.alloc(1, s);
     keys.alloc(size_t(n), s);
     sig.alloc(size_t(n), s);
     alone.alloc(size_t(n), s);
@@ -215,20 +200,37 @@ struct Side {
   }
   // update_color_id (folding_kernels.cu:165-210): split colours by the float
   // value of `value`; optionally write each member's new colour signature.
-  void update(const double* value, double tol, bool write_sig, uint64_t seed, cudaStream_t s) {
-    const int g = grid_stride_blocks(n);
-    GPP_LAUNCH(fd_pack, g, kThreads, 0, s, n, ids.p, value, keys.p, perm.p);
+  // Once sorted, one scan over the keys numbers the colours and writes each
+  // member's id, its signature and whether it has the colour to itself.  The
+  // colour count stays on the device; with `other` the counts of both sides
+  // are posted to the host.
+  void update(const double* value, double tol, bool write_sig, uint64_t seed, cudaStream_t s,
+              const int32_t* other = nullptr, uint32_t seq = 0) {
+    GPP_LAUNCH(fd_pack, grid_stride_blocks(n), kThreads, 0, s, n, ids.p, value, keys.p, perm.p);
     radix_sort_pairs(keys.p, perm.p, n, s, (bits_up_to(n) << 32) | 0xffffffffu);
-    GPP_LAUNCH(fd_starts, g, kThreads, 0, s, n, keys.p, tol, start.p);
-    exclusive_scan_i32(start.p, excl.p, n, s);
-    GPP_LAUNCH(fd_write, g, kThreads, 0, s, n, perm.p, start.p, excl.p, int(write_sig), seed, ids.p, sig.p,
-               alone.p);
+    Mailbox* mail = ctx().mail;
+    const uint64_t* sorted = keys.p;
+    scan_items<int32_t, 1>(
+        n, [sorted, tol] __device__(int64_t i, int32_t(&v)[1]) { v[0] = starts_color(sorted, i, tol); },
+        [sorted, tol, top = n, members = perm.p, colors_of = ids.p, lone = alone.p, out_sig = write_sig ? sig.p : nullptr,
+         seed] __device__(int64_t i, const int32_t(&before)[1], const int32_t(&v)[1]) {
+          const int id = before[0] + v[0];   // inclusive: colours are 1-based
+          const int member = members[i];
+          colors_of[member] = id;
+          lone[member] = v[0] && (i + 1 == top || starts_color(sorted, i + 1, tol));
+          if (out_sig) out_sig[member] = color_signature(seed, id);
+        },
+        [total = count.p, other, mail, seq] __device__(const int32_t(&sum)[1]) {
+          *total = sum[0];
+          if (other) post_values(mail, seq, sum[0], *other);
+        },
+        s);
   }
   // One refinement step: split the colours by the signatures M x.  With every
   // member alone nothing can split, and only the colours' own signatures of
   // the round are needed.
   void refine(const gpp_csr& M, const double* x, double tol, uint64_t seed, DBuf<double>& value,
-              DBuf<int32_t>& long_rows, cudaStream_t s) {
+              DBuf<int32_t>& long_rows, cudaStream_t s, const int32_t* other = nullptr, uint32_t seq = 0) {
     if (colors == n) {
       GPP_LAUNCH(fd_signatures, grid_stride_blocks(n), kThreads, 0, s, n, ids.p, seed, sig.p);
       return;
@@ -238,9 +240,8 @@ struct Side {
     GPP_LAUNCH(fd_spmv, grid_stride_blocks(n), kThreads, 0, s, n, M.rowPtr, M.colVal, M.nzVal, x, alone.p, value.p,
                long_rows.p, long_count);
     GPP_LAUNCH(fd_spmv_long, kNumSMs, kThreads, 0, s, long_rows.p, long_count, M.rowPtr, M.colVal, M.nzVal, x, value.p);
-    update(value.p, tol, true, seed, s);
+    update(value.p, tol, true, seed, s, other, seq);
   }
-  int count() { return read_scalar(excl.p + n); }
 };
 
 bool too_little(const Side& r, const Side& c) {
@@ -253,9 +254,14 @@ bool refine(const gpp_lp& lp, double tol, Side& rows, Side& cols, cudaStream_t s
   rows.update(lp.AU, tol, false, 0, s);
   cols.update(lp.c, tol, false, 0, s);
   cols.update(lp.l, tol, false, 0, s);
-  cols.update(lp.u, tol, false, 0, s);
-  rows.colors = rows.count();
-  cols.colors = cols.count();
+  auto& c = ctx();
+  uint32_t seq = c.open_mail();
+  cols.update(lp.u, tol, false, 0, s, rows.count.p, seq);
+  {
+    const int64_t* counts = c.await(c.mail, seq, "colours");
+    cols.colors = int(counts[0]);
+    rows.colors = int(counts[1]);
+  }
   GPP_LAUNCH(fd_signatures, grid_stride_blocks(rows.n), kThreads, 0, s, rows.n, rows.ids.p, round_seed(0, 2),
              rows.sig.p);
   GPP_LAUNCH(fd_signatures, grid_stride_blocks(cols.n), kThreads, 0, s, cols.n, cols.ids.p, round_seed(0, 5),
@@ -267,10 +273,19 @@ bool refine(const gpp_lp& lp, double tol, Side& rows, Side& cols, cudaStream_t s
   const int max_round = std::max(1, rows.n + cols.n);
   for (int round = 1; round <= max_round; ++round) {
     const int prev_cols = cols.colors, prev_rows = rows.colors;
-    cols.refine(lp.AT, rows.sig.p, tol, round_seed(round, 1), value, long_rows, s);
-    rows.refine(lp.A, cols.sig.p, tol, round_seed(round, 2), value, long_rows, s);
-    rows.colors = rows.count();
-    cols.colors = cols.count();
+    // The side updated last posts both counts; a side whose members all stand
+    // alone has nothing left to count.
+    const bool rows_last = rows.colors < rows.n, cols_last = !rows_last && cols.colors < cols.n;
+    seq = c.open_mail();
+    cols.refine(lp.AT, rows.sig.p, tol, round_seed(round, 1), value, long_rows, s, cols_last ? rows.count.p : nullptr,
+                seq);
+    rows.refine(lp.A, cols.sig.p, tol, round_seed(round, 2), value, long_rows, s, rows_last ? cols.count.p : nullptr,
+                seq);
+    if (rows_last || cols_last) {
+      const int64_t* counts = c.await(c.mail, seq, "colours");
+      (rows_last ? rows : cols).colors = int(counts[0]);
+      (rows_last ? cols : rows).colors = int(counts[1]);
+    }
     if (too_little(rows, cols)) return false;
     if (!(rows.colors > prev_rows || cols.colors > prev_cols)) return true;
   }

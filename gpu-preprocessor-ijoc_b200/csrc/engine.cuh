@@ -134,6 +134,10 @@ struct Plan {
   // Column max |a| over the kept rows, as of the statistics' version.
   DBuf<double> col_max;
   uint64_t col_max_version = 0;
+  // What dual fixing asks of each row, left by a redundant-row test that acted
+  // on none (row_kinds_current until the next of the two rules).
+  DBuf<uint8_t> row_kinds;
+  bool row_kinds_current = false;
   // Singleton columns' row owners and status words, cleared by the Cleanup
   // probe on its way (sc_ready) or by the rule.
   DBuf<int32_t> sc_owner, sc_words;
@@ -220,9 +224,14 @@ void mirror_bounds(Plan& plan, int32_t n, cudaStream_t s);
 struct RedundantTest {
   const double *AL, *AU;
   double tol;
-  uint8_t* action;
+  uint8_t *action, *kinds;
   Report report;
 };
+// Row kinds: kept, with a finite lower and upper side.
+constexpr uint8_t kRowKept = 1, kRowLower = 2, kRowUpper = 4;
+__device__ __forceinline__ uint8_t row_kind(bool kept, double al, double au) {
+  return kept ? uint8_t(kRowKept | (isfinite(al) ? kRowLower : 0) | (isfinite(au) ? kRowUpper : 0)) : uint8_t(0);
+}
 void redundant_rows_test(const DevCsr& A, const double2* lu, const uint8_t* keep_row, const int32_t* live_deg,
                          const RedundantTest& test, cudaStream_t s, uint64_t degrees_version);
 void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStream_t s);

@@ -126,11 +126,21 @@ struct ActivityTerm {
 constexpr int kGroupRowMax = 32;
 
 // The test of one row from its plain sums (rule_infeasible_and_redundant_rows.cu:158-240).
-__device__ __forceinline__ uint32_t redundant_test(const RedundantTest& t, int row, bool tested, double lo, double hi) {
+// Its sides are loaded with the row's entries, ahead of the sums.
+struct RowSides {
+  double al, au;
+  bool kept, tested;
+  __device__ __forceinline__ RowSides(const RedundantTest& t, int row, const uint8_t* keep_row,
+                                      const int32_t* live_deg)
+      : al(t.AL[row]), au(t.AU[row]), kept(keep_row[row]), tested(kept && live_deg[row] > 1) {}
+  __device__ __forceinline__ RowSides() : al(0.0), au(0.0), kept(false), tested(false) {}
+};
+__device__ __forceinline__ uint32_t redundant_test(const RedundantTest& t, int row, const RowSides& sides, double lo,
+                                                   double hi) {
   uint32_t found = 0;
   uint8_t a = 0;
-  if (tested) {
-    const double al = t.AL[row], au = t.AU[row];
+  const double al = sides.al, au = sides.au;
+  if (sides.tested) {
     const bool lf = isfinite(al), uf = isfinite(au);
     if (!(lf && uf && fabs(au - al) <= t.tol)) {
       if ((lf && hi < al - t.tol) || (uf && lo > au + t.tol)) {
@@ -144,6 +154,7 @@ __device__ __forceinline__ uint32_t redundant_test(const RedundantTest& t, int r
     }
   }
   t.action[row] = a;
+  t.kinds[row] = row_kind(sides.kept, al, au);
   return found;
 }
 
@@ -169,9 +180,13 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
   const ActivityTerm<Plain> term{idx, val, lu, zero_tol, l2_hints()};
   const auto live_at = [&](offset_t p) { return !removed_column(term.bounds(p)); };
   uint32_t found = 0;
-  const auto finish = [&](int row, double lo, double hi, int ni, int pi) {
+  const auto sides_of = [&](int row) {
+    if constexpr (Plain) return RowSides(test, row, keep_row, live_deg);
+    else return 0;
+  };
+  const auto finish = [&](int row, const auto& sides, double lo, double hi, int ni, int pi) {
     if constexpr (Plain) {
-      found |= redundant_test(test, row, keep_row[row] && live_deg[row] > 1, lo, hi);
+      found |= redundant_test(test, row, sides, lo, hi);
     } else {
       min_fin[row] = lo; max_fin[row] = hi;
       if (min_inf) { min_inf[row] = ni; max_inf[row] = pi; }
@@ -192,6 +207,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
       last_next = i_next < m ? ptr[i_next + 1] : 0;
       len_next = i_next < m && live_deg ? live_deg[i_next] : int(last_next - first_next);
       if (len > kShortRow) continue;
+      const auto sides = sides_of(i);
       double lo = 0.0, hi = 0.0;
       int ni = 0, pi = 0;
       if (keep_row && !keep_row[i]) {
@@ -217,7 +233,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
           if (!removed_column(bnd)) term(p, bnd, lo, hi, ni, pi);
         }
       }
-      finish(i, lo, hi, ni, pi);
+      finish(i, sides, lo, hi, ni, pi);
     }
   } else if (b < short_blocks + medium_blocks) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -227,6 +243,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
     double* glo = group_lo + (warp * 4 + grp) * kGroupRowMax;
     double* ghi = group_hi + (warp * 4 + grp) * kGroupRowMax;
     const auto full_row = [&](int row) {
+      const auto sides = sides_of(row);
       double lo = 0.0, hi = 0.0;
       int ni = 0, pi = 0;
       const offset_t first = ptr[row], last = ptr[row + 1];
@@ -235,7 +252,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
         live_visit_by<32>(first, last, all_live, live_at, slots + warp * 32, nullptr,
                           [&](offset_t p) { term(p, term.bounds(p), lo, hi, ni, pi); });
       lo = warp_sum_down(lo); hi = warp_sum_down(hi); ni = warp_sum_down(ni); pi = warp_sum_down(pi);
-      if (lane == 0) finish(row, lo, hi, ni, pi);
+      if (lane == 0) finish(row, sides, lo, hi, ni, pi);
     };
     // The row ids and row pointers of later iterations are loaded ahead (the
     // queue entry two iterations ahead, the pointers one ahead), so each
@@ -257,6 +274,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
       const bool kept = have && (!keep_row || keep_row[row]);
       const bool grouped = have && (!kept || last - first <= kGroupRowMax);
       const offset_t end = grouped && kept ? last : first;
+      const auto sides = sides_of(row);   // row 0's past the last
       // Every load of the row's (up to) four entries per lane first.
       int col[4];
       double a[4];
@@ -302,7 +320,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
         ni = ni + __shfl_down_sync(0xffffffffu, ni, off, 8);
         pi = pi + __shfl_down_sync(0xffffffffu, pi, off, 8);
       }
-      if (grouped && gl == 0) finish(row, lo, hi, ni, pi);
+      if (grouped && gl == 0) finish(row, sides, lo, hi, ni, pi);
       // Longer medium rows: one warp each, as before.
       unsigned rest = __ballot_sync(0xffffffffu, have && !grouped && gl == 0);
       while (rest) {
@@ -317,6 +335,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
     const int count = counts[1];
     for (int q = lb; q < count; q += nlong) {
       const int row = longq[q];
+      const auto sides = sides_of(row);
       double lo = 0.0, hi = 0.0;
       int ni = 0, pi = 0;
       const offset_t first = ptr[row], last = ptr[row + 1];
@@ -328,7 +347,7 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
       hi = block_sum_cub_order(hi, dagg);
       ni = block_sum_cub_order(ni, iagg);
       pi = block_sum_cub_order(pi, iagg);
-      if (threadIdx.x == 0) finish(row, lo, hi, ni, pi);
+      if (threadIdx.x == 0) finish(row, sides, lo, hi, ni, pi);
       __syncthreads();
     }
   }

@@ -22,10 +22,18 @@ __global__ void redundant_apply(int m, const uint8_t* __restrict__ action, uint8
 }
 
 // _kernel_dual_fix_candidates (rule_dual_fix.cu:205-309).
-__global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col, const uint8_t* __restrict__ keep_row,
+// Bound by the chain from a column's pointers over its entries to their rows,
+// so four entries are loaded at once and a row answers with one byte (its mask
+// and the finiteness of its sides, 17 bytes in three places otherwise).
+__global__ void row_kinds_kernel(int m, const uint8_t* __restrict__ keep_row, const double* __restrict__ AL,
+                                 const double* __restrict__ AU, uint8_t* __restrict__ kinds) {
+  after_previous_kernel();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+    kinds[i] = row_kind(keep_row[i], AL[i], AU[i]);
+}
+__global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col, const uint8_t* __restrict__ kinds,
                                     const double* __restrict__ c, const double* __restrict__ l,
-                                    const double* __restrict__ u, const double* __restrict__ AL,
-                                    const double* __restrict__ AU, const offset_t* __restrict__ at_ptr,
+                                    const double* __restrict__ u, const offset_t* __restrict__ at_ptr,
                                     const int32_t* __restrict__ at_idx, const double* __restrict__ at_val,
                                     double zt, double bound_tol, int max_degree, const int32_t* __restrict__ col_nnz,
                                     uint8_t* __restrict__ fixed, uint8_t* __restrict__ inf_fix,
@@ -40,13 +48,26 @@ __global__ void dual_fix_candidates(int n, const uint8_t* __restrict__ keep_col,
     const double cj = c[j];
     if (fabs(cj) > zt && col_nnz[j] > max_degree) continue;
     bool down = false, up = false;
-    for (offset_t p = at_ptr[j]; p < at_ptr[j + 1]; ++p) {
-      const int row = at_idx[p];
-      if (!keep_row[row]) continue;
-      const double a = at_val[p];
-      if (a > zt) { down = down || isfinite(AL[row]); up = up || isfinite(AU[row]); }
-      else if (a < -zt) { down = down || isfinite(AU[row]); up = up || isfinite(AL[row]); }
-      if (down && up) break;
+    const offset_t end = at_ptr[j + 1];
+    for (offset_t p = at_ptr[j]; p < end && !(down && up); p += 4) {
+      int row[4];
+      double a[4];
+      uint8_t kind[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        row[k] = p + k < end ? at_idx[p + k] : -1;
+        a[k] = p + k < end ? at_val[p + k] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) kind[k] = row[k] >= 0 ? kinds[row[k]] : uint8_t(0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint8_t low = a[k] > zt ? kRowLower : a[k] < -zt ? kRowUpper : uint8_t(0);
+        if (low) {
+          down = down || (kind[k] & low);
+          up = up || (kind[k] & ((kRowLower | kRowUpper) ^ low));
+        }
+      }
     }
     bool f = false, fi = false;
     double v = 0.0;
@@ -174,13 +195,18 @@ void rule_redundant_rows(Plan& plan, const WorkingLp& lp, const Stats& stats, co
   if (m == 0) return;
   auto s = ctx().stream;
   DBuf<uint8_t> action(size_t(m), s);
+  if (plan.row_kinds.n < size_t(m)) plan.row_kinds.alloc(size_t(m), s);
+  plan.row_kinds_current = false;
   mirror_bounds(plan, lp.n(), s);
   const Report report = ctx().open_report(1);
   redundant_rows_test(lp.A, plan.lu.p, plan.keep_row.p, stats.row_nnz.p,
-                      RedundantTest{plan.AL.p, plan.AU.p, p.bound_tol, action.p, report}, s, stats.version);
+                      RedundantTest{plan.AL.p, plan.AU.p, p.bound_tol, action.p, plan.row_kinds.p, report}, s, stats.version);
   const uint32_t found = uint32_t(ctx().await(report)[0]);
   if (found & 1u) { plan.has_infeasible = true; return; }
-  if (!found) return;
+  if (!found) {
+    plan.row_kinds_current = true;
+    return;
+  }
   const bool deleted = (found & 2u) != 0;
   GPP_LAUNCH(redundant_apply, grid_stride_blocks(m), kThreads, 0, s, m, action.p, plan.keep_row.p, plan.AL.p,
              plan.AU.p);
@@ -197,9 +223,14 @@ void rule_dual_fix(Plan& plan, const WorkingLp& lp, const Stats& stats, const gp
   auto s = ctx().stream;
   DBuf<uint8_t> fixed(size_t(n), s), inf_fix(size_t(n), s), finite, remove;
   DBuf<double> fval(size_t(n), s), contrib(size_t(n), s), shift(size_t(std::max(m, 1)), s);
+  if (!std::exchange(plan.row_kinds_current, false) && m) {
+    if (plan.row_kinds.n < size_t(m)) plan.row_kinds.alloc(size_t(m), s);
+    GPP_LAUNCH(row_kinds_kernel, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, plan.AL.p, plan.AU.p,
+               plan.row_kinds.p);
+  }
   Report report = ctx().open_report(1);
-  GPP_LAUNCH(dual_fix_candidates, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.keep_row.p,
-             plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, lp.AT.ptr, lp.AT.idx, lp.AT.val, p.zero_tol,
+  GPP_LAUNCH(dual_fix_candidates, grid_stride_blocks(n), kThreads, 0, s, n, plan.keep_col.p, plan.row_kinds.p,
+             plan.c.p, plan.l.p, plan.u.p, lp.AT.ptr, lp.AT.idx, lp.AT.val, p.zero_tol,
              p.bound_tol, p.dual_fix_max_nonzero_cost_col_degree, stats.col_nnz.p, fixed.p, inf_fix.p, fval.p,
              contrib.p, report);
   const uint32_t found = uint32_t(ctx().await(report)[0]);

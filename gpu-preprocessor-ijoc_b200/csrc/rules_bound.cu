@@ -228,125 +228,140 @@ __device__ __forceinline__ void support_rows(const SupportArgs& g, int j, double
 }
 
 // What the finalisation leaves per column.  `change` bits: 1 lower, 2 upper
-// bound moved, 4 fixed (at its new lower bound); the support rows and the
-// records' positions stand for the moved ones only.
+// bound moved, 4 fixed (at its new lower bound); new bounds and support rows
+// stand for the moved ones only.  `before`: per tile of kThreads columns the
+// records (x) and their indices (y) of the columns before it, and the totals.
 struct FinalBounds {
   double *l, *u;
   uint8_t* change;
-  int32_t *sup_l, *sup_u, *rec_pos, *idx_pos;
+  int32_t *sup_l, *sup_u;
+  uint32_t* tile_counts;
+  int2* before;
 };
+// A column's records and their indices, 16 bits each.
+__device__ __forceinline__ uint32_t bound_records(uint32_t change, int sup_l, int sup_u) {
+  const uint32_t lc = change & 1u, uc = change >> 1 & 1u;
+  const uint32_t recs = lc + uc;
+  return recs | (recs + (lc && sup_l != INT_MAX ? 1u : 0u) + (uc && sup_u != INT_MAX ? 1u : 0u)) << 16;
+}
 
 // Finalisation, support rows and the records' positions (:970-1008) in one
-// pass over the columns, 32 consecutive ones per warp and round: the records
-// of a column, at most two with at most four indices, are ranked by ballots
-// within the warp and by a look-back over the tiles.  The packed bounds and the
-// candidates are left as the next sweep needs them.  Report: word 0 flags (1
-// infeasible, 2 a bound moves, 4 a column is fixed), 1 records, 2 indices.
-__global__ void __launch_bounds__(kThreads)
+// pass over the columns: a tile's records are counted as it goes, and the last
+// block to finish sums the tiles' counts (commit_bounds ranks within the tile).
+// A column whose bounds stand costs its reads alone; the packed bounds and the
+// candidates, which the next sweep starts from, are written where they differ.
+// Bound by DRAM (49 bytes a column); a form that handed its tiles out in order
+// and looked back for the records before them took 442 us for the 29.8M-nnz
+// LP's columns, 69 us for the 2M-nnz one's.  Report: word 0 flags (1 infeasible, 2 a
+// bound moves, 4 a column is fixed), 1 records, 2 indices.
+__global__ void __launch_bounds__(kThreads, 3)
 finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
                 const double* __restrict__ u, double* __restrict__ cand_l, double* __restrict__ cand_u,
                 double2* __restrict__ lu, const double* __restrict__ c, const double* __restrict__ vmax,
-                int preserve_free_zero_cost, double ft, double upper_relax, bool records, SupportArgs g, FinalBounds out,
-                unsigned long long* words, unsigned int* counters, int32_t* error, Report report) {
+                int preserve_free_zero_cost, double ft, double upper_relax, bool records, SupportArgs g,
+                FinalBounds out, Report report) {
   after_previous_kernel();
-  __shared__ int warp_sums[2][kThreads / 32];
-  __shared__ long long tile_before[2];
-  __shared__ unsigned int ticket;
-  if (threadIdx.x == 0) ticket = tiles > 1 ? atomicAdd(counters, 1u) : 0u;
-  __syncthreads();
+  __shared__ uint32_t warp_sums[2][kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t t = ticket;
-  const int64_t base = t * kScanTile + warp * 32 * kScanItems + lane;
   uint32_t found = 0;
-  unsigned packed = 0;   // per round: 2 bits records, 2 bits indices beyond one per record
-  int sum0 = 0, sum1 = 0;
-#pragma unroll 1
-  for (int k = 0; k < kScanItems; ++k) {
-    const int64_t j64 = base + k * 32;
-    unsigned recs = 0, extra = 0;
+  int turn = 0;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x, turn ^= 1) {
+    const int64_t j64 = int64_t(t) * kThreads + threadIdx.x;
+    uint32_t mine = 0;
     if (j64 < n) {
       const int j = int(j64);
-      const double lj = l[j], uj = u[j];
-      ColumnBounds b{lj, uj, 0.0, false, false, false, false};
-      const bool kept = keep_col[j];
-      if (kept)
-        b = finalize_column(lj, uj, cand_l[j], cand_u[j], c[j], vmax[j], preserve_free_zero_cost != 0, g.zero_tol, ft,
-                            upper_relax);
-      if (b.infeasible) {
-        found |= 1u;
-        b = ColumnBounds{lj, uj, 0.0, false, false, false, false};
-      }
-      if (b.fixed) found |= 4u;
-      if (b.l_changed || b.u_changed) {
-        found |= 2u;
-        if (records) {
-          int sl, su;
-          support_rows(g, j, lj, uj, b, sl, su);
-          recs = unsigned(b.l_changed) + unsigned(b.u_changed);
-          extra = unsigned(b.l_changed && sl != INT_MAX) + unsigned(b.u_changed && su != INT_MAX);
-          out.sup_l[j] = sl;
-          out.sup_u[j] = su;
+      uint32_t change = 0;
+      if (keep_col[j]) {
+        const double lj = l[j], uj = u[j], cl = cand_l[j], cu = cand_u[j];
+        ColumnBounds b = finalize_column(lj, uj, cl, cu, c[j], vmax[j], preserve_free_zero_cost != 0, g.zero_tol, ft,
+                                         upper_relax);
+        if (b.infeasible) {
+          found |= 1u;
+          b = ColumnBounds{lj, uj, 0.0, false, false, false, false};
         }
+        change = (b.l_changed ? 1u : 0u) | (b.u_changed ? 2u : 0u) | (b.fixed ? 4u : 0u);
+        if (change) {
+          found |= b.fixed ? 4u : 0u;
+          out.l[j] = b.l;
+          out.u[j] = b.u;
+          const double removed = __longlong_as_double(static_cast<long long>(kRemovedColumnBits));
+          lu[j] = b.fixed ? make_double2(removed, removed) : make_double2(b.l, b.u);
+        }
+        if (change & 3u) {
+          found |= 2u;
+          if (records) {
+            int sl, su;
+            support_rows(g, j, lj, uj, b, sl, su);
+            mine = bound_records(change, sl, su);
+            out.sup_l[j] = sl;
+            out.sup_u[j] = su;
+          }
+        }
+        if (__double_as_longlong(cl) != __double_as_longlong(b.l)) cand_l[j] = b.l;
+        if (__double_as_longlong(cu) != __double_as_longlong(b.u)) cand_u[j] = b.u;
       }
-      out.l[j] = b.l;
-      out.u[j] = b.u;
-      out.change[j] = uint8_t((b.l_changed ? 1 : 0) | (b.u_changed ? 2 : 0) | (b.fixed ? 4 : 0));
-      cand_l[j] = b.l;
-      cand_u[j] = b.u;
-      if (kept && !b.fixed) lu[j] = make_double2(b.l, b.u);
-      else {
-        const double removed = __longlong_as_double(static_cast<long long>(kRemovedColumnBits));
-        lu[j] = make_double2(removed, removed);
-      }
+      out.change[j] = uint8_t(change);
     }
-    packed |= (recs | extra << 2) << (4 * k);
-    const int r = __popc(__ballot_sync(0xffffffffu, recs & 1)) + 2 * __popc(__ballot_sync(0xffffffffu, recs >> 1));
-    sum0 += r;
-    sum1 += r + __popc(__ballot_sync(0xffffffffu, extra & 1)) + 2 * __popc(__ballot_sync(0xffffffffu, extra >> 1));
-  }
-  if (lane == 0) {
-    warp_sums[0][warp] = sum0;
-    warp_sums[1][warp] = sum1;
-  }
-  __syncthreads();
-  if (warp < 2) {
-    int all = 0;
+    if (!records) continue;
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) warp_sums[turn][warp] = mine;
+    __syncthreads();   // the other turn's sums are read before the next one
+    if (threadIdx.x == 0) {
+      uint32_t sum = 0;
 #pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w) all += warp_sums[warp][w];
-    const long long before = publish_and_look_back(words + int64_t(warp) * tiles, t, tiles, all, error);
-    if (lane == 0) {
-      tile_before[warp] = before;
-      if (t == tiles - 1) report.words[1 + warp] = int32_t(before + all);
+      for (int w = 0; w < kThreads / 32; ++w) sum += warp_sums[turn][w];
+      out.tile_counts[t] = sum;
     }
   }
-  __syncthreads();
-  if (records) {
-    int at0 = int(tile_before[0]), at1 = int(tile_before[1]);
-#pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w) {
-      at0 += w < warp ? warp_sums[0][w] : 0;
-      at1 += w < warp ? warp_sums[1][w] : 0;
-    }
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll 1
-    for (int k = 0; k < kScanItems; ++k) {
-      const unsigned recs = packed >> (4 * k) & 3u, extra = packed >> (4 * k + 2) & 3u;
-      const unsigned r0 = __ballot_sync(0xffffffffu, recs & 1), r1 = __ballot_sync(0xffffffffu, recs >> 1);
-      const unsigned e0 = __ballot_sync(0xffffffffu, extra & 1), e1 = __ballot_sync(0xffffffffu, extra >> 1);
-      if (recs) {
-        const int64_t j = base + k * 32;
-        const int rb = __popc(r0 & below) + 2 * __popc(r1 & below);
-        out.rec_pos[j] = at0 + rb;
-        out.idx_pos[j] = at1 + rb + __popc(e0 & below) + 2 * __popc(e1 & below);
-      }
-      const int r = __popc(r0) + 2 * __popc(r1);
-      at0 += r;
-      at1 += r + __popc(e0) + 2 * __popc(e1);
-    }
-  }
-  if (tiles > 1) leave_zeroed(words, int64_t(tiles) * 2, counters);
   gather_flags(report, found);
-  post_report(report);
+  if (!last_to_report(report)) return;
+  if (records) {
+    constexpr int kEach = 4;
+    __shared__ int2 warp_totals[kThreads / 32];
+    int2 total = make_int2(0, 0);
+    for (int first = 0; first < tiles; first += kThreads * kEach) {
+      uint32_t v[kEach];
+      int2 own = make_int2(0, 0);
+#pragma unroll
+      for (int k = 0; k < kEach; ++k) {
+        const int t = first + int(threadIdx.x) * kEach + k;
+        v[k] = t < tiles ? __ldcg(out.tile_counts + t) : 0u;
+        own.x += int(v[k] & 0xffffu);
+        own.y += int(v[k] >> 16);
+      }
+      int2 upto = own;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto.x, off), y = __shfl_up_sync(0xffffffffu, upto.y, off);
+        if (lane >= off) { upto.x += x; upto.y += y; }
+      }
+      if (lane == 31) warp_totals[warp] = upto;
+      __syncthreads();
+      int2 at = make_int2(total.x + upto.x - own.x, total.y + upto.y - own.y);
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) {
+        const int2 s = warp_totals[w];
+        if (w < warp) { at.x += s.x; at.y += s.y; }
+        total.x += s.x;
+        total.y += s.y;
+      }
+#pragma unroll
+      for (int k = 0; k < kEach; ++k) {
+        const int t = first + int(threadIdx.x) * kEach + k;
+        if (t < tiles) out.before[t] = at;
+        at.x += int(v[k] & 0xffffu);
+        at.y += int(v[k] >> 16);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      out.before[tiles] = total;
+      report.words[1] = total.x;
+      report.words[2] = total.y;
+    }
+    __syncthreads();
+  }
+  post_words(report);
 }
 
 constexpr int kVariableBoundChange = 11, kRowImpliedBoundChange = 12, kFixedVariable = 0;
@@ -358,22 +373,51 @@ struct BoundRecords {
   int32_t* idx;
   double* val;
 };
-__global__ void commit_bounds(int n, FinalBounds f, bool records, BoundRecords rec, double* __restrict__ l,
-                              double* __restrict__ u, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ fixed,
-                              double* __restrict__ fixed_at) {
+__global__ void __launch_bounds__(kThreads)
+commit_bounds(int n, int tiles, FinalBounds f, bool records, BoundRecords rec, double* __restrict__ l,
+              double* __restrict__ u, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ fixed,
+              double* __restrict__ fixed_at) {
   after_previous_kernel();
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    if (records && j == 0) { rec.is[0] = 0; rec.vs[0] = 0; }
-    const uint8_t change = f.change[j];
-    if (fixed) {
-      fixed[j] = (change & 4) != 0;
-      fixed_at[j] = (change & 4) ? f.l[j] : 0.0;
+  __shared__ uint32_t warp_sums[2][kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int turn = 0;
+  if (records && blockIdx.x == 0 && threadIdx.x == 0) { rec.is[0] = 0; rec.vs[0] = 0; }
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int64_t j64 = int64_t(t) * kThreads + threadIdx.x;
+    const uint32_t change = j64 < n ? f.change[j64] : 0u;
+    const int j = int(j64);
+    if (fixed && j64 < n) {
+      fixed[j] = (change & 4u) != 0;
+      fixed_at[j] = (change & 4u) ? f.l[j] : 0.0;
+    }
+    const bool lc = change & 1u, uc = change & 2u;
+    int sl = INT_MAX, su = INT_MAX;
+    int2 at = make_int2(0, 0);
+    if (records) {
+      at = f.before[t];
+      if (f.before[t + 1].x != at.x) {   // block-uniform: the tile has records
+        if (lc || uc) { sl = f.sup_l[j]; su = f.sup_u[j]; }
+        const uint32_t own = bound_records(change, sl, su);
+        uint32_t upto = own;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, upto, off);
+          if (lane >= off) upto += v;
+        }
+        if (lane == 31) warp_sums[turn][warp] = upto;
+        __syncthreads();   // the other turn's sums are read before the next one
+        uint32_t rank = upto - own;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) rank += w < warp ? warp_sums[turn][w] : 0u;
+        turn ^= 1;
+        at.x += int(rank & 0xffffu);
+        at.y += int(rank >> 16);
+      }
     }
     if (!change) continue;
     const double nl = f.l[j], nu = f.u[j];
-    const bool lc = change & 1, uc = change & 2;
     if (records && (lc || uc)) {
-      int64_t k = f.rec_pos[j], ip = f.idx_pos[j];
+      int64_t k = at.x, ip = at.y;
       double cur_l = l[j];
       const double cur_u = u[j];
       auto emit = [&](int sup, double a, double b, double c2, double d) {
@@ -386,14 +430,14 @@ __global__ void commit_bounds(int n, FinalBounds f, bool records, BoundRecords r
         ++k;
       };
       if (lc) {
-        emit(f.sup_l[j], cur_l, cur_u, nl, cur_u);
+        emit(sl, cur_l, cur_u, nl, cur_u);
         cur_l = nl;
       }
-      if (uc) emit(f.sup_u[j], cur_l, cur_u, cur_l, nu);
+      if (uc) emit(su, cur_l, cur_u, cur_l, nu);
     }
     l[j] = nl;
     u[j] = nu;
-    if (change & 4) keep_col[j] = 0;
+    if (change & 4u) keep_col[j] = 0;
   }
 }
 
@@ -512,21 +556,26 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   const bool records = p.record_postsolve_tape != 0;
   DBuf<double> fl(size_t(n), s), fu(size_t(n), s);
   DBuf<uint8_t> change(size_t(n), s);
-  DBuf<int32_t> sl, su, rpos, ipos;
-  if (records)
-    for (DBuf<int32_t>* b : {&sl, &su, &rpos, &ipos}) b->alloc(size_t(n), s);
-  const FinalBounds fin{fl.p, fu.p, change.p, sl.p, su.p, rpos.p, ipos.p};
+  const int tiles = int((int64_t(n) + kThreads - 1) / kThreads);
+  DBuf<int32_t> sl, su;
+  DBuf<uint32_t> tile_counts;
+  DBuf<int2> before;
+  if (records) {
+    sl.alloc(size_t(n), s);
+    su.alloc(size_t(n), s);
+    tile_counts.alloc(size_t(tiles), s);
+    before.alloc(size_t(tiles) + 1, s);
+  }
+  const FinalBounds fin{fl.p, fu.p, change.p, sl.p, su.p, tile_counts.p, before.p};
   const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
   const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p, stats.row_nnz.p, plan.AL.p,
                             plan.AU.p, rs,        p.zero_tol, p.bound_tol,    support_tol};
-  const int tiles = int((int64_t(n) + kScanTile - 1) / kScanTile);
-  LookbackSpace w(size_t(tiles) * 2, s);
   Report report = ctx().open_report(3);
-  GPP_LAUNCH(finalize_kernel, tiles, kThreads, 0, s, n, tiles, plan.keep_col.p, plan.l.p, plan.u.p, plan.cand_l.p,
-             plan.cand_u.p, plan.lu.p, plan.c.p, plan.col_max.p, int(p.bound_strengthening_preserve_free_zero_cost),
-             p.feasibility_tol, p.bound_strengthening_upper_relaxation_factor, records, support, fin, w.words, w.counters,
-             ctx().host_error, report);
-  const volatile int64_t* answer = ctx().await(report);
+  GPP_LAUNCH(finalize_kernel, std::min(tiles, kNumSMs * 12), kThreads, 0, s, n, tiles, plan.keep_col.p, plan.l.p,
+             plan.u.p, plan.cand_l.p, plan.cand_u.p, plan.lu.p, plan.c.p, plan.col_max.p,
+             int(p.bound_strengthening_preserve_free_zero_cost), p.feasibility_tol,
+             p.bound_strengthening_upper_relaxation_factor, records, support, fin, report);
+  const int64_t* answer = ctx().await(report);
   const uint32_t found = uint32_t(answer[0]);
   if (found & 1u) { plan.has_infeasible = true; return; }
   const bool changed = (found & 2u) != 0, fixed = (found & 4u) != 0;
@@ -545,7 +594,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     fx.alloc(size_t(n), s);
     fixv.alloc(size_t(n), s);
   }
-  GPP_LAUNCH(commit_bounds, grid_stride_blocks(n), kThreads, 0, s, n, fin, recs > 0, rec, plan.l.p, plan.u.p,
+  GPP_LAUNCH(commit_bounds, std::min(tiles, kNumSMs * 8), kThreads, 0, s, n, tiles, fin, recs > 0, rec, plan.l.p, plan.u.p,
              plan.keep_col.p, fx.p, fixv.p);
   if (recs) plan.tape.push_back(std::move(seg));
   double obj_delta = 0.0;

@@ -115,23 +115,46 @@ struct CacheOut {
   }
 };
 
+// A column's bounds for the cache: the packed records where the plan holds
+// them as it stands (one access of 16 bytes), the mask and both bounds else.
+template <bool kPacked>
+struct CacheBounds {
+  const double2* lu;
+  const uint8_t* keep_col;
+  const double *l, *u;
+  __device__ __forceinline__ bool get(int col, double2& b) const {
+    if constexpr (kPacked) {
+      b = lu[col];
+      return !removed_column(b);
+    } else {
+      if (!keep_col[col]) return false;
+      b = make_double2(l[col], u[col]);
+      return true;
+    }
+  }
+};
+
 // _kernel_singleton_row_activity_cache (:555-614) for rows of live length
 // <= 1024.  The reference's sequential loop skips a NaN term entirely, counts
 // an infinite term and adds a finite one; the counts and the NaN flag are
-// order-free, so they come from ballots, and the finite sums are formed in
-// stored order by the same shuffle-add chain on every lane of the row.  A
+// order-free, so they come from ballots (where a row of the warp has such a
+// term), and the finite sums are formed in stored order, from shared memory, by
+// one lane each, for as many steps as the warp's longest row has (a chain of 32
+// shuffles over all lanes kept the shuffle unit busy: 162 us at the 29.8M-nnz
+// LP).  A
 // skipped term enters the chain as +0.0, which is exact: a sum that starts at
 // +0.0 never becomes -0.0 in round-to-nearest, and x + (+0.0) == x for every
 // other x.  Rows of at most 32 stored entries (nearly all) take eight lanes
 // each, four rows per warp, with all of a row's loads issued before its
 // chain; longer rows take a whole warp, 32 entries at a time.
+template <bool kPacked>
 __device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, const int32_t* __restrict__ st,
                               const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
                               const int32_t* __restrict__ idx, const double* __restrict__ val,
-                              const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
-                              const double* __restrict__ u, CacheOut out) {
+                              CacheBounds<kPacked> bounds, CacheOut out) {
+  __shared__ double terms[kThreads / 32][2][4][33];   // by warp, sum and row; a row's padded by one
   const int count = st[kStRows];
-  const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
+  const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7, warp = threadIdx.x >> 5;
   const int warps = blocks * (blockDim.x >> 5);
   const auto group_bits = [&](bool v) { return (__ballot_sync(0xffffffffu, v) >> (grp * 8)) & 0xffu; };
   const auto whole_row = [&](int row) {
@@ -143,11 +166,12 @@ __device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, cons
       bool live = false;
       if (p < end) {
         const int col = __ldcs(idx + p);
-        if (keep_col[col]) {
-          live = true;
+        double2 b;
+        live = bounds.get(col, b);
+        if (live) {
           const double a = __ldcs(val + p);
-          tmin = a >= 0.0 ? a * l[col] : a * u[col];
-          tmax = a >= 0.0 ? a * u[col] : a * l[col];
+          tmin = a >= 0.0 ? a * b.x : a * b.y;
+          tmax = a >= 0.0 ? a * b.y : a * b.x;
         }
       }
       const bool nan = live && (isnan(tmin) || isnan(tmax));
@@ -198,32 +222,49 @@ __device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, cons
       a[j] = p < stop ? __ldcs(val + p) : 0.0;
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) live[j] = col[j] >= 0 && keep_col[col[j]];
-#pragma unroll
     for (int j = 0; j < 4; ++j) {
-      lj[j] = live[j] ? l[col[j]] : 0.0;
-      uj[j] = live[j] ? u[col[j]] : 0.0;
+      double2 b = make_double2(0.0, 0.0);
+      live[j] = col[j] >= 0 && bounds.get(col[j], b);
+      lj[j] = b.x;
+      uj[j] = b.y;
     }
     RowCache r{0.0, 0.0, 0, 0, 0, 0, 0};
+    const int steps = __reduce_max_sync(0xffffffffu, int(stop - first));   // of the warp's longest row
+    bool odd = false;   // a NaN or infinite term in the warp's rows
+    double tmin[4], tmax[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const double tmin = live[j] ? (a[j] >= 0.0 ? a[j] * lj[j] : a[j] * uj[j]) : 0.0;
-      const double tmax = live[j] ? (a[j] >= 0.0 ? a[j] * uj[j] : a[j] * lj[j]) : 0.0;
-      const bool nan = live[j] && (isnan(tmin) || isnan(tmax));
-      const bool counted = live[j] && !nan;
-      r.invalid |= group_bits(nan) != 0;
-      r.min_neg += __popc(group_bits(counted && isinf(tmin) && tmin < 0.0));
-      r.min_pos += __popc(group_bits(counted && isinf(tmin) && tmin > 0.0));
-      r.max_neg += __popc(group_bits(counted && isinf(tmax) && tmax < 0.0));
-      r.max_pos += __popc(group_bits(counted && isinf(tmax) && tmax > 0.0));
-      const double fmin_term = counted && isfinite(tmin) ? tmin : 0.0;
-      const double fmax_term = counted && isfinite(tmax) ? tmax : 0.0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        r.fmin += __shfl_sync(0xffffffffu, fmin_term, k, 8);
-        r.fmax += __shfl_sync(0xffffffffu, fmax_term, k, 8);
+      tmin[j] = live[j] ? (a[j] >= 0.0 ? a[j] * lj[j] : a[j] * uj[j]) : 0.0;
+      tmax[j] = live[j] ? (a[j] >= 0.0 ? a[j] * uj[j] : a[j] * lj[j]) : 0.0;
+      odd = odd || !isfinite(tmin[j]) || !isfinite(tmax[j]);
+      if (8 * j < steps) {
+        const bool counted = !isnan(tmin[j]) && !isnan(tmax[j]);
+        terms[warp][0][grp][gl + 8 * j] = counted && isfinite(tmin[j]) ? tmin[j] : 0.0;
+        terms[warp][1][grp][gl + 8 * j] = counted && isfinite(tmax[j]) ? tmax[j] : 0.0;
       }
     }
+    if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool nan = isnan(tmin[j]) || isnan(tmax[j]);
+        r.invalid |= group_bits(nan) != 0;
+        r.min_neg += __popc(group_bits(!nan && isinf(tmin[j]) && tmin[j] < 0.0));
+        r.min_pos += __popc(group_bits(!nan && isinf(tmin[j]) && tmin[j] > 0.0));
+        r.max_neg += __popc(group_bits(!nan && isinf(tmax[j]) && tmax[j] < 0.0));
+        r.max_pos += __popc(group_bits(!nan && isinf(tmax[j]) && tmax[j] > 0.0));
+      }
+    }
+    __syncwarp();
+    double sum = 0.0;
+    if (gl < 2) {   // lane 0 of a row folds its minimum, lane 1 its maximum
+      const double* term = terms[warp][gl][grp];
+      for (int k = 0; k < steps; k += 8)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sum += term[k + q];
+    }
+    __syncwarp();
+    r.fmin = sum;
+    r.fmax = __shfl_down_sync(0xffffffffu, sum, 1);
     if (grouped && gl == 0) out.store(row, r);
     unsigned rest = __ballot_sync(0xffffffffu, take && !grouped && gl == 0);
     while (rest) {
@@ -236,11 +277,11 @@ __device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, cons
 
 // _kernel_singleton_long_row_activity_cache (:642-754): block per row; live
 // rank k goes to thread k mod 256, then a shared-memory halving tree.
+template <bool kPacked>
 __device__ void sc_cache_long(int block, int blocks, const int32_t* __restrict__ long_rows,
                               const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz,
                               const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
-                              const double* __restrict__ val, const uint8_t* __restrict__ keep_col,
-                              const double* __restrict__ l, const double* __restrict__ u, CacheOut out) {
+                              const double* __restrict__ val, CacheBounds<kPacked> bounds, CacheOut out) {
   __shared__ int slots[kThreads];
   __shared__ int warp_counts[8];
   __shared__ double s_min[kThreads], s_max[kThreads];
@@ -250,11 +291,12 @@ __device__ void sc_cache_long(int block, int blocks, const int32_t* __restrict__
   for (int q = block; q < count; q += blocks) {
     const int row = long_rows[q];
     const offset_t first = ptr[row], last = ptr[row + 1];
-    const uint8_t* mask = row_nnz[row] != int(last - first) ? keep_col : nullptr;
+    const uint8_t* mask = row_nnz[row] != int(last - first) ? bounds.keep_col : nullptr;
     RowCache r{0.0, 0.0, 0, 0, 0, 0, 0};
     live_visit<kThreads>(first, last, idx, mask, slots, warp_counts, [&](offset_t p) {
       const int col = idx[p];
-      if (keep_col[col]) cache_term(r, val[p], l[col], u[col]);
+      double2 b;
+      if (bounds.get(col, b)) cache_term(r, val[p], b.x, b.y);
     });
     s_min[t] = r.fmin;
     s_max[t] = r.fmax;
@@ -280,17 +322,17 @@ __device__ void sc_cache_long(int block, int blocks, const int32_t* __restrict__
 // rows of up to kLongRow live entries, the rest the long ones.  The grid does
 // not know their numbers (the rule asks the host once, at its end); blocks
 // without rows return at once.
+template <bool kPacked>
 __global__ void __launch_bounds__(kThreads)
 sc_cache(int row_blocks, const int32_t* __restrict__ rows, const int32_t* __restrict__ long_rows,
          const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
-         const int32_t* __restrict__ idx, const double* __restrict__ val, const uint8_t* __restrict__ keep_col,
-         const double* __restrict__ l, const double* __restrict__ u, CacheOut out) {
+         const int32_t* __restrict__ idx, const double* __restrict__ val, CacheBounds<kPacked> bounds, CacheOut out) {
   after_previous_kernel();
   if (int(blockIdx.x) < row_blocks)
-    sc_cache_rows(row_blocks, rows, st, row_nnz, ptr, idx, val, keep_col, l, u, out);
+    sc_cache_rows(row_blocks, rows, st, row_nnz, ptr, idx, val, bounds, out);
   else
     sc_cache_long(int(blockIdx.x) - row_blocks, int(gridDim.x) - row_blocks, long_rows, st, row_nnz, ptr, idx, val,
-                  keep_col, l, u, out);
+                  bounds, out);
 }
 
 // Propose (:905-1018) over the candidate list.
@@ -675,8 +717,14 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   const CacheOut cache{fmin.p, fmax.p, counts.p, invalid.p};
   const int row_blocks = std::max(1, std::min((claims + 31) / 32, kNumSMs * 16));
   const int long_blocks = std::max(1, std::min(kNumSMs * 4, int(lp.A.nnz / kLongRow)));
-  GPP_LAUNCH(sc_cache, row_blocks + long_blocks, kThreads, 0, s, row_blocks, rows.p, long_rows.p, st,
-             stats.row_nnz.p, lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_col.p, plan.l.p, plan.u.p, cache);
+  const auto fill_cache = [&](auto packed) {
+    constexpr bool kPacked = decltype(packed)::value;
+    const CacheBounds<kPacked> bounds{plan.lu.p, plan.keep_col.p, plan.l.p, plan.u.p};
+    GPP_LAUNCH(sc_cache<kPacked>, row_blocks + long_blocks, kThreads, 0, s, row_blocks, rows.p, long_rows.p, st,
+               stats.row_nnz.p, lp.A.ptr, lp.A.idx, lp.A.val, bounds, cache);
+  };
+  if (plan.bounds_mirrored) fill_cache(std::true_type{});
+  else fill_cache(std::false_type{});
   DBuf<uint8_t> action(size_t(n), s), kind(size_t(m), s);
   DBuf<double> side(size_t(n), s), contrib_val(size_t(claims), s);
   DBuf<int64_t> contrib_idx(size_t(claims), s);
@@ -688,7 +736,7 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
   GPP_LAUNCH(sc_stage, grid_stride_blocks(claims), kThreads, 0, s, rows.p, st, n, action.p, side.p,
              stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.bound_tol, owner.p,
              plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p, report);
-  const volatile int64_t* f = ctx().await(report);
+  const int64_t* f = ctx().await(report);
   if (f[kStUnbounded]) { plan.has_unbounded = true; return; }
   const int nwin = int(f[kStWin]), nelim = int(f[kStElim]);
   const bool any_side = f[kStSide] != 0;
@@ -735,7 +783,7 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
             post_values(mail, seq, sum[0], sum[1]);
           },
           s);
-      const volatile int64_t* sums = ctx().await(ctx().mail, seq, "substitution records");
+      const int64_t* sums = ctx().await(ctx().mail, seq, "substitution records");
       const int64_t recs = sums[0], support = sums[1];
       if (recs) {
         PostsolveSegment seg = make_segment(recs, 3 * recs + support, 6 * recs + support);

@@ -397,7 +397,7 @@ void compact_sides(CompactSides& sides, DevCsr* const (&out)[2], cudaStream_t s)
     if (d.tiles) bytes += 12.0 * d.nnz + 4.0 * d.cols + 0.375 * d.nnz;
   LookbackSpace w(size_t(tiles), s);
   const Report report = c.open_report(2);
-  GPP_LAUNCH_BYTES(compact_tiles, bytes, std::min(tiles, kNumSMs * 4), kThreads, 0, s, sides, w.words, w.counters,
+  GPP_LAUNCH_BYTES(compact_tiles, bytes, std::min(tiles, kNumSMs * 5), kThreads, 0, s, sides, w.words, w.counters,
                    c.host_error, report);
   const int64_t record = profile_last();
   GPP_LAUNCH(compact_row_pointers, rows_grid, kThreads, 0, s, sides);

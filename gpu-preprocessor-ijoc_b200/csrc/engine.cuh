@@ -232,6 +232,18 @@ constexpr uint8_t kRowKept = 1, kRowLower = 2, kRowUpper = 4;
 __device__ __forceinline__ uint8_t row_kind(bool kept, double al, double au) {
   return kept ? uint8_t(kRowKept | (isfinite(al) ? kRowLower : 0) | (isfinite(au) ? kRowUpper : 0)) : uint8_t(0);
 }
+// What bound strengthening asks of a row, from the activity sweep: its sides
+// and finite activities in one 32-byte sector (live rows: kept, of more than one
+// live entry) and a byte of flags, bits 0-1 and 2-3 the infinite terms of the
+// minimum and maximum activity (3 for more) and bit 4 live.  An entry's gather
+// costs two sectors where the eight arrays cost eight.
+constexpr uint8_t kRowLive = 16;
+struct RowRecords {
+  double2* sums;   // two per row: AL and AU, minimum and maximum activity
+  uint8_t* flags;
+};
+void row_activity_records(const DevCsr& A, const double2* lu, double zero_tol, const Plan& plan,
+                          const int32_t* live_deg, const RowRecords& out, cudaStream_t s, uint64_t degrees_version);
 void redundant_rows_test(const DevCsr& A, const double2* lu, const uint8_t* keep_row, const int32_t* live_deg,
                          const RedundantTest& test, cudaStream_t s, uint64_t degrees_version);
 void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStream_t s);

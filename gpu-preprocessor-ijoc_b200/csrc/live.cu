@@ -161,16 +161,21 @@ __device__ __forceinline__ uint32_t redundant_test(const RedundantTest& t, int r
 // With Plain the kernel forms the redundant-row rule's sums, in which
 // infinities propagate, and tests each row as soon as its sums stand; the sums
 // themselves are not stored.
-template <bool Plain>
-__global__ void __launch_bounds__(kThreads)
+//
+// Latency-bound (every warp waits for its gathers, the L2 at a third of its
+// rate), so the registers are held to four blocks an SM.
+enum class Sums { kFinite, kRecords, kPlain };
+template <Sums Form>
+__global__ void __launch_bounds__(kThreads, 4)
 activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                 const double* __restrict__ val, const double2* __restrict__ lu, double zero_tol,
                 const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ live_deg,
                 const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
                 const int32_t* __restrict__ counts, int short_blocks, int medium_blocks,
                 double* __restrict__ min_fin, double* __restrict__ max_fin, int32_t* __restrict__ min_inf,
-                int32_t* __restrict__ max_inf, RedundantTest test) {
+                int32_t* __restrict__ max_inf, RowRecords records, RedundantTest test) {
   after_previous_kernel();
+  constexpr bool Plain = Form == Sums::kPlain;
   __shared__ int slots[256];
   __shared__ int warp_counts[8];
   __shared__ double dagg[8];
@@ -181,12 +186,18 @@ activity_kernel(int m, const offset_t* __restrict__ ptr, const int32_t* __restri
   const auto live_at = [&](offset_t p) { return !removed_column(term.bounds(p)); };
   uint32_t found = 0;
   const auto sides_of = [&](int row) {
-    if constexpr (Plain) return RowSides(test, row, keep_row, live_deg);
+    if constexpr (Form != Sums::kFinite) return RowSides(test, row, keep_row, live_deg);
     else return 0;
   };
   const auto finish = [&](int row, const auto& sides, double lo, double hi, int ni, int pi) {
     if constexpr (Plain) {
       found |= redundant_test(test, row, sides, lo, hi);
+    } else if constexpr (Form == Sums::kRecords) {
+      records.flags[row] = uint8_t(min(ni, 3) | min(pi, 3) << 2 | (sides.tested ? kRowLive : 0));
+      if (sides.tested) {
+        records.sums[2 * int64_t(row)] = make_double2(sides.al, sides.au);
+        records.sums[2 * int64_t(row) + 1] = make_double2(lo, hi);
+      }
     } else {
       min_fin[row] = lo; max_fin[row] = hi;
       if (min_inf) { min_inf[row] = ni; max_inf[row] = pi; }
@@ -892,10 +903,11 @@ void pack_bounds(const double* l, const double* u, const uint8_t* keep_col, int3
 }
 
 namespace {
-template <bool Plain>
+template <Sums Form>
 void launch_activity(const DevCsr& A, const double2* lu, double zero_tol, const uint8_t* keep_row,
                      const int32_t* live_deg, double* lo, double* hi, int32_t* ni, int32_t* pi, double out_bytes,
-                     cudaStream_t s, uint64_t degrees_version, const RedundantTest& test = {}) {
+                     cudaStream_t s, uint64_t degrees_version, const RedundantTest& test = {},
+                     const RowRecords& records = {}) {
   static thread_local RowSchedule* live_schedule = new RowSchedule;  // never destroyed (see schedule_cache)
   const RowSchedule* sch;
   if (live_deg) {
@@ -915,14 +927,18 @@ void launch_activity(const DevCsr& A, const double2* lu, double zero_tol, const 
   const double bytes = 4.0 * (A.rows + 1) + 12.0 * A.nnz + 16.0 * A.cols + (keep_row ? A.rows : 0) +
                        (live_deg ? 4.0 * A.rows : 0) + out_bytes * A.rows;
   const int grid = r.short_blocks + r.medium_blocks + r.long_blocks;
-  if constexpr (Plain)
-    GPP_LAUNCH_BYTES(activity_kernel<true>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu, zero_tol,
-                     keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
-                     r.medium_blocks, lo, hi, ni, pi, test);
+  if constexpr (Form == Sums::kPlain)
+    GPP_LAUNCH_BYTES(activity_kernel<Sums::kPlain>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu,
+                     zero_tol, keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
+                     r.medium_blocks, lo, hi, ni, pi, records, test);
+  else if constexpr (Form == Sums::kRecords)
+    GPP_LAUNCH_BYTES(activity_kernel<Sums::kRecords>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu,
+                     zero_tol, keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
+                     r.medium_blocks, lo, hi, ni, pi, records, test);
   else
-    GPP_LAUNCH_BYTES(activity_kernel<false>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu, zero_tol,
-                     keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
-                     r.medium_blocks, lo, hi, ni, pi, test);
+    GPP_LAUNCH_BYTES(activity_kernel<Sums::kFinite>, bytes, grid, kThreads, 0, s, A.rows, A.ptr, A.idx, A.val, lu,
+                     zero_tol, keep_row, live_deg, sch->medium.p, sch->long_rows.p, sch->counts.p, r.short_blocks,
+                     r.medium_blocks, lo, hi, ni, pi, records, test);
 }
 }  // namespace
 
@@ -931,7 +947,7 @@ void row_activity_summary_packed(const DevCsr& A, const double2* lu, double zero
                                  int32_t* max_inf, cudaStream_t s, uint64_t degrees_version) {
   // compute_row_activity_summary (gpu_presolve_kernels.cu:744-787).
   if (!A.rows) return;
-  launch_activity<false>(A, lu, zero_tol, keep_row, live_deg, min_fin, max_fin, min_inf, max_inf, 24.0, s,
+  launch_activity<Sums::kFinite>(A, lu, zero_tol, keep_row, live_deg, min_fin, max_fin, min_inf, max_inf, 24.0, s,
                          degrees_version);
 }
 
@@ -945,9 +961,19 @@ void row_activity_summary(const DevCsr& A, const double* l, const double* u, dou
   row_activity_summary_packed(A, lu.p, zero_tol, keep_row, live_deg, min_fin, max_fin, min_inf, max_inf, s);
 }
 
+void row_activity_records(const DevCsr& A, const double2* lu, double zero_tol, const Plan& plan,
+                          const int32_t* live_deg, const RowRecords& out, cudaStream_t s, uint64_t degrees_version) {
+  if (!A.rows) return;
+  RedundantTest sides{};
+  sides.AL = plan.AL.p;
+  sides.AU = plan.AU.p;
+  launch_activity<Sums::kRecords>(A, lu, zero_tol, plan.keep_row.p, live_deg, nullptr, nullptr, nullptr, nullptr, 49.0,
+                                  s, degrees_version, sides, out);
+}
+
 void redundant_rows_test(const DevCsr& A, const double2* lu, const uint8_t* keep_row, const int32_t* live_deg,
                          const RedundantTest& test, cudaStream_t s, uint64_t degrees_version) {
-  launch_activity<true>(A, lu, 0.0, keep_row, live_deg, nullptr, nullptr, nullptr, nullptr, 17.0, s, degrees_version,
+  launch_activity<Sums::kPlain>(A, lu, 0.0, keep_row, live_deg, nullptr, nullptr, nullptr, nullptr, 17.0, s, degrees_version,
                         test);
 }
 

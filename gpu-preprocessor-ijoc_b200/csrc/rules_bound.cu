@@ -15,13 +15,6 @@ namespace gpp {
 namespace {
 
 
-struct RowSummary {
-  const double* mn;
-  const double* mx;
-  const int32_t* ni;
-  const int32_t* pi;
-};
-
 // Implied bounds of the column of entry a from its row (reference :349-430).
 __device__ __forceinline__ void implied_bounds(double a, double lj, double uj, double al, double au, double mn,
                                                double mx, int ni, int pi, double& il, double& iu) {
@@ -49,12 +42,8 @@ struct CandArgs {
   const offset_t* ptr;
   const int32_t* idx;
   const double* val;
-  const uint8_t* keep_row;
-  const int32_t* row_nnz;
-  const double* AL;
-  const double* AU;
   const double2* lu;   // packed column bounds, removed columns marked
-  RowSummary rs;
+  RowRecords rows;
   double zero_tol;
   double* cand_l;
   double* cand_u;
@@ -64,9 +53,12 @@ struct CandArgs {
 struct RowCtx {
   double al, au, mn, mx;
   int ni, pi;
+  bool live;
 };
-__device__ __forceinline__ RowCtx row_ctx(const CandArgs& g, int i) {
-  return RowCtx{g.AL[i], g.AU[i], g.rs.mn[i], g.rs.mx[i], g.rs.ni[i], g.rs.pi[i]};
+__device__ __forceinline__ RowCtx row_ctx(const RowRecords& rows, int i) {
+  const uint8_t f = rows.flags[i];
+  const double2 sides = rows.sums[2 * int64_t(i)], sums = rows.sums[2 * int64_t(i) + 1];
+  return RowCtx{sides.x, sides.y, sums.x, sums.y, f & 3, f >> 2 & 3, (f & kRowLive) != 0};
 }
 
 // Candidate bounds of column j from one entry a of a row (reference
@@ -115,13 +107,12 @@ candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, CandArgs g)
       const double an = next ? ld_stream(g.val + pn, hint.stream) : 0.0;
       const int i = staged ? r0 + row_of(sptr, 0, r1 - r0 + 1, p) : row_of(g.ptr, r0, r1 + 1, p);
       // Every load of the entry at once (the column's bounds do not depend on
-      // the row; the row's flags and summary come from one or two lines that
-      // the warp's neighbouring entries share), so an entry waits for one
-      // memory round trip instead of two.
+      // the row; the row's record and flags are lines that the warp's
+      // neighbouring entries share), so an entry waits for one memory round
+      // trip instead of two.
       const double2 b = ld_keep(g.lu + j, hint.keep);
-      const bool row_live = (g.keep_row[i] != 0) & (g.row_nnz[i] > 1);
-      const RowCtx rc = row_ctx(g, i);
-      if (row_live && !removed_column(b) && !(fabs(a) <= g.zero_tol)) candidate_update(g, rc, j, a, b);
+      const RowCtx rc = row_ctx(g.rows, i);
+      if (rc.live && !removed_column(b) && !(fabs(a) <= g.zero_tol)) candidate_update(g, rc, j, a, b);
       j = jn;
       a = an;
     }
@@ -182,10 +173,7 @@ struct SupportArgs {
   const offset_t* at_ptr;
   const int32_t* at_idx;
   const double* at_val;
-  const uint8_t* keep_row;
-  const int32_t* row_nnz;
-  const double *AL, *AU;
-  RowSummary rs;
+  RowRecords rows;
   double zero_tol, tol, support_tol;
 };
 // Support rows of a changed column (reference :815-960): the smallest row that
@@ -207,20 +195,14 @@ __device__ __forceinline__ void support_rows(const SupportArgs& g, int j, double
       row[k] = p0 + k < end ? g.at_idx[p0 + k] : -1;
       a[k] = p0 + k < end ? g.at_val[p0 + k] : 0.0;
     }
-    bool live[kBatch];
-    double al[kBatch], au[kBatch], mn[kBatch], mx[kBatch];
-    int ni[kBatch], pi[kBatch];
+    RowCtx rc[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) rc[k] = row_ctx(g.rows, row[k] >= 0 ? row[k] : 0);
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) {
-      const int i = row[k] >= 0 ? row[k] : 0;
-      live[k] = row[k] >= 0 && (g.keep_row[i] != 0) & (g.row_nnz[i] > 1);
-      al[k] = g.AL[i]; au[k] = g.AU[i]; mn[k] = g.rs.mn[i]; mx[k] = g.rs.mx[i]; ni[k] = g.rs.ni[i]; pi[k] = g.rs.pi[i];
-    }
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
-      if (!live[k] || fabs(a[k]) <= g.zero_tol) continue;
+      if (row[k] < 0 || !rc[k].live || fabs(a[k]) <= g.zero_tol) continue;
       double il, iu;
-      implied_bounds(a[k], lj, uj, al[k], au[k], mn[k], mx[k], ni[k], pi[k], il, iu);
+      implied_bounds(a[k], lj, uj, rc[k].al, rc[k].au, rc[k].mn, rc[k].mx, rc[k].ni, rc[k].pi, il, iu);
       if (want_l && isfinite(il) && fabs(il - b.l) <= g.support_tol) sl = min(sl, row[k]);
       if (want_u && isfinite(iu) && fabs(iu - b.u) <= g.support_tol) su = min(su, row[k]);
     }
@@ -503,16 +485,16 @@ __global__ void fixed_record_pack(int n, const uint8_t* __restrict__ fx, const o
 
 // Live rows binned by infinite-term count of their minimum and maximum
 // activity (0, 1, 2, >= 3): the learned schedule's histogram features.
-__global__ void inf_histogram(int m, const uint8_t* __restrict__ keep_row, const int32_t* __restrict__ ni,
-                              const int32_t* __restrict__ pi, uint32_t* __restrict__ hist) {
+__global__ void inf_histogram(int m, const uint8_t* __restrict__ keep_row, const uint8_t* __restrict__ flags,
+                              uint32_t* __restrict__ hist) {
   after_previous_kernel();
   __shared__ uint32_t bins[8];
   if (threadIdx.x < 8) bins[threadIdx.x] = 0;
   __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     if (!keep_row[i]) continue;
-    atomicAdd(&bins[min(ni[i], 3)], 1u);
-    atomicAdd(&bins[4 + min(pi[i], 3)], 1u);
+    atomicAdd(&bins[flags[i] & 3], 1u);
+    atomicAdd(&bins[4 + (flags[i] >> 2 & 3)], 1u);
   }
   __syncthreads();
   if (threadIdx.x < 8 && bins[threadIdx.x]) atomicAdd(hist + threadIdx.x, bins[threadIdx.x]);
@@ -525,23 +507,21 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   const int m = lp.m(), n = lp.n();
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
-  DBuf<double> mn(size_t(m), s), mx(size_t(m), s);
-  DBuf<int32_t> ni(size_t(m), s), pi(size_t(m), s);
+  DBuf<double2> row_sums(2 * size_t(m), s);
+  DBuf<uint8_t> row_flags(size_t(m), s);
+  const RowRecords rows{row_sums.p, row_flags.p};
   // One packed bounds array serves the activity sweep, the candidate sweep
   // and the redundant-row test after them.
   mirror_bounds(plan, n, s);
-  row_activity_summary_packed(lp.A, plan.lu.p, p.zero_tol, plan.keep_row.p, stats.row_nnz.p, mn.p, mx.p, ni.p, pi.p, s,
-                              stats.version);
-  const RowSummary rs{mn.p, mx.p, ni.p, pi.p};
+  row_activity_records(lp.A, plan.lu.p, p.zero_tol, plan, stats.row_nnz.p, rows, s, stats.version);
   if (plan.inf_hist) {
     check(cudaMemsetAsync(plan.inf_hist, 0, 8 * sizeof(uint32_t), s), "inf_hist");
-    GPP_LAUNCH(inf_histogram, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, ni.p, pi.p, plan.inf_hist);
+    GPP_LAUNCH(inf_histogram, grid_stride_blocks(m), kThreads, 0, s, m, plan.keep_row.p, row_flags.p,
+               plan.inf_hist);
   }
   {
-    CandArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, stats.row_nnz.p, plan.AL.p, plan.AU.p, plan.lu.p, rs,
-               p.zero_tol, plan.cand_l.p, plan.cand_u.p};
-    const double bytes = 4.0 * (m + 1) + 12.0 * lp.A.nnz + double(m) + 4.0 * m + 16.0 * m + 24.0 * m + 16.0 * n +
-                         16.0 * n;
+    CandArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.lu.p, rows, p.zero_tol, plan.cand_l.p, plan.cand_u.p};
+    const double bytes = 4.0 * (m + 1) + 12.0 * lp.A.nnz + 33.0 * m + 16.0 * n + 16.0 * n;
     const RowSchedule& sch = stored_schedule(lp.A);
     GPP_LAUNCH_BYTES(candidates_entries, bytes, int(std::max<int64_t>(1, std::min<int64_t>(sch.tiles, kNumSMs * 8))),
                      kThreads, 0, s, lp.A.nnz, sch.tile_rows.p, g);
@@ -568,8 +548,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   }
   const FinalBounds fin{fl.p, fu.p, change.p, sl.p, su.p, tile_counts.p, before.p};
   const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
-  const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p, stats.row_nnz.p, plan.AL.p,
-                            plan.AU.p, rs,        p.zero_tol, p.bound_tol,    support_tol};
+  const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, rows, p.zero_tol, p.bound_tol, support_tol};
   Report report = ctx().open_report(3);
   GPP_LAUNCH(finalize_kernel, std::min(tiles, kNumSMs * 12), kThreads, 0, s, n, tiles, plan.keep_col.p, plan.l.p,
              plan.u.p, plan.cand_l.p, plan.cand_u.p, plan.lu.p, plan.c.p, plan.col_max.p,

@@ -54,107 +54,102 @@ __device__ void row_hash_thread(const RowHashArgs& g, int i) {
   g.out[i] = g.use_xor ? mix(h, agg) : h;
 }
 
-// Long rows (past kLongRow stored entries), one block per row.  The FNV fold
-// visits the entries in stored order, two dependent 64-bit multiplications
-// each, so one thread does nothing else: the other seven warps form the live
-// entries' (column, bits of value / pivot) pairs of the next stage in shared
-// memory meanwhile.  A warp that did both, through shuffles, took 0.9 ms for
-// the 5,000-entry hub rows of the 29.8M-nnz LP.
-constexpr int kHashLoaders = kThreads - 32;
+// Long rows (past kLongRow stored entries), eight to a block.  The FNV fold
+// visits a row's entries in stored order, two dependent 64-bit multiplications
+// each (about 75 us for a 5,000-entry row), so eight lanes of one warp fold a
+// row each and do nothing else; the other seven warps form the next stage of
+// the rows' (column, bits of value / pivot) pairs in shared memory meanwhile,
+// removed columns marked.  One row to a block left the 2,000 such rows of the
+// 29.8M-nnz LP to take turns (943 us for all rows of that model).
+constexpr int kHashRows = 8, kHashStage = 112;   // 28 loaders a row, four entries each
 struct HashStage {
-  uint64_t col[kHashLoaders], bits[kHashLoaders];
-  int count;
+  int32_t col[kHashRows][kHashStage + 1];
+  uint64_t bits[kHashRows][kHashStage + 1];
 };
-__device__ void row_hash_block(const RowHashArgs& g, int i, HashStage* stage) {
-  __shared__ int warp_live[kThreads / 32];
-  __shared__ long long first_live;
-  __shared__ int live_len;
-  __shared__ unsigned long long agg_shared;
+__device__ void row_hash_block(const RowHashArgs& g, const int32_t* rows, int count, HashStage* stage) {
+  __shared__ offset_t from_shared[kHashRows], end_shared[kHashRows];
+  __shared__ double pivot_shared[kHashRows];
+  __shared__ int len_shared[kHashRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (!g.keep_row[i]) {   // block-uniform
-    if (threadIdx.x == 0) g.out[i] = uint64_t(i);
-    return;
-  }
-  const offset_t a = g.ptr[i], e = g.ptr[i + 1];
-  if (threadIdx.x == 0) {
-    first_live = LLONG_MAX;
-    live_len = 0;
-    agg_shared = 0;
+  {   // a warp per row: its live length and first live entry (the pivot)
+    const int i = warp < count ? rows[warp] : -1;
+    const bool keep = i >= 0 && g.keep_row[i];
+    const offset_t a = keep ? g.ptr[i] : 0, e = keep ? g.ptr[i + 1] : 0;
+    int len = int(e - a);
+    offset_t first = a;
+    if (g.keep_col) {
+      len = 0;
+      first = -1;
+      for (int at = 0; e - a > at; at += 128) {
+        bool live[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          live[k] = e - a > at + 32 * k + lane && g.keep_col[__ldcs(g.idx + a + at + 32 * k + lane)];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned mask = __ballot_sync(0xffffffffu, live[k]);
+          if (first < 0 && mask) first = a + at + 32 * k + (__ffs(mask) - 1);
+          len += __popc(mask);
+        }
+      }
+    }
+    const bool trivial = !keep || len == 0 || fabs(g.val[first]) <= g.tol;
+    if (lane == 0) {
+      from_shared[warp] = trivial ? e : first;
+      end_shared[warp] = e;
+      pivot_shared[warp] = trivial ? 1.0 : g.val[first];
+      len_shared[warp] = len;
+      if (i >= 0 && trivial) g.out[i] = keep ? mix(kFnvOffset, uint64_t(i)) : uint64_t(i);
+    }
   }
   __syncthreads();
-  long long first = LLONG_MAX;
-  int len = 0;
-  for (offset_t p = a + offset_t(threadIdx.x); p < e; p += kThreads)
-    if (!g.keep_col || g.keep_col[g.idx[p]]) { first = min(first, (long long)p); ++len; }
-  for (int off = 16; off; off >>= 1) {
-    len += __shfl_xor_sync(0xffffffffu, len, off);
-    first = min(first, __shfl_xor_sync(0xffffffffu, first, off));
-  }
-  if (lane == 0 && len) {
-    atomicAdd(&live_len, len);
-    atomicMin(&first_live, first);
-  }
-  __syncthreads();
-  len = live_len;
-  if (len == 0 || fabs(g.val[first_live]) <= g.tol) {
-    if (threadIdx.x == 0) g.out[i] = mix(kFnvOffset, uint64_t(i));
-    __syncthreads();
-    return;
-  }
-  const offset_t from = offset_t(first_live);
-  const double pivot = g.val[from];
-  uint64_t h = mix(kFnvOffset, uint64_t(len));
-  if (g.use_xor) {
-    uint64_t agg = 0;
-    for (offset_t p = from + offset_t(threadIdx.x); p < e; p += kThreads)
-      if (!g.keep_col || g.keep_col[g.idx[p]]) agg ^= mix(mix(kFnvOffset, uint64_t(g.idx[p])), dbits(g.val[p] / pivot));
-    for (int off = 16; off; off >>= 1) agg ^= __shfl_xor_sync(0xffffffffu, agg, off);
-    if (lane == 0) atomicXor(&agg_shared, (unsigned long long)agg);
-    __syncthreads();
-    if (threadIdx.x == 0) g.out[i] = mix(h, agg_shared);
-    __syncthreads();
-    return;
-  }
-  const int chunks = int((int64_t(e) - from + kHashLoaders - 1) / kHashLoaders);
+  int chunks = 0;
+#pragma unroll
+  for (int r = 0; r < kHashRows; ++r)
+    chunks = max(chunks, int((int64_t(end_shared[r]) - from_shared[r] + kHashStage - 1) / kHashStage));
+  const bool folds = threadIdx.x < kHashRows;
+  const int row = folds ? int(threadIdx.x) : (int(threadIdx.x) - 32) / 28, slot = (int(threadIdx.x) - 32) % 28;
+  const offset_t from = row >= 0 && row < kHashRows ? from_shared[row] : 0;
+  const offset_t end = row >= 0 && row < kHashRows ? end_shared[row] : 0;
+  const double pivot = pivot_shared[row >= 0 && row < kHashRows ? row : 0];
+  uint64_t h = folds ? mix(kFnvOffset, uint64_t(len_shared[row])) : 0, agg = 0;
   for (int c = 0; c <= chunks; ++c) {
-    HashStage& next = stage[c & 1];
-    bool live = false;
-    uint64_t col = 0, bits = 0;
-    int rank = 0;
     if (warp > 0 && c < chunks) {
-      const int64_t p = int64_t(from) + int64_t(c) * kHashLoaders + (threadIdx.x - 32);
-      if (p < e) {
-        const int j = g.idx[p];
-        live = !g.keep_col || g.keep_col[j];
-        col = uint64_t(j);
-        if (live) bits = dbits(g.val[p] / pivot);
+      const int64_t base = int64_t(from) + int64_t(c) * kHashStage + slot;
+      int col[4];
+      double v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        col[k] = base + 28 * k < end ? __ldcs(g.idx + base + 28 * k) : -1;
+        v[k] = base + 28 * k < end ? __ldcs(g.val + base + 28 * k) : 0.0;
       }
-      const unsigned mask = __ballot_sync(0xffffffffu, live);
-      rank = __popc(mask & ((1u << lane) - 1u));
-      if (lane == 0) warp_live[warp] = __popc(mask);
+      if (g.keep_col) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (col[k] >= 0 && !g.keep_col[col[k]]) col[k] = -1;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        stage[c & 1].col[row][slot + 28 * k] = col[k];
+        stage[c & 1].bits[row][slot + 28 * k] = dbits(v[k] / pivot);
+      }
     }
-    __syncthreads();   // the loaders' counts; the fold of the stage before last is over
-    if (warp > 0 && c < chunks) {
-      int before = 0, all = 0;
-      for (int w = 1; w < kThreads / 32; ++w) {
-        before += w < warp ? warp_live[w] : 0;
-        all += warp_live[w];
-      }
-      if (live) {
-        next.col[before + rank] = col;
-        next.bits[before + rank] = bits;
-      }
-      if (threadIdx.x == 32) next.count = all;
-    }
-    if (threadIdx.x == 0 && c > 0) {
+    if (folds && c > 0) {
       const HashStage& last = stage[(c - 1) & 1];
-      const int n = last.count;
-#pragma unroll 4
-      for (int k = 0; k < n; ++k) h = mix(mix(h, last.col[k]), last.bits[k]);
+      const int n = int(min(int64_t(kHashStage), int64_t(end) - from - int64_t(c - 1) * kHashStage));
+#pragma unroll 8
+      for (int k = 0; k < n; ++k) {
+        const int32_t j = last.col[row][k];
+        const uint64_t b = last.bits[row][k];
+        if (j < 0) continue;
+        if (g.use_xor) agg ^= mix(mix(kFnvOffset, uint64_t(j)), b);
+        else h = mix(mix(h, uint64_t(j)), b);
+      }
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) g.out[i] = h;
+  if (folds && row < count && from < end) g.out[rows[row]] = g.use_xor ? mix(h, agg) : h;
+  __syncthreads();
 }
 
 // Four rows per warp, eight lanes (a group) per row, eight stored entries per
@@ -210,27 +205,43 @@ __device__ void row_hash_grouped(const RowHashArgs& g, int i) {
   }
 }
 
+// Blocks for the long rows, which take longest, then for the medium and the
+// short ones.
+struct HashRoles {
+  int long_blocks, medium_blocks, short_blocks;
+  int grid() const { return long_blocks + medium_blocks + short_blocks; }
+};
+HashRoles hash_roles(int rows, offset_t nnz) {
+  return HashRoles{int(std::min<int64_t>(kNumSMs * 2, int64_t(nnz) / (int64_t(kLongRow) * kHashRows) + 1)),
+                   int(std::min<int64_t>(kNumSMs * 8, (int64_t(rows) + 31) / 32)),
+                   grid_stride_blocks(rows, kThreads, 16)};
+}
+
 __global__ void __launch_bounds__(kThreads)
 row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
-                const int32_t* __restrict__ counts, int short_blocks) {
+                const int32_t* __restrict__ counts, HashRoles roles) {
   after_previous_kernel();
-  const int b = blockIdx.x;
-  if (b < short_blocks) {
-    for (int i = b * blockDim.x + threadIdx.x; i < rows; i += short_blocks * blockDim.x)
-      if (g.ptr[i + 1] - g.ptr[i] <= kShortRow) row_hash_thread(g, i);
+  __shared__ HashStage stage[2];
+  int b = blockIdx.x;
+  if (b < roles.long_blocks) {
+    const int count = counts[1];
+    for (int q = b * kHashRows; q < count; q += roles.long_blocks * kHashRows)
+      row_hash_block(g, longq + q, min(kHashRows, count - q), stage);
     return;
   }
-  // Long rows (> kLongRow stored entries) first, one to a block; then medium
-  // rows, four to a warp.
-  __shared__ HashStage stage[2];
-  for (int q = b - short_blocks; q < counts[1]; q += int(gridDim.x) - short_blocks) row_hash_block(g, longq[q], stage);
-  const int nwarps = (gridDim.x - short_blocks) * (kThreads / 32);
-  const int wid = (b - short_blocks) * (kThreads / 32) + (threadIdx.x >> 5);
-  const int nmedium = counts[0];
-  for (int q0 = wid * 4; q0 < nmedium; q0 += nwarps * 4) {
-    const int q = q0 + ((threadIdx.x & 31) >> 3);
-    row_hash_grouped(g, q < nmedium ? medium[q] : -1);
+  b -= roles.long_blocks;
+  if (b < roles.medium_blocks) {   // four rows to a warp
+    const int nwarps = roles.medium_blocks * (kThreads / 32);
+    const int nmedium = counts[0];
+    for (int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 4; q0 < nmedium; q0 += nwarps * 4) {
+      const int q = q0 + int((threadIdx.x & 31) >> 3);
+      row_hash_grouped(g, q < nmedium ? medium[q] : -1);
+    }
+    return;
   }
+  b -= roles.medium_blocks;
+  for (int i = b * int(blockDim.x) + int(threadIdx.x); i < rows; i += roles.short_blocks * int(blockDim.x))
+    if (g.ptr[i + 1] - g.ptr[i] <= kShortRow) row_hash_thread(g, i);
 }
 
 // Repeated-hash filter.  Only a hash that two or more live items share can
@@ -762,11 +773,11 @@ void parallel_row_hashes(const DevCsr& A, const uint8_t* keep_row, const uint8_t
     keep_row = ones.p;
   }
   const RowSchedule& sch = stored_schedule(A);
-  const int sb = grid_stride_blocks(A.rows, kThreads, 16), wb = std::min<int>(kNumSMs * 8, (A.rows + 7) / 8);
+  const HashRoles roles = hash_roles(A.rows, A.nnz);
   RowHashArgs g{A.ptr, A.idx, A.val, keep_row, keep_col, 1e-10, use_xor, hashes};
   const double bytes = 4.0 * (A.rows + 1) + 12.0 * A.nnz + A.rows + (keep_col ? A.cols : 0) + 8.0 * A.rows;
-  GPP_LAUNCH_BYTES(row_hash_kernel, bytes, sb + wb, kThreads, 0, s, A.rows, g, sch.medium.p, sch.long_rows.p,
-                   sch.counts.p, sb);
+  GPP_LAUNCH_BYTES(row_hash_kernel, bytes, roles.grid(), kThreads, 0, s, A.rows, g, sch.medium.p, sch.long_rows.p,
+                   sch.counts.p, roles);
 }
 
 void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp_params& p) {
@@ -779,11 +790,11 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
   {
     const bool use_xor = int64_t(lp.A.nnz) > 32LL * m;
     const RowSchedule& sch = stored_schedule(lp.A);
-    const int sb = grid_stride_blocks(m, kThreads, 16), wb = std::min<int>(kNumSMs * 8, (m + 7) / 8);
+    const HashRoles roles = hash_roles(m, lp.A.nnz);
     RowHashArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, plan.keep_col.p, p.zero_tol, use_xor, hash.p};
     const double bytes = 4.0 * (m + 1) + 12.0 * lp.A.nnz + m + lp.n() + 8.0 * m;
-    GPP_LAUNCH_BYTES(row_hash_kernel, bytes, sb + wb, kThreads, 0, s, m, g, sch.medium.p, sch.long_rows.p,
-                     sch.counts.p, sb);
+    GPP_LAUNCH_BYTES(row_hash_kernel, bytes, roles.grid(), kThreads, 0, s, m, g, sch.medium.p, sch.long_rows.p,
+                     sch.counts.p, roles);
   }
   DBuf<uint64_t> keys;
   DBuf<int32_t> ids;

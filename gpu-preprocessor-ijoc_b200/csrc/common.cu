@@ -43,9 +43,9 @@ Context::Context() {
   check(cudaMallocHost(reinterpret_cast<void**>(&host_scalar), 16), "cudaMallocHost scalar");
   check(cudaMallocHost(reinterpret_cast<void**>(&host_error), sizeof(int32_t)), "cudaMallocHost error");
   *host_error = 0;
-  check(cudaMallocHost(reinterpret_cast<void**>(&mail), sizeof(Mailbox) * (1 + kNnzBoxes)), "cudaMallocHost mail");
-  std::memset(static_cast<void*>(mail), 0, sizeof(Mailbox) * (1 + kNnzBoxes));
-  nnz_mail = mail + 1;
+  check(cudaMallocHost(reinterpret_cast<void**>(&mail), sizeof(Mailbox) * (kMailBoxes + kNnzBoxes)), "cudaMallocHost mail");
+  std::memset(static_cast<void*>(mail), 0, sizeof(Mailbox) * (kMailBoxes + kNnzBoxes));
+  nnz_mail = mail + kMailBoxes;
   check(cudaMalloc(reinterpret_cast<void**>(&report_words), sizeof(int32_t) * 16), "cudaMalloc report");
   check(cudaMemsetAsync(report_words, 0, sizeof(int32_t) * 16, stream), "report words");
 }
@@ -63,10 +63,12 @@ void Context::sync(const char* label) {
 }
 
 Report Context::open_report(int count) {
-  return Report{report_words, reinterpret_cast<unsigned int*>(report_words + 15), mail, ++mail_seq, count, false};
+  const uint32_t seq = open_mail();
+  return Report{report_words, reinterpret_cast<unsigned int*>(report_words + 15), box(seq), seq, count, false};
 }
 Report Context::open_report(int count, int32_t* words) {
-  return Report{words, reinterpret_cast<unsigned int*>(report_words + 15), mail, ++mail_seq, count, true};
+  const uint32_t seq = open_mail();
+  return Report{words, reinterpret_cast<unsigned int*>(report_words + 15), box(seq), seq, count, true};
 }
 
 void Context::poll(const Mailbox* box, uint32_t seq, int words, const char* where) {
@@ -322,8 +324,8 @@ void exclusive_scan_i32(const int32_t* in, int32_t* out, int64_t n, cudaStream_t
 }
 int32_t exclusive_scan_total(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s, const char* where) {
   auto& c = ctx();
-  Mailbox* mail = c.mail;
   const uint32_t seq = c.open_mail();
+  Mailbox* mail = c.box(seq);
   scan_items<int32_t, 1>(
       n, [in] __device__(int64_t i, int32_t(&v)[1]) { v[0] = in[i]; },
       [out] __device__(int64_t i, const int32_t(&before)[1], const int32_t(&)[1]) { out[i] = before[0]; },
@@ -337,8 +339,8 @@ int32_t exclusive_scan_total(const int32_t* in, int32_t* out, int64_t n, cudaStr
 std::pair<int64_t, int64_t> exclusive_scan_pair_i64(const int64_t* a, int64_t* a_out, const int64_t* b, int64_t* b_out,
                                                     int64_t n, cudaStream_t s, const char* where) {
   auto& c = ctx();
-  Mailbox* mail = c.mail;
   const uint32_t seq = c.open_mail();
+  Mailbox* mail = c.box(seq);
   scan_items<int64_t, 2>(
       n,
       [=] __device__(int64_t i, int64_t(&v)[2]) {

@@ -328,9 +328,11 @@ struct Context {
   // Row bits of the compaction (compact.cu), zero between compactions.
   uint2* row_bits = nullptr;
   size_t row_bits_words = 0;
-  // Mailbox of the kernels' answers and the words they gather them in; one
-  // question is open at a time (the host waits for its answer).
+  // Mailboxes of the kernels' answers, taken in turn (two questions may be open
+  // at once), and the words they gather them in, one kernel after the other.
+  static constexpr uint32_t kMailBoxes = 4;
   Mailbox* mail = nullptr;
+  Mailbox* box(uint32_t seq) { return mail + seq % kMailBoxes; }
   uint32_t mail_seq = 0;
   int32_t* report_words = nullptr;   // device: 15 words, then the block counter
   // Live-nnz answers, read some time after they were posted (Engine).

@@ -315,8 +315,8 @@ std::pair<int32_t, int32_t> build_old_to_new_pair(const uint8_t* keep_row, int32
                                                   cudaStream_t s) {
   // Both masks in one launch, as the prefix sums of m + n items.
   auto& c = ctx();
-  Mailbox* mail = c.mail;
   const uint32_t seq = c.open_mail();
+  Mailbox* mail = c.box(seq);
   scan_items<int32_t, 2>(
       int64_t(m) + n,
       [=] __device__(int64_t i, int32_t(&v)[2]) {

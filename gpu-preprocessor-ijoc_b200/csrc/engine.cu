@@ -455,9 +455,12 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
     }
     const bool tail = gate(kGateRedundantRowsDualFix, p.enable_infeasible_and_redundant_rows || p.enable_dual_fix);
     e.plan.row_kinds_current = false;
-    bool tail_changed = deferred(tail && p.enable_infeasible_and_redundant_rows, "infeasible_and_redundant_rows",
-                                 [&] { rule_redundant_rows(e.plan, cur, e.stats, p); });
-    tail_changed = deferred(tail && p.enable_dual_fix, "dual_fix", [&] { rule_dual_fix(e.plan, cur, e.stats, p); }) ||
+    DualFixTest ahead;
+    bool tail_changed =
+        deferred(tail && p.enable_infeasible_and_redundant_rows, "infeasible_and_redundant_rows",
+                 [&] { rule_redundant_rows(e.plan, cur, e.stats, p, p.enable_dual_fix ? &ahead : nullptr); });
+    tail_changed = deferred(tail && p.enable_dual_fix, "dual_fix",
+                            [&] { rule_dual_fix(e.plan, cur, e.stats, p, &ahead); }) ||
                    tail_changed;
     note(kGateRedundantRowsDualFix, tail_changed);
     return bounds_changed;

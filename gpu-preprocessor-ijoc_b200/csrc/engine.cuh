@@ -303,8 +303,17 @@ void rule_empty_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_
 void rule_singleton_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
-void rule_redundant_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
-void rule_dual_fix(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
+// Dual fixing's test of the columns, which the redundant-row rule may launch
+// behind its own (`asked`): it stands if that rule then acts on no row.
+struct DualFixTest {
+  DBuf<uint8_t> fixed, inf_fix;
+  DBuf<double> fval, contrib;
+  Report report;
+  bool asked = false;
+};
+void rule_redundant_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p,
+                         DualFixTest* ahead = nullptr);
+void rule_dual_fix(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p, DualFixTest* ahead = nullptr);
 // rules_startup.cu: structure-specific Startup rules.
 void rule_column_domination(Plan& plan, const WorkingLp& lp, const gpp_params& p);
 void rule_two_row_variable_elimination(Plan& plan, const WorkingLp& lp, const gpp_params& p);

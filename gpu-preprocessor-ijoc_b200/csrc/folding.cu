@@ -208,7 +208,7 @@ struct Side {
               const int32_t* other = nullptr, uint32_t seq = 0) {
     GPP_LAUNCH(fd_pack, grid_stride_blocks(n), kThreads, 0, s, n, ids.p, value, keys.p, perm.p);
     radix_sort_pairs(keys.p, perm.p, n, s, (bits_up_to(n) << 32) | 0xffffffffu);
-    Mailbox* mail = ctx().mail;
+    Mailbox* mail = ctx().box(seq);
     const uint64_t* sorted = keys.p;
     scan_items<int32_t, 1>(
         n, [sorted, tol] __device__(int64_t i, int32_t(&v)[1]) { v[0] = starts_color(sorted, i, tol); },
@@ -258,7 +258,7 @@ bool refine(const gpp_lp& lp, double tol, Side& rows, Side& cols, cudaStream_t s
   uint32_t seq = c.open_mail();
   cols.update(lp.u, tol, false, 0, s, rows.count.p, seq);
   {
-    const int64_t* counts = c.await(c.mail, seq, "colours");
+    const int64_t* counts = c.await(c.box(seq), seq, "colours");
     cols.colors = int(counts[0]);
     rows.colors = int(counts[1]);
   }
@@ -282,7 +282,7 @@ bool refine(const gpp_lp& lp, double tol, Side& rows, Side& cols, cudaStream_t s
     rows.refine(lp.A, cols.sig.p, tol, round_seed(round, 2), value, long_rows, s, rows_last ? cols.count.p : nullptr,
                 seq);
     if (rows_last || cols_last) {
-      const int64_t* counts = c.await(c.mail, seq, "colours");
+      const int64_t* counts = c.await(c.box(seq), seq, "colours");
       (rows_last ? rows : cols).colors = int(counts[0]);
       (rows_last ? cols : rows).colors = int(counts[1]);
     }

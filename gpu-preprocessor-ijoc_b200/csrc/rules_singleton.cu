@@ -777,13 +777,13 @@ void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats,
             rec[i] = int32_t(before[0]);
             spos[i] = before[1];
           },
-          [rec = rec.p + nelim, spos = spos.p + nelim, mail = ctx().mail, seq] __device__(const int64_t(&sum)[2]) {
+          [rec = rec.p + nelim, spos = spos.p + nelim, mail = ctx().box(seq), seq] __device__(const int64_t(&sum)[2]) {
             *rec = int32_t(sum[0]);
             *spos = sum[1];
             post_values(mail, seq, sum[0], sum[1]);
           },
           s);
-      const int64_t* sums = ctx().await(ctx().mail, seq, "substitution records");
+      const int64_t* sums = ctx().await(ctx().box(seq), seq, "substitution records");
       const int64_t recs = sums[0], support = sums[1];
       if (recs) {
         PostsolveSegment seg = make_segment(recs, 3 * recs + support, 6 * recs + support);

@@ -243,9 +243,9 @@ int32_t select_and_count(int64_t n, Pred pred, Emit emit, cudaStream_t s, const 
   LookbackSpace w(size_t(tiles), s);
   auto& c = ctx();
   const uint32_t seq = c.open_mail();
-  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, nullptr, c.mail, seq, w.words,
+  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, nullptr, c.box(seq), seq, w.words,
              w.counters, c.host_error);
-  return int32_t(c.await(c.mail, seq, where)[0]);
+  return int32_t(c.await(c.box(seq), seq, where)[0]);
 }
 
 }  // namespace gpp

@@ -419,10 +419,15 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
                             (p.enable_empty_columns ? kProbeEmptyColumns : 0u) |
                             (p.enable_empty_rows ? kProbeEmptyRows : 0u) |
                             (p.enable_singleton_rows ? kProbeSingletonRows : 0u);
+    // Singleton columns' test goes along with the probe (not under a time
+    // limit, which may end the round between the two).
+    const bool columns = gate(kGateSingletonColumns, p.enable_singleton_columns);
+    SingletonTest ahead;
     if (probed && !e.terminal && !time_exceeded()) {
       e.prepare();
       e.refresh();
-      may = cleanup_probe(e.plan, cur, e.stats, p, probed);
+      may = cleanup_probe(e.plan, cur, e.stats, p, probed, columns && !has_time_limit ? &ahead : nullptr);
+      if (may) ahead.asked = false;   // its kernels did nothing
     }
     bool quiet = true;
     auto step = [&](uint32_t bit, bool enabled, const char* name, auto rule) {
@@ -440,8 +445,8 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
     ch = step(kProbeSingletonRows, p.enable_singleton_rows, "singleton_rows",
               [&] { rule_singleton_rows(e.plan, cur, e.stats, p); }) || ch;
     ch = note(kGateSingletonColumns,
-              deferred(gate(kGateSingletonColumns, p.enable_singleton_columns), "singleton_columns",
-                       [&] { rule_singleton_columns(e.plan, cur, e.stats, p); })) || ch;
+              deferred(columns, "singleton_columns",
+                       [&] { rule_singleton_columns(e.plan, cur, e.stats, p, &ahead); })) || ch;
     return ch;
   };
   auto propagation = [&]() {

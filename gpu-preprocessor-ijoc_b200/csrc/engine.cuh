@@ -296,12 +296,35 @@ void capture_variable_pair(Record& r, VarPairRecovery&& step);
 constexpr int32_t kUnclaimedRow = INT32_MAX;   // Plan::sc_owner of a row without a candidate
 constexpr int kSingletonWords = 8;             // Plan::sc_words
 constexpr uint32_t kProbeFixed = 1, kProbeEmptyColumns = 2, kProbeEmptyRows = 4, kProbeSingletonRows = 8;
-uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules);
+// The singleton-column rule up to its one question, which the probe may ask
+// along with its own: where the probe finds nothing (most rounds) the rule runs
+// on the plan as it stands, so its kernels follow the probe's without a wait,
+// and on the device do nothing when the probe found something.  Up to
+// kFusedCleanup rows and columns probe and rule are one launch of one cluster.
+struct SingletonTest {
+  DBuf<int32_t> cand, rows, long_rows, winners;
+  DBuf<double> fmin, fmax, side, contrib_val;
+  DBuf<int4> counts;
+  DBuf<uint8_t> invalid, action, kind;
+  DBuf<int64_t> contrib_idx;
+  Report report;
+  bool asked = false, answered = false;
+  int64_t answer[kSingletonWords] = {};
+};
+constexpr int kFusedCleanup = 8192;
+struct ProbeArgs;
+void ask_singleton_columns(SingletonTest& t, Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p,
+                           const int32_t* gate);
+uint32_t probe_and_ask_singleton_columns(const ProbeArgs& probe, SingletonTest& t, Plan& plan, const WorkingLp& lp,
+                                         const Stats& stats, const gpp_params& p);
+uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules,
+                       SingletonTest* ahead = nullptr);
+void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p,
+                            SingletonTest* ahead = nullptr);
 void rule_fixed_variables(Plan& plan, const WorkingLp& lp, const gpp_params& p);
 void rule_empty_columns(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 void rule_empty_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 void rule_singleton_rows(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
-void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& s, const gpp_params& p);
 // Dual fixing's test of the columns, which the redundant-row rule may launch
 // behind its own (`asked`): it stands if that rule then acts on no row.

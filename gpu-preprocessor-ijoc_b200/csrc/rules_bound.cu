@@ -82,13 +82,18 @@ __device__ __forceinline__ void candidate_update(const CandArgs& g, const RowCtx
 constexpr int kTileRows = 2048;
 
 __global__ void __launch_bounds__(kThreads)
-candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, CandArgs g) {
+candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, int parts, CandArgs g) {
   after_previous_kernel();
   __shared__ offset_t sptr[kTileRows + 1];
   const L2Hints hint = l2_hints();
-  for (offset_t base = offset_t(blockIdx.x) * kEntryTile; base < nnz; base += offset_t(gridDim.x) * kEntryTile) {
-    const offset_t last = min(nnz, base + kEntryTile) - 1;
-    const int2 span = tile_rows[base / kEntryTile];   // rows of the tile's first and last entry
+  // A block takes a tile, or on small models one of its `parts` equal parts.
+  const int part_entries = kEntryTile / parts;
+  const int64_t tiles = (int64_t(nnz) + kEntryTile - 1) / kEntryTile;
+  for (int64_t w = blockIdx.x; w < tiles * parts; w += gridDim.x) {
+    if (w * part_entries >= nnz) break;   // block-uniform
+    const offset_t base = offset_t(w * part_entries);
+    const offset_t last = offset_t(min(int64_t(nnz), w * part_entries + part_entries) - 1);
+    const int2 span = tile_rows[w / parts];   // rows of the tile's first and last entry
     const int r0 = span.x, r1 = span.y;
     const bool staged = r1 - r0 + 1 <= kTileRows;
     if (staged)
@@ -96,7 +101,7 @@ candidates_entries(offset_t nnz, const int2* __restrict__ tile_rows, CandArgs g)
     __syncthreads();
     // The next entry's index and value are loaded one iteration ahead, so an
     // entry's critical path starts at its gather.
-    constexpr int K = kEntryTile / kThreads;
+    const int K = part_entries / kThreads;
     offset_t p = base + threadIdx.x;
     int j = p <= last ? ld_stream(g.idx + p, hint.stream) : -1;
     double a = p <= last ? ld_stream(g.val + p, hint.stream) : 0.0;
@@ -523,8 +528,13 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     CandArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.lu.p, rows, p.zero_tol, plan.cand_l.p, plan.cand_u.p};
     const double bytes = 4.0 * (m + 1) + 12.0 * lp.A.nnz + 33.0 * m + 16.0 * n + 16.0 * n;
     const RowSchedule& sch = stored_schedule(lp.A);
-    GPP_LAUNCH_BYTES(candidates_entries, bytes, int(std::max<int64_t>(1, std::min<int64_t>(sch.tiles, kNumSMs * 8))),
-                     kThreads, 0, s, lp.A.nnz, sch.tile_rows.p, g);
+    // Small models have fewer tiles than the GPU has room for blocks: parts of
+    // tiles then, down to one entry a thread (18 us a sweep of a 10,000-entry
+    // model with whole tiles, eight dependent rounds).
+    int parts = 1;
+    while (parts < kEntryTile / kThreads && sch.tiles * parts * 2 <= kNumSMs * 8) parts *= 2;
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(sch.tiles * parts, kNumSMs * 8));
+    GPP_LAUNCH_BYTES(candidates_entries, bytes, int(blocks), kThreads, 0, s, lp.A.nnz, sch.tile_rows.p, parts, g);
   }
   // Column maxima depend on the kept rows alone: rounds that only move bounds
   // share one sweep.

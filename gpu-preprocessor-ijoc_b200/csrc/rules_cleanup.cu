@@ -6,6 +6,7 @@
 // Reference: rules/rule_infeasible_and_fixed_variables.cu:65-348,
 // rules/empty_rows_and_columns/columns.cu:64-249, rows.cu:26-121,
 // rules/rule_singleton_rows.cu:76-275.
+#include "cleanup_probe.cuh"
 #include "engine.cuh"
 
 namespace gpp {
@@ -246,53 +247,20 @@ double domain_objective(const double* contrib, const uint8_t* entry_keep, int32_
 }
 
 namespace {
-// What the first checks of the four rules below find on the current plan, in
-// one pass: a thread reads one column and one row and flags the rules that may
-// act.
-//  - fixed variables: a kept column whose finite bounds lie within bound_tol;
-//  - empty columns: any kept empty column (fixed, infeasible or unbounded);
-//  - empty rows: any kept row without live entries;
-//  - singleton rows: a row that gives a bound, or, when there is none (the
-//    candidate bounds are then the columns' own), a column whose bounds cross
-//    by more than bound_tol or are NaN.
-// Bound by its reads, 18 bytes a column and 6 a row; the four detection kernels
-// of the rules, which also fill the arrays that the rules go on with, took 7
-// launches and copies and about 230 bytes a column.
-__global__ void __launch_bounds__(kThreads)
-cleanup_probe_kernel(int m, int n, uint32_t rules, const uint8_t* __restrict__ keep_row,
-                     const uint8_t* __restrict__ keep_col, const double* __restrict__ l, const double* __restrict__ u,
-                     const uint8_t* __restrict__ empty_col, const int32_t* __restrict__ row_nnz,
-                     const uint8_t* __restrict__ singleton_row, const int32_t* __restrict__ scol,
-                     const double* __restrict__ sval, double bound_tol, double zero_tol, int32_t* __restrict__ sc_owner,
-                     int32_t* __restrict__ sc_words, Report report) {
+// The probe by itself.  The last block also leaves what was found for the
+// singleton columns' kernels launched behind it, which do nothing then.
+__global__ void __launch_bounds__(kThreads) cleanup_probe_kernel(ProbeArgs g, Report report) {
   after_previous_kernel();
-  uint32_t f = 0;
-  // The singleton-column rule's scratch, which it needs cleared.
-  if (blockIdx.x == 0 && threadIdx.x < kSingletonWords) sc_words[threadIdx.x] = 0;
-  const int top = n > m ? n : m;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < top; k += gridDim.x * blockDim.x) {
-    if (k < n) {
-      const double lj = l[k], uj = u[k];
-      if (keep_col[k]) {
-        if (isfinite(lj) && isfinite(uj) && lj <= uj && uj - lj <= bound_tol) f |= kProbeFixed;
-        if (empty_col[k]) f |= kProbeEmptyColumns;
-      }
-      if (lj > uj + bound_tol || lj != lj || uj != uj) f |= kProbeSingletonRows;
-    }
-    if (k < m) sc_owner[k] = kUnclaimedRow;
-    if (k < m && keep_row[k]) {
-      if (row_nnz[k] == 0) f |= kProbeEmptyRows;
-      if (singleton_row[k]) {
-        const int col = scol[k];
-        if (col >= 0 && col < n && fabs(sval[k]) > zero_tol) f |= kProbeSingletonRows;
-      }
-    }
-  }
-  post_flags(report, f & rules);
+  if (blockIdx.x == 0 && threadIdx.x < kSingletonWords) g.sc_words[threadIdx.x] = 0;
+  gather_flags(report, probe_part(g));
+  if (!last_to_report(report)) return;
+  if (threadIdx.x == 0) g.sc_words[kSingletonWords] = __ldcg(report.words);
+  post_words(report);
 }
 }  // namespace
 
-uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules) {
+uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p, uint32_t rules,
+                       SingletonTest* ahead) {
   // The first-stage detections of the four rules below, on the current plan,
   // with one launch and one readback; a rule whose detection finds nothing
   // (no candidate, no infeasibility) returns without touching the plan.
@@ -303,13 +271,17 @@ uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, cons
   if (!rules) return 0;
   auto s = ctx().stream;
   if (plan.sc_owner.n < size_t(m)) plan.sc_owner.alloc(size_t(m), s);
-  if (!plan.sc_words.p) plan.sc_words.alloc(kSingletonWords, s);
+  if (!plan.sc_words.p) plan.sc_words.alloc(kSingletonWords + 1, s);
   plan.sc_ready = true;
+  const ProbeArgs g{m, n, rules, plan.keep_row.p, plan.keep_col.p, plan.l.p, plan.u.p, stats.empty_col.p,
+                    stats.row_nnz.p, stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol,
+                    plan.sc_owner.p, plan.sc_words.p};
+  if (ahead && (n == 0 || m == 0)) ahead = nullptr;
+  if (ahead && std::max(n, m) <= kFusedCleanup) return probe_and_ask_singleton_columns(g, *ahead, plan, lp, stats, p);
   const Report report = ctx().open_report(1);
-  GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 10.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, m, n,
-                   rules, plan.keep_row.p, plan.keep_col.p, plan.l.p, plan.u.p, stats.empty_col.p, stats.row_nnz.p,
-                   stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol, plan.sc_owner.p,
-                   plan.sc_words.p, report);
+  GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 10.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, g,
+                   report);
+  if (ahead) ask_singleton_columns(*ahead, plan, lp, stats, p, plan.sc_words.p + kSingletonWords);
   return uint32_t(ctx().await(report)[0]);
 }
 

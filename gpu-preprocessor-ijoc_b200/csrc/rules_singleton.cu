@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <climits>
 
+#include "cleanup_probe.cuh"
 #include "engine.cuh"
 #include "live_visit.cuh"
 #include "scan.cuh"
@@ -52,41 +53,66 @@ __device__ __forceinline__ bool direct_unbounded(double cj, double a, double lhs
          (cj < -zt && a > zt && !isfinite(rhs) && !isfinite(ub));
 }
 
+// What the rule's kernels read, and the lists and scratch that one writes and
+// the next reads (no `__restrict__`: the fused kernel runs all four).
+struct ScArgs {
+  int n, m, row_blocks, long_blocks;
+  const uint8_t* singleton;
+  const int32_t* srow;
+  const double* sval;
+  const int32_t* row_nnz;
+  const double *c, *l, *u;
+  const double2* lu;
+  const offset_t* ptr;
+  const int32_t* idx;
+  const double* val;
+  double tol, zero_tol;
+  double *AL, *AU;
+  uint8_t *keep_row, *keep_col;
+  int32_t *owner, *cand, *rows, *long_rows, *st, *winners;
+  double *fmin, *fmax;
+  int4* counts;
+  uint8_t *invalid, *action, *kind;
+  double *side, *contrib_val;
+  int64_t* contrib_idx;
+};
+
 // Candidates (:905-940): kept singleton column in a kept row with another
 // live entry and |a| > zero_tol.  Directly unbounded candidates only raise the
 // flag.  The first candidate of a row claims it for the cache and stage lists.
-__global__ void sc_candidates(int n, int m, const uint8_t* __restrict__ keep_col, const uint8_t* __restrict__ keep_row,
-                              const uint8_t* __restrict__ singleton, const int32_t* __restrict__ srow,
-                              const double* __restrict__ sval, const int32_t* __restrict__ row_nnz,
-                              const double* __restrict__ c, const double* __restrict__ l, const double* __restrict__ u,
-                              const double* __restrict__ AL, const double* __restrict__ AU, double zero_tol,
-                              int32_t* __restrict__ owner, int32_t* __restrict__ cand, int32_t* __restrict__ rows,
-                              int32_t* __restrict__ long_rows, int32_t* st) {
-  after_previous_kernel();
+__device__ __forceinline__ void sc_candidates_part(const ScArgs& g) {
+  const int n = g.n, m = g.m;
+  const double zero_tol = g.zero_tol;
+  int32_t* const st = g.st;
   const int stride = gridDim.x * blockDim.x;
   const int top = (n + stride - 1) / stride * stride;   // every thread of a block runs the same trips
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < top; j += stride) {
     bool take = false, claim = false, is_long = false;
-    if (j < n && keep_col[j] && singleton[j]) {
-      const int row = srow[j];
-      const double a = sval[j];
-      if (row >= 0 && row < m && keep_row[row] && !(fabs(a) <= zero_tol) && row_nnz[row] > 1) {
-        if (direct_unbounded(c[j], a, AL[row], AU[row], l[j], u[j], zero_tol)) {
+    if (j < n && g.keep_col[j] && g.singleton[j]) {
+      const int row = g.srow[j];
+      const double a = g.sval[j];
+      if (row >= 0 && row < m && g.keep_row[row] && !(fabs(a) <= zero_tol) && g.row_nnz[row] > 1) {
+        if (direct_unbounded(g.c[j], a, g.AL[row], g.AU[row], g.l[j], g.u[j], zero_tol)) {
           atomicOr(st + kStUnbounded, 1);
         } else {
           take = true;
-          claim = atomicCAS(owner + row, kUnclaimed, kClaimed) == kUnclaimed;
-          is_long = claim && row_nnz[row] > kLongRow;
+          claim = atomicCAS(g.owner + row, kUnclaimed, kClaimed) == kUnclaimed;
+          is_long = claim && g.row_nnz[row] > kLongRow;
         }
       }
     }
     const int pc = block_append(st + kStCand, take);
-    if (take) cand[pc] = j;
+    if (take) g.cand[pc] = j;
     const int pr = block_append(st + kStRows, claim);
-    if (claim) rows[pr] = srow[j];
+    if (claim) g.rows[pr] = g.srow[j];
     const int pl = block_append(st + kStLong, is_long);
-    if (is_long) long_rows[pl] = srow[j];
+    if (is_long) g.long_rows[pl] = g.srow[j];
   }
+}
+__global__ void __launch_bounds__(kThreads) sc_candidates(ScArgs g, const int32_t* gate) {
+  after_previous_kernel();
+  if (gate && *gate) return;   // the lists stay empty for the kernels behind
+  sc_candidates_part(g);
 }
 
 struct RowCache {
@@ -148,7 +174,7 @@ struct CacheBounds {
 // each, four rows per warp, with all of a row's loads issued before its
 // chain; longer rows take a whole warp, 32 entries at a time.
 template <bool kPacked>
-__device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, const int32_t* __restrict__ st,
+__device__ void sc_cache_rows(int blocks, const int32_t* rows, const int32_t* st,
                               const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
                               const int32_t* __restrict__ idx, const double* __restrict__ val,
                               CacheBounds<kPacked> bounds, CacheOut out) {
@@ -278,8 +304,8 @@ __device__ void sc_cache_rows(int blocks, const int32_t* __restrict__ rows, cons
 // _kernel_singleton_long_row_activity_cache (:642-754): block per row; live
 // rank k goes to thread k mod 256, then a shared-memory halving tree.
 template <bool kPacked>
-__device__ void sc_cache_long(int block, int blocks, const int32_t* __restrict__ long_rows,
-                              const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz,
+__device__ void sc_cache_long(int block, int blocks, const int32_t* long_rows,
+                              const int32_t* st, const int32_t* __restrict__ row_nnz,
                               const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                               const double* __restrict__ val, CacheBounds<kPacked> bounds, CacheOut out) {
   __shared__ int slots[kThreads];
@@ -323,48 +349,44 @@ __device__ void sc_cache_long(int block, int blocks, const int32_t* __restrict__
 // not know their numbers (the rule asks the host once, at its end); blocks
 // without rows return at once.
 template <bool kPacked>
-__global__ void __launch_bounds__(kThreads)
-sc_cache(int row_blocks, const int32_t* __restrict__ rows, const int32_t* __restrict__ long_rows,
-         const int32_t* __restrict__ st, const int32_t* __restrict__ row_nnz, const offset_t* __restrict__ ptr,
-         const int32_t* __restrict__ idx, const double* __restrict__ val, CacheBounds<kPacked> bounds, CacheOut out) {
+__device__ __forceinline__ CacheBounds<kPacked> cache_bounds(const ScArgs& g) {
+  return CacheBounds<kPacked>{g.lu, g.keep_col, g.l, g.u};
+}
+template <bool kPacked>
+__global__ void __launch_bounds__(kThreads) sc_cache(ScArgs g) {
   after_previous_kernel();
-  if (int(blockIdx.x) < row_blocks)
-    sc_cache_rows(row_blocks, rows, st, row_nnz, ptr, idx, val, bounds, out);
+  const CacheOut out{g.fmin, g.fmax, g.counts, g.invalid};
+  if (int(blockIdx.x) < g.row_blocks)
+    sc_cache_rows(g.row_blocks, g.rows, g.st, g.row_nnz, g.ptr, g.idx, g.val, cache_bounds<kPacked>(g), out);
   else
-    sc_cache_long(int(blockIdx.x) - row_blocks, int(gridDim.x) - row_blocks, long_rows, st, row_nnz, ptr, idx, val,
-                  bounds, out);
+    sc_cache_long(int(blockIdx.x) - g.row_blocks, g.long_blocks, g.long_rows, g.st, g.row_nnz, g.ptr, g.idx, g.val,
+                  cache_bounds<kPacked>(g), out);
 }
 
 // Propose (:905-1018) over the candidate list.
-__global__ void sc_propose(const int32_t* __restrict__ cand, const int32_t* __restrict__ st,
-                           const int32_t* __restrict__ srow, const double* __restrict__ sval,
-                           const double* __restrict__ c, const double* __restrict__ l, const double* __restrict__ u,
-                           const double* __restrict__ AL, const double* __restrict__ AU,
-                           const double* __restrict__ cache_min, const double* __restrict__ cache_max,
-                           const int4* __restrict__ counts, const uint8_t* __restrict__ invalid, double tol,
-                           double zero_tol, uint8_t* __restrict__ action, double* __restrict__ side,
-                           int32_t* __restrict__ owner) {
-  after_previous_kernel();
+__device__ __forceinline__ void sc_propose_part(const ScArgs& g) {
+  const int32_t* const st = g.st;
+  const double tol = g.tol, zero_tol = g.zero_tol;
   const int count = st[kStCand];
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-    const int j = cand[q];
-    const int row = srow[j];
-    const double a = sval[j];
-    const double lj = l[j], uj = u[j], cj = c[j];
+    const int j = g.cand[q];
+    const int row = g.srow[j];
+    const double a = g.sval[j];
+    const double lj = g.l[j], uj = g.u[j], cj = g.c[j];
     // _singleton_column_activity_bounds_from_cache (:756-816).
-    if (invalid[row]) continue;
+    if (g.invalid[row]) continue;
     const double tmin = a >= 0.0 ? a * lj : a * uj;
     const double tmax = a >= 0.0 ? a * uj : a * lj;
     if (isnan(tmin) || isnan(tmax)) continue;
-    int4 k = counts[row];
-    double vmin = cache_min[row], vmax = cache_max[row];
+    int4 k = g.counts[row];
+    double vmin = g.fmin[row], vmax = g.fmax[row];
     if (isinf(tmin)) { if (tmin < 0.0) --k.x; else --k.y; } else { vmin -= tmin; }
     if (isinf(tmax)) { if (tmax < 0.0) --k.z; else --k.w; } else { vmax -= tmax; }
     if (k.x < 0 || k.y < 0 || k.z < 0 || k.w < 0 || (k.x > 0 && k.y > 0) || (k.z > 0 && k.w > 0)) continue;
     const double rmin = k.x > 0 ? -INFINITY : (k.y > 0 ? INFINITY : vmin);
     const double rmax = k.z > 0 ? -INFINITY : (k.w > 0 ? INFINITY : vmax);
     if (isnan(rmin) || isnan(rmax)) continue;
-    const double lhs = AL[row], rhs = AU[row];
+    const double lhs = g.AL[row], rhs = g.AU[row];
     uint8_t act = kNone;
     double sd = 0.0;
     if (isfinite(lhs) && isfinite(rhs) && fabs(lhs - rhs) <= tol) {
@@ -407,23 +429,23 @@ __global__ void sc_propose(const int32_t* __restrict__ cand, const int32_t* __re
         continue;
       }
     }
-    action[j] = act;
-    side[j] = sd;
-    atomicMin(owner + row, act == kEliminateFree ? j - INT_MAX : j);
+    g.action[j] = act;
+    g.side[j] = sd;
+    atomicMin(g.owner + row, act == kEliminateFree ? j - INT_MAX : j);
   }
+}
+__global__ void __launch_bounds__(kThreads) sc_propose(ScArgs g) {
+  after_previous_kernel();
+  sc_propose_part(g);
 }
 
 // Stage + commit (:1021-1073, :1157-1189) over the claimed rows.  Every read
 // is of the owner's own row and column, so the plan is updated in place; the
 // row keeps its owner in `owner` only when the owner column is eliminated.
-__global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, const uint8_t* __restrict__ action,
-                         const double* __restrict__ side, const double* __restrict__ sval,
-                         const double* __restrict__ c, const double* __restrict__ l, const double* __restrict__ u,
-                         double* __restrict__ AL, double* __restrict__ AU, double tol, int32_t* __restrict__ owner,
-                         uint8_t* __restrict__ keep_row, uint8_t* __restrict__ keep_col, uint8_t* __restrict__ kind,
-                         int32_t* __restrict__ winners, int64_t* __restrict__ contrib_idx,
-                         double* __restrict__ contrib_val, Report report) {
-  after_previous_kernel();
+__device__ __forceinline__ void sc_stage_part(const ScArgs& g) {
+  int32_t* const st = g.st;
+  const int n = g.n;
+  const double tol = g.tol;
   // An unbounded candidate ends the rule with the plan as it was.
   const int count = st[kStUnbounded] ? 0 : st[kStRows];
   const int stride = gridDim.x * blockDim.x;
@@ -433,58 +455,97 @@ __global__ void sc_stage(const int32_t* __restrict__ rows, int32_t* st, int n, c
     uint8_t k = 0;
     double contrib = 0.0;
     if (q < count) {
-      row = rows[q];
-      const int key = owner[row];
+      row = g.rows[q];
+      const int key = g.owner[row];
       j = key < 0 ? key + INT_MAX : key;
       if (j >= 0 && j < n) {
-        const uint8_t act = action[j];
-        const double lhs = AL[row], rhs = AU[row];
+        const uint8_t act = g.action[j];
+        const double lhs = g.AL[row], rhs = g.AU[row];
         if (act == kEliminateFree || act == kEliminateFreeAbove || act == kEliminateFreeBelow) {
-          const double a = sval[j];
-          contrib = c[j] * rhs / a;
+          const double a = g.sval[j];
+          contrib = g.c[j] * rhs / a;
           if (act == kEliminateFree) {
-            keep_row[row] = 0;
+            g.keep_row[row] = 0;
             k = kRowElimDeleted;
           } else {
             const bool above = act == kEliminateFreeAbove;
-            const double bound = above ? l[j] : u[j];
+            const double bound = above ? g.l[j] : g.u[j];
             const bool keep_lower = above ? a < 0.0 : a > 0.0;
             const double shifted = rhs - a * bound;
-            if (keep_lower) { AL[row] = shifted; AU[row] = INFINITY; }
-            else { AL[row] = -INFINITY; AU[row] = shifted; }
+            if (keep_lower) { g.AL[row] = shifted; g.AU[row] = INFINITY; }
+            else { g.AL[row] = -INFINITY; g.AU[row] = shifted; }
             k = kRowElimKept;
           }
-          keep_col[j] = 0;
-          owner[row] = j;
+          g.keep_col[j] = 0;
+          g.owner[row] = j;
         } else {
           bool lo = false, hi = false;
-          const double sd = side[j];
+          const double sd = g.side[j];
           if (act == kSetRowSide) {
             lo = !isfinite(lhs) || fabs(lhs - sd) > tol;
             hi = !isfinite(rhs) || fabs(rhs - sd) > tol;
-            AL[row] = sd;
-            AU[row] = sd;
+            g.AL[row] = sd;
+            g.AU[row] = sd;
           } else if (act == kTightenLhs) {
             lo = true;
-            AL[row] = rhs;
+            g.AL[row] = rhs;
           } else if (act == kTightenRhs) {
             hi = true;
-            AU[row] = lhs;
+            g.AU[row] = lhs;
           }
           atomicOr(st + kStSide, 1);
           if (lo || hi) k = kRowDualShift;
-          owner[row] = kUnclaimed;
+          g.owner[row] = kUnclaimed;
         }
       } else {
-        owner[row] = kUnclaimed;
+        g.owner[row] = kUnclaimed;
       }
-      if (k) kind[row] = k;
+      if (k) g.kind[row] = k;
     }
     const bool elim = k == kRowElimKept || k == kRowElimDeleted;
     const int pe = block_append(st + kStElim, elim);
-    if (elim) { contrib_idx[pe] = j; contrib_val[pe] = contrib; }
+    if (elim) { g.contrib_idx[pe] = j; g.contrib_val[pe] = contrib; }
     const int pw = block_append(st + kStWin, k != 0);
-    if (k) winners[pw] = row;
+    if (k) g.winners[pw] = row;
+  }
+}
+__global__ void __launch_bounds__(kThreads) sc_stage(ScArgs g, Report report) {
+  after_previous_kernel();
+  sc_stage_part(g);
+  post_report(report);
+}
+
+// Probe and rule as one cluster, for models whose kernels are shorter than
+// their launches: the cluster's barrier stands where a launch did.  Its blocks
+// are scheduled together, so nothing spins.  At 2,000 x 5,000 the five launches
+// and two waits took about 52 us.
+constexpr int kCleanupCluster = 8;
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <bool kPacked>
+__global__ void __cluster_dims__(kCleanupCluster, 1, 1) __launch_bounds__(kThreads)
+probe_and_singleton_columns(ProbeArgs probe, ScArgs g, Report report) {
+  after_previous_kernel();
+  if (blockIdx.x == 0 && threadIdx.x <= kSingletonWords) g.st[threadIdx.x] = 0;
+  const uint32_t found = probe_part(probe);
+  cluster_barrier();   // words and owners are cleared
+  Report probed = report;
+  probed.words = g.st + kSingletonWords;
+  gather_flags(probed, found);
+  cluster_barrier();
+  if (*static_cast<volatile int32_t*>(probed.words) == 0) {   // the same in every block
+    sc_candidates_part(g);
+    cluster_barrier();
+    const CacheOut out{g.fmin, g.fmax, g.counts, g.invalid};
+    sc_cache_rows(kCleanupCluster, g.rows, g.st, g.row_nnz, g.ptr, g.idx, g.val, cache_bounds<kPacked>(g), out);
+    sc_cache_long(int(blockIdx.x), kCleanupCluster, g.long_rows, g.st, g.row_nnz, g.ptr, g.idx, g.val,
+                  cache_bounds<kPacked>(g), out);
+    cluster_barrier();
+    sc_propose_part(g);
+    cluster_barrier();
+    sc_stage_part(g);
   }
   post_report(report);
 }
@@ -688,55 +749,123 @@ __global__ void sc_winner_keys(const int32_t* __restrict__ winners, int count, c
 
 }  // namespace
 
-void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p) {
+namespace {
+ScArgs singleton_args(SingletonTest& t, Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p) {
+  const int m = lp.m(), n = lp.n();
+  auto s = ctx().stream;
+  const int claims = std::min(m, n);   // at most: one per row and per candidate
+  t.cand.alloc(size_t(n), s);
+  t.rows.alloc(size_t(m), s);
+  t.long_rows.alloc(size_t(m), s);
+  t.winners.alloc(size_t(claims), s);
+  t.fmin.alloc(size_t(m), s);
+  t.fmax.alloc(size_t(m), s);
+  t.side.alloc(size_t(n), s);
+  t.contrib_val.alloc(size_t(claims), s);
+  t.counts.alloc(size_t(m), s);
+  t.invalid.alloc(size_t(m), s);
+  t.action.alloc(size_t(n), s);
+  t.kind.alloc(size_t(m), s);
+  t.contrib_idx.alloc(size_t(claims), s);
+  ScArgs g{};
+  g.n = n;
+  g.m = m;
+  g.row_blocks = std::max(1, std::min((claims + 31) / 32, kNumSMs * 16));
+  g.long_blocks = std::max(1, std::min(kNumSMs * 4, int(lp.A.nnz / kLongRow)));
+  g.singleton = stats.singleton_col.p;
+  g.srow = stats.scol_row.p;
+  g.sval = stats.scol_val.p;
+  g.row_nnz = stats.row_nnz.p;
+  g.c = plan.c.p;
+  g.l = plan.l.p;
+  g.u = plan.u.p;
+  g.lu = plan.lu.p;
+  g.ptr = lp.A.ptr;
+  g.idx = lp.A.idx;
+  g.val = lp.A.val;
+  g.tol = p.bound_tol;
+  g.zero_tol = p.zero_tol;
+  g.AL = plan.AL.p;
+  g.AU = plan.AU.p;
+  g.keep_row = plan.keep_row.p;
+  g.keep_col = plan.keep_col.p;
+  g.owner = plan.sc_owner.p;
+  g.st = plan.sc_words.p;
+  g.cand = t.cand.p;
+  g.rows = t.rows.p;
+  g.long_rows = t.long_rows.p;
+  g.winners = t.winners.p;
+  g.fmin = t.fmin.p;
+  g.fmax = t.fmax.p;
+  g.counts = t.counts.p;
+  g.invalid = t.invalid.p;
+  g.action = t.action.p;
+  g.kind = t.kind.p;
+  g.side = t.side.p;
+  g.contrib_val = t.contrib_val.p;
+  g.contrib_idx = t.contrib_idx.p;
+  return g;
+}
+}  // namespace
+
+void ask_singleton_columns(SingletonTest& t, Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p,
+                           const int32_t* gate) {
+  const int m = lp.m(), n = lp.n();
+  auto s = ctx().stream;
+  const ScArgs g = singleton_args(t, plan, lp, stats, p);
+  GPP_LAUNCH_BYTES(sc_candidates, double(n) * 11 + 16.0 * n, grid_stride_blocks(n), kThreads, 0, s, g, gate);
+  // Activity cache of the claimed rows, proposals and their staging follow with
+  // no wait between: the kernels read the candidate and row counts on the
+  // device, and the one answer, after the staging, tells what the rule did.
+  if (plan.bounds_mirrored) GPP_LAUNCH(sc_cache<true>, g.row_blocks + g.long_blocks, kThreads, 0, s, g);
+  else GPP_LAUNCH(sc_cache<false>, g.row_blocks + g.long_blocks, kThreads, 0, s, g);
+  GPP_LAUNCH(sc_propose, grid_stride_blocks(n), kThreads, 0, s, g);
+  t.report = ctx().open_report(kStWords, g.st);
+  GPP_LAUNCH(sc_stage, grid_stride_blocks(std::min(m, n)), kThreads, 0, s, g, t.report);
+  t.asked = true;
+}
+
+uint32_t probe_and_ask_singleton_columns(const ProbeArgs& probe, SingletonTest& t, Plan& plan, const WorkingLp& lp,
+                                         const Stats& stats, const gpp_params& p) {
+  auto s = ctx().stream;
+  const ScArgs g = singleton_args(t, plan, lp, stats, p);
+  const Report report = ctx().open_report(kStWords + 1, g.st);
+  if (plan.bounds_mirrored)
+    GPP_LAUNCH(probe_and_singleton_columns<true>, kCleanupCluster, kThreads, 0, s, probe, g, report);
+  else
+    GPP_LAUNCH(probe_and_singleton_columns<false>, kCleanupCluster, kThreads, 0, s, probe, g, report);
+  const int64_t* f = ctx().await(report);
+  std::copy(f, f + kStWords, t.answer);
+  t.asked = t.answered = true;
+  return uint32_t(f[kStWords]);
+}
+
+void rule_singleton_columns(Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p,
+                            SingletonTest* ahead) {
   if (plan.has_infeasible || plan.has_unbounded || !p.enable_singleton_columns) return;
   const int m = lp.m(), n = lp.n();
   if (m == 0 || n == 0) return;
   auto s = ctx().stream;
-  DBuf<int32_t> cand(size_t(n), s), rows(size_t(m), s), long_rows(size_t(m), s);
-  if (!plan.sc_ready) {
-    if (plan.sc_owner.n < size_t(m)) plan.sc_owner.alloc(size_t(m), s);
-    if (!plan.sc_words.p) plan.sc_words.alloc(kSingletonWords, s);
-    GPP_LAUNCH(sc_start, grid_stride_blocks(m), kThreads, 0, s, plan.sc_owner.p, m, kUnclaimed, plan.sc_words.p);
+  SingletonTest own;
+  SingletonTest& t = ahead && ahead->asked ? *ahead : own;
+  if (!t.asked) {
+    if (!plan.sc_ready) {
+      if (plan.sc_owner.n < size_t(m)) plan.sc_owner.alloc(size_t(m), s);
+      if (!plan.sc_words.p) plan.sc_words.alloc(kSingletonWords + 1, s);
+      GPP_LAUNCH(sc_start, grid_stride_blocks(m), kThreads, 0, s, plan.sc_owner.p, m, kUnclaimed, plan.sc_words.p);
+    }
+    ask_singleton_columns(t, plan, lp, stats, p, nullptr);
   }
   plan.sc_ready = false;
   DBuf<int32_t>& owner = plan.sc_owner;
   int32_t* const st = plan.sc_words.p;
-  GPP_LAUNCH_BYTES(sc_candidates, double(n) * 11 + 16.0 * n, grid_stride_blocks(n), kThreads, 0, s, n, m,
-                   plan.keep_col.p, plan.keep_row.p, stats.singleton_col.p, stats.scol_row.p, stats.scol_val.p,
-                   stats.row_nnz.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.zero_tol, owner.p, cand.p,
-                   rows.p, long_rows.p, st);
-
-  // Activity cache of the claimed rows, proposals and their staging follow with
-  // no wait between: the kernels read the candidate and row counts on the
-  // device, and the one answer, after the staging, tells what the rule did.
-  const int claims = std::min(m, n);   // at most: one per row and per candidate
-  DBuf<double> fmin(size_t(m), s), fmax(size_t(m), s);
-  DBuf<int4> counts(size_t(m), s);
-  DBuf<uint8_t> invalid(size_t(m), s);
-  const CacheOut cache{fmin.p, fmax.p, counts.p, invalid.p};
-  const int row_blocks = std::max(1, std::min((claims + 31) / 32, kNumSMs * 16));
-  const int long_blocks = std::max(1, std::min(kNumSMs * 4, int(lp.A.nnz / kLongRow)));
-  const auto fill_cache = [&](auto packed) {
-    constexpr bool kPacked = decltype(packed)::value;
-    const CacheBounds<kPacked> bounds{plan.lu.p, plan.keep_col.p, plan.l.p, plan.u.p};
-    GPP_LAUNCH(sc_cache<kPacked>, row_blocks + long_blocks, kThreads, 0, s, row_blocks, rows.p, long_rows.p, st,
-               stats.row_nnz.p, lp.A.ptr, lp.A.idx, lp.A.val, bounds, cache);
-  };
-  if (plan.bounds_mirrored) fill_cache(std::true_type{});
-  else fill_cache(std::false_type{});
-  DBuf<uint8_t> action(size_t(n), s), kind(size_t(m), s);
-  DBuf<double> side(size_t(n), s), contrib_val(size_t(claims), s);
-  DBuf<int64_t> contrib_idx(size_t(claims), s);
-  DBuf<int32_t> winners(size_t(claims), s);
-  GPP_LAUNCH(sc_propose, grid_stride_blocks(n), kThreads, 0, s, cand.p, st, stats.scol_row.p, stats.scol_val.p,
-             plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, fmin.p, fmax.p, counts.p, invalid.p, p.bound_tol,
-             p.zero_tol, action.p, side.p, owner.p);
-  const Report report = ctx().open_report(kStWords, st);
-  GPP_LAUNCH(sc_stage, grid_stride_blocks(claims), kThreads, 0, s, rows.p, st, n, action.p, side.p,
-             stats.scol_val.p, plan.c.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, p.bound_tol, owner.p,
-             plan.keep_row.p, plan.keep_col.p, kind.p, winners.p, contrib_idx.p, contrib_val.p, report);
-  const int64_t* f = ctx().await(report);
+  const int claims = std::min(m, n);
+  DBuf<int32_t>& winners = t.winners;
+  DBuf<uint8_t>& kind = t.kind;
+  DBuf<int64_t>& contrib_idx = t.contrib_idx;
+  DBuf<double>&contrib_val = t.contrib_val, &side = t.side;
+  if (!t.answered) std::copy_n(ctx().await(t.report), int(kStWords), t.answer);
+  const int64_t* f = t.answer;
   if (f[kStUnbounded]) { plan.has_unbounded = true; return; }
   const int nwin = int(f[kStWin]), nelim = int(f[kStElim]);
   const bool any_side = f[kStSide] != 0;

@@ -340,6 +340,11 @@ struct Context {
   Mailbox* nnz_mail = nullptr;       // kNnzBoxes, taken in turn
   uint32_t nnz_seq = 0;
   Mailbox* nnz_box(uint32_t seq) { return nnz_mail + seq % kNnzBoxes; }
+  // Answers that the host needs later in the same call: sums (taken in turn, an
+  // Objective holds at most kLateSums) and the count of the last fixed columns.
+  static constexpr uint32_t kLateBoxes = 64;
+  Mailbox *late_mail = nullptr, *fixed_mail = nullptr;
+  uint32_t late_seq = 0;
   Report open_report(int count);                       // words of this context
   Report open_report(int count, int32_t* words);       // the caller's words (zero at launch), kept
   uint32_t open_mail() { return ++mail_seq; }
@@ -522,6 +527,13 @@ std::pair<int64_t, int64_t> exclusive_scan_pair_i64(const int64_t* a, int64_t* a
 // totals added in order).  Items whose `mask` byte is 0 count as 0.0 (mask may
 // be null).  Returns the value on the host.
 double det_sum(const double* v, const uint8_t* mask, int64_t n, cudaStream_t s);
+// The same sum, read when it is needed (within the call, and before 64 more).
+struct LateValue {
+  double known = 0.0;
+  uint32_t seq = 0;   // 0: known
+  double get() const;
+};
+LateValue det_sum_later(const double* v, const uint8_t* mask, int64_t n, cudaStream_t s);
 
 struct ProfileSummary {
   std::string name;

@@ -178,7 +178,7 @@ struct Engine {
     const bool changed = plan.has_change && !terminal;
     if (changed) {
       if (plan.has_row_deletion || plan.has_col_action) ++deletion_serial;
-      cur.obj += plan.obj_delta;
+      cur.obj.add(plan.obj_delta);
       capture_tape(out.record, plan.tape);
       if (plan.has_col_action)
         append_fixed(out.record, plan.keep_col.p, stats.seen_col.p, plan.l.p, plan.u.p, cur.n());
@@ -217,7 +217,7 @@ struct Engine {
       capture_tape(r, pl.tape);
       GPP_LAUNCH_BYTES(gather_kept, 52.0 * n + 36.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s(), m, n,
                        rmap.p, cmap.p, vectors(pl), vectors(cur), nullptr, nullptr, nullptr, nullptr);
-      cur.obj += pl.obj_delta;
+      cur.obj.add(pl.obj_delta);
       return;
     }
     WorkingLp next;
@@ -239,7 +239,8 @@ struct Engine {
     next.u = dalloc<double>(size_t(n_new));
     next.AL = dalloc<double>(size_t(m_new));
     next.AU = dalloc<double>(size_t(m_new));
-    next.obj = cur.obj + pl.obj_delta;
+    next.obj = cur.obj;
+    next.obj.add(pl.obj_delta);
     // update_device_recovery (device_recovery.cu:892-975).
     capture_tape(r, pl.tape);
     if (pl.absval) {
@@ -605,6 +606,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
   }
   e.materialize("finalize");
   e.save_vectors();
+  settle_fixed(out.record);
   ctx().sync("presolve finalize");
   out.reduced_rows = cur.m();
   out.reduced_cols = cur.n();

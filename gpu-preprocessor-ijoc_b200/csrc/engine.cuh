@@ -98,6 +98,54 @@ struct RecoveryCheckpoint {
   int64_t tape_position = 0;
 };
 
+// A total whose terms may still be on their way from the device; reading it
+// waits for them and adds everything in the order it was put in.  A rule's sum
+// is not needed before the call's end, so no wait stands behind it (about 8 us).
+class Objective {
+ public:
+  static constexpr size_t kLateSums = 16;   // at most: three totals share kLateBoxes
+  Objective(double v = 0.0) : total_(v) {}
+  operator double() const {
+    for (const Group& g : later_) {
+      double sum = g.terms[0].get();
+      for (size_t k = 1; k < g.terms.size(); ++k) sum += g.terms[k].get();
+      total_ += sum;
+    }
+    later_.clear();
+    late_ = 0;
+    return total_;
+  }
+  Objective& operator+=(double x) { return *this += LateValue{x, 0}; }
+  Objective& operator+=(const LateValue& x) {
+    if (x.seq == 0 && later_.empty()) total_ += x.known;
+    else put(Group{{x}}, x.seq ? 1 : 0);
+    return *this;
+  }
+  // Adds a delta as one term.
+  void add(const Objective& delta) {
+    Group g{{LateValue{delta.total_, 0}}};
+    for (const Group& d : delta.later_) {
+      if (d.terms.size() != 1) { *this += double(delta); return; }
+      g.terms.push_back(d.terms[0]);
+    }
+    if (g.terms.size() == 1) *this += delta.total_;
+    else put(std::move(g), delta.late_);
+  }
+
+ private:
+  struct Group {
+    std::vector<LateValue> terms;
+  };
+  void put(Group g, size_t late) {
+    later_.push_back(std::move(g));
+    late_ += late;
+    if (late_ >= kLateSums) static_cast<void>(double(*this));
+  }
+  mutable double total_;
+  mutable std::vector<Group> later_;
+  mutable size_t late_ = 0;
+};
+
 struct Record {
   int32_t m0 = 0, n0 = 0;
   DBuf<int32_t> rows, cols;   // current index -> original index
@@ -108,12 +156,19 @@ struct Record {
   std::vector<VarPairRecovery> varpair;
   std::vector<RecoveryCheckpoint> timeline;
   int64_t records = 0, indices = 0, values = 0;
+  // The last fixed columns, packed, while their count is on its way.
+  struct {
+    DBuf<int32_t> idx;
+    DBuf<double> val;
+    uint32_t seq = 0;
+    bool open = false;
+  } late_fixed;
 };
 
 struct Plan {
   DBuf<uint8_t> keep_row, keep_col;
   DBuf<double> c, l, u, AL, AU;
-  double obj_delta = 0.0;
+  Objective obj_delta;
   bool has_change = false, has_row_action = false, has_col_action = false;
   bool has_redundant_row_deletion = false, has_row_deletion = false;
   bool has_infeasible = false, has_unbounded = false;
@@ -177,7 +232,7 @@ bool rows_strictly_sorted(const DevCsr& M, cudaStream_t s);
 struct WorkingLp {
   DevCsr A, AT;
   double *c = nullptr, *AL = nullptr, *AU = nullptr, *l = nullptr, *u = nullptr;
-  double obj = 0.0;
+  Objective obj;
   bool owns = false;
   // Rows of A / AT strictly ascending: 1 yes, 0 no, -1 not checked yet.
   // Compaction keeps a subsequence of every row, so it keeps the property;
@@ -278,6 +333,7 @@ void free_csr(DevCsr& M);
 void init_record(Record& r, int32_t m, int32_t n);
 void globalize_segment(PostsolveSegment& s, const Record& r, cudaStream_t st);
 void capture_tape(Record& r, std::vector<PostsolveSegment>& tape);
+void settle_fixed(Record& r);   // adds the columns of the last append_fixed
 void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, const double* l,
                   const double* u, int32_t n);
 // Builds a device segment from host-side packed arrays (records laid out
@@ -359,6 +415,6 @@ void rule_variable_pair(Plan& plan, const WorkingLp& lp, const gpp_params& p);
 void row_gather_shift(const DevCsr& A, const DevCsr& AT, const uint8_t* keep_row, const uint8_t* selected,
                       const double* value, const double* radius, double* out, cudaStream_t s);
 // Canonical objective sum of contrib over the rule-entry domain.
-double domain_objective(const double* contrib, const uint8_t* entry_keep, int32_t n, cudaStream_t s);
+LateValue domain_objective(const double* contrib, const uint8_t* entry_keep, int32_t n, cudaStream_t s);
 
 }  // namespace gpp

@@ -179,20 +179,44 @@ void capture_tape(Record& r, std::vector<PostsolveSegment>& tape) {
   tape.clear();
 }
 
+void settle_fixed(Record& r) {
+  auto& late = r.late_fixed;
+  if (!late.open) return;
+  auto& c = ctx();
+  late.open = false;
+  const int64_t count = c.await(c.fixed_mail, late.seq, "append_fixed")[0];
+  if (count) {
+    FixedSegment f;
+    f.count = count;
+    f.idx.alloc(size_t(count), c.stream);
+    f.val.alloc(size_t(count), c.stream);
+    f.idx.copy_from(late.idx.p, size_t(count));
+    f.val.copy_from(late.val.p, size_t(count));
+    r.fixed.push_back(std::move(f));
+  }
+  late.idx.release();
+  late.val.release();
+}
+
 void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, const double* l, const double* u,
                   int32_t n) {
   // append_fixed (device_recovery.cu:233-276).
   if (!n) return;
+  settle_fixed(r);
   auto s = ctx().stream;
   // One selection over the columns finds the fixed ones and packs them (into
   // arrays for all columns, as their number is not known yet); the segment
-  // keeps the packed part.
-  DBuf<int32_t> idx(size_t(n), s);
-  DBuf<double> val(size_t(n), s);
+  // keeps the packed part, once the next call or the presolve's end has read the
+  // number without a wait of its own.
+  auto& late = r.late_fixed;
+  late.idx.alloc(size_t(n), s);
+  late.val.alloc(size_t(n), s);
+  late.seq = ctx().open_mail();
+  late.open = true;
   const int32_t* cols = r.cols.p;
-  int32_t* out_idx = idx.p;
-  double* out_val = val.p;
-  const int32_t count = select_and_count(
+  int32_t* out_idx = late.idx.p;
+  double* out_val = late.val.p;
+  select_and_post(
       n,
       [=] __device__(int64_t i) {
         return (!prior || prior[i]) && !keep_col[i] && isfinite(l[i]) && isfinite(u[i]) && fabs(l[i] - u[i]) <= 1e-9;
@@ -202,15 +226,7 @@ void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, cons
         out_idx[at] = cols[i];
         out_val[at] = 0.5 * (l[i] + u[i]);
       },
-      s);
-  if (!count) return;
-  FixedSegment f;
-  f.count = count;
-  f.idx.alloc(size_t(count), s);
-  f.val.alloc(size_t(count), s);
-  f.idx.copy_from(idx.p, size_t(count));
-  f.val.copy_from(val.p, size_t(count));
-  r.fixed.push_back(std::move(f));
+      ctx().fixed_mail, late.seq, s);
 }
 
 }  // namespace gpp

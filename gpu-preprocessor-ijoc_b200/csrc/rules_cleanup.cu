@@ -239,11 +239,10 @@ void row_gather_shift(const DevCsr& A, const DevCsr& AT, const uint8_t* keep_row
              radius, out);
 }
 
-double domain_objective(const double* contrib, const uint8_t* entry_keep, int32_t n, cudaStream_t s) {
+LateValue domain_objective(const double* contrib, const uint8_t* entry_keep, int32_t n, cudaStream_t s) {
   // sum_cleanup_domain (cleanup_support.cuh:13-31): the sum over the rule's
   // entry domain, with the canonical deterministic reduction.
-  if (n <= 0) return 0.0;
-  return det_sum(contrib, entry_keep, n, s);
+  return det_sum_later(contrib, entry_keep, n, s);
 }
 
 namespace {

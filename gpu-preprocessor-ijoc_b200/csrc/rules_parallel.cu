@@ -908,7 +908,7 @@ void rule_parallel_columns(Plan& plan, const WorkingLp& lp, const Stats&, const 
   }
   GPP_LAUNCH(col_apply, grid_stride_blocks(std::max(n, m)), kThreads, 0, s, n, m, del.p, fixed.p, fval.p, plan.c.p,
              any_fixed ? shift.p : nullptr, plan.keep_col.p, plan.l.p, plan.u.p, plan.AL.p, plan.AU.p, contrib.p);
-  plan.obj_delta += any_fixed ? det_sum(contrib.p, nullptr, n, s) : 0.0;
+  plan.obj_delta += any_fixed ? det_sum_later(contrib.p, nullptr, n, s) : LateValue{};
   plan.has_col_action = plan.has_change = true;
 }
 

@@ -235,16 +235,22 @@ void select_items(int64_t n, Pred pred, Emit emit, int32_t* count, cudaStream_t 
              w.counters, ctx().host_error);
 }
 
+// The same, the number taken being posted to `mail`.
+template <class Pred, class Emit>
+void select_and_post(int64_t n, Pred pred, Emit emit, Mailbox* mail, uint32_t seq, cudaStream_t s) {
+  const int64_t tiles = n > 0 ? (n + kScanTile - 1) / kScanTile : 1;
+  LookbackSpace w(size_t(tiles), s);
+  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, nullptr, mail, seq, w.words,
+             w.counters, ctx().host_error);
+}
+
 // The same, waiting for the number taken.
 template <class Pred, class Emit>
 int32_t select_and_count(int64_t n, Pred pred, Emit emit, cudaStream_t s, const char* where = __builtin_FUNCTION()) {
   if (n <= 0) return 0;
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  LookbackSpace w(size_t(tiles), s);
   auto& c = ctx();
   const uint32_t seq = c.open_mail();
-  GPP_LAUNCH((select_tiles<Pred, Emit>), int(tiles), kThreads, 0, s, n, tiles, pred, emit, nullptr, c.box(seq), seq, w.words,
-             w.counters, c.host_error);
+  select_and_post(n, pred, emit, c.box(seq), seq, s);
   return int32_t(c.await(c.box(seq), seq, where)[0]);
 }
 

@@ -152,54 +152,91 @@ __device__ void row_hash_block(const RowHashArgs& g, const int32_t* rows, int co
   __syncthreads();
 }
 
-// Four rows per warp, eight lanes (a group) per row, eight stored entries per
-// round.  A first sweep finds the live length and the first live entry (the
-// pivot); the second forms the hash: the XOR aggregate is order-free, the
-// sequential fold visits the group's live entries of each round in stored
-// order through shuffles.  Every lane runs the same number of rounds (the
-// warp's maximum), so ballots and shuffles stay warp-uniform; rounds past a
-// row's end have no live entry.
-__device__ void row_hash_grouped(const RowHashArgs& g, int i) {
-  const int lane = threadIdx.x & 31, group = lane >> 3, gl = lane & 7;
-  const unsigned shift = unsigned(group * 8);
+// A warp's 32 medium rows, one to a lane, eight stored entries of each per
+// round.  Eight lanes load a row's eight (four rows at a time), divide by its
+// pivot and stage the pairs in shared memory, where the row's lane folds them
+// in stored order (an entry's fold is a serial chain of 64-bit multiplies, so
+// one lane runs it; a form in which all eight lanes of a row ran it over
+// shuffles took 904 us at the 29.8M-nnz LP, this one 805).  A first sweep under a column mask
+// finds the live length and the first live entry (the pivot).  Rounds last as
+// long as the longest row; rows that have ended are passed over in fours.
+struct RowStage {
+  int32_t col[32 * 9];   // rows padded to 9 entries: no bank conflicts either way
+  uint64_t bits[32 * 9];
+};
+__device__ void row_hash_rows(const RowHashArgs& g, int i, RowStage& stage) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, sub = lane >> 3, gl = lane & 7;
   const bool keep = i >= 0 && g.keep_row[i];
   const offset_t a = keep ? g.ptr[i] : 0, e = keep ? g.ptr[i + 1] : 0;
-  const int rounds = __reduce_max_sync(0xffffffffu, int((e - a + 7) >> 3));
-  int len = 0;
-  offset_t first = -1;
-  for (int k = 0; k < rounds; ++k) {
-    const offset_t p = a + offset_t(k) * 8 + gl;
-    const bool live = p < e && (!g.keep_col || g.keep_col[__ldcs(g.idx + p)]);
-    const unsigned bits = (__ballot_sync(0xffffffffu, live) >> shift) & 0xFFu;
-    if (first < 0 && bits) first = a + offset_t(k) * 8 + (__ffs(bits) - 1);
-    len += __popc(bits);
+  int len = int(e - a);
+  offset_t first = a;
+  if (g.keep_col) {
+    len = 0;
+    first = -1;
+    for (int at = 0;; at += 8) {
+      if (!__any_sync(kAll, e - a > at)) break;
+      int col[8];
+      unsigned mine = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const offset_t ra = __shfl_sync(kAll, a, 4 * k + sub), re = __shfl_sync(kAll, e, 4 * k + sub);
+        col[k] = re - ra > at + gl ? __ldcs(g.idx + ra + at + gl) : -1;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const unsigned live = __ballot_sync(kAll, col[k] >= 0 && g.keep_col[max(col[k], 0)]);
+        if (lane >> 2 == k) mine = live >> (8 * (lane & 3)) & 0xffu;
+      }
+      if (first < 0 && mine) first = a + at + (__ffs(mine) - 1);
+      len += __popc(mine);
+    }
   }
   const bool trivial = !keep || len == 0 || fabs(g.val[first]) <= g.tol;
   const double pivot = trivial ? 1.0 : g.val[first];
   const offset_t from = trivial ? e : first;
-  const int rounds2 = __reduce_max_sync(0xffffffffu, int((e - from + 7) >> 3));
   uint64_t h = mix(kFnvOffset, uint64_t(len)), agg = 0;
-  for (int k = 0; k < rounds2; ++k) {
-    const offset_t p = from + offset_t(k) * 8 + gl;
-    const bool live = p < e && (!g.keep_col || g.keep_col[__ldcs(g.idx + p)]);
-    const uint64_t col = live ? uint64_t(__ldcs(g.idx + p)) : 0;
-    const uint64_t b = live ? dbits(__ldcs(g.val + p) / pivot) : 0;
-    if (g.use_xor) {
-      if (live) agg ^= mix(mix(kFnvOffset, col), b);
-    } else {
-      const unsigned bits = (__ballot_sync(0xffffffffu, live) >> shift) & 0xFFu;
+  for (int at = 0;; at += 8) {
+    const unsigned need = __ballot_sync(kAll, e - from > at);
+    if (!need) break;
+    int col[8];
+    double v[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const uint64_t ct = __shfl_sync(0xffffffffu, col, t, 8);
-        const uint64_t bt = __shfl_sync(0xffffffffu, b, t, 8);
-        if ((bits >> t) & 1u) h = mix(mix(h, ct), bt);
+    for (int k = 0; k < 8; ++k) {
+      const offset_t rf = __shfl_sync(kAll, from, 4 * k + sub), re = __shfl_sync(kAll, e, 4 * k + sub);
+      const bool in = re - rf > at + gl;
+      col[k] = in ? __ldcs(g.idx + rf + at + gl) : -1;
+      v[k] = in ? __ldcs(g.val + rf + at + gl) : 0.0;
+    }
+    if (g.keep_col) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (col[k] >= 0 && !g.keep_col[col[k]]) col[k] = -1;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const double by = __shfl_sync(kAll, pivot, 4 * k + sub);
+      if (need >> (4 * k) & 15u) {
+        const int slot = (4 * k + sub) * 9 + gl;
+        stage.col[slot] = col[k];
+        stage.bits[slot] = dbits(v[k] / by);
       }
     }
+    __syncwarp();
+    if (need >> lane & 1u) {
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const int32_t c = stage.col[lane * 9 + t];
+        const uint64_t b = stage.bits[lane * 9 + t];
+        if (c < 0) continue;
+        if (g.use_xor) agg ^= mix(mix(kFnvOffset, uint64_t(c)), b);
+        else h = mix(mix(h, uint64_t(c)), b);
+      }
+    }
+    __syncwarp();
   }
-  if (g.use_xor)
-    for (int off = 4; off; off >>= 1) agg ^= __shfl_xor_sync(0xffffffffu, agg, off, 8);
-  if (gl == 0 && i >= 0) {
-    if (!g.keep_row[i]) g.out[i] = uint64_t(i);
+  if (i >= 0) {
+    if (!keep) g.out[i] = uint64_t(i);
     else if (trivial) g.out[i] = mix(kFnvOffset, uint64_t(i));
     else g.out[i] = g.use_xor ? mix(h, agg) : h;
   }
@@ -221,21 +258,24 @@ __global__ void __launch_bounds__(kThreads)
 row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
                 const int32_t* __restrict__ counts, HashRoles roles) {
   after_previous_kernel();
-  __shared__ HashStage stage[2];
+  __shared__ union {
+    HashStage block[2];
+    RowStage warp[kThreads / 32];
+  } stage;
   int b = blockIdx.x;
   if (b < roles.long_blocks) {
     const int count = counts[1];
     for (int q = b * kHashRows; q < count; q += roles.long_blocks * kHashRows)
-      row_hash_block(g, longq + q, min(kHashRows, count - q), stage);
+      row_hash_block(g, longq + q, min(kHashRows, count - q), stage.block);
     return;
   }
   b -= roles.long_blocks;
-  if (b < roles.medium_blocks) {   // four rows to a warp
+  if (b < roles.medium_blocks) {   // 32 rows to a warp
     const int nwarps = roles.medium_blocks * (kThreads / 32);
     const int nmedium = counts[0];
-    for (int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 4; q0 < nmedium; q0 += nwarps * 4) {
-      const int q = q0 + int((threadIdx.x & 31) >> 3);
-      row_hash_grouped(g, q < nmedium ? medium[q] : -1);
+    for (int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 32; q0 < nmedium; q0 += nwarps * 32) {
+      const int q = q0 + int(threadIdx.x & 31);
+      row_hash_rows(g, q < nmedium ? medium[q] : -1, stage.warp[threadIdx.x >> 5]);
     }
     return;
   }

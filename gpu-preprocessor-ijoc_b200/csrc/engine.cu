@@ -252,6 +252,7 @@ struct Engine {
       pl.varpair.reset();
     }
     if (!cleanup_captured && n_new != n) append_fixed(r, pl.keep_col.p, nullptr, pl.l.p, pl.u.p, n);
+    globalize_segments(r);
     // The vectors and, where the maps change, the original ids.
     DBuf<int32_t> rows, cols;
     if (m_new != r.m) rows.alloc(size_t(m_new), s());
@@ -607,6 +608,7 @@ void run_presolve(const gpp_lp& input, const gpp_params& p, PresolveOutput& out,
   e.materialize("finalize");
   e.save_vectors();
   settle_fixed(out.record);
+  globalize_segments(out.record);
   ctx().sync("presolve finalize");
   out.reduced_rows = cur.m();
   out.reduced_cols = cur.n();

@@ -151,6 +151,7 @@ struct Record {
   DBuf<int32_t> rows, cols;   // current index -> original index
   int32_t m = 0, n = 0;
   std::vector<PostsolveSegment> segments;
+  size_t globalized = 0;      // segments that hold original ids already
   std::vector<FixedSegment> fixed;
   std::vector<AbsValueRecovery> absval;
   std::vector<VarPairRecovery> varpair;
@@ -331,7 +332,9 @@ void free_csr(DevCsr& M);
 
 // recovery.cu
 void init_record(Record& r, int32_t m, int32_t n);
-void globalize_segment(PostsolveSegment& s, const Record& r, cudaStream_t st);
+// Original ids in the segments captured since the last call; before the maps
+// change, and at the end.
+void globalize_segments(Record& r);
 void capture_tape(Record& r, std::vector<PostsolveSegment>& tape);
 void settle_fixed(Record& r);   // adds the columns of the last append_fixed
 void append_fixed(Record& r, const uint8_t* keep_col, const uint8_t* prior, const double* l,

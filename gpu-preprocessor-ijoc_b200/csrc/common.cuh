@@ -236,6 +236,20 @@ __device__ __forceinline__ int block_append(int32_t* counter, bool take) {
   return slot;
 }
 
+// Small models run some chains of kernels as one launch of one thread-block
+// cluster: its hardware barrier, which also orders the blocks' accesses to global
+// memory, stands where the launches did, and its blocks are scheduled together, so
+// nothing spins.  Eight blocks is the portable size.  Such a chain costs about as
+// much as one of its launches while eight SMs keep up with the work: up to 8,192
+// rows and columns.  At 2,000 x 5,000 the Cleanup chain takes 20 us in place of 51;
+// at 20,000 x 50,000 it is the slower form (a presolve 8.85 against 7.0 ms).
+constexpr int kSmallCluster = 8;
+constexpr int kSmallModel = 8192;
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Answers to the host.  Between two rules the host asks the device a question
 // (does the rule act, how many items were selected) and waits for the answer.

@@ -359,7 +359,7 @@ constexpr uint32_t kProbeFixed = 1, kProbeEmptyColumns = 2, kProbeEmptyRows = 4,
 // along with its own: where the probe finds nothing (most rounds) the rule runs
 // on the plan as it stands, so its kernels follow the probe's without a wait,
 // and on the device do nothing when the probe found something.  Up to
-// kFusedCleanup rows and columns probe and rule are one launch of one cluster.
+// kSmallModel rows and columns probe and rule are one launch of one cluster.
 struct SingletonTest {
   DBuf<int32_t> cand, rows, long_rows, winners;
   DBuf<double> fmin, fmax, side, contrib_val;
@@ -370,7 +370,6 @@ struct SingletonTest {
   bool asked = false, answered = false;
   int64_t answer[kSingletonWords] = {};
 };
-constexpr int kFusedCleanup = 8192;
 struct ProbeArgs;
 void ask_singleton_columns(SingletonTest& t, Plan& plan, const WorkingLp& lp, const Stats& stats, const gpp_params& p,
                            const int32_t* gate);

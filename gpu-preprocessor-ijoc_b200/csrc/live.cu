@@ -756,10 +756,9 @@ struct SideStats {
 // degree and, for a deleted column, by one per kept row it leaves; added up in
 // registers, one atomic per warp (an atomic per item on the one total took 152
 // us when 0.8M rows went at once, on the QAP N = 30 relaxation).
-__global__ void __launch_bounds__(kThreads) inc_walk(int m, const int32_t* __restrict__ list,
-                                                     const int32_t* __restrict__ counters, SideStats rows,
-                                                     SideStats cols, unsigned long long* live_nnz) {
-  after_previous_kernel();
+__device__ __forceinline__ void walk_deleted(int m, const int32_t* list, const int32_t* counters,
+                                             const SideStats& rows, const SideStats& cols,
+                                             unsigned long long* live_nnz) {
   const int half = gridDim.x / 2;
   const bool row_side = int(blockIdx.x) < half;
   const SideStats& outer = row_side ? rows : cols;
@@ -788,6 +787,11 @@ __global__ void __launch_bounds__(kThreads) inc_walk(int m, const int32_t* __res
   }
   for (int off = 16; off; off >>= 1) dropped += __shfl_down_sync(0xffffffffu, dropped, off);
   if ((threadIdx.x & 31) == 0 && dropped) atomicAdd(live_nnz, 0ULL - dropped);
+}
+__global__ void __launch_bounds__(kThreads) inc_walk(int m, const int32_t* list, const int32_t* counters,
+                                                     SideStats rows, SideStats cols, unsigned long long* live_nnz) {
+  after_previous_kernel();
+  walk_deleted(m, list, counters, rows, cols, live_nnz);
 }
 
 // Flags of the dirty kept items; a degree-1 item finds its only live entry.
@@ -818,6 +822,23 @@ __global__ void inc_fix(int m, int n, SideStats rows, SideStats cols, int32_t* _
   after_previous_kernel();
   if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;   // for the next refresh
   if (blockIdx.x == 0 && threadIdx.x == 0) post_values(box, seq, int64_t(*live_nnz));
+  fix_dirty(m, rows, cols.keep);
+  fix_dirty(n, cols, rows.keep);
+}
+
+// The three in one cluster, for small models.
+__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kThreads)
+inc_small(int m, int n, uint8_t* seen_row, uint8_t* seen_col, int32_t* list, int32_t* counters, SideStats rows,
+          SideStats cols, unsigned long long* live_nnz, Mailbox* box, uint32_t seq) {
+  after_previous_kernel();
+  find_deleted(m, seen_row, rows.keep, list, counters);
+  find_deleted(n, seen_col, cols.keep, list + m, counters + 1);
+  cluster_barrier();
+  walk_deleted(m, list, counters, rows, cols, live_nnz);
+  cluster_barrier();
+  if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;   // for the next refresh
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    post_values(box, seq, int64_t(*static_cast<volatile unsigned long long*>(live_nnz)));
   fix_dirty(m, rows, cols.keep);
   fix_dirty(n, cols, rows.keep);
 }
@@ -880,13 +901,20 @@ void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan) {
     st.seen_col.copy_from(plan.keep_col.p, size_t(n));
     st.nnz_known = int64_t(read_scalar(st.live_nnz.p));
   } else {
-    GPP_LAUNCH_BYTES(inc_deleted, 2.0 * (double(m) + n), grid_stride_blocks(std::max(m, n) / 16 + 1), kThreads, 0, s, m,
-                     n, st.seen_row.p, plan.keep_row.p, st.seen_col.p, plan.keep_col.p, st.deleted.p, st.counters.p);
-    const int g = 2 * std::max(1, std::min(kNumSMs * 4, (std::max(m, n) + kThreads / 8 - 1) / (kThreads / 8)));
-    GPP_LAUNCH(inc_walk, g, kThreads, 0, s, m, st.deleted.p, st.counters.p, rows, cols, st.live_nnz.p);
     const uint32_t seq = ++ctx().nnz_seq;
-    GPP_LAUNCH(inc_fix, grid_stride_blocks(std::max(m, n) / 4 + 1), kThreads, 0, s, m, n, rows, cols, st.counters.p,
-               st.live_nnz.p, ctx().nnz_box(seq), seq);
+    Mailbox* const box = ctx().nnz_box(seq);
+    if (std::max(m, n) <= kSmallModel) {
+      GPP_LAUNCH_BYTES(inc_small, 2.0 * (double(m) + n), kSmallCluster, kThreads, 0, s, m, n, st.seen_row.p,
+                       st.seen_col.p, st.deleted.p, st.counters.p, rows, cols, st.live_nnz.p, box, seq);
+    } else {
+      GPP_LAUNCH_BYTES(inc_deleted, 2.0 * (double(m) + n), grid_stride_blocks(std::max(m, n) / 16 + 1), kThreads, 0, s,
+                       m, n, st.seen_row.p, plan.keep_row.p, st.seen_col.p, plan.keep_col.p, st.deleted.p,
+                       st.counters.p);
+      const int g = 2 * std::max(1, std::min(kNumSMs * 4, (std::max(m, n) + kThreads / 8 - 1) / (kThreads / 8)));
+      GPP_LAUNCH(inc_walk, g, kThreads, 0, s, m, st.deleted.p, st.counters.p, rows, cols, st.live_nnz.p);
+      GPP_LAUNCH(inc_fix, grid_stride_blocks(std::max(m, n) / 4 + 1), kThreads, 0, s, m, n, rows, cols, st.counters.p,
+                 st.live_nnz.p, box, seq);
+    }
     st.nnz_known = -1;
     st.nnz_seq = seq;
   }

@@ -569,13 +569,8 @@ __global__ void __launch_bounds__(kThreads) sc_stage(ScArgs g, Report report) {
 // their launches: the cluster's barrier stands where a launch did.  Its blocks
 // are scheduled together, so nothing spins.  At 2,000 x 5,000 the five launches
 // and two waits took about 52 us.
-constexpr int kCleanupCluster = 8;
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 template <bool kPacked>
-__global__ void __cluster_dims__(kCleanupCluster, 1, 1) __launch_bounds__(kThreads)
+__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kThreads)
 probe_and_singleton_columns(ProbeArgs probe, ScArgs g, Report report) {
   after_previous_kernel();
   if (blockIdx.x == 0 && threadIdx.x <= kSingletonWords) g.st[threadIdx.x] = 0;
@@ -589,8 +584,8 @@ probe_and_singleton_columns(ProbeArgs probe, ScArgs g, Report report) {
     sc_candidates_part(g);
     cluster_barrier();
     const CacheOut out{g.fmin, g.fmax, g.counts, g.invalid};
-    sc_cache_rows(kCleanupCluster, g.rows, g.st, g.row_nnz, g.ptr, g.idx, g.val, cache_bounds<kPacked>(g), out);
-    sc_cache_long(int(blockIdx.x), kCleanupCluster, g.long_rows, g.st, g.row_nnz, g.ptr, g.idx, g.val,
+    sc_cache_rows(kSmallCluster, g.rows, g.st, g.row_nnz, g.ptr, g.idx, g.val, cache_bounds<kPacked>(g), out);
+    sc_cache_long(int(blockIdx.x), kSmallCluster, g.long_rows, g.st, g.row_nnz, g.ptr, g.idx, g.val,
                   cache_bounds<kPacked>(g), out);
     cluster_barrier();
     sc_propose_part(g);
@@ -882,9 +877,9 @@ uint32_t probe_and_ask_singleton_columns(const ProbeArgs& probe, SingletonTest& 
   const ScArgs g = singleton_args(t, plan, lp, stats, p);
   const Report report = ctx().open_report(kStWords + 1, g.st);
   if (plan.bounds_mirrored)
-    GPP_LAUNCH(probe_and_singleton_columns<true>, kCleanupCluster, kThreads, 0, s, probe, g, report);
+    GPP_LAUNCH(probe_and_singleton_columns<true>, kSmallCluster, kThreads, 0, s, probe, g, report);
   else
-    GPP_LAUNCH(probe_and_singleton_columns<false>, kCleanupCluster, kThreads, 0, s, probe, g, report);
+    GPP_LAUNCH(probe_and_singleton_columns<false>, kSmallCluster, kThreads, 0, s, probe, g, report);
   const int64_t* f = ctx().await(report);
   std::copy(f, f + kStWords, t.answer);
   t.asked = t.answered = true;

@@ -187,9 +187,6 @@ struct Plan {
   DBuf<double2> lu;
   DBuf<double> cand_l, cand_u;
   bool bounds_mirrored = false;
-  // Column max |a| over the kept rows, as of the statistics' version.
-  DBuf<double> col_max;
-  uint64_t col_max_version = 0;
   // What dual fixing asks of each row, left by a redundant-row test that acted
   // on none (row_kinds_current until the next of the two rules).
   DBuf<uint8_t> row_kinds;

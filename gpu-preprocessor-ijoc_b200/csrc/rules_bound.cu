@@ -178,9 +178,48 @@ struct SupportArgs {
   const offset_t* at_ptr;
   const int32_t* at_idx;
   const double* at_val;
+  const uint8_t* keep_row;
   RowRecords rows;
   double zero_tol, tol, support_tol;
 };
+// The largest |a| of a column over its kept rows (reference :789-809), which the
+// finalisation needs where a candidate would move a bound (`wanted`).  A thread
+// walks its own column, four entries at a time; the warp takes columns of more
+// than kWideColumn entries together.  All lanes call it.
+constexpr int kWideColumn = 64;
+__device__ __forceinline__ double column_max(const SupportArgs& g, int j, bool wanted) {
+  constexpr int kBatch = 4;
+  const auto walk = [&](offset_t first, offset_t end, int step) {
+    double v = 0.0;
+    for (int64_t p = first; p < end; p += kBatch * step) {
+      int row[kBatch];
+      double a[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        const bool in = end - p > k * step;
+        row[k] = in ? g.at_idx[p + k * step] : -1;
+        a[k] = in ? g.at_val[p + k * step] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (row[k] >= 0 && g.keep_row[row[k]]) v = fmax(v, fabs(a[k]));
+    }
+    return v;
+  };
+  const offset_t first = wanted ? g.at_ptr[j] : 0, end = wanted ? g.at_ptr[j + 1] : 0;
+  const bool wide = end - first > kWideColumn;
+  double v = wide ? 0.0 : walk(first, end, 1);
+  const int lane = threadIdx.x & 31;
+  for (unsigned left = __ballot_sync(0xffffffffu, wide); left; left &= left - 1) {
+    const int src = __ffs(left) - 1;
+    const offset_t f = __shfl_sync(0xffffffffu, first, src), e = __shfl_sync(0xffffffffu, end, src);
+    double m = f + lane < e ? walk(f + lane, e, 32) : 0.0;
+#pragma unroll
+    for (int off = 16; off; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+    if (lane == src) v = m;
+  }
+  return v;
+}
 // Support rows of a changed column (reference :815-960): the smallest row that
 // implies each new bound, INT_MAX when none does.
 __device__ __forceinline__ void support_rows(const SupportArgs& g, int j, double lj, double uj, const ColumnBounds& b,
@@ -237,16 +276,16 @@ __device__ __forceinline__ uint32_t bound_records(uint32_t change, int sup_l, in
 // block to finish sums the tiles' counts (commit_bounds ranks within the tile).
 // A column whose bounds stand costs its reads alone; the packed bounds and the
 // candidates, which the next sweep starts from, are written where they differ.
-// Bound by DRAM (49 bytes a column); a form that handed its tiles out in order
+// Bound by DRAM (41 bytes a column) where bounds stand, by the gathers of the
+// moved columns' rows else; a form that handed its tiles out in order
 // and looked back for the records before them took 442 us for the 29.8M-nnz
 // LP's columns, 69 us for the 2M-nnz one's.  Report: word 0 flags (1 infeasible, 2 a
 // bound moves, 4 a column is fixed), 1 records, 2 indices.
 __global__ void __launch_bounds__(kThreads, 3)
 finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
                 const double* __restrict__ u, double* __restrict__ cand_l, double* __restrict__ cand_u,
-                double2* __restrict__ lu, const double* __restrict__ c, const double* __restrict__ vmax,
-                int preserve_free_zero_cost, double ft, double upper_relax, bool records, SupportArgs g,
-                FinalBounds out, Report report) {
+                double2* __restrict__ lu, const double* __restrict__ c, int preserve_free_zero_cost, double ft,
+                double upper_relax, bool records, SupportArgs g, FinalBounds out, Report report) {
   after_previous_kernel();
   __shared__ uint32_t warp_sums[2][kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -254,13 +293,16 @@ finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const do
   int turn = 0;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x, turn ^= 1) {
     const int64_t j64 = int64_t(t) * kThreads + threadIdx.x;
+    const int j = int(j64);
+    const bool kept = j64 < n && keep_col[j] != 0;
+    const double lj = kept ? l[j] : 0.0, uj = kept ? u[j] : 0.0;
+    const double cl = kept ? cand_l[j] : 0.0, cu = kept ? cand_u[j] : 0.0;
+    const double vmax = column_max(g, j, (isfinite(cl) && cl > lj) || (isfinite(cu) && cu < uj));
     uint32_t mine = 0;
     if (j64 < n) {
-      const int j = int(j64);
       uint32_t change = 0;
-      if (keep_col[j]) {
-        const double lj = l[j], uj = u[j], cl = cand_l[j], cu = cand_u[j];
-        ColumnBounds b = finalize_column(lj, uj, cl, cu, c[j], vmax[j], preserve_free_zero_cost != 0, g.zero_tol, ft,
+      if (kept) {
+        ColumnBounds b = finalize_column(lj, uj, cl, cu, c[j], vmax, preserve_free_zero_cost != 0, g.zero_tol, ft,
                                          upper_relax);
         if (b.infeasible) {
           found |= 1u;
@@ -536,13 +578,6 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(sch.tiles * parts, kNumSMs * 8));
     GPP_LAUNCH_BYTES(candidates_entries, bytes, int(blocks), kThreads, 0, s, lp.A.nnz, sch.tile_rows.p, parts, g);
   }
-  // Column maxima depend on the kept rows alone: rounds that only move bounds
-  // share one sweep.
-  if (stats.version == 0 || plan.col_max_version != stats.version) {
-    if (plan.col_max.n < size_t(n)) plan.col_max.alloc(size_t(n), s);
-    col_max_abs(lp.AT, plan.keep_row.p, plan.col_max.p, s);
-    plan.col_max_version = stats.version;
-  }
   const bool records = p.record_postsolve_tape != 0;
   DBuf<double> fl(size_t(n), s), fu(size_t(n), s);
   DBuf<uint8_t> change(size_t(n), s);
@@ -558,10 +593,11 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   }
   const FinalBounds fin{fl.p, fu.p, change.p, sl.p, su.p, tile_counts.p, before.p};
   const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
-  const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, rows, p.zero_tol, p.bound_tol, support_tol};
+  const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p, rows,
+                            p.zero_tol, p.bound_tol, support_tol};
   Report report = ctx().open_report(3);
   GPP_LAUNCH(finalize_kernel, std::min(tiles, kNumSMs * 12), kThreads, 0, s, n, tiles, plan.keep_col.p, plan.l.p,
-             plan.u.p, plan.cand_l.p, plan.cand_u.p, plan.lu.p, plan.c.p, plan.col_max.p,
+             plan.u.p, plan.cand_l.p, plan.cand_u.p, plan.lu.p, plan.c.p,
              int(p.bound_strengthening_preserve_free_zero_cost), p.feasibility_tol,
              p.bound_strengthening_upper_relaxation_factor, records, support, fin, report);
   const int64_t* answer = ctx().await(report);

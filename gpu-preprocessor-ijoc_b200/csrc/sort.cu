@@ -289,7 +289,8 @@ __device__ __forceinline__ void st_word(unsigned long long* p, unsigned long lon
 // kItems x 256 pairs: sixteen items keep the look-back short against the
 // tile's work on large inputs, eight spread mid-size inputs over the SMs.
 // 2,000,003 random pairs: 506 us before (four launches a pass: histogram, two
-// of scan, scatter), measured figures beside the dispatch below.
+// of scan, scatter), 317 now; the look-back by one tile a round trip took 327
+// (and 129 against 113 for 250,000 pairs).
 constexpr int kPolls = 1 << 22;
 
 template <int kItems>
@@ -298,8 +299,10 @@ struct SortTile {
   static constexpr size_t kBytes = size_t(kPairs) * (sizeof(uint64_t) + sizeof(int32_t));
 };
 
+constexpr int kAhead = 4;
+
 template <int kItems, class Word>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kItems == 8 ? 4 : 3)   // as shared memory allows
 sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int64_t n, int pass, int shift,
           SortPlan* plan, Word* words, int32_t* error) {
   after_previous_kernel();
@@ -344,6 +347,7 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
   for (int q = 0; q < kItems; ++q)
     rank[q] = warp_rank(counts[warp], p0 + q * 32 < tile_n ? digit_of(key[q], shift) : kDigits);
   __syncthreads();
+  int tile_total;
   {
     const int d = threadIdx.x;   // one digit per thread
     int total = 0;
@@ -355,28 +359,12 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
     }
     Word* own = words + size_t(tile) * kDigits + d;
     st_word(own, (tile == 0 ? W::kAll : W::kOwn) | Word(total));
-    const int start = scan_digits(total, warp_sums);
-    local_start[d] = start;
-    Word before = 0;
-    for (int64_t t = tile - 1; t >= 0; --t) {
-      const Word* at = words + size_t(t) * kDigits + d;
-      Word w = ld_word(at);
-      for (int polls = 1; (w >> W::kShift) == 0; ++polls) {
-        if (polls == kPolls) {
-          *reinterpret_cast<volatile int32_t*>(error) = 1;
-          __threadfence_system();   // before any answer
-          w = W::kAll;
-          break;
-        }
-        w = ld_word(at);
-      }
-      before += w & W::kValue;
-      if ((w >> W::kShift) == 2) break;
-    }
-    if (tile > 0) st_word(own, W::kAll | (before + Word(total)));
-    out_base[d] = plan->start[pass][d] + (long long)before - start;
+    local_start[d] = scan_digits(total, warp_sums);
+    tile_total = total;
   }
   __syncthreads();
+  // The tile's own order first, so that the registers are free and the published
+  // counts have arrived when the look-back starts.
 #pragma unroll
   for (int q = 0; q < kItems; ++q) {
     if (p0 + q * 32 >= tile_n) continue;
@@ -384,6 +372,36 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
     const int slot = local_start[d] + counts[warp][d] + rank[q];
     tile_keys[slot] = key[q];
     tile_vals[slot] = val[q];
+  }
+  {
+    // One digit per thread goes back kAhead tiles per round trip: tiles that run
+    // at the same time publish their own counts at about the same time, and one
+    // word at a time kept the last of many tiles waiting.
+    const int d = threadIdx.x;
+    Word before = 0;
+    bool done = tile == 0;
+    for (int64_t t = tile - 1; !done; t -= kAhead) {
+      Word w[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) w[q] = t >= q ? ld_word(words + size_t(t - q) * kDigits + d) : W::kAll;
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        if (done) continue;
+        for (int polls = 1; (w[q] >> W::kShift) == 0; ++polls) {
+          if (polls == kPolls) {
+            *reinterpret_cast<volatile int32_t*>(error) = 1;
+            __threadfence_system();   // before any answer
+            w[q] = W::kAll;
+            break;
+          }
+          w[q] = ld_word(words + size_t(t - q) * kDigits + d);
+        }
+        before += w[q] & W::kValue;
+        done = (w[q] >> W::kShift) == 2;
+      }
+    }
+    if (tile > 0) st_word(words + size_t(tile) * kDigits + d, W::kAll | (before + Word(tile_total)));
+    out_base[d] = plan->start[pass][d] + (long long)before - local_start[d];
   }
   __syncthreads();
   for (int q = threadIdx.x; q < tile_n; q += kThreads) {

@@ -48,10 +48,23 @@ __global__ void dt_col_nnz(int n, const offset_t* __restrict__ tptr, const int32
                            const double* __restrict__ tval, const uint8_t* __restrict__ keep_row,
                            const uint8_t* __restrict__ keep_col, double zt, int32_t* __restrict__ col_nnz) {
   after_previous_kernel();
+  constexpr int kBatch = 4;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     int cnt = 0;
-    if (keep_col[j])
-      for (offset_t q = tptr[j]; q < tptr[j + 1]; ++q) cnt += keep_row[tidx[q]] && fabs(tval[q]) > zt ? 1 : 0;
+    if (keep_col[j]) {
+      const offset_t end = tptr[j + 1];
+      for (int64_t q = tptr[j]; q < end; q += kBatch) {   // four entries' loads at once
+        int row[kBatch];
+        double a[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          row[k] = q + k < end ? tidx[q + k] : -1;
+          a[k] = q + k < end ? tval[q + k] : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) cnt += row[k] >= 0 && keep_row[row[k]] && fabs(a[k]) > zt ? 1 : 0;
+      }
+    }
     col_nnz[j] = cnt;
   }
 }
@@ -328,29 +341,72 @@ __global__ void dt_roles(int sel, const int32_t* __restrict__ rows, const int32_
   }
 }
 
+// A row's or column's entries by eight lanes, four items to a warp, or by the
+// whole warp when there are more than kGroupItem.  `range` gives an item's
+// entries or declines it; `body` walks them in `rounds` rounds of W entries, the
+// same number for every lane of the warp.  Bound by the round trips of an item
+// (mask, pointers, entries), so four items in flight a warp: with a warp an item
+// the rebuild of the QAP N = 30 relaxation's 1.7M short rows took 308 + 256 us.
+constexpr int kGroupItem = 64;
+template <int W>
+struct Lanes {
+  static constexpr int width = W;
+  int lane, shift, rounds;
+  __device__ __forceinline__ unsigned ballot(bool v) const {
+    const unsigned b = __ballot_sync(0xffffffffu, v);
+    return W == 32 ? b : b >> shift & 0xffu;
+  }
+  __device__ __forceinline__ double get(double v, int k) const { return __shfl_sync(0xffffffffu, v, k, W); }
+};
+template <class Range, class Body>
+__device__ __forceinline__ void by_groups(int count, const Range& range, const Body& body) {
+  const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
+  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t w0 = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4; w0 < count; w0 += warps * 4) {
+    const int w = int(w0) + grp;
+    offset_t first = 0, last = 0;
+    const bool have = w0 + grp < count && range(w, gl, first, last);
+    const bool wide = have && last - first > kGroupItem;
+    const bool mine = have && !wide;
+    const int rounds = __reduce_max_sync(0xffffffffu, mine ? int(last - first + 7) / 8 : 0);
+    body(Lanes<8>{gl, grp * 8, rounds}, w, mine, first, mine ? last : first);
+    for (unsigned rest = __ballot_sync(0xffffffffu, wide && gl == 0); rest; rest &= rest - 1) {
+      const int src = __ffs(rest) - 1;
+      const offset_t f = __shfl_sync(0xffffffffu, first, src), l = __shfl_sync(0xffffffffu, last, src);
+      body(Lanes<32>{lane, 0, int((int64_t(l) - f + 31) / 32)}, __shfl_sync(0xffffffffu, w, src), true, f, l);
+    }
+  }
+}
+
 // Rows holding a shifting column, each listed once.
 __global__ void dt_touch(int sel, const int32_t* __restrict__ role_col, const offset_t* __restrict__ tptr,
                          const int32_t* __restrict__ tidx, uint32_t* __restrict__ claimed,
                          int32_t* __restrict__ touched, int32_t* st, Report report) {
   after_previous_kernel();
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
-    const int col = role_col[w];
-    if (col < 0) continue;
-    for (offset_t chunk = tptr[col]; chunk < tptr[col + 1]; chunk += 32) {
-      const offset_t p = chunk + lane;
-      bool take = false;
-      int r = 0;
-      if (p < tptr[col + 1]) {
-        r = tidx[p];
-        const uint32_t bit = 1u << (r & 31);
-        take = (atomicOr(claimed + (r >> 5), bit) & bit) == 0;
-      }
-      const int at = warp_append(st + kStTouched, take);
-      if (take) touched[at] = r;
-    }
-  }
+  by_groups(
+      sel,
+      [&](int w, int, offset_t& first, offset_t& last) {
+        const int col = role_col[w];
+        if (col < 0) return false;
+        first = tptr[col];
+        last = tptr[col + 1];
+        return true;
+      },
+      [&](auto lanes, int, bool, offset_t first, offset_t last) {
+        constexpr int W = lanes.width;
+        for (int k = 0; k < lanes.rounds; ++k) {
+          const int at_entry = k * W + lanes.lane;
+          bool take = false;
+          int r = 0;
+          if (last - first > at_entry) {
+            r = tidx[first + at_entry];
+            const uint32_t bit = 1u << (r & 31);
+            take = (atomicOr(claimed + (r >> 5), bit) & bit) == 0;
+          }
+          const int at = warp_append(st + kStTouched, take);
+          if (take) touched[at] = r;
+        }
+      });
   post_report(report);
 }
 
@@ -361,30 +417,41 @@ __global__ void dt_shift(const int32_t* __restrict__ touched, const int32_t* __r
                          const uint8_t* __restrict__ role, const double* __restrict__ value, double zt,
                          double* __restrict__ AL, double* __restrict__ AU) {
   after_previous_kernel();
-  const int count = st[kStTouched];
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < count; w += warps) {
-    const int r = touched[w];
-    if (!keep_row[r]) continue;
-    double shift = 0.0;
-    for (offset_t chunk = ptr[r]; chunk < ptr[r + 1]; chunk += 32) {
-      const offset_t p = chunk + lane;
-      double term = 0.0;
-      bool has = false;
-      if (p < ptr[r + 1]) {
-        const int j = idx[p];
-        const double a = val[p];
-        if (role[j] && fabs(a) > zt) { has = true; term = a * value[j]; }
-      }
-      const unsigned hv = __ballot_sync(0xffffffffu, has);
-      for (int k = 0; k < 32; ++k) {
-        const double v = __shfl_sync(0xffffffffu, term, k);
-        if (hv >> k & 1u) shift += v;
-      }
-    }
-    if (lane == 0) { AL[r] -= shift; AU[r] -= shift; }
-  }
+  by_groups(
+      st[kStTouched],
+      [&](int w, int, offset_t& first, offset_t& last) {
+        const int r = touched[w];
+        if (!keep_row[r]) return false;
+        first = ptr[r];
+        last = ptr[r + 1];
+        return true;
+      },
+      [&](auto lanes, int w, bool mine, offset_t first, offset_t last) {
+        constexpr int W = lanes.width;
+        double shift = 0.0;
+        for (int k = 0; k < lanes.rounds; ++k) {
+          const int at = k * W + lanes.lane;
+          double term = 0.0;
+          bool has = false;
+          if (last - first > at) {
+            const int j = idx[first + at];
+            const double a = val[first + at];
+            if (role[j] && fabs(a) > zt) { has = true; term = a * value[j]; }
+          }
+          if (!__any_sync(0xffffffffu, has)) continue;
+          const unsigned hv = lanes.ballot(has);
+#pragma unroll
+          for (int q = 0; q < W; ++q) {
+            const double v = lanes.get(term, q);
+            if (hv >> q & 1u) shift += v;
+          }
+        }
+        if (mine && lanes.lane == 0) {
+          const int r = touched[w];
+          AL[r] -= shift;
+          AU[r] -= shift;
+        }
+      });
 }
 
 // Substitution deltas alpha * a_(r, elim) at (r, keep) for kept rows r other
@@ -394,20 +461,33 @@ __global__ void dt_delta_count(int sel, const int32_t* __restrict__ rows, const 
                                const int32_t* __restrict__ tidx, const double* __restrict__ tval,
                                const uint8_t* __restrict__ keep_row, double zt, int32_t* __restrict__ cnt) {
   after_previous_kernel();
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
-    int c = 0;
-    if (kind[w] == kPairSubst) {
-      const int row = rows[w], e = elim_c[row];
-      for (offset_t p = tptr[e] + lane; p < tptr[e + 1]; p += 32) {
-        const int r = tidx[p];
-        c += r != row && keep_row[r] && fabs(tval[p]) > zt ? 1 : 0;
-      }
-      for (int off = 16; off > 0; off >>= 1) c += __shfl_down_sync(0xffffffffu, c, off);
-    }
-    if (lane == 0) cnt[w] = c;
-  }
+  by_groups(
+      sel,
+      [&](int w, int gl, offset_t& first, offset_t& last) {
+        if (kind[w] != kPairSubst) {
+          if (gl == 0) cnt[w] = 0;
+          return false;
+        }
+        const int e = elim_c[rows[w]];
+        first = tptr[e];
+        last = tptr[e + 1];
+        return true;
+      },
+      [&](auto lanes, int w, bool mine, offset_t first, offset_t last) {
+        constexpr int W = lanes.width;
+        const int row = mine ? rows[w] : -1;
+        int c = 0;
+        for (int k = 0; k < lanes.rounds; ++k) {
+          const int at = k * W + lanes.lane;
+          bool take = false;
+          if (last - first > at) {
+            const int r = tidx[first + at];
+            take = r != row && keep_row[r] && fabs(tval[first + at]) > zt;
+          }
+          c += __popc(lanes.ballot(take));
+        }
+        if (mine && lanes.lane == 0) cnt[w] = c;
+      });
 }
 __global__ void dt_delta_fill(int sel, const int32_t* __restrict__ rows, const int32_t* __restrict__ keep_c,
                               const int32_t* __restrict__ elim_c, const uint8_t* __restrict__ kind,
@@ -416,33 +496,40 @@ __global__ void dt_delta_fill(int sel, const int32_t* __restrict__ rows, const i
                               const uint8_t* __restrict__ keep_row, double zt, const int32_t* __restrict__ pos,
                               uint64_t* __restrict__ keys, int32_t* __restrict__ order, double* __restrict__ dval) {
   after_previous_kernel();
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < sel; w += warps) {
-    if (kind[w] != kPairSubst) continue;
-    const int row = rows[w], e = elim_c[row], k = keep_c[row];
-    const double al = alpha[w];
-    int64_t out = pos[w];
-    for (offset_t chunk = tptr[e]; chunk < tptr[e + 1]; chunk += 32) {
-      const offset_t p = chunk + lane;
-      bool take = false;
-      int r = 0;
-      double a = 0.0;
-      if (p < tptr[e + 1]) {
-        r = tidx[p];
-        a = tval[p];
-        take = r != row && keep_row[r] && fabs(a) > zt;
-      }
-      const unsigned mask = __ballot_sync(0xffffffffu, take);
-      if (take) {
-        const int64_t o = out + __popc(mask & ((1u << lane) - 1u));
-        keys[o] = (uint64_t(uint32_t(r)) << 32) | uint32_t(k);
-        order[o] = int32_t(o);
-        dval[o] = al * a;
-      }
-      out += __popc(mask);
-    }
-  }
+  by_groups(
+      sel,
+      [&](int w, int, offset_t& first, offset_t& last) {
+        if (kind[w] != kPairSubst) return false;
+        const int e = elim_c[rows[w]];
+        first = tptr[e];
+        last = tptr[e + 1];
+        return true;
+      },
+      [&](auto lanes, int w, bool mine, offset_t first, offset_t last) {
+        constexpr int W = lanes.width;
+        const int row = mine ? rows[w] : -1, col = mine ? keep_c[row] : 0;
+        const double al = mine ? alpha[w] : 0.0;
+        int64_t out = mine ? pos[w] : 0;
+        for (int k = 0; k < lanes.rounds; ++k) {
+          const int at = k * W + lanes.lane;
+          bool take = false;
+          int r = 0;
+          double a = 0.0;
+          if (last - first > at) {
+            r = tidx[first + at];
+            a = tval[first + at];
+            take = r != row && keep_row[r] && fabs(a) > zt;
+          }
+          const unsigned mask = lanes.ballot(take);
+          if (take) {
+            const int64_t o = out + __popc(mask & ((1u << lanes.lane) - 1u));
+            keys[o] = (uint64_t(uint32_t(r)) << 32) | uint32_t(col);
+            order[o] = int32_t(o);
+            dval[o] = al * a;
+          }
+          out += __popc(mask);
+        }
+      });
 }
 __global__ void dt_delta_rows(int64_t total, const uint64_t* __restrict__ keys, const int32_t* __restrict__ order,
                               const double* __restrict__ raw, int32_t* __restrict__ dcol, double* __restrict__ dv,
@@ -487,32 +574,39 @@ __global__ void dt_rebuild(int m, const offset_t* __restrict__ ptr, const int32_
                            int32_t* __restrict__ cnt, const offset_t* __restrict__ optr, int32_t* __restrict__ oidx,
                            double* __restrict__ oval) {
   after_previous_kernel();
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += warps) {
-    const offset_t p0 = ptr[r], p1 = ptr[r + 1];
-    const int q0 = dptr[r], q1 = dptr[r + 1];
-    if (q0 == q1 && sorted) {
-      offset_t out = Write ? optr[r] : 0;
-      for (offset_t chunk = p0; chunk < p1; chunk += 32) {
-        const offset_t p = chunk + lane;
-        const bool keep = p < p1 && fabs(val[p]) > zt;
-        const unsigned mask = __ballot_sync(0xffffffffu, keep);
-        if (Write && keep) {
-          const offset_t o = out + __popc(mask & ((1u << lane) - 1u));
-          oidx[o] = idx[p];
-          oval[o] = 0.0 + val[p];
+  by_groups(
+      m,
+      [&](int r, int gl, offset_t& first, offset_t& last) {
+        first = ptr[r];
+        last = ptr[r + 1];
+        const int q0 = dptr[r], q1 = dptr[r + 1];
+        if (q0 == q1 && sorted) return true;
+        if (sorted && last - first > kBlockMergeRow && q1 - q0 <= kBlockMergeDeltas) return false;   // dt_rebuild_block
+        if (gl == 0) {
+          if (Write) merge_row<true>(first, last, idx, val, q0, q1, dcol, dv, zt, oidx + optr[r], oval + optr[r]);
+          else cnt[r] = merge_row<false>(first, last, idx, val, q0, q1, dcol, dv, zt, nullptr, nullptr);
         }
-        out += __popc(mask);
-      }
-      if (!Write && lane == 0) cnt[r] = int32_t(out);
-    } else if (sorted && p1 - p0 > kBlockMergeRow && q1 - q0 <= kBlockMergeDeltas) {
-      continue;  // dt_rebuild_block
-    } else if (lane == 0) {
-      if (Write) merge_row<true>(p0, p1, idx, val, q0, q1, dcol, dv, zt, oidx + optr[r], oval + optr[r]);
-      else cnt[r] = merge_row<false>(p0, p1, idx, val, q0, q1, dcol, dv, zt, nullptr, nullptr);
-    }
-  }
+        return false;
+      },
+      [&](auto lanes, int r, bool mine, offset_t first, offset_t last) {
+        constexpr int W = lanes.width;
+        int64_t out = Write && mine ? int64_t(optr[r]) : 0;
+        for (int k = 0; k < lanes.rounds; ++k) {
+          const int at = k * W + lanes.lane;
+          const bool in = last - first > at;
+          const double a = in ? val[first + at] : 0.0;
+          const int col = Write && in ? idx[first + at] : 0;
+          const bool keep = in && fabs(a) > zt;
+          const unsigned mask = lanes.ballot(keep);
+          if (Write && keep) {
+            const int64_t o = out + __popc(mask & ((1u << lanes.lane) - 1u));
+            oidx[o] = col;
+            oval[o] = 0.0 + a;
+          }
+          out += __popc(mask);
+        }
+        if (!Write && mine && lanes.lane == 0) cnt[r] = int32_t(out);
+      });
 }
 
 // Long rows with deltas (of a strictly sorted matrix): the rows the warp

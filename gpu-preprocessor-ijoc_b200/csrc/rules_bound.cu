@@ -183,37 +183,44 @@ struct SupportArgs {
   double zero_tol, tol, support_tol;
 };
 // The largest |a| of a column over its kept rows (reference :789-809), which the
-// finalisation needs where a candidate would move a bound (`wanted`).  A thread
-// walks its own column, four entries at a time; the warp takes columns of more
-// than kWideColumn entries together.  All lanes call it.
+// finalisation needs where a candidate would move a bound (`wanted`), for tests of
+// the form d * max <= ft alone.  `d_min` is the least d: once an entry makes it
+// too large, so is every test's product with the maximum (both round monotonely), and
+// the walk ends there, most often at the first entries.  A thread walks its own
+// column; the warp takes columns of more than kWideColumn entries together.  All
+// lanes call it.
 constexpr int kWideColumn = 64;
-__device__ __forceinline__ double column_max(const SupportArgs& g, int j, bool wanted) {
-  constexpr int kBatch = 4;
-  const auto walk = [&](offset_t first, offset_t end, int step) {
-    double v = 0.0;
-    for (int64_t p = first; p < end; p += kBatch * step) {
-      int row[kBatch];
-      double a[kBatch];
+__device__ __forceinline__ double column_max(const SupportArgs& g, int j, bool wanted, double d_min, double ft) {
+  const auto visit = [&](auto batch, int64_t p, offset_t end, int step, double& v) {
+    constexpr int kBatch = decltype(batch)::value;
+    int row[kBatch];
+    double a[kBatch];
 #pragma unroll
-      for (int k = 0; k < kBatch; ++k) {
-        const bool in = end - p > k * step;
-        row[k] = in ? g.at_idx[p + k * step] : -1;
-        a[k] = in ? g.at_val[p + k * step] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < kBatch; ++k)
-        if (row[k] >= 0 && g.keep_row[row[k]]) v = fmax(v, fabs(a[k]));
+    for (int k = 0; k < kBatch; ++k) {
+      const bool in = end - p > k * step;
+      row[k] = in ? g.at_idx[p + k * step] : -1;
+      a[k] = in ? g.at_val[p + k * step] : 0.0;
     }
-    return v;
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+      if (row[k] >= 0 && g.keep_row[row[k]]) v = fmax(v, fabs(a[k]));
   };
+  using Two = std::integral_constant<int, 2>;
+  using Four = std::integral_constant<int, 4>;
   const offset_t first = wanted ? g.at_ptr[j] : 0, end = wanted ? g.at_ptr[j + 1] : 0;
-  const bool wide = end - first > kWideColumn;
-  double v = wide ? 0.0 : walk(first, end, 1);
+  double v = 0.0;
+  const auto enough = [&] { return d_min > 0.0 && d_min * v > ft; };
+  if (first < end) visit(Two{}, first, end, 1, v);
+  const bool more = end - first > 2 && !enough();
+  const bool wide = more && end - first > kWideColumn;
+  if (more && !wide)
+    for (int64_t p = int64_t(first) + 2; p < end && !enough(); p += 4) visit(Four{}, p, end, 1, v);
   const int lane = threadIdx.x & 31;
   for (unsigned left = __ballot_sync(0xffffffffu, wide); left; left &= left - 1) {
     const int src = __ffs(left) - 1;
     const offset_t f = __shfl_sync(0xffffffffu, first, src), e = __shfl_sync(0xffffffffu, end, src);
-    double m = f + lane < e ? walk(f + lane, e, 32) : 0.0;
+    double m = 0.0;
+    for (int64_t p = int64_t(f) + lane; p < e; p += 4 * 32) visit(Four{}, p, e, 32, m);
 #pragma unroll
     for (int off = 16; off; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
     if (lane == src) v = m;
@@ -297,7 +304,8 @@ finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const do
     const bool kept = j64 < n && keep_col[j] != 0;
     const double lj = kept ? l[j] : 0.0, uj = kept ? u[j] : 0.0;
     const double cl = kept ? cand_l[j] : 0.0, cu = kept ? cand_u[j] : 0.0;
-    const double vmax = column_max(g, j, (isfinite(cl) && cl > lj) || (isfinite(cu) && cu < uj));
+    const double vmax = column_max(g, j, (isfinite(cl) && cl > lj) || (isfinite(cu) && cu < uj),
+                                   fmin(fmin(uj - cl, cu - lj), cu - cl), ft);
     uint32_t mine = 0;
     if (j64 < n) {
       uint32_t change = 0;

@@ -46,10 +46,10 @@ RULES = ["infeasible_and_fixed_variables", "empty_columns", "empty_rows", "singl
 # Kernel -> the source files whose text fixes its code; a DRAM traffic
 # figure measured by ncu is used only while these files are unchanged.
 KERNEL_SOURCES = {
-    "activity_kernel<false>": ["csrc/live.cu", "csrc/live_visit.cuh", "csrc/common.cuh"],
-    "activity_kernel<true>": ["csrc/live.cu", "csrc/live_visit.cuh", "csrc/common.cuh"],
+    "activity_kernel<Sums::kRecords>": ["csrc/live.cu", "csrc/live_visit.cuh", "csrc/common.cuh"],
+    "activity_kernel<Sums::kPlain>": ["csrc/live.cu", "csrc/live_visit.cuh", "csrc/common.cuh"],
     "candidates_entries": ["csrc/rules_bound.cu", "csrc/common.cuh"],
-    "compact_tiles<true>": ["csrc/compact.cu", "csrc/common.cuh"],
+    "compact_tiles": ["csrc/compact.cu", "csrc/scan.cuh", "csrc/common.cuh"],
 }
 
 

@@ -45,7 +45,7 @@ namespace {
 // three block barriers (the ticket, the warps' counts, the offset) against the
 // ten of a form that ranked and staged over the block, which took 287 us.  A
 // form whose warps walked the rows of their part stalled on long runs of empty
-// rows (1.5 ms a launch on the QAP N = 30 relaxation, 0.2 ms now).
+// rows (1.56 ms a launch on the QAP N = 30 relaxation, 0.06 ms now).
 constexpr int kCompactRounds = 8;
 constexpr int kCompactWarp = 32 * kCompactRounds;
 constexpr int kCompactWarps = kThreads / 32;

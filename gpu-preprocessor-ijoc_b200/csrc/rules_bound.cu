@@ -284,9 +284,10 @@ __device__ __forceinline__ uint32_t bound_records(uint32_t change, int sup_l, in
 // A column whose bounds stand costs its reads alone; the packed bounds and the
 // candidates, which the next sweep starts from, are written where they differ.
 // Bound by DRAM (41 bytes a column) where bounds stand, by the gathers of the
-// moved columns' rows else; a form that handed its tiles out in order
-// and looked back for the records before them took 442 us for the 29.8M-nnz
-// LP's columns, 69 us for the 2M-nnz one's.  Report: word 0 flags (1 infeasible, 2 a
+// moved columns' rows else: 376 us a sweep of the 29.8M-nnz LP's 5M columns, 446
+// before the maximum's walk ended early.  A form that handed its tiles out in order
+// and looked back for the records before them took 69 us against 45 at 500,001
+// columns.  Report: word 0 flags (1 infeasible, 2 a
 // bound moves, 4 a column is fixed), 1 records, 2 indices.
 __global__ void __launch_bounds__(kThreads, 3)
 finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,

@@ -370,12 +370,24 @@ void compact_sides(CompactSides& sides, DevCsr* const (&out)[2], cudaStream_t s)
   if (tiles == 0) return;
   const size_t parts = size_t(tiles) * kCompactWarps, words32 = parts * kCompactRounds;
   auto& c = ctx();
-  if (c.row_bits_words < words32) {   // zero between compactions
-    const size_t grown = std::max(words32, 2 * c.row_bits_words);
-    uint2* p = dalloc<uint2>(grown);
-    dfree(std::exchange(c.row_bits, p));
-    c.row_bits_words = grown;
-    check(cudaMemsetAsync(p, 0, sizeof(uint2) * grown, s), "row bits");
+  // Row bits, zero before and after: up to 1 MB stays with the context (a memset
+  // of a small model's costs as much as its kernels), past that they are the call's.
+  constexpr size_t kKeptRowBits = size_t(1) << 17;
+  DBuf<uint2> large_bits;
+  uint2* row_bits;
+  if (words32 > kKeptRowBits) {
+    large_bits.alloc(words32, s);
+    large_bits.zero();
+    row_bits = large_bits.p;
+  } else {
+    if (c.row_bits_words < words32) {
+      const size_t grown = std::min(kKeptRowBits, std::max(words32, 2 * c.row_bits_words));
+      uint2* p = dalloc<uint2>(grown);
+      dfree(std::exchange(c.row_bits, p));
+      c.row_bits_words = grown;
+      check(cudaMemsetAsync(p, 0, sizeof(uint2) * grown, s), "row bits");
+    }
+    row_bits = c.row_bits;
   }
   DBuf<uint32_t> masks(words32, s);
   DBuf<int32_t> before(parts, s);
@@ -383,11 +395,13 @@ void compact_sides(CompactSides& sides, DevCsr* const (&out)[2], cudaStream_t s)
   for (int k = 0; k < 2; ++k) {
     CompactSide& d = sides.side[k];
     const size_t first = k ? size_t(sides.side[0].tiles) * kCompactWarps : 0;
-    d.rows_at = c.row_bits + first * kCompactRounds;
+    d.rows_at = row_bits + first * kCompactRounds;
     d.masks = masks.p + first * kCompactRounds;
     d.before = before.p + first;
     d.part_kept = part_kept.p + first;
   }
+  // Every allocation before the first launch: one that fails leaves the bits zero.
+  LookbackSpace w(size_t(tiles), s);
   const int rows_grid = grid_stride_blocks(std::max(sides.side[0].rows, sides.side[1].rows));
   GPP_LAUNCH(compact_mark_rows, rows_grid, kThreads, 0, s, sides);
   // Reads; the writes (12 nnz') are added to the launch's profile record once
@@ -395,7 +409,6 @@ void compact_sides(CompactSides& sides, DevCsr* const (&out)[2], cudaStream_t s)
   double bytes = 0.0;
   for (const CompactSide& d : sides.side)
     if (d.tiles) bytes += 12.0 * d.nnz + 4.0 * d.cols + 0.375 * d.nnz;
-  LookbackSpace w(size_t(tiles), s);
   const Report report = c.open_report(2);
   GPP_LAUNCH_BYTES(compact_tiles, bytes, std::min(tiles, kNumSMs * 5), kThreads, 0, s, sides, w.words, w.counters,
                    c.host_error, report);

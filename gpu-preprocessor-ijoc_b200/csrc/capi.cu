@@ -818,7 +818,7 @@ int gpp_device_alloc(void** ptr, size_t bytes) {
 void gpp_device_free(void* p) {
   if (!p) return;
   try {
-    cudaFreeAsync(p, gpp::ctx().stream);
+    gpp::release_to_driver(p, gpp::ctx().stream);
     gpp::ctx().sync("device free");
   } catch (...) {
   }

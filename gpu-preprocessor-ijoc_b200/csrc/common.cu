@@ -9,8 +9,6 @@
 #include <chrono>
 #include <string>
 #include <memory>
-#include <mutex>
-#include <unordered_map>
 
 namespace gpp {
 
@@ -141,50 +139,23 @@ void inject_alloc_failure(int64_t after) { g_alloc_countdown.store(after < 0 ? -
 // thousand scratch buffers, each a cudaMallocFromPoolAsync / cudaFreeAsync
 // pair of driver calls on the host's critical path between launches.  Blocks
 // are rounded up to a size class (at most 25% over) and a block its own
-// context frees on that context's stream goes to the context's free list; the
-// next request of that class on that stream takes it back with no driver
-// call.  Reuse is safe without events: everything on one stream runs in issue
-// order, so a kernel that gets the block runs after every kernel that used it.
-// A block freed by another thread or on another stream goes back to the pool.
-// At most kCachedCap bytes are held this way across all contexts; past that a
-// freed block goes back to the pool.  The lists and the record of blocks in use
-// belong to the context, so the batched form's threads share nothing here but
-// the cap, drawn on in steps of kCreditStep.  GPP_ALLOC_CACHE=0 turns the reuse
-// off.
+// context frees on that context's stream goes to the context's book
+// (block_book.hpp); the next request of that class on that stream takes it back
+// with no driver call.  Reuse is safe without events: everything on one stream
+// runs in issue order, so a kernel that gets the block runs after every kernel
+// that used it.  A block freed by another thread or on another stream goes back
+// to the pool, and out of the book of the context that had handed it out: the
+// address may come back from any pool, as a block of another size.
+// At most BlockBook::kCap bytes are held this way across all contexts; past that
+// a freed block goes back to the pool.  The batched form's threads share nothing
+// here but that cap.  GPP_ALLOC_CACHE=0 turns the reuse off.
 namespace {
-std::atomic<int64_t> g_cache_credit{0};
-constexpr int64_t kCachedCap = int64_t(8) << 30;
-constexpr int64_t kCreditStep = int64_t(64) << 20;
-
 bool alloc_cache_on() {
   static const bool on = [] {
     const char* e = std::getenv("GPP_ALLOC_CACHE");
     return !(e && e[0] == '0');
   }();
   return on;
-}
-size_t size_class(size_t bytes) {
-  if (bytes <= 256) return 256;
-  const int high = 63 - __builtin_clzll(uint64_t(bytes));
-  const size_t grain = size_t(1) << std::max(8, high - 2);
-  return (bytes + grain - 1) / grain * grain;
-}
-// Index of a size class: its power of two and its quarter.
-int class_index(size_t cls) {
-  const int high = 63 - __builtin_clzll(uint64_t(cls));
-  return high * 4 + int((cls >> (high - 2)) & 3);
-}
-// Whether the context may hold `bytes` more.
-bool may_cache(Context& c, int64_t bytes) {
-  const int64_t over = c.cached_bytes + bytes - c.cache_credit;
-  if (over <= 0) return true;
-  const int64_t draw = (over + kCreditStep - 1) / kCreditStep * kCreditStep;
-  if (g_cache_credit.fetch_add(draw, std::memory_order_relaxed) + draw > kCachedCap) {
-    g_cache_credit.fetch_sub(draw, std::memory_order_relaxed);
-    return false;
-  }
-  c.cache_credit += draw;
-  return true;
 }
 }  // namespace
 
@@ -200,39 +171,26 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   }
   Context& c = ctx();
   if (!alloc_cache_on()) return cudaMallocFromPoolAsync(p, bytes, c.pool, s);
-  const size_t cls = size_class(bytes);
-  if (s == c.stream) {
-    auto& list = c.free_blocks[class_index(cls)];
-    if (!list.empty()) {
-      *p = list.back();
-      list.pop_back();
-      c.cached_bytes -= int64_t(cls);
-      c.handed_out[*p] = cls;
-      return cudaSuccess;
-    }
-  }
+  const size_t cls = BlockBook::size_class(bytes);
+  if (s == c.stream && (*p = c.blocks.take(cls))) return cudaSuccess;
   const cudaError_t e = cudaMallocFromPoolAsync(p, cls, c.pool, s);
-  if (e == cudaSuccess) c.handed_out[*p] = cls;
+  if (e == cudaSuccess) c.blocks.lend(*p, cls);
   return e;
 }
 
 void pool_free(void* p, cudaStream_t s) {
   if (!p) return;
   if (alloc_cache_on()) {
-    // A block of another context is in that context's record only; its entry
-    // there is overwritten when its pool hands the address out again.
     Context& c = ctx();
-    const auto it = c.handed_out.find(p);
-    if (it != c.handed_out.end()) {
-      const size_t cls = it->second;
-      c.handed_out.erase(it);
-      if (s == c.stream && may_cache(c, int64_t(cls))) {
-        c.cached_bytes += int64_t(cls);
-        c.free_blocks[class_index(cls)].push_back(p);
-        return;
-      }
-    }
+    const size_t cls = c.blocks.give_back(p);
+    if (cls == 0) BlockBook::forget(p);   // another context's
+    else if (s == c.stream && c.blocks.hold(p, cls)) return;
   }
+  cudaFreeAsync(p, s);
+}
+
+void release_to_driver(void* p, cudaStream_t s) {
+  if (alloc_cache_on()) BlockBook::forget(p);
   cudaFreeAsync(p, s);
 }
 

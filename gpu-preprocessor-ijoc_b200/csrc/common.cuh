@@ -10,11 +10,11 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
-#include <unordered_map>
 #include <utility>
 #include <vector>
 
 #include "../../include/gpp.h"
+#include "block_book.hpp"
 
 namespace gpp {
 
@@ -378,14 +378,9 @@ struct Context {
   int64_t answer[16] = {};
   void poll(const Mailbox* box, uint32_t seq, int words, const char* where);
   cudaStream_t side = nullptr;
-  // Scratch blocks this context freed on its own stream, by size class,
-  // ready to be handed out again without a driver call (pool_alloc/free), and
-  // the classes of the blocks it handed out.  Only this context's thread
-  // touches them.
-  static constexpr int kBlockClasses = 256;
-  std::vector<void*> free_blocks[kBlockClasses];
-  std::unordered_map<void*, size_t> handed_out;
-  int64_t cached_bytes = 0, cache_credit = 0;
+  // The blocks this context handed out and those it holds for reuse without a
+  // driver call (pool_alloc/free).
+  BlockBook blocks;
   static constexpr int kStatusWords = 64;
   // A second stream for host-to-device copies that overlap the engine
   // stream's kernels (created on first use; ordered by events).
@@ -408,6 +403,8 @@ Context& ctx();
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
 // Every engine device release (buffers of pool_alloc only).
 void pool_free(void* p, cudaStream_t s);
+// A release by the caller (gpp_device_free), of any device memory.
+void release_to_driver(void* p, cudaStream_t s);
 void inject_alloc_failure(int64_t after);
 
 template <class T>

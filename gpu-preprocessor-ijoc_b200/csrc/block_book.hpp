@@ -15,7 +15,7 @@ namespace gpp {
 class BlockBook {
  public:
   static constexpr int64_t kCap = int64_t(8) << 30;          // bytes held by all books
-  static constexpr int64_t kCreditStep = int64_t(64) << 20;  // a book draws on the cap in these steps
+  static constexpr int64_t kCreditStep = int64_t(64) << 20;  // a book draws on the cap, and returns, in these steps
 
   BlockBook() {
     std::lock_guard<std::mutex> lock(registry().mu);
@@ -40,6 +40,7 @@ class BlockBook {
     list.pop_back();
     held_ -= int64_t(cls);
     lend(p, cls);
+    return_credit();
     return p;
   }
   // The pool has handed out a block.
@@ -103,6 +104,15 @@ class BlockBook {
     }
     credit_ += draw;
     return true;
+  }
+
+  // Credit past what is held goes back in whole steps, but for one: blocks that
+  // come and go within a step draw and return nothing.
+  void return_credit() {
+    const int64_t spare = (credit_ - held_) / kCreditStep - 1;
+    if (spare <= 0) return;
+    credit_ -= spare * kCreditStep;
+    drawn().fetch_sub(spare * kCreditStep, std::memory_order_relaxed);
   }
 
   // The record of blocks in use is the one part that other threads reach (forget).

@@ -44,8 +44,32 @@ static int freed_elsewhere() {
   return 0;
 }
 
+// What one context held does not stay taken from the others once its blocks are in
+// use again, and all together hold no more than the cap.
+static int credit_returns() {
+  BlockBook* a = new BlockBook;
+  BlockBook* b = new BlockBook;
+  const size_t cls = BlockBook::size_class(size_t(64) << 20);
+  const int64_t most = BlockBook::kCap / int64_t(cls);
+  for (int64_t k = 1; k <= most; ++k) CHECK(a->hold(address(k), cls));
+  CHECK(!a->hold(address(most + 1), cls) && !b->hold(address(most + 1), cls));
+  for (int64_t k = 1; k <= most; ++k) CHECK(a->take(cls) != nullptr);
+  CHECK(a->held() == 0 && a->credit() <= 2 * BlockBook::kCreditStep);
+  int64_t held = 0;
+  while (b->hold(address(1000 + held), cls)) ++held;
+  CHECK(held >= most - 2 && held <= most);
+  CHECK(b->held() + a->credit() <= BlockBook::kCap && b->credit() >= b->held());
+  // Small blocks that come and go within a step return nothing.
+  const size_t small = BlockBook::size_class(4096);
+  CHECK(a->hold(address(5), small));
+  const int64_t credit = a->credit();
+  CHECK(a->take(small) == address(5) && a->credit() == credit && a->hold(address(5), small) && a->credit() == credit);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "freed_elsewhere")) return freed_elsewhere();
+  if (argc == 2 && !std::strcmp(argv[1], "credit_returns")) return credit_returns();
   std::printf("unknown check\n");
   return 2;
 }

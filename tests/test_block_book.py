@@ -21,7 +21,7 @@ def program(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["freed_elsewhere"])
+@pytest.mark.parametrize("check", ["freed_elsewhere", "credit_returns"])
 def test_book(program, check):
     r = subprocess.run([program, check], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout

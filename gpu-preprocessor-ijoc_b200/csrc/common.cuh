@@ -417,8 +417,8 @@ struct DBuf {
   void alloc(size_t count, cudaStream_t stream = nullptr) {
     release();
     s = stream ? stream : ctx().stream;
-    n = count;
     if (count) check(pool_alloc(reinterpret_cast<void**>(&p), count * sizeof(T), s), "cudaMallocFromPoolAsync");
+    n = count;   // not before: a buffer that outlives a failed call holds nothing, not `count` of nothing
   }
   void release() {
     if (p) pool_free(p, s);

@@ -806,6 +806,7 @@ int gpp_sort_pairs_static(uint64_t* keys, int32_t* values, int64_t n, void* stre
 }
 
 void gpp_inject_alloc_failure(int64_t after) { gpp::inject_alloc_failure(after); }
+void gpp_inject_sort_wait_limit(int polls) { gpp::inject_sort_wait_limit(polls); }
 
 int gpp_device_alloc(void** ptr, size_t bytes) {
   return guarded([&] {

@@ -14,6 +14,7 @@
 // sort waits for nothing).
 #include "sort.hpp"
 
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -201,6 +202,7 @@ struct SortPlan {
   int source[kMaxPasses + 1];   // 0 the caller's arrays, 1 the scratch copy; the last entry after all passes
   unsigned int tickets[kMaxPasses];
   unsigned int blocks_done;
+  int failed;   // a look-back's wait ran out
 };
 
 __global__ void __launch_bounds__(kThreads)
@@ -283,8 +285,14 @@ __device__ __forceinline__ void st_word(unsigned long long* p, unsigned long lon
 }
 
 // One pass over one tile.  Tiles are taken in ticket order, so every tile that
-// a look-back waits for is running; a wait still gives up after kPolls polls,
-// sets the error word that the host checks at its next wait, and goes on.
+// a look-back waits for is running; a wait still gives up after `max_polls` polls
+// and sets the error word that the host checks at its next wait.  The tile goes on
+// with a count that is too small: its pairs stay within their digits' ranges, but
+// some positions of the pass are then never written.  The later passes, whose digit
+// counts would no longer hold, are marked constant and so do not run (a flag of its
+// own, looked at as each pass starts, took 9 us of a sort of 2 million pairs), and
+// the last launch gives every pair key and value 0, which the kernels between here
+// and the host's check can use as an index.
 // Bound by the memory traffic (24 bytes a pair) and the ranking; tiles of
 // kItems x 256 pairs: sixteen items keep the look-back short against the
 // tile's work on large inputs, eight spread mid-size inputs over the SMs.
@@ -292,6 +300,7 @@ __device__ __forceinline__ void st_word(unsigned long long* p, unsigned long lon
 // of scan, scatter), 317 now; the look-back by one tile a round trip took 327
 // (and 129 against 113 for 250,000 pairs).
 constexpr int kPolls = 1 << 22;
+std::atomic<int> g_max_polls{kPolls};
 
 template <int kItems>
 struct SortTile {
@@ -304,7 +313,7 @@ constexpr int kAhead = 4;
 template <int kItems, class Word>
 __global__ void __launch_bounds__(kThreads, kItems == 8 ? 4 : 3)   // as shared memory allows
 sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int64_t n, int pass, int shift,
-          SortPlan* plan, Word* words, int32_t* error) {
+          SortPlan* plan, Word* words, int max_polls, int32_t* error) {
   after_previous_kernel();
   constexpr int kPairs = SortTile<kItems>::kPairs;
   using W = TileWord<Word>;
@@ -388,7 +397,9 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
       for (int q = 0; q < kAhead; ++q) {
         if (done) continue;
         for (int polls = 1; (w[q] >> W::kShift) == 0; ++polls) {
-          if (polls == kPolls) {
+          if (polls >= max_polls) {
+            plan->failed = 1;
+            for (int p = pass + 1; p < kMaxPasses; ++p) plan->constant[p] = 1;
             *reinterpret_cast<volatile int32_t*>(error) = 1;
             __threadfence_system();   // before any answer
             w[q] = W::kAll;
@@ -413,15 +424,16 @@ sort_pass(uint64_t* keys0, int32_t* vals0, uint64_t* keys1, int32_t* vals1, int6
 }
 
 // The pairs back into the caller's arrays when the passes left them in the
-// scratch copy.
+// scratch copy; zeros after a failed pass.
 __global__ void sort_copy_back(int64_t n, int passes, const SortPlan* __restrict__ plan, uint64_t* __restrict__ keys,
                                int32_t* __restrict__ vals, const uint64_t* __restrict__ from_keys,
                                const int32_t* __restrict__ from_vals) {
   after_previous_kernel();
-  if (plan->source[passes] == 0) return;
+  const bool failed = plan->failed != 0;
+  if (plan->source[passes] == 0 && !failed) return;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    keys[i] = from_keys[i];
-    vals[i] = from_vals[i];
+    keys[i] = failed ? 0 : from_keys[i];
+    vals[i] = failed ? 0 : from_vals[i];
   }
 }
 
@@ -458,11 +470,14 @@ void sort_tiles(uint64_t* keys, int32_t* vals, int64_t n, const SortPasses& pass
   GPP_LAUNCH_BYTES(sort_histogram, 8.0 * n, grid_stride_blocks(n, kThreads, 4), kThreads, 0, s, keys, n, passes, plan);
   for (int p = 0; p < passes.count; ++p)
     GPP_LAUNCH_BYTES((sort_pass<kItems, Word>), 24.0 * n, int(tiles), kThreads, SortTile<kItems>::kBytes, s, keys, vals,
-                     k2.p, v2.p, n, p, passes.shift[p], plan, tile_words + words * size_t(p), ctx().host_error);
+                     k2.p, v2.p, n, p, passes.shift[p], plan, tile_words + words * size_t(p),
+                     g_max_polls.load(std::memory_order_relaxed), ctx().host_error);
   GPP_LAUNCH(sort_copy_back, grid_stride_blocks(n), kThreads, 0, s, n, passes.count, plan, keys, vals, k2.p, v2.p);
 }
 
 }  // namespace
+
+void inject_sort_wait_limit(int polls) { g_max_polls.store(polls > 0 ? polls : kPolls); }
 
 void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, uint64_t may_vary) {
   if (n <= 1 || may_vary == 0) return;

@@ -12,6 +12,8 @@ inline uint64_t bits_up_to(int64_t top) {
 // key bits to sort by: those that can differ between keys, or only the upper
 // ones of them when the input is already in order by the lower ones.
 void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, uint64_t may_vary = ~uint64_t(0));
+// Test hook: the polls after which a look-back gives up (<= 0 for the default).
+void inject_sort_wait_limit(int polls);
 // The same sort with its scratch in a fixed device array (no allocation);
 // n is at most GPP_SORT_STATIC_MAX_PAIRS.
 void radix_sort_pairs_static(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s);

@@ -627,6 +627,12 @@ GPP_API void gpp_device_free(void* device_ptr);
  * device is not touched, so later calls run normally. */
 GPP_API void gpp_inject_alloc_failure(int64_t after);
 
+/* Test hook for failure handling: the number of polls after which a tile of a
+ * device sort stops waiting for the counts of the tiles before it (about 4
+ * million by default; `polls` <= 0 restores that).  A sort whose wait ran out
+ * leaves keys and values of 0, and the call that made it returns GPP_ERR_CUDA. */
+GPP_API void gpp_inject_sort_wait_limit(int polls);
+
 /* Last error message of the calling thread ("" when none). */
 GPP_API const char* gpp_last_error(void);
 

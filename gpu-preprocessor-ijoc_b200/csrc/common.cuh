@@ -245,9 +245,12 @@ __device__ __forceinline__ int block_append(int32_t* counter, bool take) {
 // at 20,000 x 50,000 it is the slower form (a presolve 8.85 against 7.0 ms).
 constexpr int kSmallCluster = 8;
 constexpr int kSmallModel = 8192;
+// The forms without .aligned: a warp's lanes come here from loops that they leave at
+// different trips, and the aligned ones want all of a warp's threads to execute the
+// instruction together.
 __device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------

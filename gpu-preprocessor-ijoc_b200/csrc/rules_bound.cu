@@ -269,7 +269,7 @@ struct FinalBounds {
   uint8_t* change;
   int32_t *sup_l, *sup_u;
   uint32_t* tile_counts;
-  int2* before;
+  longlong2* before;   // four indices a column: past 2^31 from 537 million columns on
 };
 // A column's records and their indices, 16 bits each.
 __device__ __forceinline__ uint32_t bound_records(uint32_t change, int sup_l, int sup_u) {
@@ -288,7 +288,7 @@ __device__ __forceinline__ uint32_t bound_records(uint32_t change, int sup_l, in
 // before the maximum's walk ended early.  A form that handed its tiles out in order
 // and looked back for the records before them took 69 us against 45 at 500,001
 // columns.  Report: word 0 flags (1 infeasible, 2 a
-// bound moves, 4 a column is fixed), 1 records, 2 indices.
+// bound moves, 4 a column is fixed), 1-2 records, 3-4 indices (low half first).
 __global__ void __launch_bounds__(kThreads, 3)
 finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const double* __restrict__ l,
                 const double* __restrict__ u, double* __restrict__ cand_l, double* __restrict__ cand_u,
@@ -355,8 +355,8 @@ finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const do
   if (!last_to_report(report)) return;
   if (records) {
     constexpr int kEach = 4;
-    __shared__ int2 warp_totals[kThreads / 32];
-    int2 total = make_int2(0, 0);
+    __shared__ int2 warp_totals[kThreads / 32];   // of 1,024 tiles at a time
+    longlong2 total = make_longlong2(0, 0);
     for (int first = 0; first < tiles; first += kThreads * kEach) {
       uint32_t v[kEach];
       int2 own = make_int2(0, 0);
@@ -375,7 +375,7 @@ finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const do
       }
       if (lane == 31) warp_totals[warp] = upto;
       __syncthreads();
-      int2 at = make_int2(total.x + upto.x - own.x, total.y + upto.y - own.y);
+      longlong2 at = make_longlong2(total.x + upto.x - own.x, total.y + upto.y - own.y);
 #pragma unroll
       for (int w = 0; w < kThreads / 32; ++w) {
         const int2 s = warp_totals[w];
@@ -394,8 +394,10 @@ finalize_kernel(int n, int tiles, const uint8_t* __restrict__ keep_col, const do
     }
     if (threadIdx.x == 0) {
       out.before[tiles] = total;
-      report.words[1] = total.x;
-      report.words[2] = total.y;
+      report.words[1] = int32_t(total.x);
+      report.words[2] = int32_t(total.x >> 32);
+      report.words[3] = int32_t(total.y);
+      report.words[4] = int32_t(total.y >> 32);
     }
     __syncthreads();
   }
@@ -430,7 +432,7 @@ commit_bounds(int n, int tiles, FinalBounds f, bool records, BoundRecords rec, d
     }
     const bool lc = change & 1u, uc = change & 2u;
     int sl = INT_MAX, su = INT_MAX;
-    int2 at = make_int2(0, 0);
+    longlong2 at = make_longlong2(0, 0);
     if (records) {
       at = f.before[t];
       if (f.before[t + 1].x != at.x) {   // block-uniform: the tile has records
@@ -593,7 +595,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   const int tiles = int((int64_t(n) + kThreads - 1) / kThreads);
   DBuf<int32_t> sl, su;
   DBuf<uint32_t> tile_counts;
-  DBuf<int2> before;
+  DBuf<longlong2> before;
   if (records) {
     sl.alloc(size_t(n), s);
     su.alloc(size_t(n), s);
@@ -604,7 +606,7 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   const double support_tol = std::fmax(10.0 * p.bound_tol, 1.0e-10);
   const SupportArgs support{lp.AT.ptr, lp.AT.idx, lp.AT.val, plan.keep_row.p, rows,
                             p.zero_tol, p.bound_tol, support_tol};
-  Report report = ctx().open_report(3);
+  Report report = ctx().open_report(5);
   GPP_LAUNCH(finalize_kernel, std::min(tiles, kNumSMs * 12), kThreads, 0, s, n, tiles, plan.keep_col.p, plan.l.p,
              plan.u.p, plan.cand_l.p, plan.cand_u.p, plan.lu.p, plan.c.p,
              int(p.bound_strengthening_preserve_free_zero_cost), p.feasibility_tol,
@@ -616,7 +618,8 @@ void rule_bound_strengthening(Plan& plan, const WorkingLp& lp, const Stats& stat
   if (!changed && !fixed) return;
   BoundRecords rec{};
   PostsolveSegment seg;
-  const int64_t recs = answer[1], nidx = answer[2];
+  const auto count_of = [answer](int k) { return int64_t(uint32_t(answer[k])) | answer[k + 1] << 32; };
+  const int64_t recs = count_of(1), nidx = count_of(3);
   if (recs) {
     seg = make_segment(recs, nidx, 4 * recs);
     rec = BoundRecords{seg.types.p, seg.is.p, seg.vs.p, seg.idx.p, seg.val.p};

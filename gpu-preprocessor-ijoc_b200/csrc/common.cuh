@@ -240,11 +240,23 @@ __device__ __forceinline__ int block_append(int32_t* counter, bool take) {
 // cluster: its hardware barrier, which also orders the blocks' accesses to global
 // memory, stands where the launches did, and its blocks are scheduled together, so
 // nothing spins.  Eight blocks is the portable size.  Such a chain costs about as
-// much as one of its launches while eight SMs keep up with the work: up to 8,192
-// rows and columns.  At 2,000 x 5,000 the Cleanup chain takes 20 us in place of 51;
-// at 20,000 x 50,000 it is the slower form (a presolve 8.85 against 7.0 ms).
+// much as one of its launches while eight SMs keep up with the work, which is rows
+// and columns in some stages and entries in the others, so both are bounded.  A
+// presolve with the cluster and without it:
+//   rows x columns       entries   with     without
+//   400 x 1,117            5,100   1.93 ms  1.96 ms
+//   3,000 x 7,500         18,000   2.31     2.37
+//   2,000 x 5,000         25,600   1.83     1.84
+//   3,000 x 7,500         33,000   1.36     1.36
+//   3,000 x 7,500         63,000   0.99     0.93
+//   3,000 x 7,500        963,000   2.50     1.80
+//   20,000 x 50,000      240,000   8.85     7.0
 constexpr int kSmallCluster = 8;
 constexpr int kSmallModel = 8192;
+constexpr offset_t kSmallEntries = 32768;
+inline bool small_model(int rows, int cols, offset_t nnz) {
+  return rows <= kSmallModel && cols <= kSmallModel && nnz <= kSmallEntries;
+}
 // The forms without .aligned: a warp's lanes come here from loops that they leave at
 // different trips, and the aligned ones want all of a warp's threads to execute the
 // instruction together.

@@ -903,7 +903,7 @@ void refresh_stats(Stats& st, const WorkingLp& lp, const Plan& plan) {
   } else {
     const uint32_t seq = ++ctx().nnz_seq;
     Mailbox* const box = ctx().nnz_box(seq);
-    if (std::max(m, n) <= kSmallModel) {
+    if (small_model(m, n, lp.A.nnz)) {
       GPP_LAUNCH_BYTES(inc_small, 2.0 * (double(m) + n), kSmallCluster, kThreads, 0, s, m, n, st.seen_row.p,
                        st.seen_col.p, st.deleted.p, st.counters.p, rows, cols, st.live_nnz.p, box, seq);
     } else {

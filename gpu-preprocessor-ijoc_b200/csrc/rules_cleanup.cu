@@ -276,7 +276,7 @@ uint32_t cleanup_probe(Plan& plan, const WorkingLp& lp, const Stats& stats, cons
                     stats.row_nnz.p, stats.singleton_row.p, stats.srow_col.p, stats.srow_val.p, p.bound_tol, p.zero_tol,
                     plan.sc_owner.p, plan.sc_words.p};
   if (ahead && (n == 0 || m == 0)) ahead = nullptr;
-  if (ahead && std::max(n, m) <= kSmallModel) return probe_and_ask_singleton_columns(g, *ahead, plan, lp, stats, p);
+  if (ahead && small_model(m, n, lp.A.nnz)) return probe_and_ask_singleton_columns(g, *ahead, plan, lp, stats, p);
   const Report report = ctx().open_report(1);
   GPP_LAUNCH_BYTES(cleanup_probe_kernel, 18.0 * n + 10.0 * m, grid_stride_blocks(std::max(m, n)), kThreads, 0, s, g,
                    report);

@@ -1,0 +1,58 @@
+"""Dense models under the forms that suit sparse ones: which kernels they take, and
+that the model and the recovered point are the oracle's bit for bit."""
+import numpy as np
+import pytest
+
+import pyoracle
+from gpp_b200 import capi, device, lpgen
+from test_gpu_large_groups import compare
+
+pytestmark = pytest.mark.gpu
+
+
+def dense_lp(m, n, per, seed, slack=None):
+    """m rows of `per` entries over n columns; with `slack`, equality rows with a singleton
+    column each, bounded below ("bounded") or free with a cost ("free")."""
+    rng = np.random.default_rng(seed)
+    idx = np.concatenate([np.sort(rng.choice(n, per, replace=False)) for _ in range(m)])
+    val = np.round(rng.uniform(-10.0, 10.0, m * per), 3) + 0.0005
+    rows = np.repeat(np.arange(m), per)
+    u = rng.uniform(1.0, 10.0, n)
+    act = np.bincount(rows, weights=val * (rng.random(n) * u)[idx], minlength=m)
+    l, c = np.zeros(n), rng.standard_normal(n)
+    AL = np.where(rng.random(m) < 0.6, act - rng.uniform(0.5, 5.0, m), -np.inf)
+    AU = np.where(rng.random(m) < 0.6, act + rng.uniform(0.5, 5.0, m), np.inf)
+    if slack:
+        rows, idx = np.concatenate([rows, np.arange(m)]), np.concatenate([idx, n + np.arange(m)])
+        val = np.concatenate([val, np.where(rng.random(m) < 0.5, 1.0, -1.0)])
+        l = np.concatenate([l, np.full(m, -np.inf if slack == "free" else 0.0)])
+        u = np.concatenate([u, np.full(m, np.inf)])
+        c = np.concatenate([c, rng.standard_normal(m) if slack == "free" else np.zeros(m)])
+        AL, AU, n = act.copy(), act.copy(), n + m
+    p, i, v = lpgen.coo_to_csr(m, rows, idx, val)
+    return lpgen.HostLP(m, n, p, i, v, c, AL, AU, l, u).ensure_transpose()
+
+
+def kernels_of(call):
+    lib = capi.load()
+    lib.gpp_profile_enable(1)
+    try:
+        call()
+        return [name for name, *_ in capi.profile_read()]
+    finally:
+        lib.gpp_profile_enable(0)
+
+
+def presolve(lp, params):
+    dlp = device.DeviceLp(lp)
+    return lambda: device.free_summary(device.preprocess(dlp, params))
+
+
+@pytest.mark.parametrize("m,per,fused", [(256, 128, True), (257, 128, False), (1000, 300, False)])
+def test_small_models_are_bounded_by_entries(m, per, fused):
+    params = capi.Params.defaults(enable_folding=0)
+    lp = dense_lp(m, 2000, per - 1, seed=m, slack="bounded")   # m * per entries: the line is at 32,768
+    names = kernels_of(presolve(lp, params))
+    assert any("probe_and_singleton_columns" in k for k in names) == fused, names
+    assert fused or not any("inc_small" in k for k in names), names
+    compare(lp, params)

@@ -635,8 +635,14 @@ __global__ void rg_replay_groups(TapeView t, int64_t lo, int listed, const uint6
 // short is bound by launches: the passes above cost about eight launches and
 // a wait each, and one thread alone walks a record in 1-2 us (the 400 x 1,000
 // slack LP's tape took 0.47 ms; with the block its call went from 7.1 to
-// 6.5 ms).
+// 6.5 ms).  A record's entries are walked by one thread, three times a pass, so
+// past one record a thread the grid's threads are worth more than the launches
+// once the records are long: 1,000 records of 23, 43, 163 and 323 entries take 130,
+// 168, 437 and 766 us in the block and about 130, 143, 236 and 358 us on the grid.
+// The line is drawn on the entries walked: the tape's indices, and a row or column
+// of the model for each record, which some types walk.
 constexpr int kBlockTape = 2048;
+constexpr double kBlockTapeEntries = 65536.0;
 constexpr int kBlockReplayThreads = 512;
 __global__ void __launch_bounds__(kBlockReplayThreads)
 replay_block(TapeView t, int64_t lo, int count, int primal, int dual, int m, int n, Sol s, Model M, int32_t* owner) {
@@ -698,14 +704,14 @@ replay_block(TapeView t, int64_t lo, int count, int primal, int dual, int m, int
 }
 
 // Replays the records [lo, hi) of the whole tape (global indices): the primal
-// pass, the dual pass or both.
-void replay_range(const TapeView& t, int m0, int n0, const Sol& s, const Model& M, bool primal, bool dual,
-                  cudaStream_t st, int64_t lo, int64_t hi) {
+// pass, the dual pass or both.  A record walks about `entries` entries.
+void replay_range(const TapeView& t, double entries, int m0, int n0, const Sol& s, const Model& M, bool primal,
+                  bool dual, cudaStream_t st, int64_t lo, int64_t hi) {
   if (lo >= hi) return;
   if (hi - lo > INT32_MAX) throw LengthError("postsolve: more than 2^31 - 1 tape records");
   const int count = int(hi - lo);
   const size_t resources = size_t(m0) + size_t(n0);
-  if (count <= kBlockTape) {
+  if (count <= kBlockReplayThreads || (count <= kBlockTape && entries * count <= kBlockTapeEntries)) {
     DBuf<int32_t> owner(std::max<size_t>(resources, 1), st);
     owner.zero();
     GPP_LAUNCH(replay_block, 1, kBlockReplayThreads, 0, st, t, lo, count, int(primal), int(dual), m0, n0, s, M,
@@ -890,17 +896,19 @@ void run_postsolve(const PresolveOutput& out, const double* x_red, const double*
   // records after a checkpoint, then its recovery (postsolve_gpu,
   // gpu_postsolve.cu:637-663); the dual pass over the whole tape.
   int64_t range_end = r.records;
+  double entries = total ? double(r.indices) / double(total) : 0.0;
+  if (original) entries += double(original->A.nnz) / std::max(1, std::min(m0, n0));
   for (auto it = r.timeline.rbegin(); it != r.timeline.rend(); ++it) {
-    replay_range(t, m0, n0, s, M, true, false, st, it->tape_position, range_end);
+    replay_range(t, entries, m0, n0, s, M, true, false, st, it->tape_position, range_end);
     if (it->kind == 0) restore_absolute_value(x, r.absval[size_t(it->payload)], lower, st);
     else restore_variable_pair(x, r.varpair[size_t(it->payload)], st);
     range_end = it->tape_position;
   }
   if (r.timeline.empty()) {
-    replay_range(t, m0, n0, s, M, true, true, st, 0, r.records);
+    replay_range(t, entries, m0, n0, s, M, true, true, st, 0, r.records);
   } else {
-    replay_range(t, m0, n0, s, M, true, false, st, 0, range_end);
-    replay_range(t, m0, n0, s, M, false, true, st, 0, r.records);
+    replay_range(t, entries, m0, n0, s, M, true, false, st, 0, range_end);
+    replay_range(t, entries, m0, n0, s, M, false, true, st, 0, r.records);
   }
   if (original && y && z && n0) {
     if (total) GPP_LAUNCH(mark_protected, grid_stride_blocks(total), kThreads, 0, st, t, prot, n0);

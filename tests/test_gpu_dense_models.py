@@ -56,3 +56,24 @@ def test_small_models_are_bounded_by_entries(m, per, fused):
     assert any("probe_and_singleton_columns" in k for k in names) == fused, names
     assert fused or not any("inc_small" in k for k in names), names
     compare(lp, params)
+
+
+@pytest.mark.parametrize("m,per,block", [(512, 300, True), (520, 40, True), (520, 300, False), (2040, 4, True), (2040, 60, False)])
+def test_short_tapes_of_long_records(m, per, block):
+    import torch
+    params = capi.Params.defaults(enable_folding=0)
+    lp = dense_lp(m, 2000, per, seed=m + per, slack="free")   # one substitution a row, of `per` entries
+    dlp = device.DeviceLp(lp)
+    s = device.preprocess(dlp, params)
+    try:
+        gpu = device.Result(s)
+        assert len(gpu.tape_types) >= m and (block or len(gpu.tape_types) <= 2048)
+        rng = np.random.default_rng(1)
+        point = [rng.standard_normal(k) for k in (s.reduced_cols, s.reduced_rows, s.reduced_cols)]
+        got = []
+        names = kernels_of(lambda: got.extend(device.postprocess(*(torch.from_numpy(v).cuda() for v in point), s, dlp)))
+        assert any("replay_block" in k for k in names) == block, (len(gpu.tape_types), names)
+        for a, b in zip(got, pyoracle.presolve(lp, params).postsolve(*point)):
+            assert np.array_equal(a, b)
+    finally:
+        device.free_summary(s)

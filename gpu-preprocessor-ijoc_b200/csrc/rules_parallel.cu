@@ -54,8 +54,8 @@ __device__ void row_hash_thread(const RowHashArgs& g, int i) {
   g.out[i] = g.use_xor ? mix(h, agg) : h;
 }
 
-// Long rows (past kLongRow stored entries), eight to a block.  The FNV fold
-// visits a row's entries in stored order, two dependent 64-bit multiplications
+// Long rows (past kLongRow stored entries) under the ordered fold, eight to a
+// block.  The fold visits a row's entries in stored order, two dependent 64-bit multiplications
 // each (about 75 us for a 5,000-entry row), so eight lanes of one warp fold a
 // row each and do nothing else; the other seven warps form the next stage of
 // the rows' (column, bits of value / pivot) pairs in shared memory meanwhile,
@@ -112,7 +112,7 @@ __device__ void row_hash_block(const RowHashArgs& g, const int32_t* rows, int co
   const offset_t from = row >= 0 && row < kHashRows ? from_shared[row] : 0;
   const offset_t end = row >= 0 && row < kHashRows ? end_shared[row] : 0;
   const double pivot = pivot_shared[row >= 0 && row < kHashRows ? row : 0];
-  uint64_t h = folds ? mix(kFnvOffset, uint64_t(len_shared[row])) : 0, agg = 0;
+  uint64_t h = folds ? mix(kFnvOffset, uint64_t(len_shared[row])) : 0;
   for (int c = 0; c <= chunks; ++c) {
     if (warp > 0 && c < chunks) {
       const int64_t base = int64_t(from) + int64_t(c) * kHashStage + slot;
@@ -141,23 +141,21 @@ __device__ void row_hash_block(const RowHashArgs& g, const int32_t* rows, int co
       for (int k = 0; k < n; ++k) {
         const int32_t j = last.col[row][k];
         const uint64_t b = last.bits[row][k];
-        if (j < 0) continue;
-        if (g.use_xor) agg ^= mix(mix(kFnvOffset, uint64_t(j)), b);
-        else h = mix(mix(h, uint64_t(j)), b);
+        if (j >= 0) h = mix(mix(h, uint64_t(j)), b);
       }
     }
     __syncthreads();
   }
-  if (folds && row < count && from < end) g.out[rows[row]] = g.use_xor ? mix(h, agg) : h;
+  if (folds && row < count && from < end) g.out[rows[row]] = h;
   __syncthreads();
 }
 
-// A warp's 32 medium rows, one to a lane, eight stored entries of each per
-// round.  Eight lanes load a row's eight (four rows at a time), divide by its
-// pivot and stage the pairs in shared memory, where the row's lane folds them
-// in stored order (an entry's fold is a serial chain of 64-bit multiplies, so
-// one lane runs it; a form in which all eight lanes of a row ran it over
-// shuffles took 904 us at the 29.8M-nnz LP, this one 805).  A first sweep under a column mask
+// A warp's 32 medium rows under the ordered fold, one to a lane, eight stored
+// entries of each per round.  Eight lanes load a row's eight (four rows at a time),
+// divide by its pivot and stage the pairs in shared memory, where the row's lane
+// folds them in stored order (an entry's fold is a serial chain of 64-bit multiplies,
+// so one lane runs it; a form in which all eight lanes of a row ran it over shuffles
+// took 904 us at the 29.8M-nnz LP, this one 805).  A first sweep under a column mask
 // finds the live length and the first live entry (the pivot).  Rounds last as
 // long as the longest row; rows that have ended are passed over in fours.
 struct RowStage {
@@ -195,7 +193,7 @@ __device__ void row_hash_rows(const RowHashArgs& g, int i, RowStage& stage) {
   const bool trivial = !keep || len == 0 || fabs(g.val[first]) <= g.tol;
   const double pivot = trivial ? 1.0 : g.val[first];
   const offset_t from = trivial ? e : first;
-  uint64_t h = mix(kFnvOffset, uint64_t(len)), agg = 0;
+  uint64_t h = mix(kFnvOffset, uint64_t(len));
   for (int at = 0;; at += 8) {
     const unsigned need = __ballot_sync(kAll, e - from > at);
     if (!need) break;
@@ -228,9 +226,7 @@ __device__ void row_hash_rows(const RowHashArgs& g, int i, RowStage& stage) {
       for (int t = 0; t < 8; ++t) {
         const int32_t c = stage.col[lane * 9 + t];
         const uint64_t b = stage.bits[lane * 9 + t];
-        if (c < 0) continue;
-        if (g.use_xor) agg ^= mix(mix(kFnvOffset, uint64_t(c)), b);
-        else h = mix(mix(h, uint64_t(c)), b);
+        if (c >= 0) h = mix(mix(h, uint64_t(c)), b);
       }
     }
     __syncwarp();
@@ -238,8 +234,164 @@ __device__ void row_hash_rows(const RowHashArgs& g, int i, RowStage& stage) {
   if (i >= 0) {
     if (!keep) g.out[i] = uint64_t(i);
     else if (trivial) g.out[i] = mix(kFnvOffset, uint64_t(i));
-    else g.out[i] = g.use_xor ? mix(h, agg) : h;
+    else g.out[i] = h;
   }
+}
+
+// The ordered fold of few medium rows: four to a warp, eight lanes each, which all
+// run the row's fold over shuffles.  The form above keeps eight times fewer warps
+// busy, and each round of its warps is longer.  So this form while the grid has a warp
+// for every four rows: 1,000 rows of 300 entries take 49 us (62 under a column mask),
+// 91 (134) in the form above, 1,000 rows of 1,000 entries 108 (155) against 240 (382);
+// 100,000 rows of 64 entries, more than that, 54 (76) above and 91 (106) in fours.
+__device__ void row_hash_four(const RowHashArgs& g, int i) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int gl = threadIdx.x & 7, shift = int(threadIdx.x & 24);
+  const bool keep = i >= 0 && g.keep_row[i];
+  const offset_t a = keep ? g.ptr[i] : 0, e = keep ? g.ptr[i + 1] : 0;
+  int len = int(e - a);
+  offset_t first = a;
+  if (g.keep_col) {
+    len = 0;
+    first = -1;
+    for (int at = 0; __any_sync(kAll, e - a > at); at += 8) {
+      const bool live = e - a > at + gl && g.keep_col[__ldcs(g.idx + a + at + gl)];
+      const unsigned bits = __ballot_sync(kAll, live) >> shift & 0xffu;
+      if (first < 0 && bits) first = a + at + (__ffs(bits) - 1);
+      len += __popc(bits);
+    }
+  }
+  const bool trivial = !keep || len == 0 || fabs(g.val[first]) <= g.tol;
+  const double pivot = trivial ? 1.0 : g.val[first];
+  const offset_t from = trivial ? e : first;
+  uint64_t h = mix(kFnvOffset, uint64_t(len));
+  for (int at = 0; __any_sync(kAll, e - from > at); at += 8) {
+    const bool in = e - from > at + gl;
+    const int col = in ? __ldcs(g.idx + from + at + gl) : -1;
+    const double v = in ? __ldcs(g.val + from + at + gl) : 0.0;
+    const bool live = in && (!g.keep_col || g.keep_col[col]);
+    const uint64_t bits = live ? dbits(v / pivot) : 0;
+    const unsigned mask = __ballot_sync(kAll, live) >> shift & 0xffu;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const int c = __shfl_sync(kAll, col, t, 8);
+      const uint64_t b = __shfl_sync(kAll, bits, t, 8);
+      if (mask >> t & 1u) h = mix(mix(h, uint64_t(c)), b);
+    }
+  }
+  if (gl == 0 && i >= 0) g.out[i] = !keep ? uint64_t(i) : trivial ? mix(kFnvOffset, uint64_t(i)) : h;
+}
+
+// The XOR aggregate (dense matrices) takes a row's entries in any order, so there
+// is no fold to wait for: every lane of a row's group, eight lanes to a medium row
+// and a block to a long one, aggregates its own entries, four in flight.  One lane to a
+// row, as in the forms above, 200 rows of 20,000 entries took 956 us, 40 here, and
+// 1,000 rows of 300 entries 93 against 29.
+template <int W>
+__device__ __forceinline__ uint64_t group_xor(uint64_t v) {
+#pragma unroll
+  for (int off = W / 2; off; off >>= 1) v ^= __shfl_xor_sync(0xffffffffu, v, off, W);
+  return v;
+}
+// What a lane finds in its share of the row's entries.
+struct LiveShare {
+  int len = 0, first = INT_MAX;   // live entries, the first one's position in the row
+};
+__device__ __forceinline__ LiveShare live_share(const RowHashArgs& g, offset_t a, int size, int lane, int width) {
+  LiveShare s;
+  for (int64_t at = lane; at < size; at += 4 * width) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t q = at + k * width;
+      if (q < size && g.keep_col[__ldcs(g.idx + a + q)]) {
+        ++s.len;
+        s.first = min(s.first, int(q));
+      }
+    }
+  }
+  return s;
+}
+__device__ __forceinline__ uint64_t xor_share(const RowHashArgs& g, offset_t a, int size, double pivot, int lane,
+                                              int width) {
+  uint64_t agg = 0;
+  for (int64_t at = lane; at < size; at += 4 * width) {
+    int col[4];
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t q = at + k * width;
+      col[k] = q < size ? __ldcs(g.idx + a + q) : -1;
+      v[k] = q < size ? __ldcs(g.val + a + q) : 0.0;
+    }
+    if (g.keep_col) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (col[k] >= 0 && !g.keep_col[col[k]]) col[k] = -1;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (col[k] >= 0) agg ^= mix(mix(kFnvOffset, uint64_t(col[k])), dbits(v[k] / pivot));
+  }
+  return agg;
+}
+__device__ __forceinline__ uint64_t xor_hash(const RowHashArgs& g, int i, bool keep, bool trivial, int len, uint64_t agg) {
+  return !keep ? uint64_t(i) : trivial ? mix(kFnvOffset, uint64_t(i)) : mix(mix(kFnvOffset, uint64_t(len)), agg);
+}
+// Eight lanes a row; i < 0 for none.  All lanes of the warp call it.
+__device__ void row_xor_group(const RowHashArgs& g, int i) {
+  const int gl = threadIdx.x & 7;
+  const bool keep = i >= 0 && g.keep_row[i];
+  const offset_t a = keep ? g.ptr[i] : 0;
+  const int size = keep ? int(g.ptr[i + 1] - a) : 0;
+  int len = size, first = 0;
+  if (g.keep_col) {
+    const LiveShare s = live_share(g, a, size, gl, 8);
+    len = s.len;
+    first = s.first;
+#pragma unroll
+    for (int off = 4; off; off >>= 1) {
+      len += __shfl_xor_sync(0xffffffffu, len, off, 8);
+      first = min(first, __shfl_xor_sync(0xffffffffu, first, off, 8));
+    }
+  }
+  const bool trivial = !keep || len == 0 || fabs(g.val[a + first]) <= g.tol;
+  const uint64_t agg = group_xor<8>(trivial ? 0 : xor_share(g, a, size, g.val[a + first], gl, 8));
+  if (gl == 0 && i >= 0) g.out[i] = xor_hash(g, i, keep, trivial, len, agg);
+}
+__device__ void row_xor_block(const RowHashArgs& g, int i) {
+  __shared__ int lens[kThreads / 32], firsts[kThreads / 32];
+  __shared__ uint64_t aggs[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool keep = g.keep_row[i] != 0;
+  const offset_t a = g.ptr[i];
+  const int size = keep ? int(g.ptr[i + 1] - a) : 0;
+  int len = size, first = 0;
+  if (g.keep_col) {
+    const LiveShare s = live_share(g, a, size, threadIdx.x, kThreads);
+    len = __reduce_add_sync(0xffffffffu, s.len);
+    first = __reduce_min_sync(0xffffffffu, s.first);
+    if (lane == 0) {
+      lens[warp] = len;
+      firsts[warp] = first;
+    }
+    __syncthreads();
+    len = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+      len += lens[w];
+      first = min(first, firsts[w]);
+    }
+  }
+  const bool trivial = !keep || len == 0 || fabs(g.val[a + first]) <= g.tol;
+  uint64_t agg = group_xor<32>(trivial ? 0 : xor_share(g, a, size, g.val[a + first], threadIdx.x, kThreads));
+  if (lane == 0) aggs[warp] = agg;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < kThreads / 32; ++w) agg ^= aggs[w];
+    g.out[i] = xor_hash(g, i, keep, trivial, len, agg);
+  }
+  __syncthreads();   // the shares are reused by the block's next row
 }
 
 // Blocks for the long rows, which take longest, then for the medium and the
@@ -248,40 +400,76 @@ struct HashRoles {
   int long_blocks, medium_blocks, short_blocks;
   int grid() const { return long_blocks + medium_blocks + short_blocks; }
 };
-HashRoles hash_roles(int rows, offset_t nnz) {
-  return HashRoles{int(std::min<int64_t>(kNumSMs * 2, int64_t(nnz) / (int64_t(kLongRow) * kHashRows) + 1)),
+HashRoles hash_roles(int rows, offset_t nnz, bool use_xor) {
+  const int64_t long_rows = int64_t(nnz) / kLongRow + 1;   // at most
+  return HashRoles{int(use_xor ? std::min<int64_t>(kNumSMs * 4, long_rows)
+                               : std::min<int64_t>(kNumSMs * 2, (long_rows + kHashRows - 1) / kHashRows)),
                    int(std::min<int64_t>(kNumSMs * 8, (int64_t(rows) + 31) / 32)),
                    grid_stride_blocks(rows, kThreads, 16)};
 }
 
+template <bool Xor>
 __global__ void __launch_bounds__(kThreads)
 row_hash_kernel(int rows, RowHashArgs g, const int32_t* __restrict__ medium, const int32_t* __restrict__ longq,
                 const int32_t* __restrict__ counts, HashRoles roles) {
   after_previous_kernel();
-  __shared__ union {
-    HashStage block[2];
-    RowStage warp[kThreads / 32];
-  } stage;
   int b = blockIdx.x;
-  if (b < roles.long_blocks) {
-    const int count = counts[1];
-    for (int q = b * kHashRows; q < count; q += roles.long_blocks * kHashRows)
-      row_hash_block(g, longq + q, min(kHashRows, count - q), stage.block);
-    return;
-  }
-  b -= roles.long_blocks;
-  if (b < roles.medium_blocks) {   // 32 rows to a warp
-    const int nwarps = roles.medium_blocks * (kThreads / 32);
-    const int nmedium = counts[0];
-    for (int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 32; q0 < nmedium; q0 += nwarps * 32) {
-      const int q = q0 + int(threadIdx.x & 31);
-      row_hash_rows(g, q < nmedium ? medium[q] : -1, stage.warp[threadIdx.x >> 5]);
+  if constexpr (Xor) {
+    if (b < roles.long_blocks) {
+      for (int q = b; q < counts[1]; q += roles.long_blocks) row_xor_block(g, longq[q]);
+      return;
     }
-    return;
+    b -= roles.long_blocks;
+    if (b < roles.medium_blocks) {   // four rows to a warp
+      const int nwarps = roles.medium_blocks * (kThreads / 32);
+      const int nmedium = counts[0];
+      for (int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 4; q0 < nmedium; q0 += nwarps * 4) {
+        const int q = q0 + int(threadIdx.x & 31) / 8;
+        row_xor_group(g, q < nmedium ? medium[q] : -1);
+      }
+      return;
+    }
+  } else {
+    __shared__ union {
+      HashStage block[2];
+      RowStage warp[kThreads / 32];
+    } stage;
+    if (b < roles.long_blocks) {
+      const int count = counts[1];
+      for (int q = b * kHashRows; q < count; q += roles.long_blocks * kHashRows)
+        row_hash_block(g, longq + q, min(kHashRows, count - q), stage.block);
+      return;
+    }
+    b -= roles.long_blocks;
+    if (b < roles.medium_blocks) {   // 32 rows to a warp, or four while there are warps
+      const int nwarps = roles.medium_blocks * (kThreads / 32);
+      const int nmedium = counts[0];
+      if (nmedium <= nwarps * 4) {
+        const int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 4, q = q0 + int(threadIdx.x & 31) / 8;
+        if (q0 < nmedium) row_hash_four(g, q < nmedium ? medium[q] : -1);
+        return;
+      }
+      for (int q0 = (b * (kThreads / 32) + int(threadIdx.x >> 5)) * 32; q0 < nmedium; q0 += nwarps * 32) {
+        const int q = q0 + int(threadIdx.x & 31);
+        row_hash_rows(g, q < nmedium ? medium[q] : -1, stage.warp[threadIdx.x >> 5]);
+      }
+      return;
+    }
   }
   b -= roles.medium_blocks;
   for (int i = b * int(blockDim.x) + int(threadIdx.x); i < rows; i += roles.short_blocks * int(blockDim.x))
     if (g.ptr[i + 1] - g.ptr[i] <= kShortRow) row_hash_thread(g, i);
+}
+void launch_row_hash(const DevCsr& A, const RowHashArgs& g, cudaStream_t s) {
+  const RowSchedule& sch = stored_schedule(A);
+  const HashRoles roles = hash_roles(A.rows, A.nnz, g.use_xor);
+  const double bytes = 4.0 * (A.rows + 1) + 12.0 * A.nnz + A.rows + (g.keep_col ? A.cols : 0) + 8.0 * A.rows;
+  if (g.use_xor)
+    GPP_LAUNCH_BYTES(row_hash_kernel<true>, bytes, roles.grid(), kThreads, 0, s, A.rows, g, sch.medium.p,
+                     sch.long_rows.p, sch.counts.p, roles);
+  else
+    GPP_LAUNCH_BYTES(row_hash_kernel<false>, bytes, roles.grid(), kThreads, 0, s, A.rows, g, sch.medium.p,
+                     sch.long_rows.p, sch.counts.p, roles);
 }
 
 // Repeated-hash filter.  Only a hash that two or more live items share can
@@ -812,12 +1000,7 @@ void parallel_row_hashes(const DevCsr& A, const uint8_t* keep_row, const uint8_t
     check(cudaMemsetAsync(ones.p, 1, size_t(A.rows), s), "keep all rows");
     keep_row = ones.p;
   }
-  const RowSchedule& sch = stored_schedule(A);
-  const HashRoles roles = hash_roles(A.rows, A.nnz);
-  RowHashArgs g{A.ptr, A.idx, A.val, keep_row, keep_col, 1e-10, use_xor, hashes};
-  const double bytes = 4.0 * (A.rows + 1) + 12.0 * A.nnz + A.rows + (keep_col ? A.cols : 0) + 8.0 * A.rows;
-  GPP_LAUNCH_BYTES(row_hash_kernel, bytes, roles.grid(), kThreads, 0, s, A.rows, g, sch.medium.p, sch.long_rows.p,
-                   sch.counts.p, roles);
+  launch_row_hash(A, RowHashArgs{A.ptr, A.idx, A.val, keep_row, keep_col, 1e-10, use_xor, hashes}, s);
 }
 
 void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp_params& p) {
@@ -827,15 +1010,10 @@ void rule_parallel_rows(Plan& plan, const WorkingLp& lp, const Stats&, const gpp
   if (m <= 1) return;
   auto s = ctx().stream;
   DBuf<uint64_t> hash(size_t(m), s);
-  {
-    const bool use_xor = int64_t(lp.A.nnz) > 32LL * m;
-    const RowSchedule& sch = stored_schedule(lp.A);
-    const HashRoles roles = hash_roles(m, lp.A.nnz);
-    RowHashArgs g{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, plan.keep_col.p, p.zero_tol, use_xor, hash.p};
-    const double bytes = 4.0 * (m + 1) + 12.0 * lp.A.nnz + m + lp.n() + 8.0 * m;
-    GPP_LAUNCH_BYTES(row_hash_kernel, bytes, roles.grid(), kThreads, 0, s, m, g, sch.medium.p, sch.long_rows.p,
-                     sch.counts.p, roles);
-  }
+  launch_row_hash(lp.A,
+                  RowHashArgs{lp.A.ptr, lp.A.idx, lp.A.val, plan.keep_row.p, plan.keep_col.p, p.zero_tol,
+                              int64_t(lp.A.nnz) > 32LL * m, hash.p},
+                  s);
   DBuf<uint64_t> keys;
   DBuf<int32_t> ids;
   const int32_t count = sorted_live_hashes(hash.p, plan.keep_row.p, m, keys, ids, s);

@@ -748,14 +748,41 @@ struct SideStats {
   uint8_t* dirty;
 };
 
+// Still-kept items among entries p, p + step, .. of a deleted one: each loses one
+// degree and is marked dirty.  Returns their number.
+__device__ __forceinline__ int leave_inner(const SideStats& outer, const SideStats& inner, int64_t p, offset_t end,
+                                           int step) {
+  int left = 0;
+  for (; p < end; p += 4 * step) {
+    int c[4];
+    bool kept[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = end - p > k * step ? outer.idx[p + k * step] : -1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) kept[k] = c[k] >= 0 && inner.keep[c[k]];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (!kept[k]) continue;
+      atomicSub(inner.degree + c[k], 1);
+      inner.dirty[c[k]] = 1;
+      ++left;
+    }
+  }
+  return left;
+}
 // Deleted rows by the first half of the blocks, deleted columns by the rest
 // (the halves touch different items: a deleted item's own statistics, and the
-// degrees of kept items of the other side).  Eight lanes per deleted item: its
-// own statistics are reset, and every still-kept item it touches loses one
-// degree and is marked dirty.  The live total drops by a deleted row's old
-// degree and, for a deleted column, by one per kept row it leaves; added up in
-// registers, one atomic per warp (an atomic per item on the one total took 152
-// us when 0.8M rows went at once, on the QAP N = 30 relaxation).
+// degrees of kept items of the other side).  Eight lanes per deleted item, four items
+// to a warp, taken so that few items go to warps of their own; one of more than
+// kWideItem entries by its whole warp.  A deleted item's own statistics are reset, and
+// every still-kept item it touches loses one degree and is marked dirty.  The live total
+// drops by a deleted row's old degree and, for a deleted column, by one per kept row it
+// leaves; added up in registers, one atomic per warp (an atomic per item on the one total
+// took 152 us when 0.8M rows went at once, on the QAP N = 30 relaxation).  Bound by the
+// round trips of an item's entries: eight lanes to the 4 rows of 400,000 entries of a
+// 200,000 x 500,000 LP took 19.0 ms, a warp with one entry a lane in flight 6.6 ms, this
+// 2.8 ms.
+constexpr int kWideItem = 64;
 __device__ __forceinline__ void walk_deleted(int m, const int32_t* list, const int32_t* counters,
                                              const SideStats& rows, const SideStats& cols,
                                              unsigned long long* live_nnz) {
@@ -765,28 +792,31 @@ __device__ __forceinline__ void walk_deleted(int m, const int32_t* list, const i
   const SideStats& inner = row_side ? cols : rows;
   const int32_t* deleted = row_side ? list : list + m;
   const int count = counters[row_side ? 0 : 1];
-  const int gl = threadIdx.x & 7;
+  const int lane = threadIdx.x & 31, gl = lane & 7;
   const int block = row_side ? int(blockIdx.x) : int(blockIdx.x) - half;
-  const int blocks = row_side ? half : int(gridDim.x) - half;
+  const int64_t warps = int64_t(row_side ? half : int(gridDim.x) - half) * (kThreads / 32);
   unsigned long long dropped = 0;
-  for (int w = block * (kThreads / 8) + (threadIdx.x >> 3); w < count; w += blocks * (kThreads / 8)) {
-    const int r = deleted[w];
-    for (offset_t p = outer.ptr[r] + gl; p < outer.ptr[r + 1]; p += 8) {
-      const int c = outer.idx[p];
-      if (inner.keep[c]) {
-        atomicSub(inner.degree + c, 1);
-        inner.dirty[c] = 1;
-        if (!row_side) ++dropped;
-      }
+  for (int64_t w0 = block * (kThreads / 32) + (threadIdx.x >> 5); w0 < count; w0 += warps * 4) {
+    const int64_t w = w0 + (lane >> 3) * warps;
+    const bool have = w < count;
+    const int r = have ? deleted[w] : 0;
+    const offset_t first = have ? outer.ptr[r] : 0, end = have ? outer.ptr[r + 1] : 0;
+    const bool wide = end - first > kWideItem;
+    int left = wide ? 0 : leave_inner(outer, inner, int64_t(first) + gl, end, 8);
+    for (unsigned rest = __ballot_sync(0xffffffffu, wide && gl == 0); rest; rest &= rest - 1) {
+      const int src = __ffs(rest) - 1;
+      const offset_t f = __shfl_sync(0xffffffffu, first, src), e = __shfl_sync(0xffffffffu, end, src);
+      left += leave_inner(outer, inner, int64_t(f) + lane, e, 32);
     }
-    if (gl == 0) {
+    if (!row_side) dropped += unsigned(left);
+    if (have && gl == 0) {
       if (row_side) dropped += (unsigned long long)outer.degree[r];
       outer.degree[r] = 0; outer.empty[r] = 0; outer.singleton[r] = 0; outer.support[r] = -1;
       outer.coefficient[r] = 0.0;
     }
   }
   for (int off = 16; off; off >>= 1) dropped += __shfl_down_sync(0xffffffffu, dropped, off);
-  if ((threadIdx.x & 31) == 0 && dropped) atomicAdd(live_nnz, 0ULL - dropped);
+  if (lane == 0 && dropped) atomicAdd(live_nnz, 0ULL - dropped);
 }
 __global__ void __launch_bounds__(kThreads) inc_walk(int m, const int32_t* list, const int32_t* counters,
                                                      SideStats rows, SideStats cols, unsigned long long* live_nnz) {

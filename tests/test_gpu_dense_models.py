@@ -77,3 +77,28 @@ def test_short_tapes_of_long_records(m, per, block):
             assert np.array_equal(a, b)
     finally:
         device.free_summary(s)
+
+
+@pytest.mark.parametrize("n", [1200, 9000])   # the fused refresh, and the launches
+@pytest.mark.parametrize("seed", range(3))
+def test_statistics_after_long_rows_and_columns_go(n, seed):
+    """Rows without sides and columns with equal bounds go, of lengths around the rounds of a
+    lane group (8, 32) and of a warp (65, 128); what then has one entry or none is found by
+    the statistics that are left."""
+    rng = np.random.default_rng(seed)
+    lengths = [1, 2, 7, 8, 9, 31, 32, 33, 63, 64, 65, 66, 127, 128, 129, 193, 600, 1000]
+    base = lpgen.random_lp(n // 3, n, seed, slack_frac=0.2)
+    m, n, k = base.m, base.n, len(lengths)
+    rows, cols = [np.repeat(np.arange(m), np.diff(base.row_ptr))], [base.col_idx]
+    vals = [base.values]
+    for i, length in enumerate(lengths):   # free rows, then fixed columns over the others' rows
+        rows.append(np.full(length, m + i)); cols.append(np.sort(rng.choice(n, length, replace=False)))
+        size = min(length, m)
+        rows.append(np.sort(rng.choice(m, size, replace=False))); cols.append(np.full(size, n + i))
+        vals += [rng.uniform(1.0, 2.0, length), rng.uniform(-2.0, 2.0, size)]
+    p, i, v = lpgen.coo_to_csr(m + k, *(np.concatenate(a) for a in (rows, cols, vals)))
+    lp = lpgen.HostLP(m + k, n + k, p, i, v, np.concatenate([base.c, rng.standard_normal(k)]),
+                      np.concatenate([base.AL, np.full(k, -np.inf)]), np.concatenate([base.AU, np.full(k, np.inf)]),
+                      np.concatenate([base.l, np.zeros(k)]), np.concatenate([base.u, np.zeros(k)])).ensure_transpose()
+    assert (max(lp.m, lp.n) <= 8192 and lp.nnz <= 32768) == (n < 5000)
+    compare(lp, capi.Params.defaults(enable_folding=0))

@@ -98,18 +98,18 @@ __global__ void fd_signatures(int n, const int32_t* __restrict__ ids, uint64_t s
 constexpr int kSpmvThread = 16;
 constexpr int kSpmvWarp = 1024;
 __global__ void __launch_bounds__(kThreads)
-fd_spmv(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
+fd_spmv(int rows, int per_warp, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx, const double* __restrict__ val,
         const double* __restrict__ x, const uint8_t* __restrict__ alone, double* __restrict__ y,
         int32_t* __restrict__ long_rows, int32_t* long_count) {
   after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int64_t first = int64_t(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; first < rows;
-       first += int64_t(warps) * 32) {
+  for (int64_t first = int64_t(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp; first < rows;
+       first += int64_t(warps) * per_warp) {
     const int64_t r = first + lane;
     offset_t a = 0, e = 0;
     bool mine = false;
-    if (r < rows) {
+    if (r < rows && lane < per_warp) {
       mine = !alone[r];
       if (mine) {
         a = ptr[r];
@@ -142,6 +142,12 @@ fd_spmv(int rows, const offset_t* __restrict__ ptr, const int32_t* __restrict__ 
       if (lane == 0) y[first + src] = acc;
     }
   }
+}
+// Rows to a warp of fd_spmv: a power of two, 32 once the grid's warps are used up.
+int rows_per_warp(int rows) {
+  int per = 1;
+  while (per < 32 && int64_t(per) * kNumSMs * 8 * (kThreads / 32) < rows) per *= 2;
+  return per;
 }
 // The listed long rows, one block each: seven warps form the next products in
 // shared memory while one thread adds the last ones, so a row costs its chain
@@ -237,8 +243,9 @@ struct Side {
     }
     int32_t* long_count = long_rows.p + n;
     check(cudaMemsetAsync(long_count, 0, sizeof(int32_t), s), "long rows");
-    GPP_LAUNCH(fd_spmv, grid_stride_blocks(n), kThreads, 0, s, n, M.rowPtr, M.colVal, M.nzVal, x, alone.p, value.p,
-               long_rows.p, long_count);
+    const int per_warp = rows_per_warp(n);
+    GPP_LAUNCH(fd_spmv, grid_stride_blocks((int64_t(n) + per_warp - 1) / per_warp * 32), kThreads, 0, s, n, per_warp,
+               M.rowPtr, M.colVal, M.nzVal, x, alone.p, value.p, long_rows.p, long_count);
     GPP_LAUNCH(fd_spmv_long, kNumSMs, kThreads, 0, s, long_rows.p, long_count, M.rowPtr, M.colVal, M.nzVal, x, value.p);
     update(value.p, tol, true, seed, s, other, seq);
   }

@@ -248,12 +248,14 @@ __device__ __forceinline__ int block_append(int32_t* counter, bool take) {
 //   3,000 x 7,500         18,000   2.31     2.37
 //   2,000 x 5,000         25,600   1.83     1.84
 //   3,000 x 7,500         33,000   1.36     1.36
+//   2,193 x 7,154         35,700   3.96     3.98
+//   3,200 x 8,000         41,000   2.26     2.24
 //   3,000 x 7,500         63,000   0.99     0.93
 //   3,000 x 7,500        963,000   2.50     1.80
 //   20,000 x 50,000      240,000   8.85     7.0
 constexpr int kSmallCluster = 8;
 constexpr int kSmallModel = 8192;
-constexpr offset_t kSmallEntries = 32768;
+constexpr offset_t kSmallEntries = 40960;
 inline bool small_model(int rows, int cols, offset_t nnz) {
   return rows <= kSmallModel && cols <= kSmallModel && nnz <= kSmallEntries;
 }

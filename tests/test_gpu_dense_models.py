@@ -48,10 +48,10 @@ def presolve(lp, params):
     return lambda: device.free_summary(device.preprocess(dlp, params))
 
 
-@pytest.mark.parametrize("m,per,fused", [(256, 128, True), (257, 128, False), (1000, 300, False)])
+@pytest.mark.parametrize("m,per,fused", [(320, 128, True), (321, 128, False), (1000, 300, False)])
 def test_small_models_are_bounded_by_entries(m, per, fused):
     params = capi.Params.defaults(enable_folding=0)
-    lp = dense_lp(m, 2000, per - 1, seed=m, slack="bounded")   # m * per entries: the line is at 32,768
+    lp = dense_lp(m, 2000, per - 1, seed=m, slack="bounded")   # m * per entries: the line is at 40,960
     names = kernels_of(presolve(lp, params))
     assert any("probe_and_singleton_columns" in k for k in names) == fused, names
     assert fused or not any("inc_small" in k for k in names), names
@@ -100,5 +100,5 @@ def test_statistics_after_long_rows_and_columns_go(n, seed):
     lp = lpgen.HostLP(m + k, n + k, p, i, v, np.concatenate([base.c, rng.standard_normal(k)]),
                       np.concatenate([base.AL, np.full(k, -np.inf)]), np.concatenate([base.AU, np.full(k, np.inf)]),
                       np.concatenate([base.l, np.zeros(k)]), np.concatenate([base.u, np.zeros(k)])).ensure_transpose()
-    assert (max(lp.m, lp.n) <= 8192 and lp.nnz <= 32768) == (n < 5000)
+    assert (max(lp.m, lp.n) <= 8192 and lp.nnz <= 40960) == (n < 5000)
     compare(lp, capi.Params.defaults(enable_folding=0))

@@ -341,12 +341,13 @@ __global__ void dt_roles(int sel, const int32_t* __restrict__ rows, const int32_
   }
 }
 
-// A row's or column's entries by eight lanes, four items to a warp, or by the
-// whole warp when there are more than kGroupItem.  `range` gives an item's
-// entries or declines it; `body` walks them in `rounds` rounds of W entries, the
-// same number for every lane of the warp.  Bound by the round trips of an item
-// (mask, pointers, entries), so four items in flight a warp: with a warp an item
-// the rebuild of the QAP N = 30 relaxation's 1.7M short rows took 308 + 256 us.
+// A row's or column's entries by eight lanes, `per` items to a warp (items_per_warp),
+// or by the whole warp when there are more than kGroupItem, or than eight while there
+// are warps to spare.  `range` gives an item's entries or declines it; `body` walks them
+// in `rounds` rounds of W entries, the same number for every lane of the warp.  Bound by
+// the round trips of an item (mask, pointers, entries), so four items in flight a warp:
+// with a warp an item the rebuild of the QAP N = 30 relaxation's 1.7M short rows took
+// 308 + 256 us.
 constexpr int kGroupItem = 64;
 template <int W>
 struct Lanes {
@@ -359,14 +360,15 @@ struct Lanes {
   __device__ __forceinline__ double get(double v, int k) const { return __shfl_sync(0xffffffffu, v, k, W); }
 };
 template <class Range, class Body>
-__device__ __forceinline__ void by_groups(int count, const Range& range, const Body& body) {
+__device__ __forceinline__ void by_groups(int count, int per, const Range& range, const Body& body) {
   const int lane = threadIdx.x & 31, grp = lane >> 3, gl = lane & 7;
   const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t w0 = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4; w0 < count; w0 += warps * 4) {
+  const int group_item = per == 4 ? kGroupItem : 8;
+  for (int64_t w0 = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; w0 < count; w0 += warps * per) {
     const int w = int(w0) + grp;
     offset_t first = 0, last = 0;
-    const bool have = w0 + grp < count && range(w, gl, first, last);
-    const bool wide = have && last - first > kGroupItem;
+    const bool have = grp < per && w0 + grp < count && range(w, gl, first, last);
+    const bool wide = have && last - first > group_item;
     const bool mine = have && !wide;
     const int rounds = __reduce_max_sync(0xffffffffu, mine ? int(last - first + 7) / 8 : 0);
     body(Lanes<8>{gl, grp * 8, rounds}, w, mine, first, mine ? last : first);
@@ -379,12 +381,12 @@ __device__ __forceinline__ void by_groups(int count, const Range& range, const B
 }
 
 // Rows holding a shifting column, each listed once.
-__global__ void dt_touch(int sel, const int32_t* __restrict__ role_col, const offset_t* __restrict__ tptr,
+__global__ void dt_touch(int per, int sel, const int32_t* __restrict__ role_col, const offset_t* __restrict__ tptr,
                          const int32_t* __restrict__ tidx, uint32_t* __restrict__ claimed,
                          int32_t* __restrict__ touched, int32_t* st, Report report) {
   after_previous_kernel();
   by_groups(
-      sel,
+      sel, per,
       [&](int w, int, offset_t& first, offset_t& last) {
         const int col = role_col[w];
         if (col < 0) return false;
@@ -411,14 +413,14 @@ __global__ void dt_touch(int sel, const int32_t* __restrict__ role_col, const of
 }
 
 // Row shift of a touched kept row: its terms added in stored column order.
-__global__ void dt_shift(const int32_t* __restrict__ touched, const int32_t* __restrict__ st,
+__global__ void dt_shift(int per, const int32_t* __restrict__ touched, const int32_t* __restrict__ st,
                          const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                          const double* __restrict__ val, const uint8_t* __restrict__ keep_row,
                          const uint8_t* __restrict__ role, const double* __restrict__ value, double zt,
                          double* __restrict__ AL, double* __restrict__ AU) {
   after_previous_kernel();
   by_groups(
-      st[kStTouched],
+      st[kStTouched], per,
       [&](int w, int, offset_t& first, offset_t& last) {
         const int r = touched[w];
         if (!keep_row[r]) return false;
@@ -456,13 +458,13 @@ __global__ void dt_shift(const int32_t* __restrict__ touched, const int32_t* __r
 
 // Substitution deltas alpha * a_(r, elim) at (r, keep) for kept rows r other
 // than the doubleton row (:1127-1151, :1191-1229).
-__global__ void dt_delta_count(int sel, const int32_t* __restrict__ rows, const int32_t* __restrict__ elim_c,
+__global__ void dt_delta_count(int per, int sel, const int32_t* __restrict__ rows, const int32_t* __restrict__ elim_c,
                                const uint8_t* __restrict__ kind, const offset_t* __restrict__ tptr,
                                const int32_t* __restrict__ tidx, const double* __restrict__ tval,
                                const uint8_t* __restrict__ keep_row, double zt, int32_t* __restrict__ cnt) {
   after_previous_kernel();
   by_groups(
-      sel,
+      sel, per,
       [&](int w, int gl, offset_t& first, offset_t& last) {
         if (kind[w] != kPairSubst) {
           if (gl == 0) cnt[w] = 0;
@@ -489,7 +491,7 @@ __global__ void dt_delta_count(int sel, const int32_t* __restrict__ rows, const 
         if (mine && lanes.lane == 0) cnt[w] = c;
       });
 }
-__global__ void dt_delta_fill(int sel, const int32_t* __restrict__ rows, const int32_t* __restrict__ keep_c,
+__global__ void dt_delta_fill(int per, int sel, const int32_t* __restrict__ rows, const int32_t* __restrict__ keep_c,
                               const int32_t* __restrict__ elim_c, const uint8_t* __restrict__ kind,
                               const double* __restrict__ alpha, const offset_t* __restrict__ tptr,
                               const int32_t* __restrict__ tidx, const double* __restrict__ tval,
@@ -497,7 +499,7 @@ __global__ void dt_delta_fill(int sel, const int32_t* __restrict__ rows, const i
                               uint64_t* __restrict__ keys, int32_t* __restrict__ order, double* __restrict__ dval) {
   after_previous_kernel();
   by_groups(
-      sel,
+      sel, per,
       [&](int w, int, offset_t& first, offset_t& last) {
         if (kind[w] != kPairSubst) return false;
         const int e = elim_c[rows[w]];
@@ -568,14 +570,14 @@ __device__ int merge_row(offset_t p, offset_t pe, const int32_t* idx, const doub
 // entries with |a| > zero_tol (warp ballot, order kept); other rows merge
 // sequentially.
 template <bool Write>
-__global__ void dt_rebuild(int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+__global__ void dt_rebuild(int per, int m, const offset_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                            const double* __restrict__ val, const int32_t* __restrict__ dptr,
                            const int32_t* __restrict__ dcol, const double* __restrict__ dv, double zt, bool sorted,
                            int32_t* __restrict__ cnt, const offset_t* __restrict__ optr, int32_t* __restrict__ oidx,
                            double* __restrict__ oval) {
   after_previous_kernel();
   by_groups(
-      m,
+      m, per,
       [&](int r, int gl, offset_t& first, offset_t& last) {
         first = ptr[r];
         last = ptr[r + 1];
@@ -842,6 +844,16 @@ int warp_grid(int64_t items) {
   return int(std::max<int64_t>(1, std::min<int64_t>((items + 7) / 8, int64_t(kNumSMs) * 16)));
 }
 
+// Items to a warp of by_groups, of `mean` entries.  A warp takes its long items one
+// after the other, so they go to a warp each while the grid has one for each: the
+// shifts of 200 rows of 20,000 entries took 1,610 us in fours, 404 so, and rewriting 2,000
+// rows of 1,000 entries 51 us, 19 so.  Short items to a warp each only while they are
+// few: 16,000 rows of 10 entries take 16.5 + 18.6 us in fours, 20.7 + 22.8 with a warp each.
+int items_per_warp(int64_t items, double mean) {
+  const int64_t one = mean > kGroupItem ? kNumSMs * 128 : kNumSMs * 16;
+  return items <= one ? 1 : items <= 2 * one ? 2 : 4;
+}
+
 // Single-row mode (doubleton_equations_scan = 0; rule_doubleton_equations.cu:
 // 1948-2126): the smallest acceptable row (over the stored AT, unsorted as
 // given) is substituted alone.
@@ -981,6 +993,8 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     plan.tape.push_back(std::move(seg));
   }
 
+  const double row_mean = double(lp.A.nnz) / m, col_mean = double(AT.nnz) / n;
+
   // Row shifts.
   {
     DBuf<uint8_t> role(size_t(n), s);
@@ -994,18 +1008,18 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     report = ctx().open_report(kStWords, st.d);
     GPP_LAUNCH(dt_roles, gs, kThreads, 0, s, sel, rows.p, keep_c.p, elim_c.p, kind.p, beta.p, plan.l.p, role.p,
                value.p, role_col.p);
-    GPP_LAUNCH(dt_touch, warp_grid(sel), kThreads, 0, s, sel, role_col.p, AT.ptr, AT.idx, claimed.p, touched.p, st.d,
+    GPP_LAUNCH(dt_touch, warp_grid(sel), kThreads, 0, s, items_per_warp(sel, col_mean), sel, role_col.p, AT.ptr, AT.idx, claimed.p, touched.p, st.d,
                report);
     const int ntouched = int(ctx().await(report)[kStTouched]);
     if (ntouched)
-      GPP_LAUNCH(dt_shift, warp_grid(ntouched), kThreads, 0, s, touched.p, st.d, lp.A.ptr, lp.A.idx, lp.A.val,
+      GPP_LAUNCH(dt_shift, warp_grid(ntouched), kThreads, 0, s, items_per_warp(ntouched, row_mean), touched.p, st.d, lp.A.ptr, lp.A.idx, lp.A.val,
                  plan.keep_row.p, role.p, value.p, zt, plan.AL.p, plan.AU.p);
   }
 
   // Rebuilt matrix.
   if (subst) {
     DBuf<int32_t> dcnt(size_t(sel) + 1, s), dpos(size_t(sel) + 1, s);
-    GPP_LAUNCH(dt_delta_count, warp_grid(sel), kThreads, 0, s, sel, rows.p, elim_c.p, kind.p, AT.ptr, AT.idx, AT.val,
+    GPP_LAUNCH(dt_delta_count, warp_grid(sel), kThreads, 0, s, items_per_warp(sel, col_mean), sel, rows.p, elim_c.p, kind.p, AT.ptr, AT.idx, AT.val,
                plan.keep_row.p, zt, dcnt.p);
     const int total = exclusive_scan_total(dcnt.p, dpos.p, sel, s);
     DBuf<uint64_t> keys(size_t(std::max(total, 1)), s);
@@ -1014,7 +1028,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     DBuf<double> raw(size_t(std::max(total, 1)), s), dv(size_t(std::max(total, 1)), s);
     row_cnt.zero();
     if (total) {
-      GPP_LAUNCH(dt_delta_fill, warp_grid(sel), kThreads, 0, s, sel, rows.p, keep_c.p, elim_c.p, kind.p, alpha.p,
+      GPP_LAUNCH(dt_delta_fill, warp_grid(sel), kThreads, 0, s, items_per_warp(sel, col_mean), sel, rows.p, keep_c.p, elim_c.p, kind.p, alpha.p,
                  AT.ptr, AT.idx, AT.val, plan.keep_row.p, zt, dpos.p, keys.p, order.p, raw.p);
       radix_sort_pairs(keys.p, order.p, total, s, (bits_up_to(m - 1) << 32) | bits_up_to(n - 1));
       GPP_LAUNCH(dt_delta_rows, grid_stride_blocks(total), kThreads, 0, s, int64_t(total), keys.p, order.p, raw.p,
@@ -1027,7 +1041,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     if (a_sorted)
       GPP_LAUNCH(dt_long_delta_rows, grid_stride_blocks(m), kThreads, 0, s, m, lp.A.ptr, dptr.p, long_rows.p,
                  long_count.p);
-    GPP_LAUNCH(dt_rebuild<false>, warp_grid(m), kThreads, 0, s, m, lp.A.ptr, lp.A.idx, lp.A.val, dptr.p, dcol.p,
+    GPP_LAUNCH(dt_rebuild<false>, warp_grid(m), kThreads, 0, s, items_per_warp(m, row_mean), m, lp.A.ptr, lp.A.idx, lp.A.val, dptr.p, dcol.p,
                dv.p, zt, a_sorted, cnt.p, nullptr, nullptr, nullptr);
     if (a_sorted)
       GPP_LAUNCH(dt_rebuild_block<false>, kNumSMs * 4, kThreads, 0, s, long_rows.p, long_count.p, lp.A.ptr, lp.A.idx,
@@ -1039,7 +1053,7 @@ void rule_doubleton_equations(Plan& plan, const WorkingLp& lp, const gpp_params&
     out.nnz = exclusive_scan_total(cnt.p, out.ptr, m, s);
     out.idx = dalloc<int32_t>(size_t(out.nnz));
     out.val = dalloc<double>(size_t(out.nnz));
-    GPP_LAUNCH(dt_rebuild<true>, warp_grid(m), kThreads, 0, s, m, lp.A.ptr, lp.A.idx, lp.A.val, dptr.p, dcol.p,
+    GPP_LAUNCH(dt_rebuild<true>, warp_grid(m), kThreads, 0, s, items_per_warp(m, row_mean), m, lp.A.ptr, lp.A.idx, lp.A.val, dptr.p, dcol.p,
                dv.p, zt, a_sorted, nullptr, out.ptr, out.idx, out.val);
     if (a_sorted)
       GPP_LAUNCH(dt_rebuild_block<true>, kNumSMs * 4, kThreads, 0, s, long_rows.p, long_count.p, lp.A.ptr, lp.A.idx,

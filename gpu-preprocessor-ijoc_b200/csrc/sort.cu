@@ -94,11 +94,23 @@ __device__ __forceinline__ int warp_rank(int* counts, int d) {
 // sorted by.  Against the bitonic network over (key, position) this replaced
 // (78 barriered rounds at 4,096 pairs, 34 us on average over a presolve's
 // sorts) it takes 8-12 us for the two to four windows those sorts have.
+//
+// Few pairs are ranked by comparing each with all, a thread to a pair: 8 to 10 us for up
+// to 100 pairs, 13 for 256 and 18 for 384, where the passes take 8.4 us and 1.65 for each
+// window that varies, whatever the number of pairs (the bitonic network: 8 to 18 us for
+// 2 to 256 pairs).
+constexpr int kCountSort = 48;   // pairs for each byte that varies
 constexpr int kBlockSortMax = 8192;
 constexpr int kBlockSortThreads = 1024;
 constexpr int kBlockSortWarps = kBlockSortThreads / 32;
 constexpr int kBlockSortItems = kBlockSortMax / kBlockSortThreads;
 constexpr size_t kBlockSortCounts = sizeof(int) * kBlockSortWarps * kDigits;
+
+// Bytes that vary: about the passes.
+__device__ __forceinline__ int varying_bytes(uint64_t varying) {
+  return __popc(__vsetgtu4(uint32_t(varying), 0u)) + __popc(__vsetgtu4(uint32_t(varying >> 32), 0u));
+}
+static_assert(kCountSort * 8 <= kBlockSortThreads, "a thread for each pair");
 
 size_t block_sort_smem(int n) {
   const size_t padded = size_t(n + 7) / 8 * 8;
@@ -134,6 +146,24 @@ block_sort_pairs(uint64_t* keys, int32_t* vals, int n, uint64_t may_vary) {
   if (lane == 0 && (lo | hi)) atomicOr(&varies, (uint64_t(hi) << 32) | lo);
   __syncthreads();
   uint64_t left = varies & may_vary;
+  if (n <= kCountSort * varying_bytes(left)) {
+    const int i = threadIdx.x;
+    if (i < n) {
+      const uint64_t mine = k[i] & may_vary;
+      int rank = 0;
+#pragma unroll 8
+      for (int j = 0; j < n; ++j) {
+        const uint64_t other = k[j] & may_vary;
+        rank += other < mine || (other == mine && j < i) ? 1 : 0;
+      }
+      to[rank] = uint16_t(i);
+    }
+    __syncthreads();
+    auto* t = from;
+    from = to;
+    to = t;
+    left = 0;
+  }
   int* own = counts + warp * kDigits;
   const int base = warp * 32 * items + lane;   // a warp owns consecutive positions
   while (left) {

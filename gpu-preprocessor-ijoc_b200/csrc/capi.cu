@@ -796,7 +796,7 @@ int gpp_parallel_row_hashes(const gpp_csr* A, const uint8_t* keep_row, const uin
 
 int gpp_sort_pairs(uint64_t* keys, int32_t* values, int64_t n) {
   return guarded([&] {
-    gpp::radix_sort_pairs(keys, values, n, gpp::ctx().stream);
+    gpp::radix_sort_pairs(keys, values, n, gpp::ctx().stream, ~uint64_t(0), true);
     gpp::ctx().sync("sort pairs");
   });
 }

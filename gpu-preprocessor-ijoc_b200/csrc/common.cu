@@ -71,7 +71,7 @@ Report Context::open_report(int count, int32_t* words) {
   return Report{words, reinterpret_cast<unsigned int*>(report_words + 15), box(seq), seq, count, true};
 }
 
-void Context::poll(const Mailbox* box, uint32_t seq, int words, const char* where) {
+void Context::poll(const Mailbox* box, uint32_t seq, int words, const char* where, bool raise) {
   int k = 0;   // words seen
   auto posted = [&] {
     while (k < words && uint32_t(box->words[k] >> 32) == seq) ++k;
@@ -91,7 +91,7 @@ void Context::poll(const Mailbox* box, uint32_t seq, int words, const char* wher
   std::atomic_thread_fence(std::memory_order_acquire);
   if (profiling())
     profile_sync(where, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
-  raise_device_error(where);
+  if (raise) raise_device_error(where);
 }
 
 void Context::raise_device_error(const char* where) {

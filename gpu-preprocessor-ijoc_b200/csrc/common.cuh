@@ -393,7 +393,8 @@ struct Context {
     return answer;
   }
   int64_t answer[16] = {};
-  void poll(const Mailbox* box, uint32_t seq, int words, const char* where);
+  // Without `raise` the device's error word is left to the next wait.
+  void poll(const Mailbox* box, uint32_t seq, int words, const char* where, bool raise = true);
   cudaStream_t side = nullptr;
   // The blocks this context handed out and those it holds for reuse without a
   // driver call (pool_alloc/free).

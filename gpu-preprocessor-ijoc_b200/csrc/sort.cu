@@ -11,7 +11,7 @@
 // tile ranks its keys, publishes its digit counts and finds its output
 // offsets by a decoupled look-back over its predecessors.  A digit that turns
 // out constant makes its pass return at once (decided on the device, so the
-// sort waits for nothing).
+// sort waits for nothing unless it is told to).
 #include "sort.hpp"
 
 #include <atomic>
@@ -235,33 +235,79 @@ struct SortPlan {
   int failed;   // a look-back's wait ran out
 };
 
+// Digit counts of all passes.  Bound by the eight shared-memory atomics of a key, and
+// before that, with one key of a thread in flight and every shared digit added by itself,
+// by the load's latency and the conflicts on one counter: 154 us for 8 million random
+// keys, 66 now; 8 million equal ones 154 and 33.
+constexpr int kHistogramKeys = 4;   // a thread's keys in flight
 __global__ void __launch_bounds__(kThreads)
-sort_histogram(const uint64_t* __restrict__ keys, int64_t n, SortPasses passes, SortPlan* plan) {
+sort_histogram(const uint64_t* __restrict__ keys, int64_t n, SortPasses passes, SortPlan* plan, Mailbox* mail,
+               uint32_t seq) {
   after_previous_kernel();
   __shared__ int h[kMaxPasses][kDigits];
   __shared__ bool last;
   __shared__ int warp_sums[8];
   for (int p = 0; p < passes.count; ++p) h[p][threadIdx.x] = 0;
   __syncthreads();
-  const int64_t stride = int64_t(gridDim.x) * kThreads;
-  const int64_t top = (n + stride - 1) / stride * stride;
-  for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < top; i += stride) {
-    const bool in = i < n;
-    const uint64_t key = in ? keys[i] : 0;
-    // A digit that all lanes share (high digits of small keys) is added once.
-    const uint64_t lead = __shfl_sync(0xffffffffu, key, 0);
-    const uint64_t diff = in ? key ^ lead : ~0ull;
-    const uint64_t varies = (uint64_t(__reduce_or_sync(0xffffffffu, uint32_t(diff >> 32))) << 32) |
-                            __reduce_or_sync(0xffffffffu, uint32_t(diff));
-    for (int p = 0; p < passes.count; ++p) {
-      const int d = digit_of(key, passes.shift[p]);
-      if (digit_of(varies, passes.shift[p]) == 0) {
-        if ((threadIdx.x & 31) == 0) atomicAdd(&h[p][d], 32);
-      } else if (in) {
-        atomicAdd(&h[p][d], 1);
+  // A digit that all lanes share (high digits of small keys) is counted for the warp, as
+  // long as it stays the same, and added when it changes; so is a whole key.
+  uint64_t run_key = 0;
+  int run_keys = 0;
+  int run_digit[kMaxPasses], run_count[kMaxPasses];
+#pragma unroll
+  for (int p = 0; p < kMaxPasses; ++p) run_digit[p] = run_count[p] = 0;
+  const int lane = threadIdx.x & 31;
+  const auto add_run = [&] {
+    if (run_keys && lane < passes.count) atomicAdd(&h[lane][digit_of(run_key, passes.shift[lane])], run_keys);
+  };
+  const int64_t stride = int64_t(gridDim.x) * kThreads * kHistogramKeys;
+  for (int64_t base = (int64_t(blockIdx.x) * kThreads + threadIdx.x - lane) * kHistogramKeys; base < n; base += stride) {
+    uint64_t key[kHistogramKeys];
+#pragma unroll
+    for (int q = 0; q < kHistogramKeys; ++q) {
+      const int64_t i = base + q * 32 + lane;
+      key[q] = i < n ? keys[i] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kHistogramKeys; ++q) {
+      const int64_t first = base + q * 32;
+      if (first >= n) break;   // warp-uniform
+      const bool in = first + lane < n;
+      const uint64_t lead = __shfl_sync(0xffffffffu, key[q], 0);
+      const uint64_t diff = in ? key[q] ^ lead : ~0ull;
+      const uint64_t varies = (uint64_t(__reduce_or_sync(0xffffffffu, uint32_t(diff >> 32))) << 32) |
+                              __reduce_or_sync(0xffffffffu, uint32_t(diff));
+      if (varies == 0) {
+        if (lead == run_key) {
+          run_keys += 32;
+          continue;
+        }
+        add_run();
+        run_key = lead;
+        run_keys = 32;
+        continue;
+      }
+#pragma unroll
+      for (int p = 0; p < kMaxPasses; ++p) {
+        if (p >= passes.count) break;
+        const int d = digit_of(key[q], passes.shift[p]);
+        if (digit_of(varies, passes.shift[p]) == 0) {
+          if (d != run_digit[p]) {
+            if (lane == 0 && run_count[p]) atomicAdd(&h[p][run_digit[p]], run_count[p]);
+            run_digit[p] = d;
+            run_count[p] = 0;
+          }
+          run_count[p] += 32;
+        } else if (in) {
+          atomicAdd(&h[p][d], 1);
+        }
       }
     }
   }
+  add_run();
+#pragma unroll
+  for (int p = 0; p < kMaxPasses; ++p)
+    if (lane == 0 && run_count[p]) atomicAdd(&h[p][run_digit[p]], run_count[p]);
   __syncthreads();
   for (int p = 0; p < passes.count; ++p) {
     const int c = h[p][threadIdx.x];
@@ -274,9 +320,11 @@ sort_histogram(const uint64_t* __restrict__ keys, int64_t n, SortPasses passes, 
   if (!last) return;
   __threadfence();
   int source = 0;
+  uint32_t constants = 0;
   for (int p = 0; p < passes.count; ++p) {
     const unsigned long long c = __ldcg(&plan->counts[p][threadIdx.x]);
-    // 64-bit scan of the counts as two 31-bit halves (their sums stay below 2^31 x 256).
+    // 64-bit scan of the counts as two halves split at bit 22 (256 low halves stay below
+    // 2^30, the high ones' sum is at most n / 2^22).
     const int low = scan_digits(int(c & 0x3fffff), warp_sums), high = scan_digits(int(c >> 22), warp_sums);
     plan->start[p][threadIdx.x] = (long long)low + ((long long)high << 22);
     const int constant = __syncthreads_or(c == (unsigned long long)n);
@@ -284,9 +332,13 @@ sort_histogram(const uint64_t* __restrict__ keys, int64_t n, SortPasses passes, 
       plan->constant[p] = constant;
       plan->source[p] = source;
     }
-    if (!constant) source ^= 1;
+    if (constant) constants |= 1u << p;
+    else source ^= 1;
   }
-  if (threadIdx.x == 0) plan->source[passes.count] = source;
+  if (threadIdx.x == 0) {
+    plan->source[passes.count] = source;
+    if (mail) post_values(mail, seq, constants);
+  }
 }
 
 // A tile's published word per digit: two flag bits (0 nothing yet, 1 the
@@ -327,7 +379,7 @@ __device__ __forceinline__ void st_word(unsigned long long* p, unsigned long lon
 // kItems x 256 pairs: sixteen items keep the look-back short against the
 // tile's work on large inputs, eight spread mid-size inputs over the SMs.
 // 2,000,003 random pairs: 506 us before (four launches a pass: histogram, two
-// of scan, scatter), 317 now; the look-back by one tile a round trip took 327
+// of scan, scatter), 294 now; the look-back by one tile a round trip took 10 us more
 // (and 129 against 113 for 250,000 pairs).
 constexpr int kPolls = 1 << 22;
 std::atomic<int> g_max_polls{kPolls};
@@ -487,8 +539,15 @@ void allow_shared_memory() {
   configured[size_t(dev)] = true;
 }
 
+// With `ask` the host learns from the histogram which digits are constant and leaves
+// their passes out.  It waits for that behind the first kAskBehind passes, so the device
+// has work meanwhile.  A pass that returns at once costs 2 to 5 us: 20,000 equal keys
+// took 42 us, 24 so, and 8 million with one byte that varies 292, 201 so with the
+// histogram's share of that.
+constexpr int kAskBehind = 2;
+
 template <int kItems, class Word>
-void sort_tiles(uint64_t* keys, int32_t* vals, int64_t n, const SortPasses& passes, cudaStream_t s) {
+void sort_tiles(uint64_t* keys, int32_t* vals, int64_t n, const SortPasses& passes, cudaStream_t s, bool ask) {
   const int64_t tiles = (n + SortTile<kItems>::kPairs - 1) / SortTile<kItems>::kPairs;
   const size_t words = size_t(tiles) * kDigits;
   DBuf<uint64_t> k2(size_t(n), s);
@@ -497,11 +556,24 @@ void sort_tiles(uint64_t* keys, int32_t* vals, int64_t n, const SortPasses& pass
   scratch.zero();
   auto* plan = reinterpret_cast<SortPlan*>(scratch.p);
   auto* tile_words = reinterpret_cast<Word*>(scratch.p + sizeof(SortPlan));
-  GPP_LAUNCH_BYTES(sort_histogram, 8.0 * n, grid_stride_blocks(n, kThreads, 4), kThreads, 0, s, keys, n, passes, plan);
-  for (int p = 0; p < passes.count; ++p)
+  auto& c = ctx();
+  ask = ask && passes.count > kAskBehind;
+  const uint32_t seq = ask ? c.open_mail() : 0;
+  Mailbox* const mail = ask ? c.box(seq) : nullptr;
+  GPP_LAUNCH_BYTES(sort_histogram, 8.0 * n, grid_stride_blocks((n + kHistogramKeys - 1) / kHistogramKeys, kThreads, 4),
+                   kThreads, 0, s, keys, n, passes, plan, mail, seq);
+  uint64_t constants = 0;
+  for (int p = 0; p < passes.count; ++p) {
+    if (ask && p == kAskBehind) {
+      c.poll(mail, seq, 4, "constant digits", false);   // an expired wait still needs the last launch
+      constants = mail->words[0] & 0xffffffffu;
+    }
+    if (constants >> p & 1u) continue;
     GPP_LAUNCH_BYTES((sort_pass<kItems, Word>), 24.0 * n, int(tiles), kThreads, SortTile<kItems>::kBytes, s, keys, vals,
                      k2.p, v2.p, n, p, passes.shift[p], plan, tile_words + words * size_t(p),
-                     g_max_polls.load(std::memory_order_relaxed), ctx().host_error);
+                     g_max_polls.load(std::memory_order_relaxed), c.host_error);
+  }
+  if (constants + 1 == uint64_t(1) << passes.count) return;   // nothing moved
   GPP_LAUNCH(sort_copy_back, grid_stride_blocks(n), kThreads, 0, s, n, passes.count, plan, keys, vals, k2.p, v2.p);
 }
 
@@ -509,7 +581,7 @@ void sort_tiles(uint64_t* keys, int32_t* vals, int64_t n, const SortPasses& pass
 
 void inject_sort_wait_limit(int polls) { g_max_polls.store(polls > 0 ? polls : kPolls); }
 
-void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, uint64_t may_vary) {
+void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, uint64_t may_vary, bool ask) {
   if (n <= 1 || may_vary == 0) return;
   allow_shared_memory();
   if (n <= kBlockSortMax) {
@@ -517,9 +589,9 @@ void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, 
     return;
   }
   const SortPasses passes = passes_of(may_vary);
-  if (n < (int64_t(1) << 20)) sort_tiles<8, uint32_t>(keys, vals, n, passes, s);
-  else if (n < (int64_t(1) << 30)) sort_tiles<16, uint32_t>(keys, vals, n, passes, s);
-  else sort_tiles<16, unsigned long long>(keys, vals, n, passes, s);   // counts past 30 bits
+  if (n < (int64_t(1) << 20)) sort_tiles<8, uint32_t>(keys, vals, n, passes, s, ask);
+  else if (n < (int64_t(1) << 30)) sort_tiles<16, uint32_t>(keys, vals, n, passes, s, ask);
+  else sort_tiles<16, unsigned long long>(keys, vals, n, passes, s, ask);   // counts past 30 bits
 }
 
 }  // namespace gpp

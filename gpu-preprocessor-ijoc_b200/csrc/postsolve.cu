@@ -320,17 +320,21 @@ __global__ void scatter_solution(Sol s, const double* __restrict__ x_red, const 
   }
 }
 
-// The fixed-value segments of a record: a column is removed once, so it is in
-// one of them at most and they can be restored together.
-struct FixedView {
-  const int32_t* idx;
-  const double* val;
-  int64_t count;
+// The fixed-value segments of a record, up to 64 a launch: a column is removed once, so
+// it is in one of them at most and they can be restored together.
+struct FixedViews {
+  static constexpr int kMax = 64;
+  int count;
+  struct {
+    const int32_t* idx;
+    const double* val;
+    int64_t count;
+  } segment[kMax];
 };
-__global__ void restore_fixed(double* __restrict__ x, const FixedView* __restrict__ fixed, int segments) {
+__global__ void restore_fixed(double* __restrict__ x, FixedViews fixed) {
   after_previous_kernel();
-  for (int k = 0; k < segments; ++k) {
-    const FixedView f = fixed[k];
+  for (int k = 0; k < fixed.count; ++k) {
+    const auto& f = fixed.segment[k];
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < f.count; i += int64_t(gridDim.x) * blockDim.x)
       x[f.idx[i]] = f.val[i];
   }
@@ -855,38 +859,38 @@ void run_postsolve(const PresolveOutput& out, const double* x_red, const double*
   if (r.n || r.m)
     GPP_LAUNCH(scatter_solution, grid_stride_blocks(std::max(r.n, r.m)), kThreads, 0, st, s, x_red, y_red, z_red,
                r.rows.p, r.m, r.cols.p, r.n);
-  // Views of the record's segments, uploaded together: the tape's segments,
-  // the global index of each one's first record, the fixed-value segments.
+  for (size_t first = 0; first < r.fixed.size();) {
+    FixedViews v{};
+    int64_t most = 0;
+    for (; first < r.fixed.size() && v.count < FixedViews::kMax; ++first) {
+      const FixedSegment& f = r.fixed[first];
+      if (!f.count) continue;
+      v.segment[v.count++] = {f.idx.p, f.val.p, f.count};
+      most = std::max(most, f.count);
+    }
+    if (v.count) GPP_LAUNCH(restore_fixed, grid_stride_blocks(most), kThreads, 0, st, x, v);
+  }
+  // Views of the tape's segments and the global index of each one's first record,
+  // uploaded together.
   std::vector<SegView> segs;
   std::vector<int64_t> starts;
-  std::vector<FixedView> fixed;
-  int64_t total = 0, most_fixed = 0;
+  int64_t total = 0;
   for (const auto& seg : r.segments) {
     if (!seg.count) continue;
     segs.push_back(view(seg));
     starts.push_back(total);
     total += seg.count;
   }
-  for (const auto& f : r.fixed) {
-    if (!f.count) continue;
-    fixed.push_back({f.idx.p, f.val.p, f.count});
-    most_fixed = std::max(most_fixed, f.count);
-  }
-  const size_t seg_bytes = sizeof(SegView) * segs.size(), start_bytes = sizeof(int64_t) * starts.size(),
-               fixed_bytes = sizeof(FixedView) * fixed.size();
-  std::vector<unsigned char> packed(seg_bytes + start_bytes + fixed_bytes);
+  const size_t seg_bytes = sizeof(SegView) * segs.size(), start_bytes = sizeof(int64_t) * starts.size();
+  std::vector<unsigned char> packed(seg_bytes + start_bytes);
   DBuf<unsigned char> views(packed.size(), st);
   if (!packed.empty()) {
-    if (seg_bytes) std::memcpy(packed.data(), segs.data(), seg_bytes);
-    if (start_bytes) std::memcpy(packed.data() + seg_bytes, starts.data(), start_bytes);
-    if (fixed_bytes) std::memcpy(packed.data() + seg_bytes + start_bytes, fixed.data(), fixed_bytes);
+    std::memcpy(packed.data(), segs.data(), seg_bytes);
+    std::memcpy(packed.data() + seg_bytes, starts.data(), start_bytes);
     check(cudaMemcpyAsync(views.p, packed.data(), packed.size(), cudaMemcpyHostToDevice, st), "record views");
   }
   const TapeView t{reinterpret_cast<const SegView*>(views.p), reinterpret_cast<const int64_t*>(views.p + seg_bytes),
                    int(segs.size()), total};
-  if (!fixed.empty())
-    GPP_LAUNCH(restore_fixed, grid_stride_blocks(most_fixed), kThreads, 0, st, x,
-               reinterpret_cast<const FixedView*>(views.p + seg_bytes + start_bytes), int(fixed.size()));
   Model M{};
   if (original) {
     M = Model{original->A.rowPtr, original->AT.rowPtr, original->A.colVal, original->AT.colVal, original->A.nzVal,

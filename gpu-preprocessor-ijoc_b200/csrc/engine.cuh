@@ -303,7 +303,7 @@ void col_max_abs(const DevCsr& AT, const uint8_t* keep_row, double* out, cudaStr
 
 // compact.cu
 int32_t build_old_to_new(const uint8_t* keep, int32_t n, int32_t* old_to_new, cudaStream_t s);
-// Both maps of a materialisation at once (two launches, one readback); returns
+// Both maps of a materialisation at once (one launch, one answer); returns
 // the kept row and column counts.
 std::pair<int32_t, int32_t> build_old_to_new_pair(const uint8_t* keep_row, int32_t m, int32_t* row_map,
                                                   const uint8_t* keep_col, int32_t n, int32_t* col_map,

@@ -405,11 +405,14 @@ __device__ __forceinline__ bool replays_in(int type, bool dual) {
 // A record that replay_record leaves without a write whatever z, y and the
 // retrieval flags hold.  A row-implied bound change acts only if exactly one
 // of its bounds moved and x sits at the implied one (x is final before the
-// dual pass).  On most points almost none does, while each would tie all
-// columns of its row into one group: on the QAP N = 30 relaxation the 0.8M
+// dual pass).  At a point off the bounds almost none does, while each would tie
+// all columns of its row into one group: on the QAP N = 30 relaxation the 0.8M
 // records formed one group that a single thread replayed in 1,325 ms; without
 // the records that cannot act the whole call (presolve and postsolve) takes
-// 13.2 ms, 1,350 ms before.
+// 7.2 ms, 1,306 ms before.  At a point on the bounds, as a solver's is, they act
+// and the groups stay: the QAP N = 12 relaxation's postsolve takes 0.1 ms for a
+// point off all bounds (29.6 before), 36 ms with half of x on them (49) and 57
+// ms with all (66).
 __device__ __forceinline__ bool acts_in_dual(int type, const int32_t* id, int64_t ni, const double* v,
                                              const Model& M, const double* x) {
   if (type != kRowImpliedBoundChange) return true;
@@ -596,7 +599,7 @@ __global__ void rg_roots(int count, int32_t* parent, uint8_t* __restrict__ share
 // are listed as (root, record) for the sort.  Most records are alone, so the
 // sort sees few, and the whole tape needs one wait per pass (500,000 x
 // 1,250,000 random LP: 862 us before, with every record sorted, four waits
-// and one marking launch per segment; 375 us now).
+// and one marking launch per segment; 272 us now).
 __global__ void __launch_bounds__(kThreads) rg_replay_alone(TapeView t, int64_t lo, int count, int dual, Sol s, Model M,
                                                             int32_t* parent, const uint8_t* __restrict__ shared_root,
                                                             uint64_t* __restrict__ keys, int32_t* __restrict__ vals,

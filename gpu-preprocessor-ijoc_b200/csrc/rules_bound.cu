@@ -439,7 +439,7 @@ __device__ __forceinline__ void sum_tiles(int tiles, const FinalBounds& out, con
 // block to finish sums the tiles' counts (commit_bounds ranks within the tile).
 // A column whose bounds stand costs its reads alone; the packed bounds and the
 // candidates, which the next sweep starts from, are written where they differ.
-// Bound by DRAM (41 bytes a column) where bounds stand, by the gathers of the
+// Bound by DRAM (42 bytes a column) where bounds stand, by the gathers of the
 // moved columns' rows else: 376 us a sweep of the 29.8M-nnz LP's 5M columns, 446
 // before the maximum's walk ended early.  A form that handed its tiles out in order
 // and looked back for the records before them took 69 us against 45 at 500,001

@@ -23,7 +23,10 @@ namespace gpp {
 namespace {
 
 constexpr int kDigits = 256;
-constexpr int kMaxPasses = 8;   // windows are disjoint and eight bits wide, of a 64-bit key
+// Windows are eight bits wide, of a 64-bit key; they start at their lowest varying bit, but
+// at bit 56 at most, where the last may cover bits of the one before it (harmless, as a
+// pass is stable).
+constexpr int kMaxPasses = 8;
 
 struct SortPasses {
   int count = 0;

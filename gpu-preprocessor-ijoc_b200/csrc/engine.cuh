@@ -355,8 +355,8 @@ constexpr uint32_t kProbeFixed = 1, kProbeEmptyColumns = 2, kProbeEmptyRows = 4,
 // The singleton-column rule up to its one question, which the probe may ask
 // along with its own: where the probe finds nothing (most rounds) the rule runs
 // on the plan as it stands, so its kernels follow the probe's without a wait,
-// and on the device do nothing when the probe found something.  Up to
-// kSmallModel rows and columns probe and rule are one launch of one cluster.
+// and on the device do nothing when the probe found something.  In small models
+// (small_model) probe and rule are one launch of one cluster.
 struct SingletonTest {
   DBuf<int32_t> cand, rows, long_rows, winners;
   DBuf<double> fmin, fmax, side, contrib_val;

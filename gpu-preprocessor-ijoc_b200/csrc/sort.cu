@@ -110,8 +110,11 @@ constexpr int kBlockSortItems = kBlockSortMax / kBlockSortThreads;
 constexpr size_t kBlockSortCounts = sizeof(int) * kBlockSortWarps * kDigits;
 
 // Bytes that vary: about the passes.
-__device__ __forceinline__ int varying_bytes(uint64_t varying) {
-  return __popc(__vsetgtu4(uint32_t(varying), 0u)) + __popc(__vsetgtu4(uint32_t(varying >> 32), 0u));
+__host__ __device__ __forceinline__ int varying_bytes(uint64_t varying) {
+  int count = 0;
+#pragma unroll
+  for (int k = 0; k < 64; k += 8) count += (varying >> k & 0xff) != 0;
+  return count;
 }
 static_assert(kCountSort * 8 <= kBlockSortThreads, "a thread for each pair");
 
@@ -120,6 +123,7 @@ size_t block_sort_smem(int n) {
   return kBlockSortCounts + padded * (sizeof(uint64_t) + 2 * sizeof(uint16_t));
 }
 
+template <bool kMayCount>
 __global__ void __launch_bounds__(kBlockSortThreads)
 block_sort_pairs(uint64_t* keys, int32_t* vals, int n, uint64_t may_vary) {
   after_previous_kernel();
@@ -149,7 +153,7 @@ block_sort_pairs(uint64_t* keys, int32_t* vals, int n, uint64_t may_vary) {
   if (lane == 0 && (lo | hi)) atomicOr(&varies, (uint64_t(hi) << 32) | lo);
   __syncthreads();
   uint64_t left = varies & may_vary;
-  if (n <= kCountSort * varying_bytes(left)) {
+  if (kMayCount && n <= kCountSort * varying_bytes(left)) {
     const int i = threadIdx.x;
     if (i < n) {
       const uint64_t mine = k[i] & may_vary;
@@ -535,7 +539,8 @@ void allow_shared_memory() {
   const auto set = [](auto kernel, size_t bytes) {
     check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)), "sort smem");
   };
-  set(block_sort_pairs, block_sort_smem(kBlockSortMax));
+  set(block_sort_pairs<false>, block_sort_smem(kBlockSortMax));
+  set(block_sort_pairs<true>, block_sort_smem(kCountSort * 8));
   set(sort_pass<8, uint32_t>, SortTile<8>::kBytes);
   set(sort_pass<16, uint32_t>, SortTile<16>::kBytes);
   set(sort_pass<16, unsigned long long>, SortTile<16>::kBytes);
@@ -588,7 +593,10 @@ void radix_sort_pairs(uint64_t* keys, int32_t* vals, int64_t n, cudaStream_t s, 
   if (n <= 1 || may_vary == 0) return;
   allow_shared_memory();
   if (n <= kBlockSortMax) {
-    GPP_LAUNCH(block_sort_pairs, 1, kBlockSortThreads, block_sort_smem(int(n)), s, keys, vals, int(n), may_vary);
+    if (n <= kCountSort * varying_bytes(may_vary))   // few enough for the counting, as far as the host knows
+      GPP_LAUNCH(block_sort_pairs<true>, 1, kBlockSortThreads, block_sort_smem(int(n)), s, keys, vals, int(n), may_vary);
+    else
+      GPP_LAUNCH(block_sort_pairs<false>, 1, kBlockSortThreads, block_sort_smem(int(n)), s, keys, vals, int(n), may_vary);
     return;
   }
   const SortPasses passes = passes_of(may_vary);
